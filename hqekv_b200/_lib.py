@@ -121,6 +121,22 @@ def _load():
 lib = _load()
 
 
+def _load_host():
+    """The operators' host path (csrc/host.cpp), bound to the library loaded above."""
+    import importlib.util
+    path = os.path.join(HERE, "_host.so")
+    if not os.path.exists(path):
+        raise ImportError(f"{path} is missing: build it with `python -m hqekv_b200.build`")
+    spec = importlib.util.spec_from_file_location("hqekv_b200._host", path)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    module.bind(*[C.cast(getattr(lib, name), C.c_void_p).value for name in
+                  ("hqkv_decode_workspace_bytes", "hqkv_decode_attention", "hqkv_decode_attention_headsum",
+                   "hqkv_quantize_pack", "hqkv_dequantize_unpack", "hqkv_head_sum")],
+                decode_workspace)
+    return module
+
+
 def check(rc):
     if rc != 0:
         raise HqkvError(rc, lib.hqkv_last_error().decode())
@@ -169,3 +185,6 @@ def decode_workspace(device, nbytes, stream=None):
         buf = torch.zeros(grow, dtype=torch.uint8, device=device)
         _decode_ws[key] = buf
     return buf
+
+
+host = _load_host()

@@ -1,4 +1,5 @@
-"""Build libhqkv.so (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Build libhqkv.so (the C-ABI library) in-tree with nvcc for sm_100a, and _host.so (the operators' host path, a CPython
+module over it) with g++.
 
     python -m hqekv_b200.build          # rebuild if the library was not compiled from the sources present
     python -m hqekv_b200.build --force
@@ -17,6 +18,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB_PATH = os.path.join(HERE, "libhqkv.so")
+HOST_PATH = os.path.join(HERE, "_host.so")
 SOURCES = ["codec.cu", "decode.cu", "gemv.cu", "policy.cu"]
 NVCC_FLAGS = [
     "-std=c++17", "-O3", "-lineinfo",
@@ -58,8 +60,8 @@ def library_id(path=LIB_PATH):
 
 
 def needs_build():
-    """True when the library is missing or was compiled from other sources than the ones present."""
-    return not os.path.exists(LIB_PATH) or library_id(LIB_PATH) != source_id()
+    """True when the library or the host module is missing or was compiled from other sources than the ones present."""
+    return library_id(LIB_PATH) != source_id() or library_id(HOST_PATH) != source_id()
 
 
 CHECKED_LIB_PATH = os.path.join(HERE, "libhqkv_checked.so")
@@ -76,7 +78,27 @@ def build(force=False, verbose=False, checks=False):
         return _compile(CHECKED_LIB_PATH, os.path.join(HERE, "build", "checked"), ["-DHQKV_CHECKS"], verbose)
     if not force and not needs_build():
         return LIB_PATH
-    return _compile(LIB_PATH, os.path.join(HERE, "build"), [], verbose)
+    host = _compile_host()
+    path = _compile(LIB_PATH, os.path.join(HERE, "build"), [], verbose)
+    out, _ = host.communicate()
+    if host.returncode != 0:
+        raise RuntimeError(f"g++ failed on host.cpp:\n{out}")
+    return path
+
+
+def _compile_host():
+    """Start the compiler on the host module; torch's headers and libraries are those of the running interpreter."""
+    import sysconfig
+    import torch
+    root = os.path.join(os.path.dirname(torch.__file__))
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DHQKV_BUILD_ID="{source_id()}"',
+           "-I", INCLUDE, "-I", os.path.join(root, "include"), "-I", os.path.join(cuda, "include"),
+           "-I", sysconfig.get_paths()["include"], os.path.join(CSRC, "host.cpp"), "-o", HOST_PATH,
+           "-L", os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
+           "-Wl,-rpath," + os.path.join(root, "lib")]
+    return subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
 
 
 def _compile(lib_path, objdir, extra, verbose):

@@ -1,0 +1,329 @@
+// Host path of the per-layer operators in native code (a CPython module over libhqkv's C ABI).
+//
+// A decode step calls these once per layer; the two kernels of a call take 10 - 20 us at batch 1, and walking the
+// 42-slot tuple, filling a ctypes descriptor and allocating the results from Python took 18 - 25 us.  Here the tuple
+// is read directly (40 pointer loads, no memo to look up or to keep valid), the results come from torch's allocator
+// and the library is called through its function pointers: 5 - 6 us.
+//
+// Every function returns None for arguments it does not take as they are (non-contiguous tiers, wrong types, CPU
+// tensors, an error status): the Python operator then goes its general way, which copies or raises.
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <cmath>
+#include <vector>
+
+#include "hqkv.h"
+
+#ifndef HQKV_BUILD_ID
+#define HQKV_BUILD_ID "unstamped"
+#endif
+static const char g_build_stamp[] = "HQKV_BUILD_ID=" HQKV_BUILD_ID;
+
+namespace {
+
+// entry points of the library that _lib.py has loaded (it may be another build of it, so nothing is linked here)
+struct Lib {
+  decltype(&hqkv_decode_workspace_bytes) decode_workspace_bytes;
+  decltype(&hqkv_decode_attention) decode_attention;
+  decltype(&hqkv_decode_attention_headsum) decode_attention_headsum;
+  decltype(&hqkv_quantize_pack) quantize_pack;
+  decltype(&hqkv_dequantize_unpack) dequantize_unpack;
+  decltype(&hqkv_head_sum) head_sum;
+} L;
+PyObject* g_workspace_fn = nullptr;  // _lib.decode_workspace(device, bytes, stream): owns the scratch buffers
+bool g_bound = false;
+
+constexpr int kSlotK[HQKV_NUM_TIERS] = {0, 4, 12, 20, 28}, kSlotV[HQKV_NUM_TIERS] = {2, 8, 16, 24, 32};
+constexpr int kBits[HQKV_NUM_TIERS] = {16, 8, 4, 2, 1};
+constexpr int kSlotNewK = 39, kSlotNewV = 40, kSlots = 42;
+
+// a slot as a contiguous CUDA tensor: false if it is something else; *t stays null for None
+inline bool slot(PyObject* o, const at::Tensor** t) {
+  if (o == Py_None) {
+    *t = nullptr;
+    return true;
+  }
+  if (!THPVariable_Check(o)) return false;
+  const at::Tensor& v = THPVariable_Unpack(o);
+  if (!v.is_cuda() || !v.is_contiguous()) return false;
+  *t = &v;
+  return true;
+}
+inline void* ptr(const at::Tensor* t) { return t ? t->data_ptr() : nullptr; }
+
+PyObject* none() { Py_RETURN_NONE; }
+
+PyObject* bind(PyObject*, PyObject* args) {
+  unsigned long long a[6];
+  PyObject* fn;
+  if (!PyArg_ParseTuple(args, "KKKKKKO", &a[0], &a[1], &a[2], &a[3], &a[4], &a[5], &fn)) return nullptr;
+  L.decode_workspace_bytes = reinterpret_cast<decltype(L.decode_workspace_bytes)>(a[0]);
+  L.decode_attention = reinterpret_cast<decltype(L.decode_attention)>(a[1]);
+  L.decode_attention_headsum = reinterpret_cast<decltype(L.decode_attention_headsum)>(a[2]);
+  L.quantize_pack = reinterpret_cast<decltype(L.quantize_pack)>(a[3]);
+  L.dequantize_unpack = reinterpret_cast<decltype(L.dequantize_unpack)>(a[4]);
+  L.head_sum = reinterpret_cast<decltype(L.head_sum)>(a[5]);
+  Py_INCREF(fn);
+  Py_XDECREF(g_workspace_fn);
+  g_workspace_fn = fn;
+  g_bound = true;
+  Py_RETURN_NONE;
+}
+
+// ---- scratch of the decode call: the buffers belong to _lib.decode_workspace, one per (device, stream), and are
+//      never released; here only their addresses are remembered (under the GIL)
+struct Scratch {
+  int dev;
+  cudaStream_t stream;
+  void* p;
+  size_t bytes;
+};
+std::vector<Scratch> g_scratch;
+
+bool scratch(int dev, cudaStream_t st, size_t need, PyObject* any_tensor, void** p, size_t* bytes) {
+  for (const Scratch& s : g_scratch)
+    if (s.dev == dev && s.stream == st && s.bytes >= need) {
+      *p = s.p;
+      *bytes = s.bytes;
+      return true;
+    }
+  PyObject* device = PyObject_GetAttrString(any_tensor, "device");
+  if (!device) return false;
+  PyObject* buf = PyObject_CallFunction(g_workspace_fn, "OKK", device, static_cast<unsigned long long>(need),
+                                        static_cast<unsigned long long>(reinterpret_cast<uintptr_t>(st)));
+  Py_DECREF(device);
+  if (!buf) return false;
+  const at::Tensor& t = THPVariable_Unpack(buf);
+  Scratch s{dev, st, t.data_ptr(), static_cast<size_t>(t.numel())};
+  Py_DECREF(buf);
+  bool known = false;
+  for (Scratch& o : g_scratch)
+    if (o.dev == dev && o.stream == st) {
+      o = s;
+      known = true;
+    }
+  if (!known) g_scratch.push_back(s);
+  *p = s.p;
+  *bytes = s.bytes;
+  return true;
+}
+
+inline cudaStream_t current_stream(const at::Tensor& t) {
+  return c10::cuda::getCurrentCUDAStream(t.device().index()).stream();
+}
+
+PyObject* pack(std::initializer_list<at::Tensor> ts) {
+  PyObject* out = PyTuple_New(static_cast<Py_ssize_t>(ts.size()));
+  if (!out) return nullptr;
+  Py_ssize_t i = 0;
+  for (const at::Tensor& t : ts) {
+    PyObject* w = THPVariable_Wrap(t);
+    if (!w) {
+      Py_DECREF(out);
+      return nullptr;
+    }
+    PyTuple_SET_ITEM(out, i++, w);
+  }
+  return out;
+}
+
+// decode(q, cache, block_size, group_size, low_codec, head_sum_row | None) -> (attn_weights, attn_output) | None
+PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  if (!g_bound || na != 6 || !THPVariable_Check(a[0]) || !PyTuple_Check(a[1]) || PyTuple_GET_SIZE(a[1]) != kSlots)
+    return none();
+  const at::Tensor& q_in = THPVariable_Unpack(a[0]);
+  if (!q_in.is_cuda() || q_in.scalar_type() != at::kHalf || q_in.dim() != 4 || q_in.size(2) != 1) return none();
+  PyObject* cache = a[1];
+  hqkv_cache_desc_t d = {};
+  d.group_k = static_cast<int32_t>(PyLong_AsLong(a[2]));
+  d.group_v = static_cast<int32_t>(PyLong_AsLong(a[3]));
+  const int low_codec = static_cast<int>(PyLong_AsLong(a[4]));
+  if (PyErr_Occurred()) {
+    PyErr_Clear();
+    return none();
+  }
+  int64_t B = 0, H = 0, D = 0, n_k = 0;
+  const at::Tensor* where = nullptr;
+  for (int t = 0; t < HQKV_NUM_TIERS; ++t) {
+    const at::Tensor *k[4] = {}, *v[4] = {};
+    const int parts = t == 0 ? 2 : 4;
+    for (int i = 0; i < parts; ++i)
+      if (!slot(PyTuple_GET_ITEM(cache, kSlotK[t] + i), &k[i]) || !slot(PyTuple_GET_ITEM(cache, kSlotV[t] + i), &v[i]))
+        return none();
+    hqkv_tier_t& T = d.tier[t];
+    T.bits = kBits[t];
+    T.codec = kBits[t] == 1 ? low_codec : 0;
+    for (const at::Tensor* idx : {k[1], v[1]})
+      if (idx && idx->scalar_type() != at::kLong) return none();
+    T.n_k = k[1] ? static_cast<int32_t>(k[1]->numel()) : 0;
+    T.n_v = v[1] ? static_cast<int32_t>(v[1]->numel()) : 0;
+    n_k += T.n_k;
+    T.k_data = ptr(k[0]);
+    T.k_idx = static_cast<const int64_t*>(ptr(k[1]));
+    T.k_scale = ptr(k[2]);
+    T.k_zero = ptr(k[3]);
+    T.v_data = ptr(v[0]);
+    T.v_idx = static_cast<const int64_t*>(ptr(v[1]));
+    T.v_scale = ptr(v[2]);
+    T.v_zero = ptr(v[3]);
+    if (v[0]) {
+      if (v[0]->dim() != 4) return none();
+      B = v[0]->size(0);
+      H = v[0]->size(1);
+      D = v[0]->size(3) * (t == 0 ? 1 : 32 / kBits[t]);
+      where = v[0];
+    }
+  }
+  const at::Tensor *nk, *nv;
+  if (!slot(PyTuple_GET_ITEM(cache, kSlotNewK), &nk) || !slot(PyTuple_GET_ITEM(cache, kSlotNewV), &nv)) return none();
+  if (nv) {
+    if (nv->dim() != 4 || (where && (nv->size(0) != B || nv->size(1) != H || nv->size(3) != D))) return none();
+    B = nv->size(0);
+    H = nv->size(1);
+    D = nv->size(3);
+    d.n_new = static_cast<int32_t>(nv->size(2));
+    where = nv;
+  }
+  if (!where || where->device() != q_in.device() || q_in.size(0) != B || q_in.size(3) != D) return none();
+  d.new_k = ptr(nk);
+  d.new_v = ptr(nv);
+  const int64_t nh_q = q_in.size(1), len = n_k + d.n_new;
+  d.B = static_cast<int32_t>(B);
+  d.H = static_cast<int32_t>(H);
+  d.D = static_cast<int32_t>(D);
+  d.nh_q = static_cast<int32_t>(nh_q);
+  d.softmax_scale = static_cast<float>(1.0 / std::sqrt(static_cast<double>(D)));
+  void* row = nullptr;
+  if (a[5] != Py_None) {
+    if (!THPVariable_Check(a[5])) return none();
+    const at::Tensor& r = THPVariable_Unpack(a[5]);
+    if (r.scalar_type() != at::kHalf || r.device() != q_in.device() || r.dim() != 1 || r.numel() < len || r.stride(0) != 1)
+      return none();
+    row = r.data_ptr();
+  }
+  const size_t need = L.decode_workspace_bytes(&d);
+  if (need == 0) return none();
+  const c10::cuda::OptionalCUDAGuard guard(q_in.device());
+  const cudaStream_t st = current_stream(q_in);
+  void* ws;
+  size_t ws_bytes;
+  if (!scratch(q_in.device().index(), st, need, a[0], &ws, &ws_bytes)) return nullptr;
+  const at::Tensor q = q_in.contiguous();
+  at::Tensor weights = at::empty({B, nh_q, 1, len}, q.options());
+  at::Tensor out = at::empty({B, nh_q, 1, D}, q.options());
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = row ? L.decode_attention_headsum(&d, q.data_ptr(), weights.data_ptr(), out.data_ptr(), row, ws, ws_bytes, st)
+           : L.decode_attention(&d, q.data_ptr(), weights.data_ptr(), out.data_ptr(), ws, ws_bytes, st);
+  Py_END_ALLOW_THREADS
+  return rc ? none() : pack({weights, out});
+  END_HANDLE_TH_ERRORS
+}
+
+// quantize_pack(data, group_size, bit) -> (code, scale, mn) | None
+PyObject* quantize_pack(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  if (!g_bound || na != 3 || !THPVariable_Check(a[0])) return none();
+  at::Tensor x = THPVariable_Unpack(a[0]);
+  const int64_t group = PyLong_AsLong(a[1]), bit = PyLong_AsLong(a[2]);
+  if (PyErr_Occurred()) {
+    PyErr_Clear();
+    return none();
+  }
+  if (!x.is_cuda() || x.scalar_type() != at::kHalf || x.dim() != 4 || group <= 0 || x.size(3) % group ||
+      (bit != 8 && bit != 4 && bit != 2 && bit != 1))
+    return none();
+  const int64_t B = x.size(0), nh = x.size(1), D = x.size(2), T = x.size(3);
+  const c10::cuda::OptionalCUDAGuard guard(x.device());
+  const bool collapsible = B == 1 || x.stride(0) == nh * x.stride(1);
+  if (!(collapsible && (x.stride(3) == 1 || x.stride(2) == 1)) || D == 1 || T == 1) x = x.contiguous();
+  const auto opt = x.options();
+  at::Tensor code = at::empty({B, nh, D, T * bit / 32}, opt.dtype(at::kInt));
+  at::Tensor scale = at::empty({B, nh, D, T / group}, opt), mn = at::empty({B, nh, D, T / group}, opt);
+  const cudaStream_t st = current_stream(x);
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = L.quantize_pack(x.data_ptr(), B * nh * D, T, D, x.stride(1), x.stride(2), x.stride(3), static_cast<int>(group),
+                       static_cast<int>(bit), code.data_ptr(), scale.data_ptr(), mn.data_ptr(), st);
+  Py_END_ALLOW_THREADS
+  return rc ? none() : pack({code, scale, mn});
+  END_HANDLE_TH_ERRORS
+}
+
+// dequantize_unpack(code, scale, mn, group_size, bit) -> values | None
+PyObject* dequantize_unpack(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  const at::Tensor *code, *scale, *mn;
+  if (!g_bound || na != 5 || !slot(a[0], &code) || !slot(a[1], &scale) || !slot(a[2], &mn) || !code || !scale || !mn)
+    return none();
+  const int64_t group = PyLong_AsLong(a[3]), bit = PyLong_AsLong(a[4]);
+  if (PyErr_Occurred()) {
+    PyErr_Clear();
+    return none();
+  }
+  if (code->dim() != 4 || (bit != 8 && bit != 4 && bit != 2 && bit != 1)) return none();
+  const int64_t B = code->size(0), nh = code->size(1), D = code->size(2), T = code->size(3) * (32 / bit);
+  const c10::cuda::OptionalCUDAGuard guard(code->device());
+  at::Tensor out = at::empty({B, nh, D, T}, code->options().dtype(at::kHalf));
+  const cudaStream_t st = current_stream(*code);
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = L.dequantize_unpack(code->data_ptr(), scale->data_ptr(), mn->data_ptr(), B * nh * D, T, static_cast<int>(group),
+                           static_cast<int>(bit), out.data_ptr(), st);
+  Py_END_ALLOW_THREADS
+  return rc ? none() : THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
+// head_sum(attn_weights [B, nh, 1, L], ring [rows, cap], row) -> True | None
+PyObject* head_sum(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  const at::Tensor *w, *ring;
+  if (!g_bound || na != 3 || !slot(a[0], &w) || !slot(a[1], &ring) || !w || !ring) return none();
+  const int64_t row = PyLong_AsLong(a[2]);
+  if (PyErr_Occurred()) {
+    PyErr_Clear();
+    return none();
+  }
+  if (w->dim() != 4 || w->size(2) != 1 || w->scalar_type() != at::kHalf || ring->scalar_type() != at::kHalf || ring->dim() != 2 ||
+      row < 0 || row >= ring->size(0) || w->size(3) > ring->size(1) || w->device() != ring->device())
+    return none();
+  const c10::cuda::OptionalCUDAGuard guard(w->device());
+  const int64_t len = w->size(3);
+  void* out = static_cast<at::Half*>(ring->data_ptr()) + row * ring->size(1);
+  const cudaStream_t st = current_stream(*w);
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = L.head_sum(w->data_ptr(), static_cast<int>(w->size(0)), static_cast<int>(w->size(1)), len, len, out, st);
+  Py_END_ALLOW_THREADS
+  if (rc) return none();
+  Py_RETURN_TRUE;
+  END_HANDLE_TH_ERRORS
+}
+
+PyObject* build_id(PyObject*, PyObject*) { return PyUnicode_FromString(g_build_stamp + 14); }
+
+template <typename F>
+PyCFunction fast(F f) {
+  return reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f));
+}
+
+PyMethodDef methods[] = {
+    {"bind", bind, METH_VARARGS, "addresses of the library's entry points, and the owner of the decode scratch"},
+    {"build_id", build_id, METH_NOARGS, "hash of the sources this module was compiled from"},
+    {"decode", fast(decode), METH_FASTCALL, nullptr},
+    {"quantize_pack", fast(quantize_pack), METH_FASTCALL, nullptr},
+    {"dequantize_unpack", fast(dequantize_unpack), METH_FASTCALL, nullptr},
+    {"head_sum", fast(head_sum), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&module); }

@@ -7,7 +7,7 @@ of the decode path and are not provided.
 """
 import torch
 
-from .._lib import check, lib, ptr, require_cuda, stream_ptr
+from .._lib import check, host, lib, ptr, require_cuda, stream_ptr
 
 
 def calculate_new_token_range(new_cache: torch.Tensor):
@@ -139,6 +139,9 @@ class last_attn_weights:
             self.weights = torch.zeros(self.last_length, self.max_length, dtype=attn_weights.dtype,
                                        device=attn_weights.device)
         B, nh, q_len, L = attn_weights.shape
+        if q_len == 1 and host.head_sum(attn_weights, self.weights, self.next_line):  # one decode step
+            self.advance(L)
+            return
         w = attn_weights if attn_weights.is_contiguous() else attn_weights.contiguous()
         if w.dtype != torch.float16:
             raise ValueError("attn_weights must be float16")

@@ -7,7 +7,7 @@ from typing import Tuple
 
 import torch
 
-from .._lib import CODEC_NORMAL, CODEC_UNIFORM, HqkvError, check, decode_workspace, lib, ptr, require_cuda, stream_ptr
+from .._lib import CODEC_NORMAL, CODEC_UNIFORM, HqkvError, check, decode_workspace, host, lib, ptr, require_cuda, stream_ptr
 from ._cache import UNIFORM_STRATEGIES, cached_cache_desc
 
 
@@ -33,6 +33,10 @@ def qkv_matmul_hqe_2(q: torch.Tensor, past_key_value: Tuple, attention_mask: tor
     if len(past_key_value) != 42:
         raise ValueError("invalid past_key_value")
     low_codec = CODEC_UNIFORM if quant_strategy == "uniform_group" else CODEC_NORMAL
+    done = host.decode(q, past_key_value, block_size, group_size, low_codec, head_sum_out)
+    if done is not None:
+        return done
+    # what the native path does not take as it is: operands to be made contiguous, and everything that is an error
     require_cuda(q)
     if q.dtype != torch.float16 or q.dim() != 4 or q.shape[2] != 1:
         raise ValueError("q must be float16 of shape [B, nh_q, 1, head_dim]")

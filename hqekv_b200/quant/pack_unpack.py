@@ -10,7 +10,7 @@ Differences a caller can observe:
 import torch
 from scipy.stats import norm
 
-from .._lib import check, lib, ptr, require_cuda, stream_ptr
+from .._lib import check, host, lib, ptr, require_cuda, stream_ptr
 
 n_bits_range = [8, 4, 2, 1]
 # Gaussian-quantile codebooks of the "normal" codec (quant/pack_unpack.py:6-14); kept because other
@@ -34,6 +34,9 @@ def uniform_group_quantize_pack_last_dim(data: torch.Tensor, group_size: int, bi
     """quant/pack_unpack.py:156-193.  data fp16 [B, nh, D, T] (any strides; a ``transpose(2, 3)``
     view of token-major K is read in place) -> (code int32 [B,nh,D,T*bit/32], scale fp16
     [B,nh,D,T/group], mn fp16 [B,nh,D,T/group])."""
+    done = host.quantize_pack(data, group_size, bit)
+    if done is not None:
+        return done
     _check_bits(bit)
     require_cuda(data)
     if data.dtype != torch.float16 or data.dim() != 4:
@@ -58,6 +61,9 @@ def uniform_group_quantize_pack_last_dim(data: torch.Tensor, group_size: int, bi
 def uniform_group_dequantize_unpack_last_dim(code: torch.Tensor, scale: torch.Tensor, mn: torch.Tensor,
                                              group_size: int, bit: int):
     """quant/pack_unpack.py:316-333: x = half(half(code*scale) + mn) as fp16 [B, nh, D, T]."""
+    done = host.dequantize_unpack(code, scale, mn, group_size, bit)
+    if done is not None:
+        return done
     _check_bits(bit)
     require_cuda(code, scale, mn)
     B, nh, D, T_d = code.shape
