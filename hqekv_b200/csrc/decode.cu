@@ -1,8 +1,8 @@
 // Fused mixed-precision decode attention over the tiered KV cache (sm_100a).
 //
 // Two launches per call:
-//   k_pass : logits[h, pos] = scale * q_h . K^_pos for every tier (8/4/2/1-bit packed, fp16 tier,
-//            fp16 residual), written to an fp32 scratch row at the tokens' logical positions,
+//   k_pass : logits[pos][h] = scale * q_h . K^_pos for every tier (8/4/2/1-bit packed, fp16 tier,
+//            fp16 residual), written to an fp32 scratch at the tokens' logical positions,
 //            plus one (max, sum-exp) pair per CTA and head.
 //   v_pass : every CTA first folds the k_pass pairs into the global (max, sum) of its heads; each
 //            warp then writes the normalised probabilities of its own tokens and accumulates
@@ -10,7 +10,7 @@
 //            accumulators, and the last CTA of each (batch, kv head) normalises and writes fp16.
 //
 // The roofline is HBM: every packed word, scale and zero is read exactly once per call and is
-// shared by all query heads of its kv head (GQA).  At 2-4 bits there are 1.6-2.7 codes per byte;
+// shared by the query heads of its kv head (GQA).  At 2-4 bits there are 1.6-2.7 codes per byte;
 // four query heads need four FMAs per code, more than the FP32 pipes can issue at HBM speed, so the
 // dot products run on the tensor pipe (mma.sync m16n8k16, fp32 accumulation).  Tiles of codes are
 // staged in shared memory with 16-byte cp.async and read back with ldmatrix.trans, which delivers the
@@ -18,6 +18,9 @@
 // AND per pair) and the scale is folded into the B operand, carried exactly as hi + lo.
 // Both kernels are chained with programmatic dependent launch: whatever a kernel needs only from the
 // cache is requested before it waits for the kernel ahead of it.
+//
+// A CTA serves up to four query heads.  With eight per kv head the kv head is served by two CTAs ("virtual" kv heads
+// of four query heads each, neighbours in the grid, so that the second read of the tile hits L2).
 #include <math.h>
 #include <string.h>
 
@@ -28,7 +31,8 @@ namespace hqkv {
 HQKV_DEFINE_CHECK_COUNTER
 
 constexpr int D = 128;           // head dim
-constexpr int MAX_REP = 8;       // query heads per kv head (n of the m16n8k16 tile)
+constexpr int MAX_REP = 8;       // query heads per kv head
+constexpr int MAX_R4 = 4;        // query heads per CTA
 
 struct TierDev {
   const void* k_data;
@@ -42,27 +46,32 @@ struct TierDev {
   int n_k, n_v;
   int bits;
   int normal;  // 1-bit tier in the Gaussian-codebook codec: value = std * (+-C) + mean, scale slots = std, zero = mean
-  int k_chunk0, k_chunk_tokens;  // first chunk id of this tier in the k_pass grid, tokens per chunk
-  int v_chunk0, v_chunk_tokens;
+  int k_unit0, v_unit0;      // where the tier's units start in the list of a plane's units (K pass, V pass)
+  int k_cta0, v_cta0;        // ... and its CTAs in the list of the plane's, where no CTA has units of two tiers
 };
 
 struct DecodeParams {
   TierDev tier[HQKV_NUM_TIERS + 1];  // [5] = fp16 residual window (token-major K and V)
-  int B, H, nh_q, rep, rep_shift, L;
+  int B, H, nh_q, L;
+  int halves;              // virtual kv heads per kv head: 2 with eight query heads per kv head, else 1
+  int r4, r4_shift;        // query heads per virtual kv head: 1, 2, 4
   int gk_shift, gv_shift;
-  int nk_chunks, nv_chunks;
+  int nk_ctas, nv_ctas;    // CTAs per plane = grid rows
+  // Units per CTA.  more >= 0: equal shares, the first `more` CTAs take one more; -1: no CTA has units of two tiers (in
+  // the K pass 8-bit units, which are half as long, count half).
+  int k_per, k_more, v_per, v_more;
   float scale;
   const __half* q;
   const __half* mask;      // additive mask on the logits (null: none); element (b, head, pos) at b*bstride + head*hstride + pos
   long long mask_bstride, mask_hstride;
   const __half* probs_in;  // V pass on caller-supplied weights [B*nh_q][L] (null: softmax of the scratch logits)
   __half* head_sum;        // [L] sum of the probabilities over batch and heads, written by the V pass (null: not wanted)
-  unsigned* hs_count;      // [nv_chunks] arrival counters of that sum
+  unsigned* hs_count;      // [nv_ctas] arrival counters of that sum
   __half* weights;
   __half* out;
-  float* logits;   // [B*nh_q][L]
-  float2* k_part;  // [B*H][nk_chunks][MAX_REP]
-  double* v_acc;   // [B*H][rep][D] output accumulators: cleared by the K pass, summed into by the V pass
+  float* logits;   // [B][virtual kv head][L][r4]
+  float2* k_part;  // [B][virtual kv head][r4][nk_ctas]
+  double* v_acc;   // [B][nh_q][D] output accumulators: cleared by the K pass, summed into by the V pass
   __half* peer_out[HQKV_MAX_PEERS];  // copies of `out` in other GPUs' memory (kv-head sharding), n_peers used
   int n_peers;
   int peer_flagged;  // 1: peer_out are flagged 8-byte entries {two fp16 values, call number}, see peer_unpack_kernel
@@ -74,13 +83,57 @@ struct DecodeParams {
   unsigned* counters;  // [B*H]
 };
 
+// The tokens of a (batch, virtual kv head) plane are a list of UNITS - 256 tokens of one tier (128 at 8 bits, 64 of the
+// fp16 tier and of the residual window), tiers in order - and its CTAs take consecutive shares of it.
+__host__ __device__ constexpr int unit_tokens(int bits) { return bits == 16 ? 64 : bits == 8 ? 128 : 256; }
+// This CTA's tokens [t0, t1) of tier ti; false: none.
+template <bool V>
+__device__ __forceinline__ bool share_of(const DecodeParams& P, int ti, int bits, int& t0, int& t1) {
+  const TierDev& T = P.tier[ti];
+  const int i = blockIdx.y, per = V ? P.v_per : P.k_per, more = V ? P.v_more : P.k_more;
+  const int u0 = i * per + min(i, more) - (V ? T.v_unit0 : T.k_unit0), u1 = u0 + per + (i < more ? 1 : 0);
+  t0 = max(u0, 0) * unit_tokens(bits);
+  t1 = min(u1 * unit_tokens(bits), V ? T.n_v : T.n_k);
+  return t0 < t1;
+}
+// The same where no CTA has units of two tiers: the tier, too.
+template <bool V>
+__device__ __forceinline__ int only_share(const DecodeParams& P, int& t0, int& t1) {
+  const int i = blockIdx.y;
+  int ti = 0;
+#pragma unroll
+  for (int t = 1; t <= HQKV_NUM_TIERS; ++t)
+    if (i >= (V ? P.tier[t].v_cta0 : P.tier[t].k_cta0)) ti = t;
+  const TierDev& T = P.tier[ti];
+  const int n = (V ? P.v_per : P.k_per * (T.bits == 8 ? 2 : 1)) * unit_tokens(T.bits);
+  t0 = (i - (V ? T.v_cta0 : T.k_cta0)) * n;
+  t1 = min(t0 + n, V ? T.n_v : T.n_k);
+  return ti;
+}
+
+// Grid: x = virtual kv head, y = share of the plane's units, z = batch.
+struct Where {
+  int b, vh;   // batch, virtual kv head
+  int bh;      // (batch, kv head) plane of the cache
+  int bvh;     // (batch, virtual kv head) plane of the scratch
+  int h0;      // first query head
+};
+__device__ __forceinline__ Where where(const DecodeParams& P) {
+  Where w;
+  w.b = blockIdx.z;
+  w.vh = blockIdx.x;
+  w.bh = w.b * P.H + (P.halves == 2 ? w.vh >> 1 : w.vh);
+  w.bvh = w.b * gridDim.x + w.vh;
+  w.h0 = w.vh * P.r4;
+  return w;
+}
 
 // ------------------------------------------------------------------------------------------------
 // fragments
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                          uint32_t b0, uint32_t b1) {
-  asm volatile(
+  asm(
       "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
@@ -88,6 +141,18 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
 
 __device__ __forceinline__ uint32_t h2_as_u32(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 __device__ __forceinline__ __half2 u32_as_h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
+__device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) { return h2_as_u32(__hmul2(u32_as_h2(a), u32_as_h2(b))); }
+__device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
+  return h2_as_u32(__hfma2(u32_as_h2(a), u32_as_h2(b), u32_as_h2(c)));
+}
+// a*b - c, with c = fp16(a*b): the exact remainder
+__device__ __forceinline__ uint32_t h2_rem(uint32_t a, uint32_t b, uint32_t c) {
+  return h2_as_u32(__hfma2(u32_as_h2(a), u32_as_h2(b), __hneg2(u32_as_h2(c))));
+}
+// 16-bit halves of two words -> one half2 register: low halves, high halves
+__device__ __forceinline__ uint32_t pack_lo16(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x5410); }
+__device__ __forceinline__ uint32_t pack_hi16(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); }
+__device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) { return h2_as_u32(__floats2half2_rn(lo, hi)); }
 
 // Streaming loads: the cache is read once per call, keep it out of L1.
 __device__ __forceinline__ uint2 ld_stream(const uint2* p) {
@@ -103,68 +168,65 @@ __device__ __forceinline__ uint4 ld_stream(const uint4* p) {
   return v;
 }
 
-// Storage formats.  A "word" is what one thread loads for one (row, column) slot; it holds FPI
-// values of one row.  SUB = independently decoded sub-units of a word (bytes of a packed word,
-// 32-bit lanes of a uint4 of halfs), CPS = values per sub-unit.
-template <int BITS>
-struct Fmt;
-template <>
-struct Fmt<16> {
-  using word_t = uint4;  // eight halfs
-  static constexpr int FPI = 8, SUB = 4, CPS = 2;
-};
-
-// Decode sub-unit `sub` of the words wa (first row of the pair) and wb (second row) into CPS
-// half2 values (value of row a in the low half, row b in the high half): v = code*scale + zero
-// with one fp16 rounding; `sz` packs the scales of the two rows, `zz` their zeros.
-template <int BITS>
-struct Decode;
-
-template <>
-struct Decode<16> {
-  template <int SUBI>
-  static __device__ __forceinline__ void run(const uint4& wa, const uint4& wb, __half2, __half2, uint32_t (&out)[2]) {
-    const uint32_t a = SUBI == 0 ? wa.x : SUBI == 1 ? wa.y : SUBI == 2 ? wa.z : wa.w;
-    const uint32_t b = SUBI == 0 ? wb.x : SUBI == 1 ? wb.y : SUBI == 2 ? wb.z : wb.w;
-    out[0] = __byte_perm(a, b, 0x5410);
-    out[1] = __byte_perm(a, b, 0x7632);
-  }
-};
-
-// One 16-deep contraction step over all M-tiles of a thread's slots.
-//   w[p][r]: word of row-pair member p (0,1 -> fragment columns 2tig,2tig+1; 2,3 -> +8,+9) and row
-//            slot r (0 -> fragment row g, 1 -> row g+8)
-//   sz/zz[q][r]: scales/zeros of pair q (0: p=0,1; 1: p=2,3) for slot r
-// M-tile index of sub-unit s, value k: s*CPS + k.
-template <int BITS, int SUBI, int NM>
-__device__ __forceinline__ void mma_sub(float (&acc)[NM][4], const typename Fmt<BITS>::word_t (&w)[4][2],
-                                        const __half2 (&sz)[2][2], const __half2 (&zz)[2][2], uint32_t b0,
-                                        uint32_t b1) {
-  constexpr int CPS = Fmt<BITS>::CPS;
-  uint32_t a0[CPS], a1[CPS], a2[CPS], a3[CPS];
-  Decode<BITS>::template run<SUBI>(w[0][0], w[1][0], sz[0][0], zz[0][0], a0);
-  Decode<BITS>::template run<SUBI>(w[0][1], w[1][1], sz[0][1], zz[0][1], a1);
-  Decode<BITS>::template run<SUBI>(w[2][0], w[3][0], sz[1][0], zz[1][0], a2);
-  Decode<BITS>::template run<SUBI>(w[2][1], w[3][1], sz[1][1], zz[1][1], a3);
-#pragma unroll
-  for (int k = 0; k < CPS; ++k) mma16816(acc[SUBI * CPS + k], a0[k], a1[k], a2[k], a3[k], b0, b1);
+// shared memory by 32-bit address: loads with compile-time offsets, no generic-address arithmetic
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ uint32_t lds16(uint32_t a) {
+  unsigned short v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void sts16(uint32_t a, uint32_t v) {
+  asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"(static_cast<unsigned short>(v)) : "memory");
+}
+__device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ void sts64(uint32_t a, uint32_t x, uint32_t y) {
+  asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(a), "r"(x), "r"(y) : "memory");
 }
 
-template <int BITS, int NM>
-__device__ __forceinline__ void mma_words(float (&acc)[NM][4], const typename Fmt<BITS>::word_t (&w)[4][2],
-                                          const __half2 (&sz)[2][2], const __half2 (&zz)[2][2], uint32_t b0,
-                                          uint32_t b1) {
-  constexpr int SUB = Fmt<BITS>::SUB;
-  mma_sub<BITS, 0, NM>(acc, w, sz, zz, b0, b1);
-  mma_sub<BITS, 1, NM>(acc, w, sz, zz, b0, b1);
-  mma_sub<BITS, 2, NM>(acc, w, sz, zz, b0, b1);
-  mma_sub<BITS, 3, NM>(acc, w, sz, zz, b0, b1);
-  if constexpr (SUB == 8) {
-    mma_sub<BITS, 4, NM>(acc, w, sz, zz, b0, b1);
-    mma_sub<BITS, 5, NM>(acc, w, sz, zz, b0, b1);
-    mma_sub<BITS, 6, NM>(acc, w, sz, zz, b0, b1);
-    mma_sub<BITS, 7, NM>(acc, w, sz, zz, b0, b1);
-  }
+// global -> shared copies without a register round trip; completion = wait_group + barrier
+__device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_8(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// four 8x8 matrices of 16-bit elements, transposed: lane (g, tig) gets elements (row 2*tig, col g) and
+// (row 2*tig+1, col g) of matrix i in r[i]; lanes 8*i .. 8*i+7 supply the row addresses of matrix i
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t row_addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(row_addr) : "memory");
+}
+
+// the same without the transposition: lane (g, tig) gets elements 2*tig, 2*tig+1 of row g
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t row_addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(row_addr) : "memory");
 }
 
 // 2^x on the special-function unit (about 2 ulp; 2^-inf = 0)
@@ -173,765 +235,813 @@ __device__ __forceinline__ float fast_exp2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+constexpr float LOG2E = 1.4426950408889634f;
 
 __device__ __forceinline__ void softmax_merge(float& m, float& l, float m2, float l2) {
   const float mx = fmaxf(m, m2);
   if (mx == -INFINITY) return;  // both empty
-  l = l * fast_exp2((m - mx) * 1.4426950408889634f) + l2 * fast_exp2((m2 - mx) * 1.4426950408889634f);
+  l = l * fast_exp2((m - mx) * LOG2E) + l2 * fast_exp2((m2 - mx) * LOG2E);
   m = mx;
 }
-
 
 // ------------------------------------------------------------------------------------------------
 // k_pass
 // ------------------------------------------------------------------------------------------------
-// Quantised K tier: rows = channels, packed words along tokens.  Every warp of a CTA owns one TILE:
-// all 128 channel rows x 64 bytes of codes (32 bytes at 2 bits), i.e. 64 / 128 / 128 tokens at
-// 8 / 4 / 2 bits, plus the tile's logical positions; the CTA shares the scale / zero rows of its 256
-// or 512 tokens and q.  All of it is copied global -> shared with 16-byte cp.async as the first
-// action (no registers are tied up, ~45 KB per CTA are in flight at once) and each warp then works
-// out of shared memory in sub-spans of 64 tokens.  Wide copies in, ldmatrix out: the L1 data pipe
-// moves 128 bytes per wavefront both ways.  (Per-lane loads of the 1-4 bytes a thread needs - from
-// global or from shared memory - saturate that pipe at a quarter of the HBM bandwidth.)
+// Quantised K tier: rows = channels, packed words along tokens.  A CTA of four warps walks a run of CHUNKS of one tier
+// and (batch, kv head): 128 channel rows x 128 bytes of codes at 8 / 4 bits (128 / 256 tokens), x 64 / 32 bytes at 2 / 1
+// bits (256 tokens).  Codes go global -> shared with 16-byte cp.async into one of two buffers (the next chunk's while
+// this one is worked on); each warp works on its quarter of the tokens out of shared memory.  Wide copies in,
+// ldmatrix out: the L1 data pipe moves 128 bytes per wavefront both ways.  (Per-lane loads of the 1-4 bytes a
+// thread needs - from global or from shared memory - saturate that pipe at a quarter of the HBM bandwidth.)
 //
 // ldmatrix.trans over 8 channel rows x 16 bytes hands lane (g, tig) the 16-bit block g of channels
 // 2*tig and 2*tig+1 in one register: exactly the two K-neighbours of an m16n8k16 A fragment for the
-// tokens of block g (2 / 4 / 8 tokens at 8 / 4 / 2 bits).  What keeps the instruction count low:
+// tokens of block g (2 / 4 / 8 tokens at 8 / 4 / 2 bits).  What bounds the kernel below 8 bits is the number of
+// instructions a warp issues per token, so everything here serves that number:
 //  * the integer codes enter the tensor pipe as they are: a masked field at bit k < 10 of a 16-bit
 //    lane IS the fp16 subnormal code * 2^(k-24), exactly, so one AND per pair of codes builds an A
 //    fragment register; the power of two comes back out in the epilogue;
-//  * the scale lives in the B operand: logit = sum_c (q_c * scale_c) * code_c + sum_c q_c * zero_c.
-//    A sub-span holds two 32-token scale groups; B columns 0-3 hold q*scale of the first group for
-//    four query heads and columns 4-7 that of the second, and each fragment row keeps the half of
-//    its accumulators whose group matches.  With eight query heads per kv head the warp walks its
-//    tile once per half of the heads;
-//  * q*scale (11 x 11 significant bits) is carried EXACTLY as hi = fp16(q*scale) and
-//    lo = q*scale - hi, two MMAs into the same fp32 accumulator.  (One fp16 rounding of it - or of
-//    the dequantised K value - costs ~2e-3 on the attention output with x10 outlier channels.)
-//  * the zero point enters through Zq[group][head] = sum_c zero_c * q_c, one small MMA per tile;
-//  * every lane scatters its own logits from registers and keeps a running (max, sum-exp).
-constexpr int K_MIN_CTAS = 4;  // CTAs per SM the K pass is compiled for
+//  * the scale lives in the B operand: logit = sum_c (q_c * scale_c) * code_c + sum_c q_c * zero_c;
+//  * q*scale (11 x 11 significant bits) is carried EXACTLY as hi = fp16(q*scale) and lo = q*scale - hi.  (One fp16
+//    rounding of it - or of the dequantised K value - costs ~2e-3 on the attention output with x10 outlier
+//    channels.)  At 8 and 4 bits the 16 rows of an M-tile are tokens of ONE scale group of 32, and the eight columns
+//    of the B operand are (head 0 hi, head 0 lo, head 1 hi, ...): one MMA does both and a lane adds the two
+//    accumulators of its head.  A 16-byte piece of 2-bit codes spans two groups: there the columns are (head 0 first
+//    group, head 0 second group, ...), a row keeps the column of its own group, and hi and lo are two MMAs;
+//  * a lane's accumulators all belong to query head tig, so logits, softmax statistics and stores need no exchange;
+//  * the scales of two 16-channel steps are ONE 16-byte shared-memory read: the scale rows are transposed to
+//    [group][channel] in shared memory, channels ordered as a lane's B fragment wants them.  They are fetched for 512
+//    tokens at a time, a row's (up to) 48 bytes by neighbouring lanes: one 16-byte piece per lane and row cost the L1
+//    tag stage a lookup each, more than the codes did;
+//  * the zero point enters through Zq[group][head] = sum_c zero_c * q_c: every warp takes the 32 channels it has
+//    transposed itself for all sixteen groups of those 512 tokens (two MMAs), the four partial sums meet in shared memory;
+//  * blocks of tokens stay together in a tier, so 32 stored tokens have 32 consecutive positions: checked with one
+//    vote, after which the logits are stored at constant offsets.  (Any other list takes the general store.)
+constexpr int K_MIN_CTAS = 4;  // CTAs per SM the K pass is compiled for (128 registers; shared memory allows four)
 constexpr int KWARPS = 4;
 constexpr int KTHREADS = KWARPS * 32;
-constexpr int K_SPAN = 64;                   // tokens per sub-span: four M-tiles of 16
+constexpr int K_SPAN = 64;                   // fp16 tier: tokens at a time
 constexpr int K_SLOT = 4;                    // fp16 tier: tokens per 8-byte slot
-constexpr int K_TILE_BYTES = D * 64;         // codes of one tile
-constexpr int K_MAX_TT = 128;                // tokens per tile at most
-constexpr int K_CHUNK_GROUPS = KWARPS * K_MAX_TT / 32;  // scale groups per CTA at most (group size 32)
-constexpr int K_RAW_HALFS = K_CHUNK_GROUPS + 8;         // staged halfs per channel row: three aligned 16-byte pieces
-constexpr int K_TROW = MAX_REP + 1;          // floats per token row of the logit tile (odd: no bank conflicts)
-constexpr float LOG2E = 1.4426950408889634f;
+constexpr int K_BLOCK = 512;                 // tokens whose scales are fetched at a time
+constexpr int K_GROUPS = K_BLOCK / 32;       // scale groups of those at most
+constexpr int K_RAW = 48;                    // bytes of a raw scale row: three aligned 16-byte pieces cover 16 halfs at any alignment
+constexpr int K_SROW = D * 2;                // bytes of a transposed scale row
+constexpr int K_ZROW = 80;                   // bytes of a warp's transposed zero row (32 channels; ldmatrix rows in different banks)
+constexpr int K_TROW = MAX_R4 + 1;           // floats per token row of the logit tile (odd: no bank conflicts)
+constexpr int K_CODES = D * 128;             // bytes of a code buffer
 
 template <int BITS>
 struct KTile {
-  static constexpr int PITCH = BITS == 1 ? 16 : BITS == 2 ? 32 : 64;  // bytes per channel row
-  static constexpr int TOKENS = PITCH * 8 / BITS;         // 64, 128, 128, 128 at 8, 4, 2, 1 bits
-  static constexpr int NSUB = TOKENS / K_SPAN;            // sub-spans: 1, 2, 2, 2
-  static constexpr int TPC = 128 / BITS;                  // tokens per 16-byte piece: 16, 32, 64, 128
-  static constexpr int CPS = BITS == 1 ? 1 : K_SPAN / TPC;  // pieces of a row per sub-span: 4, 2, 1 (1 bit: half a piece)
-  // byte offset of 16-byte piece c of a channel row.  The piece index is XORed with row bits so that
-  // the eight rows of an ldmatrix (same logical piece) and the pieces a cp.async instruction writes
-  // both spread over all banks.
-  static __device__ __forceinline__ uint32_t offset(uint32_t row, uint32_t c) {
-    if constexpr (PITCH == 64) {
-      return row * 64u + ((c ^ ((row >> 1) & 3u)) << 4);
-    } else if constexpr (PITCH == 32) {
-      return row * 32u + ((c ^ ((row >> 2) & 1u)) << 4);
-    } else {
-      return row * 16u;  // 1 bit: read with 2-byte loads, see k_tile_compute
-    }
-  }
+  static constexpr int PITCH = BITS == 1 ? 40 : BITS == 2 ? 64 : 128;  // bytes per channel row in shared memory
+  static constexpr int TOKENS = BITS == 8 ? 128 : 256;                 // tokens per chunk
+  static constexpr int WTOK = TOKENS / KWARPS;                         // tokens per warp: 32, 64, 64, 64
+  static constexpr int HALVES = WTOK / 32;                             // 32-token units per warp
+  static constexpr bool ONE_GROUP = BITS >= 4;                         // an M-tile's rows are tokens of one unit
+  static constexpr int NX = WTOK / 8;                                  // tokens per lane: 4, 8, 8, 8
 };
-
-// global -> shared copies without a register round trip; completion = wait_group + barrier
-__device__ __forceinline__ void cp_async_4(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-               "l"(src));
-}
-__device__ __forceinline__ void cp_async_8(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-               "l"(src));
-}
-__device__ __forceinline__ void cp_async_16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-               "l"(src));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// four 8x8 matrices of 16-bit elements, transposed: lane (g, tig) gets elements (row 2*tig, col g) and
-// (row 2*tig+1, col g) of matrix i in r[i]; lanes 8*i .. 8*i+7 supply the row addresses of matrix i
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* row_ptr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(row_ptr))));
-}
-
-struct KWarpShared {
-  union {
-    unsigned char codes[K_TILE_BYTES];
-    float tile[64 * K_TROW];  // fp16 tier / residual: logits [token][head]
-  } u;
-  int64_t idx[K_MAX_TT];      // logical positions of the tile's tokens
-  float zq[4][MAX_REP];       // sum_c zero*q per group of the tile and head
-};
+static_assert(KTile<8>::TOKENS == unit_tokens(8) && KTile<4>::TOKENS == unit_tokens(4) && KTile<1>::TOKENS == unit_tokens(1), "a unit is a chunk");
 
 struct KShared {
-  // B fragments of q per 16-channel step and lane: channels 16*kt + 2*tig + (0,1 | 8,9).  fp16 tier /
-  // residual CTAs: [0] with column n = head n.  Quantised CTAs: [hh] with column n = head
-  // 4*hh + (n & 3) (columns 4-7 repeat 0-3).
-  uint2 qb[2][8][32];
-  // scale / zero rows of the CTA's tokens as they lie in memory: channel c, three aligned 16-byte
-  // pieces starting at or before the chunk's first group
-  __half s[D][K_RAW_HALFS];
-  __half z[D][K_RAW_HALFS];
-  float red_m[KWARPS][MAX_REP], red_l[KWARPS][MAX_REP];
-  KWarpShared w[KWARPS];
+  union {
+    unsigned char codes[2][K_CODES];
+    float tile[KWARPS][K_SPAN * K_TROW];  // fp16 tier / residual: logits [token][head] of each warp
+  } u;
+  union {
+    unsigned char raw[2][KWARPS][32 * K_RAW];  // scale and zero rows as in memory, 32 channels per warp
+    struct {
+      float m[KWARPS][MAX_R4], l[KWARPS][MAX_R4];  // softmax pairs of the warps, after the last chunk
+    } red;
+  } v;
+  unsigned char s[K_GROUPS * K_SROW];          // [group][k_order(channel)]
+  unsigned char z[KWARPS][K_GROUPS * K_ZROW];  // [group][channel of the warp]
+  float zq[K_GROUPS][MAX_R4][KWARPS];          // the warps' partial Zq
+  // B fragments of q per pair of 16-channel steps and lane: channels 16*kt + 2*tig + (0,1 | 8,9) of the even step, then
+  // of the odd one; column n = g is head n >> 1
+  uint4 q[4][32];
 };
+constexpr int K_RAW_PLANE = KWARPS * 32 * K_RAW;
 
-// Request the scale / zero rows of the CTA's chunk: thread t copies channel t.  The chunk's groups
-// [g0c, g0c + ngc) of a channel are 2*ngc bytes at any 2-byte alignment; the (up to) three aligned
-// 16-byte pieces that cover them go to shared memory as they are, so group gamma of channel c is
-// half ((c*G + g0c) & 7) + gamma of row c.  (The planes hold B*H*128*G halfs, a multiple of 8, and
-// start 16-byte aligned, so every aligned piece that begins inside a plane also ends inside it.)
-__device__ __forceinline__ void k_scales_request(const DecodeParams& P, const TierDev& T, KShared& sh, int bh, int g0c,
-                                                 int ngc) {
-  const int ch = threadIdx.x;  // KTHREADS == D
-  const int G = T.n_k >> P.gk_shift;
-  const int64_t e0 = (static_cast<int64_t>(bh) * D + ch) * G + g0c;
-  const int64_t a = e0 & ~static_cast<int64_t>(7);
-#pragma unroll
-  for (int p = 0; p < K_RAW_HALFS / 8; ++p)
-    if (a + 8 * p < e0 + ngc) {
-      cp_async_16(&sh.s[ch][8 * p], T.k_scale + a + 8 * p);
-      cp_async_16(&sh.z[ch][8 * p], T.k_zero + a + 8 * p);
-    }
+// Position of a channel in a transposed scale row: per pair of 16-channel steps and lane quarter tig the eight channels
+// of the lane's two B fragments are neighbours, {2tig, +1, +8, +9} of the even step, then of the odd one.
+__device__ __forceinline__ int k_order(int ch) {
+  return (ch & ~31) | ((ch & 6) << 2) | ((ch & 16) >> 2) | ((ch & 8) >> 2) | (ch & 1);
 }
-static_assert(KTHREADS == D, "one thread per channel row");
 
-// Request a tile: four commit groups, the codes of channel rows 0-31 (with the positions), 32-63,
-// 64-95, 96-127 (two 16-channel steps each).  ntok = valid tokens of the tile (a multiple of 32).
-template <int BITS>
-__device__ __forceinline__ void k_tile_request(const TierDev& T, KWarpShared& ws, int bh, int tile_t0, int ntok) {
-  using TL = KTile<BITS>;
+// halfs off .. off+15 of the 24 in (a, b, c)
+__device__ __forceinline__ void align_halfs(const uint4& a, const uint4& b, const uint4& c, int off, uint32_t (&o)[8]) {
+  uint32_t w[12] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
+#pragma unroll
+  for (int i = 0; i < 10; ++i) w[i] = (off & 4) ? w[i + 2] : w[i];
+#pragma unroll
+  for (int i = 0; i < 9; ++i) w[i] = (off & 2) ? w[i + 1] : w[i];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) o[i] = __funnelshift_r(w[i], w[i + 1], 16 * (off & 1));
+}
+
+// Scale / zero rows of up to 512 tokens, warp = 32 channels.  The groups [g0, g0 + ng) of a channel are ng halfs at any
+// 2-byte alignment; the (up to) three aligned 16-byte pieces that cover them are copied as they are and shifted into
+// place on the way to the transposed rows.  (The planes hold B*H*128*G halfs, a multiple of 8, and start 16-byte
+// aligned, so every aligned piece that begins inside a plane also ends inside it.)
+struct KScales {
+  int64_t row0;      // index of half 0 of the warp's first channel row
+  int G;             // groups per row
+  uint32_t raw, s_at, z_at, z_row;
+};
+__device__ __forceinline__ void k_scales_request(const TierDev& T, const KScales& k, int g0, int ng) {
   const int lane = threadIdx.x & 31;
-  const int n = T.n_k;
 #pragma unroll
-  for (int j = 0; j < TL::TOKENS / 32; ++j) {
-    const int t = lane + 32 * j;
-    if (t < ntok) cp_async_8(&ws.idx[t], T.k_idx + tile_t0 + t);
-  }
-  const int64_t row_bytes = static_cast<int64_t>(n) * BITS / 8;
-  const unsigned char* src = reinterpret_cast<const unsigned char*>(T.k_data) + static_cast<int64_t>(bh) * D * row_bytes +
-                             static_cast<int64_t>(tile_t0) * BITS / 8;
-  const int valid_bytes = ntok * BITS / 8;  // per row: a multiple of 8 (of 4 at 1 bit)
-  if constexpr (BITS == 1) {
-    // 16 bytes per row at 4-byte alignment: four 4-byte pieces; a copy instruction moves 8 rows
-#pragma unroll
-    for (int quarter = 0; quarter < 4; ++quarter) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int row = quarter * 32 + i * 8 + (lane >> 2), c4 = 4 * (lane & 3);
-        if (c4 < valid_bytes) cp_async_4(ws.u.codes + row * 16 + c4, src + row * row_bytes + c4);
-      }
-      cp_async_commit();
+  for (int i = 0; i < 3; ++i) {
+    const int id = i * 32 + lane, row = id / 3, piece = id - 3 * row;
+    const int64_t e = k.row0 + static_cast<int64_t>(row) * k.G + g0;
+    if (8 * piece < static_cast<int>(e & 7) + ng) {
+      const int64_t a = (e & ~static_cast<int64_t>(7)) + 8 * piece;
+      cp_async_16(k.raw + id * 16, T.k_scale + a);
+      cp_async_16(k.raw + K_RAW_PLANE + id * 16, T.k_zero + a);
     }
+  }
+}
+__device__ __forceinline__ void k_scales_transpose(const KScales& k, int g0, int ng) {
+  const int lane = threadIdx.x & 31;
+  const int off = static_cast<int>((k.row0 + static_cast<int64_t>(lane) * k.G + g0) & 7);
+  const uint32_t src = k.raw + lane * K_RAW;
+#pragma unroll
+  for (int plane = 0; plane < 2; ++plane) {
+    const uint32_t p = src + plane * (K_RAW_PLANE);
+    const uint4 a = lds128(p), b = lds128(p + 16), c = lds128(p + 32);
+    uint32_t o[8];
+    align_halfs(a, b, c, off, o);
+    const uint32_t at = plane ? k.z_at : k.s_at;
+    const int pitch = plane ? K_ZROW : K_SROW;
+#pragma unroll
+    for (int i = 0; i < K_GROUPS / 2; ++i)
+      if (2 * i < ng) {  // (an odd count stores one row more: nobody reads it)
+        sts16(at + (2 * i) * pitch, o[i] & 0xFFFFu);
+        sts16(at + (2 * i + 1) * pitch, o[i] >> 16);
+      }
+  }
+}
+// Partial Zq of the warp's 32 channels: rows = groups.  q = the B fragments of those channels.
+__device__ __forceinline__ void k_zero_term(const KScales& k, const uint4& q, float (*zq)[MAX_R4][KWARPS], uint32_t other_rows, bool normal) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  uint32_t r[4];
+  ldmatrix_x4(r, k.z_row);        // matrices (groups 0-7, channels 0-7), (8-15, 0-7), (0-7, 8-15), (8-15, 8-15)
+  mma16816(acc, r[0], r[1], r[2], r[3], q.x, q.y);
+  ldmatrix_x4(r, k.z_row + 32);
+  mma16816(acc, r[0], r[1], r[2], r[3], q.z, q.w);
+  if (normal) {  // a value is std * C * (2 code - 1) + mean: the code-free term is sum_c (mean - C std) q
+    float n[4] = {0.f, 0.f, 0.f, 0.f};
+    const uint32_t even = other_rows, odd = other_rows + 8;  // this lane's channels in the transposed scale rows
+    uint2 x = lds64(even), y = lds64(even + 8 * K_SROW);
+    mma16816(n, x.x, y.x, x.y, y.y, q.x, q.y);
+    x = lds64(odd), y = lds64(odd + 8 * K_SROW);
+    mma16816(n, x.x, y.x, x.y, y.y, q.z, q.w);
+    acc[0] = fmaf(-HQKV_NORMAL1_CENTER, n[0], acc[0]);
+    acc[2] = fmaf(-HQKV_NORMAL1_CENTER, n[2], acc[2]);
+  }
+  zq[g][tig][threadIdx.x >> 5] = acc[0];
+  zq[g + 8][tig][threadIdx.x >> 5] = acc[2];
+}
+
+// Request the codes of a chunk: src / dst = this thread's first piece, valid = bytes per row (a multiple of 32, 16, 8, 4
+// at 8, 4, 2, 1 bits).  The rows of the 2-bit tier are only 8-byte aligned unless its token count is a multiple of 64
+// (wide2), those of the 1-bit tier 4-byte.
+// The piece index is XORed with row bits so that the eight rows of an ldmatrix (same logical piece) and the pieces a
+// cp.async instruction writes both spread over all banks.
+template <int BITS>
+struct KCopy {
+  const unsigned char* src;
+  uint32_t dst;
+  uint32_t step;   // bytes of memory between this thread's rows
+  int first;       // first byte of the row that this thread copies
+};
+template <int BITS>
+__device__ __forceinline__ KCopy<BITS> k_copy_init(const TierDev& T, int bh, int t0, uint32_t codes, bool wide2) {
+  using TL = KTile<BITS>;
+  const int tid = threadIdx.x;
+  const int64_t row_bytes = static_cast<int64_t>(T.n_k) * BITS / 8;
+  KCopy<BITS> k;
+  int c, r0, bytes, rows;
+  if (BITS == 2 && wide2) {
+    c = tid & 3, r0 = tid >> 2, bytes = 16, rows = 32;
+    k.dst = codes + r0 * 64 + ((c ^ ((r0 >> 1) & 3)) << 4);
+  } else {
+    c = tid & 7, r0 = tid >> 3, bytes = BITS >= 4 ? 16 : BITS == 2 ? 8 : 4, rows = 16;
+    k.dst = codes + (BITS >= 4 ? r0 * 128 + ((c ^ (r0 & 7)) << 4)
+                               : BITS == 2 ? r0 * 64 + (((c >> 1) ^ ((r0 >> 1) & 3)) << 4) + 8 * (c & 1) : r0 * TL::PITCH + 4 * c);
+  }
+  k.first = c * bytes;
+  k.step = static_cast<uint32_t>(rows * row_bytes);
+  k.src = reinterpret_cast<const unsigned char*>(T.k_data) + (static_cast<int64_t>(bh) * D + r0) * row_bytes +
+          static_cast<int64_t>(t0) * BITS / 8 + k.first;
+  return k;
+}
+template <int BITS>
+__device__ __forceinline__ void k_codes_request(const KCopy<BITS>& k, int chunk, int valid, bool wide2) {
+  using TL = KTile<BITS>;
+  if (k.first >= valid) return;
+  const unsigned char* s = k.src + static_cast<int64_t>(chunk) * (TL::TOKENS * BITS / 8);
+  const uint32_t d = k.dst + (chunk & 1) * K_CODES;
+  if (BITS == 2 && wide2) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) cp_async_16(d + i * 32 * TL::PITCH, s + static_cast<uint64_t>(k.step) * i);
     return;
   }
-  // a copy instruction moves 8 rows x 64 bytes (16 rows x 32 bytes at 2 bits)
-  constexpr int LPR = BITS == 2 ? 2 : 4;    // lanes per row
-  constexpr int RPI = 32 / LPR;             // rows per instruction
-  const int c = lane % LPR, r0 = lane / LPR;
 #pragma unroll
-  for (int quarter = 0; quarter < 4; ++quarter) {
-#pragma unroll
-    for (int i = 0; i < 32 / RPI; ++i) {
-      const int row = quarter * 32 + i * RPI + r0;
-      const unsigned char* s = src + row * row_bytes + 16 * c;
-      unsigned char* d = ws.u.codes + TL::offset(row, c);
-      if constexpr (BITS == 2) {  // rows of 2-bit codes are only 8-byte aligned in memory
-        if (16 * c < valid_bytes) cp_async_8(d, s);
-        if (16 * c + 8 < valid_bytes) cp_async_8(d + 8, s + 8);
-      } else {
-        if (16 * c < valid_bytes) cp_async_16(d, s);
-      }
-    }
-    cp_async_commit();
+  for (int i = 0; i < 8; ++i) {
+    const unsigned char* p = s + static_cast<uint64_t>(k.step) * i;
+    if (BITS >= 4) cp_async_16(d + i * 16 * TL::PITCH, p);
+    else if (BITS == 2) cp_async_8(d + i * 16 * TL::PITCH, p);
+    else cp_async_4(d + i * 16 * TL::PITCH, p);
   }
 }
 
-// 16-bit halves of two words -> one half2 register (low half from a)
-__device__ __forceinline__ uint32_t pack_lo16(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x5410); }
-
-// Zq[group][head] of the tile for half hh of the heads: rows of the A operand are the tile's groups
-// (at most four; rows 4-7 repeat them, rows 8-15 are zero).  zrow: this lane's two staged zero rows
-// (channels 2*tig and 2*tig+1) at the half of the tile's first group.
-// Gaussian-codebook tier (s_even / s_odd non-null: the std rows at the same halves): a value is
-// std * C * (2 code - 1) + mean, so the term that does not depend on the code is sum_c (mean - C std) q.
-__device__ __forceinline__ void k_tile_zq(KShared& sh, KWarpShared& ws, int hh, const __half* z_even, const __half* z_odd,
-                                          const __half* s_even = nullptr, const __half* s_odd = nullptr) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-  const int gam = g & 3;
-  float zacc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 2
-  for (int kt = 0; kt < 8; ++kt) {
-    const int o = (16 * kt) * K_RAW_HALFS + gam;
-    const uint32_t a0 = pack_lo16(__half_as_ushort(z_even[o]), __half_as_ushort(z_odd[o]));
-    const uint32_t a2 = pack_lo16(__half_as_ushort(z_even[o + 8 * K_RAW_HALFS]), __half_as_ushort(z_odd[o + 8 * K_RAW_HALFS]));
-    const uint2 bq = sh.qb[hh][kt][lane];
-    mma16816(zacc, a0, 0u, a2, 0u, bq.x, bq.y);
-  }
-  if (s_even) {
-    float sacc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 2
-    for (int kt = 0; kt < 8; ++kt) {
-      const int o = (16 * kt) * K_RAW_HALFS + gam;
-      const uint32_t a0 = pack_lo16(__half_as_ushort(s_even[o]), __half_as_ushort(s_odd[o]));
-      const uint32_t a2 = pack_lo16(__half_as_ushort(s_even[o + 8 * K_RAW_HALFS]), __half_as_ushort(s_odd[o + 8 * K_RAW_HALFS]));
-      const uint2 bq = sh.qb[hh][kt][lane];
-      mma16816(sacc, a0, 0u, a2, 0u, bq.x, bq.y);
-    }
-    zacc[0] = fmaf(-HQKV_NORMAL1_CENTER, sacc[0], zacc[0]);
-    zacc[1] = fmaf(-HQKV_NORMAL1_CENTER, sacc[1], zacc[1]);
-  }
-  __syncwarp();  // readers of the previous half are done
-  if (g < 4 && tig < 2) {  // columns 0-3 are the four heads of this half; 4-7 repeat them
-    ws.zq[g][2 * tig] = zacc[0];
-    ws.zq[g][2 * tig + 1] = zacc[1];
-  }
-  __syncwarp();
-}
-
-// A fragment registers of the four M-tiles of a sub-span from the ldmatrix registers of one 8-channel
-// octet.  R[c]: 16-byte piece c of the sub-span; each 16-bit half = block g of one channel.
-// lo[i] -> fragment row g of M-tile i, hi[i] -> row g+8.  Fields are fp16 subnormals code * 2^(k-24);
-// KField<BITS>::shift(i) gives k of M-tile i.
-//   8 bits: block = 2 tokens.  M-tile i = (piece p = i>>1, token e = i&1): row g <- piece p, row g+8 <-
-//           piece p+2.  Tokens: row g = 16p + 2g + e, row g+8 = 32 + 16p + 2g + e.
-//   4 bits: block = 4 tokens.  M-tile i: row g <- piece 0 token i, row g+8 <- piece 1 token i.
-//           Tokens: row g = 4g + i, row g+8 = 32 + 4g + i.
-//   2 bits: block = 8 tokens, one piece.  M-tile i: row g <- token i, row g+8 <- token 4+i of block g.
-//           Tokens: row g = 8g + i, row g+8 = 8g + 4 + i.
-//   1 bit:  block = 16 tokens, four blocks per sub-span (no ldmatrix: lane g reads block g & 3 with a
-//           2-byte load).  M-tile i: row g <- token 4*(g>>2) + i, row g+8 <- token 8 + 4*(g>>2) + i of
-//           block g & 3.  Tokens: row g = 16*(g&3) + 4*(g>>2) + i, row g+8 = +8.
+// Token of a lane's logit j = (unit or M-tile, then row g / g+8) within the warp's tokens: see k_logit_index.
+//   8 bits: M-tile i: row g = token 2g + i, row g+8 = 16 + 2g + i;   4 bits, unit u: 32u + 4g + i and 32u + 4g + 2 + i
+//   2 bits: 8g + i and 8g + 4 + i;   1 bit: 16(g&3) + 4(g>>2) + i and + 8
+// k_lane_base: the part that depends on the lane, within its unit; k_step: the rest, within the unit of logit j.
 template <int BITS>
-struct KField {
-  static __host__ __device__ constexpr int shift(int i) {
-    return BITS == 8 ? 0 : BITS == 4 ? 4 * (i & 1) : BITS == 2 ? 2 * i : i;
-  }
-};
+__device__ __forceinline__ int k_lane_unit() {  // (not used at 4 bits, where a lane has tokens of both units)
+  const int g = (threadIdx.x & 31) >> 2;
+  return BITS == 2 ? g >> 2 : BITS == 1 ? (g & 3) >> 1 : 0;
+}
 template <int BITS>
-__device__ __forceinline__ void octet_frags(const uint32_t* R, uint32_t (&lo)[4], uint32_t (&hi)[4]) {
-  if constexpr (BITS == 8) {
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      lo[2 * p] = R[p] & 0x00FF00FFu;
-      lo[2 * p + 1] = __byte_perm(R[p], 0u, 0x4341);
-      hi[2 * p] = R[p + 2] & 0x00FF00FFu;
-      hi[2 * p + 1] = __byte_perm(R[p + 2], 0u, 0x4341);
-    }
-  } else if constexpr (BITS == 4) {
-    const uint32_t a = R[0], as = R[0] >> 8, b = R[1], bs = R[1] >> 8;
-    lo[0] = a & 0x000F000Fu;
-    lo[1] = a & 0x00F000F0u;
-    lo[2] = as & 0x000F000Fu;
-    lo[3] = as & 0x00F000F0u;
-    hi[0] = b & 0x000F000Fu;
-    hi[1] = b & 0x00F000F0u;
-    hi[2] = bs & 0x000F000Fu;
-    hi[3] = bs & 0x00F000F0u;
-  } else {
-    const uint32_t a = R[0], as = R[0] >> 8;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      lo[i] = a & (0x00030003u << (2 * i));
-      hi[i] = as & (0x00030003u << (2 * i));
-    }
-  }
+__device__ __forceinline__ int k_lane_base() {
+  const int g = (threadIdx.x & 31) >> 2;
+  return BITS == 8 ? 2 * g : BITS == 4 ? 4 * g : BITS == 2 ? 8 * (g & 3) : 16 * (g & 1) + 4 * (g >> 2);
+}
+template <int BITS>
+__host__ __device__ constexpr int k_step(int j) {
+  const int r = j & 1, i = BITS == 4 ? (j >> 1) & 1 : j >> 1;
+  return i + r * (BITS == 8 ? 16 : BITS == 4 ? 2 : BITS == 2 ? 4 : 8);
 }
 
-// running (max, sum-exp) of a lane over values it produces four at a time; -inf marks "no value"
-__device__ __forceinline__ void softmax_push4(float& m, float& l, const float (&x)[4]) {
-  const float mn = fmaxf(fmaxf(m, fmaxf(x[0], x[1])), fmaxf(x[2], x[3]));
+// running (max, sum-exp) of a lane; -inf marks "no value"
+template <int N>
+__device__ __forceinline__ void softmax_push(float& m, float& l, const float (&x)[N]) {
+  float mn = m;
+#pragma unroll
+  for (int j = 0; j < N; ++j) mn = fmaxf(mn, x[j]);
   const float ref = (mn == -INFINITY ? 0.f : mn) * LOG2E;
-  l = l * fast_exp2(fmaf(m, LOG2E, -ref)) + (fast_exp2(fmaf(x[0], LOG2E, -ref)) + fast_exp2(fmaf(x[1], LOG2E, -ref))) +
-      (fast_exp2(fmaf(x[2], LOG2E, -ref)) + fast_exp2(fmaf(x[3], LOG2E, -ref)));
+  l *= fast_exp2(fmaf(m, LOG2E, -ref));
+#pragma unroll
+  for (int j = 0; j < N; ++j) l += fast_exp2(fmaf(x[j], LOG2E, -ref));
   m = mn;
 }
 
-// One tile of a quantised tier, already requested: all heads of this kv head.
-// g0c = first scale group of the CTA's chunk.  m/l: this lane's running softmax pairs, [hh][e] for
-// head 4*hh + 2*(tig&1) + e.
+// The lane's logits of one chunk: x[j], j = NX logits of head tig.  zq = zero terms of the chunk's first group on, scale =
+// softmax scale (pscale: that of the code term).  codes = address of the chunk's
+// codes, srow0 = scale row of the chunk's first group, qrow = this lane's B fragments of q.
 template <int BITS>
-__device__ __forceinline__ void k_tile_compute(const DecodeParams& P, const TierDev& T, KShared& sh, KWarpShared& ws,
-                                               int tile_t0, int ntok, int g0c, int nh, float* row0, const __half* mask0,
-                                               float (&m)[2][2], float (&l)[2][2]) {
+__device__ __forceinline__ void k_chunk_logits(float (&x)[KTile<BITS>::NX], uint32_t codes, uint32_t srow0, uint32_t qrow,
+                                               const float (*zq)[MAX_R4][KWARPS], float scale, float pscale, int gk_shift) {
   using TL = KTile<BITS>;
-  const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-  const int G = T.n_k >> P.gk_shift;
-  // staged scale / zero rows of this lane's channels 2*tig (even) and 2*tig+1 (odd) of step 0, at the
-  // half of the chunk's first group; a step adds 16 rows, the +8 channels add 8 rows
-  const int sh_even = static_cast<int>((static_cast<int64_t>(2 * tig) * G + g0c) & 7);
-  const int sh_odd = static_cast<int>((static_cast<int64_t>(2 * tig + 1) * G + g0c) & 7);
-  const int gt0 = (tile_t0 >> P.gk_shift) - g0c;  // first group of the tile within the chunk
-  // ldmatrix row address of this lane for step 0 / sub-span 0 (see the loop for the matrix order)
-  uint32_t lm_off;
-  {
-    const int mi = lane >> 3, rr = lane & 7;
-    if constexpr (BITS == 8) {
-      lm_off = TL::offset(rr, mi);                           // octet 0; pieces 0..3
-    } else if constexpr (BITS == 4) {
-      lm_off = TL::offset(8 * (mi >> 1) + rr, mi & 1);       // (octet 0, piece 0), (0,1), (1,0), (1,1)
-    } else if constexpr (BITS == 2) {
-      lm_off = TL::offset(8 * mi + rr, 0);                   // steps kt, kt+1: octets 0..3 of 32 channels
-    } else {
-      lm_off = (2 * tig) * 16 + 2 * (g & 3);                 // 1 bit: this lane's block of channel 2*tig
-    }
+  constexpr bool ONE_GROUP = TL::ONE_GROUP;
+  constexpr int UNITS = BITS == 4 ? 2 : 1;          // accumulator sets
+  constexpr int NM = ONE_GROUP ? 2 : 4;             // M-tiles per set
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tig = lane & 3;
+  const uint32_t remainder = (g & 1) ? 0xFFFFFFFFu : 0u;
+  // scale rows of this lane's B column
+  uint32_t srow[UNITS];
+#pragma unroll
+  for (int u = 0; u < UNITS; ++u) srow[u] = srow0 + ((warp * TL::WTOK + 32 * (ONE_GROUP ? u : (g & 1))) >> gk_shift) * K_SROW + tig * 16;
+  // ldmatrix row address of this lane for step 0
+  uint32_t kb = codes, kb1 = 0;
+  if constexpr (BITS == 8) {
+    const int mi = lane >> 3, rr = lane & 7;        // matrices (octet, piece): (0,0), (0,1), (1,0), (1,1)
+    kb += (8 * (mi >> 1) + rr) * 128 + (((2 * warp + (mi & 1)) ^ rr) << 4);
+  } else if constexpr (BITS == 4) {
+    kb += lane * 128 + (((2 * warp) ^ (lane & 7)) << 4);   // octets 0..3 of 32 channels; unit 1: the other piece of the pair
+    kb1 = kb ^ 16u;
+  } else if constexpr (BITS == 2) {
+    kb += lane * 64 + ((warp ^ ((lane >> 1) & 3)) << 4);
+  } else {
+    kb += (2 * tig) * TL::PITCH + 8 * warp + 2 * (g & 3);  // block g & 3 of channel 2tig
   }
-  const int hp = tig & 1;
-  // Gaussian-codebook 1-bit tier: the code term carries the factor 2C
-  const bool normal = BITS == 1 && T.normal != 0;
-  const float pscale = normal ? P.scale * (2.f * HQKV_NORMAL1_CENTER) : P.scale;
-
-  for (int hh = 0; hh < nh; ++hh) {
-    if (normal)
-      k_tile_zq(sh, ws, hh, &sh.z[2 * tig][sh_even + gt0], &sh.z[2 * tig + 1][sh_odd + gt0], &sh.s[2 * tig][sh_even + gt0],
-                &sh.s[2 * tig + 1][sh_odd + gt0]);
-    else
-      k_tile_zq(sh, ws, hh, &sh.z[2 * tig][sh_even + gt0], &sh.z[2 * tig + 1][sh_odd + gt0]);
-    const uint2* qb = &sh.qb[hh][0][lane];
-#pragma unroll 1
-    for (int j = 0; j < TL::NSUB; ++j) {
-      // as a B column this lane is n = g: columns 0-3 carry the scale group of tokens 0-31 of the
-      // sub-span, columns 4-7 that of tokens 32-63
-      const int gam = ((tile_t0 + j * K_SPAN + 32 * (g >> 2)) >> P.gk_shift) - g0c;
-      const __half* s_even = &sh.s[2 * tig][sh_even + gam];
-      const __half* s_odd = &sh.s[2 * tig + 1][sh_odd + gam];
-      const unsigned char* kb = ws.u.codes + (BITS == 1 ? lm_off + j * 8 : (lm_off ^ (j * TL::CPS * 16)));
-      const uint2* qk = qb;
-      float acc[4][4];
+  float acc[UNITS][NM][4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-      // two 16-channel steps per iteration (short loop body: the instruction cache is cold in every CTA
-      // when the whole cache is one wave of CTAs)
-#pragma unroll 1
-      for (int kk = 0; kk < 4; ++kk) {
-        if (hh == 0 && j == 0) {  // the codes arrive two steps at a time
-          if (kk == 0) cp_async_wait<3>();
-          else if (kk == 1) cp_async_wait<2>();
-          else if (kk == 2) cp_async_wait<1>();
-          else cp_async_wait<0>();
-          __syncwarp();
-        }
-        uint32_t R2[4];  // 2 bits: one ldmatrix feeds both steps
-        if constexpr (BITS == 2) ldmatrix_x4_trans(R2, kb);
-        (void)R2;
+  for (int u = 0; u < UNITS; ++u)
 #pragma unroll
-        for (int k2 = 0; k2 < 2; ++k2) {
-          // A fragments: lo/hi of octet 0 -> registers 0/1 (channels 2tig, 2tig+1), of octet 1 -> 2/3 (+8)
-          uint32_t a[4][4];  // [register][M-tile]
-          if constexpr (BITS == 8) {
-            uint32_t R[4];
-            ldmatrix_x4_trans(R, kb + k2 * 16 * TL::PITCH);
-            octet_frags<8>(R, a[0], a[1]);
-            ldmatrix_x4_trans(R, kb + k2 * 16 * TL::PITCH + 8 * TL::PITCH);
-            octet_frags<8>(R, a[2], a[3]);
-          } else if constexpr (BITS == 4) {
-            uint32_t R[4];
-            ldmatrix_x4_trans(R, kb + k2 * 16 * TL::PITCH);
-            octet_frags<4>(R, a[0], a[1]);
-            octet_frags<4>(R + 2, a[2], a[3]);
-          } else if constexpr (BITS == 2) {
-            octet_frags<2>(R2 + 2 * k2, a[0], a[1]);
-            octet_frags<2>(R2 + 2 * k2 + 1, a[2], a[3]);
-          } else {
-#pragma unroll
-            for (int o = 0; o < 2; ++o) {  // channels 2tig, 2tig+1 (o = 0) and +8, +9 (o = 1)
-              const unsigned char* cb = kb + (k2 * 16 + o * 8) * 16;
-              const uint32_t t = pack_lo16(*reinterpret_cast<const uint16_t*>(cb), *reinterpret_cast<const uint16_t*>(cb + 16));
-              const uint32_t lo = t >> (4 * (g >> 2)), hi = lo >> 8;
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                a[2 * o][i] = lo & (0x00010001u << i);
-                a[2 * o + 1][i] = hi & (0x00010001u << i);
-              }
-            }
-          }
-          const int o = (16 * k2) * K_RAW_HALFS;
-          const __half2 s0 = u32_as_h2(pack_lo16(__half_as_ushort(s_even[o]), __half_as_ushort(s_odd[o])));
-          const __half2 s1 = u32_as_h2(pack_lo16(__half_as_ushort(s_even[o + 8 * K_RAW_HALFS]),
-                                                 __half_as_ushort(s_odd[o + 8 * K_RAW_HALFS])));
-          const uint2 qv = qk[k2 * 32];
-          const __half2 hi0 = __hmul2(u32_as_h2(qv.x), s0);
-          const __half2 hi1 = __hmul2(u32_as_h2(qv.y), s1);
-          const __half2 lo0 = __hfma2(u32_as_h2(qv.x), s0, __hneg2(hi0));  // exact remainder
-          const __half2 lo1 = __hfma2(u32_as_h2(qv.y), s1, __hneg2(hi1));
-          // the two MMAs into one accumulator are issued four apart (they depend on each other)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) mma16816(acc[i], a[0][i], a[1][i], a[2][i], a[3][i], h2_as_u32(hi0), h2_as_u32(hi1));
-#pragma unroll
-          for (int i = 0; i < 4; ++i) mma16816(acc[i], a[0][i], a[1][i], a[2][i], a[3][i], h2_as_u32(lo0), h2_as_u32(lo1));
-        }
-        kb += 32 * TL::PITCH;
-        s_even += 32 * K_RAW_HALFS;
-        s_odd += 32 * K_RAW_HALFS;
-        qk += 64;
-      }
-      // Epilogue from registers: a lane keeps the accumulator columns whose scale group is its row's, and
-      // every lane ends up with four tokens x two heads (heads 2*(tig&1), +1).
-      //  8 / 4 bits: rows 0-7 are tokens 0-31, rows 8-15 tokens 32-63: lanes tig 0,1 own row g, lanes
-      //              tig 2,3 own row g+8.
-      //  2 bits:     rows g and g+8 are the eight tokens of block g, valid in the lanes with
-      //              (g < 4) == (tig < 2); such a lane keeps the row of its tig half and hands the
-      //              other row to lane tig ^ 2, whose own accumulators belong to the wrong scale group.
-      //  1 bit:      the same with block g & 3: valid where ((g & 3) < 2) == (tig < 2).
-      const int sub_t0 = j * K_SPAN;
-      const int r = tig >> 1;
-      float val[4][2];
+    for (int i = 0; i < NM; ++i) acc[u][i][0] = acc[u][i][1] = acc[u][i][2] = acc[u][i][3] = 0.f;
+  // Two 16-channel steps per iteration.  The operands of the next iteration are requested before this one's are used:
+  // with four warps per scheduler the round trip to shared memory is not covered by other warps.
+  uint32_t Rb[2][2][4];
+  uint4 qb[2], sb4[2][UNITS];
+  auto fetch = [&](int p) {
+    uint32_t(&R)[2][4] = Rb[p & 1];
+    if constexpr (BITS == 8) {
+      ldmatrix_x4_trans(R[0], kb + p * 4096);
+      ldmatrix_x4_trans(R[1], kb + p * 4096 + 2048);
+    } else if constexpr (BITS == 4) {
+      ldmatrix_x4_trans(R[0], kb + p * 4096);
+      ldmatrix_x4_trans(R[1], kb1 + p * 4096);
+    } else if constexpr (BITS == 2) {
+      ldmatrix_x4_trans(R[0], kb + p * 2048);
+    } else {  // 16-bit pieces of channels 2tig, 2tig+1 (+8, +9; next step)
 #pragma unroll
       for (int i = 0; i < 4; ++i)
+        R[0][i] = pack_lo16(lds16(kb + (32 * p + 8 * i) * TL::PITCH), lds16(kb + (32 * p + 8 * i + 1) * TL::PITCH));
+    }
+    qb[p & 1] = lds128(qrow + p * sizeof(KShared::q[0]));
 #pragma unroll
-        for (int e = 0; e < 2; ++e) val[i][e] = r ? acc[i][2 + e] : acc[i][e];
-      if constexpr (BITS <= 2) {
-        const bool valid = BITS == 2 ? (g < 4) == (tig < 2) : ((g & 3) < 2) == (tig < 2);
+    for (int u = 0; u < UNITS; ++u) sb4[p & 1][u] = lds128(srow[u] + p * 64);
+  };
+  fetch(0);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+  for (int p = 0; p < 4; ++p) {
+    if (p < 3) fetch(p + 1);
+    const uint32_t(&R)[2][4] = Rb[p & 1];
+    const uint4 q4 = qb[p & 1];
+    const uint32_t q[2][2] = {{q4.x, q4.y}, {q4.z, q4.w}};
+    if constexpr (ONE_GROUP) {
+      uint32_t qm[2][2];
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float other = __shfl_xor_sync(0xffffffffu, r ? acc[i][e] : acc[i][2 + e], 2);
-            if (!valid) val[i][e] = other;
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) qm[k][h] = (q[k][h] ^ 0x80008000u) & remainder;
+#pragma unroll
+      for (int u = 0; u < UNITS; ++u) {
+        const uint4 s4 = sb4[p & 1][u];
+        const uint32_t s[2][2] = {{s4.x, s4.y}, {s4.z, s4.w}};
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          // even columns (qm = 0): hi = fp16(q*s); odd columns (qm = -q): the exact remainder q*s - hi
+          const uint32_t b0 = h2_fma(q[k][0], s[k][0], h2_mul(qm[k][0], s[k][0]));
+          const uint32_t b1 = h2_fma(q[k][1], s[k][1], h2_mul(qm[k][1], s[k][1]));
+          if constexpr (BITS == 8) {
+            const uint32_t* r = R[k];
+            mma16816(acc[u][0], r[0] & 0x00FF00FFu, r[1] & 0x00FF00FFu, r[2] & 0x00FF00FFu, r[3] & 0x00FF00FFu, b0, b1);
+            mma16816(acc[u][1], __byte_perm(r[0], 0u, 0x4341), __byte_perm(r[1], 0u, 0x4341), __byte_perm(r[2], 0u, 0x4341),
+                     __byte_perm(r[3], 0u, 0x4341), b0, b1);
+          } else {
+            const uint32_t ra = R[u][2 * k], rb = R[u][2 * k + 1], sa = ra >> 8, sb = rb >> 8;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              const uint32_t m = 0x000F000Fu << (4 * i);
+              mma16816(acc[u][i], ra & m, sa & m, rb & m, sb & m, b0, b1);
+            }
           }
-      }
-      // first of this lane's tokens (8 bits: tokens my_tok, +1, +16, +17; 4 and 2 bits: my_tok .. my_tok+3)
-      const int my_tok = sub_t0 + (BITS == 8 ? 32 * r + 2 * g : BITS == 4 ? 32 * r + 4 * g : BITS == 2 ? 8 * g + 4 * r
-                                                                : 16 * (g & 3) + 4 * (g >> 2) + 8 * r);
-      const bool live = my_tok < ntok;
-      const int my_gam = ((tile_t0 + my_tok) >> P.gk_shift) - g0c - gt0;
-      uint32_t pos[4];
-      if constexpr (BITS == 8) {
-        const int4 pa = *reinterpret_cast<const int4*>(&ws.idx[my_tok]);  // low words of int64 positions: .x and .z
-        const int4 pb = *reinterpret_cast<const int4*>(&ws.idx[my_tok + 16]);
-        pos[0] = static_cast<uint32_t>(pa.x), pos[1] = static_cast<uint32_t>(pa.z);
-        pos[2] = static_cast<uint32_t>(pb.x), pos[3] = static_cast<uint32_t>(pb.z);
-      } else {
-        const int4* ip = reinterpret_cast<const int4*>(&ws.idx[my_tok]);
-        const int4 p01 = ip[0], p23 = ip[1];
-        pos[0] = static_cast<uint32_t>(p01.x), pos[1] = static_cast<uint32_t>(p01.z);
-        pos[2] = static_cast<uint32_t>(p23.x), pos[3] = static_cast<uint32_t>(p23.z);
-      }
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int head = 4 * hh + 2 * hp + e;
-        const bool on = live && head < P.rep;
-        const float zqs = ws.zq[my_gam & 3][2 * hp + e] * P.scale;
-        float* row = row0 + static_cast<int64_t>(head) * P.L;
-        const __half* mrow = mask0 ? mask0 + head * P.mask_hstride : nullptr;
-        float x[4];
-        bool ok[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float unscale = static_cast<float>(1 << (24 - KField<BITS>::shift(i)));
-          ok[i] = on && HQKV_INDEX_OK(pos[i], P.L);
-          x[i] = ok[i] ? fmaf(val[i][e], pscale * unscale, zqs) : -INFINITY;
         }
-        if (mrow) {  // one branch for the calls without a mask
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            if (ok[i]) x[i] += __half2float(mrow[pos[i]]);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (ok[i]) row[pos[i]] = x[i];
-        softmax_push4(m[hh][e], l[hh][e], x);
       }
+    } else {
+      const uint4 s4 = sb4[p & 1][0];
+      const uint32_t s[2][2] = {{s4.x, s4.y}, {s4.z, s4.w}};
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const uint32_t h0 = h2_mul(q[k][0], s[k][0]), h1 = h2_mul(q[k][1], s[k][1]);
+        const uint32_t l0 = h2_rem(q[k][0], s[k][0], h0), l1 = h2_rem(q[k][1], s[k][1], h1);
+        uint32_t a[4][4];  // [register][M-tile]
+#pragma unroll
+        for (int o = 0; o < 2; ++o) {
+          const uint32_t lo = BITS == 2 ? R[0][2 * k + o] : R[0][2 * k + o] >> (4 * (g >> 2));
+          const uint32_t hi = lo >> 8;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t m = BITS == 2 ? 0x00030003u << (2 * i) : 0x00010001u << i;
+            a[2 * o][i] = lo & m;
+            a[2 * o + 1][i] = hi & m;
+          }
+        }
+        // the two MMAs into one accumulator are issued four apart (they depend on each other)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mma16816(acc[0][i], a[0][i], a[1][i], a[2][i], a[3][i], h0, h1);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mma16816(acc[0][i], a[0][i], a[1][i], a[2][i], a[3][i], l0, l1);
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < UNITS; ++u) {
+    const bool second = !ONE_GROUP && k_lane_unit<BITS>() == 1;
+    const int gam = (warp * TL::WTOK + 32 * (BITS == 4 ? u : k_lane_unit<BITS>())) >> gk_shift;
+    const float4 zp = *reinterpret_cast<const float4*>(zq[gam][tig]);
+    const float z = ((zp.x + zp.y) + (zp.z + zp.w)) * scale;
+#pragma unroll
+    for (int i = 0; i < NM; ++i)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        constexpr int SH = BITS == 8 ? 0 : BITS;  // M-tile i holds the field at bit SH * i
+        const float unscale = static_cast<float>(1 << 24) / static_cast<float>(1 << (SH * i));
+        const float* a = &acc[u][i][2 * r];
+        x[(u * NM + i) * 2 + r] = fmaf(ONE_GROUP ? a[0] + a[1] : (second ? a[1] : a[0]), pscale * unscale, z);
+      }
+  }
+}
+
+// Positions of the warp's tokens: pu[u] = position of stored token 32*u + lane of the warp (low word of the int64).
+template <int BITS>
+__device__ __forceinline__ void k_positions(const TierDev& T, uint32_t (&pu)[KTile<BITS>::HALVES], int t0) {
+  const int t = t0 + (threadIdx.x >> 5) * KTile<BITS>::WTOK + (threadIdx.x & 31);
+#pragma unroll
+  for (int u = 0; u < KTile<BITS>::HALVES; ++u)
+    pu[u] = t + 32 * u < T.n_k ? __ldg(reinterpret_cast<const uint32_t*>(T.k_idx + t + 32 * u)) : 0u;
+}
+
+// Any positions, any number of heads, masks: the lane's logits, as they count (-inf: none), in x.
+template <int BITS>
+__device__ __forceinline__ void k_store_any(const DecodeParams& P, const TierDev& T, const Where& w, float (&x)[KTile<BITS>::NX],
+                                         const uint32_t (&pu)[KTile<BITS>::HALVES], int wt0) {
+  using TL = KTile<BITS>;
+  constexpr int NX = TL::NX, HALVES = TL::HALVES;
+  const int tig = threadIdx.x & 3, lb = k_lane_base<BITS>();
+  float* out = P.logits + static_cast<int64_t>(w.bvh) * P.L * P.r4 + tig;
+  bool valid[HALVES];
+#pragma unroll
+  for (int u = 0; u < HALVES; ++u) valid[u] = wt0 + 32 * u < T.n_k;
+      const bool on = tig < P.r4;
+      const __half* mrow = P.mask ? P.mask + w.b * P.mask_bstride + (w.h0 + (on ? tig : 0)) * P.mask_hstride : nullptr;
+  #pragma unroll
+      for (int j = 0; j < NX; ++j) {
+        const int src = lb + k_step<BITS>(j);
+        uint32_t pos = __shfl_sync(0xffffffffu, pu[BITS == 4 ? j >> 2 : 0], src);
+        bool ok = on && valid[BITS == 4 ? j >> 2 : 0];
+        if constexpr (BITS <= 2) {
+          const uint32_t pos1 = __shfl_sync(0xffffffffu, pu[HALVES - 1], src);
+          if (k_lane_unit<BITS>() == 1) {
+            pos = pos1;
+            ok = on && valid[HALVES - 1];
+          }
+        }
+        ok = ok && HQKV_INDEX_OK(pos, P.L);
+        if (ok) {
+          if (mrow) x[j] += __half2float(mrow[pos]);
+          out[static_cast<int64_t>(pos) * P.r4] = x[j];
+        } else {
+          x[j] = -INFINITY;
+        }
+      }
+}
+
+// Store the lane's logits at their positions and add them to its running softmax statistics.  wt0 = the warp's first
+// token in the tier.
+template <int BITS>
+__device__ __forceinline__ void k_emit(const DecodeParams& P, const TierDev& T, const Where& w, float (&x)[KTile<BITS>::NX],
+                                       const uint32_t (&pu)[KTile<BITS>::HALVES], int wt0, float& m, float& l) {
+  using TL = KTile<BITS>;
+  constexpr int NX = TL::NX, HALVES = TL::HALVES;
+  const int lane = threadIdx.x & 31, tig = lane & 3;
+  const int lb = k_lane_base<BITS>();
+  float* out = P.logits + static_cast<int64_t>(w.bvh) * P.L * P.r4 + tig;
+  // whole 32-token units are valid or not (a tier holds a multiple of 32 tokens)
+  bool valid[HALVES], dense = P.r4 == MAX_R4 && P.mask == nullptr;
+  uint32_t base[HALVES];
+#pragma unroll
+  for (int u = 0; u < HALVES; ++u) {
+    valid[u] = wt0 + 32 * u < T.n_k;
+    base[u] = __shfl_sync(0xffffffffu, pu[u], 0);
+    dense = dense && (!valid[u] || (pu[u] == base[u] + lane && HQKV_INDEX_OK(pu[u], P.L)));
+  }
+  if (__all_sync(0xffffffffu, dense)) {
+    if constexpr (BITS == 4 || BITS == 8) {
+#pragma unroll
+      for (int u = 0; u < HALVES; ++u) {
+        float* o = out + static_cast<int64_t>(base[u] + lb) * MAX_R4;
+#pragma unroll
+        for (int j = 4 * u; j < 4 * u + 4; ++j) {
+          if (valid[u]) o[k_step<BITS>(j) * MAX_R4] = x[j];
+          else x[j] = -INFINITY;
+        }
+      }
+    } else {
+      const bool second = k_lane_unit<BITS>() == 1;
+      const bool ok = second ? valid[HALVES - 1] : valid[0];
+      float* o = out + static_cast<int64_t>((second ? base[HALVES - 1] : base[0]) + lb) * MAX_R4;
+#pragma unroll
+      for (int j = 0; j < NX; ++j) {
+        if (ok) o[k_step<BITS>(j) * MAX_R4] = x[j];
+        else x[j] = -INFINITY;
+      }
+    }
+  } else {
+    k_store_any<BITS>(P, T, w, x, pu, wt0);
+  }
+  softmax_push<NX>(m, l, x);
+}
+
+// Tokens [t0, t1) of a quantised tier; m, l: the lane's running softmax pair (head tig).  `first`: nothing has run before
+// in this CTA.
+template <int BITS>
+__device__ __forceinline__ void k_run(const DecodeParams& P, const TierDev& T, KShared& sh, const Where& w, int t0, int t1,
+                                      float& m, float& l, bool& first) {
+  using TL = KTile<BITS>;
+  constexpr int PER_BLOCK = K_BLOCK / TL::TOKENS;   // chunks per fetch of scales
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tig = lane & 3;
+  const int chunks = (t1 - t0 + TL::TOKENS - 1) / TL::TOKENS;
+  const bool wide2 = BITS == 2 && (T.n_k & 63) == 0;
+  const bool normal = BITS == 1 && T.normal != 0;   // Gaussian-codebook 1-bit tier: the code term carries the factor 2C
+  const float pscale = normal ? P.scale * (2.f * HQKV_NORMAL1_CENTER) : P.scale;
+  const uint32_t codes = smem_u32(sh.u.codes), srows = smem_u32(sh.s), qrow = smem_u32(&sh.q[0][lane]);
+  KScales k;
+  k.G = T.n_k >> P.gk_shift;
+  k.row0 = (static_cast<int64_t>(w.bh) * D + 32 * warp) * k.G;
+  k.raw = smem_u32(sh.v.raw[0][warp]);
+  k.s_at = srows + 2 * k_order(tid);
+  k.z_at = smem_u32(sh.z[warp]) + 2 * lane;
+  k.z_row = smem_u32(sh.z[warp]) + ((lane & 7) + 8 * ((lane >> 3) & 1)) * K_ZROW + 16 * (lane >> 4);
+  auto tokens = [&](int c) { return min(TL::TOKENS, t1 - t0 - c * TL::TOKENS); };
+  auto groups = [&](int blk) { return (min(K_BLOCK, t1 - t0 - blk * K_BLOCK) + (1 << P.gk_shift) - 1) >> P.gk_shift; };
+  auto first_group = [&](int blk) { return (t0 + blk * K_BLOCK) >> P.gk_shift; };
+  if (!first) __syncthreads();  // every warp is done with the buffers
+  k_scales_request(T, k, first_group(0), groups(0));
+  cp_async_commit();
+  const KCopy<BITS> copy = k_copy_init<BITS>(T, w.bh, t0, codes, wide2);
+  k_codes_request<BITS>(copy, 0, tokens(0) * BITS / 8, wide2);
+  cp_async_commit();
+  if (chunks > 1) k_codes_request<BITS>(copy, 1, tokens(1) * BITS / 8, wide2);
+  cp_async_commit();
+  uint32_t pu[TL::HALVES];
+  k_positions<BITS>(T, pu, t0);
+  cp_async_wait<2>();
+  __syncwarp();
+  k_scales_transpose(k, first_group(0), groups(0));
+  // Everything above reads only the cache.  From here on this grid reads q - the one input an earlier kernel of the
+  // stream may still be writing - and writes the scratch that the previous decode call may still be using: wait for the
+  // kernels before it.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  first = false;
+  // every warp fetches the fragments of its own 32 channels, which it also needs for the zero term
+  uint4 qz = make_uint4(0u, 0u, 0u, 0u);
+  if ((g >> 1) < P.r4) {
+    const uint32_t* qh = reinterpret_cast<const uint32_t*>(P.q + (static_cast<int64_t>(w.b) * P.nh_q + w.h0 + (g >> 1)) * D) +
+                         16 * warp + tig;
+    qz = make_uint4(qh[0], qh[4], qh[8], qh[12]);
+  }
+  sh.q[warp][lane] = qz;
+#pragma unroll 1
+  for (int c = 0; c < chunks; ++c) {
+    if (c == 0) cp_async_wait<1>();
+    else cp_async_wait<0>();
+    __syncthreads();  // the codes of chunk c are there; every warp is done with chunk c - 1
+    if (c > 0 && c + 1 < chunks) k_codes_request<BITS>(copy, c + 1, tokens(c + 1) * BITS / 8, wide2);
+    cp_async_commit();
+    if (c % PER_BLOCK == 0) {
+      const int blk = c / PER_BLOCK;
+      if (c > 0) k_scales_transpose(k, first_group(blk), groups(blk));
+      __syncwarp();
+      k_zero_term(k, qz, sh.zq, srows + g * K_SROW + warp * 64 + tig * 16, normal);
+      __syncthreads();
+      if (c + PER_BLOCK < chunks) k_scales_request(T, k, first_group(blk + 1), groups(blk + 1));
+      cp_async_commit();
+    }
+    const int wt0 = t0 + c * TL::TOKENS + warp * TL::WTOK;
+    if (wt0 < t1) {
+      uint32_t at[TL::HALVES];
+#pragma unroll
+      for (int u = 0; u < TL::HALVES; ++u) at[u] = pu[u];
+      if (c + 1 < chunks) k_positions<BITS>(T, pu, t0 + (c + 1) * TL::TOKENS);
+      const int in_block = (c % PER_BLOCK) * TL::TOKENS;
+      float x[TL::NX];
+      const int g0 = in_block >> P.gk_shift;  // first group of the chunk within the block
+      k_chunk_logits<BITS>(x, codes + (c & 1) * K_CODES, srows + g0 * K_SROW, qrow, sh.zq + g0, P.scale, pscale, P.gk_shift);
+      k_emit<BITS>(P, T, w, x, at, wt0, m, l);
     }
   }
 }
+
 // Write out a warp's logit tile [ntok][K_TROW] (already scaled) at the tokens' logical positions and
-// leave the warp's (max, sum-exp) per head in red_m / red_l.  Element = (token, head) with the head
-// fastest across lanes, so every lane owns ONE head for the whole call (rep divides 32): its running
-// max and sum are scalars, and index loads and stores are spread over all 32 lanes.
+// add them to the running softmax pairs.  Element = (token, head) with the head
+// fastest across lanes, so every lane owns ONE head for the whole call (r4 divides 32).
 // (fp16 tier and residual window only; the quantised tiers write from registers.)
-__device__ __forceinline__ void k_write_tile(const DecodeParams& P, float* tile, int ntok, const int64_t* idx,
-                                             int64_t first_pos, int b, int kvh, float* red_m, float* red_l) {
+__device__ __forceinline__ void k_write_tile(const DecodeParams& P, const Where& w, float* tile, int ntok, const int64_t* idx,
+                                             int64_t first_pos, float& m_out, float& l_out) {
   const int lane = threadIdx.x & 31;
-  const int rep = P.rep, rshift = P.rep_shift;
+  const int rep = P.r4, rshift = P.r4_shift;
   const int h = lane & (rep - 1);
-  float* row = P.logits + (static_cast<int64_t>(b) * P.nh_q + kvh * rep + h) * P.L;
-  const __half* mrow = P.mask ? P.mask + b * P.mask_bstride + static_cast<int64_t>(kvh * rep + h) * P.mask_hstride : nullptr;
+  float* out = P.logits + static_cast<int64_t>(w.bvh) * P.L * rep + h;
+  const __half* mrow = P.mask ? P.mask + w.b * P.mask_bstride + static_cast<int64_t>(w.h0 + h) * P.mask_hstride : nullptr;
   const int tpr = 32 >> rshift;  // tokens per round
-  float mx = -INFINITY;
+  float m = -INFINITY, l = 0.f;
 #pragma unroll 2
   for (int t = lane >> rshift; t < ntok; t += tpr) {
     const int64_t pos = idx ? idx[t] : first_pos + t;
-    float x = -INFINITY;
+    float x[1] = {-INFINITY};
     if (HQKV_INDEX_OK(pos, P.L)) {
-      x = tile[t * K_TROW + h];
-      if (mrow) x += __half2float(mrow[pos]);
-      row[pos] = x;
+      x[0] = tile[t * K_TROW + h];
+      if (mrow) x[0] += __half2float(mrow[pos]);
+      out[pos * rep] = x[0];
     }
-    tile[t * K_TROW + h] = x;  // the masked value is what the sum below sees
-    mx = fmaxf(mx, x);
+    softmax_push<1>(m, l, x);
   }
+  float mx = m;
   for (int off = rep; off < 32; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-  const float ref = mx == -INFINITY ? 0.f : mx;  // every position masked out: the sum is 0, not NaN
-  float sum = 0.f;
-#pragma unroll 2
-  for (int t = lane >> rshift; t < ntok; t += tpr) sum += fast_exp2((tile[t * K_TROW + h] - ref) * LOG2E);
+  float sum = l * fast_exp2((m - (mx == -INFINITY ? 0.f : mx)) * LOG2E);  // every position masked out: 0, not NaN
   for (int off = rep; off < 32; off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-  if (lane < rep) {
-    red_m[lane] = mx;
-    red_l[lane] = sum;
-  }
+  // lane h now holds head h; lanes 0-3 take it into their pairs (head tig)
+  if (lane < rep) softmax_merge(m_out, l_out, mx, sum);
 }
 
-
-// One tile per warp: request everything that depends only on the cache, wait for the kernels before
-// this one, fetch q, agree that q and the scale rows are in shared memory, compute.
-template <int BITS, typename LoadQ>
-__device__ __forceinline__ void k_chunk(const DecodeParams& P, const TierDev& T, KShared& sh, int bh, int b, int kvh,
-                                        int chunk_t0, int nh, LoadQ load_q) {
-  using TL = KTile<BITS>;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  KWarpShared& ws = sh.w[warp];
-  const int chunk_end = min(chunk_t0 + KWARPS * TL::TOKENS, T.n_k);
-  const int g0c = chunk_t0 >> P.gk_shift;
-  const int ngc = ((chunk_end - 1) >> P.gk_shift) - g0c + 1;
-  k_scales_request(P, T, sh, bh, g0c, ngc);
-  cp_async_commit();  // oldest group: the scale / zero rows
-  const int tile_t0 = chunk_t0 + warp * TL::TOKENS;
-  const int ntok = min(TL::TOKENS, T.n_k - tile_t0);  // <= 0: this warp has no tile
-  if (ntok > 0) k_tile_request<BITS>(T, ws, bh, tile_t0, ntok);
-  // Everything above reads only the cache.  From here on this grid reads q and writes the scratch that
-  // the previous decode call of the stream may still be using: wait for the kernels before it.
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  load_q();
-  if (ntok > 0) {
-    cp_async_wait<4>();
-  } else {
-    cp_async_wait<0>();
-  }
-  __syncthreads();
-  float m[2][2] = {{-INFINITY, -INFINITY}, {-INFINITY, -INFINITY}}, l[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-  if (ntok > 0) {
-    float* row0 = P.logits + (static_cast<int64_t>(b) * P.nh_q + kvh * P.rep) * P.L;
-    // additive mask rows of this kv head's query heads (null: none)
-    const __half* mask0 = P.mask ? P.mask + b * P.mask_bstride + static_cast<int64_t>(kvh * P.rep) * P.mask_hstride : nullptr;
-    k_tile_compute<BITS>(P, T, sh, ws, tile_t0, ntok, g0c, nh, row0, mask0, m, l);
-  }
-  // the warp's (max, sum-exp) per head: lanes that share tig & 1 hold pairs of the same two heads
-  for (int hh = 0; hh < nh; ++hh)
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      float mx = m[hh][e];
-#pragma unroll
-      for (int o = 2; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      float sum = l[hh][e] * fast_exp2((m[hh][e] - (mx == -INFINITY ? 0.f : mx)) * LOG2E);
-#pragma unroll
-      for (int o = 2; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      if (lane < 2) {
-        sh.red_m[warp][4 * hh + 2 * lane + e] = mx;
-        sh.red_l[warp][4 * hh + 2 * lane + e] = sum;
-      }
-    }
+// B fragment of q for the fp16 tier / residual: column n = g is head n; qh: that head's row at channel 2*tig (null: none)
+__device__ __forceinline__ uint2 k_plain_q(const uint32_t* qh, int kt) {
+  return qh ? make_uint2(qh[8 * kt], qh[8 * kt + 4]) : make_uint2(0u, 0u);
 }
 
-// fp16 tier, channel-major rows [D][n]: four tokens per 8-byte slot, no scales; B = q exactly.
-__device__ __forceinline__ void k_f16_span(const DecodeParams& P, const TierDev& T, KShared& sh, int bh, int b, int kvh,
-                                           int span_t0) {
+// fp16 tier, channel-major rows [D][n]: four tokens per 8-byte slot, no scales; B = q exactly.  64 tokens by the whole CTA,
+// a warp for 32 of the channels: all of a warp's loads are in flight together (one warp for all channels went through
+// eight dependent rounds of them); the partial logits meet in shared memory.
+__device__ __forceinline__ void k_f16_block(const DecodeParams& P, const TierDev& T, KShared& sh, const Where& w, const uint32_t* qh,
+                                            int t0, float& m, float& l) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tig = lane & 3;
   const int n = T.n_k;
   const int64_t nslot = n / K_SLOT;
-  const uint2* base = reinterpret_cast<const uint2*>(T.k_data) + static_cast<int64_t>(bh) * D * nslot;
+  const uint2* base = reinterpret_cast<const uint2*>(T.k_data) + static_cast<int64_t>(w.bh) * D * nslot;
   int64_t sl[2];
 #pragma unroll
-  for (int r = 0; r < 2; ++r) sl[r] = min(static_cast<int64_t>(span_t0 / K_SLOT + r * 8 + g), nslot - 1);
+  for (int r = 0; r < 2; ++r) sl[r] = min(static_cast<int64_t>(t0 / K_SLOT + r * 8 + g), nslot - 1);
   float acc[K_SLOT][4];
 #pragma unroll
   for (int i = 0; i < K_SLOT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-#pragma unroll 2
-  for (int kt = 0; kt < 8; ++kt) {
-    uint2 w[4][2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int kt = 2 * warp + k;
+    uint2 v[4][2];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int ch = 16 * kt + 8 * (e >> 1) + 2 * tig + (e & 1);
 #pragma unroll
-      for (int r = 0; r < 2; ++r) w[e][r] = ld_stream(base + ch * nslot + sl[r]);
+      for (int r = 0; r < 2; ++r) v[e][r] = ld_stream(base + ch * nslot + sl[r]);
     }
-    const uint2 bq = sh.qb[0][kt][lane];
+    const uint2 bq = k_plain_q(qh, kt);
     // token i of a slot: halfs (x.lo, x.hi, y.lo, y.hi); pair the same token of two channel rows
     uint32_t a[K_SLOT][4];
 #pragma unroll
     for (int q = 0; q < 2; ++q)
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
-        const uint2 wa = w[2 * q][r], wb = w[2 * q + 1][r];
-        a[0][q * 2 + r] = __byte_perm(wa.x, wb.x, 0x5410);
-        a[1][q * 2 + r] = __byte_perm(wa.x, wb.x, 0x7632);
-        a[2][q * 2 + r] = __byte_perm(wa.y, wb.y, 0x5410);
-        a[3][q * 2 + r] = __byte_perm(wa.y, wb.y, 0x7632);
+        const uint2 va = v[2 * q][r], vb = v[2 * q + 1][r];
+        a[0][q * 2 + r] = pack_lo16(va.x, vb.x);
+        a[1][q * 2 + r] = pack_hi16(va.x, vb.x);
+        a[2][q * 2 + r] = pack_lo16(va.y, vb.y);
+        a[3][q * 2 + r] = pack_hi16(va.y, vb.y);
       }
 #pragma unroll
     for (int i = 0; i < K_SLOT; ++i) mma16816(acc[i], a[i][0], a[i][1], a[i][2], a[i][3], bq.x, bq.y);
   }
-  float* tile = sh.w[warp].u.tile;
+  float* part = sh.u.tile[warp];
+  if (tig < 2) {  // columns 0-3 are heads, 4-7 are empty
 #pragma unroll
-  for (int r = 0; r < 2; ++r)
+    for (int r = 0; r < 2; ++r)
 #pragma unroll
-    for (int e = 0; e < 2; ++e)
+      for (int e = 0; e < 2; ++e)
 #pragma unroll
-      for (int i = 0; i < K_SLOT; ++i)
-        tile[((r * 8 + g) * K_SLOT + i) * K_TROW + 2 * tig + e] = acc[i][r * 2 + e] * P.scale;
+        for (int i = 0; i < K_SLOT; ++i) part[((r * 8 + g) * K_SLOT + i) * K_TROW + 2 * tig + e] = acc[i][r * 2 + e] * P.scale;
+  }
+  __syncthreads();
+  // 16 tokens per warp: the sum goes into the first partial tile
+  constexpr int MINE = K_SPAN / KWARPS * K_TROW;
+  float* tile = sh.u.tile[0] + warp * MINE;
+  for (int i = lane; i < MINE; i += 32) {
+    float v = tile[i];
+#pragma unroll
+    for (int o = 1; o < KWARPS; ++o) v += sh.u.tile[o][warp * MINE + i];
+    tile[i] = v;
+  }
   __syncwarp();
-  k_write_tile(P, tile, min(K_SPAN, n - span_t0), T.k_idx + span_t0, 0, b, kvh, sh.red_m[warp], sh.red_l[warp]);
+  const int first = t0 + warp * (K_SPAN / KWARPS);
+  k_write_tile(P, w, tile, min(K_SPAN / KWARPS, n - first), T.k_idx + first, 0, m, l);
+  __syncthreads();
 }
 
 // fp16 residual window, token-major [r][D]: A fragments are read directly; one 16-token tile per warp.
-__device__ __forceinline__ void k_residual_tile(const DecodeParams& P, const TierDev& T, KShared& sh, int bh, int b,
-                                                int kvh, int tile_t0) {
+__device__ __forceinline__ void k_residual_tile(const DecodeParams& P, const TierDev& T, KShared& sh, const Where& w, const uint32_t* qh, int tile_t0, float& m, float& l) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tig = lane & 3;
   const int n = T.n_k;
-  const __half* base = reinterpret_cast<const __half*>(T.k_data) + static_cast<int64_t>(bh) * n * D;
+  const __half* base = reinterpret_cast<const __half*>(T.k_data) + static_cast<int64_t>(w.bh) * n * D;
   const int t[2] = {min(tile_t0 + g, n - 1), min(tile_t0 + g + 8, n - 1)};
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  uint32_t a[8][4];
 #pragma unroll
-  for (int kt = 0; kt < 8; ++kt)
+  for (int kt = 0; kt < 8; ++kt) {
+    uint32_t a[4];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       const __half* p = base + static_cast<int64_t>(t[r]) * D + 16 * kt + 2 * tig;
-      a[kt][r] = *reinterpret_cast<const uint32_t*>(p);
-      a[kt][2 + r] = *reinterpret_cast<const uint32_t*>(p + 8);
+      a[r] = *reinterpret_cast<const uint32_t*>(p);
+      a[2 + r] = *reinterpret_cast<const uint32_t*>(p + 8);
     }
-#pragma unroll
-  for (int kt = 0; kt < 8; ++kt) {
-    const uint2 bq = sh.qb[0][kt][lane];
-    mma16816(acc, a[kt][0], a[kt][1], a[kt][2], a[kt][3], bq.x, bq.y);
+    const uint2 bq = k_plain_q(qh, kt);
+    mma16816(acc, a[0], a[1], a[2], a[3], bq.x, bq.y);
   }
-  float* tile = sh.w[warp].u.tile;
+  float* tile = sh.u.tile[warp];
+  if (tig < 2) {
 #pragma unroll
-  for (int r = 0; r < 2; ++r)
+    for (int r = 0; r < 2; ++r)
 #pragma unroll
-    for (int e = 0; e < 2; ++e) tile[(r * 8 + g) * K_TROW + 2 * tig + e] = acc[r * 2 + e] * P.scale;
+      for (int e = 0; e < 2; ++e) tile[(r * 8 + g) * K_TROW + 2 * tig + e] = acc[r * 2 + e] * P.scale;
+  }
   __syncwarp();
-  k_write_tile(P, tile, min(16, n - tile_t0), nullptr, static_cast<int64_t>(P.L) - n + tile_t0, b, kvh, sh.red_m[warp],
-               sh.red_l[warp]);
+  k_write_tile(P, w, tile, min(16, n - tile_t0), nullptr, static_cast<int64_t>(P.L) - n + tile_t0, m, l);
 }
 
+// ONE_TIER: no CTA has units of two tiers.
+template <bool ONE_TIER>
 __global__ void __launch_bounds__(KTHREADS, K_MIN_CTAS) k_pass_kernel(const __grid_constant__ DecodeParams P) {
   extern __shared__ __align__(128) unsigned char k_smem[];
   KShared& sh = *reinterpret_cast<KShared*>(k_smem);
-  const int chunk = blockIdx.y, bh = blockIdx.x;  // (batch, head) fastest: neighbouring CTAs run the same tier code
-  const int b = bh / P.H, kvh = bh - b * P.H;
+  const Where w = where(P);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tig = lane & 3;
 
   // Let the V pass of this call (launched with programmatic stream serialisation) start its own
   // prologue - V words, index lists, scale/zero tiles - as soon as SM resources free up; it waits for
   // this grid to finish (griddepcontrol.wait) before it touches the logits or the softmax pairs.
   asm volatile("griddepcontrol.launch_dependents;");
-  if (tid < KWARPS * MAX_REP) {
-    (&sh.red_m[0][0])[tid] = -INFINITY;
-    (&sh.red_l[0][0])[tid] = 0.f;
-  }
-
-  int ti = HQKV_NUM_TIERS;
-#pragma unroll
-  for (int t = 0; t < HQKV_NUM_TIERS; ++t)
-    if (chunk >= P.tier[t].k_chunk0 && chunk < P.tier[t + 1].k_chunk0) ti = t;
-  const TierDev& T = P.tier[ti];
-  const int chunk_t0 = (chunk - T.k_chunk0) * T.k_chunk_tokens;
-  const bool plain = ti == HQKV_NUM_TIERS || T.bits == 16;
-
-  // B fragments of q: rows are channels 16*kt + 2*tig + (0,1 | 8,9), column n = g is a query head of
-  // this kv head (see KShared::qb); warp hh stores its half.  q is the only input that an earlier
-  // kernel of the stream may still be writing, so it is read after griddepcontrol.wait.
-  const int nh = (!plain && P.rep > 4) ? 2 : 1;
-  auto load_q = [&]() {
-    if (warp < nh) {
-      const int head = plain ? g : 4 * warp + (g & 3);
-      const __half* qh = P.q + (static_cast<int64_t>(b) * P.nh_q + kvh * P.rep + head) * D + 2 * tig;
-      uint2 qf[8];
-#pragma unroll
-      for (int kt = 0; kt < 8; ++kt) {
-        qf[kt] = make_uint2(0u, 0u);
-        if (head < P.rep) {
-          qf[kt].x = *reinterpret_cast<const uint32_t*>(qh + 16 * kt);
-          qf[kt].y = *reinterpret_cast<const uint32_t*>(qh + 16 * kt + 8);
-        }
-      }
-#pragma unroll
-      for (int kt = 0; kt < 8; ++kt) sh.qb[warp][kt][lane] = qf[kt];
+  float m = -INFINITY, l = 0.f;  // this lane's softmax pair: head tig
+  bool first = true;
+  auto plain = [&](int ti, int t0, int t1) {  // fp16 tier, residual window
+    const TierDev& T = P.tier[ti];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!first) __syncthreads();
+    first = false;
+    const uint32_t* q =
+        g < P.r4 ? reinterpret_cast<const uint32_t*>(P.q + (static_cast<int64_t>(w.b) * P.nh_q + w.h0 + g) * D) + tig : nullptr;
+    if (ti == 0) {
+      for (int t = t0; t < t1; t += K_SPAN) k_f16_block(P, T, sh, w, q, t, m, l);
+    } else {
+      for (int t = t0 + warp * 16; t < t1; t += KWARPS * 16) k_residual_tile(P, T, sh, w, q, t, m, l);
     }
   };
-
-  if (plain) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    load_q();
-    __syncthreads();
-    const int chunk_end = min(chunk_t0 + T.k_chunk_tokens, T.n_k);
-    if (ti == HQKV_NUM_TIERS) {
-      const int t0 = chunk_t0 + warp * 16;  // residual chunks are KWARPS * 16 tokens
-      if (t0 < chunk_end) k_residual_tile(P, T, sh, bh, b, kvh, t0);
-    } else {
-      const int t0 = chunk_t0 + warp * K_SPAN;
-      if (t0 < chunk_end) k_f16_span(P, T, sh, bh, b, kvh, t0);
-    }
-  } else if (T.bits == 8) {
-    k_chunk<8>(P, T, sh, bh, b, kvh, chunk_t0, nh, load_q);
-  } else if (T.bits == 4) {
-    k_chunk<4>(P, T, sh, bh, b, kvh, chunk_t0, nh, load_q);
-  } else if (T.bits == 2) {
-    k_chunk<2>(P, T, sh, bh, b, kvh, chunk_t0, nh, load_q);
+  int t0, t1;
+  if constexpr (ONE_TIER) {
+    const int ti = only_share<false>(P, t0, t1);
+    if (ti == 1) k_run<8>(P, P.tier[1], sh, w, t0, t1, m, l, first);
+    else if (ti == 2) k_run<4>(P, P.tier[2], sh, w, t0, t1, m, l, first);
+    else if (ti == 3) k_run<2>(P, P.tier[3], sh, w, t0, t1, m, l, first);
+    else if (ti == 4) k_run<1>(P, P.tier[4], sh, w, t0, t1, m, l, first);
+    else plain(ti, t0, t1);
   } else {
-    k_chunk<1>(P, T, sh, bh, b, kvh, chunk_t0, nh, load_q);
+    if (share_of<false>(P, 1, 8, t0, t1)) k_run<8>(P, P.tier[1], sh, w, t0, t1, m, l, first);
+    if (share_of<false>(P, 2, 4, t0, t1)) k_run<4>(P, P.tier[2], sh, w, t0, t1, m, l, first);
+    if (share_of<false>(P, 3, 2, t0, t1)) k_run<2>(P, P.tier[3], sh, w, t0, t1, m, l, first);
+    if (share_of<false>(P, 4, 1, t0, t1)) k_run<1>(P, P.tier[4], sh, w, t0, t1, m, l, first);
+    for (int ti = 0; ti <= HQKV_NUM_TIERS; ti += HQKV_NUM_TIERS)
+      if (share_of<false>(P, ti, 16, t0, t1)) plain(ti, t0, t1);
+  }
+  // the warp's (max, sum-exp) per head: the eight lanes with the same tig
+  {
+    float mx = m;
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    float sum = l * fast_exp2((m - (mx == -INFINITY ? 0.f : mx)) * LOG2E);
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane < MAX_R4) {
+      sh.v.red.m[warp][tig] = mx;
+      sh.v.red.l[warp][tig] = sum;
+    }
   }
 
-  // the output accumulators of this (batch, kv head) start from zero in every call (the V pass, which
-  // adds into them, starts after this grid has finished); both branches above have passed their
+  // the output accumulators of these heads start from zero in every call (the V pass, which
+  // adds into them, starts after this grid has finished); everything above has passed its
   // griddepcontrol.wait, so the previous call is done with them
-  if (chunk == 0) {
-    double* accum = P.v_acc + static_cast<int64_t>(bh) * P.rep * D;
-    for (int i = tid; i < P.rep * D; i += KTHREADS) accum[i] = 0.0;
+  if (blockIdx.y == 0) {
+    double* accum = P.v_acc + (static_cast<int64_t>(w.b) * P.nh_q + w.h0) * D;
+    for (int i = tid; i < P.r4 * D; i += KTHREADS) accum[i] = 0.0;
   }
   // (max, sum) of this CTA per head from the warps' pairs
   __syncthreads();
-  if (tid < MAX_REP) {
-    float m = sh.red_m[0][tid], l = sh.red_l[0][tid];
-    for (int w = 1; w < KWARPS; ++w) softmax_merge(m, l, sh.red_m[w][tid], sh.red_l[w][tid]);
-    P.k_part[(static_cast<int64_t>(bh) * P.nk_chunks + chunk) * MAX_REP + tid] = make_float2(m, l);
+  if (tid < P.r4) {
+    float m = sh.v.red.m[0][tid], l = sh.v.red.l[0][tid];
+#pragma unroll
+    for (int i = 1; i < KWARPS; ++i) softmax_merge(m, l, sh.v.red.m[i][tid], sh.v.red.l[i][tid]);
+    P.k_part[(static_cast<int64_t>(w.bvh) * P.r4 + tid) * P.nk_ctas + blockIdx.y] = make_float2(m, l);
   }
 }
 
 // ------------------------------------------------------------------------------------------------
 // v_pass
 // ------------------------------------------------------------------------------------------------
-// V tier, token-major rows of 128 channels.  Every warp of a CTA owns one TILE of consecutive tokens
-// (8 KB of codes at 8 / 4 bits = 64 / 128 tokens, 4 KB at 2 bits = 128 tokens) with their scales,
-// zeros and logical positions, all copied global -> shared with cp.async before anything else.
+// V tier, token-major rows of 128 channels.  Every warp of a CTA walks TILES of consecutive tokens of one tier on its own
+// (4 KB of codes at 8 / 4 bits = 32 / 64 tokens, 64 tokens at 2 / 1 bits) and keeps the output of all 128 channels x
+// four heads in its accumulators from tile to tile, so nothing but the end of the kernel needs the other warps.
 // The contraction runs over tokens, 16 per step.  ldmatrix.trans over 8 token rows x 16 bytes hands
 // lane (g, tig) the 16-bit block g (2 / 4 / 8 channels) of tokens 2*tig and 2*tig+1 in one register:
 // the two K-neighbours of an m16n8k16 A fragment.  As in the K pass the codes enter the tensor pipe
-// as fp16 subnormals (one AND per pair of codes) and the scale - here per token and 32-channel
+// as fp16 subnormals (one AND per pair of codes) and the scale - here per token and channel
 // group - is folded into the B operand: out[h][c] = sum_t (p_t * scale_t,G) * code_t,c + sum_t p_t *
-// zero_t,G, with p*scale carried exactly as hi + lo and B columns 0-3 / 4-7 holding the two channel
-// groups of a 64-channel half.  The zero term is one small MMA per step (rows = groups).
-constexpr int V_MIN_CTAS = 4;  // CTAs per SM the V pass is compiled for
+// zero_t,G, with p*scale carried exactly as hi + lo in neighbouring columns (2-bit pieces of 64 channels: columns are
+// two channel groups, hi and lo are two MMAs).
+// A tile has two phases.  In the first a lane computes exp(logit - max) of four tokens for two heads (one at 8 bits),
+// writes the probabilities out, and leaves the finished B operand - p*scale, hi and lo, of every head, token pair and
+// channel group - in shared memory in the order the MMAs want it: computed once, where forming it per step in every
+// lane that holds a column cost twice the arithmetic plus the packing of scales.  The second phase is ldmatrix, masks
+// and MMAs.
+// Codes are streamed through ONE tile buffer: the copy of a 16-token step of the next tile is issued when this tile's
+// step has been consumed, so a whole tile's work lies between a request and its use.
+#ifndef HQKV_VM
+#define HQKV_VM 4
+#endif
+constexpr int V_MIN_CTAS = HQKV_VM;  // CTAs per SM the V pass is compiled for (102 registers; shared memory allows five)
 constexpr int VWARPS = 4;
 constexpr int VTHREADS = VWARPS * 32;
-constexpr int V_MAX_TT = 128;                 // tokens per tile at most
-constexpr int V_PROW = V_MAX_TT + 8;          // halfs per staged probability row (pitch 68 words: rows 4 banks apart)
+constexpr int V_ST = 72 * 4;                       // bytes per 16-token step of a B plane (64 words + 8: no bank conflicts)
+constexpr int V_PLANE = 4 * V_ST + 32;             // B plane of one channel group: 4 steps (+ 8 words, likewise)
 
 template <int BITS>
 struct VTile {
   static constexpr int PITCH = 16 * BITS;                  // bytes per token row: 128, 64, 32, 16
-  static constexpr int TOKENS = BITS == 8 ? 64 : 128;
+  static constexpr int TOKENS = BITS == 8 ? 32 : 64;
   static constexpr int STEPS = TOKENS / 16;
   static constexpr int NPIECE = PITCH / 16;                // 16-byte pieces per row: 8, 4, 2, 1
+  static constexpr int HPL = BITS == 8 ? 1 : 2;            // heads per lane in the first phase
+  static constexpr int STEP_BYTES = 16 * PITCH;
   static __device__ __forceinline__ uint32_t offset(uint32_t row, uint32_t c) {
     if constexpr (PITCH == 128) {
       return row * 128u + ((c ^ (row & 7u)) << 4);
@@ -944,399 +1054,627 @@ struct VTile {
     }
   }
 };
+static_assert(VWARPS * VTile<8>::TOKENS == unit_tokens(8) && VWARPS * VTile<4>::TOKENS == unit_tokens(4), "a unit is a tile per warp");
 
-struct VWarpShared {
-  union {
-    unsigned char codes[8192];
-    float red[4][D];            // partial output of the last walk over the tile (heads of that half)
-  } u;
-  union {
-    struct {
-      int64_t pos[V_MAX_TT];    // logical positions of the tile's tokens
-      __half p[4][V_PROW];      // exp(logit - max) of heads 0-3
-    } a;
-    float red0[4][D];           // eight query heads per kv head: partial output of the first walk
-  } v;
-  __half p_hi[4][V_PROW];       // heads 4-7
-  __half s[V_MAX_TT * 4];       // scales as in memory: [token][group]
-  __half z[V_MAX_TT * 4];
-  float zt[4][MAX_REP];         // sum_t p*zero per channel group and head
+struct VTileShared {
+  unsigned char codes[4096];
+  unsigned char s[512];            // scales as in memory: [token][group]
+  unsigned char z[512];
+  unsigned char b[4 * V_PLANE];    // [group][step][2 * head + (hi, lo)][tig]{tokens 2tig, +1 | +8, +9}
+  unsigned char p[4 * 128];        // [step][head][tig]{the same token pairs}: B operand of the zero term
+  unsigned char zt[4 * 128];       // zeros, [group][step pair][tig]{even step, odd step, even step +8, odd step +8}
 };
-static_assert(sizeof(float) * 4 * D <= sizeof(int64_t) * V_MAX_TT + sizeof(__half) * 4 * V_PROW, "red0 fits its union");
+static_assert(sizeof(VTileShared) % 128 == 0, "tile buffers stay aligned");
+constexpr int V_STD = 2048;        // Gaussian-codebook tier (1 bit: 1 KB of codes): std in the same order, behind the codes
+struct VWarpShared {
+  VTileShared t;
+  float red[MAX_R4][D];            // partial output of the tiers that are done
+};
 
 // importance row emitted by the V pass: staging limits (positions + per-head halfs live in the warps' tile buffers)
-constexpr int HS_TOKENS = 512;   // tokens of the largest chunk
+constexpr int HS_TOKENS = 512;   // tokens per round
 constexpr int HS_HEADS = 32;     // query heads it is built for (beyond that a separate launch sums the heads)
 struct VShared {
-  float gm[MAX_REP], gl[MAX_REP];          // global max / sum of this kv head's query heads
-  float wm[VWARPS][MAX_REP], wl[VWARPS][MAX_REP];
+  float gm[MAX_R4], ginv[MAX_R4];          // max * log2(e) and 1 / sum of the query heads
   unsigned is_last;
-  unsigned pad_[3 + 12];
-  VWarpShared w[VWARPS];
+  unsigned pad_[3 + 4];
+  alignas(128) VWarpShared w[VWARPS];  // (lane addresses are formed by XOR within 128 bytes)
 };
 
-// A fragment registers from one ldmatrix quad R[0..3] = sources of fragment registers a0..a3
-// (a0: row g, tokens 2tig,2tig+1; a1: row g+8; a2 / a3: the same rows, tokens +8).
-//   field f of a 16-bit block as the fp16 subnormal code * 2^(k-24); VField<BITS>::shift(f) gives k.
+// field f of a 16-bit block as the fp16 subnormal code * 2^(k-24), k = v_shift(f)
 template <int BITS>
-struct VField {
-  static constexpr int N = BITS == 8 ? 2 : 4;  // fields taken from one register per fragment row
-  static __host__ __device__ constexpr int shift(int f) {
-    return BITS == 8 ? 0 : BITS == 4 ? 4 * (f & 1) : BITS == 2 ? 2 * f : f;
-  }
-};
-template <int BITS>
-__device__ __forceinline__ uint32_t v_field(uint32_t r, uint32_t r_shr8, int f) {
-  if constexpr (BITS == 8) {
-    return f == 0 ? (r & 0x00FF00FFu) : __byte_perm(r, 0u, 0x4341);
-  } else if constexpr (BITS == 4) {
-    return (f < 2 ? r : r_shr8) & (0x000F000Fu << (4 * (f & 1)));
-  } else {
-    return r & (0x00030003u << (2 * f));  // 2 bits: fields 0-3 of r (row g) or of r >> 8 (row g+8)
-  }
-}
+__host__ __device__ constexpr int v_shift(int f) { return BITS == 8 ? 0 : BITS * f; }
 
-// Request a tile: positions, scales, zeros in the oldest commit group, then the codes in four groups
-// of a quarter of the steps each.  ntok = valid tokens (a multiple of 32), ng = channel groups.
+// The tiles of one warp: tokens t0 + warp * TOKENS, then every fourth tile up to t1.
 template <int BITS>
-__device__ __forceinline__ void v_tile_request(const TierDev& T, VWarpShared& ws, int bh, int tile_t0, int ntok, int ng) {
+struct VRun {
+  const unsigned char *codes, *s, *z;   // this lane's first 16 (8) bytes of the next tile to request
+  const int64_t* idx;                   // the lane's first token of the next tile whose positions are wanted
+  int left;                             // tokens from the next tile to request on (may be <= 0)
+};
+
+// Copy step st of the next tile; dst = where this lane's first piece goes in step 0 of the buffer.
+template <int BITS>
+__device__ __forceinline__ void v_request_step(const VRun<BITS>& r, uint32_t dst, int st, bool whole) {
   using TL = VTile<BITS>;
   const int lane = threadIdx.x & 31;
-  const int64_t tok0 = static_cast<int64_t>(bh) * T.n_v + tile_t0;
+  constexpr int N = (TL::STEP_BYTES + 511) / 512, RPI = 32 / TL::NPIECE;  // copies per lane: 4, 2, 1, 1; rows per copy
+  const unsigned char* src = r.codes + st * TL::STEP_BYTES;
+  dst += st * TL::STEP_BYTES;
+  if (TL::STEP_BYTES < 512 && lane >= TL::STEP_BYTES / 16) return;
 #pragma unroll
-  for (int j = 0; j < TL::TOKENS / 32; ++j) {
-    const int t = lane + 32 * j;
-    if (t < ntok) cp_async_8(&ws.v.a.pos[t], T.v_idx + tile_t0 + t);
-  }
-  // scale / zero rows are ng halfs per token, contiguous over the tile: 8-byte pieces
-  {
-    const int bytes = ntok * ng * 2;
-    const unsigned char* s = reinterpret_cast<const unsigned char*>(T.v_scale + tok0 * ng);
-    const unsigned char* z = reinterpret_cast<const unsigned char*>(T.v_zero + tok0 * ng);
+  for (int i = 0; i < N; ++i)
+    // (four rows on, bit 2 of the row changes: the other half of the swizzle at 8 bits)
+    if (whole || 16 * st + i * RPI + lane / TL::NPIECE < r.left)
+      cp_async_16((BITS == 8 ? dst ^ ((i & 1) * 64u) : dst) + i * 512, src + i * 512);
+}
+// scale / zero rows of a tile: ng halfs per token, contiguous, 8-byte pieces
+template <int BITS>
+__device__ __forceinline__ void v_request_scales(const VRun<BITS>& r, uint32_t s, uint32_t z, int ng2) {
+  const int lane = threadIdx.x & 31;
+  const int bytes = min(VTile<BITS>::TOKENS, r.left) * ng2;
 #pragma unroll
-    for (int j = 0; j < V_MAX_TT * 4 * 2 / (32 * 8); ++j) {
-      const int o = (lane + 32 * j) * 8;
-      if (o < bytes) {
-        cp_async_8(reinterpret_cast<unsigned char*>(ws.s) + o, s + o);
-        cp_async_8(reinterpret_cast<unsigned char*>(ws.z) + o, z + o);
-      }
+  for (int o = 0; o < VTile<BITS>::TOKENS * 8; o += 256)
+    if (o + 8 * lane < bytes) {
+      cp_async_8(s + o + 8 * lane, r.s + o);
+      cp_async_8(z + o + 8 * lane, r.z + o);
     }
-  }
-  cp_async_commit();
-  const unsigned char* src = reinterpret_cast<const unsigned char*>(T.v_data) + tok0 * TL::PITCH;
-  constexpr int PIECES = TL::TOKENS * TL::NPIECE;  // 512 (256 at 2 bits, 128 at 1 bit)
-  constexpr int PER_Q = PIECES / 4 / 32;           // copies per lane and quarter: 4 (2, 1)
-#pragma unroll
-  for (int quarter = 0; quarter < 4; ++quarter) {
-#pragma unroll
-    for (int i = 0; i < PER_Q; ++i) {
-      const int id = (quarter * PER_Q + i) * 32 + lane;
-      const int row = id / TL::NPIECE, c = id % TL::NPIECE;
-      if (row < ntok) cp_async_16(ws.u.codes + TL::offset(row, c), src + static_cast<int64_t>(id) * 16);
-    }
-    cp_async_commit();
-  }
 }
 
-// exp(logit - max) of the tile's tokens for heads h0..h0+3 into prow[0..3][token], and the
-// normalised probabilities into the output row; the gathers of four heads are in flight together.
-template <int TOKENS>
-__device__ __forceinline__ void v_tile_probs(const DecodeParams& P, const VShared& sh, const int64_t* pos_s, __half (*prow)[V_PROW],
-                                             int b, int kvh, int h0, int ntok, int64_t first_pos) {
-  const int lane = threadIdx.x & 31;
-  const int rep = P.rep;
-  constexpr int PER = TOKENS / 32;
-  uint32_t pos[PER];
-#pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    const int t = lane + 32 * j;
-    pos[j] = t < ntok ? (pos_s ? static_cast<uint32_t>(pos_s[t]) : static_cast<uint32_t>(first_pos + t)) : 0u;
+// First phase, lane map: 16-token step st, token pairs 2tq, 2tq+1 and +8, +9 of it, heads h0 .. h0 + HPL - 1.
+template <int BITS>
+struct VLane {
+  int st, tq, h0, tok;
+  __device__ __forceinline__ VLane() {
+    const int lane = threadIdx.x & 31;
+    constexpr int QUADS = VTile<BITS>::TOKENS / 4;
+    const int quad = lane & (QUADS - 1);
+    st = quad >> 2;
+    tq = quad & 3;
+    tok = 16 * st + 2 * tq;
+    h0 = (lane / QUADS) * VTile<BITS>::HPL;
   }
-  bool ok[PER];
+};
+__device__ __forceinline__ constexpr int v_tok(int j) { return (j & 1) + 8 * (j >> 1); }
+
+// positions (low words) of the lane's four tokens, `none` beyond the tier
+__device__ __forceinline__ void v_positions(uint32_t (&pos)[4], const int64_t* idx, int ntok, int tok, uint32_t none) {
 #pragma unroll
-  for (int j = 0; j < PER; ++j) ok[j] = lane + 32 * j < ntok && HQKV_INDEX_OK(pos[j], P.L);
+  for (int j = 0; j < 4; ++j) {
+    pos[j] = none;
+    if (tok + v_tok(j) < ntok) pos[j] = __ldg(reinterpret_cast<const uint32_t*>(idx + v_tok(j)));
+  }
+}
+// logits (or given weights) of the lane's tokens and heads
+template <int HPL>
+__device__ __forceinline__ void v_gather(const DecodeParams& P, const Where& w, float (&x)[4][HPL], uint32_t (&pos)[4], int h0) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (pos[j] != 0xFFFFFFFFu && !HQKV_INDEX_OK(pos[j], P.L)) pos[j] = 0xFFFFFFFFu;
   if (P.probs_in) {
-    // caller-supplied weights: staged as they are, nothing is written back
-#pragma unroll 1
-    for (int hh = 0; hh < 4; ++hh) {
-      const int h = h0 + hh;
-      const unsigned short* row = reinterpret_cast<const unsigned short*>(P.probs_in) +
-                                  (static_cast<int64_t>(b) * P.nh_q + kvh * rep + min(h, rep - 1)) * P.L;
 #pragma unroll
-      for (int j = 0; j < PER; ++j)
-        prow[hh][lane + 32 * j] = __ushort_as_half((h < rep && ok[j]) ? __ldcg(row + pos[j]) : static_cast<unsigned short>(0));
-    }
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int h = 0; h < HPL; ++h) {
+        const unsigned short* row = reinterpret_cast<const unsigned short*>(P.probs_in) +
+                                    (static_cast<int64_t>(w.b) * P.nh_q + w.h0 + h0 + h) * P.L;
+        x[j][h] = pos[j] != 0xFFFFFFFFu && h0 + h < P.r4 ? __half2float(__ushort_as_half(__ldcg(row + pos[j]))) : 0.f;
+      }
     return;
   }
-  float x[4][PER];
+  const float* base = P.logits + static_cast<int64_t>(w.bvh) * P.L * P.r4 + h0;
+  if (P.r4 == MAX_R4) {
 #pragma unroll
-  for (int hh = 0; hh < 4; ++hh) {
-    const int h = min(h0 + hh, rep - 1);
-    const float* row = P.logits + (static_cast<int64_t>(b) * P.nh_q + kvh * rep + h) * P.L;
-#pragma unroll
-    for (int j = 0; j < PER; ++j) x[hh][j] = ok[j] ? __ldcg(row + pos[j]) : -INFINITY;
-  }
-#pragma unroll
-  for (int hh = 0; hh < 4; ++hh) {
-    const int h = h0 + hh;
-    const bool on = h < rep;
-    const float mh = on ? sh.gm[h] * LOG2E : 0.f, inv = on ? 1.f / sh.gl[h] : 0.f;
-    __half* wrow = P.weights + (static_cast<int64_t>(b) * P.nh_q + kvh * rep + min(h, rep - 1)) * P.L;
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      const int t = lane + 32 * j;
-      const float e = on ? fast_exp2(fmaf(x[hh][j], LOG2E, -mh)) : 0.f;  // exp2(-inf) = 0 beyond the tile
-      prow[hh][t] = __float2half_rn(e);
-      if (on && ok[j]) wrow[pos[j]] = __float2half_rn(e * inv);
+    for (int j = 0; j < 4; ++j) {
+      const float* p = base + static_cast<int64_t>(pos[j]) * MAX_R4;
+      if constexpr (HPL == 2) {
+        const float2 v = pos[j] != 0xFFFFFFFFu ? __ldcg(reinterpret_cast<const float2*>(p)) : make_float2(-INFINITY, -INFINITY);
+        x[j][0] = v.x;
+        x[j][1] = v.y;
+      } else {
+        x[j][0] = pos[j] != 0xFFFFFFFFu ? __ldcg(p) : -INFINITY;
+      }
     }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int h = 0; h < HPL; ++h)
+        x[j][h] = pos[j] != 0xFFFFFFFFu && h0 + h < P.r4 ? __ldcg(base + static_cast<int64_t>(pos[j]) * P.r4 + h) : -INFINITY;
   }
 }
 
-// One tile of a quantised V tier for half hh of the heads: acc[mt] = M-tile mt of the output
-// (channels x heads, see the channel map in v_tile_store), zacc = zero term rows.
+// Two neighbouring tokens' probabilities of one head (packed) to their positions.
+__device__ __forceinline__ void v_store_pair(__half* row, uint32_t p0, uint32_t p1, uint32_t packed, bool even) {
+  if (even) {  // consecutive positions that start on a 4-byte boundary
+    *reinterpret_cast<uint32_t*>(row + p0) = packed;
+    return;
+  }
+  if (p0 != 0xFFFFFFFFu) row[p0] = __ushort_as_half(static_cast<unsigned short>(packed));
+  if (p1 != 0xFFFFFFFFu) row[p1] = __ushort_as_half(static_cast<unsigned short>(packed >> 16));
+}
+
+// First phase of a tile (see above), any number of heads, tokens, groups; given weights.  x: logits of the lane's tokens.
+// Not inlined: partial tiles and unusual calls, whose code would only be in the way of the other tiles'.
 template <int BITS>
-__device__ __forceinline__ void v_tile_walk(const DecodeParams& P, VWarpShared& ws, const __half (*prow)[V_PROW], int ntok,
-                                            float (&acc)[8][4], float (&zacc)[4], bool normal) {
+__device__ __noinline__ void v_prepare_any(const DecodeParams& P, const Where& w, const VShared& sh, uint32_t tile,
+                                           const float (&x)[4][VTile<BITS>::HPL], const uint32_t (&pos)[4], int ntok, bool normal) {
+  const VLane<BITS> L;
   using TL = VTile<BITS>;
-  const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-  const int ng_shift = 7 - P.gv_shift;  // log2(groups per token): 2, 1, 0
-  // ldmatrix row address of this lane for step 0, quad 0: matrices (token octet, piece) =
-  //   8/4 bits: (0, c), (0, c'), (1, c), (1, c');  2 bits: (0, 0), (0, 1), (1, 0), (1, 1)
-  // with (c, c') = the quad's two pieces: 4 bits (2pp, 2pp+1); 8 bits (4q+u, 4q+2+u)
-  const int mi = lane >> 3, rr = lane & 7;
-  const int lm_row = 8 * (mi >> 1) + rr;
-  // as a B column this lane is n = g: head (n & 3) of this half, channel group of channels
-  // 64q + 32*(n >> 2) for quad set q
-  const __half* pr = &prow[g & 3][2 * tig];
-  int gq[2];
+  constexpr int HPL = TL::HPL;
+  using S = VTileShared;
+  const uint32_t s_a = tile + offsetof(S, s), z_a = tile + offsetof(S, z), b_a = tile + offsetof(S, b), p_a = tile + offsetof(S, p),
+                 zt_a = tile + offsetof(S, zt), nt_a = tile + V_STD;
+  uint32_t p2[HPL][2];  // [head][token pair]
 #pragma unroll
-  for (int q = 0; q < 2; ++q) gq[q] = (64 * q + 32 * (g >> 2)) >> P.gv_shift;
-  const int zg = (g & 3) & ((1 << ng_shift) - 1);  // zero-term row g = group g (rows beyond ng repeat)
-#pragma unroll
-  for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-  zacc[0] = zacc[1] = zacc[2] = zacc[3] = 0.f;
-  float sacc[4] = {0.f, 0.f, 0.f, 0.f};  // Gaussian-codebook tier: sum_t p * std per channel group
-
-  const int nsteps = ntok >> 4;
-#pragma unroll 1
-  for (int st = 0; st < nsteps; ++st) {
-    const int t0 = st * 16;
-    // B operands: p pairs of tokens (2tig, 2tig+1) and (+8, +9); scales of the same tokens
-    const uint32_t p0 = *reinterpret_cast<const uint32_t*>(pr + t0);
-    const uint32_t p1 = *reinterpret_cast<const uint32_t*>(pr + t0 + 8);
-    const __half* sb = ws.s + ((t0 + 2 * tig) << ng_shift);
-    const __half* zb = ws.z + ((t0 + 2 * tig) << ng_shift);
-    uint32_t bh_[2][2], bl_[2][2];
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const __half2 s0 = u32_as_h2(pack_lo16(__half_as_ushort(sb[gq[q]]), __half_as_ushort(sb[(1 << ng_shift) + gq[q]])));
-      const __half2 s1 = u32_as_h2(pack_lo16(__half_as_ushort(sb[(8 << ng_shift) + gq[q]]),
-                                             __half_as_ushort(sb[(9 << ng_shift) + gq[q]])));
-      const __half2 h0 = __hmul2(u32_as_h2(p0), s0), h1 = __hmul2(u32_as_h2(p1), s1);
-      bh_[q][0] = h2_as_u32(h0);
-      bh_[q][1] = h2_as_u32(h1);
-      bl_[q][0] = h2_as_u32(__hfma2(u32_as_h2(p0), s0, __hneg2(h0)));  // exact remainder
-      bl_[q][1] = h2_as_u32(__hfma2(u32_as_h2(p1), s1, __hneg2(h1)));
-    }
-    {  // zero term: A rows = channel groups, exact fp16 x fp16 products
-      const uint32_t a0 = pack_lo16(__half_as_ushort(zb[zg]), __half_as_ushort(zb[(1 << ng_shift) + zg]));
-      const uint32_t a2 = pack_lo16(__half_as_ushort(zb[(8 << ng_shift) + zg]), __half_as_ushort(zb[(9 << ng_shift) + zg]));
-      mma16816(zacc, a0, 0u, a2, 0u, p0, p1);
-    }
-    if (BITS == 1 && normal) {
-      const uint32_t a0 = pack_lo16(__half_as_ushort(sb[zg]), __half_as_ushort(sb[(1 << ng_shift) + zg]));
-      const uint32_t a2 = pack_lo16(__half_as_ushort(sb[(8 << ng_shift) + zg]), __half_as_ushort(sb[(9 << ng_shift) + zg]));
-      mma16816(sacc, a0, 0u, a2, 0u, p0, p1);
-    }
-    const unsigned char* rowp = ws.u.codes;
-    if constexpr (BITS == 1) {
-      // block = 16 channels, four blocks per 64-channel half c; lane g reads block 4c + (g & 3) of tokens
-      // 2tig, 2tig+1 (+8, +9) with 2-byte loads; rows g / g+8 of M-tile f are channels 4*(g>>2) + f and +8
-      const unsigned char* tb = rowp + (t0 + 2 * tig) * 16 + 2 * (g & 3);
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const uint32_t r0 = pack_lo16(*reinterpret_cast<const uint16_t*>(tb + 8 * c), *reinterpret_cast<const uint16_t*>(tb + 8 * c + 16));
-        const uint32_t r1 = pack_lo16(*reinterpret_cast<const uint16_t*>(tb + 8 * c + 128), *reinterpret_cast<const uint16_t*>(tb + 8 * c + 144));
-        const uint32_t lo0 = r0 >> (4 * (g >> 2)), hi0 = lo0 >> 8, lo1 = r1 >> (4 * (g >> 2)), hi1 = lo1 >> 8;
-#pragma unroll
-        for (int f = 0; f < 4; ++f) {
-          const uint32_t msk = 0x00010001u << f;
-          mma16816(acc[4 * c + f], lo0 & msk, hi0 & msk, lo1 & msk, hi1 & msk, bh_[c][0], bh_[c][1]);
-        }
-#pragma unroll
-        for (int f = 0; f < 4; ++f) {
-          const uint32_t msk = 0x00010001u << f;
-          mma16816(acc[4 * c + f], lo0 & msk, hi0 & msk, lo1 & msk, hi1 & msk, bl_[c][0], bl_[c][1]);
-        }
-      }
-    } else if constexpr (BITS == 2) {
-      uint32_t R[4];
-      ldmatrix_x4_trans(R, rowp + TL::offset(t0 + lm_row, mi & 1));
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const uint32_t lo0 = R[c], hi0 = R[c] >> 8, lo1 = R[2 + c], hi1 = R[2 + c] >> 8;
-        uint32_t fa[4][4];
-#pragma unroll
-        for (int f = 0; f < 4; ++f) {
-          fa[f][0] = v_field<2>(lo0, 0u, f), fa[f][1] = v_field<2>(hi0, 0u, f);
-          fa[f][2] = v_field<2>(lo1, 0u, f), fa[f][3] = v_field<2>(hi1, 0u, f);
-        }
-#pragma unroll
-        for (int f = 0; f < 4; ++f) mma16816(acc[4 * c + f], fa[f][0], fa[f][1], fa[f][2], fa[f][3], bh_[c][0], bh_[c][1]);
-#pragma unroll
-        for (int f = 0; f < 4; ++f) mma16816(acc[4 * c + f], fa[f][0], fa[f][1], fa[f][2], fa[f][3], bl_[c][0], bl_[c][1]);
-      }
-    } else if constexpr (BITS == 4) {
-#pragma unroll
-      for (int pp = 0; pp < 2; ++pp) {
-        uint32_t R[4], S[4];
-        ldmatrix_x4_trans(R, rowp + TL::offset(t0 + lm_row, 2 * pp + (mi & 1)));
-#pragma unroll
-        for (int k = 0; k < 4; ++k) S[k] = R[k] >> 8;
-        uint32_t fa[4][4];
-#pragma unroll
-        for (int f = 0; f < 4; ++f)
-#pragma unroll
-          for (int k = 0; k < 4; ++k) fa[f][k] = v_field<4>(R[k], S[k], f);
-#pragma unroll
-        for (int f = 0; f < 4; ++f) mma16816(acc[4 * pp + f], fa[f][0], fa[f][1], fa[f][2], fa[f][3], bh_[pp][0], bh_[pp][1]);
-#pragma unroll
-        for (int f = 0; f < 4; ++f) mma16816(acc[4 * pp + f], fa[f][0], fa[f][1], fa[f][2], fa[f][3], bl_[pp][0], bl_[pp][1]);
-      }
+  for (int h = 0; h < HPL; ++h) {
+    const int head = L.h0 + h;
+    const bool on = head < P.r4;
+    if (P.probs_in) {
+      p2[h][0] = pack_f16x2(x[0][h], x[1][h]);
+      p2[h][1] = pack_f16x2(x[2][h], x[3][h]);
     } else {
+      const float mh = sh.gm[on ? head : 0], inv = sh.ginv[on ? head : 0];
+      float e[4];
 #pragma unroll
-      for (int q = 0; q < 2; ++q)
+      for (int j = 0; j < 4; ++j) e[j] = on ? fast_exp2(fmaf(x[j][h], LOG2E, -mh)) : 0.f;  // exp2(-inf) = 0 beyond the tile
+      p2[h][0] = pack_f16x2(e[0], e[1]);
+      p2[h][1] = pack_f16x2(e[2], e[3]);
+      if (on) {
+        const int64_t at = (static_cast<int64_t>(w.b) * P.nh_q + w.h0 + head) * P.L;
+        __half* row = P.weights + at;
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          uint32_t R[4];
-          ldmatrix_x4_trans(R, rowp + TL::offset(t0 + lm_row, 4 * q + u + 2 * (mi & 1)));
-          uint32_t fa[2][4];
-#pragma unroll
-          for (int f = 0; f < 2; ++f)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) fa[f][k] = v_field<8>(R[k], 0u, f);
-#pragma unroll
-          for (int f = 0; f < 2; ++f) mma16816(acc[4 * q + 2 * u + f], fa[f][0], fa[f][1], fa[f][2], fa[f][3], bh_[q][0], bh_[q][1]);
-#pragma unroll
-          for (int f = 0; f < 2; ++f) mma16816(acc[4 * q + 2 * u + f], fa[f][0], fa[f][1], fa[f][2], fa[f][3], bl_[q][0], bl_[q][1]);
+        for (int k = 0; k < 2; ++k) {
+          const uint32_t a = pos[2 * k], b = pos[2 * k + 1];
+          const bool even = b == a + 1 && b != 0 && ((reinterpret_cast<uintptr_t>(row + a) & 3) == 0);
+          v_store_pair(row, a, b, pack_f16x2(e[2 * k] * inv, e[2 * k + 1] * inv), even);
         }
+      }
+    }
+    sts64(p_a + L.st * 128 + (L.h0 + h) * 32 + L.tq * 8, p2[h][0], p2[h][1]);
+  }
+  // scales and zeros of the two token pairs, one word per channel group
+  const int ng = D >> P.gv_shift;
+  uint32_t s2[2][4], z2[2][4];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int t = L.tok + 8 * k;
+    if (ng == 4) {
+      const uint4 sv = lds128(s_a + t * 8), zv = lds128(z_a + t * 8);
+      s2[k][0] = pack_lo16(sv.x, sv.z), s2[k][1] = pack_hi16(sv.x, sv.z), s2[k][2] = pack_lo16(sv.y, sv.w), s2[k][3] = pack_hi16(sv.y, sv.w);
+      z2[k][0] = pack_lo16(zv.x, zv.z), z2[k][1] = pack_hi16(zv.x, zv.z), z2[k][2] = pack_lo16(zv.y, zv.w), z2[k][3] = pack_hi16(zv.y, zv.w);
+    } else if (ng == 2) {
+      const uint2 sv = lds64(s_a + t * 4), zv = lds64(z_a + t * 4);
+      s2[k][0] = pack_lo16(sv.x, sv.y), s2[k][1] = pack_hi16(sv.x, sv.y);
+      z2[k][0] = pack_lo16(zv.x, zv.y), z2[k][1] = pack_hi16(zv.x, zv.y);
+    } else {
+      s2[k][0] = lds32(s_a + t * 2), z2[k][0] = lds32(z_a + t * 2);
+    }
+    if (ntok < TL::TOKENS) {  // the scales of tokens beyond the tile are not there
+      const uint32_t keep = (t < ntok ? 0xFFFFu : 0u) | (t + 1 < ntok ? 0xFFFF0000u : 0u);
+#pragma unroll
+      for (int G = 0; G < 4; ++G) {
+        s2[k][G] &= keep;
+        z2[k][G] &= keep;
+      }
     }
   }
-  if (BITS == 1 && normal) {  // value = std * C * (2 code - 1) + mean: the code-free term is sum_t p (mean - C std)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) zacc[i] = fmaf(-HQKV_NORMAL1_CENTER, sacc[i], zacc[i]);
+  for (int G = 0; G < 4; ++G) {
+    if (G < ng) {
+      const uint32_t bp = b_a + G * V_PLANE + L.st * V_ST + L.h0 * 64 + L.tq * 8;
+#pragma unroll
+      for (int h = 0; h < HPL; ++h) {
+        const uint32_t h0 = h2_mul(p2[h][0], s2[0][G]), h1 = h2_mul(p2[h][1], s2[1][G]);
+        sts64(bp + h * 64, h0, h1);
+        sts64(bp + h * 64 + 32, h2_rem(p2[h][0], s2[0][G], h0), h2_rem(p2[h][1], s2[1][G], h1));
+      }
+      // A operand of the zero term: one of the lanes that share these tokens writes it
+      if (BITS == 8 ? L.h0 == G : L.h0 == 2 * (G & 1)) {
+        const uint32_t zp = G * 128 + (L.st >> 1) * 64 + L.tq * 16 + (L.st & 1) * 4;
+        sts32(zt_a + zp, z2[0][G]);
+        sts32(zt_a + zp + 8, z2[1][G]);
+        if (BITS == 1 && normal) {
+          sts32(nt_a + zp, s2[0][G]);
+          sts32(nt_a + zp + 8, s2[1][G]);
+        }
+      }
+    }
   }
 }
 
-// Accumulators of one walk -> red[head of this half][channel] (every element has exactly one owner).
-//   8 / 4 bits: rows 0-7 and 8-15 of an M-tile are two different channel groups: lanes tig 0,1 own row g
-//               (columns 0-3), lanes tig 2,3 own row g+8 (columns 4-7).
-//   2 bits:     rows g and g+8 are channels of the same block: lanes with (g < 4) == (tig < 2) own both.
-// M-tile -> channels:  8 bits  mt = 4q + 2u + f : row g = 64q + 16u + 2g + f,  row g+8 = +32
-//                      4 bits  mt = 4pp + f     : row g = 64pp + 4g + f,        row g+8 = +32
-//                      2 bits  mt = 4c + f      : row g = 64c + 8g + f,         row g+8 = +4
-//                      1 bit   mt = 4c + f      : row g = 64c + 16(g&3) + 4(g>>2) + f, row g+8 = +8
-//                              (owned by the lanes with ((g & 3) < 2) == (tig < 2))
+// The same for a whole tile, four query heads and 128 >> GV channel groups known at compile time.  mh / inv: max *
+// log2(e) and 1 / sum of the lane's heads, wrow: their rows of probabilities.
+template <int BITS, int GV>
+__device__ __forceinline__ void v_prepare(uint32_t tile, const float (&x)[4][VTile<BITS>::HPL], const uint32_t (&pos)[4],
+                                          const VLane<BITS>& L, const float (&mh)[VTile<BITS>::HPL],
+                                          const float (&inv)[VTile<BITS>::HPL], __half* const (&wrow)[VTile<BITS>::HPL], bool normal) {
+  using TL = VTile<BITS>;
+  using S = VTileShared;
+  constexpr int HPL = TL::HPL, NG = D >> GV;
+  uint32_t s2[2][NG], z2[2][NG];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const uint32_t at = tile + offsetof(S, s) + (L.tok + 8 * k) * NG * 2, to_z = offsetof(S, z) - offsetof(S, s);
+    if constexpr (NG == 4) {
+      const uint4 sv = lds128(at), zv = lds128(at + to_z);
+      s2[k][0] = pack_lo16(sv.x, sv.z), s2[k][1] = pack_hi16(sv.x, sv.z), s2[k][2] = pack_lo16(sv.y, sv.w), s2[k][3] = pack_hi16(sv.y, sv.w);
+      z2[k][0] = pack_lo16(zv.x, zv.z), z2[k][1] = pack_hi16(zv.x, zv.z), z2[k][2] = pack_lo16(zv.y, zv.w), z2[k][3] = pack_hi16(zv.y, zv.w);
+    } else if constexpr (NG == 2) {
+      const uint2 sv = lds64(at), zv = lds64(at + to_z);
+      s2[k][0] = pack_lo16(sv.x, sv.y), s2[k][1] = pack_hi16(sv.x, sv.y);
+      z2[k][0] = pack_lo16(zv.x, zv.y), z2[k][1] = pack_hi16(zv.x, zv.y);
+    } else {
+      s2[k][0] = lds32(at), z2[k][0] = lds32(at + to_z);
+    }
+  }
+  uint32_t p2[HPL][2], n2[HPL][2];  // [head][token pair]: exp(logit - max), probability
+#pragma unroll
+  for (int h = 0; h < HPL; ++h)
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const float e0 = fast_exp2(fmaf(x[2 * k][h], LOG2E, -mh[h])), e1 = fast_exp2(fmaf(x[2 * k + 1][h], LOG2E, -mh[h]));
+      p2[h][k] = pack_f16x2(e0, e1);
+      n2[h][k] = pack_f16x2(e0 * inv[h], e1 * inv[h]);
+    }
+  const bool adjacent = pos[1] == pos[0] + 1 && pos[3] == pos[2] + 1;
+#pragma unroll
+  for (int h = 0; h < HPL; ++h) {
+    __half *a = wrow[h] + pos[0], *b = wrow[h] + pos[2];
+    if (adjacent && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 3) == 0) {
+      *reinterpret_cast<uint32_t*>(a) = n2[h][0];
+      *reinterpret_cast<uint32_t*>(b) = n2[h][1];
+    } else {
+      a[0] = __ushort_as_half(static_cast<unsigned short>(n2[h][0]));
+      wrow[h][pos[1]] = __ushort_as_half(static_cast<unsigned short>(n2[h][0] >> 16));
+      b[0] = __ushort_as_half(static_cast<unsigned short>(n2[h][1]));
+      wrow[h][pos[3]] = __ushort_as_half(static_cast<unsigned short>(n2[h][1] >> 16));
+    }
+    sts64(tile + offsetof(S, p) + L.st * 128 + (L.h0 + h) * 32 + L.tq * 8, p2[h][0], p2[h][1]);
+  }
+  const uint32_t bp = tile + offsetof(S, b) + L.st * V_ST + L.h0 * 64 + L.tq * 8;
+  const uint32_t zp = tile + offsetof(S, zt) + (L.st >> 1) * 64 + L.tq * 16 + (L.st & 1) * 4;
+#pragma unroll
+  for (int G = 0; G < NG; ++G) {
+#pragma unroll
+    for (int h = 0; h < HPL; ++h) {
+      const uint32_t h0 = h2_mul(p2[h][0], s2[0][G]), h1 = h2_mul(p2[h][1], s2[1][G]);
+      sts64(bp + G * V_PLANE + h * 64, h0, h1);
+      sts64(bp + G * V_PLANE + h * 64 + 32, h2_rem(p2[h][0], s2[0][G], h0), h2_rem(p2[h][1], s2[1][G], h1));
+    }
+    // A operand of the zero term: one of the lanes that share these tokens writes it
+    if (BITS == 8 ? L.h0 == G : L.h0 == 2 * (G & 1)) {
+      sts32(zp + G * 128, z2[0][G]);
+      sts32(zp + G * 128 + 8, z2[1][G]);
+      if (BITS == 1 && normal) {
+        sts32(zp + G * 128 + V_STD - offsetof(S, zt), s2[0][G]);
+        sts32(zp + G * 128 + V_STD - offsetof(S, zt) + 8, s2[1][G]);
+      }
+    }
+  }
+}
+
+// Four query heads: positions and logits of the lane's tokens without conditions (position 0 stands in beyond the tier).
+template <int HPL>
+__device__ __forceinline__ void v_gather4(float (&x)[4][HPL], const uint32_t (&pos)[4], const float* base) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float* p = base + static_cast<uint64_t>(pos[j]) * MAX_R4;
+    if constexpr (HPL == 2) {
+      const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
+      x[j][0] = v.x;
+      x[j][1] = v.y;
+    } else {
+      x[j][0] = __ldcg(p);
+    }
+  }
+}
+
+// Second phase: one 16-token step of a tile into acc[M-tile] (channels x columns, see v_store_output).  lm = this lane's
+// ldmatrix row of the step, piece 0 or 1 (1 bit: its first 2-byte block); bl = the step in B plane 0 at this lane's column.
+template <int BITS, int GV>
+__device__ __forceinline__ void v_step(float (&acc)[8][4], uint32_t lm, uint32_t bl, int gv_runtime) {
+  const int gv_shift = GV ? GV : gv_runtime;
+  if constexpr (BITS >= 4) {
+    uint32_t R[4];
+#pragma unroll
+    for (int cb = 0; cb < 4; ++cb) {   // 32 channels: one channel group, two M-tiles
+      uint32_t a[2][4];
+      if constexpr (BITS == 8) {
+        ldmatrix_x4_trans(R, lm ^ (cb * 32u));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          a[0][k] = R[k] & 0x00FF00FFu;
+          a[1][k] = __byte_perm(R[k], 0u, 0x4341);
+        }
+      } else {
+        if ((cb & 1) == 0) ldmatrix_x4_trans(R, lm ^ (cb * 16u));
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const uint32_t r = R[2 * k + (cb & 1)], rs = r >> 8;
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            a[i][2 * k] = r & (0x000F000Fu << (4 * i));
+            a[i][2 * k + 1] = rs & (0x000F000Fu << (4 * i));
+          }
+        }
+      }
+      const uint2 b = lds64(bl + (cb >> (gv_shift - 5)) * V_PLANE);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) mma16816(acc[2 * cb + i], a[i][0], a[i][1], a[i][2], a[i][3], b.x, b.y);
+    }
+  } else {
+    const int g = (threadIdx.x & 31) >> 2;
+    uint32_t R[4];
+    if constexpr (BITS == 2) ldmatrix_x4_trans(R, lm);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {      // 64 channels: two channel groups of 32 in neighbouring columns
+      uint32_t lo0, lo1;
+      if constexpr (BITS == 2) {
+        lo0 = R[c], lo1 = R[2 + c];
+      } else {  // block 4c + (g & 3) of tokens 2tig, 2tig+1 (+8, +9) with 2-byte loads
+        const uint32_t tb = lm + 8 * c;
+        lo0 = pack_lo16(lds16(tb), lds16(tb + 16)) >> (4 * (g >> 2));
+        lo1 = pack_lo16(lds16(tb + 128), lds16(tb + 144)) >> (4 * (g >> 2));
+      }
+      const uint32_t hi0 = lo0 >> 8, hi1 = lo1 >> 8;
+      // column n = g: head n >> 1, channel group of channels 64c + 32*(n & 1)
+      const uint32_t bp = bl + ((2 * c + (g & 1)) >> (gv_shift - 5)) * V_PLANE;
+      const uint2 bh = lds64(bp), bl2 = lds64(bp + 32);
+      uint32_t a[4][4];
+#pragma unroll
+      for (int f = 0; f < 4; ++f) {
+        const uint32_t m = BITS == 2 ? 0x00030003u << (2 * f) : 0x00010001u << f;
+        a[f][0] = lo0 & m, a[f][1] = hi0 & m, a[f][2] = lo1 & m, a[f][3] = hi1 & m;
+      }
+#pragma unroll
+      for (int f = 0; f < 4; ++f) mma16816(acc[4 * c + f], a[f][0], a[f][1], a[f][2], a[f][3], bh.x, bh.y);
+#pragma unroll
+      for (int f = 0; f < 4; ++f) mma16816(acc[4 * c + f], a[f][0], a[f][1], a[f][2], a[f][3], bl2.x, bl2.y);
+    }
+  }
+}
+
+// Accumulators and zero term (lane: channel group g, head tig) added to red[head tig][channel] (`fresh`: nothing is in there yet).
+//   8 / 4 bits: M-tile 2*cb + i: rows g / g+8 = channels 32cb + 2g + i / + 16 (8 bits), 32cb + 4g + i / + 2 (4 bits);
+//               a head's neighbouring columns are hi and lo
+//   2 bits:     M-tile 4c + f: 64c + 8g + f / + 4;   1 bit: 64c + 16(g&3) + 4(g>>2) + f / + 8;   the columns are two
+//               channel groups, a row keeps its own
 template <int BITS>
-__device__ __forceinline__ void v_tile_store(float (*red)[D], const float (&acc)[8][4], float gain) {
+__device__ __forceinline__ void v_store_output(float (*red)[D], const float (&acc)[8][4], float gain, float zt, int gv_shift, bool fresh) {
   const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-  const int hp = tig & 1, r = tig >> 1;
 #pragma unroll
   for (int mt = 0; mt < 8; ++mt) {
-    const int f = BITS == 8 ? (mt & 1) : (mt & 3);
-    const float unscale = static_cast<float>(1 << (24 - VField<BITS>::shift(f))) * gain;
-    if constexpr (BITS <= 2) {
-      const bool mine = BITS == 2 ? (g < 4) == (tig < 2) : ((g & 3) < 2) == (tig < 2);
-      if (mine) {
-        const int ch = 64 * (mt >> 2) + (BITS == 2 ? 8 * g : 16 * (g & 3) + 4 * (g >> 2)) + f;
-        constexpr int UP = BITS == 2 ? 4 : 8;  // channel distance of row g+8
+    const int f = BITS >= 4 ? mt & 1 : mt & 3;
+    const float unscale = static_cast<float>(1 << 24) / static_cast<float>(1 << v_shift<BITS>(f)) * gain;
+    // the zero term of the M-tile's channels: 32-channel block mt >> 1 (8 / 4 bits), or the one this lane's rows are in
+    const int block = BITS >= 4 ? mt >> 1 : 2 * (mt >> 2) + (BITS == 2 ? g >> 2 : (g & 3) >> 1);
+    const float z = __shfl_sync(0xffffffffu, zt, 4 * (block >> (gv_shift - 5)) + tig);
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          red[2 * hp + e][ch] = acc[mt][e] * unscale;
-          red[2 * hp + e][ch + UP] = acc[mt][2 + e] * unscale;
-        }
+    for (int r = 0; r < 2; ++r) {
+      const float* a = &acc[mt][2 * r];
+      int ch;
+      float v;
+      if constexpr (BITS >= 4) {
+        ch = 32 * (mt >> 1) + (BITS == 8 ? 2 * g + 16 * r : 4 * g + 2 * r) + f;
+        v = a[0] + a[1];
+      } else {
+        ch = 64 * (mt >> 2) + (BITS == 2 ? 8 * g + 4 * r : 16 * (g & 3) + 4 * (g >> 2) + 8 * r) + f;
+        v = (BITS == 2 ? g >> 2 : (g & 3) >> 1) ? a[1] : a[0];
       }
-    } else {
-      const int ch = BITS == 8 ? 64 * (mt >> 2) + 16 * ((mt >> 1) & 1) + 2 * g + f + 32 * r
-                               : 64 * (mt >> 2) + 4 * g + f + 32 * r;
-#pragma unroll
-      for (int e = 0; e < 2; ++e) red[2 * hp + e][ch] = (r ? acc[mt][2 + e] : acc[mt][e]) * unscale;
+      const float y = fmaf(v, unscale, z);
+      red[tig][ch] = fresh ? y : red[tig][ch] + y;
     }
   }
 }
 
-// Everything a warp does for its tile of a quantised V tier.
-template <int BITS>
-__device__ __forceinline__ void v_tile(const DecodeParams& P, const TierDev& T, VShared& sh, VWarpShared& ws, int b,
-                                       int kvh, int ntok, int nh) {
+// Everything a warp does for its tiles of tokens [t0, t1) of a quantised V tier.  UNROLL: steps of the inner loop (one where
+// a CTA's code is that of several tiers: they run side by side on an SM and the instruction cache does not hold more).  `fold` folds the
+// K pass's softmax pairs (once per CTA; all its warps take part).
+template <int BITS, int GV, int UNROLL, typename Fold>
+__device__ __forceinline__ void v_run(const DecodeParams& P, const TierDev& T, VShared& sh, const Where& w, int t0, int t1,
+                                      Fold fold, bool& fresh) {
   using TL = VTile<BITS>;
-  const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-  cp_async_wait<4>();  // positions, scales, zeros
-  __syncwarp();
-  for (int hh = 0; hh < nh; ++hh)
-    v_tile_probs<TL::TOKENS>(P, sh, ws.v.a.pos, hh ? ws.p_hi : ws.v.a.p, b, kvh, 4 * hh, ntok, 0);
-  cp_async_wait<0>();  // the gathers above took at least as long as the codes
-  __syncwarp();
-  for (int hh = 0; hh < nh; ++hh) {
-    float acc[8][4], zacc[4];
-    const bool normal = BITS == 1 && T.normal != 0;
-    v_tile_walk<BITS>(P, ws, hh ? ws.p_hi : ws.v.a.p, ntok, acc, zacc, normal);
-    __syncwarp();  // all lanes are done with the codes (last walk) or with p of heads 0-3 (first of two)
-    v_tile_store<BITS>(hh + 1 < nh ? ws.v.red0 : ws.u.red, acc, normal ? 2.f * HQKV_NORMAL1_CENTER : 1.f);
-    if (g < 4 && tig < 2) {
-      ws.zt[g][4 * hh + 2 * tig] = zacc[0];
-      ws.zt[g][4 * hh + 2 * tig + 1] = zacc[1];
+  using S = VTileShared;
+  constexpr int STRIDE = VWARPS * TL::TOKENS;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tig = lane & 3;
+  VWarpShared& ws = sh.w[warp];
+  const uint32_t tile = smem_u32(&ws.t);
+  const uint32_t codes = tile + offsetof(S, codes), b_a = tile + offsetof(S, b), s_a = tile + offsetof(S, s), z_a = tile + offsetof(S, z);
+  constexpr bool FAST = GV != 0;
+  constexpr uint32_t NONE = FAST ? 0u : 0xFFFFFFFFu;
+  const int gv_shift = GV ? GV : P.gv_shift;
+  const int ng2 = (D >> gv_shift) * 2;
+  const bool normal = BITS == 1 && T.normal != 0;
+  const VLane<BITS> L;
+  const int first = t0 + warp * TL::TOKENS;
+  const int64_t tok0 = static_cast<int64_t>(w.bh) * T.n_v + first;
+  VRun<BITS> r;
+  r.codes = reinterpret_cast<const unsigned char*>(T.v_data) + tok0 * TL::PITCH + lane * 16;
+  r.s = reinterpret_cast<const unsigned char*>(T.v_scale) + tok0 * ng2 + lane * 8;
+  r.z = reinterpret_cast<const unsigned char*>(T.v_zero) + tok0 * ng2 + lane * 8;
+  r.idx = T.v_idx + first + L.tok;
+  r.left = t1 - first;
+  // lane addresses: first piece of a step's copy; ldmatrix row - matrices (token octet, piece) (0, c), (0, c'), (1, c),
+  // (1, c') - or 2-byte block; column of the B planes
+  const uint32_t dst = codes + TL::offset(lane / TL::NPIECE, lane % TL::NPIECE);
+  const uint32_t lm = BITS == 1 ? codes + 2 * tig * 16 + 2 * (g & 3) : codes + TL::offset(8 * (lane >> 4) + (lane & 7), (lane >> 3) & 1);
+  const uint32_t bl = b_a + (BITS >= 4 ? lane * 8 : (g >> 1) * 64 + tig * 8);
+  auto advance = [&]() {
+    r.codes += STRIDE * TL::PITCH;
+    r.s += STRIDE * ng2;
+    r.z += STRIDE * ng2;
+    r.left -= STRIDE;
+  };
+  __syncwarp();  // (the buffers may have served another tier)
+  // requests that read only the cache go out before the K pass is known to be complete
+  v_request_scales<BITS>(r, s_a, z_a, ng2);
+  cp_async_commit();
+#pragma unroll
+  for (int st = 0; st < TL::STEPS; ++st) {
+    v_request_step<BITS>(r, dst, st, false);
+    cp_async_commit();
+  }
+  uint32_t pos[4];
+  v_positions(pos, r.idx, r.left, L.tok, NONE);
+  advance();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  float x[4][TL::HPL];
+  const float* lrow = P.logits + static_cast<int64_t>(w.bvh) * P.L * MAX_R4 + L.h0;
+  auto gather = [&]() {
+    if constexpr (FAST) v_gather4<TL::HPL>(x, pos, lrow);
+    else v_gather<TL::HPL>(P, w, x, pos, L.h0);
+  };
+  gather();
+  fold();
+  float mh[TL::HPL], inv[TL::HPL];
+  __half* wrow[TL::HPL];
+  if constexpr (FAST) {
+#pragma unroll
+    for (int h = 0; h < TL::HPL; ++h) {
+      mh[h] = sh.gm[L.h0 + h];
+      inv[h] = sh.ginv[L.h0 + h];
+      wrow[h] = P.weights + (static_cast<int64_t>(w.b) * P.nh_q + w.h0 + L.h0 + h) * P.L;
     }
   }
+  float acc[8][4], za[4] = {0.f, 0.f, 0.f, 0.f}, zb[4] = {0.f, 0.f, 0.f, 0.f};
+  float na[4] = {0.f, 0.f, 0.f, 0.f}, nb[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+  const int zg = g & ((D >> gv_shift) - 1);  // zero-term row g = group g (rows beyond the groups repeat)
+#pragma unroll 1
+  for (int left = t1 - first; left > 0; left -= STRIDE) {
+    const int ntok = min(TL::TOKENS, left);
+    uint32_t next[4];
+    r.idx += STRIDE;
+    v_positions(next, r.idx, r.left, L.tok, NONE);
+    cp_async_wait<TL::STEPS>();  // scales and zeros (the codes of the tile may still be on their way)
+    __syncwarp();
+    if (FAST && ntok == TL::TOKENS) {
+      if constexpr (FAST) v_prepare<BITS, GV>(tile, x, pos, L, mh, inv, wrow, normal);
+    } else {
+      float xa[4][TL::HPL];
+      uint32_t pa[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const bool in = L.tok + v_tok(j) < ntok;
+        pa[j] = in ? pos[j] : 0xFFFFFFFFu;
+#pragma unroll
+        for (int h = 0; h < TL::HPL; ++h) xa[j][h] = in ? x[j][h] : P.probs_in ? 0.f : -INFINITY;
+      }
+      v_prepare_any<BITS>(P, w, sh, tile, xa, pa, ntok, normal);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) pos[j] = next[j];
+    gather();
+    __syncwarp();  // the B operand is complete, the scale buffers are free
+    v_request_scales<BITS>(r, s_a, z_a, ng2);
+    cp_async_commit();
+#pragma unroll
+    for (int sp = 0; sp < TL::STEPS / 2; ++sp) {
+      const uint4 z4 = lds128(tile + offsetof(S, zt) + zg * 128 + sp * 64 + tig * 16);
+      const uint2 pe = lds64(tile + offsetof(S, p) + (2 * sp) * 128 + (g >> 1) * 32 + tig * 8);
+      const uint2 po = lds64(tile + offsetof(S, p) + (2 * sp + 1) * 128 + (g >> 1) * 32 + tig * 8);
+      mma16816(za, z4.x, z4.y, z4.z, z4.w, pe.x, pe.y);   // rows 0-7: the even step's tokens
+      mma16816(zb, z4.x, z4.y, z4.z, z4.w, po.x, po.y);   // rows 8-15: the odd step's
+      if (BITS == 1 && normal) {
+        const uint4 n4 = lds128(tile + V_STD + zg * 128 + sp * 64 + tig * 16);
+        mma16816(na, n4.x, n4.y, n4.z, n4.w, pe.x, pe.y);
+        mma16816(nb, n4.x, n4.y, n4.z, n4.w, po.x, po.y);
+      }
+    }
+    const bool whole = r.left >= TL::TOKENS;
+  #pragma unroll UNROLL
+    for (int st = 0; st < TL::STEPS; ++st) {
+      cp_async_wait<TL::STEPS>();
+      __syncwarp();
+      v_step<BITS, GV>(acc, lm + st * TL::STEP_BYTES, bl + st * V_ST, gv_shift);
+      // (the MMAs have used the step's codes, and keep the warp together: no lane still reads them)
+      v_request_step<BITS>(r, dst, st, whole);
+      cp_async_commit();
+    }
+    advance();
+    __syncwarp();
+  }
+  cp_async_wait<0>();
+  __syncwarp();
+  // value = std * C * (2 code - 1) + mean: the code-free term is sum_t p (mean - C std)
+  const float zt = za[0] + zb[2] + (normal ? -HQKV_NORMAL1_CENTER * (na[0] + nb[2]) : 0.f);  // channel group g, head tig
+  v_store_output<BITS>(ws.red, acc, normal ? 2.f * HQKV_NORMAL1_CENTER : 1.f, zt, gv_shift, fresh);
+  fresh = false;
 }
 
 // fp16 tier and residual window, token-major rows [n][D] halfs: one 16-token step per warp straight
-// from global memory; B = p.  Writes the partial outputs of all (up to eight) heads.
-__device__ __forceinline__ void v_plain_tile(const DecodeParams& P, const TierDev& T, VShared& sh, VWarpShared& ws, int bh,
-                                             int b, int kvh, int t0, int ntok, bool is_res) {
+// from global memory; B = p, column n = head n.
+__device__ __forceinline__ void v_plain_tile(const DecodeParams& P, const TierDev& T, VShared& sh, VWarpShared& ws, const Where& w,
+                                             int t0, int ntok, bool is_res) {
   const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-  const int rep = P.rep;
-  const uint4* base = reinterpret_cast<const uint4*>(T.v_data) + static_cast<int64_t>(bh) * T.n_v * 16;
-  uint4 w[4][2];
+  const uint4* base = reinterpret_cast<const uint4*>(T.v_data) + static_cast<int64_t>(w.bh) * T.n_v * 16;
+  uint4 v[4][2];
 #pragma unroll
   for (int p = 0; p < 4; ++p) {
     const int tl = 2 * tig + (p & 1) + (p >> 1) * 8;
     const int64_t tok = t0 + min(tl, ntok - 1);
 #pragma unroll
-    for (int s = 0; s < 2; ++s) w[p][s] = ld_stream(base + tok * 16 + s * 8 + g);
+    for (int s = 0; s < 2; ++s) v[p][s] = ld_stream(base + tok * 16 + s * 8 + g);
   }
-  const int64_t first_pos = static_cast<int64_t>(P.L) - T.n_v + t0;
-  for (int hh = 0; hh < (rep > 4 ? 2 : 1); ++hh)
-    v_tile_probs<32>(P, sh, is_res ? nullptr : T.v_idx + t0, hh ? ws.p_hi : ws.v.a.p, b, kvh, 4 * hh, ntok, first_pos);
+  __half* ps = reinterpret_cast<__half*>(ws.t.p);  // [head][16 tokens]
+  {
+    const int t = lane & 15;
+    uint32_t pos = 0xFFFFFFFFu;
+    if (t < ntok) pos = is_res ? static_cast<uint32_t>(P.L - T.n_v + t0 + t) : __ldg(reinterpret_cast<const uint32_t*>(T.v_idx + t0 + t));
+    if (pos != 0xFFFFFFFFu && !HQKV_INDEX_OK(pos, P.L)) pos = 0xFFFFFFFFu;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int h = 2 * (lane >> 4) + i;
+      const bool on = h < P.r4 && pos != 0xFFFFFFFFu;
+      const int64_t at = (static_cast<int64_t>(w.b) * P.nh_q + w.h0 + h) * P.L + pos;
+      __half e = __float2half_rn(0.f);
+      if (on) {
+        if (P.probs_in) {
+          e = __ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(P.probs_in) + at));
+        } else {
+          const float x = __ldcg(P.logits + (static_cast<int64_t>(w.bvh) * P.L + pos) * P.r4 + h);
+          const float f = fast_exp2(fmaf(x, LOG2E, -sh.gm[h]));
+          e = __float2half_rn(f);
+          P.weights[at] = __float2half_rn(f * sh.ginv[h]);
+        }
+      }
+      ps[h * 16 + t] = e;
+    }
+  }
   __syncwarp();
   float acc[8][4];
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
   uint32_t b0 = 0u, b1 = 0u;
-  if (g < rep) {
-    const __half* pr = g < 4 ? ws.v.a.p[g] : ws.p_hi[g - 4];
-    b0 = *reinterpret_cast<const uint32_t*>(pr + 2 * tig);
-    b1 = *reinterpret_cast<const uint32_t*>(pr + 2 * tig + 8);
+  if (g < MAX_R4) {
+    b0 = *reinterpret_cast<const uint32_t*>(ps + g * 16 + 2 * tig);
+    b1 = *reinterpret_cast<const uint32_t*>(ps + g * 16 + 2 * tig + 8);
   }
-  const __half2 none[2][2] = {};
-  mma_words<16, 8>(acc, w, none, none, b0, b1);
-  __syncwarp();
-  // M-tile mt, slot s: channel 8*(8s + g) + mt; columns 2tig, 2tig+1 = heads
+  auto word = [](const uint4& u, int s) { return s == 0 ? u.x : s == 1 ? u.y : s == 2 ? u.z : u.w; };
 #pragma unroll
-  for (int mt = 0; mt < 8; ++mt)
+  for (int s = 0; s < 4; ++s)
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const int ch = 8 * (s * 8 + g) + mt;
+    for (int k = 0; k < 2; ++k) {  // M-tile 2s + k: half k of word s of the lane's eight channels
+      uint32_t a[4];
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int h = 2 * tig + e;  // heads 0-3 are the first of two halves when there are eight
-        if (rep > 4) {
-          (h < 4 ? ws.v.red0 : ws.u.red)[h & 3][ch] = acc[mt][s * 2 + e];
-        } else if (h < 4) {
-          ws.u.red[h][ch] = acc[mt][s * 2 + e];
-        }
+      for (int q = 0; q < 4; ++q) {  // fragment register: row slot q & 1, token pair q >> 1
+        const uint32_t x0 = word(v[2 * (q >> 1)][q & 1], s), x1 = word(v[2 * (q >> 1) + 1][q & 1], s);
+        a[q] = k ? pack_hi16(x0, x1) : pack_lo16(x0, x1);
       }
+      mma16816(acc[2 * s + k], a[0], a[1], a[2], a[3], b0, b1);
     }
+  __syncwarp();
+  // M-tile mt, slot s: channel 8*(8s + g) + mt; columns 2tig, 2tig+1 = heads (4-7: none)
+  if (tig < 2) {
+#pragma unroll
+    for (int mt = 0; mt < 8; ++mt)
+#pragma unroll
+      for (int s = 0; s < 2; ++s)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) ws.red[2 * tig + e][8 * (s * 8 + g) + mt] += acc[mt][s * 2 + e];
+  }
 }
 
 // Cross-GPU barrier of one call, run by up to `world` threads of one CTA: thread r tells peer r "my stores
@@ -1371,12 +1709,11 @@ __device__ __forceinline__ void peer_barrier_device(unsigned* const* pad, int ra
 }
 
 static_assert(sizeof(VWarpShared) * VWARPS >= HS_TOKENS * 4 + HS_TOKENS * HS_HEADS * 2, "importance-row staging fits the tile buffers");
-// Importance row of one chunk of tokens, run by the last CTA to finish it (not inlined: its registers are its own).
-__device__ __noinline__ void head_sum_chunk(const DecodeParams& P, const TierDev& T, VShared& sh, int chunk, bool is_res) {
+// Importance row of n tokens from token c0 of a tier on, run by the last CTA to finish their grid row (not inlined: its registers are its own).
+__device__ __noinline__ void head_sum_chunk(const DecodeParams& P, const TierDev& T, VShared& sh, int c0, int n, bool is_res) {
   const int tid = threadIdx.x;
   __threadfence();
-  const int c0 = (chunk - T.v_chunk0) * T.v_chunk_tokens;
-  const int n = min(T.v_chunk_tokens, T.n_v - c0);
+  __syncthreads();  // the round before is done with the staging buffers
   // The warps' tile buffers are free by now: they stage the chunk's positions and, per token and head, the sum
   // over the batch rounded to fp16.  Loads first, all of them independent: an item is (token, eight heads),
   // four items - 32 gathers per batch entry - are in flight per thread; then one thread per token adds the
@@ -1431,137 +1768,106 @@ __device__ __noinline__ void head_sum_chunk(const DecodeParams& P, const TierDev
   }
 }
 
+// GV: log2 of the channel group, with four query heads per CTA and the softmax of the scratch logits; 0: everything else.
+// ONE_TIER: no CTA has units of two tiers.
+template <int GV, bool ONE_TIER>
 __global__ void __launch_bounds__(VTHREADS, V_MIN_CTAS) v_pass_kernel(const __grid_constant__ DecodeParams P) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   VShared& sh = *reinterpret_cast<VShared*>(smem_raw);
-  const int chunk = blockIdx.y, bh = blockIdx.x;
-  const int b = bh / P.H, kvh = bh - b * P.H;
+  const Where w = where(P);
+  const int row = blockIdx.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int rep = P.rep;
-  const int nh = rep > 4 ? 2 : 1;
-
-  int ti = HQKV_NUM_TIERS;
-#pragma unroll
-  for (int t = 0; t < HQKV_NUM_TIERS; ++t)
-    if (chunk >= P.tier[t].v_chunk0 && chunk < P.tier[t + 1].v_chunk0) ti = t;
-  const TierDev& T = P.tier[ti];
-  const bool is_res = ti == HQKV_NUM_TIERS;
-  const int vb = is_res ? 16 : T.bits;
-  const int tile_tokens = T.v_chunk_tokens / VWARPS;
-  const int tile_t0 = (chunk - T.v_chunk0) * T.v_chunk_tokens + warp * tile_tokens;
-  const int ntok = min(tile_tokens, T.n_v - tile_t0);  // <= 0: this warp has no tile
-  VWarpShared& ws = sh.w[warp];
-  const int ng = D >> P.gv_shift;
 
   // The next kernel of the stream - the K pass of the next decode call, if it was launched with
   // programmatic stream serialisation - may start its cache-only prologue while this grid drains.
   asm volatile("griddepcontrol.launch_dependents;");
-  // ---- requests that read only the cache go out before the K pass is known to be complete
-  if (ntok > 0) {
-    if (vb == 8) v_tile_request<8>(T, ws, bh, tile_t0, ntok, ng);
-    else if (vb == 4) v_tile_request<4>(T, ws, bh, tile_t0, ntok, ng);
-    else if (vb == 2) v_tile_request<2>(T, ws, bh, tile_t0, ntok, ng);
-    else if (vb == 1) v_tile_request<1>(T, ws, bh, tile_t0, ntok, ng);
-  }
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-
-  if (P.probs_in) {  // weights are given: nothing to fold, nothing to normalise by
-    if (tid < rep) {
-      sh.gm[tid] = 0.f;
-      sh.gl[tid] = 1.f;
-    }
-    __syncthreads();
-  } else
-  // ---- global (max, sum) of the heads from the k_pass pairs: thread = (head, slice of the chunks);
-  //      only the heads that exist are read, up to four pairs per thread in flight (one round of loads
-  //      up to 4 * 128 / rep chunks), then slices are folded by shuffles and across warps
-  {
-    const int rs = P.rep_shift;
-    const int h = tid & (rep - 1), slice = tid >> rs, slices = VTHREADS >> rs;
-    const float2* part = P.k_part + static_cast<int64_t>(bh) * P.nk_chunks * MAX_REP;
-    float m = -INFINITY, l = 0.f;
-    for (int c0 = slice; c0 < P.nk_chunks; c0 += 4 * slices) {
-      float2 v[4];
+  VWarpShared& ws = sh.w[warp];
+  bool fresh = true;  // the warp's partial output is still to be set
+  // ---- global (max, sum) of the heads from the K pass's pairs: warp = head, up to four pairs per lane in
+  //      flight (weights given by the caller: nothing to fold, nothing to normalise by)
+  bool folded = false;
+  auto fold = [&]() {
+    if (folded) return;
+    folded = true;
+    if (!P.probs_in && warp < P.r4) {
+      const float2* part = P.k_part + (static_cast<int64_t>(w.bvh) * P.r4 + warp) * P.nk_ctas;
+      float m = -INFINITY, l = 0.f;
+      for (int c0 = lane; c0 < P.nk_ctas; c0 += 4 * 32) {
+        float2 v[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c = c0 + slices * j;
-        v[j] = c < P.nk_chunks ? __ldcg(part + c * MAX_REP + h) : make_float2(-INFINITY, 0.f);
+        for (int j = 0; j < 4; ++j) v[j] = c0 + 32 * j < P.nk_ctas ? __ldcg(part + c0 + 32 * j) : make_float2(-INFINITY, 0.f);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) softmax_merge(m, l, v[j].x, v[j].y);
       }
+      float mx = m;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) softmax_merge(m, l, v[j].x, v[j].y);
-    }
-    for (int off = rep; off < 32; off <<= 1) {
-      const float m2 = __shfl_xor_sync(0xffffffffu, m, off);
-      const float l2 = __shfl_xor_sync(0xffffffffu, l, off);
-      softmax_merge(m, l, m2, l2);
-    }
-    if (lane < rep) {
-      sh.wm[warp][lane] = m;
-      sh.wl[warp][lane] = l;
+      for (int o = 1; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      float sum = l * fast_exp2((m - (mx == -INFINITY ? 0.f : mx)) * LOG2E);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (lane == 0) {
+        sh.gm[warp] = mx * LOG2E;
+        sh.ginv[warp] = 1.f / sum;
+      }
     }
     __syncthreads();
-    if (tid < rep) {
-      float mm = sh.wm[0][tid], ll = sh.wl[0][tid];
-      for (int w = 1; w < VWARPS; ++w) softmax_merge(mm, ll, sh.wm[w][tid], sh.wl[w][tid]);
-      sh.gm[tid] = mm;
-      sh.gl[tid] = ll;
+  };
+  // ---- the warp's tiles: probabilities of its tokens, then sum_t p_t * V_t
+  auto plain = [&](int ti, int t0, int t1) {  // fp16 tier, residual window
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    fold();
+    if (fresh) {
+#pragma unroll
+      for (int i = 0; i < MAX_R4; ++i) reinterpret_cast<float4*>(ws.red[i])[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+      fresh = false;
     }
-    __syncthreads();
-  }
-  // ---- the warp's tile: probabilities of its tokens, then sum_t p_t * V_t
-  if (ntok > 0 && vb != 16) {
-    if (vb == 8) v_tile<8>(P, T, sh, ws, b, kvh, ntok, nh);
-    else if (vb == 4) v_tile<4>(P, T, sh, ws, b, kvh, ntok, nh);
-    else if (vb == 2) v_tile<2>(P, T, sh, ws, b, kvh, ntok, nh);
-    else v_tile<1>(P, T, sh, ws, b, kvh, ntok, nh);
+    for (int t = t0 + 16 * warp; t < t1; t += 16 * VWARPS) v_plain_tile(P, P.tier[ti], sh, ws, w, t, min(16, t1 - t), ti != 0);
+  };
+  int t0, t1;
+  if constexpr (ONE_TIER) {
+    const int ti = only_share<true>(P, t0, t1);
+    if (ti == 1) v_run<8, GV, 2>(P, P.tier[1], sh, w, t0, t1, fold, fresh);
+    else if (ti == 2) v_run<4, GV, 2>(P, P.tier[2], sh, w, t0, t1, fold, fresh);
+    else if (ti == 3) v_run<2, GV, 2>(P, P.tier[3], sh, w, t0, t1, fold, fresh);
+    else if (ti == 4) v_run<1, GV, 2>(P, P.tier[4], sh, w, t0, t1, fold, fresh);
+    else plain(ti, t0, t1);
   } else {
-    if (ntok > 0) {
-      v_plain_tile(P, T, sh, ws, bh, b, kvh, tile_t0, ntok, is_res);
-    } else {
-      for (int i = lane; i < 4 * D; i += 32) {
-        (&ws.u.red[0][0])[i] = 0.f;
-        if (nh == 2) (&ws.v.red0[0][0])[i] = 0.f;
-      }
-    }
-    (&ws.zt[0][0])[lane] = 0.f;  // 4 x MAX_REP floats
+    if (share_of<true>(P, 1, 8, t0, t1)) v_run<8, GV, 1>(P, P.tier[1], sh, w, t0, t1, fold, fresh);
+    if (share_of<true>(P, 2, 4, t0, t1)) v_run<4, GV, 1>(P, P.tier[2], sh, w, t0, t1, fold, fresh);
+    if (share_of<true>(P, 3, 2, t0, t1)) v_run<2, GV, 1>(P, P.tier[3], sh, w, t0, t1, fold, fresh);
+    if (share_of<true>(P, 4, 1, t0, t1)) v_run<1, GV, 1>(P, P.tier[4], sh, w, t0, t1, fold, fresh);
+    for (int ti = 0; ti <= HQKV_NUM_TIERS; ti += HQKV_NUM_TIERS)
+      if (share_of<true>(P, ti, 16, t0, t1)) plain(ti, t0, t1);
   }
   __syncthreads();
-  // ---- partial output of this chunk (warps added in index order) joins the accumulators of this
-  //      (batch, kv head).  The adds are fire-and-forget fp64 reductions: the sum of the fp32 partials
+  // ---- partial output of this CTA (warps added in index order) joins the accumulators of its heads.  The adds are
+  //      fire-and-forget fp64 reductions: the sum of the fp32 partials
   //      depends on their order only below 2^-53, far below the fp16 rounding of the output, and no
   //      CTA has to read other CTAs' partials back (a chain of dependent L2 round trips that used to
   //      be a quarter of the kernel at batch 1).
-  {
-    double* accum = P.v_acc + static_cast<int64_t>(bh) * rep * D;
-    for (int i = tid; i < rep * D; i += VTHREADS) {
-      const int h = i >> 7, ch = i & (D - 1);
-      const bool first_of_two = (h >> 2) + 1 < nh;
-      float v = 0.f;
+  double* accum = P.v_acc + (static_cast<int64_t>(w.b) * P.nh_q + w.h0) * D;
+  for (int h = 0; h < P.r4; ++h) {
+    float v = 0.f;
 #pragma unroll
-      for (int w = 0; w < VWARPS; ++w) {
-        const VWarpShared& o = sh.w[w];
-        v += (first_of_two ? o.v.red0[h & 3][ch] : o.u.red[h & 3][ch]) + o.zt[ch >> P.gv_shift][h];
-      }
-      atomicAdd(accum + i, static_cast<double>(v));
-    }
+    for (int i = 0; i < VWARPS; ++i) v += sh.w[i].red[h][tid];
+    atomicAdd(accum + h * D + tid, static_cast<double>(v));
   }
-  // ---- the last CTA of this (batch, kv head) normalises and writes the output
-  __threadfence();
+  // ---- the last CTA of this (batch, virtual kv head) normalises and writes the output
   __syncthreads();
   if (tid == 0) {
-    const unsigned prev = atomicAdd(&P.counters[bh], 1u);
-    sh.is_last = (prev == static_cast<unsigned>(P.nv_chunks) - 1u) ? 1u : 0u;
-    if (sh.is_last) P.counters[bh] = 0u;  // ready for the next call
+    __threadfence();  // the CTA's adds, which the barrier has ordered before this thread's fence
+    const unsigned prev = atomicAdd(&P.counters[w.bvh], 1u);
+    sh.is_last = (prev == static_cast<unsigned>(P.nv_ctas) - 1u) ? 1u : 0u;
+    if (sh.is_last) P.counters[w.bvh] = 0u;  // ready for the next call
   }
   __syncthreads();
   if (sh.is_last) {
     __threadfence();
-    double* accum = P.v_acc + static_cast<int64_t>(bh) * rep * D;
-    for (int i = tid * 2; i < rep * D; i += VTHREADS * 2) {
+    for (int i = tid * 2; i < P.r4 * D; i += VTHREADS * 2) {
       const double2 v = __ldcg(reinterpret_cast<const double2*>(accum + i));
-      const float inv = 1.f / sh.gl[i >> 7];
+      const float inv = P.probs_in ? 1.f : sh.ginv[i >> 7];
       const __half2 o = __floats2half2_rn(static_cast<float>(v.x) * inv, static_cast<float>(v.y) * inv);
-      const int64_t at = (static_cast<int64_t>(b) * P.nh_q + kvh * rep) * D + i;
+      const int64_t at = (static_cast<int64_t>(w.b) * P.nh_q + w.h0) * D + i;
       *reinterpret_cast<__half2*>(P.out + at) = o;
       // kv-head sharding: the same rows go straight into every peer's copy of the gathered output
       // (plain stores over NVLink; the callers' cross-GPU barrier makes them visible before use)
@@ -1580,7 +1886,7 @@ __global__ void __launch_bounds__(VTHREADS, V_MIN_CTAS) v_pass_kernel(const __gr
       __syncthreads();
       if (tid == 0) {
         const unsigned done = atomicAdd(P.peer_state + 2, 1u);
-        sh.is_last = (done == static_cast<unsigned>(P.B * P.H) - 1u) ? 1u : 0u;
+        sh.is_last = (done == gridDim.x * gridDim.z - 1u) ? 1u : 0u;
         if (sh.is_last) P.peer_state[2] = 0u;
       }
       __syncthreads();
@@ -1593,26 +1899,37 @@ __global__ void __launch_bounds__(VTHREADS, V_MIN_CTAS) v_pass_kernel(const __gr
       }
     }
   }
-  // ---- importance row: sum of the probabilities over batch, then over heads, for the tokens of this chunk.
-  //      The CTAs of all (batch, kv head) pairs that hold this chunk index wrote these tokens' probabilities; the
+  // ---- importance row: sum of the probabilities over batch, then over heads, for the tokens of this share.
+  //      The CTAs of all (batch, kv head) pairs with the same share wrote these tokens' probabilities; the
   //      last of them to arrive adds them in fixed order with the roundings of attn_weights.sum(0).sum(0) on fp16
   //      tensors (fp32 accumulation, one fp16 rounding per sum; model/public_func.py:253-254 of the reference).
   if (P.head_sum) {
     __threadfence();  // this CTA's probabilities
     __syncthreads();
     if (tid == 0) {
-      const unsigned prev = atomicAdd(&P.hs_count[chunk], 1u);
-      sh.is_last = (prev == static_cast<unsigned>(P.B * P.H) - 1u) ? 1u : 0u;
-      if (sh.is_last) P.hs_count[chunk] = 0u;  // ready for the next call
+      const unsigned prev = atomicAdd(&P.hs_count[row], 1u);
+      sh.is_last = (prev == gridDim.x * gridDim.z - 1u) ? 1u : 0u;
+      if (sh.is_last) P.hs_count[row] = 0u;  // ready for the next call
     }
     __syncthreads();
-    if (sh.is_last) head_sum_chunk(P, T, sh, chunk, is_res);
+    if (sh.is_last) {
+      const int only = ONE_TIER ? only_share<true>(P, t0, t1) : -1;
+      for (int ti = 0; ti <= HQKV_NUM_TIERS; ++ti)
+        if (ONE_TIER ? ti == only : share_of<true>(P, ti, P.tier[ti].bits, t0, t1))
+          for (int c0 = t0; c0 < t1; c0 += HS_TOKENS) head_sum_chunk(P, P.tier[ti], sh, c0, min(HS_TOKENS, t1 - c0), ti == HQKV_NUM_TIERS);
+    }
   }
 }
 
 // ------------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------------
+// Both passes ask for the same amount of shared memory: their CTAs follow each other on an SM, and with two sizes the
+// gaps that one kind leaves do not fit the other (four of one kind, then only three of the other, half the SMs a wave
+// behind: 77 against 60 us per layer at batch 8).
+constexpr size_t PASS_SMEM = sizeof(KShared) > sizeof(VShared) ? sizeof(KShared) : sizeof(VShared);
+static_assert(4 * (PASS_SMEM + 1024) <= 228 * 1024, "four CTAs per SM");
+
 static int ilog2(int v) {
   int s = 0;
   while ((1 << s) < v) ++s;
@@ -1622,6 +1939,35 @@ static int ilog2(int v) {
 struct Layout {
   size_t acc_off, logits_off, kpart_off, total;
 };
+
+// How the CTAs of a plane share its units.  A CTA pays for its prologue, the softmax pairs and the output reduction
+// whatever it walks - about as much as two units - and the last wave of CTAs should be full: of one to four waves the
+// number of CTAs that finishes first.  Where that leaves a CTA one or two units, a second tier would double its latency:
+// there a CTA keeps to one tier.
+static void divide(DecodeParams& P, int64_t planes, int slots, bool v) {
+  int units = 0;
+  for (const TierDev& t : P.tier) units += static_cast<int>(ceil_div(v ? t.n_v : t.n_k, unit_tokens(t.bits)));
+  int ctas = 0, per = 0, more = 0;
+  int64_t best = -1;
+  for (int waves = 1; units > 0 && waves <= 4; ++waves) {
+    int64_t n = static_cast<int64_t>(slots) * waves / planes;
+    n = n < 1 ? 1 : n > units ? units : n;
+    const int64_t share = ceil_div(units, n), cost = ceil_div(ceil_div(units, share) * planes, slots) * (share + 2);
+    if (best < 0 || cost < best) best = cost, ctas = static_cast<int>(ceil_div(units, share)), per = units / ctas, more = units % ctas;
+  }
+  if (units > 0 && per + (more > 0) <= 2) {
+    int n = 0;
+    const int most = per + (more > 0);
+    for (TierDev& t : P.tier) {
+      (v ? t.v_cta0 : t.k_cta0) = n;
+      n += static_cast<int>(ceil_div(v ? t.n_v : t.n_k, unit_tokens(t.bits) * most * (!v && t.bits == 8 ? 2 : 1)));
+    }
+    ctas = n, per = most, more = -1;
+  }
+  (v ? P.nv_ctas : P.nk_ctas) = ctas;
+  (v ? P.v_per : P.k_per) = per;
+  (v ? P.v_more : P.k_more) = more;
+}
 
 // sides: 1 = only the K side of the descriptor is looked at, 2 = only the V side, 3 = both
 static int build_params(const hqkv_cache_desc_t* c, DecodeParams& P, Layout& lay, int sides = 3) {
@@ -1638,9 +1984,11 @@ static int build_params(const hqkv_cache_desc_t* c, DecodeParams& P, Layout& lay
   P.B = c->B;
   P.H = c->H;
   P.nh_q = c->nh_q;
-  P.rep = c->nh_q / c->H;
-  HQKV_REQUIRE((P.rep & (P.rep - 1)) == 0, "decode: nh_q / H must be 1, 2, 4 or 8 (got %d)", P.rep);
-  P.rep_shift = ilog2(P.rep);
+  const int rep = c->nh_q / c->H;
+  HQKV_REQUIRE((rep & (rep - 1)) == 0, "decode: nh_q / H must be 1, 2, 4 or 8 (got %d)", rep);
+  P.halves = rep > MAX_R4 ? 2 : 1;
+  P.r4 = rep / P.halves;
+  P.r4_shift = ilog2(P.r4);
   P.gk_shift = ilog2(c->group_k);
   P.gv_shift = ilog2(c->group_v);
   P.scale = c->softmax_scale;
@@ -1689,15 +2037,11 @@ static int build_params(const hqkv_cache_desc_t* c, DecodeParams& P, Layout& lay
     d.v_scale = static_cast<const __half*>(s.v_scale);
     d.v_zero = static_cast<const __half*>(s.v_zero);
     d.v_idx = s.v_idx;
-    // chunk sizes: about the same number of bytes per CTA whatever the width
-    const int b = d.bits;
-    d.k_chunk_tokens = KWARPS * (b == 8 || b == 16 ? 64 : 128);  // one tile per warp
-    HQKV_REQUIRE(static_cast<int64_t>(s.n_k) * D * b / 8 < (1ll << 31), "decode: tier %d K plane of one head exceeds 2 GiB", t);
-    d.v_chunk_tokens = VWARPS * (b == 8 ? 64 : b == 16 ? 16 : 128);  // one tile per warp
-    d.k_chunk0 = kc;
-    d.v_chunk0 = vc;
-    kc += static_cast<int>(ceil_div(d.n_k, d.k_chunk_tokens));
-    vc += static_cast<int>(ceil_div(d.n_v, d.v_chunk_tokens));
+    HQKV_REQUIRE(static_cast<int64_t>(s.n_k) * D * d.bits / 8 < (1ll << 31), "decode: tier %d K plane of one head exceeds 2 GiB", t);
+    d.k_unit0 = kc;
+    d.v_unit0 = vc;
+    kc += static_cast<int>(ceil_div(d.n_k, unit_tokens(d.bits)));
+    vc += static_cast<int>(ceil_div(d.n_v, unit_tokens(d.bits)));
     nk_total += d.n_k;
     nv_total += d.n_v;
   }
@@ -1713,25 +2057,23 @@ static int build_params(const hqkv_cache_desc_t* c, DecodeParams& P, Layout& lay
   }
   r.k_data = c->new_k;
   r.v_data = c->new_v;
-  r.k_chunk_tokens = KWARPS * 16;
-  r.v_chunk_tokens = VWARPS * 16;
-  r.k_chunk0 = kc;
-  r.v_chunk0 = vc;
-  kc += static_cast<int>(ceil_div(r.n_k, r.k_chunk_tokens));
-  vc += static_cast<int>(ceil_div(r.n_v, r.v_chunk_tokens));
+  r.k_unit0 = kc;
+  r.v_unit0 = vc;
+  kc += static_cast<int>(ceil_div(r.n_k, unit_tokens(16)));
+  vc += static_cast<int>(ceil_div(r.n_v, unit_tokens(16)));
   const int64_t L = ((sides & 1) ? nk_total : nv_total) + c->n_new;
   HQKV_REQUIRE(L > 0, "decode: the cache is empty");
   HQKV_REQUIRE(L < (1ll << 30), "decode: cache too long");
   P.L = static_cast<int>(L);
-  P.nk_chunks = kc;
-  P.nv_chunks = vc;
-  const int64_t BH = static_cast<int64_t>(c->B) * c->H;
+  const int64_t planes = static_cast<int64_t>(c->B) * c->H * P.halves;
+  divide(P, planes, 148 * K_MIN_CTAS, false);
+  divide(P, planes, 148 * V_MIN_CTAS, true);
   lay.acc_off = HQKV_WS_HEADER_BYTES;
-  lay.logits_off = (lay.acc_off + static_cast<size_t>(BH) * P.rep * D * sizeof(double) + 255) & ~static_cast<size_t>(255);
+  lay.logits_off = (lay.acc_off + static_cast<size_t>(c->B) * c->nh_q * D * sizeof(double) + 255) & ~static_cast<size_t>(255);
   size_t off = lay.logits_off + static_cast<size_t>(c->B) * c->nh_q * L * sizeof(float);
   off = (off + 255) & ~static_cast<size_t>(255);
   lay.kpart_off = off;
-  off += static_cast<size_t>(BH) * kc * MAX_REP * sizeof(float2);
+  off += static_cast<size_t>(c->B) * c->nh_q * P.nk_ctas * sizeof(float2);
   lay.total = (off + 255) & ~static_cast<size_t>(255);
   return HQKV_OK;
 }
@@ -1804,6 +2146,12 @@ extern "C" int hqkv_decode_attention_gather(const hqkv_cache_desc_t* cache_host,
   return decode_launch(cache_host, q, attn_weights, attn_output, workspace, workspace_bytes, 3, pa, stream);
 }
 
+using PassKernel = void (*)(const DecodeParams);
+static constexpr PassKernel k_kernels[2] = {k_pass_kernel<false>, k_pass_kernel<true>};  // [one tier per CTA]
+static constexpr PassKernel v_kernels[2][4] = {
+    {v_pass_kernel<0, false>, v_pass_kernel<5, false>, v_pass_kernel<6, false>, v_pass_kernel<7, false>},
+    {v_pass_kernel<0, true>, v_pass_kernel<5, true>, v_pass_kernel<6, true>, v_pass_kernel<7, true>}};
+
 static int hqkv::decode_launch(const hqkv_cache_desc_t* cache_host, const void* q, void* attn_weights, void* attn_output,
                                void* workspace, size_t workspace_bytes, int phases, const PeerArgs& peers, void* stream,
                                const void* probs_in, const void* mask, long long mask_bstride, long long mask_hstride,
@@ -1849,18 +2197,21 @@ static int hqkv::decode_launch(const hqkv_cache_desc_t* cache_host, const void* 
   P.k_part = reinterpret_cast<float2*>(ws + lay.kpart_off);
   P.v_acc = reinterpret_cast<double*>(ws + lay.acc_off);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const unsigned BH = static_cast<unsigned>(P.B * P.H);
-  HQKV_REQUIRE(P.nk_chunks <= 65535 && P.nv_chunks <= 65535, "decode: too many chunks");
+  const unsigned VH = static_cast<unsigned>(P.H * P.halves);
+  HQKV_REQUIRE(P.nk_ctas <= 65535 && P.nv_ctas <= 65535, "decode: too many chunks");
   {
     // opt in to >48 KB of dynamic shared memory once per device
     static bool attr_set[64] = {};
     int dev = 0;
     HQKV_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-      HQKV_CUDA(cudaFuncSetAttribute(v_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(sizeof(VShared))));
-      HQKV_CUDA(cudaFuncSetAttribute(k_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(sizeof(KShared))));
+      // all of them with the same (largest) share of the L1 for shared memory: CTAs of kernels that ask for different
+      // shares cannot be on an SM together
+      for (int one = 0; one < 2; ++one)
+        for (PassKernel f : {k_kernels[one], v_kernels[one][0], v_kernels[one][1], v_kernels[one][2], v_kernels[one][3]}) {
+          HQKV_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(PASS_SMEM)));
+          HQKV_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        }
       if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
   }
@@ -1870,25 +2221,26 @@ static int hqkv::decode_launch(const hqkv_cache_desc_t* cache_host, const void* 
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  if ((phases & 1) && P.nk_chunks > 0) {
+  if ((phases & 1) && P.nk_ctas > 0) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(BH, P.nk_chunks);
+    cfg.gridDim = dim3(VH, P.nk_ctas, P.B);
     cfg.blockDim = dim3(KTHREADS);
-    cfg.dynamicSmemBytes = sizeof(KShared);
+    cfg.dynamicSmemBytes = PASS_SMEM;
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    HQKV_CUDA(cudaLaunchKernelEx(&cfg, k_pass_kernel, P));
+    HQKV_CUDA(cudaLaunchKernelEx(&cfg, k_kernels[P.k_more < 0], P));
   }
-  if ((phases & 2) && P.nv_chunks > 0) {
+  if ((phases & 2) && P.nv_ctas > 0) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(BH, P.nv_chunks);
+    cfg.gridDim = dim3(VH, P.nv_ctas, P.B);
     cfg.blockDim = dim3(VTHREADS);
-    cfg.dynamicSmemBytes = sizeof(VShared);
+    cfg.dynamicSmemBytes = PASS_SMEM;
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    HQKV_CUDA(cudaLaunchKernelEx(&cfg, v_pass_kernel, P));
+    const bool fast = P.r4 == MAX_R4 && !P.probs_in && !HQKV_CHECKS_ENABLED;
+    HQKV_CUDA(cudaLaunchKernelEx(&cfg, v_kernels[P.v_more < 0][fast ? P.gv_shift - 4 : 0], P));
   }
   return HQKV_OK;
 }
@@ -1914,7 +2266,7 @@ extern "C" int hqkv_decode_attention_headsum(const hqkv_cache_desc_t* cache_host
   Layout lay;
   int rc = build_params(cache_host, P, lay);
   if (rc) return rc;
-  const bool fused = P.B * P.nh_q <= HEAD_SUM_MAX_ROWS && P.nh_q <= HS_HEADS && P.nv_chunks <= HEAD_SUM_MAX_CHUNKS;
+  const bool fused = P.B * P.nh_q <= HEAD_SUM_MAX_ROWS && P.nh_q <= HS_HEADS && P.nv_ctas <= HEAD_SUM_MAX_CHUNKS;
   rc = decode_launch(cache_host, q, attn_weights, attn_output, workspace, workspace_bytes, 3, hqkv::PeerArgs(), stream,
                      nullptr, nullptr, 0, 0, fused ? head_sum_row : nullptr);
   if (rc || fused) return rc;
@@ -1926,11 +2278,13 @@ extern "C" int hqkv_decode_attention_headsum(const hqkv_cache_desc_t* cache_host
 // The two passes as operators of their own: raw logits of every tier, and the product of given weights with V
 // ------------------------------------------------------------------------------------------------
 namespace hqkv {
-// fp32 logits of the scratch -> fp16 rows
-__global__ void __launch_bounds__(256) logits_out_kernel(const float* logits, __half* out, int64_t n) {
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
-    out[i] = __float2half_rn(__ldcg(logits + i));
+// fp32 logits of the scratch [plane][L][heads] -> fp16 rows [plane][head][L]
+__global__ void __launch_bounds__(256) logits_out_kernel(const float* logits, __half* out, int64_t planes, int64_t L, int heads) {
+  const int64_t n = planes * L, stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
+    const int64_t plane = i / L, pos = i - plane * L;
+    for (int h = 0; h < heads; ++h) out[(plane * heads + h) * L + pos] = __float2half_rn(__ldcg(logits + i * heads + h));
+  }
 }
 }  // namespace hqkv
 
@@ -1943,11 +2297,11 @@ extern "C" int hqkv_decode_logits(const hqkv_cache_desc_t* cache_host, const voi
   Layout lay;
   rc = build_params(cache_host, P, lay, 1);
   if (rc) return rc;
-  const int64_t n = static_cast<int64_t>(P.B) * P.nh_q * P.L;
-  const int blocks = static_cast<int>(n / 2048 > 592 ? 592 : (n / 2048 > 0 ? n / 2048 : 1));
+  const int64_t planes = static_cast<int64_t>(P.B) * P.H * P.halves, n = planes * P.L;
+  const int blocks = static_cast<int>(n / 512 > 592 ? 592 : (n / 512 > 0 ? n / 512 : 1));
   hqkv::logits_out_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const float*>(static_cast<unsigned char*>(workspace) + lay.logits_off),
-      static_cast<__half*>(logits_f16), n);
+      static_cast<__half*>(logits_f16), planes, P.L, P.r4);
   HQKV_LAUNCH_CHECK("decode_logits");
   return HQKV_OK;
 }
