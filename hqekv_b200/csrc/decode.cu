@@ -80,7 +80,7 @@ struct DecodeParams {
   int rank, world;
   unsigned* peer_state;  // call number, status, finished (batch, kv head) count
   long long max_spins;
-  unsigned* counters;  // [B*H]
+  unsigned* counters;  // [B][virtual kv head]
 };
 
 // The tokens of a (batch, virtual kv head) plane are a list of UNITS - 256 tokens of one tier (128 at 8 bits, 64 of the
