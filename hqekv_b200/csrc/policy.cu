@@ -72,12 +72,12 @@ __global__ void __launch_bounds__(256) token_importance_kernel(const __half* __r
   const int64_t l = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (l >= L) return;
   float acc = 0.f;
-  for (int r0 = 0; r0 < rows; r0 += 4) {  // four loads in flight, adds in row order
-    __half v[4];
+  for (int r0 = 0; r0 < rows; r0 += 10) {  // ten loads in flight (half of the models' twenty rows), adds in row order
+    __half v[10];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = r0 + j < rows ? ring[(r0 + j) * stride + l] : __float2half_rn(0.f);
+    for (int j = 0; j < 10; ++j) v[j] = ring[min(r0 + j, rows - 1) * stride + l];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < 10; ++j)
       if (r0 + j < rows) acc = __fadd_rn(acc, __half2float(v[j]));
   }
   const int64_t age = L - l;
@@ -114,117 +114,165 @@ __global__ void __launch_bounds__(128) token_range_kernel(const __half* __restri
   if (lane == 0) out[t] = __float2half_rn(over_heads);
 }
 
-// head_dim 128, 8-byte aligned rows: one 8-byte load per lane and row, eight rows in flight, half2 min / max.
-// Same additions in the same order as above.
-__global__ void __launch_bounds__(128) token_range128_kernel(const __half* __restrict__ v, int B, int H, int64_t T,
-                                                             int64_t b_stride, int64_t h_stride,
-                                                             __half* __restrict__ out) {
-  const int lane = threadIdx.x & 31;
-  const int64_t t = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (t >= T) return;
-  const int n = B * H;  // rows of this token, head-major: r = h * B + b
-  float over_heads = 0.f, over_batch = 0.f;
-  for (int r0 = 0; r0 < n; r0 += 8) {
-    uint2 w[8];
+// head_dim 128, 16-byte aligned rows.  The rows of a token - a (batch, head) pair each - are independent up to the two sums
+// over them, so they are spread over half-warps (16 bytes per lane, four rows in flight, minimum and negated maximum
+// reduced together) and only the sums, in the order above, are one thread's.  A warp per token walked the rows eight at
+// a time: with 32 tokens of 64 rows each the whole launch was eight warps long (41 us; 31 us for 32 k tokens of 8 rows).
+// CTA = 2^tshift tokens; `old` = the ranges of the tokens before these, copied to the front of `out` by the CTAs behind.
+constexpr int RANGE_THREADS = 256;
+constexpr int RANGE_MAX_ROWS = 8192;
+__global__ void __launch_bounds__(RANGE_THREADS) token_range128_kernel(const __half* __restrict__ v, int B, int n, int64_t T,
+                                                                       int64_t b_stride, int64_t h_stride, int tshift,
+                                                                       const __half* __restrict__ old, int64_t n_old, int ctas,
+                                                                       __half* __restrict__ out) {
+  extern __shared__ __half range_s[];  // [token][row], row = h * B + b
+  const int tid = threadIdx.x;
+  if (static_cast<int>(blockIdx.x) >= ctas) {
+    const int64_t base = (static_cast<int64_t>(blockIdx.x) - ctas) * RANGE_THREADS * 8 + tid;
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int r = min(r0 + u, n - 1), h = r / B, b = r - h * B;
-      w[u] = *reinterpret_cast<const uint2*>(v + b * b_stride + h * h_stride + t * 128 + 4 * lane);
+    for (int j = 0; j < 8; ++j)
+      if (base + j * RANGE_THREADS < n_old) out[base + j * RANGE_THREADS] = old[base + j * RANGE_THREADS];
+    return;
+  }
+  const int hw = tid >> 4, l16 = tid & 15, tpc = 1 << tshift;
+  const int64_t t0 = static_cast<int64_t>(blockIdx.x) << tshift;
+  const int items = n << tshift;  // token fastest: neighbouring half-warps read neighbouring rows of memory
+  for (int base = hw; base - (hw & 1) < items; base += 4 * (RANGE_THREADS / 16)) {  // (both halves of a warp take part)
+    uint4 w[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int it = min(base + u * (RANGE_THREADS / 16), items - 1), r = it >> tshift, h = r / B, b = r - h * B;
+      const int64_t t = min(t0 + (it & (tpc - 1)), T - 1);
+      w[u] = *reinterpret_cast<const uint4*>(v + b * b_stride + h * h_stride + t * 128 + 8 * l16);
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      if (r0 + u >= n) break;
-      const __half2 a = *reinterpret_cast<const __half2*>(&w[u].x), c = *reinterpret_cast<const __half2*>(&w[u].y);
-      __half2 lo = __hmin2_nan(a, c), hi = __hmax2_nan(a, c);
+    for (int u = 0; u < 4; ++u) {
+      const __half2* x = reinterpret_cast<const __half2*>(&w[u]);
+      const __half2 lo2 = __hmin2_nan(__hmin2_nan(x[0], x[1]), __hmin2_nan(x[2], x[3]));
+      const __half2 hi2 = __hmax2_nan(__hmax2_nan(x[0], x[1]), __hmax2_nan(x[2], x[3]));
+      __half2 m = __halves2half2(__hmin_nan(__low2half(lo2), __high2half(lo2)), __hneg(__hmax_nan(__low2half(hi2), __high2half(hi2))));
 #pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        lo = __hmin2_nan(lo, __shfl_xor_sync(0xffffffffu, lo, off));
-        hi = __hmax2_nan(hi, __shfl_xor_sync(0xffffffffu, hi, off));
-      }
-      const __half l1 = __hmin_nan(__low2half(lo), __high2half(lo)), h1 = __hmax_nan(__low2half(hi), __high2half(hi));
-      over_batch = __fadd_rn(over_batch, __half2float(h_sub(h1, l1)));
-      if ((r0 + u) % B == B - 1) {  // last batch entry of this head
-        over_heads = __fadd_rn(over_heads, __half2float(__float2half_rn(over_batch)));
-        over_batch = 0.f;
-      }
+      for (int off = 1; off < 16; off <<= 1) m = __hmin2_nan(m, __shfl_xor_sync(0xffffffffu, m, off));
+      const int it = base + u * (RANGE_THREADS / 16);
+      if (l16 == 0 && it < items) range_s[(it & (tpc - 1)) * n + (it >> tshift)] = h_sub(__hneg(__high2half(m)), __low2half(m));
     }
   }
-  if (lane == 0) out[t] = __float2half_rn(over_heads);
+  __syncthreads();
+  if (tid < tpc && t0 + tid < T) {
+    float over_heads = 0.f, over_batch = 0.f;
+    const __half* r = range_s + tid * n;
+    for (int i = 0, b = 0; i < n; ++i) {
+      over_batch = __fadd_rn(over_batch, __half2float(r[i]));
+      if (++b == B) {  // last batch entry of this head
+        over_heads = __fadd_rn(over_heads, __half2float(__float2half_rn(over_batch)));
+        over_batch = 0.f;
+        b = 0;
+      }
+    }
+    out[n_old + t0 + tid] = __float2half_rn(over_heads);
+  }
 }
 
 // ------------------------------------------------------------------------------------------------
-// block ranking: one thread-block cluster; bitonic sort of (inverted key, block id) in the shared memory of its
-// first CTA
+// block ranking: one thread-block cluster
 // ------------------------------------------------------------------------------------------------
-// The elementwise pass, the block keys and the final expansion to token ids are spread over the CTAs of the
-// cluster (one launch of one CTA spent most of its time walking 32 k tokens with 1024 threads); the keys meet in
-// the first CTA's shared memory (distributed shared memory stores), which sorts them alone, and all CTAs read the
-// sorted keys back from there.  Cluster barriers separate the passes and order the in-place update of
-// `importance` between the CTAs.
+// Each CTA of the cluster forms the keys of its share of the blocks (elementwise pass, then one thread per block adds in
+// order) and stores them into the shared memory of all CTAs.  The keys - fp16 key, then block id - are all different, so a
+// block's place is the number of smaller keys: every warp counts for its own blocks, with no exchange between the
+// steps of a sort.  16.7 -> 6 us for 508 blocks and 25 -> 7 us for 1 020 against a bitonic sort by one CTA; the comparisons
+// grow with the square of the blocks, and beyond RANK_COUNT_MAX the sort is kept.
 constexpr int RANK_THREADS = 1024;
 constexpr int RANK_CLUSTER = 8;
 constexpr int RANK_MAX_BLOCKS = 8192;
+constexpr int RANK_COUNT_MAX = 4096;
 
-__global__ void __launch_bounds__(RANK_THREADS) block_rank_kernel(__half* __restrict__ importance,
-                                                                  const __half* __restrict__ range, int block,
-                                                                  int nblocks, int npow2,
+__global__ void __launch_bounds__(RANK_THREADS) block_rank_kernel(const __half* importance, const __half* __restrict__ range,
+                                                                  __half* divided, int block, int nblocks, int npow2,
                                                                   int64_t* __restrict__ sorted_ids) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
-  extern __shared__ uint32_t keys[];  // npow2 entries; only the first CTA's copy is used
-  uint32_t* keys0 = cluster.map_shared_rank(keys, 0);
-  const int crank = static_cast<int>(cluster.block_rank());
-  const int64_t gtid = static_cast<int64_t>(crank) * RANK_THREADS + threadIdx.x;
-  constexpr int64_t GTHREADS = static_cast<int64_t>(RANK_THREADS) * RANK_CLUSTER;
+  extern __shared__ uint32_t keys[];  // [npow2]
+  auto started = cluster.barrier_arrive();  // (the other CTAs' shared memory may be written once they all run)
+  const int crank = static_cast<int>(cluster.block_rank()), lane = threadIdx.x & 31;
+  const int share = (nblocks + RANK_CLUSTER - 1) / RANK_CLUSTER, k0 = min(crank * share, nblocks), k1 = min(k0 + share, nblocks);
   const int64_t total = static_cast<int64_t>(nblocks) * block;
   const float fblock = static_cast<float>(block);
-  // elementwise: optional product with the range, then the in-place divide
-  for (int64_t i = gtid; i < total; i += GTHREADS) {
+  // elementwise: optional product with the range, then the divide
+#pragma unroll 4
+  for (int64_t i = static_cast<int64_t>(k0) * block + threadIdx.x; i < static_cast<int64_t>(k1) * block; i += RANK_THREADS) {
     __half x = importance[i];
     if (range) x = h_mul(x, range[i]);
-    importance[i] = h_divf(x, fblock);
+    divided[i] = h_divf(x, fblock);
   }
-  cluster.sync();
-  for (int64_t k = gtid; k < npow2; k += GTHREADS) {
-    uint32_t composite = 0xFFFFFFFFu;
-    if (k < nblocks) {
-      float acc = 0.f;
-      const __half* p = importance + k * block;
+  __syncthreads();
+  cluster.barrier_wait(std::move(started));
+  const bool vec = block % 8 == 0 && (reinterpret_cast<uintptr_t>(divided) & 15) == 0;
+  for (int k = k0 + threadIdx.x; k < k1; k += RANK_THREADS) {
+    float acc = 0.f;
+    const __half* p = divided + static_cast<int64_t>(k) * block;
+    if (vec) {
+      for (int i = 0; i < block; i += 8) {
+        const uint4 w = *reinterpret_cast<const uint4*>(p + i);
+        const __half* e = reinterpret_cast<const __half*>(&w);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc = __fadd_rn(acc, __half2float(e[j]));
+      }
+    } else {
       for (int i = 0; i < block; ++i) acc = __fadd_rn(acc, __half2float(p[i]));
-      const __half key = __float2half_rn(acc);
-      uint16_t bits = __half_as_ushort(key);
-      if ((bits & 0x7FFFu) == 0) bits = 0;                                  // -0 sorts like +0
-      const uint16_t asc = (bits & 0x8000u) ? static_cast<uint16_t>(~bits) : static_cast<uint16_t>(bits | 0x8000u);
-      const uint16_t desc = static_cast<uint16_t>(0xFFFFu - asc);           // larger key first
-      composite = (static_cast<uint32_t>(desc) << 16) | static_cast<uint32_t>(k);  // ties: lower id first
     }
-    keys0[k] = composite;
+    const __half key = __float2half_rn(acc);
+    uint16_t bits = __half_as_ushort(key);
+    if ((bits & 0x7FFFu) == 0) bits = 0;                                  // -0 sorts like +0
+    const uint16_t asc = (bits & 0x8000u) ? static_cast<uint16_t>(~bits) : static_cast<uint16_t>(bits | 0x8000u);
+    const uint16_t desc = static_cast<uint16_t>(0xFFFFu - asc);           // larger key first
+    const uint32_t composite = (static_cast<uint32_t>(desc) << 16) | static_cast<uint32_t>(k);  // ties: lower id first
+#pragma unroll
+    for (int c = 0; c < RANK_CLUSTER; ++c) cluster.map_shared_rank(keys, c)[k] = composite;
   }
+  if (nblocks > RANK_COUNT_MAX)
+    for (int k = nblocks + threadIdx.x; k < npow2; k += RANK_THREADS) keys[k] = 0xFFFFFFFFu;
   cluster.sync();
-  if (crank == 0) {
-    for (int size = 2; size <= npow2; size <<= 1) {
-      for (int stride = size >> 1; stride > 0; stride >>= 1) {
-        for (int i = threadIdx.x; i < (npow2 >> 1); i += RANK_THREADS) {
-          const int lo = 2 * i - (i & (stride - 1));  // index with the `stride` bit clear
-          const int hi = lo + stride;
-          const bool up = (lo & size) == 0;
-          const uint32_t a = keys[lo], b = keys[hi];
-          if ((a > b) == up) {
-            keys[lo] = b;
-            keys[hi] = a;
-          }
-        }
-        __syncthreads();
+  if (nblocks <= RANK_COUNT_MAX) {
+    constexpr int WARPS = RANK_THREADS / 32 * RANK_CLUSTER;
+    for (int m0 = crank * (RANK_THREADS / 32) + (threadIdx.x >> 5); m0 < nblocks; m0 += 4 * WARPS) {
+      uint32_t mine[4], below[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) mine[q] = m0 + q * WARPS < nblocks ? keys[m0 + q * WARPS] : 0u;
+      for (int j = lane; j < nblocks; j += 32) {
+        const uint32_t other = keys[j];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) below[q] += other < mine[q] ? 1u : 0u;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (m0 + q * WARPS >= nblocks) break;
+        const int64_t place = __reduce_add_sync(0xffffffffu, below[q]), blk = m0 + q * WARPS;
+        for (int i = lane; i < block; i += 32) sorted_ids[place * block + i] = blk * block + i;
       }
     }
+    return;
   }
-  cluster.sync();
-  for (int64_t i = gtid; i < total; i += GTHREADS) {
+  // bitonic sort of (inverted key, block id), every CTA for itself
+  for (int size = 2; size <= npow2; size <<= 1) {
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      for (int i = threadIdx.x; i < (npow2 >> 1); i += RANK_THREADS) {
+        const int lo = 2 * i - (i & (stride - 1));  // index with the `stride` bit clear
+        const int hi = lo + stride;
+        const bool up = (lo & size) == 0;
+        const uint32_t a = keys[lo], b = keys[hi];
+        if ((a > b) == up) {
+          keys[lo] = b;
+          keys[hi] = a;
+        }
+      }
+      __syncthreads();
+    }
+  }
+  for (int64_t i = static_cast<int64_t>(crank) * RANK_THREADS + threadIdx.x; i < total; i += RANK_THREADS * RANK_CLUSTER) {
     const int j = static_cast<int>(i / block);
-    const int64_t blk = keys0[j] & 0xFFFFu;
+    const int64_t blk = keys[j] & 0xFFFFu;
     sorted_ids[i] = blk * block + (i - static_cast<int64_t>(j) * block);
   }
-  cluster.sync();  // the first CTA's shared memory stays until every CTA has read the sorted keys
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -233,65 +281,72 @@ __global__ void __launch_bounds__(RANK_THREADS) block_rank_kernel(__half* __rest
 constexpr int PLAN_THREADS = 1024;
 constexpr int PLAN_CLUSTER = 8;   // CTAs of the cluster (the portable maximum)
 
-struct PlanArgs {
+struct PlanSide {
   const int64_t* tier_idx[HQKV_NUM_TIERS];
   int32_t tier_n[HQKV_NUM_TIERS];
-  int64_t hist, compress;
   int64_t cum[6];
   const int64_t* sorted_ids;
   int32_t* plan_src;   // [5][total]
   int64_t* plan_ids;   // [5][total]
   int64_t* survivors;  // [total]
   int32_t* counts;     // [8]
-  // scratch, each [total]
-  int8_t* tgt;         // by token id
-  int8_t* fin;         // by enumeration slot
-  int32_t* rank;       // by token id: rank among survivors
+  // scratch
+  int8_t* tgt;         // [total] by token id, 16-byte aligned
+  int8_t* fin;         // [total] by enumeration slot: category
+  int32_t* rank;       // [total] by token id: rank among survivors
   int32_t* gcnt;       // [PLAN_CATS][PLAN_CLUSTER * PLAN_WARPS] per-warp category counts of the whole cluster
-  int32_t* flags;      // [0] = something is evicted
+};
+struct PlanArgs {
+  PlanSide side[2];    // one cluster each
+  int64_t hist, compress;
 };
 
 // Enumeration order of every cached token: residual (ascending id), then the 16-, 8-, 4-, 2-, 1-bit
 // tier in storage order.  Slot -> (source tier, position, token id).
-__device__ __forceinline__ void enum_slot(const PlanArgs& A, int64_t slot, int& src, int64_t& pos, int64_t& id) {
+__device__ __forceinline__ void enum_slot(const PlanArgs& A, const PlanSide& S, int64_t slot, int& src, int32_t& pos, int64_t& id) {
   if (slot < A.compress) {
     src = -1;
-    pos = slot;
+    pos = static_cast<int32_t>(slot);
     id = A.hist + slot;
     return;
   }
-  int64_t s = slot - A.compress;
-  for (int t = 0; t < HQKV_NUM_TIERS; ++t) {
-    if (s < A.tier_n[t]) {
-      src = t;
-      pos = s;
-      id = A.tier_idx[t][s];
-      return;
-    }
-    s -= A.tier_n[t];
-  }
+  int32_t s = static_cast<int32_t>(slot - A.compress);
   src = -2;
   pos = 0;
   id = 0;
+#pragma unroll
+  for (int t = 0; t < HQKV_NUM_TIERS; ++t) {
+    if (src == -2 && s < S.tier_n[t]) {
+      src = t;
+      pos = s;
+      id = S.tier_idx[t][s];
+    }
+    s -= S.tier_n[t];
+  }
 }
 
-// One cluster of PLAN_CLUSTER CTAs of 32 warps.  Every pass walks the enumeration (or the token ids) in
+// One cluster of PLAN_CLUSTER CTAs of 32 warps per side.  Every pass walks the enumeration (or the token ids) in
 // warp-contiguous ranges - warp w of CTA r is range r * 32 + w - PLAN_BATCH iterations at a time so that the
 // dependent loads of a batch (index list -> target -> rank) are in flight together; ordered positions come from
 // per-warp counts (left in global memory for the other CTAs), one scan over all warps of the cluster, and ballot /
 // match prefixes inside a warp.  The passes are separated by cluster barriers, which also order the global-memory
 // scratch between the CTAs.  Categories: 2*t = kept member of tier t, 2*t + 1 = arrival in tier t (destination
 // order: kept members first, then arrivals, both in enumeration order); 10 = surviving token id.
+// What bounds it is the chain of dependent L2 round trips, two or three per pass: both sides in one launch, survival read
+// off the targets instead of a pass of its own, and the scan by one warp per category instead of 256 steps by one
+// thread took the two plans of a 32 k-token flush from 2 x 24.5 us to 17 us together.
 constexpr int PLAN_WARPS = PLAN_THREADS / 32;
 constexpr int PLAN_GWARPS = PLAN_WARPS * PLAN_CLUSTER;
-constexpr int PLAN_BATCH = 8;
+constexpr int PLAN_BATCH = 4;
 constexpr int PLAN_CATS = 2 * HQKV_NUM_TIERS + 1;
+constexpr int PLAN_NONE = PLAN_CATS;  // no destination: evicted, or residual without a target
 
 __global__ void __launch_bounds__(PLAN_THREADS) flush_plan_kernel(const __grid_constant__ PlanArgs A) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
-  __shared__ int cnt[PLAN_CATS][PLAN_WARPS];  // this CTA's per-warp totals, then their exclusive offsets over the cluster
+  __shared__ int cnt[PLAN_CATS + 1][PLAN_WARPS];  // per-warp totals, then their exclusive offsets over the cluster
   __shared__ int tot[PLAN_CATS];
+  const PlanSide& S = A.side[blockIdx.y];
   const int64_t total = A.hist + A.compress;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int crank = static_cast<int>(cluster.block_rank());
@@ -302,157 +357,156 @@ __global__ void __launch_bounds__(PLAN_THREADS) flush_plan_kernel(const __grid_c
   // warp gw owns elements [gw * span, (gw + 1) * span), span a multiple of 32
   const int64_t iters = (total + GTHREADS - 1) / GTHREADS;
   const int64_t span = iters * 32, first = gwarp * span;
-  if (gtid == 0) A.flags[0] = 0;
-  if (tid < PLAN_CATS * PLAN_WARPS) (&cnt[0][0])[tid] = 0;
-  // 1. targets by token id
-  for (int64_t i = gtid; i < total; i += GTHREADS) A.tgt[i] = -1;
+  const bool any_evict = S.cum[5] > S.cum[4];
+  if (tid < (PLAN_CATS + 1) * PLAN_WARPS) (&cnt[0][0])[tid] = 0;
+  // 1. targets by token id (-1: not in the ranked list)
+  for (int64_t i = gtid; i < (total + 15) / 16; i += GTHREADS)
+    reinterpret_cast<uint4*>(S.tgt)[i] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
   cluster.sync();
-  for (int64_t j = gtid; j < total; j += GTHREADS) {
-    int t = -1;
+#pragma unroll 4
+  for (int64_t j = gtid; j < S.cum[5]; j += GTHREADS) {
+    int t = 0;
 #pragma unroll
-    for (int k = 5; k >= 0; --k)
-      if (j < A.cum[k] && j >= (k ? A.cum[k - 1] : 0)) t = k;
-    if (t >= 0) {
-      if (HQKV_INDEX_OK(A.sorted_ids[j], total)) A.tgt[A.sorted_ids[j]] = static_cast<int8_t>(t);
-      if (t == 5) A.flags[0] = 1;
-    }
+    for (int k = 0; k < 5; ++k) t += j >= S.cum[k] ? 1 : 0;
+    const int64_t id = S.sorted_ids[j];
+    if (HQKV_INDEX_OK(id, total)) S.tgt[id] = static_cast<int8_t>(t);
   }
   cluster.sync();
-  // 2. final tier of every enumeration slot (0..4 tier, 5 evicted, 6 dropped: residual without target),
-  //    survival by token id, and the per-warp category counts
+  // 2. category of every enumeration slot; per-warp counts of the categories and of the surviving token ids
+  int mine = 0;
   for (int64_t j0 = 0; j0 < iters; j0 += PLAN_BATCH) {
-    int src[PLAN_BATCH];
+    int src[PLAN_BATCH], tg[PLAN_BATCH], own[PLAN_BATCH];
     int64_t id[PLAN_BATCH];
-    int tg[PLAN_BATCH];
 #pragma unroll
     for (int u = 0; u < PLAN_BATCH; ++u) {
       const int64_t s = first + (j0 + u) * 32 + lane;
-      int64_t pos;
+      int32_t pos;
       src[u] = -2;
       id[u] = 0;
-      if (j0 + u < iters && s < total) enum_slot(A, s, src[u], pos, id[u]);
+      own[u] = 5;
+      if (j0 + u < iters && s < total) {
+        enum_slot(A, S, s, src[u], pos, id[u]);
+        own[u] = S.tgt[s];
+      }
     }
 #pragma unroll
-    for (int u = 0; u < PLAN_BATCH; ++u) tg[u] = (src[u] != -2 && HQKV_INDEX_OK(id[u], total)) ? A.tgt[id[u]] : -1;
+    for (int u = 0; u < PLAN_BATCH; ++u) tg[u] = (src[u] != -2 && HQKV_INDEX_OK(id[u], total)) ? S.tgt[id[u]] : -1;
 #pragma unroll
     for (int u = 0; u < PLAN_BATCH; ++u) {
-      if (src[u] == -2) continue;
       const int64_t s = first + (j0 + u) * 32 + lane;
-      int f;
-      if (tg[u] == 5) f = 5;
-      else if (src[u] < 0) f = tg[u] < 0 ? 6 : tg[u];
-      else f = tg[u] > src[u] ? tg[u] : src[u];  // only moves to fewer bits (larger index); tg == -1 stays
-      A.fin[s] = static_cast<int8_t>(f);
-      A.rank[id[u]] = (tg[u] != 5) ? 1 : 0;  // token ids are a permutation of 0..total-1 over the enumeration
-      if (f < HQKV_NUM_TIERS) atomicAdd(&cnt[2 * f + (src[u] == f ? 0 : 1)][warp], 1);
-    }
-  }
-  cluster.sync();
-  // 3. survivor counts per warp range of token ids
-  {
-    int mine = 0;
-    for (int64_t j0 = 0; j0 < iters; j0 += PLAN_BATCH) {
-      int fl[PLAN_BATCH];
-#pragma unroll
-      for (int u = 0; u < PLAN_BATCH; ++u) {
-        const int64_t i = first + (j0 + u) * 32 + lane;
-        fl[u] = (j0 + u < iters && i < total) ? A.rank[i] : 0;
+      int cat = PLAN_NONE;
+      if (src[u] != -2 && tg[u] != 5) {
+        const int f = tg[u] > src[u] ? tg[u] : src[u];  // only moves to fewer bits (larger index); tg == -1 stays
+        if (f >= 0) cat = 2 * f + (src[u] == f ? 0 : 1);
       }
-#pragma unroll
-      for (int u = 0; u < PLAN_BATCH; ++u) mine += fl[u];
+      if (src[u] != -2) S.fin[s] = static_cast<int8_t>(cat);
+      const unsigned same = __match_any_sync(0xffffffffu, cat);
+      if ((same & lt) == 0) cnt[cat][warp] += __popc(same);  // (one lane per category; the row is this warp's)
+      __syncwarp();
+      mine += own[u] != 5 ? 1 : 0;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-    if (lane == 0) cnt[PLAN_CATS - 1][warp] = mine;
   }
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  if (lane == 0) cnt[PLAN_CATS - 1][warp] = mine;
   __syncthreads();
   // this CTA's per-warp totals -> global memory, for the scan over all warps of the cluster
   if (tid < PLAN_CATS * PLAN_WARPS) {
     const int c = tid / PLAN_WARPS, w = tid - c * PLAN_WARPS;
-    A.gcnt[c * PLAN_GWARPS + crank * PLAN_WARPS + w] = cnt[c][w];
+    S.gcnt[c * PLAN_GWARPS + crank * PLAN_WARPS + w] = cnt[c][w];
   }
   cluster.sync();
-  // exclusive offsets of every category over the warps of the cluster (every CTA scans for its own warps)
-  if (tid < PLAN_CATS) {
-    int acc = 0;
-    for (int w = 0; w < PLAN_GWARPS; ++w) {
-      const int c = A.gcnt[tid * PLAN_GWARPS + w];
-      if (w >= crank * PLAN_WARPS && w < (crank + 1) * PLAN_WARPS) cnt[tid][w - crank * PLAN_WARPS] = acc;
-      acc += c;
+  // exclusive offsets of every category over the warps of the cluster (every CTA scans for its own warps): warp =
+  // category, eight cluster warps per lane
+  static_assert(PLAN_GWARPS == 256, "eight counts per lane");
+  if (warp < PLAN_CATS) {
+    const int4* g = reinterpret_cast<const int4*>(S.gcnt + warp * PLAN_GWARPS) + 2 * lane;
+    const int4 a = __ldcg(g), b = __ldcg(g + 1);
+    const int v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    int sum = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sum += v[i];
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += up;
     }
-    tot[tid] = acc;
+    int run = incl - sum;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int w = 8 * lane + i - crank * PLAN_WARPS;
+      if (w >= 0 && w < PLAN_WARPS) cnt[warp][w] = run;
+      run += v[i];
+    }
+    if (lane == 31) tot[warp] = incl;
   }
   __syncthreads();
-  const int any_evict = A.flags[0];
-  // 4. survivor ranks by token id: rank[i] = survivors with a smaller id; survivors[rank] = id
+  // 3. survivor ranks by token id: rank[i] = survivors with a smaller id; survivors[rank] = id
   {
     int running = cnt[PLAN_CATS - 1][warp];
     for (int64_t j0 = 0; j0 < iters; j0 += PLAN_BATCH) {
-      int fl[PLAN_BATCH];
+      int own[PLAN_BATCH];
 #pragma unroll
       for (int u = 0; u < PLAN_BATCH; ++u) {
         const int64_t i = first + (j0 + u) * 32 + lane;
-        fl[u] = (j0 + u < iters && i < total) ? A.rank[i] : -1;
+        own[u] = (j0 + u < iters && i < total) ? S.tgt[i] : 5;
       }
 #pragma unroll
       for (int u = 0; u < PLAN_BATCH; ++u) {
-        const unsigned ballot = __ballot_sync(0xffffffffu, fl[u] > 0);
+        const unsigned ballot = __ballot_sync(0xffffffffu, own[u] != 5);
         const int64_t i = first + (j0 + u) * 32 + lane;
         const int r = running + __popc(ballot & lt);
-        if (fl[u] >= 0) A.rank[i] = r;
-        if (fl[u] > 0) A.survivors[r] = i;
+        if (any_evict && i < total && j0 + u < iters) S.rank[i] = r;
+        if (own[u] != 5) S.survivors[r] = i;
         running += __popc(ballot);
       }
     }
   }
-  cluster.sync();
-  // 5. destination lists
-  {
-    for (int64_t j0 = 0; j0 < iters; j0 += PLAN_BATCH) {
-      int src[PLAN_BATCH], f[PLAN_BATCH];
-      int64_t pos[PLAN_BATCH], id[PLAN_BATCH];
+  if (any_evict) cluster.sync();
+  // 4. destination lists
+  for (int64_t j0 = 0; j0 < iters; j0 += PLAN_BATCH) {
+    int src[PLAN_BATCH], cat[PLAN_BATCH];
+    int32_t pos[PLAN_BATCH];
+    int64_t id[PLAN_BATCH];
 #pragma unroll
-      for (int u = 0; u < PLAN_BATCH; ++u) {
-        const int64_t s = first + (j0 + u) * 32 + lane;
-        src[u] = -2;
-        pos[u] = id[u] = 0;
-        f[u] = 6;
-        if (j0 + u < iters && s < total) {
-          enum_slot(A, s, src[u], pos[u], id[u]);
-          f[u] = A.fin[s];
-        }
+    for (int u = 0; u < PLAN_BATCH; ++u) {
+      const int64_t s = first + (j0 + u) * 32 + lane;
+      src[u] = -2;
+      pos[u] = 0;
+      id[u] = 0;
+      cat[u] = PLAN_NONE;
+      if (j0 + u < iters && s < total) {
+        enum_slot(A, S, s, src[u], pos[u], id[u]);
+        cat[u] = S.fin[s];
       }
-      int64_t outid[PLAN_BATCH];
+    }
+    if (any_evict) {
 #pragma unroll
       for (int u = 0; u < PLAN_BATCH; ++u)
-        outid[u] = (any_evict && f[u] < HQKV_NUM_TIERS) ? static_cast<int64_t>(A.rank[id[u]]) : id[u];
+        if (cat[u] != PLAN_NONE) id[u] = __ldcg(S.rank + id[u]);
+    }
 #pragma unroll
-      for (int u = 0; u < PLAN_BATCH; ++u) {
-        const bool on = f[u] < HQKV_NUM_TIERS;
-        const int cat = on ? 2 * f[u] + (src[u] == f[u] ? 0 : 1) : PLAN_CATS;  // PLAN_CATS: no destination
-        const unsigned same = __match_any_sync(0xffffffffu, cat);
-        if (on) {
-          const int base = cnt[cat][warp];  // this warp's running offset of the category (only this warp touches it)
-          const int64_t j = (cat & 1 ? tot[cat - 1] : 0) + base + __popc(same & lt);
-          A.plan_src[f[u] * total + j] = ((src[u] + 1) << 28) | static_cast<int32_t>(pos[u]);
-          A.plan_ids[f[u] * total + j] = outid[u];
-        }
-        __syncwarp();
-        if (on && (same & lt) == 0) cnt[cat][warp] += __popc(same);
-        __syncwarp();
+    for (int u = 0; u < PLAN_BATCH; ++u) {
+      const unsigned same = __match_any_sync(0xffffffffu, cat[u]);
+      const int base = cnt[cat[u]][warp];  // this warp's running offset of the category (only this warp touches it)
+      __syncwarp();
+      if (cat[u] != PLAN_NONE) {
+        const int64_t j = (cat[u] & 1 ? tot[cat[u] - 1] : 0) + base + __popc(same & lt), at = (cat[u] >> 1) * total + j;
+        S.plan_src[at] = ((src[u] + 1) << 28) | pos[u];
+        S.plan_ids[at] = id[u];
+        if ((same & lt) == 0) cnt[cat[u]][warp] = base + __popc(same);
       }
+      __syncwarp();
     }
   }
   if (crank == 0) {
-    if (tid < HQKV_NUM_TIERS) A.counts[tid] = tot[2 * tid] + tot[2 * tid + 1];
+    if (tid < HQKV_NUM_TIERS) S.counts[tid] = tot[2 * tid] + tot[2 * tid + 1];
     if (tid == 0) {
-      A.counts[5] = tot[PLAN_CATS - 1];
-      A.counts[6] = any_evict;
-      A.counts[7] = 0;
+      S.counts[5] = tot[PLAN_CATS - 1];
+      S.counts[6] = any_evict ? 1 : 0;
+      S.counts[7] = 0;
     }
   }
-  cluster.sync();  // no CTA of the cluster exits while another may still read its shared memory - none does, but the
-                   // barrier is cheap and keeps the exit orderly
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -747,19 +801,60 @@ extern "C" int hqkv_token_importance(const void* ring, int rows, int64_t ring_st
   return HQKV_OK;
 }
 
+// Ranges of T tokens behind the n_old that are copied.
+static int launch_range(const void* v, int B, int H, int64_t T, int64_t b_stride, int64_t h_stride, const void* old, int64_t n_old,
+                        void* out, void* stream) {
+  // tokens per CTA: one until every SM has four CTAs, then up to sixteen (32 KB of ranges at most)
+  const int n = B * H;
+  int tshift = 0;
+  while (tshift < 4 && T >> (tshift + 1) >= 4 * 148 && (static_cast<int64_t>(n) << (tshift + 2)) <= 2 * RANGE_MAX_ROWS) ++tshift;
+  const int64_t ctas = ceil_div(T, 1 << tshift), copies = ceil_div(n_old, 8 * RANGE_THREADS);
+  token_range128_kernel<<<static_cast<unsigned>(ctas + copies), RANGE_THREADS, (static_cast<size_t>(n) << tshift) * sizeof(__half),
+                          static_cast<cudaStream_t>(stream)>>>(static_cast<const __half*>(v), B, n, T, b_stride, h_stride, tshift,
+                                                               static_cast<const __half*>(old), n_old, static_cast<int>(ctas),
+                                                               static_cast<__half*>(out));
+  HQKV_LAUNCH_CHECK("token_range");
+  return HQKV_OK;
+}
+
 extern "C" int hqkv_token_range(const void* v, int B, int H, int64_t T, int Dd, int64_t b_stride, int64_t h_stride,
                                 void* out, void* stream) {
   HQKV_REQUIRE(B > 0 && H > 0 && T >= 0 && Dd >= 32, "token_range: bad sizes");
   if (T == 0) return HQKV_OK;
   HQKV_REQUIRE(v && out, "token_range: null pointer");
-  if (Dd == 128 && aligned(v, 8) && b_stride % 4 == 0 && h_stride % 4 == 0) {
-    token_range128_kernel<<<static_cast<unsigned>(ceil_div(T, 4)), 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __half*>(v), B, H, T, b_stride, h_stride, static_cast<__half*>(out));
-  } else {
-    token_range_kernel<<<static_cast<unsigned>(ceil_div(T, 4)), 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __half*>(v), B, H, T, Dd, b_stride, h_stride, static_cast<__half*>(out));
-  }
+  if (Dd == 128 && aligned(v, 16) && b_stride % 8 == 0 && h_stride % 8 == 0 && static_cast<int64_t>(B) * H <= RANGE_MAX_ROWS)
+    return launch_range(v, B, H, T, b_stride, h_stride, nullptr, 0, out, stream);
+  token_range_kernel<<<static_cast<unsigned>(ceil_div(T, 4)), 128, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const __half*>(v), B, H, T, Dd, b_stride, h_stride, static_cast<__half*>(out));
   HQKV_LAUNCH_CHECK("token_range");
+  return HQKV_OK;
+}
+
+static cudaLaunchConfig_t cluster_config(cudaLaunchAttribute* attr, int ctas, int rows, int threads, size_t smem, void* stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas, rows);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ctas;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// importance -> (x range) / block -> `divided` (may be importance itself) -> token ids in ranked order
+static int launch_rank(const void* importance, const void* range_or_null, void* divided, int block, int nblocks, int64_t* sorted_ids,
+                       void* stream) {
+  int npow2 = 2;
+  while (npow2 < nblocks) npow2 <<= 1;
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = cluster_config(attr, RANK_CLUSTER, 1, RANK_THREADS, npow2 * sizeof(uint32_t), stream);
+  HQKV_CUDA(cudaLaunchKernelEx(&cfg, block_rank_kernel, static_cast<const __half*>(importance),
+                               static_cast<const __half*>(range_or_null), static_cast<__half*>(divided), block, nblocks, npow2,
+                               sorted_ids));
   return HQKV_OK;
 }
 
@@ -769,31 +864,54 @@ extern "C" int hqkv_block_rank(void* importance, const void* range_or_null, int 
   HQKV_REQUIRE(nblocks <= RANK_MAX_BLOCKS, "block_rank: at most %d blocks (got %d)", RANK_MAX_BLOCKS, nblocks);
   if (nblocks == 0) return HQKV_OK;
   HQKV_REQUIRE(importance && sorted_ids, "block_rank: null pointer");
-  int npow2 = 2;
-  while (npow2 < nblocks) npow2 <<= 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(RANK_CLUSTER);
-  cfg.blockDim = dim3(RANK_THREADS);
-  cfg.dynamicSmemBytes = npow2 * sizeof(uint32_t);
-  cfg.stream = static_cast<cudaStream_t>(stream);
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = RANK_CLUSTER;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  HQKV_CUDA(cudaLaunchKernelEx(&cfg, block_rank_kernel, static_cast<__half*>(importance),
-                               static_cast<const __half*>(range_or_null), block, nblocks, npow2, sorted_ids));
-  return HQKV_OK;
+  return launch_rank(importance, range_or_null, importance, block, nblocks, sorted_ids, stream);
 }
 
 extern "C" size_t hqkv_flush_plan_workspace_bytes(int64_t total) {
   if (total < 0) return 0;
   const size_t t = static_cast<size_t>(total);
-  // tgt (1 B) + fin (1 B) + rank (4 B) per token, each region rounded to 256 bytes; per-warp counts; flags
+  // tgt (1 B) + fin (1 B) + rank (4 B) per token, each region rounded to 256 bytes; per-warp counts
   auto up = [](size_t v) { return (v + 255) & ~static_cast<size_t>(255); };
-  return up(t) + up(t) + up(4 * t) + up(sizeof(int32_t) * PLAN_CATS * PLAN_GWARPS) + 256;
+  return up(t) + up(t) + up(4 * t) + up(sizeof(int32_t) * PLAN_CATS * PLAN_GWARPS);
+}
+
+static int fill_plan_side(PlanSide& S, const int64_t* const* tier_idx_host, const int32_t* tier_n_host, int64_t hist, int64_t total,
+                          const int64_t* sorted_ids, const int64_t* cum_counts_host, int32_t* plan_src, int64_t* plan_ids,
+                          int64_t* survivors, int32_t* counts, unsigned char* ws) {
+  int64_t in_tiers = 0;
+  for (int t = 0; t < HQKV_NUM_TIERS; ++t) {
+    HQKV_REQUIRE(tier_n_host[t] >= 0, "flush_plan: negative tier size");
+    HQKV_REQUIRE(tier_n_host[t] == 0 || tier_idx_host[t], "flush_plan: tier %d has tokens but no id list", t);
+    S.tier_idx[t] = tier_idx_host[t];
+    S.tier_n[t] = tier_n_host[t];
+    in_tiers += tier_n_host[t];
+  }
+  HQKV_REQUIRE(in_tiers == hist, "flush_plan: tiers hold %lld tokens but history_length is %lld", (long long)in_tiers,
+               (long long)hist);
+  int64_t prev = 0;
+  for (int k = 0; k < 6; ++k) {
+    HQKV_REQUIRE(cum_counts_host[k] >= prev && cum_counts_host[k] <= total,
+                 "flush_plan: cumulative counts must be non-decreasing and at most hist+compress");
+    S.cum[k] = cum_counts_host[k];
+    prev = cum_counts_host[k];
+  }
+  auto up = [](size_t v) { return (v + 255) & ~static_cast<size_t>(255); };
+  S.tgt = reinterpret_cast<int8_t*>(ws);
+  S.fin = reinterpret_cast<int8_t*>(ws + up(total));
+  S.rank = reinterpret_cast<int32_t*>(ws + 2 * up(total));
+  S.gcnt = reinterpret_cast<int32_t*>(ws + 2 * up(total) + up(4 * static_cast<size_t>(total)));
+  S.sorted_ids = sorted_ids;
+  S.plan_src = plan_src;
+  S.plan_ids = plan_ids;
+  S.survivors = survivors;
+  S.counts = counts;
+  return HQKV_OK;
+}
+static int launch_plan(const PlanArgs& A, int sides, void* stream) {
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = cluster_config(attr, PLAN_CLUSTER, sides, PLAN_THREADS, 0, stream);
+  HQKV_CUDA(cudaLaunchKernelEx(&cfg, flush_plan_kernel, A));
+  return HQKV_OK;
 }
 
 extern "C" int hqkv_flush_plan(const int64_t* const* tier_idx_host, const int32_t* tier_n_host, int64_t hist,
@@ -805,55 +923,18 @@ extern "C" int hqkv_flush_plan(const int64_t* const* tier_idx_host, const int32_
   const int64_t total = hist + compress;
   HQKV_REQUIRE(total > 0 && total < (1ll << 28), "flush_plan: total length out of range");
   HQKV_REQUIRE(sorted_ids && plan_src && plan_ids && survivors && counts && workspace, "flush_plan: null pointer");
-  int64_t in_tiers = 0;
+  HQKV_REQUIRE(aligned(workspace, 16), "flush_plan: workspace must be 16-byte aligned");
   PlanArgs A;
   memset(&A, 0, sizeof(A));
-  for (int t = 0; t < HQKV_NUM_TIERS; ++t) {
-    HQKV_REQUIRE(tier_n_host[t] >= 0, "flush_plan: negative tier size");
-    HQKV_REQUIRE(tier_n_host[t] == 0 || tier_idx_host[t], "flush_plan: tier %d has tokens but no id list", t);
-    A.tier_idx[t] = tier_idx_host[t];
-    A.tier_n[t] = tier_n_host[t];
-    in_tiers += tier_n_host[t];
-  }
-  HQKV_REQUIRE(in_tiers == hist, "flush_plan: tiers hold %lld tokens but history_length is %lld", (long long)in_tiers,
-               (long long)hist);
-  int64_t prev = 0;
-  for (int k = 0; k < 6; ++k) {
-    HQKV_REQUIRE(cum_counts_host[k] >= prev && cum_counts_host[k] <= total,
-                 "flush_plan: cumulative counts must be non-decreasing and at most hist+compress");
-    A.cum[k] = cum_counts_host[k];
-    prev = cum_counts_host[k];
-  }
+  A.hist = hist;
+  A.compress = compress;
+  int rc = fill_plan_side(A.side[0], tier_idx_host, tier_n_host, hist, total, sorted_ids, cum_counts_host, plan_src, plan_ids,
+                          survivors, counts, static_cast<unsigned char*>(workspace));
+  if (rc) return rc;
   const size_t need = hqkv_flush_plan_workspace_bytes(total);
   if (workspace_bytes < need)
     return fail(HQKV_E_WORKSPACE, "flush_plan: workspace holds %zu bytes, %zu needed", workspace_bytes, need);
-  auto up = [](size_t v) { return (v + 255) & ~static_cast<size_t>(255); };
-  unsigned char* ws = static_cast<unsigned char*>(workspace);
-  A.tgt = reinterpret_cast<int8_t*>(ws);
-  A.fin = reinterpret_cast<int8_t*>(ws + up(total));
-  A.rank = reinterpret_cast<int32_t*>(ws + 2 * up(total));
-  A.gcnt = reinterpret_cast<int32_t*>(ws + 2 * up(total) + up(4 * static_cast<size_t>(total)));
-  A.flags = A.gcnt + ((up(sizeof(int32_t) * PLAN_CATS * PLAN_GWARPS)) / sizeof(int32_t));
-  A.hist = hist;
-  A.compress = compress;
-  A.sorted_ids = sorted_ids;
-  A.plan_src = plan_src;
-  A.plan_ids = plan_ids;
-  A.survivors = survivors;
-  A.counts = counts;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(PLAN_CLUSTER);
-  cfg.blockDim = dim3(PLAN_THREADS);
-  cfg.stream = static_cast<cudaStream_t>(stream);
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = PLAN_CLUSTER;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  HQKV_CUDA(cudaLaunchKernelEx(&cfg, flush_plan_kernel, A));
-  return HQKV_OK;
+  return launch_plan(A, 1, stream);
 }
 
 extern "C" int hqkv_flush_build_k(const hqkv_flush_src_t* src_host, int B, int H, int Dd, int group, int dst_tier,
