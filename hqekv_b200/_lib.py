@@ -98,6 +98,9 @@ _SIGNATURES = {
                                      C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "hqkv_flush_build_v": (C.c_int, [C.POINTER(FlushSrc), C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p,
                                      C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
+    "hqkv_flush_build": (C.c_int, [C.c_int, C.POINTER(FlushSrc), C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p,
+                                   C.c_int64, C.POINTER(C.c_int32), C.POINTER(C.c_void_p), C.POINTER(C.c_void_p),
+                                   C.POINTER(C.c_void_p), C.POINTER(C.c_void_p), C.c_int64, C.c_int64, C.c_void_p, C.c_void_p]),
     "hqkv_gather_columns_f16": (C.c_int, [C.c_void_p, C.c_int64, C.c_int, C.c_void_p, C.c_int64, C.c_void_p,
                                           C.c_int64, C.c_void_p]),
 }

@@ -19,7 +19,7 @@ CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB_PATH = os.path.join(HERE, "libhqkv.so")
 HOST_PATH = os.path.join(HERE, "_host.so")
-SOURCES = ["codec.cu", "decode.cu", "gemv.cu", "policy.cu"]
+SOURCES = ["codec.cu", "decode.cu", "flush.cu", "gemv.cu", "policy.cu"]
 NVCC_FLAGS = [
     "-std=c++17", "-O3", "-lineinfo",
     "-gencode", "arch=compute_100a,code=sm_100a",

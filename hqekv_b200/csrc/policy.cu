@@ -1,5 +1,5 @@
-// Importance bookkeeping, block ranking and the flush (evict + tier-assign + re-quantise) on the
-// device (sm_100a).  Integer / fp16 elementwise work on at most a few hundred thousand tokens; the
+// Importance bookkeeping, block ranking and the plan of the flush (evict + tier-assign; csrc/flush.cu builds the tiers) on
+// the device (sm_100a).  Integer / fp16 elementwise work on at most a few hundred thousand tokens; the
 // quantity that matters is bit-exact agreement with the reference's torch op sequence, so every
 // floating-point reduction here runs in a fixed order with one fp32 accumulator.
 #include <string.h>
@@ -509,217 +509,6 @@ __global__ void __launch_bounds__(PLAN_THREADS) flush_plan_kernel(const __grid_c
   }
 }
 
-// ------------------------------------------------------------------------------------------------
-// flush build
-// ------------------------------------------------------------------------------------------------
-struct BuildArgs {
-  const void* data[HQKV_NUM_TIERS];
-  const __half* scale[HQKV_NUM_TIERS];
-  const __half* zero[HQKV_NUM_TIERS];
-  int32_t n[HQKV_NUM_TIERS];
-  const __half* residual;
-  int64_t res_b_stride, res_h_stride;
-  int B, H, group, gshift, dst_tier, dst_bits;
-  int normal_dst;  // the destination is the 1-bit tier in the Gaussian-codebook codec
-  int per_warp;    // V side: destination tokens per warp
-  const int32_t* plan;  // [n_dst]
-  int64_t n_dst;
-  void* out_data;
-  __half* out_scale;
-  __half* out_zero;
-};
-
-__device__ __forceinline__ int tier_bits(int t) { return 16 >> t; }  // 16, 8, 4, 2, 1
-
-// K side: one CTA per (destination group of `group` tokens, batch*head); one thread per channel.
-// The tokens of a destination group come from one source and are consecutive there (tiers are
-// filled and emptied in whole blocks).
-__device__ __forceinline__ __half k_src_value(const BuildArgs& A, int src, int64_t pos, int b, int h, int d) {
-  const int64_t bh = static_cast<int64_t>(b) * A.H + h;
-  if (src < 0) return A.residual[b * A.res_b_stride + h * A.res_h_stride + pos * D + d];
-  const int64_t n = A.n[src];
-  if (src == 0) return reinterpret_cast<const __half*>(A.data[0])[(bh * D + d) * n + pos];
-  const int bits = tier_bits(src), fpi = 32 / bits;
-  const uint32_t word = reinterpret_cast<const uint32_t*>(A.data[src])[(bh * D + d) * (n / fpi) + pos / fpi];
-  const uint32_t code = (word >> ((pos % fpi) * bits)) & ((1u << bits) - 1u);
-  const int64_t G = n >> A.gshift;
-  const int64_t gi = (bh * D + d) * G + (pos >> A.gshift);
-  return dequant_2r(code, A.scale[src][gi], A.zero[src][gi]);
-}
-
-constexpr int BUILD_V_TOKENS_MAX = 8;  // destination tokens per warp when the grid would be scheduling-bound
-
-__device__ __forceinline__ void build_k_group(const BuildArgs& A, int64_t jg, int bh, int b, int h, int d) {
-  const int32_t enc = A.plan[jg * A.group];
-  const int src = (enc >> 28) - 1;
-  const int64_t pos0 = enc & 0x0FFFFFFF;
-  const int bits = A.dst_bits;
-  const int64_t row = static_cast<int64_t>(bh) * D + d;
-  if (bits == 16) {
-    __half* dst = reinterpret_cast<__half*>(A.out_data) + row * A.n_dst + jg * A.group;
-    for (int i = 0; i < A.group; ++i) dst[i] = k_src_value(A, src, pos0 + i, b, h, d);
-    return;
-  }
-  const int fpi = 32 / bits, wpg = A.group / fpi;
-  const int64_t Wd = A.n_dst / fpi, Gd = A.n_dst >> A.gshift;
-  uint32_t* dst = reinterpret_cast<uint32_t*>(A.out_data) + row * Wd + jg * wpg;
-  if (src == A.dst_tier) {  // kept block: copy words, scale, zero
-    const int64_t n = A.n[src];
-    const uint32_t* s = reinterpret_cast<const uint32_t*>(A.data[src]) + row * (n / fpi) + pos0 / fpi;
-    for (int w = 0; w < wpg; ++w) dst[w] = s[w];
-    const int64_t gi = row * (n >> A.gshift) + (pos0 >> A.gshift);
-    A.out_scale[row * Gd + jg] = A.scale[src][gi];
-    A.out_zero[row * Gd + jg] = A.zero[src][gi];
-    return;
-  }
-  if (A.normal_dst) {  // group statistics in fp64, then one code per token
-    double sum = 0.0;
-    for (int i = 0; i < A.group; ++i) sum += static_cast<double>(__half2float(k_src_value(A, src, pos0 + i, b, h, d)));
-    const double mean64 = sum / A.group;
-    double ss = 0.0;
-    for (int i = 0; i < A.group; ++i) {
-      const double dv = static_cast<double>(__half2float(k_src_value(A, src, pos0 + i, b, h, d))) - mean64;
-      ss += dv * dv;
-    }
-    const __half mean = __double2half(mean64), sd = normal1_sd(ss, A.group);
-    for (int w = 0; w < wpg; ++w) {
-      uint32_t word = 0;
-      for (int i = 0; i < 32; ++i) word |= normal1_code(k_src_value(A, src, pos0 + w * 32 + i, b, h, d), mean, sd) << i;
-      dst[w] = word;
-    }
-    A.out_scale[row * Gd + jg] = sd;
-    A.out_zero[row * Gd + jg] = mean;
-    return;
-  }
-  const float levels = static_cast<float>((1 << bits) - 1);
-  __half lo = k_src_value(A, src, pos0, b, h, d), hi = lo;
-  for (int i = 1; i < A.group; ++i) {
-    const __half v = k_src_value(A, src, pos0 + i, b, h, d);
-    lo = h_min(lo, v);
-    hi = h_max(hi, v);
-  }
-  const __half sc = quant_scale(lo, hi, levels);
-  const QuantGroup qg = quant_group(lo, sc, levels);
-  for (int w = 0; w < wpg; ++w) {
-    uint32_t word = 0;
-    for (int i = 0; i < fpi; ++i)
-      word |= quant_code_fast(k_src_value(A, src, pos0 + w * fpi + i, b, h, d), qg) << (i * bits);
-    dst[w] = word;
-  }
-  A.out_scale[row * Gd + jg] = sc;
-  A.out_zero[row * Gd + jg] = lo;
-}
-
-__global__ void __launch_bounds__(D) flush_build_k_kernel(const __grid_constant__ BuildArgs A) {
-  const int bh = blockIdx.y, b = bh / A.H, h = bh - b * A.H;
-  build_k_group(A, blockIdx.x, bh, b, h, threadIdx.x);  // one destination group per CTA
-}
-
-// V side: a warp per destination token of a (batch, head); a lane owns 4 consecutive channels.
-__device__ __forceinline__ void build_v_token(const BuildArgs& A, int64_t j, int bh, int b, int h, int lane) {
-  const int32_t enc = A.plan[j];
-  const int src = (enc >> 28) - 1;
-  const int64_t pos = enc & 0x0FFFFFFF;
-  const int bits = A.dst_bits;
-  const int ng = D >> A.gshift;
-  const int c0 = lane * 4;
-  // ---- source values of this lane's 4 channels
-  __half v[4];
-  if (src < 0) {
-    const __half* r = A.residual + b * A.res_b_stride + h * A.res_h_stride + pos * D + c0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = r[i];
-  } else if (src == 0) {
-    const __half* r = reinterpret_cast<const __half*>(A.data[0]) + (static_cast<int64_t>(bh) * A.n[0] + pos) * D + c0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = r[i];
-  } else {
-    const int sb = tier_bits(src), fpi = 32 / sb;
-    const int64_t trow = static_cast<int64_t>(bh) * A.n[src] + pos;
-    const uint32_t* words = reinterpret_cast<const uint32_t*>(A.data[src]) + trow * (D / fpi);
-    if (src == A.dst_tier) {  // kept token: copy the row verbatim
-      uint32_t* dw = reinterpret_cast<uint32_t*>(A.out_data) + (static_cast<int64_t>(bh) * A.n_dst + j) * (D / fpi);
-      for (int w = lane; w < D / fpi; w += 32) dw[w] = words[w];
-      if (lane < ng) {
-        A.out_scale[(static_cast<int64_t>(bh) * A.n_dst + j) * ng + lane] = A.scale[src][trow * ng + lane];
-        A.out_zero[(static_cast<int64_t>(bh) * A.n_dst + j) * ng + lane] = A.zero[src][trow * ng + lane];
-      }
-      return;
-    }
-    const __half sc = A.scale[src][trow * ng + (c0 >> A.gshift)];
-    const __half z = A.zero[src][trow * ng + (c0 >> A.gshift)];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int c = c0 + i;
-      const uint32_t code = (words[c / fpi] >> ((c % fpi) * sb)) & ((1u << sb) - 1u);
-      v[i] = dequant_2r(code, sc, z);
-    }
-  }
-  if (bits == 16) {
-    __half* dst = reinterpret_cast<__half*>(A.out_data) + (static_cast<int64_t>(bh) * A.n_dst + j) * D + c0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) dst[i] = v[i];
-    return;
-  }
-  // ---- quantise groups of `group` channels = group/4 adjacent lanes
-  __half lo, sc;  // zero and scale of the group (mean and std in the Gaussian-codebook codec)
-  uint32_t part = 0;
-  if (A.normal_dst) {
-    double sum = 0.0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) sum += static_cast<double>(__half2float(v[i]));
-    for (int off = 1; off < (A.group >> 2); off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-    const double mean64 = sum / A.group;
-    double ss = 0.0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const double dv = static_cast<double>(__half2float(v[i])) - mean64;
-      ss += dv * dv;
-    }
-    for (int off = 1; off < (A.group >> 2); off <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-    lo = __double2half(mean64);
-    sc = normal1_sd(ss, A.group);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) part |= normal1_code(v[i], lo, sc) << i;
-  } else {
-    const float levels = static_cast<float>((1 << bits) - 1);
-    __half hi = v[0];
-    lo = v[0];
-#pragma unroll
-    for (int i = 1; i < 4; ++i) {
-      lo = h_min(lo, v[i]);
-      hi = h_max(hi, v[i]);
-    }
-    for (int off = 1; off < (A.group >> 2); off <<= 1) {
-      lo = h_min(lo, __shfl_xor_sync(0xffffffffu, lo, off));
-      hi = h_max(hi, __shfl_xor_sync(0xffffffffu, hi, off));
-    }
-    sc = quant_scale(lo, hi, levels);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) part |= quant_code_fast(v[i], quant_group(lo, sc, levels)) << (i * bits);
-  }
-  const int lpw = 32 / (4 * bits);  // lanes per word: 1, 2, 4, 8 for 8, 4, 2, 1 bits
-  for (int off = 1; off < lpw; off <<= 1) {
-    const uint32_t other = __shfl_down_sync(0xffffffffu, part, off);
-    part |= other << (4 * bits * off);
-  }
-  const int fpi = 32 / bits;
-  uint32_t* dw = reinterpret_cast<uint32_t*>(A.out_data) + (static_cast<int64_t>(bh) * A.n_dst + j) * (D / fpi);
-  if (lane % lpw == 0) dw[lane / lpw] = part;
-  if ((c0 & (A.group - 1)) == 0) {
-    A.out_scale[(static_cast<int64_t>(bh) * A.n_dst + j) * ng + (c0 >> A.gshift)] = sc;
-    A.out_zero[(static_cast<int64_t>(bh) * A.n_dst + j) * ng + (c0 >> A.gshift)] = lo;
-  }
-}
-
-__global__ void __launch_bounds__(128) flush_build_v_kernel(const __grid_constant__ BuildArgs A) {
-  const int lane = threadIdx.x & 31;
-  const int bh = blockIdx.y, b = bh / A.H, h = bh - b * A.H;
-  const int64_t j0 = (static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5)) * A.per_warp;
-  for (int i = 0; i < A.per_warp; ++i)
-    if (j0 + i < A.n_dst) build_v_token(A, j0 + i, bh, b, h, lane);  // the whole warp takes the same branch
-}
-
 __global__ void __launch_bounds__(256) gather_columns_kernel(const __half* __restrict__ in, int64_t in_stride,
                                                              const int64_t* __restrict__ ids, int64_t n,
                                                              __half* __restrict__ out, int64_t out_stride) {
@@ -727,52 +516,6 @@ __global__ void __launch_bounds__(256) gather_columns_kernel(const __half* __res
   if (j >= n) return;
   const int r = blockIdx.y;
   out[r * out_stride + j] = in[r * in_stride + ids[j]];
-}
-
-static int ilog2(int v) {
-  int s = 0;
-  while ((1 << s) < v) ++s;
-  return s;
-}
-
-static int fill_build_args(BuildArgs& A, const hqkv_flush_src_t* src, int B, int H, int Dd, int group, int dst_tier,
-                           const int32_t* plan, int64_t n_dst, void* out_data, void* out_scale, void* out_zero,
-                           const char* who) {
-  HQKV_REQUIRE(src != nullptr, "%s: null source descriptor", who);
-  HQKV_REQUIRE(Dd == D, "%s: head dim must be 128", who);
-  HQKV_REQUIRE(B > 0 && H > 0 && static_cast<int64_t>(B) * H <= 65535, "%s: bad B/H", who);
-  HQKV_REQUIRE(valid_group(group), "%s: group must be 32, 64 or 128", who);
-  HQKV_REQUIRE(dst_tier >= 0 && dst_tier < HQKV_NUM_TIERS, "%s: dst_tier out of range", who);
-  HQKV_REQUIRE(n_dst >= 0, "%s: negative n_dst", who);
-  memset(&A, 0, sizeof(A));
-  for (int t = 0; t < HQKV_NUM_TIERS; ++t) {
-    A.data[t] = src->data[t];
-    A.scale[t] = static_cast<const __half*>(src->scale[t]);
-    A.zero[t] = static_cast<const __half*>(src->zero[t]);
-    A.n[t] = src->n[t];
-  }
-  A.residual = static_cast<const __half*>(src->residual);
-  A.res_b_stride = src->residual_b_stride;
-  A.res_h_stride = src->residual_h_stride;
-  A.B = B;
-  A.H = H;
-  A.group = group;
-  A.gshift = ilog2(group);
-  A.dst_tier = dst_tier;
-  A.dst_bits = 16 >> dst_tier;
-  HQKV_REQUIRE(src->low_codec == HQKV_CODEC_UNIFORM || src->low_codec == HQKV_CODEC_NORMAL, "%s: unknown low_codec %d",
-               who, src->low_codec);
-  A.normal_dst = (A.dst_bits == 1 && src->low_codec == HQKV_CODEC_NORMAL) ? 1 : 0;
-  A.plan = plan;
-  A.n_dst = n_dst;
-  A.out_data = out_data;
-  A.out_scale = static_cast<__half*>(out_scale);
-  A.out_zero = static_cast<__half*>(out_zero);
-  if (n_dst > 0) {
-    HQKV_REQUIRE(plan && out_data, "%s: null pointer", who);
-    HQKV_REQUIRE(dst_tier == 0 || (out_scale && out_zero), "%s: null scale/zero output", who);
-  }
-  return HQKV_OK;
 }
 
 }  // namespace hqkv
@@ -935,41 +678,6 @@ extern "C" int hqkv_flush_plan(const int64_t* const* tier_idx_host, const int32_
   if (workspace_bytes < need)
     return fail(HQKV_E_WORKSPACE, "flush_plan: workspace holds %zu bytes, %zu needed", workspace_bytes, need);
   return launch_plan(A, 1, stream);
-}
-
-extern "C" int hqkv_flush_build_k(const hqkv_flush_src_t* src_host, int B, int H, int Dd, int group, int dst_tier,
-                                  const int32_t* plan_src_row, int64_t n_dst, void* out_data, void* out_scale,
-                                  void* out_zero, void* stream) {
-  BuildArgs A;
-  int rc = fill_build_args(A, src_host, B, H, Dd, group, dst_tier, plan_src_row, n_dst, out_data, out_scale, out_zero,
-                           "flush_build_k");
-  if (rc) return rc;
-  if (n_dst == 0) return HQKV_OK;
-  HQKV_REQUIRE(n_dst % group == 0, "flush_build_k: n_dst (%lld) is not a multiple of the group %d", (long long)n_dst,
-               group);
-  flush_build_k_kernel<<<dim3(static_cast<unsigned>(n_dst / group), B * H), D, 0,
-                         static_cast<cudaStream_t>(stream)>>>(A);
-  HQKV_LAUNCH_CHECK("flush_build_k");
-  return HQKV_OK;
-}
-
-extern "C" int hqkv_flush_build_v(const hqkv_flush_src_t* src_host, int B, int H, int Dd, int group, int dst_tier,
-                                  const int32_t* plan_src_row, int64_t n_dst, void* out_data, void* out_scale,
-                                  void* out_zero, void* stream) {
-  BuildArgs A;
-  int rc = fill_build_args(A, src_host, B, H, Dd, group, dst_tier, plan_src_row, n_dst, out_data, out_scale, out_zero,
-                           "flush_build_v");
-  if (rc) return rc;
-  if (n_dst == 0) return HQKV_OK;
-  // a token row is little work for a warp: beyond ~64k CTAs the launch is bound by CTA scheduling and warps
-  // take several tokens each (222 -> 169 us at 200k CTAs); smaller launches are faster with one token per warp
-  const int64_t ctas = ceil_div(n_dst, 4) * B * H;
-  const int64_t per = ceil_div(ctas, 65536);
-  A.per_warp = static_cast<int>(per < 1 ? 1 : per > BUILD_V_TOKENS_MAX ? BUILD_V_TOKENS_MAX : per);
-  flush_build_v_kernel<<<dim3(static_cast<unsigned>(ceil_div(n_dst, 4 * A.per_warp)), B * H), 128, 0,
-                         static_cast<cudaStream_t>(stream)>>>(A);
-  HQKV_LAUNCH_CHECK("flush_build_v");
-  return HQKV_OK;
 }
 
 extern "C" int hqkv_gather_columns_f16(const void* in, int64_t in_stride, int rows, const int64_t* ids, int64_t n,

@@ -425,6 +425,16 @@ int hqkv_flush_build_v(const hqkv_flush_src_t* src_host, int B, int H, int D, in
                        const int32_t* plan_src_row, int64_t n_dst, void* out_data, void* out_scale, void* out_zero,
                        void* stream);
 
+/*
+ * Phase 2 for a whole side in one launch: all five destination tiers (counts_host[t] tokens each; outputs as above, one
+ * pointer per tier, ignored where the count is 0), their id lists (plan_ids -> out_ids_host[t]), and the copy of the `rest`
+ * tokens of the residual window behind the first `compress` ones to rest_out [B,H,rest,D].
+ */
+int hqkv_flush_build(int v_side, const hqkv_flush_src_t* src_host, int B, int H, int D, int group,
+                     const int32_t* plan_src, const int64_t* plan_ids, int64_t total, const int32_t* counts_host,
+                     void* const* out_data_host, void* const* out_scale_host, void* const* out_zero_host,
+                     int64_t* const* out_ids_host, int64_t compress, int64_t rest, void* rest_out, void* stream);
+
 /* out[r, j] = in[r, ids[j]] for fp16 rows — compaction of V_token_norm and of the importance ring to the
  * survivors (quant/hqe_2.py:733-735, last_attn_weights.eviction model/public_func.py:228-231).
  * in/out may not overlap. */
