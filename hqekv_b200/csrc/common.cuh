@@ -128,7 +128,12 @@ __device__ __forceinline__ __half dequant_2r(uint32_t code, __half scale, __half
 
 // Gaussian-codebook codec at 1 bit.  std and mean of a group are torch.std_mean (unbiased) of its fp16
 // values: computed in fp64 (the sum of up to 128 fp16 values is exact there) and rounded once to fp16.
+// The fp64 divide and square root take longer than everything else about a group; fp32 ones are off by less than 2^-22,
+// which decides the fp16 rounding of all but one group in a thousand.
 __device__ __forceinline__ __half normal1_sd(double sum_sq_dev, int group) {
+  const float s = __fsqrt_rn(__fdividef(static_cast<float>(sum_sq_dev), static_cast<float>(group - 1)));
+  const __half below = __float2half_rn(s * (1.f - 0x1p-21f)), above = __float2half_rn(s * (1.f + 0x1p-21f));
+  if (s > 1e-6f && s < 6e4f && __half_as_ushort(below) == __half_as_ushort(above)) return below;
   return __double2half(sqrt(sum_sq_dev / (group - 1)));
 }
 // code = 1 where half(half(x - mean) / std) > 0 (decision bounds [0, inf]); a NaN quotient gives 0

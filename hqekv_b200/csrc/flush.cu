@@ -211,8 +211,9 @@ __device__ __noinline__ void k_normal_group(const BuildArgs& A, KBuildShared& sh
       sum[1] += static_cast<double>(__high2float(v[t]));
     }
   }
-  mean64[0] = sum[0] / group;
-  mean64[1] = sum[1] / group;
+  const double share = 1.0 / static_cast<double>(group);  // a power of two: exact
+  mean64[0] = sum[0] * share;
+  mean64[1] = sum[1] * share;
   for (int i = 0; i < per; ++i) {
     if (per > 1) k_load32(A, sh.src[s0], sh.pos[s0] + 32 * i, bh, ch, v);
 #pragma unroll
@@ -439,7 +440,7 @@ __device__ __forceinline__ uint64_t v_quantise8(const __half2 (&v)[4], int gshif
     double sum = a + b;
     for (int off = 1; off < lpg; off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
     const int group = 1 << gshift;
-    const double mean64 = sum / group;
+    const double mean64 = sum * (1.0 / static_cast<double>(group));  // a power of two: exact
     a = b = 0.0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {

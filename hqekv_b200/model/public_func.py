@@ -41,6 +41,9 @@ def get_block_token_idx(block_size: int, block_num: int, importance: torch.Tenso
     divided by the block length IN PLACE, as the reference does to its argument; blocks are ordered by
     descending fp16 key, equal keys by ascending block id (the reference's default torch.sort leaves
     ties unspecified).  Returns the int64 token ids, block by block."""
+    done = host.block_rank(importance, _range, block_size, block_num)
+    if done is not None:
+        return done
     require_cuda(importance)
     if importance.dtype != torch.float16 or not importance.is_contiguous():
         raise ValueError("importance must be a contiguous float16 tensor")
@@ -84,6 +87,9 @@ class last_attn_weights:
 
     def calculate_token_importance(self):
         L = self.kv_seq_len
+        done = host.token_importance(self.weights, self.last_length, L)
+        if done is not None:
+            return done
         out = torch.empty(L, dtype=torch.float16, device=self.weights.device)
         with torch.cuda.device(self.weights.device):
             check(lib.hqkv_token_importance(ptr(self.weights), self.last_length, self.weights.stride(0), L, ptr(out),

@@ -9,7 +9,7 @@ copy of ten integers in between to size the new tensors.
 """
 import torch
 
-from .._lib import CODEC_NORMAL, CODEC_UNIFORM, TIER_BITS, check, lib, ptr, require_cuda, stream_ptr
+from .._lib import CODEC_NORMAL, CODEC_UNIFORM, TIER_BITS, check, host, lib, ptr, require_cuda, stream_ptr
 from ..model.public_func import calculate_token_range, get_block_token_idx, last_attn_weights
 from ._cache import (NUM_SLOTS, SLOT_K, SLOT_NEW_K, SLOT_NEW_V, SLOT_SEQ_LEN, SLOT_V, SLOT_V_TOKEN_NORM,
                      build_flush_src, cache_geometry, tier_tensors, void_p_array)
@@ -104,11 +104,18 @@ def KV_cache_hqe_2(past_key_value: tuple, compress_length: int, history_length: 
     if len(past_key_value) != NUM_SLOTS:
         raise ValueError("invalid past_key_value")
     cache = tuple(past_key_value)
+    compress_length, history_length = int(compress_length), int(history_length)
+    if last_weights is None or type(last_weights) is last_attn_weights:
+        done = host.flush(cache, compress_length, history_length, K_sorted_idx, _as_int_list(K_bit_num), _as_int_list(V_bit_num),
+                          token_importance, low_codec, None if last_weights is None else last_weights.weights, block_size,
+                          group_size, times_range)
+        if done is not None:
+            return done
+    # what the native path does not take as it is: operands to be made contiguous, and everything that is an error
     new_K, new_V = cache[SLOT_NEW_K], cache[SLOT_NEW_V]
     if new_K is None or new_V is None:
         raise ValueError("invalid past_key_value")
     require_cuda(new_K, new_V, token_importance)
-    compress_length, history_length = int(compress_length), int(history_length)
     dev = new_K.device
     B, H, _, D = new_K.shape
     res_K = new_K[:, :, compress_length:, :].clone()

@@ -435,6 +435,38 @@ int hqkv_flush_build(int v_side, const hqkv_flush_src_t* src_host, int B, int H,
                      void* const* out_data_host, void* const* out_scale_host, void* const* out_zero_host,
                      int64_t* const* out_ids_host, int64_t compress, int64_t rest, void* rest_out, void* stream);
 
+/*
+ * A whole flush (KV_cache_hqe_2, quant/hqe_2.py:456-843) in three calls, for hosts that keep launches and allocations few:
+ *   hqkv_flush_prepare   value ranges of the flushed tokens appended to norm_old (-> norm_out, hist + compress fp16),
+ *                        V ranking from `importance` (as ranked for K, i.e. divided by the block size; not modified) and,
+ *                        with times_range, those ranges; the plans of both sides; reads the counts back
+ *                        (counts_host[0..8) K, [8..16) V as in hqkv_flush_plan) and waits for the stream
+ *   hqkv_flush_tiers     hqkv_flush_build of one side from that plan
+ *   hqkv_flush_evict     compacts norm_out to the V-side survivors (-> norm_kept) and moves the survivors' columns of an
+ *                        importance ring (fp16 [rows][stride], null: none) to the front, in place
+ * `workspace`: hqkv_flush_workspace_bytes(hist + compress) bytes, 256-byte aligned, kept between the calls.
+ */
+typedef struct {
+  int32_t B, H, D, block, group, times_range;  /* block: K group = ranking block; group: V group */
+  int64_t hist, compress, rest;                /* cached tokens, tokens to flush, tokens that stay in the window */
+  hqkv_flush_src_t k, v;                       /* tiers of both sides; residual = the window [B,H,compress+rest,D] */
+  const int64_t* k_idx[HQKV_NUM_TIERS];
+  const int64_t* v_idx[HQKV_NUM_TIERS];
+  const void* importance;                      /* fp16 [hist + compress] */
+  const int64_t* k_sorted;                     /* ranked ids of the K side */
+  int64_t k_cum[6], v_cum[6];                  /* cumulative tier counts, see hqkv_flush_plan */
+  const void* norm_old;                        /* fp16 [hist], null if hist = 0 */
+  void* norm_out;
+} hqkv_flush_t;
+size_t hqkv_flush_workspace_bytes(int64_t total);
+int hqkv_flush_prepare(const hqkv_flush_t* flush_host, void* workspace, size_t workspace_bytes, int32_t* counts_host,
+                       void* stream);
+int hqkv_flush_tiers(const hqkv_flush_t* flush_host, int v_side, const void* workspace, const int32_t* counts_host,
+                     void* const* out_data_host, void* const* out_scale_host, void* const* out_zero_host,
+                     int64_t* const* out_ids_host, void* rest_out, void* stream);
+int hqkv_flush_evict(const hqkv_flush_t* flush_host, const void* workspace, int64_t survivors, void* norm_kept, void* ring,
+                     int64_t ring_stride, int ring_rows, void* stream);
+
 /* out[r, j] = in[r, ids[j]] for fp16 rows — compaction of V_token_norm and of the importance ring to the
  * survivors (quant/hqe_2.py:733-735, last_attn_weights.eviction model/public_func.py:228-231).
  * in/out may not overlap. */
