@@ -389,12 +389,12 @@ __global__ void __launch_bounds__(128) normal1_quantize_kernel(const __half* __r
     ss += d * d;
   }
   const __half mean = __double2half(mean64);
-  const __half sd = normal1_sd(ss, group);
+  const __half sd = normal1_sd(ss, group), bound = normal1_bound(sd);
   uint32_t* dst = code + (row * T + gi * group) / 32;
   for (int w = 0; w < group / 32; ++w) {
     uint32_t word = 0;
     for (int i = 0; i < 32; ++i) {
-      word |= normal1_code(src[(w * 32 + i) * t_stride], mean, sd) << i;
+      word |= normal1_code(src[(w * 32 + i) * t_stride], mean, bound) << i;
     }
     dst[w] = word;
   }

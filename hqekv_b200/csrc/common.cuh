@@ -128,17 +128,35 @@ __device__ __forceinline__ __half dequant_2r(uint32_t code, __half scale, __half
 
 // Gaussian-codebook codec at 1 bit.  std and mean of a group are torch.std_mean (unbiased) of its fp16
 // values: computed in fp64 (the sum of up to 128 fp16 values is exact there) and rounded once to fp16.
-// The fp64 divide and square root take longer than everything else about a group; fp32 ones are off by less than 2^-22,
-// which decides the fp16 rounding of all but one group in a thousand.
 __device__ __forceinline__ __half normal1_sd(double sum_sq_dev, int group) {
-  const float s = __fsqrt_rn(__fdividef(static_cast<float>(sum_sq_dev), static_cast<float>(group - 1)));
-  const __half below = __float2half_rn(s * (1.f - 0x1p-21f)), above = __float2half_rn(s * (1.f + 0x1p-21f));
-  if (s > 1e-6f && s < 6e4f && __half_as_ushort(below) == __half_as_ushort(above)) return below;
   return __double2half(sqrt(sum_sq_dev / (group - 1)));
 }
-// code = 1 where half(half(x - mean) / std) > 0 (decision bounds [0, inf]); a NaN quotient gives 0
-__device__ __forceinline__ uint32_t normal1_code(__half x, __half mean, __half sd) {
-  return __half2float(h_div(h_sub(x, mean), sd)) > 0.f ? 1u : 0u;
+// The same from fp32 sums, which decide the fp16 rounding of nearly every group (conversions to fp64, its divide and its
+// square root take longer than everything else about a group): s + c = sum of the values, compensated; ss = sum of
+// squared deviations from it, at most 40 additions deep.  False where a bound on their error - 2^-22 of the mean, unless
+// the values cancel to less than 2^-13 of their spread, and 2^-19 of the deviation - straddles a rounding boundary.
+__device__ __forceinline__ bool normal1_fast(float s, float c, float ss, int group, __half& mean, __half& sd) {
+  const float m = (s + c) * (1.f / static_cast<float>(group));  // the group is a power of two
+  const float d = __fsqrt_rn(__fdividef(ss, static_cast<float>(group - 1)));
+  mean = __float2half_rn(m * (1.f - 0x1p-22f));
+  sd = __float2half_rn(d * (1.f - 0x1p-19f));
+  return __half_as_ushort(mean) == __half_as_ushort(__float2half_rn(m * (1.f + 0x1p-22f))) &&
+         __half_as_ushort(sd) == __half_as_ushort(__float2half_rn(d * (1.f + 0x1p-19f))) && fabsf(m) >= d * 0x1p-13f && d > 1e-6f &&
+         d < 6e4f && fabsf(m) < 6e4f;
+}
+// x added to s + c, the rounding error of the addition kept in c
+__device__ __forceinline__ void add_compensated(float& s, float& c, float x) {
+  const float t = __fadd_rn(s, x), back = __fsub_rn(t, s);
+  c += __fadd_rn(__fsub_rn(s, __fsub_rn(t, back)), __fsub_rn(x, back));
+  s = t;
+}
+// code = 1 where half(half(x - mean) / std) > 0 (decision bounds [0, inf]; a NaN quotient gives 0).  The quotient of two
+// halfs rounds to zero up to 2^-25, so that is half(x - mean) > std * 2^-25, rounded down to a half (0 below std = 2).
+__device__ __forceinline__ __half normal1_bound(__half sd) { return __float2half_rd(__half2float(sd) * 0x1p-25f); }
+__device__ __forceinline__ uint32_t normal1_code(__half x, __half mean, __half bound) { return __hgt(h_sub(x, mean), bound) ? 1u : 0u; }
+// two elements: codes in bits 0 and 16
+__device__ __forceinline__ uint32_t normal1_code2(__half2 x, __half2 mean, __half2 bound) {
+  return __hgt2_mask(__hsub2(x, mean), bound) & 0x00010001u;
 }
 #define HQKV_NORMAL1_CENTER 0.67448974f
 

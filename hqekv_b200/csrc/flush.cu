@@ -191,56 +191,78 @@ __device__ __forceinline__ void k_quantise32(const __half2 (&v)[32], const Quant
   }
 }
 
-// code of the Gaussian codebook as normal1_code, the quotient by the group's reciprocal (see quant_quotient)
-__device__ __forceinline__ uint32_t normal_code(__half x, __half mean, __half sd, const QuantGroup& g, bool plain) {
-  if (!plain) return normal1_code(x, mean, sd);
-  return __half2float(__float2half_rn(quant_quotient(__half2float(__hsub(x, mean)), g))) > 0.f ? 1u : 0u;
-}
-__device__ __forceinline__ bool plain_sd(__half sd) { return __half2float(sd) > 0.f && !__hisinf(sd); }
-
-// One arrival group of the codebook tier, channels ch and ch + 1: statistics in fp64 in token order.
-__device__ __noinline__ void k_normal_group(const BuildArgs& A, KBuildShared& sh, int bh, int g, int ch) {
-  const int per = 1 << (A.gshift - 5), s0 = g * per, group = 1 << A.gshift;
+// fp64 statistics of a group of the codebook tier in token order, channels ch and ch + 1: mean, std
+__device__ __noinline__ void k_normal_stats(const BuildArgs& A, int src, int64_t pos, int bh, int ch, __half2& mean, __half2& sd) {
+  const int group = 1 << A.gshift;
+  double sum[2] = {0.0, 0.0}, ss[2] = {0.0, 0.0};
   __half2 v[32];
-  double sum[2] = {0.0, 0.0}, ss[2] = {0.0, 0.0}, mean64[2];
+  for (int pass = 0; pass < 2; ++pass)
+    for (int i = 0; i < group; i += 32) {
+      k_load32(A, src, pos + i, bh, ch, v);
+#pragma unroll
+      for (int t = 0; t < 32; ++t) {
+        const double a = static_cast<double>(__low2float(v[t])), b = static_cast<double>(__high2float(v[t]));
+        if (pass == 0) {
+          sum[0] += a;
+          sum[1] += b;
+        } else {
+          const double x = a - sum[0] / group, y = b - sum[1] / group;
+          ss[0] += x * x;
+          ss[1] += y * y;
+        }
+      }
+    }
+  mean = __halves2half2(__double2half(sum[0] / group), __double2half(sum[1] / group));
+  sd = __halves2half2(normal1_sd(ss[0], group), normal1_sd(ss[1], group));
+}
+
+// One arrival group of the codebook tier, channels ch and ch + 1.
+__device__ __noinline__ void k_normal_group(const BuildArgs& A, KBuildShared& sh, int bh, int g, int ch) {
+  const int per = 1 << (A.gshift - 5), s0 = g * per, group = 1 << A.gshift, src = sh.src[s0];
+  const int64_t pos = sh.pos[s0];
+  __half2 v[32];
+  float s[2] = {0.f, 0.f}, c[2] = {0.f, 0.f}, ss[2][4] = {};
   for (int i = 0; i < per; ++i) {
-    k_load32(A, sh.src[s0], sh.pos[s0] + 32 * i, bh, ch, v);
+    k_load32(A, src, pos + 32 * i, bh, ch, v);
 #pragma unroll
     for (int t = 0; t < 32; ++t) {
-      sum[0] += static_cast<double>(__low2float(v[t]));
-      sum[1] += static_cast<double>(__high2float(v[t]));
+      add_compensated(s[0], c[0], __low2float(v[t]));
+      add_compensated(s[1], c[1], __high2float(v[t]));
     }
   }
-  const double share = 1.0 / static_cast<double>(group);  // a power of two: exact
-  mean64[0] = sum[0] * share;
-  mean64[1] = sum[1] * share;
+  const float m0 = (s[0] + c[0]) / static_cast<float>(group), m1 = (s[1] + c[1]) / static_cast<float>(group);
   for (int i = 0; i < per; ++i) {
-    if (per > 1) k_load32(A, sh.src[s0], sh.pos[s0] + 32 * i, bh, ch, v);
+    if (per > 1) k_load32(A, src, pos + 32 * i, bh, ch, v);
 #pragma unroll
     for (int t = 0; t < 32; ++t) {
-      const double a = static_cast<double>(__low2float(v[t])) - mean64[0], b = static_cast<double>(__high2float(v[t])) - mean64[1];
-      ss[0] += a * a;
-      ss[1] += b * b;
+      const float a = __low2float(v[t]) - m0, b = __high2float(v[t]) - m1;
+      ss[0][t & 3] = fmaf(a, a, ss[0][t & 3]);
+      ss[1][t & 3] = fmaf(b, b, ss[1][t & 3]);
     }
   }
-  const __half m0 = __double2half(mean64[0]), m1 = __double2half(mean64[1]), d0 = normal1_sd(ss[0], group), d1 = normal1_sd(ss[1], group);
-  const QuantGroup q0 = quant_group(m0, d0, 1.f), q1 = quant_group(m1, d1, 1.f);
-  const bool p0 = plain_sd(d0), p1 = plain_sd(d1);
+  __half mean[2], sd[2];
+  bool sure = true;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) sure &= normal1_fast(s[k], c[k], (ss[k][0] + ss[k][1]) + (ss[k][2] + ss[k][3]), group, mean[k], sd[k]);
+  __half2 mean2 = __halves2half2(mean[0], mean[1]), sd2 = __halves2half2(sd[0], sd[1]);
+  if (!sure) k_normal_stats(A, src, pos, bh, ch, mean2, sd2);
+  const __half2 bound = __halves2half2(normal1_bound(__low2half(sd2)), normal1_bound(__high2half(sd2)));
   for (int i = 0; i < per; ++i) {
-    if (per > 1) k_load32(A, sh.src[s0], sh.pos[s0] + 32 * i, bh, ch, v);
+    if (per > 1) k_load32(A, src, pos + 32 * i, bh, ch, v);
     uint32_t a = 0, b = 0;
 #pragma unroll
     for (int t = 0; t < 32; ++t) {
-      a |= normal_code(__low2half(v[t]), m0, d0, q0, p0) << t;
-      b |= normal_code(__high2half(v[t]), m1, d1, q1, p1) << t;
+      const uint32_t k = normal1_code2(v[t], mean2, bound);
+      a |= (k & 1u) << t;
+      b |= (k >> 16) << t;
     }
     sh.words[ch * 33 + s0 + i] = a;
     sh.words[(ch + 1) * 33 + s0 + i] = b;
   }
-  sh.s[ch * KB_MAX_SUBS + g] = d0;
-  sh.z[ch * KB_MAX_SUBS + g] = m0;
-  sh.s[(ch + 1) * KB_MAX_SUBS + g] = d1;
-  sh.z[(ch + 1) * KB_MAX_SUBS + g] = m1;
+  sh.s[ch * KB_MAX_SUBS + g] = __low2half(sd2);
+  sh.z[ch * KB_MAX_SUBS + g] = __low2half(mean2);
+  sh.s[(ch + 1) * KB_MAX_SUBS + g] = __high2half(sd2);
+  sh.z[(ch + 1) * KB_MAX_SUBS + g] = __high2half(mean2);
 }
 
 template <int PIECE>
@@ -276,6 +298,22 @@ __device__ __forceinline__ void k_build_tile(const BuildArgs& A, KBuildShared& s
   __syncthreads();
   const int piece = tid & 7, r0 = tid >> 3, sub = KB::sub_of(piece);
   const bool mine = sub < nsub, kept = mine && sh.src[sub] == t;
+  // scales of kept groups, requested together with their codes
+  constexpr int SPT = 4;                                                 // scales per thread at most
+  const int gs = (BITS == 8 ? 7 : 8) - A.gshift;                         // log2(groups per tile)
+  const int64_t Gd = dst.n >> A.gshift, Gs = static_cast<int64_t>(A.n[t]) >> A.gshift, g0 = j0 >> A.gshift;
+  __half ks[SPT], kz[SPT];
+  if constexpr (BITS < 16) {
+#pragma unroll
+    for (int k = 0; k < SPT; ++k) {
+      const int i = tid + k * BUILD_THREADS, r = i >> gs, first = (i & ((1 << gs) - 1)) << (A.gshift - 5);
+      if (i < D << gs && first < nsub && sh.src[first] == t) {
+        const int64_t from = (static_cast<int64_t>(bh) * D + r) * Gs + (sh.pos[first] >> A.gshift);
+        ks[k] = A.scale[t][from];
+        kz[k] = A.zero[t][from];
+      }
+    }
+  }
   const int64_t out_row = dst.n * BITS / 8;
   unsigned char* out = reinterpret_cast<unsigned char*>(dst.data) + static_cast<int64_t>(bh) * D * out_row + j0 * BITS / 8 + piece * KB::PIECE;
   if (kept) {
@@ -374,21 +412,14 @@ __device__ __forceinline__ void k_build_tile(const BuildArgs& A, KBuildShared& s
     }
   }
   if constexpr (BITS < 16) {
-    const int gs = (BITS == 8 ? 7 : 8) - A.gshift;                       // log2(groups per tile)
-    const int64_t Gd = dst.n >> A.gshift, Gs = static_cast<int64_t>(A.n[t]) >> A.gshift, g0 = j0 >> A.gshift;
-#pragma unroll 4
-    for (int i = tid; i < D << gs; i += BUILD_THREADS) {
-      const int r = i >> gs, g = i & ((1 << gs) - 1), first = g << (A.gshift - 5);
-      if (first >= nsub) continue;
-      const int64_t row = static_cast<int64_t>(bh) * D + r, at = row * Gd + g0 + g;
-      if (sh.src[first] == t) {
-        const int64_t from = row * Gs + (sh.pos[first] >> A.gshift);
-        dst.scale[at] = A.scale[t][from];
-        dst.zero[at] = A.zero[t][from];
-      } else {
-        dst.scale[at] = sh.s[r * KB_MAX_SUBS + g];
-        dst.zero[at] = sh.z[r * KB_MAX_SUBS + g];
-      }
+#pragma unroll
+    for (int k = 0; k < SPT; ++k) {
+      const int i = tid + k * BUILD_THREADS, r = i >> gs, g = i & ((1 << gs) - 1), first = g << (A.gshift - 5);
+      if (i >= D << gs || first >= nsub) continue;
+      const int64_t at = (static_cast<int64_t>(bh) * D + r) * Gd + g0 + g;
+      const bool kept_group = sh.src[first] == t;
+      dst.scale[at] = kept_group ? ks[k] : sh.s[r * KB_MAX_SUBS + g];
+      dst.zero[at] = kept_group ? kz[k] : sh.z[r * KB_MAX_SUBS + g];
     }
   }
 }
@@ -418,6 +449,35 @@ __device__ __forceinline__ __half v_get(const void* p, int bits, int c) {  // co
   return __uint2half_rn((w >> ((c * bits) & 31)) & ((1u << bits) - 1u));
 }
 
+// fp64 statistics of a group of the codebook tier: sums of four channels, then pairwise over the group
+__device__ __noinline__ void v_normal_stats(const __half2 (&v)[4], int gshift, __half& mean, __half& sd) {
+  const int lpg = 1 << (gshift - 3), group = 1 << gshift;
+  double x[8], a = 0.0, b = 0.0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    x[2 * i] = static_cast<double>(__low2float(v[i]));
+    x[2 * i + 1] = static_cast<double>(__high2float(v[i]));
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    a += x[i];
+    b += x[4 + i];
+  }
+  double sum = a + b;
+  for (int off = 1; off < lpg; off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+  const double mean64 = sum / group;
+  a = b = 0.0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    a += (x[i] - mean64) * (x[i] - mean64);
+    b += (x[4 + i] - mean64) * (x[4 + i] - mean64);
+  }
+  double ss = a + b;
+  for (int off = 1; off < lpg; off <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+  mean = __double2half(mean64);
+  sd = normal1_sd(ss, group);
+}
+
 // Eight values quantised in groups of 2^gshift channels = 2^(gshift-3) adjacent lanes; codes -> `part`, the lane's group
 // scale and zero (std and mean) -> sc, lo.
 template <int BITS>
@@ -425,37 +485,36 @@ __device__ __forceinline__ uint64_t v_quantise8(const __half2 (&v)[4], int gshif
   const int lpg = 1 << (gshift - 3), lane = threadIdx.x & 31;
   uint64_t part = 0;
   if (BITS == 1 && normal) {
-    // sums of four channels, then pairwise over the group
-    double x[8], a = 0.0, b = 0.0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      x[2 * i] = static_cast<double>(__low2float(v[i]));
-      x[2 * i + 1] = static_cast<double>(__high2float(v[i]));
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      a += x[i];
-      b += x[4 + i];
-    }
-    double sum = a + b;
-    for (int off = 1; off < lpg; off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
     const int group = 1 << gshift;
-    const double mean64 = sum * (1.0 / static_cast<double>(group));  // a power of two: exact
-    a = b = 0.0;
+    float s = 0.f, c = 0.f, ss = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      a += (x[i] - mean64) * (x[i] - mean64);
-      b += (x[4 + i] - mean64) * (x[4 + i] - mean64);
+      add_compensated(s, c, __low2float(v[i]));
+      add_compensated(s, c, __high2float(v[i]));
     }
-    double ss = a + b;
-    for (int off = 1; off < lpg; off <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-    lo = __double2half(mean64);
-    sc = normal1_sd(ss, group);
-    const QuantGroup g = quant_group(lo, sc, 1.f);
-    const bool plain = plain_sd(sc);
+    for (int off = 1; off < lpg; off <<= 1) {
+      const float s2 = __shfl_xor_sync(0xffffffffu, s, off);
+      c += __shfl_xor_sync(0xffffffffu, c, off);
+      add_compensated(s, c, s2);
+    }
+    const float m = __shfl_sync(0xffffffffu, (s + c) / static_cast<float>(group), lane & ~(lpg - 1));
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      part |= static_cast<uint64_t>(normal_code(i & 1 ? __high2half(v[i >> 1]) : __low2half(v[i >> 1]), lo, sc, g, plain)) << i;
+    for (int i = 0; i < 4; ++i) {
+      const float a = __low2float(v[i]) - m, b = __high2float(v[i]) - m;
+      ss = fmaf(a, a, fmaf(b, b, ss));
+    }
+    for (int off = 1; off < lpg; off <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+    const bool sure = normal1_fast(s, c, ss, group, lo, sc);
+    const int first = lane & ~(lpg - 1);
+    if (__any_sync(0xffffffffu, !sure)) v_normal_stats(v, gshift, lo, sc);
+    lo = __shfl_sync(0xffffffffu, lo, first);  // one lane's result for the group
+    sc = __shfl_sync(0xffffffffu, sc, first);
+    const __half2 mean2 = __half2half2(lo), bound = __half2half2(normal1_bound(sc));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t k = normal1_code2(v[i], mean2, bound);
+      part |= static_cast<uint64_t>((k & 1u) | (k >> 15)) << (2 * i);
+    }
     return part;
   }
   constexpr float levels = static_cast<float>((1 << BITS) - 1);

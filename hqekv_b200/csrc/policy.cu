@@ -120,12 +120,13 @@ __global__ void __launch_bounds__(128) token_range_kernel(const __half* __restri
 // a time: with 32 tokens of 64 rows each the whole launch was eight warps long (41 us; 31 us for 32 k tokens of 8 rows).
 // CTA = 2^tshift tokens; `old` = the ranges of the tokens before these, copied to the front of `out` by the CTAs behind.
 constexpr int RANGE_THREADS = 256;
-constexpr int RANGE_MAX_ROWS = 8192;
+constexpr int RANGE_MAX_ROWS = 4096;
 __global__ void __launch_bounds__(RANGE_THREADS) token_range128_kernel(const __half* __restrict__ v, int B, int n, int64_t T,
                                                                        int64_t b_stride, int64_t h_stride, int tshift,
                                                                        const __half* __restrict__ old, int64_t n_old, int ctas,
                                                                        __half* __restrict__ out) {
-  extern __shared__ __half range_s[];  // [token][row], row = h * B + b
+  extern __shared__ uint32_t row_at[];  // [row = h * B + b] first element / 8, then the ranges [token][row]
+  __half* range_s = reinterpret_cast<__half*>(row_at + n);
   const int tid = threadIdx.x;
   if (static_cast<int>(blockIdx.x) >= ctas) {
     const int64_t base = (static_cast<int64_t>(blockIdx.x) - ctas) * RANGE_THREADS * 8 + tid;
@@ -134,6 +135,8 @@ __global__ void __launch_bounds__(RANGE_THREADS) token_range128_kernel(const __h
       if (base + j * RANGE_THREADS < n_old) out[base + j * RANGE_THREADS] = old[base + j * RANGE_THREADS];
     return;
   }
+  for (int r = tid; r < n; r += RANGE_THREADS) row_at[r] = static_cast<uint32_t>(((r % B) * b_stride + (r / B) * h_stride) >> 3);
+  __syncthreads();
   const int hw = tid >> 4, l16 = tid & 15, tpc = 1 << tshift;
   const int64_t t0 = static_cast<int64_t>(blockIdx.x) << tshift;
   const int items = n << tshift;  // token fastest: neighbouring half-warps read neighbouring rows of memory
@@ -141,9 +144,9 @@ __global__ void __launch_bounds__(RANGE_THREADS) token_range128_kernel(const __h
     uint4 w[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int it = min(base + u * (RANGE_THREADS / 16), items - 1), r = it >> tshift, h = r / B, b = r - h * B;
+      const int it = min(base + u * (RANGE_THREADS / 16), items - 1);
       const int64_t t = min(t0 + (it & (tpc - 1)), T - 1);
-      w[u] = *reinterpret_cast<const uint4*>(v + b * b_stride + h * h_stride + t * 128 + 8 * l16);
+      w[u] = reinterpret_cast<const uint4*>(v)[row_at[it >> tshift] + t * 16 + l16];
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -552,7 +555,7 @@ static int launch_range(const void* v, int B, int H, int64_t T, int64_t b_stride
   int tshift = 0;
   while (tshift < 4 && T >> (tshift + 1) >= 4 * 148 && (static_cast<int64_t>(n) << (tshift + 2)) <= 2 * RANGE_MAX_ROWS) ++tshift;
   const int64_t ctas = ceil_div(T, 1 << tshift), copies = ceil_div(n_old, 8 * RANGE_THREADS);
-  token_range128_kernel<<<static_cast<unsigned>(ctas + copies), RANGE_THREADS, (static_cast<size_t>(n) << tshift) * sizeof(__half),
+  token_range128_kernel<<<static_cast<unsigned>(ctas + copies), RANGE_THREADS, n * sizeof(uint32_t) + (static_cast<size_t>(n) << tshift) * sizeof(__half),
                           static_cast<cudaStream_t>(stream)>>>(static_cast<const __half*>(v), B, n, T, b_stride, h_stride, tshift,
                                                                static_cast<const __half*>(old), n_old, static_cast<int>(ctas),
                                                                static_cast<__half*>(out));
