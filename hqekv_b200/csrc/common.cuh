@@ -133,15 +133,16 @@ __device__ __forceinline__ __half normal1_sd(double sum_sq_dev, int group) {
 }
 // The same from fp32 sums, which decide the fp16 rounding of nearly every group (conversions to fp64, its divide and its
 // square root take longer than everything else about a group): s + c = sum of the values, compensated; ss = sum of
-// squared deviations from it, at most 40 additions deep.  False where a bound on their error - 2^-22 of the mean, unless
-// the values cancel to less than 2^-13 of their spread, and 2^-19 of the deviation - straddles a rounding boundary.
+// squared deviations from it, in four or more partial sums.  False where a bound on their error - 2^-22 of the mean, unless
+// the values cancel to less than 2^-13 of their spread, and (group / 8 + 6) * 2^-25 of the deviation, which is 2^-21.6 for 32 -
+// straddles a rounding boundary: one group in some 500.
 __device__ __forceinline__ bool normal1_fast(float s, float c, float ss, int group, __half& mean, __half& sd) {
   const float m = (s + c) * (1.f / static_cast<float>(group));  // the group is a power of two
-  const float d = __fsqrt_rn(__fdividef(ss, static_cast<float>(group - 1)));
+  const float d = __fsqrt_rn(__fdividef(ss, static_cast<float>(group - 1))), off = d * (static_cast<float>(group) * 0x1p-27f + 0x1p-22f);
   mean = __float2half_rn(m * (1.f - 0x1p-22f));
-  sd = __float2half_rn(d * (1.f - 0x1p-19f));
+  sd = __float2half_rn(d - off);
   return __half_as_ushort(mean) == __half_as_ushort(__float2half_rn(m * (1.f + 0x1p-22f))) &&
-         __half_as_ushort(sd) == __half_as_ushort(__float2half_rn(d * (1.f + 0x1p-19f))) && fabsf(m) >= d * 0x1p-13f && d > 1e-6f &&
+         __half_as_ushort(sd) == __half_as_ushort(__float2half_rn(d + off)) && fabsf(m) >= d * 0x1p-13f && d > 1e-6f &&
          d < 6e4f && fabsf(m) < 6e4f;
 }
 // x added to s + c, the rounding error of the addition kept in c

@@ -424,7 +424,7 @@ __device__ __forceinline__ void k_build_tile(const BuildArgs& A, KBuildShared& s
   }
 }
 
-__global__ void __launch_bounds__(BUILD_THREADS, 3) flush_build_k_kernel(const __grid_constant__ BuildArgs A) {
+__global__ void __launch_bounds__(BUILD_THREADS, 4) flush_build_k_kernel(const __grid_constant__ BuildArgs A) {
   __shared__ KBuildShared sh;
   const int x = blockIdx.x, bh = blockIdx.y;
   if (x >= A.tiles) {
