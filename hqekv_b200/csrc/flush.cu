@@ -194,26 +194,29 @@ __device__ __forceinline__ void k_quantise32(const __half2 (&v)[32], const Quant
 // fp64 statistics of a group of the codebook tier in token order, channels ch and ch + 1: mean, std
 __device__ __noinline__ void k_normal_stats(const BuildArgs& A, int src, int64_t pos, int bh, int ch, __half2& mean, __half2& sd) {
   const int group = 1 << A.gshift;
-  double sum[2] = {0.0, 0.0}, ss[2] = {0.0, 0.0};
+  const double share = static_cast<double>(1.f / static_cast<float>(group));  // (exact: a power of two)
+  double s0 = 0.0, s1 = 0.0, q0 = 0.0, q1 = 0.0;
   __half2 v[32];
-  for (int pass = 0; pass < 2; ++pass)
-    for (int i = 0; i < group; i += 32) {
-      k_load32(A, src, pos + i, bh, ch, v);
+  for (int i = 0; i < group; i += 32) {
+    k_load32(A, src, pos + i, bh, ch, v);
 #pragma unroll
-      for (int t = 0; t < 32; ++t) {
-        const double a = static_cast<double>(__low2float(v[t])), b = static_cast<double>(__high2float(v[t]));
-        if (pass == 0) {
-          sum[0] += a;
-          sum[1] += b;
-        } else {
-          const double x = a - sum[0] / group, y = b - sum[1] / group;
-          ss[0] += x * x;
-          ss[1] += y * y;
-        }
-      }
+    for (int t = 0; t < 32; ++t) {
+      s0 += static_cast<double>(__low2float(v[t]));
+      s1 += static_cast<double>(__high2float(v[t]));
     }
-  mean = __halves2half2(__double2half(sum[0] / group), __double2half(sum[1] / group));
-  sd = __halves2half2(normal1_sd(ss[0], group), normal1_sd(ss[1], group));
+  }
+  const double m0 = s0 * share, m1 = s1 * share;
+  for (int i = 0; i < group; i += 32) {
+    if (group > 32) k_load32(A, src, pos + i, bh, ch, v);
+#pragma unroll
+    for (int t = 0; t < 32; ++t) {
+      const double a = static_cast<double>(__low2float(v[t])) - m0, b = static_cast<double>(__high2float(v[t])) - m1;
+      q0 += a * a;
+      q1 += b * b;
+    }
+  }
+  mean = __halves2half2(__double2half(m0), __double2half(m1));
+  sd = __halves2half2(normal1_sd(q0, group), normal1_sd(q1, group));
 }
 
 // One arrival group of the codebook tier, channels ch and ch + 1.
@@ -221,21 +224,27 @@ __device__ __noinline__ void k_normal_group(const BuildArgs& A, KBuildShared& sh
   const int per = 1 << (A.gshift - 5), s0 = g * per, group = 1 << A.gshift, src = sh.src[s0];
   const int64_t pos = sh.pos[s0];
   __half2 v[32];
-  float s[2] = {0.f, 0.f}, c[2] = {0.f, 0.f}, ss[2][4] = {};
+  float s[2][2] = {}, c[2][2] = {}, ss[2][4] = {};
   for (int i = 0; i < per; ++i) {
     k_load32(A, src, pos + 32 * i, bh, ch, v);
 #pragma unroll
     for (int t = 0; t < 32; ++t) {
-      add_compensated(s[0], c[0], __low2float(v[t]));
-      add_compensated(s[1], c[1], __high2float(v[t]));
+      add_compensated(s[0][t & 1], c[0][t & 1], __low2float(v[t]));
+      add_compensated(s[1][t & 1], c[1][t & 1], __high2float(v[t]));
     }
   }
-  const float m0 = (s[0] + c[0]) / static_cast<float>(group), m1 = (s[1] + c[1]) / static_cast<float>(group);
+  float m[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    c[k][0] += c[k][1];
+    add_compensated(s[k][0], c[k][0], s[k][1]);
+    m[k] = (s[k][0] + c[k][0]) * (1.f / static_cast<float>(group));
+  }
   for (int i = 0; i < per; ++i) {
     if (per > 1) k_load32(A, src, pos + 32 * i, bh, ch, v);
 #pragma unroll
     for (int t = 0; t < 32; ++t) {
-      const float a = __low2float(v[t]) - m0, b = __high2float(v[t]) - m1;
+      const float a = __low2float(v[t]) - m[0], b = __high2float(v[t]) - m[1];
       ss[0][t & 3] = fmaf(a, a, ss[0][t & 3]);
       ss[1][t & 3] = fmaf(b, b, ss[1][t & 3]);
     }
@@ -243,7 +252,8 @@ __device__ __noinline__ void k_normal_group(const BuildArgs& A, KBuildShared& sh
   __half mean[2], sd[2];
   bool sure = true;
 #pragma unroll
-  for (int k = 0; k < 2; ++k) sure &= normal1_fast(s[k], c[k], (ss[k][0] + ss[k][1]) + (ss[k][2] + ss[k][3]), group, mean[k], sd[k]);
+  for (int k = 0; k < 2; ++k)
+    sure &= normal1_fast(s[k][0], c[k][0], (ss[k][0] + ss[k][1]) + (ss[k][2] + ss[k][3]), group, mean[k], sd[k]);
   __half2 mean2 = __halves2half2(mean[0], mean[1]), sd2 = __halves2half2(sd[0], sd[1]);
   if (!sure) k_normal_stats(A, src, pos, bh, ch, mean2, sd2);
   const __half2 bound = __halves2half2(normal1_bound(__low2half(sd2)), normal1_bound(__high2half(sd2)));
@@ -442,242 +452,246 @@ __global__ void __launch_bounds__(BUILD_THREADS, 4) flush_build_k_kernel(const _
 // V side: token-major tiers, groups of channels per token
 // ------------------------------------------------------------------------------------------------
 // A warp takes 32 consecutive destination tokens of a (batch, head).  Blocks of tokens move together, so they are nearly always
-// consecutive in one source (one vote): kept ones are then a contiguous copy, 16 bytes per lane, and arrivals are two tokens
-// per step, eight channels per lane.  Any other run of tokens goes one by one.
+// consecutive in one source (one vote): kept ones are then a contiguous copy, 16 bytes per lane, and arrivals are eight
+// tokens per step, 32 channels per lane: a group's scale and reciprocal are one lane's.  (With eight channels per lane four
+// lanes repeated them, and those instructions were most of the kernel.)  Any other run of tokens goes one by one.
 __device__ __forceinline__ __half v_get(const void* p, int bits, int c) {  // code c of a packed row
   const uint32_t w = reinterpret_cast<const uint32_t*>(p)[c * bits / 32];
   return __uint2half_rn((w >> ((c * bits) & 31)) & ((1u << bits) - 1u));
 }
 
 // fp64 statistics of a group of the codebook tier: sums of four channels, then pairwise over the group
-__device__ __noinline__ void v_normal_stats(const __half2 (&v)[4], int gshift, __half& mean, __half& sd) {
-  const int lpg = 1 << (gshift - 3), group = 1 << gshift;
-  double x[8], a = 0.0, b = 0.0;
+__device__ __forceinline__ void v_normal_stats(const __half2 (&v)[16], int gshift, __half& mean, __half& sd) {
+  const int lanes = 1 << (gshift - 5), group = 1 << gshift;
+  auto over_group = [&](auto value) {
+    double part[8];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    x[2 * i] = static_cast<double>(__low2float(v[i]));
-    x[2 * i + 1] = static_cast<double>(__high2float(v[i]));
-  }
+    for (int q = 0; q < 8; ++q) {
+      part[q] = 0.0;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    a += x[i];
-    b += x[4 + i];
-  }
-  double sum = a + b;
-  for (int off = 1; off < lpg; off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-  const double mean64 = sum / group;
-  a = b = 0.0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    a += (x[i] - mean64) * (x[i] - mean64);
-    b += (x[4 + i] - mean64) * (x[4 + i] - mean64);
-  }
-  double ss = a + b;
-  for (int off = 1; off < lpg; off <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+      for (int i = 0; i < 4; ++i) part[q] += value(i & 1 ? __high2float(v[2 * q + (i >> 1)]) : __low2float(v[2 * q + (i >> 1)]));
+    }
+    double sum = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
+    for (int off = 1; off < lanes; off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    return sum;
+  };
+  const double mean64 = over_group([](float x) { return static_cast<double>(x); }) * static_cast<double>(1.f / static_cast<float>(group));
+  const double ss = over_group([&](float x) {
+    const double d = static_cast<double>(x) - mean64;
+    return d * d;
+  });
   mean = __double2half(mean64);
   sd = normal1_sd(ss, group);
 }
 
-// Eight values quantised in groups of 2^gshift channels = 2^(gshift-3) adjacent lanes; codes -> `part`, the lane's group
-// scale and zero (std and mean) -> sc, lo.
+// 32 values per lane quantised in groups of 2^(gshift - 5) adjacent lanes; codes -> words, the group's scale and zero (std
+// and mean) -> sc, lo.  The whole warp takes part.
 template <int BITS>
-__device__ __forceinline__ uint64_t v_quantise8(const __half2 (&v)[4], int gshift, bool normal, __half& sc, __half& lo) {
-  const int lpg = 1 << (gshift - 3), lane = threadIdx.x & 31;
-  uint64_t part = 0;
+__device__ __forceinline__ void v_quantise32(const __half2 (&v)[16], int gshift, bool normal, uint32_t (&words)[BITS], __half& sc, __half& lo) {
+  const int lanes = 1 << (gshift - 5), lane = threadIdx.x & 31, first = lane & ~(lanes - 1);
   if (BITS == 1 && normal) {
     const int group = 1 << gshift;
-    float s = 0.f, c = 0.f, ss = 0.f;
+    float s[2] = {0.f, 0.f}, c[2] = {0.f, 0.f}, ss[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      add_compensated(s, c, __low2float(v[i]));
-      add_compensated(s, c, __high2float(v[i]));
+    for (int i = 0; i < 16; ++i) {
+      add_compensated(s[0], c[0], __low2float(v[i]));
+      add_compensated(s[1], c[1], __high2float(v[i]));
     }
-    for (int off = 1; off < lpg; off <<= 1) {
-      const float s2 = __shfl_xor_sync(0xffffffffu, s, off);
-      c += __shfl_xor_sync(0xffffffffu, c, off);
-      add_compensated(s, c, s2);
+    c[0] += c[1];
+    add_compensated(s[0], c[0], s[1]);
+    for (int off = 1; off < lanes; off <<= 1) {
+      const float other = __shfl_xor_sync(0xffffffffu, s[0], off);
+      c[0] += __shfl_xor_sync(0xffffffffu, c[0], off);
+      add_compensated(s[0], c[0], other);
     }
-    const float m = __shfl_sync(0xffffffffu, (s + c) / static_cast<float>(group), lane & ~(lpg - 1));
+    const float m = __shfl_sync(0xffffffffu, (s[0] + c[0]) * (1.f / static_cast<float>(group)), first);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < 16; ++i) {
       const float a = __low2float(v[i]) - m, b = __high2float(v[i]) - m;
-      ss = fmaf(a, a, fmaf(b, b, ss));
+      ss[(2 * i) & 3] = fmaf(a, a, ss[(2 * i) & 3]);
+      ss[(2 * i + 1) & 3] = fmaf(b, b, ss[(2 * i + 1) & 3]);
     }
-    for (int off = 1; off < lpg; off <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-    const bool sure = normal1_fast(s, c, ss, group, lo, sc);
-    const int first = lane & ~(lpg - 1);
+    float sq = (ss[0] + ss[1]) + (ss[2] + ss[3]);
+    for (int off = 1; off < lanes; off <<= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
+    const bool sure = normal1_fast(s[0], c[0], sq, group, lo, sc);
     if (__any_sync(0xffffffffu, !sure)) v_normal_stats(v, gshift, lo, sc);
     lo = __shfl_sync(0xffffffffu, lo, first);  // one lane's result for the group
     sc = __shfl_sync(0xffffffffu, sc, first);
     const __half2 mean2 = __half2half2(lo), bound = __half2half2(normal1_bound(sc));
+    uint32_t w = 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < 16; ++i) {
       const uint32_t k = normal1_code2(v[i], mean2, bound);
-      part |= static_cast<uint64_t>((k & 1u) | (k >> 15)) << (2 * i);
+      w |= ((k | (k >> 15)) & 3u) << (2 * i);
     }
-    return part;
+    words[0] = w;
+    return;
   }
   constexpr float levels = static_cast<float>((1 << BITS) - 1);
-  const __half2 lo2 = __hmin2_nan(__hmin2_nan(v[0], v[1]), __hmin2_nan(v[2], v[3]));
-  const __half2 hi2 = __hmax2_nan(__hmax2_nan(v[0], v[1]), __hmax2_nan(v[2], v[3]));
+  __half2 lo2 = v[0], hi2 = v[0];
+#pragma unroll
+  for (int i = 1; i < 16; ++i) {
+    lo2 = __hmin2_nan(lo2, v[i]);
+    hi2 = __hmax2_nan(hi2, v[i]);
+  }
   // minimum and negated maximum together
   __half2 m = __halves2half2(__hmin_nan(__low2half(lo2), __high2half(lo2)), __hneg(__hmax_nan(__low2half(hi2), __high2half(hi2))));
-  for (int off = 1; off < lpg; off <<= 1) m = __hmin2_nan(m, __shfl_xor_sync(0xffffffffu, m, off));
+  for (int off = 1; off < lanes; off <<= 1) m = __hmin2_nan(m, __shfl_xor_sync(0xffffffffu, m, off));
   lo = __low2half(m);
   __half hi = __hneg(__high2half(m));
   if (__any_sync(0xffffffffu, doubtful(lo, hi))) {  // element by element, the first lane of a group decides
     __half l = __low2half(v[0]), h = l;
 #pragma unroll
-    for (int i = 1; i < 8; ++i) {
+    for (int i = 1; i < 32; ++i) {
       const __half x = i & 1 ? __high2half(v[i >> 1]) : __low2half(v[i >> 1]);
       l = h_min(l, x);
       h = h_max(h, x);
     }
-    for (int off = 1; off < lpg; off <<= 1) {
+    for (int off = 1; off < lanes; off <<= 1) {
       l = h_min(l, __shfl_xor_sync(0xffffffffu, l, off));
       h = h_max(h, __shfl_xor_sync(0xffffffffu, h, off));
     }
-    lo = __shfl_sync(0xffffffffu, l, lane & ~(lpg - 1));
-    hi = __shfl_sync(0xffffffffu, h, lane & ~(lpg - 1));
+    lo = __shfl_sync(0xffffffffu, l, first);
+    hi = __shfl_sync(0xffffffffu, h, first);
   }
   sc = quant_scale(lo, hi, levels);
   const QuantGroup g = quant_group(lo, sc, levels);
+  constexpr int FPI = 32 / BITS;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint32_t c = quant_code_fast2(v[i], g);
-    part |= static_cast<uint64_t>((c & 0xFFFFu) | ((c >> 16) << BITS)) << (2 * i * BITS);
+  for (int w = 0; w < BITS; ++w) {
+    uint32_t word = 0;
+#pragma unroll
+    for (int i = 0; i < FPI / 2; ++i) {
+      const uint32_t c = quant_code_fast2(v[(w * FPI) / 2 + i], g);
+      word |= ((c & 0xFFFFu) | ((c >> 16) << BITS)) << (2 * i * BITS);
+    }
+    words[w] = word;
   }
-  return part;
 }
-// Store a lane's eight channels (BITS bytes) of token j and, from the first lane of a group, its scale and zero.
+// Store a lane's quarter q of token `tok` (32 channels, 4 * BITS bytes) and, from the first lane of a group, its scale and
+// zero.  live: the lane has a token.
 template <int BITS>
-__device__ __forceinline__ void v_store8(const BuildArgs& A, const BuildDst& dst, int64_t tok, int l16, const __half2 (&v)[4]) {
-  unsigned char* row = reinterpret_cast<unsigned char*>(dst.data) + tok * (16 * BITS) + l16 * BITS;
+__device__ __forceinline__ void v_store32(const BuildArgs& A, const BuildDst& dst, int64_t tok, int q, const __half2 (&v)[16], bool live) {
+  uint32_t* row = reinterpret_cast<uint32_t*>(dst.data) + tok * (4 * BITS) + q * BITS;
   if constexpr (BITS == 16) {
-    *reinterpret_cast<uint4*>(row) = make_uint4(as_u32(v[0]), as_u32(v[1]), as_u32(v[2]), as_u32(v[3]));
+    if (live) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        reinterpret_cast<uint4*>(row)[i] = make_uint4(as_u32(v[4 * i]), as_u32(v[4 * i + 1]), as_u32(v[4 * i + 2]), as_u32(v[4 * i + 3]));
+    }
   } else {
     __half sc, lo;
-    const uint64_t part = v_quantise8<BITS>(v, A.gshift, A.normal_low != 0, sc, lo);
-    if constexpr (BITS == 8) *reinterpret_cast<uint2*>(row) = make_uint2(static_cast<uint32_t>(part), static_cast<uint32_t>(part >> 32));
-    else if constexpr (BITS == 4) *reinterpret_cast<uint32_t*>(row) = static_cast<uint32_t>(part);
-    else if constexpr (BITS == 2) *reinterpret_cast<uint16_t*>(row) = static_cast<uint16_t>(part);
-    else *row = static_cast<unsigned char>(part);
-    if ((l16 & ((1 << (A.gshift - 3)) - 1)) == 0) {
-      const int64_t at = tok * (D >> A.gshift) + (l16 >> (A.gshift - 3));
+    uint32_t w[BITS];
+    v_quantise32<BITS>(v, A.gshift, A.normal_low != 0, w, sc, lo);
+    if (!live) return;
+    if constexpr (BITS == 8) {
+      reinterpret_cast<uint4*>(row)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+      reinterpret_cast<uint4*>(row)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    } else if constexpr (BITS == 4) {
+      *reinterpret_cast<uint4*>(row) = make_uint4(w[0], w[1], w[2], w[3]);
+    } else if constexpr (BITS == 2) {
+      *reinterpret_cast<uint2*>(row) = make_uint2(w[0], w[1]);
+    } else {
+      *row = w[0];
+    }
+    if ((q & ((1 << (A.gshift - 5)) - 1)) == 0) {
+      const int64_t at = tok * (D >> A.gshift) + (q >> (A.gshift - 5));
       dst.scale[at] = sc;
       dst.zero[at] = lo;
     }
   }
 }
 
-// Eight channels of the token in row `tok` of a source tier (tok counts over the (batch, head) planes), SB = its bits.
+// Quarter q of a token's row of a source tier with SB bits (row at `row`, tok = its number over the (batch, head) planes).
 template <int SB>
 struct VUnit {
-  uint4 raw;
+  uint32_t raw[SB];
   __half sc, ze;
 };
 template <int SB>
-__device__ __forceinline__ void v_unit_load(const BuildArgs& A, VUnit<SB>& u, const unsigned char* rows, int src, int64_t tok, int l16) {
-  const unsigned char* p = rows + l16 * SB;
-  if constexpr (SB == 16) {
-    u.raw = *reinterpret_cast<const uint4*>(p);
-  } else {
-    if constexpr (SB == 8) {
-      const uint2 x = *reinterpret_cast<const uint2*>(p);
-      u.raw.x = x.x;
-      u.raw.y = x.y;
-    } else if constexpr (SB == 4) {
-      u.raw.x = *reinterpret_cast<const uint32_t*>(p);
-    } else {
-      u.raw.x = *reinterpret_cast<const uint16_t*>(p);
+__device__ __forceinline__ void v_unit_load(const BuildArgs& A, VUnit<SB>& u, const unsigned char* row, int src, int64_t tok, int q) {
+  const unsigned char* p = row + q * (4 * SB);
+  if constexpr (SB >= 4) {
+#pragma unroll
+    for (int i = 0; i < SB / 4; ++i) {
+      const uint4 x = reinterpret_cast<const uint4*>(p)[i];
+      u.raw[4 * i] = x.x, u.raw[4 * i + 1] = x.y, u.raw[4 * i + 2] = x.z, u.raw[4 * i + 3] = x.w;
     }
-    const int64_t at = tok * (D >> A.gshift) + (l16 >> (A.gshift - 3));
+  } else {
+    const uint2 x = *reinterpret_cast<const uint2*>(p);
+    u.raw[0] = x.x, u.raw[1] = x.y;
+  }
+  if constexpr (SB < 16) {
+    const int64_t at = tok * (D >> A.gshift) + (q >> (A.gshift - 5));
     u.sc = A.scale[src][at];
     u.ze = A.zero[src][at];
   }
 }
 template <int SB>
-__device__ __forceinline__ void v_unit_values(const VUnit<SB>& u, __half2 (&v)[4]) {
+__device__ __forceinline__ void v_unit_values(const VUnit<SB>& u, __half2 (&v)[16]) {
   if constexpr (SB == 16) {
-    v[0] = as_h2(u.raw.x), v[1] = as_h2(u.raw.y), v[2] = as_h2(u.raw.z), v[3] = as_h2(u.raw.w);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = as_h2(u.raw[i]);
   } else {
     const __half2 sc = __half2half2(u.sc), ze = __half2half2(u.ze);
+    constexpr int PAIRS = 16 / SB;  // per word
+    constexpr uint32_t M = (1u << SB) - 1u;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      uint32_t c;
-      if constexpr (SB == 8) {
-        const uint32_t w = i < 2 ? u.raw.x : u.raw.y;
-        c = __byte_perm(w, 0u, (i & 1) ? 0x4342 : 0x4140);
-      } else {
-        const uint32_t w = u.raw.x >> (2 * i * SB), m = (1u << SB) - 1u;
-        c = (w & m) | (((w >> SB) & m) << 16);
-      }
-      v[i] = dequant2(c, sc, ze);
+    for (int i = 0; i < 16; ++i) {
+      const uint32_t w = u.raw[i / PAIRS] >> ((i % PAIRS) * 2 * SB);
+      v[i] = dequant2((w & M) | (((w >> SB) & M) << 16), sc, ze);
     }
   }
 }
-// 32 consecutive tokens that arrive from one source: rows at `rows`, `pitch` bytes apart, tok = number of the first
+// 32 consecutive tokens that arrive from one source: rows at `rows`, 16 * SB bytes apart, tok = number of the first
 template <int BITS, int SB>
-__device__ __forceinline__ void v_arrive(const BuildArgs& A, const BuildDst& dst, const unsigned char* rows, int64_t pitch, int src,
-                                         int64_t tok, int64_t out_tok) {
-  const int lane = threadIdx.x & 31, l16 = lane & 15, odd = lane >> 4;
-  VUnit<SB> u[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) v_unit_load<SB>(A, u[i], rows + (2 * i + odd) * pitch, src, tok + 2 * i + odd, l16);
+__device__ __forceinline__ void v_arrive(const BuildArgs& A, const BuildDst& dst, const unsigned char* rows, int src, int64_t tok, int64_t out_tok) {
+  const int lane = threadIdx.x & 31, q = lane & 3, row = lane >> 2;
+  VUnit<SB> u;
+  v_unit_load<SB>(A, u, rows + row * (16 * SB), src, tok + row, q);
 #pragma unroll 1
-  for (int s = 0; s < 16; s += 4) {
-    VUnit<SB> next[4];
-    if (s + 4 < 16) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) v_unit_load<SB>(A, next[i], rows + (2 * (s + 4 + i) + odd) * pitch, src, tok + 2 * (s + 4 + i) + odd, l16);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      __half2 v[4];
-      v_unit_values<SB>(u[i], v);
-      v_store8<BITS>(A, dst, out_tok + 2 * (s + i) + odd, l16, v);
-      u[i] = next[i];
-    }
+  for (int s = 0; s < 32; s += 8) {
+    __half2 v[16];
+    v_unit_values<SB>(u, v);
+    if (s + 8 < 32) v_unit_load<SB>(A, u, rows + (s + 8 + row) * (16 * SB), src, tok + s + 8 + row, q);
+    v_store32<BITS>(A, dst, out_tok + s + row, q, v, true);
   }
 }
 
-// One token from any source, by the whole warp (its upper half repeats the lower half's work).
+// One token from any source, by the first four lanes of the warp.
 template <int BITS>
 __device__ __noinline__ void v_one_token(const BuildArgs& A, int t, int32_t enc, int64_t j, int bh) {
   const BuildDst& dst = A.dst[t];
-  const int lane = threadIdx.x & 31, l16 = lane & 15, ng = D >> A.gshift;
+  const int lane = threadIdx.x & 31, q = lane & 3, ng = D >> A.gshift;
   const int src = (enc >> 28) - 1;
   const int64_t pos = enc & 0x0FFFFFFF, out_tok = static_cast<int64_t>(bh) * dst.n + j;
   if (src == t) {  // kept: copy the row verbatim
     const int64_t tok = static_cast<int64_t>(bh) * A.n[t] + pos;
-    if (lane < 4 * BITS)
-      for (int w = lane; w < 4 * BITS; w += 32)
-        reinterpret_cast<uint32_t*>(dst.data)[out_tok * (4 * BITS) + w] = reinterpret_cast<const uint32_t*>(A.data[t])[tok * (4 * BITS) + w];
+    for (int w = lane; w < 4 * BITS; w += 32)
+      reinterpret_cast<uint32_t*>(dst.data)[out_tok * (4 * BITS) + w] = reinterpret_cast<const uint32_t*>(A.data[t])[tok * (4 * BITS) + w];
     if (BITS < 16 && lane < ng) {
       dst.scale[out_tok * ng + lane] = A.scale[t][tok * ng + lane];
       dst.zero[out_tok * ng + lane] = A.zero[t][tok * ng + lane];
     }
     return;
   }
-  __half x[8];
+  __half2 v[16];
   if (src < 0 || src == 0) {
     const int b = bh / A.H, h = bh - b * A.H;
     const __half* p = src < 0 ? A.residual + b * A.res_b_stride + h * A.res_h_stride + pos * D
                               : reinterpret_cast<const __half*>(A.data[0]) + (static_cast<int64_t>(bh) * A.n[0] + pos) * D;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) x[i] = p[8 * l16 + i];
+    for (int i = 0; i < 16; ++i) v[i] = __halves2half2(p[32 * q + 2 * i], p[32 * q + 2 * i + 1]);
   } else {
     const int sb = 16 >> src;
-    const int64_t tok = static_cast<int64_t>(bh) * A.n[src] + pos, at = tok * ng + (l16 >> (A.gshift - 3));
+    const int64_t tok = static_cast<int64_t>(bh) * A.n[src] + pos, at = tok * ng + (q >> (A.gshift - 5));
     const __half sc = A.scale[src][at], ze = A.zero[src][at];
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(A.data[src]) + tok * (4 * sb);
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      x[i] = h_add(h_mul(v_get(reinterpret_cast<const uint32_t*>(A.data[src]) + tok * (4 * sb), sb, 8 * l16 + i), sc), ze);
+    for (int i = 0; i < 16; ++i)
+      v[i] = __halves2half2(h_add(h_mul(v_get(w, sb, 32 * q + 2 * i), sc), ze), h_add(h_mul(v_get(w, sb, 32 * q + 2 * i + 1), sc), ze));
   }
-  __half2 v[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) v[i] = __halves2half2(x[2 * i], x[2 * i + 1]);
-  v_store8<BITS>(A, dst, out_tok, l16, v);
+  v_store32<BITS>(A, dst, out_tok, q, v, lane < 4);
 }
 
 template <int BITS>
@@ -730,23 +744,23 @@ __device__ __forceinline__ void v_build_run(const BuildArgs& A, int t, int64_t r
   }
   if (src < 0) {
     const int b = bh / A.H, h = bh - b * A.H;
-    v_arrive<BITS, 16>(A, dst, reinterpret_cast<const unsigned char*>(A.residual + b * A.res_b_stride + h * A.res_h_stride + pos * D),
-                       2 * D, src, 0, out_tok);
+    v_arrive<BITS, 16>(A, dst, reinterpret_cast<const unsigned char*>(A.residual + b * A.res_b_stride + h * A.res_h_stride + pos * D), src,
+                       0, out_tok);
     return;
   }
   const int64_t tok = static_cast<int64_t>(bh) * A.n[src] + pos;
   const int sb = 16 >> src;
   const unsigned char* rows = reinterpret_cast<const unsigned char*>(A.data[src]) + tok * (16 * sb);
-  if (sb == 16) v_arrive<BITS, 16>(A, dst, rows, 256, src, tok, out_tok);
-  else if (BITS < 8 && sb == 8) v_arrive<BITS, 8>(A, dst, rows, 128, src, tok, out_tok);
-  else if (BITS < 4 && sb == 4) v_arrive<BITS, 4>(A, dst, rows, 64, src, tok, out_tok);
-  else if (BITS < 2 && sb == 2) v_arrive<BITS, 2>(A, dst, rows, 32, src, tok, out_tok);
+  if (sb == 16) v_arrive<BITS, 16>(A, dst, rows, src, tok, out_tok);
+  else if (BITS < 8 && sb == 8) v_arrive<BITS, 8>(A, dst, rows, src, tok, out_tok);
+  else if (BITS < 4 && sb == 4) v_arrive<BITS, 4>(A, dst, rows, src, tok, out_tok);
+  else if (BITS < 2 && sb == 2) v_arrive<BITS, 2>(A, dst, rows, src, tok, out_tok);
   else
     for (int i = 0; i < 32; ++i) v_one_token<BITS>(A, t, enc0 + i, j0 + i, bh);  // (not to wider tiers; all the same)
 }
 
 constexpr int VB_WARPS = BUILD_THREADS / 32;
-__global__ void __launch_bounds__(BUILD_THREADS, 4) flush_build_v_kernel(const __grid_constant__ BuildArgs A) {
+__global__ void __launch_bounds__(BUILD_THREADS, 3) flush_build_v_kernel(const __grid_constant__ BuildArgs A) {
   const int x = blockIdx.x, bh = blockIdx.y;
   if (x >= A.tiles) {
     copy_rest(A, bh);
