@@ -33,7 +33,7 @@ struct BuildArgs {
   int H, gshift;
   int normal_low;       // the 1-bit destination is written in the Gaussian-codebook codec
   BuildDst dst[HQKV_NUM_TIERS];
-  int tiles;            // of all destinations; the grid's columns behind them copy the rest of the residual window
+  int tiles;            // of all destinations; one more column of the grid copies the rest of the residual window
   const __half* rest;   // its first row of (batch 0, head 0), strides as the residual's
   __half* rest_out;
   int64_t rest_n;       // halfs per (batch, head)
@@ -308,33 +308,35 @@ __device__ __forceinline__ void k_build_tile(const BuildArgs& A, KBuildShared& s
   __syncthreads();
   const int piece = tid & 7, r0 = tid >> 3, sub = KB::sub_of(piece);
   const bool mine = sub < nsub, kept = mine && sh.src[sub] == t;
-  // scales of kept groups, requested together with their codes
+  // Scales of kept groups, requested together with their codes: a thread has one group of the tile and every `rstep`-th row.
   constexpr int SPT = 4;                                                 // scales per thread at most
   const int gs = (BITS == 8 ? 7 : 8) - A.gshift;                         // log2(groups per tile)
-  const int64_t Gd = dst.n >> A.gshift, Gs = static_cast<int64_t>(A.n[t]) >> A.gshift, g0 = j0 >> A.gshift;
+  const int sg = tid & ((1 << gs) - 1), srow = tid >> gs, rstep = BUILD_THREADS >> gs, sfirst = sg << (A.gshift - 5);
+  const bool scaled = BITS < 16 && sfirst < nsub, scale_kept = scaled && sh.src[sfirst] == t;
   __half ks[SPT], kz[SPT];
-  if constexpr (BITS < 16) {
+  if (scale_kept) {
+    const int64_t Gs = static_cast<int64_t>(A.n[t]) >> A.gshift, from = (static_cast<int64_t>(bh) * D + srow) * Gs + (sh.pos[sfirst] >> A.gshift);
+    const __half *ps = A.scale[t] + from, *pz = A.zero[t] + from;
+    const int64_t step = rstep * Gs;
 #pragma unroll
-    for (int k = 0; k < SPT; ++k) {
-      const int i = tid + k * BUILD_THREADS, r = i >> gs, first = (i & ((1 << gs) - 1)) << (A.gshift - 5);
-      if (i < D << gs && first < nsub && sh.src[first] == t) {
-        const int64_t from = (static_cast<int64_t>(bh) * D + r) * Gs + (sh.pos[first] >> A.gshift);
-        ks[k] = A.scale[t][from];
-        kz[k] = A.zero[t][from];
+    for (int k = 0; k < SPT; ++k)
+      if (srow + k * rstep < D) {
+        ks[k] = ps[k * step];
+        kz[k] = pz[k * step];
       }
-    }
   }
   const int64_t out_row = dst.n * BITS / 8;
-  unsigned char* out = reinterpret_cast<unsigned char*>(dst.data) + static_cast<int64_t>(bh) * D * out_row + j0 * BITS / 8 + piece * KB::PIECE;
+  unsigned char* out = reinterpret_cast<unsigned char*>(dst.data) + (static_cast<int64_t>(bh) * D + r0) * out_row + j0 * BITS / 8 + piece * KB::PIECE;
   if (kept) {
     const int64_t in_row = static_cast<int64_t>(A.n[t]) * BITS / 8;
     const unsigned char* in = reinterpret_cast<const unsigned char*>(A.data[t]) + static_cast<int64_t>(bh) * D * in_row +
                               static_cast<int64_t>(sh.pos[sub]) * BITS / 8 + (piece * KB::PIECE - sub * 4 * BITS);
+    in += r0 * in_row;
     Piece v[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const Piece*>(in + (r0 + 32 * i) * in_row);
+    for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const Piece*>(in + 32 * i * in_row);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) *reinterpret_cast<Piece*>(out + (r0 + 32 * i) * out_row) = v[i];
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<Piece*>(out + 32 * i * out_row) = v[i];
   }
   bool arrivals = false;
 #pragma unroll
@@ -417,27 +419,29 @@ __device__ __forceinline__ void k_build_tile(const BuildArgs& A, KBuildShared& s
         uint32_t* u = reinterpret_cast<uint32_t*>(&v);
 #pragma unroll
         for (int k = 0; k < W; ++k) u[k] = w[k];
-        *reinterpret_cast<Piece*>(out + (r0 + 32 * i) * out_row) = v;
+        *reinterpret_cast<Piece*>(out + 32 * i * out_row) = v;
       }
     }
   }
   if constexpr (BITS < 16) {
+    if (scaled) {
+      const int64_t Gd = dst.n >> A.gshift, at = (static_cast<int64_t>(bh) * D + srow) * Gd + (j0 >> A.gshift) + sg, step = rstep * Gd;
 #pragma unroll
-    for (int k = 0; k < SPT; ++k) {
-      const int i = tid + k * BUILD_THREADS, r = i >> gs, g = i & ((1 << gs) - 1), first = g << (A.gshift - 5);
-      if (i >= D << gs || first >= nsub) continue;
-      const int64_t at = (static_cast<int64_t>(bh) * D + r) * Gd + g0 + g;
-      const bool kept_group = sh.src[first] == t;
-      dst.scale[at] = kept_group ? ks[k] : sh.s[r * KB_MAX_SUBS + g];
-      dst.zero[at] = kept_group ? kz[k] : sh.z[r * KB_MAX_SUBS + g];
+      for (int k = 0; k < SPT; ++k) {
+        const int r = srow + k * rstep;
+        if (r >= D) break;
+        dst.scale[at + k * step] = scale_kept ? ks[k] : sh.s[r * KB_MAX_SUBS + sg];
+        dst.zero[at + k * step] = scale_kept ? kz[k] : sh.z[r * KB_MAX_SUBS + sg];
+      }
     }
   }
 }
 
 __global__ void __launch_bounds__(BUILD_THREADS, 4) flush_build_k_kernel(const __grid_constant__ BuildArgs A) {
   __shared__ KBuildShared sh;
-  const int x = blockIdx.x, bh = blockIdx.y;
-  if (x >= A.tiles) {
+  // From the back: arrivals, which take longer than copies, are at the end of a tier's list, and the lowest tier's longest.
+  const int x = A.tiles - 1 - static_cast<int>(blockIdx.x), bh = blockIdx.y;
+  if (x < 0) {
     copy_rest(A, bh);
     return;
   }
@@ -760,9 +764,9 @@ __device__ __forceinline__ void v_build_run(const BuildArgs& A, int t, int64_t r
 }
 
 constexpr int VB_WARPS = BUILD_THREADS / 32;
-__global__ void __launch_bounds__(BUILD_THREADS, 3) flush_build_v_kernel(const __grid_constant__ BuildArgs A) {
-  const int x = blockIdx.x, bh = blockIdx.y;
-  if (x >= A.tiles) {
+__global__ void __launch_bounds__(BUILD_THREADS, 4) flush_build_v_kernel(const __grid_constant__ BuildArgs A) {
+  const int x = A.tiles - 1 - static_cast<int>(blockIdx.x), bh = blockIdx.y;  // from the back, as above
+  if (x < 0) {
     copy_rest(A, bh);
     return;
   }

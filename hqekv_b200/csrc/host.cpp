@@ -363,6 +363,37 @@ PyObject* block_rank(PyObject*, PyObject* const* a, Py_ssize_t na) {
   END_HANDLE_TH_ERRORS
 }
 
+// Tensors of one allocation.  The parts of a tier (codes, ids, scales, zeros) live and die together; an allocation of their
+// own for each of them took more host time than anything else in a flush.
+struct Slab {
+  std::vector<std::pair<at::Tensor*, std::vector<int64_t>>> parts;
+  std::vector<at::ScalarType> types;
+  void add(at::Tensor* t, std::initializer_list<int64_t> sizes, at::ScalarType type) {
+    parts.emplace_back(t, sizes);
+    types.push_back(type);
+  }
+  void allocate(const at::TensorOptions& opt) {
+    auto bytes = [&](size_t i) {
+      int64_t n = static_cast<int64_t>(c10::elementSize(types[i]));
+      for (int64_t d : parts[i].second) n *= d;
+      return (n + 511) & ~int64_t{511};
+    };
+    int64_t total = 0;
+    for (size_t i = 0; i < parts.size(); ++i) total += bytes(i);
+    if (total == 0) return;
+    const at::Tensor base = at::empty({total}, opt.dtype(at::kByte));
+    int64_t at = 0;
+    for (size_t i = 0; i < parts.size(); ++i) {
+      at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(base.storage()), c10::DispatchKeySet(c10::DispatchKey::CUDA),
+                                                              c10::scalarTypeToTypeMeta(types[i]));
+      t.unsafeGetTensorImpl()->set_storage_offset(at / static_cast<int64_t>(c10::elementSize(types[i])));
+      t.unsafeGetTensorImpl()->set_sizes_contiguous(parts[i].second);
+      *parts[i].first = std::move(t);
+      at += bytes(i);
+    }
+  }
+};
+
 bool six_counts(PyObject* list, int64_t (&cum)[6]) {
   if (!PyList_Check(list) || PyList_GET_SIZE(list) != 6) return false;
   int64_t run = 0;
@@ -435,7 +466,7 @@ PyObject* flush(PyObject*, PyObject* const* a, Py_ssize_t na) {
   }
   const c10::cuda::OptionalCUDAGuard guard(dev);
   const cudaStream_t st = current_stream(*nk);
-  const auto half = nk->options(), i32 = half.dtype(at::kInt), i64 = half.dtype(at::kLong);
+  const auto half = nk->options();
   at::Tensor norm_out = at::empty({total}, half);
   at::Tensor ws = at::empty({static_cast<int64_t>(L.flush_workspace_bytes(total))}, half.dtype(at::kByte));
   f.norm_old = ptr(norm);
@@ -458,18 +489,21 @@ PyObject* flush(PyObject*, PyObject* const* a, Py_ssize_t na) {
       const int64_t n = counts[8 * side + t], bits = kBits[t];
       if (n == 0) continue;
       at::Tensor* o = out + slots[t];
+      Slab slab;
       if (t == 0) {
-        o[0] = side ? at::empty({B, H, n, D}, half) : at::empty({B, H, D, n}, half);
+        if (side) slab.add(&o[0], {B, H, n, D}, at::kHalf);
+        else slab.add(&o[0], {B, H, D, n}, at::kHalf);
       } else if (side) {
-        o[0] = at::empty({B, H, n, D * bits / 32}, i32);
-        o[2] = at::empty({B, H, n, D / group}, half);
-        o[3] = at::empty({B, H, n, D / group}, half);
+        slab.add(&o[0], {B, H, n, D * bits / 32}, at::kInt);
+        slab.add(&o[2], {B, H, n, D / group}, at::kHalf);
+        slab.add(&o[3], {B, H, n, D / group}, at::kHalf);
       } else {
-        o[0] = at::empty({B, H, D, n * bits / 32}, i32);
-        o[2] = at::empty({B, H, D, n / group}, half);
-        o[3] = at::empty({B, H, D, n / group}, half);
+        slab.add(&o[0], {B, H, D, n * bits / 32}, at::kInt);
+        slab.add(&o[2], {B, H, D, n / group}, at::kHalf);
+        slab.add(&o[3], {B, H, D, n / group}, at::kHalf);
       }
-      o[1] = at::empty({n}, i64);
+      slab.add(&o[1], {n}, at::kLong);
+      slab.allocate(half);
       data[t] = o[0].data_ptr();
       ids[t] = o[1].data_ptr<int64_t>();
       if (t) scale[t] = o[2].data_ptr(), zero[t] = o[3].data_ptr();

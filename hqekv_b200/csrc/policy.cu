@@ -293,6 +293,7 @@ struct PlanSide {
   int64_t* plan_ids;   // [5][total]
   int64_t* survivors;  // [total]
   int32_t* counts;     // [8]
+  int32_t done;        // what counts[7] says when the others are there (memory of the host: it polls)
   // scratch
   int8_t* tgt;         // [total] by token id, 16-byte aligned
   int8_t* fin;         // [total] by enumeration slot: category
@@ -444,6 +445,17 @@ __global__ void __launch_bounds__(PLAN_THREADS) flush_plan_kernel(const __grid_c
     if (lane == 31) tot[warp] = incl;
   }
   __syncthreads();
+  if (crank == 0) {
+    if (tid == 0) {
+      volatile int32_t* c = S.counts;
+#pragma unroll
+      for (int t = 0; t < HQKV_NUM_TIERS; ++t) c[t] = tot[2 * t] + tot[2 * t + 1];
+      c[5] = tot[PLAN_CATS - 1];
+      c[6] = any_evict ? 1 : 0;
+      __threadfence_system();
+      c[7] = S.done;
+    }
+  }
   // 3. survivor ranks by token id: rank[i] = survivors with a smaller id; survivors[rank] = id
   {
     int running = cnt[PLAN_CATS - 1][warp];
@@ -500,14 +512,6 @@ __global__ void __launch_bounds__(PLAN_THREADS) flush_plan_kernel(const __grid_c
         if ((same & lt) == 0) cnt[cat[u]][warp] = base + __popc(same);
       }
       __syncwarp();
-    }
-  }
-  if (crank == 0) {
-    if (tid < HQKV_NUM_TIERS) S.counts[tid] = tot[2 * tid] + tot[2 * tid + 1];
-    if (tid == 0) {
-      S.counts[5] = tot[PLAN_CATS - 1];
-      S.counts[6] = any_evict ? 1 : 0;
-      S.counts[7] = 0;
     }
   }
 }
@@ -694,7 +698,6 @@ struct FlushScratch {
   unsigned char* plan_ws[2];
   int64_t* v_sorted;
   __half* v_keys;
-  int32_t* counts;  // [2][8]
   size_t bytes;
 };
 static FlushScratch flush_scratch(void* base, int64_t total) {
@@ -702,8 +705,7 @@ static FlushScratch flush_scratch(void* base, int64_t total) {
   const size_t t = static_cast<size_t>(total);
   unsigned char* p = static_cast<unsigned char*>(base);
   FlushScratch s;
-  s.counts = reinterpret_cast<int32_t*>(p);
-  size_t at = 256;
+  size_t at = 0;
   for (int side = 0; side < 2; ++side) {
     s.plan_src[side] = reinterpret_cast<int32_t*>(p + at), at += up(HQKV_NUM_TIERS * t * 4);
     s.plan_ids[side] = reinterpret_cast<int64_t*>(p + at), at += up(HQKV_NUM_TIERS * t * 8);
@@ -768,8 +770,31 @@ extern "C" int hqkv_flush_prepare(const hqkv_flush_t* f, void* workspace, size_t
   for (int side = 0; side < 2; ++side) {
     const int rc = fill_plan_side(A.side[side], side ? f->v_idx : f->k_idx, side ? f->v.n : f->k.n, f->hist, total,
                                   side ? s.v_sorted : f->k_sorted, side ? f->v_cum : f->k_cum, s.plan_src[side], s.plan_ids[side],
-                                  s.survivors[side], s.counts + 8 * side, s.plan_ws[side]);
+                                  s.survivors[side], nullptr, s.plan_ws[side]);
     if (rc) return rc;
+  }
+  // The counts come back through memory of the host that the plan writes (64 bytes per thread, kept until it ends): they are
+  // there as soon as the tokens are counted, while the plan still writes its lists, and no copy has to be launched.
+  struct Mapped {
+    volatile int32_t* host = nullptr;
+    int32_t calls = 0;
+    ~Mapped() {
+      if (host) cudaFreeHost(const_cast<int32_t*>(host));
+    }
+  };
+  static thread_local Mapped mapped;
+  if (!mapped.host) {
+    void* p = nullptr;
+    HQKV_CUDA(cudaHostAlloc(&p, 64, cudaHostAllocPortable | cudaHostAllocMapped));
+    memset(p, 0, 64);
+    mapped.host = static_cast<volatile int32_t*>(p);
+  }
+  void* counts_dev = nullptr;
+  HQKV_CUDA(cudaHostGetDevicePointer(&counts_dev, const_cast<int32_t*>(mapped.host), 0));
+  mapped.calls = mapped.calls == 0x7FFFFFFF ? 1 : mapped.calls + 1;
+  for (int side = 0; side < 2; ++side) {
+    A.side[side].counts = static_cast<int32_t*>(counts_dev) + 8 * side;
+    A.side[side].done = mapped.calls;
   }
   int rc = launch_range(f->v.residual, f->B, f->H, f->compress, f->v.residual_b_stride, f->v.residual_h_stride, f->norm_old, f->hist,
                         f->norm_out, stream);
@@ -779,19 +804,15 @@ extern "C" int hqkv_flush_prepare(const hqkv_flush_t* f, void* workspace, size_t
   if (rc) return rc;
   rc = launch_plan(A, 2, stream);
   if (rc) return rc;
-  // the counts come back through a pinned buffer of this thread (64 bytes, kept until the thread ends)
-  struct Pinned {
-    int32_t* p = nullptr;
-    ~Pinned() {
-      if (p) cudaFreeHost(p);
-    }
-  };
-  static thread_local Pinned pinned;
-  if (!pinned.p) HQKV_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&pinned.p), 64, cudaHostAllocPortable));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  HQKV_CUDA(cudaMemcpyAsync(pinned.p, s.counts, 64, cudaMemcpyDeviceToHost, st));
-  HQKV_CUDA(cudaStreamSynchronize(st));
-  memcpy(counts_host, pinned.p, 64);
+  for (int spins = 0; mapped.host[7] != mapped.calls || mapped.host[15] != mapped.calls; ++spins) {
+    if ((spins & 0xFFFF) != 0xFFFF) continue;
+    const cudaError_t e = cudaStreamQuery(st);  // an error of the stream ends the wait
+    if (e == cudaErrorNotReady) continue;
+    HQKV_CUDA(e);
+    HQKV_REQUIRE(mapped.host[7] == mapped.calls && mapped.host[15] == mapped.calls, "flush_prepare: the plan left no counts");
+  }
+  for (int i = 0; i < 16; ++i) counts_host[i] = mapped.host[i];
   return HQKV_OK;
 }
 

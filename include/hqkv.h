@@ -439,8 +439,8 @@ int hqkv_flush_build(int v_side, const hqkv_flush_src_t* src_host, int B, int H,
  * A whole flush (KV_cache_hqe_2, quant/hqe_2.py:456-843) in three calls, for hosts that keep launches and allocations few:
  *   hqkv_flush_prepare   value ranges of the flushed tokens appended to norm_old (-> norm_out, hist + compress fp16),
  *                        V ranking from `importance` (as ranked for K, i.e. divided by the block size; not modified) and,
- *                        with times_range, those ranges; the plans of both sides; reads the counts back
- *                        (counts_host[0..8) K, [8..16) V as in hqkv_flush_plan) and waits for the stream
+ *                        with times_range, those ranges; the plans of both sides; waits for the counts
+ *                        (counts_host[0..8) K, [8..16) V as in hqkv_flush_plan)
  *   hqkv_flush_tiers     hqkv_flush_build of one side from that plan
  *   hqkv_flush_evict     compacts norm_out to the V-side survivors (-> norm_kept) and moves the survivors' columns of an
  *                        importance ring (fp16 [rows][stride], null: none) to the front, in place
