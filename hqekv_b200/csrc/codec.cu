@@ -28,103 +28,86 @@ int check_cuda(cudaError_t e, const char* what) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// Row path: groups are contiguous in memory (t_stride == 1).  One thread owns 8 consecutive
-// elements (one 16-byte load when aligned), GROUP/8 adjacent lanes own one group.
+// Row path: groups are contiguous in memory (t_stride == 1).  One thread owns 32 consecutive elements, GROUP/32 adjacent
+// lanes own one group: what is done once per group (two divisions) is shared by 32 elements, and a thread's words are
+// one store.
 // ------------------------------------------------------------------------------------------------
+template <int BYTES>  // BYTES consecutive bytes, 16 at a time or, where the address allows it, 32
+__device__ __forceinline__ void load_run(void* dst, const void* src, bool by32) {
+  uint32_t* d = static_cast<uint32_t*>(dst);
+  const char* p = static_cast<const char*>(src);
+  if (by32) {
+#pragma unroll
+    for (int i = 0; i < BYTES / 32; ++i)
+      asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                   : "=r"(d[8 * i]), "=r"(d[8 * i + 1]), "=r"(d[8 * i + 2]), "=r"(d[8 * i + 3]), "=r"(d[8 * i + 4]),
+                     "=r"(d[8 * i + 5]), "=r"(d[8 * i + 6]), "=r"(d[8 * i + 7])
+                   : "l"(p + 32 * i));
+  } else {
+#pragma unroll
+    for (int i = 0; i < BYTES / 16; ++i) {
+      const uint4 v = *reinterpret_cast<const uint4*>(p + 16 * i);
+      d[4 * i] = v.x, d[4 * i + 1] = v.y, d[4 * i + 2] = v.z, d[4 * i + 3] = v.w;
+    }
+  }
+}
+
 template <int BITS, int GROUP>
-__global__ void __launch_bounds__(256) quantize_rows_kernel(const __half* __restrict__ x, int64_t rows, int64_t T,
-                                                            int64_t inner, int64_t outer_stride,
-                                                            int64_t inner_stride, bool vec_ok,
-                                                            uint32_t* __restrict__ code, __half* __restrict__ scale,
-                                                            __half* __restrict__ mn_out) {
-  constexpr int LPG = GROUP / 8;  // lanes per group
+__global__ void __launch_bounds__(256) quantize_rows_kernel(const __half* __restrict__ x, int64_t n_units, int64_t T,
+                                                            int64_t inner, int64_t outer_stride, int64_t inner_stride,
+                                                            int align, bool vec_out, uint32_t* __restrict__ code,
+                                                            __half* __restrict__ scale, __half* __restrict__ mn_out) {
+  constexpr int LPG = GROUP / 32;  // lanes per group
   const float levels = static_cast<float>((1 << BITS) - 1);
-  const int64_t units_per_row = T / 8;
-  const int64_t total_units = rows * units_per_row;
-  // all lanes of a warp take part in the shuffles: iterate in whole-warp steps; two units per thread and step, both
-  // loads issued before either is worked on (one 16-byte load in flight per thread did not cover the memory latency)
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  const int64_t n_iter = (total_units + 2 * stride - 1) / (2 * stride);
-  // packed source (the usual case): unit u is elements [8u, 8u+8) and no 64-bit division is needed;
-  // (row*T + t0) below is 8u either way
-  const bool packed = inner_stride == T && outer_stride == inner * T;
-  const int lane = threadIdx.x & 31;
-  for (int64_t it = 0; it < n_iter; ++it) {
-    __half v[2][8];
-    int64_t row[2], t0[2];
-    bool live[2];
+  const int64_t unit = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t u = unit < n_units ? unit : n_units - 1;  // every lane takes part in the shuffles
+  const __half* src = x + u * 32;
+  if (inner_stride != T || outer_stride != inner * T) {  // rows that do not follow one another
+    const int64_t units_per_row = T / 32, row = u / units_per_row;
+    src = x + (row / inner) * outer_stride + (row % inner) * inner_stride + (u - row * units_per_row) * 32;
+  }
+  __half2 v[16];
+  if (align >= 16) {
+    load_run<64>(v, src, align >= 32);
+  } else {
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int64_t u = (2 * it + k) * stride + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-      live[k] = u < total_units;
-      row[k] = 0;
-      t0[k] = live[k] ? u * 8 : 0;
-      if (!packed && live[k]) {
-        row[k] = u / units_per_row;
-        t0[k] = (u % units_per_row) * 8;
-      }
-      if (live[k]) {
-        const __half* src = packed ? x + t0[k] : x + (row[k] / inner) * outer_stride + (row[k] % inner) * inner_stride + t0[k];
-        if (vec_ok) {
-          *reinterpret_cast<uint4*>(v[k]) = *reinterpret_cast<const uint4*>(src);
-        } else {
+    for (int i = 0; i < 16; ++i) v[i] = __halves2half2(src[2 * i], src[2 * i + 1]);
+  }
+  // min / max of the group on half2 pairs (NaN propagates, as in torch.min / torch.max)
+  __half2 lo2 = v[0], hi2 = v[0];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) v[k][i] = src[i];
-        }
-      } else {
+  for (int i = 1; i < 16; ++i) {
+    lo2 = __hmin2_nan(lo2, v[i]);
+    hi2 = __hmax2_nan(hi2, v[i]);
+  }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[k][i] = __float2half(0.f);
-      }
+  for (int off = 1; off < LPG; off <<= 1) {
+    lo2 = __hmin2_nan(lo2, __shfl_xor_sync(0xffffffffu, lo2, off));
+    hi2 = __hmax2_nan(hi2, __shfl_xor_sync(0xffffffffu, hi2, off));
+  }
+  const __half lo = __low2half(__hmin2_nan(lo2, __lowhigh2highlow(lo2))), hi = __low2half(__hmax2_nan(hi2, __lowhigh2highlow(hi2)));
+  const __half sc = quant_scale(lo, hi, levels);
+  uint32_t word[BITS];
+  quant_row32<BITS>(v, quant_pair(lo, sc), word);
+  if (unit >= n_units) return;
+  uint32_t* dst = code + u * BITS;
+  if (vec_out) {
+    if constexpr (BITS >= 4) {
+#pragma unroll
+      for (int i = 0; i < BITS / 4; ++i)
+        reinterpret_cast<uint4*>(dst)[i] = make_uint4(word[4 * i], word[4 * i + 1], word[4 * i + 2], word[4 * i + 3]);
+    } else if constexpr (BITS == 2) {
+      *reinterpret_cast<uint2*>(dst) = make_uint2(word[0], word[1]);
+    } else {
+      *dst = word[0];
     }
+  } else {
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      // min / max of the group on half2 pairs (NaN propagates, as in torch.min / torch.max)
-      const __half2* v2 = reinterpret_cast<const __half2*>(v[k]);
-      __half2 lo2 = __hmin2_nan(__hmin2_nan(v2[0], v2[1]), __hmin2_nan(v2[2], v2[3]));
-      __half2 hi2 = __hmax2_nan(__hmax2_nan(v2[0], v2[1]), __hmax2_nan(v2[2], v2[3]));
-#pragma unroll
-      for (int off = 1; off < LPG; off <<= 1) {
-        lo2 = __hmin2_nan(lo2, __shfl_xor_sync(0xffffffffu, lo2, off));
-        hi2 = __hmax2_nan(hi2, __shfl_xor_sync(0xffffffffu, hi2, off));
-      }
-      lo2 = __hmin2_nan(lo2, __lowhigh2highlow(lo2));
-      hi2 = __hmax2_nan(hi2, __lowhigh2highlow(hi2));
-      const __half lo = __low2half(lo2), hi = __low2half(hi2);
-      const __half sc = quant_scale(lo, hi, levels);
-      const QuantGroup qg = quant_group(lo, sc, levels);
-      uint64_t part = 0;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t c2 = quant_code_fast2(v2[i], qg);
-        part |= static_cast<uint64_t>((c2 & 0xFFFFu) | ((c2 >> 16) << BITS)) << (2 * i * BITS);
-      }
-      const int64_t out_bit = (row[k] * T + t0[k]) * BITS;  // bit offset of this unit in the packed row-major stream
-      if constexpr (BITS == 8) {
-        if (live[k]) {
-          uint2 w;
-          w.x = static_cast<uint32_t>(part);
-          w.y = static_cast<uint32_t>(part >> 32);
-          *reinterpret_cast<uint2*>(code + out_bit / 32) = w;
-        }
-      } else if constexpr (BITS == 4) {
-        if (live[k]) code[out_bit / 32] = static_cast<uint32_t>(part);
-      } else {
-        // 2 bits: 16 bits per thread, two lanes per word; 1 bit: 8 bits per thread, four lanes per word
-        constexpr int LPW = 32 / (8 * BITS);  // lanes per word
-        uint32_t w = static_cast<uint32_t>(part);
-#pragma unroll
-        for (int off = 1; off < LPW; off <<= 1) {
-          const uint32_t other = __shfl_down_sync(0xffffffffu, w, off);
-          w |= other << (8 * BITS * off);
-        }
-        if (live[k] && (lane % LPW) == 0) code[out_bit / 32] = w;
-      }
-      if (live[k] && (lane % LPG) == 0) {
-        const int64_t gi = (row[k] * T + t0[k]) / GROUP;
-        scale[gi] = sc;
-        mn_out[gi] = lo;
-      }
-    }
+    for (int i = 0; i < BITS; ++i) dst[i] = word[i];
+  }
+  if (u % LPG == 0) {
+    scale[u / LPG] = sc;
+    mn_out[u / LPG] = lo;
   }
 }
 
@@ -168,151 +151,187 @@ __global__ void __launch_bounds__(128) quantize_cols_kernel(const __half* __rest
   mn_out[row * G + gi] = lo;
 }
 
-// Same, two adjacent channels per thread (4-byte loads, half2 arithmetic): the usual case of an even,
-// 4-byte aligned channel count.  A warp reads 128 contiguous bytes per token.
-template <int BITS>
-__global__ void __launch_bounds__(64) quantize_cols2_kernel(const __half* __restrict__ x, int64_t inner, int64_t T,
-                                                            int64_t outer_stride, int64_t t_stride, int group,
-                                                            uint32_t* __restrict__ code, __half* __restrict__ scale,
-                                                            __half* __restrict__ mn_out) {
-  constexpr int FPI = 32 / BITS;
-  const float levels = static_cast<float>((1 << BITS) - 1);
-  const int64_t d = 2 * (static_cast<int64_t>(blockIdx.y) * blockDim.x + threadIdx.x);
-  if (d >= inner) return;
-  const int64_t o = blockIdx.z;
-  const int64_t gi = blockIdx.x;  // group index along T
-  const __half* src = x + o * outer_stride + d + gi * group * t_stride;
-  auto at = [&](int t) { return *reinterpret_cast<const __half2*>(src + t * t_stride); };
-  __half2 lo = at(0), hi = lo;
-#pragma unroll 8
-  for (int t = 1; t < group; ++t) {
-    const __half2 v = at(t);
-    lo = __hmin2_nan(lo, v);
-    hi = __hmax2_nan(hi, v);
-  }
-  const __half sc0 = quant_scale(__low2half(lo), __low2half(hi), levels);
-  const __half sc1 = quant_scale(__high2half(lo), __high2half(hi), levels);
-  const QuantGroup g0 = quant_group(__low2half(lo), sc0, levels), g1 = quant_group(__high2half(lo), sc1, levels);
-  const int64_t row = o * inner + d;
-  const int64_t W = T / FPI;
-  uint32_t* dst0 = code + row * W + gi * (group / FPI);
-  uint32_t* dst1 = dst0 + W;
-  for (int w = 0; w < group / FPI; ++w) {
-    uint32_t word0 = 0, word1 = 0;
-#pragma unroll
-    for (int i = 0; i < FPI; ++i) {
-      const uint32_t c2 = quant_code_fast2(at(w * FPI + i), g0, g1);
-      word0 |= (c2 & 0xFFFFu) << (i * BITS);
-      word1 |= (c2 >> 16) << (i * BITS);
-    }
-    dst0[w] = word0;
-    dst1[w] = word1;
-  }
-  const int64_t G = T / group;
-  scale[row * G + gi] = sc0;
-  mn_out[row * G + gi] = __low2half(lo);
-  scale[(row + 1) * G + gi] = sc1;
-  mn_out[(row + 1) * G + gi] = __high2half(lo);
-}
-
-// The same for groups of 32 tokens, a tile of 8 groups x 128 channels per CTA.  The kernel above writes every word
-// with its own 4-byte store one code row apart from its neighbour's and reads every value twice; here a thread
-// keeps the 32 values of a group in registers (one pass), the tile's words and scale / zero halfs meet in shared
-// memory, and the CTA stores each channel's 8 groups as one contiguous run (32 x BITS bytes of codes, 16 bytes of
-// scales), consecutive threads on consecutive words.  256 threads: thread = (channel pair cp, group lane gl), groups
-// gl and gl + 4 of the tile.  Arithmetic and results are those of the kernel above.
-constexpr int QT_GROUPS = 8;     // groups per tile
+// The usual case of an even, 4-byte aligned channel count: a tile of 128 tokens x 128 channels per CTA, 32 tokens of two
+// adjacent channels per thread, kept in registers (one pass over the source, 128 contiguous bytes per token and warp).
+// Groups of 64 and 128 tokens exchange their minima and maxima through shared memory.  The words and the scale / zero
+// halfs of the tile meet in shared memory too, and each channel's run (16 x BITS bytes of codes) is stored by
+// consecutive threads.
+constexpr int QT_SUBS = 4;       // runs of 32 tokens per tile
 constexpr int QT_CH = 128;       // channels per tile
 template <int BITS>
-__global__ void __launch_bounds__(256) quantize_cols_tile_kernel(const __half* __restrict__ x, int64_t inner, int64_t T,
-                                                                 int64_t outer_stride, int64_t t_stride,
-                                                                 uint32_t* __restrict__ code, __half* __restrict__ scale,
-                                                                 __half* __restrict__ mn_out) {
-  constexpr int GROUP = 32;
-  constexpr int FPI = 32 / BITS;          // codes per word
-  constexpr int WPG = GROUP / FPI;        // words per group = BITS
-  constexpr int ROW = QT_GROUPS * WPG + 1;  // words per staged channel row (+1: rows land in different banks)
-  __shared__ uint32_t s_words[QT_CH * ROW];
-  __shared__ __half s_scale[QT_CH * QT_GROUPS], s_min[QT_CH * QT_GROUPS];
+__global__ void __launch_bounds__(256, 4) quantize_cols_tile_kernel(const __half* __restrict__ x, int64_t inner, int64_t T,
+                                                                    int64_t outer_stride, int64_t t_stride, int gshift,
+                                                                    bool vec_out, uint32_t* __restrict__ code,
+                                                                    __half* __restrict__ scale, __half* __restrict__ mn_out) {
+  // words of a staged channel row: 16-byte steps, and the rows of neighbouring lanes (every other channel: even channels
+  // are staged before odd ones) start in different banks
+  constexpr int ROW = QT_SUBS * BITS + 4;
+  __shared__ __align__(16) uint32_t s_words[QT_CH * ROW];
+  __shared__ __half2 s_lo[256], s_hi[256];
+  __shared__ __half s_scale[QT_CH * QT_SUBS], s_min[QT_CH * QT_SUBS];
   const float levels = static_cast<float>((1 << BITS) - 1);
-  const int tid = threadIdx.x, cp = tid & 63, gl = tid >> 6;
-  const int64_t G = T / GROUP;
-  const int64_t g_first = static_cast<int64_t>(blockIdx.x) * QT_GROUPS;
-  const int ngr = static_cast<int>(G - g_first < QT_GROUPS ? G - g_first : QT_GROUPS);
+  const int tid = threadIdx.x, cp = tid & 63, sub = tid >> 6, gs = gshift - 5;  // 2^gs runs per group
+  const int64_t subs = T / 32, first = static_cast<int64_t>(blockIdx.x) * QT_SUBS;
+  const int nsub = static_cast<int>(subs - first < QT_SUBS ? subs - first : QT_SUBS);
   const int64_t d0 = static_cast<int64_t>(blockIdx.y) * QT_CH;
   const int nch = static_cast<int>(inner - d0 < QT_CH ? inner - d0 : QT_CH);  // even: the host checks inner % 2 == 0
   const int64_t o = blockIdx.z;
   const int ch = 2 * cp;
-  if (ch < nch) {
-    for (int gq = gl; gq < ngr; gq += 4) {
-      const __half* src = x + o * outer_stride + d0 + ch + (g_first + gq) * GROUP * t_stride;
-      __half2 v[GROUP];
+  const bool live = ch < nch && sub < nsub;
+  __half2 v[32], lo, hi;
+  if (live) {
+    const __half* src = x + o * outer_stride + d0 + ch + (first + sub) * 32 * t_stride;
 #pragma unroll
-      for (int t = 0; t < GROUP; ++t) v[t] = *reinterpret_cast<const __half2*>(src + t * t_stride);
-      __half2 lo = v[0], hi = v[0];
+    for (int t = 0; t < 32; ++t) v[t] = *reinterpret_cast<const __half2*>(src + t * t_stride);
+    lo = hi = v[0];
 #pragma unroll
-      for (int t = 1; t < GROUP; ++t) {
-        lo = __hmin2_nan(lo, v[t]);
-        hi = __hmax2_nan(hi, v[t]);
+    for (int t = 1; t < 32; ++t) {
+      lo = __hmin2_nan(lo, v[t]);
+      hi = __hmax2_nan(hi, v[t]);
+    }
+  }
+  if (gs > 0) {
+    if (live) {
+      s_lo[tid] = lo;
+      s_hi[tid] = hi;
+    }
+    __syncthreads();
+    if (live) {
+      for (int k = 1; k < (1 << gs); ++k) {  // a group's runs are all in the tile: T is a multiple of the group
+        lo = __hmin2_nan(lo, s_lo[(sub ^ k) * 64 + cp]);
+        hi = __hmax2_nan(hi, s_hi[(sub ^ k) * 64 + cp]);
       }
-      const __half sc0 = quant_scale(__low2half(lo), __low2half(hi), levels);
-      const __half sc1 = quant_scale(__high2half(lo), __high2half(hi), levels);
-      const QuantGroup g0 = quant_group(__low2half(lo), sc0, levels), g1 = quant_group(__high2half(lo), sc1, levels);
-      uint32_t* w0 = s_words + ch * ROW + gq * WPG;
-      uint32_t* w1 = w0 + ROW;
+    }
+  }
+  if (live) {
+    const __half sc0 = quant_scale(__low2half(lo), __low2half(hi), levels);
+    const __half sc1 = quant_scale(__high2half(lo), __high2half(hi), levels);
+    uint32_t w0[BITS], w1[BITS];
+    quant_cols32<BITS>(v, quant_pair(__low2half(lo), sc0, __high2half(lo), sc1), w0, w1);
+    uint32_t *r0 = s_words + cp * ROW + sub * BITS, *r1 = r0 + 64 * ROW;
+    if constexpr (BITS >= 4) {
 #pragma unroll
-      for (int w = 0; w < WPG; ++w) {
-        uint32_t word0 = 0, word1 = 0;
-#pragma unroll
-        for (int i = 0; i < FPI; ++i) {
-          const uint32_t c2 = quant_code_fast2(v[w * FPI + i], g0, g1);
-          word0 |= (c2 & 0xFFFFu) << (i * BITS);
-          word1 |= (c2 >> 16) << (i * BITS);
-        }
-        w0[w] = word0;
-        w1[w] = word1;
+      for (int i = 0; i < BITS / 4; ++i) {
+        reinterpret_cast<uint4*>(r0)[i] = make_uint4(w0[4 * i], w0[4 * i + 1], w0[4 * i + 2], w0[4 * i + 3]);
+        reinterpret_cast<uint4*>(r1)[i] = make_uint4(w1[4 * i], w1[4 * i + 1], w1[4 * i + 2], w1[4 * i + 3]);
       }
-      s_scale[ch * QT_GROUPS + gq] = sc0;
-      s_min[ch * QT_GROUPS + gq] = __low2half(lo);
-      s_scale[(ch + 1) * QT_GROUPS + gq] = sc1;
-      s_min[(ch + 1) * QT_GROUPS + gq] = __high2half(lo);
+    } else {
+#pragma unroll
+      for (int i = 0; i < BITS; ++i) {
+        r0[i] = w0[i];
+        r1[i] = w1[i];
+      }
+    }
+    if ((sub & ((1 << gs) - 1)) == 0) {
+      const int at = ch * QT_SUBS + (sub >> gs);
+      s_scale[at] = sc0;
+      s_min[at] = __low2half(lo);
+      s_scale[at + QT_SUBS] = sc1;
+      s_min[at + QT_SUBS] = __high2half(lo);
     }
   }
   __syncthreads();
-  const int64_t row0 = o * inner + d0;
-  const int64_t W = T / FPI;
-  const int wpr = ngr * WPG;  // words of one channel row in this tile
-  for (int i = tid; i < nch * wpr; i += 256) {
-    const int r = i / wpr, w = i - r * wpr;
-    code[(row0 + r) * W + g_first * WPG + w] = s_words[r * ROW + w];
+  const int64_t row0 = o * inner + d0, W = subs * BITS, G = subs >> gs, g_first = first >> gs;
+  auto staged = [&](int r) { return s_words + ((r & 1) * 64 + (r >> 1)) * ROW; };
+  if (vec_out && nsub == QT_SUBS) {
+    for (int i = tid; i < nch * BITS; i += 256) {
+      const int r = i / BITS, w = i % BITS;
+      reinterpret_cast<uint4*>(code + (row0 + r) * W + first * BITS)[w] = reinterpret_cast<const uint4*>(staged(r))[w];
+    }
+  } else {
+    for (int i = tid; i < nch * QT_SUBS * BITS; i += 256) {
+      const int r = i / (QT_SUBS * BITS), w = i % (QT_SUBS * BITS);
+      if (w < nsub * BITS) code[(row0 + r) * W + first * BITS + w] = staged(r)[w];
+    }
   }
-  for (int i = tid; i < nch * ngr; i += 256) {
-    const int r = i / ngr, g = i - r * ngr;
-    scale[(row0 + r) * G + g_first + g] = s_scale[r * QT_GROUPS + g];
-    mn_out[(row0 + r) * G + g_first + g] = s_min[r * QT_GROUPS + g];
+  const int per = 2 - gs;  // log2(groups per tile)
+  for (int i = tid; i < nch << per; i += 256) {
+    const int r = i >> per, g = i & ((1 << per) - 1);
+    if (g << gs >= nsub) continue;
+    scale[(row0 + r) * G + g_first + g] = s_scale[r * QT_SUBS + g];
+    mn_out[(row0 + r) * G + g_first + g] = s_min[r * QT_SUBS + g];
   }
 }
 
 // ------------------------------------------------------------------------------------------------
-// unpack + two-rounding dequantise; one thread writes 8 consecutive fp16 values (16 bytes)
+// unpack + two-rounding dequantise.  A thread writes 16 consecutive fp16 values (one 32-byte store where the address allows
+// it: whole sectors, a warp's store is contiguous), DQ_UNITS times, all loads before the first store; pairs of
+// elements in fp16 arithmetic, whose one rounding equals the two of "widen, operate, narrow".
 // ------------------------------------------------------------------------------------------------
+constexpr int DQ_UNITS = 2;
 template <int BITS>
 __global__ void __launch_bounds__(256) dequantize_kernel(const uint32_t* __restrict__ code,
                                                          const __half* __restrict__ scale,
-                                                         const __half* __restrict__ mn, int64_t n_units, int group,
-                                                         __half* __restrict__ out) {
-  const int64_t u = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (u >= n_units) return;
-  const int64_t e0 = u * 8;  // first element (row-major over [rows, T]; T is a multiple of the group, group of 8)
-  const int64_t bit0 = e0 * BITS;
-  uint64_t bits = code[bit0 / 32];
-  if (BITS == 8) bits |= static_cast<uint64_t>(code[bit0 / 32 + 1]) << 32;
-  bits >>= (bit0 % 32);
-  const __half sc = scale[e0 / group], z = mn[e0 / group];
-  __half v[8];
+                                                         const __half* __restrict__ mn, int64_t n_units, int gshift,
+                                                         bool vec_in, bool by32, __half* __restrict__ out) {
+  constexpr int WORDS = BITS >= 2 ? BITS / 2 : 1;  // words of 16 codes (1 bit: half a word)
+  const int64_t u0 = static_cast<int64_t>(blockIdx.x) * (256 * DQ_UNITS) + threadIdx.x;
+  uint32_t w[DQ_UNITS][WORDS];
+  __half sc[DQ_UNITS], z[DQ_UNITS];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = dequant_2r(static_cast<uint32_t>(bits >> (i * BITS)) & ((1u << BITS) - 1), sc, z);
-  *reinterpret_cast<uint4*>(out + e0) = *reinterpret_cast<const uint4*>(v);
+  for (int k = 0; k < DQ_UNITS; ++k) {
+    const int64_t u = u0 + 256 * k;
+    if (u >= n_units) break;
+    const uint32_t* src = code + u * BITS / 2;
+    if (WORDS > 1 && vec_in) {
+      if constexpr (WORDS == 4) {
+        const uint4 c = *reinterpret_cast<const uint4*>(src);
+        w[k][0] = c.x, w[k][1] = c.y, w[k][2] = c.z, w[k][3] = c.w;
+      } else if constexpr (WORDS == 2) {
+        const uint2 c = *reinterpret_cast<const uint2*>(src);
+        w[k][0] = c.x, w[k][1] = c.y;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < WORDS; ++i) w[k][i] = src[i];
+      if (BITS == 1) w[k][0] >>= 16 * (u & 1);
+    }
+    const int64_t g = (u * 16) >> gshift;
+    sc[k] = scale[g];
+    z[k] = mn[g];
+  }
+#pragma unroll
+  for (int k = 0; k < DQ_UNITS; ++k) {
+    const int64_t u = u0 + 256 * k;
+    if (u >= n_units) break;
+    const __half2 s2 = __half2half2(sc[k]), z2 = __half2half2(z[k]);
+    auto value = [&](uint32_t c) {  // codes in bits [0, 10) and [16, 26) over a biased exponent
+      const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&c), __float2half2_rn(1024.f));
+      const __half2 r = __hadd2_rn(__hmul2_rn(h, s2), z2);
+      return *reinterpret_cast<const uint32_t*>(&r);
+    };
+    uint32_t v[8];
+    if constexpr (BITS == 8) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = value(__byte_perm(w[k][i / 2], 0x64646464u, i % 2 ? 0x4342 : 0x4140));
+    } else {
+      // codes i and i + HALF meet in a pair, and are put beside their neighbours at the end
+      constexpr int HALF = 16 / BITS, PER = BITS == 4 ? 8 : 16;  // codes in half a word (of 2 and 4 bits) and per run
+      const uint32_t m = ((1u << BITS) - 1) * 0x00010001u;
+#pragma unroll
+      for (int r = 0; r < 16 / PER; ++r) {
+        constexpr int H = BITS == 1 ? 8 : HALF;
+        const uint32_t x = BITS == 1 ? (w[k][0] & 0xFFu) | (w[k][0] & 0xFF00u) << 8 : w[k][r];
+        uint32_t p[H];
+#pragma unroll
+        for (int i = 0; i < H; ++i) p[i] = value(((x >> (i * BITS)) & m) | 0x64006400u);
+#pragma unroll
+        for (int i = 0; i < H / 2; ++i) {
+          v[r * PER / 2 + i] = __byte_perm(p[2 * i], p[2 * i + 1], 0x5410);
+          v[r * PER / 2 + H / 2 + i] = __byte_perm(p[2 * i], p[2 * i + 1], 0x7632);
+        }
+      }
+    }
+    __half* dst = out + u * 16;
+    if (by32) {
+      asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+                   "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                   : "memory");
+    } else {
+      reinterpret_cast<uint4*>(dst)[0] = make_uint4(v[0], v[1], v[2], v[3]);
+      reinterpret_cast<uint4*>(dst)[1] = make_uint4(v[4], v[5], v[6], v[7]);
+    }
+  }
 }
 
 template <int BITS>
@@ -338,31 +357,22 @@ __global__ void __launch_bounds__(256) unpack_kernel(const uint32_t* __restrict_
   for (int i = 0; i < FPI; ++i) out[w * FPI + i] = __uint2half_rn((word >> (i * BITS)) & ((1u << BITS) - 1));
 }
 
-template <int BITS>
-static int launch_quant_rows(const __half* x, int64_t rows, int64_t T, int64_t inner, int64_t os, int64_t is,
-                             int group, bool vec_ok, uint32_t* code, __half* scale, __half* mn, cudaStream_t st) {
-  const int64_t units = rows * (T / 8);
-  const int threads = 256;
-  // two units per thread and step; beyond 64 CTAs per SM the grid strides, sized so that every step is full
-  // (a last step that only some CTAs take costs a whole step's time)
-  const int64_t per_step = 2 * threads;
-  const int64_t steps = ceil_div(units, per_step * 148 * 64);
-  int64_t blocks = ceil_div(units, per_step * (steps < 1 ? 1 : steps));
-  if (blocks < 1) blocks = 1;
-  switch (group) {
-    case 32:
-      quantize_rows_kernel<BITS, 32><<<blocks, threads, 0, st>>>(x, rows, T, inner, os, is, vec_ok, code, scale, mn);
-      break;
-    case 64:
-      quantize_rows_kernel<BITS, 64><<<blocks, threads, 0, st>>>(x, rows, T, inner, os, is, vec_ok, code, scale, mn);
-      break;
-    default:
-      quantize_rows_kernel<BITS, 128><<<blocks, threads, 0, st>>>(x, rows, T, inner, os, is, vec_ok, code, scale, mn);
-      break;
-  }
-  return 0;
-}
+static int log2_group(int group) { return group == 32 ? 5 : group == 64 ? 6 : 7; }
 
+template <int BITS>
+static void launch_quant_rows(const __half* x, int64_t rows, int64_t T, int64_t inner, int64_t os, int64_t is, int group,
+                              uint32_t* code, __half* scale, __half* mn, cudaStream_t st) {
+  const int64_t units = rows * (T / 32);
+  const unsigned blocks = static_cast<unsigned>(ceil_div(units, 256));
+  int align = 2;
+  if (aligned(x, 16) && os % 8 == 0 && is % 8 == 0) align = aligned(x, 32) && os % 16 == 0 && is % 16 == 0 ? 32 : 16;
+  const bool vec_out = aligned(code, 16);
+  switch (group) {
+    case 32: quantize_rows_kernel<BITS, 32><<<blocks, 256, 0, st>>>(x, units, T, inner, os, is, align, vec_out, code, scale, mn); break;
+    case 64: quantize_rows_kernel<BITS, 64><<<blocks, 256, 0, st>>>(x, units, T, inner, os, is, align, vec_out, code, scale, mn); break;
+    default: quantize_rows_kernel<BITS, 128><<<blocks, 256, 0, st>>>(x, units, T, inner, os, is, align, vec_out, code, scale, mn); break;
+  }
+}
 
 // ------------------------------------------------------------------------------------------------
 // Gaussian-codebook codec at 1 bit (the low tier of 'high_uniform_group_low_normal_group')
@@ -447,35 +457,26 @@ extern "C" int hqkv_quantize_pack(const void* x, int64_t rows, int64_t T, int64_
   __half* s = static_cast<__half*>(scale);
   __half* m = static_cast<__half*>(mn);
   if (t_stride == 1) {
-    const bool vec_ok = aligned(x, 16) && outer_stride % 8 == 0 && inner_stride % 8 == 0;
     switch (bits) {
-      case 8: launch_quant_rows<8>(xs, rows, T, inner, outer_stride, inner_stride, group, vec_ok, c, s, m, st); break;
-      case 4: launch_quant_rows<4>(xs, rows, T, inner, outer_stride, inner_stride, group, vec_ok, c, s, m, st); break;
-      case 2: launch_quant_rows<2>(xs, rows, T, inner, outer_stride, inner_stride, group, vec_ok, c, s, m, st); break;
-      default: launch_quant_rows<1>(xs, rows, T, inner, outer_stride, inner_stride, group, vec_ok, c, s, m, st); break;
+      case 8: launch_quant_rows<8>(xs, rows, T, inner, outer_stride, inner_stride, group, c, s, m, st); break;
+      case 4: launch_quant_rows<4>(xs, rows, T, inner, outer_stride, inner_stride, group, c, s, m, st); break;
+      case 2: launch_quant_rows<2>(xs, rows, T, inner, outer_stride, inner_stride, group, c, s, m, st); break;
+      default: launch_quant_rows<1>(xs, rows, T, inner, outer_stride, inner_stride, group, c, s, m, st); break;
     }
   } else if (inner_stride == 1) {
     const int64_t outer = rows / inner;
     HQKV_REQUIRE(outer <= 65535 && ceil_div(inner, 128) <= 65535, "quantize_pack: too many rows for the column path");
     dim3 grid(static_cast<unsigned>(T / group), static_cast<unsigned>(ceil_div(inner, 128)),
               static_cast<unsigned>(outer));
-    if (group == 32 && inner % 2 == 0 && aligned(x, 4) && outer_stride % 2 == 0 && t_stride % 2 == 0) {
-      dim3 gridt(static_cast<unsigned>(ceil_div(T / group, QT_GROUPS)), static_cast<unsigned>(ceil_div(inner, QT_CH)),
-                 static_cast<unsigned>(outer));
+    if (inner % 2 == 0 && aligned(x, 4) && outer_stride % 2 == 0 && t_stride % 2 == 0) {
+      const dim3 tiles(static_cast<unsigned>(ceil_div(T, 32 * QT_SUBS)), grid.y, grid.z);
+      const bool vec_out = aligned(code, 16) && T / 32 * bits % 4 == 0;
+      const int gshift = log2_group(group);
       switch (bits) {
-        case 8: quantize_cols_tile_kernel<8><<<gridt, 256, 0, st>>>(xs, inner, T, outer_stride, t_stride, c, s, m); break;
-        case 4: quantize_cols_tile_kernel<4><<<gridt, 256, 0, st>>>(xs, inner, T, outer_stride, t_stride, c, s, m); break;
-        case 2: quantize_cols_tile_kernel<2><<<gridt, 256, 0, st>>>(xs, inner, T, outer_stride, t_stride, c, s, m); break;
-        default: quantize_cols_tile_kernel<1><<<gridt, 256, 0, st>>>(xs, inner, T, outer_stride, t_stride, c, s, m); break;
-      }
-    } else if (inner % 2 == 0 && aligned(x, 4) && outer_stride % 2 == 0 && t_stride % 2 == 0) {
-      dim3 grid2(static_cast<unsigned>(T / group), static_cast<unsigned>(ceil_div(inner, 128)),
-                 static_cast<unsigned>(outer));
-      switch (bits) {
-        case 8: quantize_cols2_kernel<8><<<grid2, 64, 0, st>>>(xs, inner, T, outer_stride, t_stride, group, c, s, m); break;
-        case 4: quantize_cols2_kernel<4><<<grid2, 64, 0, st>>>(xs, inner, T, outer_stride, t_stride, group, c, s, m); break;
-        case 2: quantize_cols2_kernel<2><<<grid2, 64, 0, st>>>(xs, inner, T, outer_stride, t_stride, group, c, s, m); break;
-        default: quantize_cols2_kernel<1><<<grid2, 64, 0, st>>>(xs, inner, T, outer_stride, t_stride, group, c, s, m); break;
+        case 8: quantize_cols_tile_kernel<8><<<tiles, 256, 0, st>>>(xs, inner, T, outer_stride, t_stride, gshift, vec_out, c, s, m); break;
+        case 4: quantize_cols_tile_kernel<4><<<tiles, 256, 0, st>>>(xs, inner, T, outer_stride, t_stride, gshift, vec_out, c, s, m); break;
+        case 2: quantize_cols_tile_kernel<2><<<tiles, 256, 0, st>>>(xs, inner, T, outer_stride, t_stride, gshift, vec_out, c, s, m); break;
+        default: quantize_cols_tile_kernel<1><<<tiles, 256, 0, st>>>(xs, inner, T, outer_stride, t_stride, gshift, vec_out, c, s, m); break;
       }
     } else
     switch (bits) {
@@ -500,17 +501,19 @@ extern "C" int hqkv_dequantize_unpack(const void* code, const void* scale, const
   HQKV_REQUIRE(code && scale && mn && out, "dequantize_unpack: null pointer");
   HQKV_REQUIRE(aligned(out, 16), "dequantize_unpack: output must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int64_t units = rows * T / 8;
-  const unsigned blocks = static_cast<unsigned>(ceil_div(units, 256));
+  const int64_t units = rows * T / 16;
+  const unsigned blocks = static_cast<unsigned>(ceil_div(units, 256 * DQ_UNITS));
+  const bool vec_in = aligned(code, 16), by32 = aligned(out, 32);
+  const int gshift = log2_group(group);
   const uint32_t* c = static_cast<const uint32_t*>(code);
   const __half* s = static_cast<const __half*>(scale);
   const __half* m = static_cast<const __half*>(mn);
   __half* o = static_cast<__half*>(out);
   switch (bits) {
-    case 8: dequantize_kernel<8><<<blocks, 256, 0, st>>>(c, s, m, units, group, o); break;
-    case 4: dequantize_kernel<4><<<blocks, 256, 0, st>>>(c, s, m, units, group, o); break;
-    case 2: dequantize_kernel<2><<<blocks, 256, 0, st>>>(c, s, m, units, group, o); break;
-    default: dequantize_kernel<1><<<blocks, 256, 0, st>>>(c, s, m, units, group, o); break;
+    case 8: dequantize_kernel<8><<<blocks, 256, 0, st>>>(c, s, m, units, gshift, vec_in, by32, o); break;
+    case 4: dequantize_kernel<4><<<blocks, 256, 0, st>>>(c, s, m, units, gshift, vec_in, by32, o); break;
+    case 2: dequantize_kernel<2><<<blocks, 256, 0, st>>>(c, s, m, units, gshift, vec_in, by32, o); break;
+    default: dequantize_kernel<1><<<blocks, 256, 0, st>>>(c, s, m, units, gshift, vec_in, by32, o); break;
   }
   HQKV_LAUNCH_CHECK("dequantize_unpack");
   return HQKV_OK;

@@ -116,6 +116,83 @@ __device__ __forceinline__ uint32_t quant_code_fast2(__half2 x, const QuantGroup
 }
 __device__ __forceinline__ uint32_t quant_code_fast2(__half2 x, const QuantGroup& g) { return quant_code_fast2(x, g, g); }
 
+// Codes of 32 values at a time.  The quotient is the correctly rounded fp32 one, as above, from 1/scale in two floats: d * lo is
+// far below half an ulp, so RN(d * hi + d * lo) is RN(d / scale) wherever d / scale keeps more than 2^-46 of it from a rounding
+// boundary, and the quotient of two 11-bit significands keeps 2^-36.  Two instructions for a pair of elements (f32x2)
+// instead of six; a group whose scale is 0, inf or NaN has all codes 0, by one mask for its words instead of a test per
+// element.  Pairs are gathered into bytes and the bytes into words, four elements at a time.
+struct QuantPair {  // low half of a pair in one group, high half in another or the same
+  __half2 mn;
+  float2 rcp, lo;
+  uint32_t keep0, keep1;  // 0 where all codes of the group are 0
+};
+__device__ __forceinline__ QuantPair quant_pair(__half mn0, __half sc0, __half mn1, __half sc1) {
+  QuantPair g;
+  g.mn = __halves2half2(mn0, mn1);
+  const float s0 = __half2float(sc0), s1 = __half2float(sc1);
+  g.rcp = make_float2(__frcp_rn(s0), __frcp_rn(s1));
+  g.lo = make_float2(__fmaf_rn(-g.rcp.x, s0, 1.f) * g.rcp.x, __fmaf_rn(-g.rcp.y, s1, 1.f) * g.rcp.y);
+  g.keep0 = s0 > 0.f && s0 < __int_as_float(0x7F800000) ? 0xFFFFFFFFu : 0u;
+  g.keep1 = s1 > 0.f && s1 < __int_as_float(0x7F800000) ? 0xFFFFFFFFu : 0u;
+  return g;
+}
+__device__ __forceinline__ QuantPair quant_pair(__half mn, __half sc) { return quant_pair(mn, sc, mn, sc); }
+// the codes of a pair in bytes 0 and 2 (bytes 1 and 3 are not 0)
+template <int BITS>
+__device__ __forceinline__ uint32_t quant_pair_bytes(__half2 x, const QuantPair& g) {
+  const float2 d = __half22float2(__hsub2(x, g.mn));
+  float2 q;
+  asm("{\n.reg .b64 d, r, l, q;\nmov.b64 d, {%2, %3};\nmov.b64 r, {%4, %5};\nmov.b64 l, {%6, %7};\nmul.rn.f32x2 q, d, l;\n"
+      "fma.rn.f32x2 q, d, r, q;\nmov.b64 {%0, %1}, q;\n}"
+      : "=f"(q.x), "=f"(q.y)
+      : "f"(d.x), "f"(d.y), "f"(g.rcp.x), "f"(g.rcp.y), "f"(g.lo.x), "f"(g.lo.y));
+  __half2 u = __hmin2(__floats2half2_rn(q.x, q.y), __float2half2_rn(static_cast<float>((1 << BITS) - 1)));
+  u = __hadd2(u, __float2half2_rn(1024.f));  // 1024 + rint(u): fp16 has unit spacing there, ties to even
+  return *reinterpret_cast<uint32_t*>(&u);
+}
+// BITS words from 32 codes in 8 registers of 4 bytes
+template <int BITS>
+__device__ __forceinline__ void pack_bytes(const uint32_t* q, uint32_t keep, uint32_t* word) {
+#pragma unroll
+  for (int w = 0; w < BITS; ++w) {
+    if constexpr (BITS == 8) {
+      word[w] = q[w] & keep;
+    } else if constexpr (BITS == 4) {
+      const uint32_t a = q[2 * w] | q[2 * w] >> 4, b = q[2 * w + 1] | q[2 * w + 1] >> 4;
+      word[w] = __byte_perm(a, b, 0x6420) & keep;
+    } else {
+      uint32_t b[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        b[i] = BITS == 2 ? __dp4a(q[4 * w + i], 0x40100401u, 0u)
+                         : __dp4a(q[2 * i + 1], 0x80402010u, __dp4a(q[2 * i], 0x08040201u, 0u));
+      word[w] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410) & keep;
+    }
+  }
+}
+// 32 values of one group, in order: BITS words
+template <int BITS>
+__device__ __forceinline__ void quant_row32(const __half2 (&v)[16], const QuantPair& g, uint32_t* word) {
+  uint32_t q[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) q[i] = __byte_perm(quant_pair_bytes<BITS>(v[2 * i], g), quant_pair_bytes<BITS>(v[2 * i + 1], g), 0x6420);
+  pack_bytes<BITS>(q, g.keep0, word);
+}
+// 32 pairs, low halves of one group and high halves of another: BITS words of each
+template <int BITS>
+__device__ __forceinline__ void quant_cols32(const __half2 (&v)[32], const QuantPair& g, uint32_t* word0, uint32_t* word1) {
+  uint32_t q0[8], q1[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t a = __byte_perm(quant_pair_bytes<BITS>(v[4 * i], g), quant_pair_bytes<BITS>(v[4 * i + 1], g), 0x6240);
+    const uint32_t b = __byte_perm(quant_pair_bytes<BITS>(v[4 * i + 2], g), quant_pair_bytes<BITS>(v[4 * i + 3], g), 0x6240);
+    q0[i] = __byte_perm(a, b, 0x5410);
+    q1[i] = __byte_perm(a, b, 0x7632);
+  }
+  pack_bytes<BITS>(q0, g.keep0, word0);
+  pack_bytes<BITS>(q1, g.keep1, word1);
+}
+
 // scale = half(half(mx - mn) / levels)
 __device__ __forceinline__ __half quant_scale(__half mn, __half mx, float levels) {
   return h_divf(h_sub(mx, mn), levels);
