@@ -46,7 +46,7 @@ struct TierDev {
   int n_k, n_v;
   int bits;
   int normal;  // 1-bit tier in the Gaussian-codebook codec: value = std * (+-C) + mean, scale slots = std, zero = mean
-  int k_unit0, v_unit0;      // where the tier's units start in the list of a plane's units (K pass, V pass)
+  int k_cost0, v_cost0;      // cost of the plane's units before the tier's (K pass, V pass)
   int k_cta0, v_cta0;        // ... and its CTAs in the list of the plane's, where no CTA has units of two tiers
 };
 
@@ -84,16 +84,21 @@ struct DecodeParams {
 };
 
 // The tokens of a (batch, virtual kv head) plane are a list of UNITS - 256 tokens of one tier (128 at 8 bits, 64 of the
-// fp16 tier and of the residual window), tiers in order - and its CTAs take consecutive shares of it.
+// fp16 tier and of the residual window), tiers in order - and its CTAs take consecutive shares of it of equal COST: a unit
+// of 8 bits takes both passes 0.6 of the time of one of 4 or 2 bits (2.2 against 3.4 us in the K pass, 2.3 against 3.9
+// in the V pass with four CTAs on every SM), and the CTA with the longest share decides (20/40/40 at 24 x 8 x 15360 tokens
+// in shares of equal count: the V pass took 94 us, the time of the CTAs with 4 and 2 bits only).
 __host__ __device__ constexpr int unit_tokens(int bits) { return bits == 16 ? 64 : bits == 8 ? 128 : 256; }
+__host__ __device__ constexpr int unit_cost(int bits) { return bits == 8 ? 5 : 8; }
 // This CTA's tokens [t0, t1) of tier ti; false: none.
 template <bool V>
 __device__ __forceinline__ bool share_of(const DecodeParams& P, int ti, int bits, int& t0, int& t1) {
   const TierDev& T = P.tier[ti];
   const int i = blockIdx.y, per = V ? P.v_per : P.k_per, more = V ? P.v_more : P.k_more;
-  const int u0 = i * per + min(i, more) - (V ? T.v_unit0 : T.k_unit0), u1 = u0 + per + (i < more ? 1 : 0);
-  t0 = max(u0, 0) * unit_tokens(bits);
-  t1 = min(u1 * unit_tokens(bits), V ? T.n_v : T.n_k);
+  const int c0 = i * per + min(i, more) - (V ? T.v_cost0 : T.k_cost0), c1 = c0 + per + (i < more ? 1 : 0);
+  const int c = unit_cost(bits);  // a unit belongs to the share that its cost starts in
+  t0 = (max(c0, 0) + c - 1) / c * unit_tokens(bits);
+  t1 = min((max(c1, 0) + c - 1) / c * unit_tokens(bits), V ? T.n_v : T.n_k);
   return t0 < t1;
 }
 // The same where no CTA has units of two tiers: the tier, too.
@@ -405,7 +410,7 @@ __device__ __forceinline__ void k_zero_term(const KScales& k, const uint4& q, fl
 
 // Request the codes of a chunk: src / dst = this thread's first piece, valid = bytes per row (a multiple of 32, 16, 8, 4
 // at 8, 4, 2, 1 bits).  The rows of the 2-bit tier are only 8-byte aligned unless its token count is a multiple of 64
-// (wide2), those of the 1-bit tier 4-byte.
+// (wide2; otherwise the even rows are copied 16 bytes and the odd ones 8 bytes at a time), those of the 1-bit tier 4-byte.
 // The piece index is XORed with row bits so that the eight rows of an ldmatrix (same logical piece) and the pieces a
 // cp.async instruction writes both spread over all banks.
 template <int BITS>
@@ -414,6 +419,9 @@ struct KCopy {
   uint32_t dst;
   uint32_t step;   // bytes of memory between this thread's rows
   int first;       // first byte of the row that this thread copies
+  int64_t odd;     // 2 bits, odd rows off the 16-byte boundaries: their first piece, from src,
+  uint32_t odst;   // where it goes
+  int ofirst;      // and its first byte of the row
 };
 template <int BITS>
 __device__ __forceinline__ KCopy<BITS> k_copy_init(const TierDev& T, int bh, int t0, uint32_t codes, bool wide2) {
@@ -422,36 +430,54 @@ __device__ __forceinline__ KCopy<BITS> k_copy_init(const TierDev& T, int bh, int
   const int64_t row_bytes = static_cast<int64_t>(T.n_k) * BITS / 8;
   KCopy<BITS> k;
   int c, r0, bytes, rows;
-  if (BITS == 2 && wide2) {
-    c = tid & 3, r0 = tid >> 2, bytes = 16, rows = 32;
+  if constexpr (BITS == 2) {
+    c = tid & 3, r0 = wide2 ? tid >> 2 : 2 * (tid >> 2), bytes = 16, rows = 32;
     k.dst = codes + r0 * 64 + ((c ^ ((r0 >> 1) & 3)) << 4);
   } else {
-    c = tid & 7, r0 = tid >> 3, bytes = BITS >= 4 ? 16 : BITS == 2 ? 8 : 4, rows = 16;
+    c = tid & 7, r0 = tid >> 3, bytes = BITS >= 4 ? 16 : 4, rows = 16;
     k.dst = codes + (BITS >= 4 ? r0 * 128 + ((c ^ (r0 & 7)) << 4)
-                               : BITS == 2 ? r0 * 64 + (((c >> 1) ^ ((r0 >> 1) & 3)) << 4) + 8 * (c & 1) : r0 * TL::PITCH + 4 * c);
+                               : r0 * TL::PITCH + 4 * c);
   }
   k.first = c * bytes;
   k.step = static_cast<uint32_t>(rows * row_bytes);
   k.src = reinterpret_cast<const unsigned char*>(T.k_data) + (static_cast<int64_t>(bh) * D + r0) * row_bytes +
           static_cast<int64_t>(t0) * BITS / 8 + k.first;
+  if constexpr (BITS == 2) {
+    const int r1 = 2 * (tid >> 3) + 1, c1 = tid & 7;
+    k.ofirst = 8 * c1;
+    k.odd = (r1 - r0) * row_bytes + k.ofirst - k.first;
+    k.odst = codes + r1 * 64 + (((c1 >> 1) ^ ((r1 >> 1) & 3)) << 4) + 8 * (c1 & 1);
+  }
   return k;
 }
 template <int BITS>
 __device__ __forceinline__ void k_codes_request(const KCopy<BITS>& k, int chunk, int valid, bool wide2) {
   using TL = KTile<BITS>;
-  if (k.first >= valid) return;
   const unsigned char* s = k.src + static_cast<int64_t>(chunk) * (TL::TOKENS * BITS / 8);
   const uint32_t d = k.dst + (chunk & 1) * K_CODES;
-  if (BITS == 2 && wide2) {
+  if constexpr (BITS == 2) {
+    if (wide2) {
+      if (k.first >= valid) return;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) cp_async_16(d + i * 32 * TL::PITCH, s + static_cast<uint64_t>(k.step) * i);
+      for (int i = 0; i < 4; ++i) cp_async_16(d + i * 32 * TL::PITCH, s + static_cast<uint64_t>(k.step) * i);
+    } else {
+      if (k.first < valid) {  // (the last piece of a row may reach into the odd row behind it)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) cp_async_16(d + i * 64 * TL::PITCH, s + static_cast<uint64_t>(k.step) * (2 * i));
+      }
+      if (k.ofirst < valid) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          cp_async_8(k.odst + (chunk & 1) * K_CODES + i * 32 * TL::PITCH, s + k.odd + static_cast<uint64_t>(k.step) * i);
+      }
+    }
     return;
   }
+  if (k.first >= valid) return;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const unsigned char* p = s + static_cast<uint64_t>(k.step) * i;
     if (BITS >= 4) cp_async_16(d + i * 16 * TL::PITCH, p);
-    else if (BITS == 2) cp_async_8(d + i * 16 * TL::PITCH, p);
     else cp_async_4(d + i * 16 * TL::PITCH, p);
   }
 }
@@ -683,7 +709,7 @@ __device__ __forceinline__ void k_emit(const DecodeParams& P, const TierDev& T, 
   const int lb = k_lane_base<BITS>();
   float* out = P.logits + static_cast<int64_t>(w.bvh) * P.L * P.r4 + tig;
   // whole 32-token units are valid or not (a tier holds a multiple of 32 tokens)
-  bool valid[HALVES], dense = P.r4 == MAX_R4 && P.mask == nullptr;
+  bool valid[HALVES], dense = P.r4 >= 2 && P.mask == nullptr;
   uint32_t base[HALVES];
 #pragma unroll
   for (int u = 0; u < HALVES; ++u) {
@@ -692,26 +718,33 @@ __device__ __forceinline__ void k_emit(const DecodeParams& P, const TierDev& T, 
     dense = dense && (!valid[u] || (pu[u] == base[u] + lane && HQKV_INDEX_OK(pu[u], P.L)));
   }
   if (__all_sync(0xffffffffu, dense)) {
-    if constexpr (BITS == 4 || BITS == 8) {
+    const bool on = tig < P.r4;
+    auto store = [&](auto heads) {  // a constant distance between a lane's tokens
+      constexpr int R = decltype(heads)::value;
+      if constexpr (BITS == 4 || BITS == 8) {
 #pragma unroll
-      for (int u = 0; u < HALVES; ++u) {
-        float* o = out + static_cast<int64_t>(base[u] + lb) * MAX_R4;
+        for (int u = 0; u < HALVES; ++u) {
+          float* o = out + static_cast<int64_t>(base[u] + lb) * R;
+          const bool ok = valid[u] && (R == MAX_R4 || on);
 #pragma unroll
-        for (int j = 4 * u; j < 4 * u + 4; ++j) {
-          if (valid[u]) o[k_step<BITS>(j) * MAX_R4] = x[j];
+          for (int j = 4 * u; j < 4 * u + 4; ++j) {
+            if (ok) o[k_step<BITS>(j) * R] = x[j];
+            else x[j] = -INFINITY;
+          }
+        }
+      } else {
+        const bool second = k_lane_unit<BITS>() == 1;
+        const bool ok = (second ? valid[HALVES - 1] : valid[0]) && (R == MAX_R4 || on);
+        float* o = out + static_cast<int64_t>((second ? base[HALVES - 1] : base[0]) + lb) * R;
+#pragma unroll
+        for (int j = 0; j < NX; ++j) {
+          if (ok) o[k_step<BITS>(j) * R] = x[j];
           else x[j] = -INFINITY;
         }
       }
-    } else {
-      const bool second = k_lane_unit<BITS>() == 1;
-      const bool ok = second ? valid[HALVES - 1] : valid[0];
-      float* o = out + static_cast<int64_t>((second ? base[HALVES - 1] : base[0]) + lb) * MAX_R4;
-#pragma unroll
-      for (int j = 0; j < NX; ++j) {
-        if (ok) o[k_step<BITS>(j) * MAX_R4] = x[j];
-        else x[j] = -INFINITY;
-      }
-    }
+    };
+    if (P.r4 == MAX_R4) store(std::integral_constant<int, MAX_R4>());
+    else store(std::integral_constant<int, 2>());
   } else {
     k_store_any<BITS>(P, T, w, x, pu, wt0);
   }
@@ -1283,8 +1316,8 @@ __device__ __noinline__ void v_prepare_any(const DecodeParams& P, const Where& w
   }
 }
 
-// The same for a whole tile, four query heads and 128 >> GV channel groups known at compile time.  mh / inv: max *
-// log2(e) and 1 / sum of the lane's heads, wrow: their rows of probabilities.
+// The same for a whole tile, four or two query heads and 128 >> GV channel groups known at compile time.  mh / inv: max *
+// log2(e) and 1 / sum of the lane's heads, wrow: their rows of probabilities (null: no such heads).
 template <int BITS, int GV>
 __device__ __forceinline__ void v_prepare(uint32_t tile, const float (&x)[4][VTile<BITS>::HPL], const uint32_t (&pos)[4],
                                           const VLane<BITS>& L, const float (&mh)[VTile<BITS>::HPL],
@@ -1321,7 +1354,8 @@ __device__ __forceinline__ void v_prepare(uint32_t tile, const float (&x)[4][VTi
 #pragma unroll
   for (int h = 0; h < HPL; ++h) {
     __half *a = wrow[h] + pos[0], *b = wrow[h] + pos[2];
-    if (adjacent && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 3) == 0) {
+    if (wrow[h] == nullptr) {
+    } else if (adjacent && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 3) == 0) {
       *reinterpret_cast<uint32_t*>(a) = n2[h][0];
       *reinterpret_cast<uint32_t*>(b) = n2[h][1];
     } else {
@@ -1354,12 +1388,12 @@ __device__ __forceinline__ void v_prepare(uint32_t tile, const float (&x)[4][VTi
   }
 }
 
-// Four query heads: positions and logits of the lane's tokens without conditions (position 0 stands in beyond the tier).
+// Four or two query heads: logits of the lane's tokens without conditions (position 0 stands in beyond the tier).
 template <int HPL>
-__device__ __forceinline__ void v_gather4(float (&x)[4][HPL], const uint32_t (&pos)[4], const float* base) {
+__device__ __forceinline__ void v_gather4(float (&x)[4][HPL], const uint32_t (&pos)[4], const float* base, uint32_t heads) {
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const float* p = base + static_cast<uint64_t>(pos[j]) * MAX_R4;
+    const float* p = base + static_cast<uint64_t>(pos[j]) * heads;
     if constexpr (HPL == 2) {
       const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
       x[j][0] = v.x;
@@ -1520,9 +1554,10 @@ __device__ __forceinline__ void v_run(const DecodeParams& P, const TierDev& T, V
   advance();
   asm volatile("griddepcontrol.wait;" ::: "memory");
   float x[4][TL::HPL];
-  const float* lrow = P.logits + static_cast<int64_t>(w.bvh) * P.L * MAX_R4 + L.h0;
+  // With two query heads the lanes of the other two take the first two's logits to a probability of 0 and write none.
+  const float* lrow = P.logits + static_cast<int64_t>(w.bvh) * P.L * P.r4 + (L.h0 & (P.r4 - 1));
   auto gather = [&]() {
-    if constexpr (FAST) v_gather4<TL::HPL>(x, pos, lrow);
+    if constexpr (FAST) v_gather4<TL::HPL>(x, pos, lrow, static_cast<uint32_t>(P.r4));
     else v_gather<TL::HPL>(P, w, x, pos, L.h0);
   };
   gather();
@@ -1532,9 +1567,10 @@ __device__ __forceinline__ void v_run(const DecodeParams& P, const TierDev& T, V
   if constexpr (FAST) {
 #pragma unroll
     for (int h = 0; h < TL::HPL; ++h) {
-      mh[h] = sh.gm[L.h0 + h];
-      inv[h] = sh.ginv[L.h0 + h];
-      wrow[h] = P.weights + (static_cast<int64_t>(w.b) * P.nh_q + w.h0 + L.h0 + h) * P.L;
+      const bool on = L.h0 < P.r4;
+      mh[h] = on ? sh.gm[L.h0 + h] : INFINITY;
+      inv[h] = on ? sh.ginv[L.h0 + h] : 0.f;
+      wrow[h] = !on ? nullptr : P.weights + (static_cast<int64_t>(w.b) * P.nh_q + w.h0 + L.h0 + h) * P.L;
     }
   }
   float acc[8][4], za[4] = {0.f, 0.f, 0.f, 0.f}, zb[4] = {0.f, 0.f, 0.f, 0.f};
@@ -1768,7 +1804,7 @@ __device__ __noinline__ void head_sum_chunk(const DecodeParams& P, const TierDev
   }
 }
 
-// GV: log2 of the channel group, with four query heads per CTA and the softmax of the scratch logits; 0: everything else.
+// GV: log2 of the channel group, with four or two query heads per CTA and the softmax of the scratch logits; 0: everything else.
 // ONE_TIER: no CTA has units of two tiers.
 template <int GV, bool ONE_TIER>
 __global__ void __launch_bounds__(VTHREADS, V_MIN_CTAS) v_pass_kernel(const __grid_constant__ DecodeParams P) {
@@ -1942,22 +1978,23 @@ struct Layout {
 
 // How the CTAs of a plane share its units.  A CTA pays for its prologue, the softmax pairs and the output reduction
 // whatever it walks - about as much as two units - and the last wave of CTAs should be full: of one to four waves the
-// number of CTAs that finishes first.  Where that leaves a CTA one or two units, a second tier would double its latency:
+// number of CTAs that finishes first (counted in units of 4 bits).  Where that leaves a CTA one or two units, a second tier would double its latency:
 // there a CTA keeps to one tier.
 static void divide(DecodeParams& P, int64_t planes, int slots, bool v) {
-  int units = 0;
-  for (const TierDev& t : P.tier) units += static_cast<int>(ceil_div(v ? t.n_v : t.n_k, unit_tokens(t.bits)));
-  int ctas = 0, per = 0, more = 0;
+  int total = 0;  // cost of a plane
+  for (const TierDev& t : P.tier) total += static_cast<int>(ceil_div(v ? t.n_v : t.n_k, unit_tokens(t.bits))) * unit_cost(t.bits);
+  const int units = static_cast<int>(ceil_div(total, unit_cost(4)));
+  int ctas = 0, most = 0;
   int64_t best = -1;
   for (int waves = 1; units > 0 && waves <= 4; ++waves) {
     int64_t n = static_cast<int64_t>(slots) * waves / planes;
     n = n < 1 ? 1 : n > units ? units : n;
     const int64_t share = ceil_div(units, n), cost = ceil_div(ceil_div(units, share) * planes, slots) * (share + 2);
-    if (best < 0 || cost < best) best = cost, ctas = static_cast<int>(ceil_div(units, share)), per = units / ctas, more = units % ctas;
+    if (best < 0 || cost < best) best = cost, ctas = static_cast<int>(ceil_div(units, share)), most = static_cast<int>(share);
   }
-  if (units > 0 && per + (more > 0) <= 2) {
+  int per = ctas ? total / ctas : 0, more = ctas ? total % ctas : 0;
+  if (units > 0 && most <= 2) {
     int n = 0;
-    const int most = per + (more > 0);
     for (TierDev& t : P.tier) {
       (v ? t.v_cta0 : t.k_cta0) = n;
       n += static_cast<int>(ceil_div(v ? t.n_v : t.n_k, unit_tokens(t.bits) * most * (!v && t.bits == 8 ? 2 : 1)));
@@ -2038,10 +2075,10 @@ static int build_params(const hqkv_cache_desc_t* c, DecodeParams& P, Layout& lay
     d.v_zero = static_cast<const __half*>(s.v_zero);
     d.v_idx = s.v_idx;
     HQKV_REQUIRE(static_cast<int64_t>(s.n_k) * D * d.bits / 8 < (1ll << 31), "decode: tier %d K plane of one head exceeds 2 GiB", t);
-    d.k_unit0 = kc;
-    d.v_unit0 = vc;
-    kc += static_cast<int>(ceil_div(d.n_k, unit_tokens(d.bits)));
-    vc += static_cast<int>(ceil_div(d.n_v, unit_tokens(d.bits)));
+    d.k_cost0 = kc;
+    d.v_cost0 = vc;
+    kc += static_cast<int>(ceil_div(d.n_k, unit_tokens(d.bits))) * unit_cost(d.bits);
+    vc += static_cast<int>(ceil_div(d.n_v, unit_tokens(d.bits))) * unit_cost(d.bits);
     nk_total += d.n_k;
     nv_total += d.n_v;
   }
@@ -2057,10 +2094,8 @@ static int build_params(const hqkv_cache_desc_t* c, DecodeParams& P, Layout& lay
   }
   r.k_data = c->new_k;
   r.v_data = c->new_v;
-  r.k_unit0 = kc;
-  r.v_unit0 = vc;
-  kc += static_cast<int>(ceil_div(r.n_k, unit_tokens(16)));
-  vc += static_cast<int>(ceil_div(r.n_v, unit_tokens(16)));
+  r.k_cost0 = kc;
+  r.v_cost0 = vc;
   const int64_t L = ((sides & 1) ? nk_total : nv_total) + c->n_new;
   HQKV_REQUIRE(L > 0, "decode: the cache is empty");
   HQKV_REQUIRE(L < (1ll << 30), "decode: cache too long");
@@ -2239,7 +2274,7 @@ static int hqkv::decode_launch(const hqkv_cache_desc_t* cache_host, const void* 
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const bool fast = P.r4 == MAX_R4 && !P.probs_in && !HQKV_CHECKS_ENABLED;
+    const bool fast = P.r4 >= 2 && !P.probs_in && !HQKV_CHECKS_ENABLED;
     HQKV_CUDA(cudaLaunchKernelEx(&cfg, v_kernels[P.v_more < 0][fast ? P.gv_shift - 4 : 0], P));
   }
   return HQKV_OK;
