@@ -110,7 +110,7 @@ __device__ __forceinline__ int only_share(const DecodeParams& P, int& t0, int& t
   for (int t = 1; t <= HQKV_NUM_TIERS; ++t)
     if (i >= (V ? P.tier[t].v_cta0 : P.tier[t].k_cta0)) ti = t;
   const TierDev& T = P.tier[ti];
-  const int n = (V ? P.v_per : P.k_per * (T.bits == 8 ? 2 : 1)) * unit_tokens(T.bits);
+  const int c = unit_cost(T.bits), n = max(V ? P.v_per : P.k_per, c) / c * unit_tokens(T.bits);
   t0 = (i - (V ? T.v_cta0 : T.k_cta0)) * n;
   t1 = min(t0 + n, V ? T.n_v : T.n_k);
   return ti;
@@ -1978,28 +1978,36 @@ struct Layout {
 
 // How the CTAs of a plane share its units.  A CTA pays for its prologue, the softmax pairs and the output reduction
 // whatever it walks - about as much as two units - and the last wave of CTAs should be full: of one to four waves the
-// number of CTAs that finishes first (counted in units of 4 bits).  Where that leaves a CTA one or two units, a second tier would double its latency:
-// there a CTA keeps to one tier.
+// number of CTAs that finishes first (counted in units of 4 bits).  Where one or two units per CTA make a wave, a second tier
+// would double a CTA's latency: there a CTA keeps to one tier (two units at 8 bits).
 static void divide(DecodeParams& P, int64_t planes, int slots, bool v) {
   int total = 0;  // cost of a plane
   for (const TierDev& t : P.tier) total += static_cast<int>(ceil_div(v ? t.n_v : t.n_k, unit_tokens(t.bits))) * unit_cost(t.bits);
   const int units = static_cast<int>(ceil_div(total, unit_cost(4)));
-  int ctas = 0, most = 0;
+  int ctas = 0;
   int64_t best = -1;
   for (int waves = 1; units > 0 && waves <= 4; ++waves) {
     int64_t n = static_cast<int64_t>(slots) * waves / planes;
     n = n < 1 ? 1 : n > units ? units : n;
-    const int64_t share = ceil_div(units, n), cost = ceil_div(ceil_div(units, share) * planes, slots) * (share + 2);
-    if (best < 0 || cost < best) best = cost, ctas = static_cast<int>(ceil_div(units, share)), most = static_cast<int>(share);
+    const int64_t share = ceil_div(units, n), whole = ceil_div(units, share), cost = ceil_div(whole * planes, slots) * (share + 2);
+    // all of the wave's CTAs where each gets two units or more (the SMs' loads differ least), else those that whole shares fill
+    if (best < 0 || cost < best) best = cost, ctas = static_cast<int>(total / n >= 2 * unit_cost(4) ? n : whole);
   }
   int per = ctas ? total / ctas : 0, more = ctas ? total % ctas : 0;
-  if (units > 0 && most <= 2) {
+  // the cost that a CTA of one tier may have: the smallest with which the planes' CTAs fit one wave
+  auto one_tier = [&](int budget, bool set) {
     int n = 0;
     for (TierDev& t : P.tier) {
-      (v ? t.v_cta0 : t.k_cta0) = n;
-      n += static_cast<int>(ceil_div(v ? t.n_v : t.n_k, unit_tokens(t.bits) * most * (!v && t.bits == 8 ? 2 : 1)));
+      const int u = budget < unit_cost(t.bits) ? 1 : budget / unit_cost(t.bits);
+      if (set) (v ? t.v_cta0 : t.k_cta0) = n;
+      n += static_cast<int>(ceil_div(v ? t.n_v : t.n_k, unit_tokens(t.bits) * u));
     }
-    ctas = n, per = most, more = -1;
+    return n;
+  };
+  int budget = 2 * unit_cost(8);
+  while (budget <= 2 * unit_cost(4) && static_cast<int64_t>(one_tier(budget, false)) * planes > slots) ++budget;
+  if (total > 0 && budget <= 2 * unit_cost(4)) {
+    ctas = one_tier(budget, true), per = budget, more = -1;
   }
   (v ? P.nv_ctas : P.nk_ctas) = ctas;
   (v ? P.v_per : P.k_per) = per;
