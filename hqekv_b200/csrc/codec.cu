@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const __half* __rest
   const __half lo = __low2half(__hmin2_nan(lo2, __lowhigh2highlow(lo2))), hi = __low2half(__hmax2_nan(hi2, __lowhigh2highlow(hi2)));
   const __half sc = quant_scale(lo, hi, levels);
   uint32_t word[BITS];
-  quant_row32<BITS>(v, quant_pair(lo, sc), word);
+  quant_row32<BITS, false>(v, quant_pair(lo, sc), word);
   if (unit >= n_units) return;
   uint32_t* dst = code + u * BITS;
   if (vec_out) {
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(256, 4) quantize_cols_tile_kernel(const __half
     const __half sc0 = quant_scale(__low2half(lo), __low2half(hi), levels);
     const __half sc1 = quant_scale(__high2half(lo), __high2half(hi), levels);
     uint32_t w0[BITS], w1[BITS];
-    quant_cols32<BITS>(v, quant_pair(__low2half(lo), sc0, __high2half(lo), sc1), w0, w1);
+    quant_cols32<BITS, false>(v, quant_pair(__low2half(lo), sc0, __high2half(lo), sc1), w0, w1);
     uint32_t *r0 = s_words + cp * ROW + sub * BITS, *r1 = r0 + 64 * ROW;
     if constexpr (BITS >= 4) {
 #pragma unroll

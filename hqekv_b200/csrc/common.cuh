@@ -68,22 +68,15 @@ __device__ __forceinline__ __half h_add(__half a, __half b) {
   return __float2half_rn(__fadd_rn(__half2float(a), __half2float(b)));
 }
 
-// Code of one element: clamp(half(half(x - mn) / scale), 0, levels) rounded half-to-even.
-// A NaN quotient (constant group: scale == 0) gives code 0, as the float->int conversion on
-// the GPU does for the reference.
-__device__ __forceinline__ uint32_t quant_code(__half x, __half mn, __half scale, float levels) {
-  float u = __half2float(h_div(h_sub(x, mn), scale));
-  u = fminf(fmaxf(u, 0.f), levels);  // fmaxf(NaN, 0) == 0
-  return static_cast<uint32_t>(__float2int_rn(u));
-}
-
-// The same code for many elements of one group.  x - mn with the native fp16 subtract (one rounding
+// Code of one element: clamp(half(half(x - mn) / scale), 0, levels) rounded half-to-even; a NaN quotient (constant
+// group: scale == 0) gives code 0, as the float->int conversion on the GPU does for the reference.
+// For many elements of one group: x - mn with the native fp16 subtract (one rounding
 // of the exact difference equals the two roundings of "widen, subtract, narrow": fp32 carries 2*11 + 2
 // bits).  The quotient by Markstein's sequence: r = RN(1/scale) once per group, q0 = RN(d*r),
 // e = d - q0*scale (exact in one FMA), q1 = RN(q0 + e*r) is the correctly rounded fp32 quotient (the
 // scale has an 11-bit significand, never the all-ones fp32 significand the theorem excludes), so
-// half(q1) is what h_div returns; three FP32 instructions per element instead of a full IEEE divide.
-// A NaN or infinite intermediate (scale 0 or inf) ends as code 0 exactly as in quant_code.
+// half(q1) is the fp16 quotient; three FP32 instructions per element instead of a full IEEE divide.
+// A NaN or infinite intermediate (scale 0 or inf) ends as code 0.
 struct QuantGroup {
   __half mn;
   float scale, rcp, levels;
@@ -106,21 +99,12 @@ __device__ __forceinline__ uint32_t quant_code_fast(__half x, const QuantGroup& 
   u = fminf(fmaxf(u, 0.f), g.levels);  // fmaxf(NaN, 0) == 0
   return static_cast<uint32_t>(__float2int_rn(u));
 }
-// two elements (low half in group g, high half in group gh): codes in bits [0,10) and [16,26)
-__device__ __forceinline__ uint32_t quant_code_fast2(__half2 x, const QuantGroup& g, const QuantGroup& gh) {
-  const float2 d = __half22float2(__hsub2(x, __halves2half2(g.mn, gh.mn)));
-  __half2 u = __floats2half2_rn(quant_quotient(d.x, g), quant_quotient(d.y, gh));
-  u = __hmin2(__hmax2(u, __float2half2_rn(0.f)), __float2half2_rn(g.levels));  // max(NaN, 0) == 0
-  u = __hadd2(u, __float2half2_rn(1024.f));  // 1024 + rint(u): fp16 has unit spacing there, ties to even
-  return *reinterpret_cast<uint32_t*>(&u) & 0x03FF03FFu;
-}
-__device__ __forceinline__ uint32_t quant_code_fast2(__half2 x, const QuantGroup& g) { return quant_code_fast2(x, g, g); }
-
 // Codes of 32 values at a time.  The quotient is the correctly rounded fp32 one, as above, from 1/scale in two floats: d * lo is
 // far below half an ulp, so RN(d * hi + d * lo) is RN(d / scale) wherever d / scale keeps more than 2^-46 of it from a rounding
 // boundary, and the quotient of two 11-bit significands keeps 2^-36.  Two instructions for a pair of elements (f32x2)
 // instead of six; a group whose scale is 0, inf or NaN has all codes 0, by one mask for its words instead of a test per
-// element.  Pairs are gathered into bytes and the bytes into words, four elements at a time.
+// element.  Pairs are gathered into bytes and the bytes into words, four elements at a time.  NAN_IN: a NaN element may be in a
+// group whose scale is a number (where minimum and maximum are taken element by element); its code is 0.
 struct QuantPair {  // low half of a pair in one group, high half in another or the same
   __half2 mn;
   float2 rcp, lo;
@@ -138,7 +122,7 @@ __device__ __forceinline__ QuantPair quant_pair(__half mn0, __half sc0, __half m
 }
 __device__ __forceinline__ QuantPair quant_pair(__half mn, __half sc) { return quant_pair(mn, sc, mn, sc); }
 // the codes of a pair in bytes 0 and 2 (bytes 1 and 3 are not 0)
-template <int BITS>
+template <int BITS, bool NAN_IN>
 __device__ __forceinline__ uint32_t quant_pair_bytes(__half2 x, const QuantPair& g) {
   const float2 d = __half22float2(__hsub2(x, g.mn));
   float2 q;
@@ -146,7 +130,9 @@ __device__ __forceinline__ uint32_t quant_pair_bytes(__half2 x, const QuantPair&
       "fma.rn.f32x2 q, d, r, q;\nmov.b64 {%0, %1}, q;\n}"
       : "=f"(q.x), "=f"(q.y)
       : "f"(d.x), "f"(d.y), "f"(g.rcp.x), "f"(g.rcp.y), "f"(g.lo.x), "f"(g.lo.y));
-  __half2 u = __hmin2(__floats2half2_rn(q.x, q.y), __float2half2_rn(static_cast<float>((1 << BITS) - 1)));
+  __half2 u = __floats2half2_rn(q.x, q.y);
+  if (NAN_IN) u = __hmax2(u, __float2half2_rn(0.f));  // max(NaN, 0) == 0
+  u = __hmin2(u, __float2half2_rn(static_cast<float>((1 << BITS) - 1)));
   u = __hadd2(u, __float2half2_rn(1024.f));  // 1024 + rint(u): fp16 has unit spacing there, ties to even
   return *reinterpret_cast<uint32_t*>(&u);
 }
@@ -171,21 +157,21 @@ __device__ __forceinline__ void pack_bytes(const uint32_t* q, uint32_t keep, uin
   }
 }
 // 32 values of one group, in order: BITS words
-template <int BITS>
+template <int BITS, bool NAN_IN>
 __device__ __forceinline__ void quant_row32(const __half2 (&v)[16], const QuantPair& g, uint32_t* word) {
   uint32_t q[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) q[i] = __byte_perm(quant_pair_bytes<BITS>(v[2 * i], g), quant_pair_bytes<BITS>(v[2 * i + 1], g), 0x6420);
+  for (int i = 0; i < 8; ++i) q[i] = __byte_perm(quant_pair_bytes<BITS, NAN_IN>(v[2 * i], g), quant_pair_bytes<BITS, NAN_IN>(v[2 * i + 1], g), 0x6420);
   pack_bytes<BITS>(q, g.keep0, word);
 }
 // 32 pairs, low halves of one group and high halves of another: BITS words of each
-template <int BITS>
+template <int BITS, bool NAN_IN>
 __device__ __forceinline__ void quant_cols32(const __half2 (&v)[32], const QuantPair& g, uint32_t* word0, uint32_t* word1) {
   uint32_t q0[8], q1[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const uint32_t a = __byte_perm(quant_pair_bytes<BITS>(v[4 * i], g), quant_pair_bytes<BITS>(v[4 * i + 1], g), 0x6240);
-    const uint32_t b = __byte_perm(quant_pair_bytes<BITS>(v[4 * i + 2], g), quant_pair_bytes<BITS>(v[4 * i + 3], g), 0x6240);
+    const uint32_t a = __byte_perm(quant_pair_bytes<BITS, NAN_IN>(v[4 * i], g), quant_pair_bytes<BITS, NAN_IN>(v[4 * i + 1], g), 0x6240);
+    const uint32_t b = __byte_perm(quant_pair_bytes<BITS, NAN_IN>(v[4 * i + 2], g), quant_pair_bytes<BITS, NAN_IN>(v[4 * i + 3], g), 0x6240);
     q0[i] = __byte_perm(a, b, 0x5410);
     q1[i] = __byte_perm(a, b, 0x7632);
   }

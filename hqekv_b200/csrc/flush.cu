@@ -174,23 +174,6 @@ __device__ __forceinline__ void k_min_max(const __half2 (&v)[32], __half2& lo, _
   }
 }
 
-template <int BITS>
-__device__ __forceinline__ void k_quantise32(const __half2 (&v)[32], const QuantGroup& g0, const QuantGroup& g1, uint32_t* w0, uint32_t* w1) {
-  constexpr int FPI = 32 / BITS;
-#pragma unroll
-  for (int w = 0; w < BITS; ++w) {
-    uint32_t a = 0, b = 0;
-#pragma unroll
-    for (int i = 0; i < FPI; ++i) {
-      const uint32_t c = quant_code_fast2(v[w * FPI + i], g0, g1);
-      a |= (c & 0xFFFFu) << (i * BITS);
-      b |= (c >> 16) << (i * BITS);
-    }
-    w0[w] = a;
-    w1[w] = b;
-  }
-}
-
 // fp64 statistics of a group of the codebook tier in token order, channels ch and ch + 1: mean, std
 __device__ __noinline__ void k_normal_stats(const BuildArgs& A, int src, int64_t pos, int bh, int ch, __half2& mean, __half2& sd) {
   const int group = 1 << A.gshift;
@@ -362,8 +345,13 @@ __device__ __forceinline__ void k_build_tile(const BuildArgs& A, KBuildShared& s
       constexpr float levels = static_cast<float>((1 << BITS) - 1);
       auto finish = [&](const __half2(&v)[32], __half2 lo, __half2 hi, int i, int g) {
         const __half s0 = quant_scale(__low2half(lo), __low2half(hi), levels), s1 = quant_scale(__high2half(lo), __high2half(hi), levels);
-        k_quantise32<BITS>(v, quant_group(__low2half(lo), s0, levels), quant_group(__high2half(lo), s1, levels), w0 + i * KB::WPS,
-                           w1 + i * KB::WPS);
+        uint32_t a[BITS], b[BITS];
+        quant_cols32<BITS, true>(v, quant_pair(__low2half(lo), s0, __high2half(lo), s1), a, b);
+#pragma unroll
+        for (int w = 0; w < BITS; ++w) {
+          w0[i * KB::WPS + w] = a[w];
+          w1[i * KB::WPS + w] = b[w];
+        }
         sh.s[ch * KB_MAX_SUBS + g] = s0;
         sh.z[ch * KB_MAX_SUBS + g] = __low2half(lo);
         sh.s[(ch + 1) * KB_MAX_SUBS + g] = s1;
@@ -559,18 +547,7 @@ __device__ __forceinline__ void v_quantise32(const __half2 (&v)[16], int gshift,
     hi = __shfl_sync(0xffffffffu, h, first);
   }
   sc = quant_scale(lo, hi, levels);
-  const QuantGroup g = quant_group(lo, sc, levels);
-  constexpr int FPI = 32 / BITS;
-#pragma unroll
-  for (int w = 0; w < BITS; ++w) {
-    uint32_t word = 0;
-#pragma unroll
-    for (int i = 0; i < FPI / 2; ++i) {
-      const uint32_t c = quant_code_fast2(v[(w * FPI) / 2 + i], g);
-      word |= ((c & 0xFFFFu) | ((c >> 16) << BITS)) << (2 * i * BITS);
-    }
-    words[w] = word;
-  }
+  quant_row32<BITS, true>(v, quant_pair(lo, sc), words);
 }
 // Store a lane's quarter q of token `tok` (32 channels, 4 * BITS bytes) and, from the first lane of a group, its scale and
 // zero.  live: the lane has a token.

@@ -37,6 +37,7 @@ constexpr int HEAD_SUM_THREADS = 128;
 __global__ void __launch_bounds__(HEAD_SUM_THREADS) head_sum_kernel(const __half* __restrict__ w, int B, int nh, int64_t L,
                                                                     int64_t bh_stride, __half* __restrict__ out) {
   __shared__ float per_head[32][32];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t l = static_cast<int64_t>(blockIdx.x) * 32 + lane;
   const bool live = l < L;
@@ -533,9 +534,17 @@ extern "C" int hqkv_head_sum(const void* w, int B, int nh, int64_t L, int64_t bh
   HQKV_REQUIRE(B > 0 && nh > 0 && L >= 0 && bh_stride >= L, "head_sum: bad sizes");
   if (L == 0) return HQKV_OK;
   HQKV_REQUIRE(w && out, "head_sum: null pointer");
-  head_sum_kernel<<<static_cast<unsigned>(ceil_div(L, 32)), HEAD_SUM_THREADS, 0,
-                    static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __half*>(w), B, nh, L, bh_stride, static_cast<__half*>(out));
+  // may be placed while the V pass before it drains (the wait for it is the kernel's first instruction): 1-2 us a decode step
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(ceil_div(L, 32)));
+  cfg.blockDim = dim3(HEAD_SUM_THREADS);
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  HQKV_CUDA(cudaLaunchKernelEx(&cfg, head_sum_kernel, static_cast<const __half*>(w), B, nh, L, bh_stride, static_cast<__half*>(out)));
   HQKV_LAUNCH_CHECK("head_sum");
   return HQKV_OK;
 }
