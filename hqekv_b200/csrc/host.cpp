@@ -38,6 +38,7 @@ struct Lib {
   decltype(&hqkv_block_rank) block_rank;
   decltype(&hqkv_flush_workspace_bytes) flush_workspace_bytes;
   decltype(&hqkv_flush_prepare) flush_prepare;
+  decltype(&hqkv_flush_join) flush_join;
   decltype(&hqkv_flush_tiers) flush_tiers;
   decltype(&hqkv_flush_evict) flush_evict;
 } L;
@@ -65,10 +66,10 @@ inline void* ptr(const at::Tensor* t) { return t ? t->data_ptr() : nullptr; }
 PyObject* none() { Py_RETURN_NONE; }
 
 PyObject* bind(PyObject*, PyObject* args) {
-  unsigned long long a[12];
+  unsigned long long a[13];
   PyObject* fn;
-  if (!PyArg_ParseTuple(args, "KKKKKKKKKKKKO", &a[0], &a[1], &a[2], &a[3], &a[4], &a[5], &a[6], &a[7], &a[8], &a[9], &a[10],
-                        &a[11], &fn))
+  if (!PyArg_ParseTuple(args, "KKKKKKKKKKKKKO", &a[0], &a[1], &a[2], &a[3], &a[4], &a[5], &a[6], &a[7], &a[8], &a[9], &a[10],
+                        &a[11], &a[12], &fn))
     return nullptr;
   int i = 0;
   auto take = [&](auto& f) { f = reinterpret_cast<std::decay_t<decltype(f)>>(a[i++]); };
@@ -82,6 +83,7 @@ PyObject* bind(PyObject*, PyObject* args) {
   take(L.block_rank);
   take(L.flush_workspace_bytes);
   take(L.flush_prepare);
+  take(L.flush_join);
   take(L.flush_tiers);
   take(L.flush_evict);
   Py_INCREF(fn);
@@ -477,6 +479,18 @@ PyObject* flush(PyObject*, PyObject* const* a, Py_ssize_t na) {
   rc = L.flush_prepare(&f, ws.data_ptr(), static_cast<size_t>(ws.numel()), counts, st);
   Py_END_ALLOW_THREADS
   if (rc) return none();
+  struct Join {  // the V side runs on another stream: this one waits for it before the call's memory is let go
+    cudaStream_t st;
+    int32_t* counts;
+    bool done = false;
+    int now() {
+      done = true;
+      return L.flush_join(counts, st);
+    }
+    ~Join() {
+      if (!done) L.flush_join(nullptr, st);
+    }
+  } join{st, counts};
   for (int t = 0; t < HQKV_NUM_TIERS; ++t)
     if (counts[t] % f.block) return none();
   at::Tensor out[kSlots];
@@ -485,6 +499,12 @@ PyObject* flush(PyObject*, PyObject* const* a, Py_ssize_t na) {
     const int64_t group = side ? f.group : f.block;
     void *data[HQKV_NUM_TIERS] = {}, *scale[HQKV_NUM_TIERS] = {}, *zero[HQKV_NUM_TIERS] = {};
     int64_t* ids[HQKV_NUM_TIERS] = {};
+    if (side) {  // the K build has its work, the counts of V are needed now
+      Py_BEGIN_ALLOW_THREADS
+      rc = join.now();
+      Py_END_ALLOW_THREADS
+      if (rc) return none();
+    }
     for (int t = 0; t < HQKV_NUM_TIERS; ++t) {
       const int64_t n = counts[8 * side + t], bits = kBits[t];
       if (n == 0) continue;

@@ -302,7 +302,7 @@ struct PlanSide {
   int32_t* gcnt;       // [PLAN_CATS][PLAN_CLUSTER * PLAN_WARPS] per-warp category counts of the whole cluster
 };
 struct PlanArgs {
-  PlanSide side[2];    // one cluster each
+  PlanSide side;
   int64_t hist, compress;
 };
 
@@ -330,16 +330,16 @@ __device__ __forceinline__ void enum_slot(const PlanArgs& A, const PlanSide& S, 
   }
 }
 
-// One cluster of PLAN_CLUSTER CTAs of 32 warps per side.  Every pass walks the enumeration (or the token ids) in
+// One cluster of PLAN_CLUSTER CTAs of 32 warps.  Every pass walks the enumeration (or the token ids) in
 // warp-contiguous ranges - warp w of CTA r is range r * 32 + w - PLAN_BATCH iterations at a time so that the
 // dependent loads of a batch (index list -> target -> rank) are in flight together; ordered positions come from
 // per-warp counts (left in global memory for the other CTAs), one scan over all warps of the cluster, and ballot /
 // match prefixes inside a warp.  The passes are separated by cluster barriers, which also order the global-memory
 // scratch between the CTAs.  Categories: 2*t = kept member of tier t, 2*t + 1 = arrival in tier t (destination
 // order: kept members first, then arrivals, both in enumeration order); 10 = surviving token id.
-// What bounds it is the chain of dependent L2 round trips, two or three per pass: both sides in one launch, survival read
-// off the targets instead of a pass of its own, and the scan by one warp per category instead of 256 steps by one
-// thread took the two plans of a 32 k-token flush from 2 x 24.5 us to 17 us together.
+// What bounds it is the chain of dependent L2 round trips, two or three per pass: survival read off the targets instead
+// of a pass of its own, and the scan by one warp per category instead of 256 steps by one thread took the plan of a
+// 32 k-token flush from 24.5 us to 17 us.
 constexpr int PLAN_WARPS = PLAN_THREADS / 32;
 constexpr int PLAN_GWARPS = PLAN_WARPS * PLAN_CLUSTER;
 constexpr int PLAN_BATCH = 4;
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) flush_plan_kernel(const __grid_c
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ int cnt[PLAN_CATS + 1][PLAN_WARPS];  // per-warp totals, then their exclusive offsets over the cluster
   __shared__ int tot[PLAN_CATS];
-  const PlanSide& S = A.side[blockIdx.y];
+  const PlanSide& S = A.side;
   const int64_t total = A.hist + A.compress;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int crank = static_cast<int>(cluster.block_rank());
@@ -666,9 +666,9 @@ static int fill_plan_side(PlanSide& S, const int64_t* const* tier_idx_host, cons
   S.counts = counts;
   return HQKV_OK;
 }
-static int launch_plan(const PlanArgs& A, int sides, void* stream) {
+static int launch_plan(const PlanArgs& A, void* stream) {
   cudaLaunchAttribute attr[1];
-  const cudaLaunchConfig_t cfg = cluster_config(attr, PLAN_CLUSTER, sides, PLAN_THREADS, 0, stream);
+  const cudaLaunchConfig_t cfg = cluster_config(attr, PLAN_CLUSTER, 1, PLAN_THREADS, 0, stream);
   HQKV_CUDA(cudaLaunchKernelEx(&cfg, flush_plan_kernel, A));
   return HQKV_OK;
 }
@@ -687,13 +687,13 @@ extern "C" int hqkv_flush_plan(const int64_t* const* tier_idx_host, const int32_
   memset(&A, 0, sizeof(A));
   A.hist = hist;
   A.compress = compress;
-  int rc = fill_plan_side(A.side[0], tier_idx_host, tier_n_host, hist, total, sorted_ids, cum_counts_host, plan_src, plan_ids,
+  int rc = fill_plan_side(A.side, tier_idx_host, tier_n_host, hist, total, sorted_ids, cum_counts_host, plan_src, plan_ids,
                           survivors, counts, static_cast<unsigned char*>(workspace));
   if (rc) return rc;
   const size_t need = hqkv_flush_plan_workspace_bytes(total);
   if (workspace_bytes < need)
     return fail(HQKV_E_WORKSPACE, "flush_plan: workspace holds %zu bytes, %zu needed", workspace_bytes, need);
-  return launch_plan(A, 1, stream);
+  return launch_plan(A, stream);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -754,6 +754,62 @@ __global__ void __launch_bounds__(EVICT_THREADS) evict_kernel(__half* ring, int6
 }
 }  // namespace hqkv
 
+namespace hqkv {
+// What a thread keeps between its flushes: a second stream, two events, and 64 bytes of host memory that the plans write
+// the counts to - they are there as soon as the tokens are counted, while the plan still writes its lists, and no copy has
+// to be launched.  Made on first use, for one device at a time; given back when the thread ends.
+struct FlushLane {
+  int dev = -1;
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+  volatile int32_t* host = nullptr;
+  int32_t calls = 0;
+  int open() {
+    int now = 0;
+    HQKV_CUDA(cudaGetDevice(&now));
+    if (!host) {
+      void* p = nullptr;
+      HQKV_CUDA(cudaHostAlloc(&p, 64, cudaHostAllocPortable | cudaHostAllocMapped));
+      memset(p, 0, 64);
+      host = static_cast<volatile int32_t*>(p);
+    }
+    if (side && now == dev) return HQKV_OK;
+    close();
+    int least = 0, greatest = 0;  // ahead of the K build's CTAs: the V side's clusters need room on eight SMs at once
+    HQKV_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    HQKV_CUDA(cudaStreamCreateWithPriority(&side, cudaStreamNonBlocking, greatest));
+    HQKV_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    HQKV_CUDA(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+    dev = now;
+    return HQKV_OK;
+  }
+  void close() {
+    if (side) cudaStreamDestroy(side);
+    if (fork) cudaEventDestroy(fork);
+    if (join) cudaEventDestroy(join);
+    side = nullptr, fork = join = nullptr;
+  }
+  // waits for the counts of a side whose plan is in stream st
+  int counts(int v_side, cudaStream_t st, int32_t* out) {
+    const volatile int32_t* c = host + 8 * v_side;
+    for (int spins = 0; c[7] != calls; ++spins) {
+      if ((spins & 0xFFFF) != 0xFFFF) continue;
+      const cudaError_t e = cudaStreamQuery(st);  // an error of the stream ends the wait
+      if (e == cudaErrorNotReady) continue;
+      HQKV_CUDA(e);
+      HQKV_REQUIRE(c[7] == calls, "flush: the plan left no counts");
+    }
+    for (int i = 0; i < 8; ++i) out[i] = c[i];
+    return HQKV_OK;
+  }
+  ~FlushLane() {
+    close();
+    if (host) cudaFreeHost(const_cast<int32_t*>(host));
+  }
+};
+static thread_local FlushLane flush_lane;
+}  // namespace hqkv
+
 extern "C" size_t hqkv_flush_workspace_bytes(int64_t total) { return total < 0 ? 0 : flush_scratch(nullptr, total).bytes; }
 
 extern "C" int hqkv_flush_prepare(const hqkv_flush_t* f, void* workspace, size_t workspace_bytes, int32_t* counts_host, void* stream) {
@@ -772,57 +828,52 @@ extern "C" int hqkv_flush_prepare(const hqkv_flush_t* f, void* workspace, size_t
   HQKV_REQUIRE(aligned(f->v.residual, 16) && f->v.residual_b_stride % 8 == 0 && f->v.residual_h_stride % 8 == 0 &&
                    static_cast<int64_t>(f->B) * f->H <= RANGE_MAX_ROWS,
                "flush_prepare: the residual window must be 16-byte aligned, B*H at most %d", RANGE_MAX_ROWS);
-  PlanArgs A;
-  memset(&A, 0, sizeof(A));
-  A.hist = f->hist;
-  A.compress = f->compress;
+  PlanArgs A[2];
+  memset(A, 0, sizeof(A));
   for (int side = 0; side < 2; ++side) {
-    const int rc = fill_plan_side(A.side[side], side ? f->v_idx : f->k_idx, side ? f->v.n : f->k.n, f->hist, total,
+    A[side].hist = f->hist;
+    A[side].compress = f->compress;
+    const int rc = fill_plan_side(A[side].side, side ? f->v_idx : f->k_idx, side ? f->v.n : f->k.n, f->hist, total,
                                   side ? s.v_sorted : f->k_sorted, side ? f->v_cum : f->k_cum, s.plan_src[side], s.plan_ids[side],
                                   s.survivors[side], nullptr, s.plan_ws[side]);
     if (rc) return rc;
   }
-  // The counts come back through memory of the host that the plan writes (64 bytes per thread, kept until it ends): they are
-  // there as soon as the tokens are counted, while the plan still writes its lists, and no copy has to be launched.
-  struct Mapped {
-    volatile int32_t* host = nullptr;
-    int32_t calls = 0;
-    ~Mapped() {
-      if (host) cudaFreeHost(const_cast<int32_t*>(host));
-    }
-  };
-  static thread_local Mapped mapped;
-  if (!mapped.host) {
-    void* p = nullptr;
-    HQKV_CUDA(cudaHostAlloc(&p, 64, cudaHostAllocPortable | cudaHostAllocMapped));
-    memset(p, 0, 64);
-    mapped.host = static_cast<volatile int32_t*>(p);
-  }
+  FlushLane& lane = flush_lane;
+  int rc = lane.open();
+  if (rc) return rc;
   void* counts_dev = nullptr;
-  HQKV_CUDA(cudaHostGetDevicePointer(&counts_dev, const_cast<int32_t*>(mapped.host), 0));
-  mapped.calls = mapped.calls == 0x7FFFFFFF ? 1 : mapped.calls + 1;
+  HQKV_CUDA(cudaHostGetDevicePointer(&counts_dev, const_cast<int32_t*>(lane.host), 0));
+  lane.calls = lane.calls == 0x7FFFFFFF ? 1 : lane.calls + 1;
   for (int side = 0; side < 2; ++side) {
-    A.side[side].counts = static_cast<int32_t*>(counts_dev) + 8 * side;
-    A.side[side].done = mapped.calls;
+    A[side].side.counts = static_cast<int32_t*>(counts_dev) + 8 * side;
+    A[side].side.done = lane.calls;
   }
-  int rc = launch_range(f->v.residual, f->B, f->H, f->compress, f->v.residual_b_stride, f->v.residual_h_stride, f->norm_old, f->hist,
-                        f->norm_out, stream);
-  if (rc) return rc;
-  rc = launch_rank(f->importance, f->times_range ? f->norm_out : nullptr, s.v_keys, f->block, static_cast<int>(total / f->block), s.v_sorted,
-                   stream);
-  if (rc) return rc;
-  rc = launch_plan(A, 2, stream);
-  if (rc) return rc;
+  // ranges, ranking and plan of the V side beside the plan and the build of the K side, which need none of them
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  for (int spins = 0; mapped.host[7] != mapped.calls || mapped.host[15] != mapped.calls; ++spins) {
-    if ((spins & 0xFFFF) != 0xFFFF) continue;
-    const cudaError_t e = cudaStreamQuery(st);  // an error of the stream ends the wait
-    if (e == cudaErrorNotReady) continue;
-    HQKV_CUDA(e);
-    HQKV_REQUIRE(mapped.host[7] == mapped.calls && mapped.host[15] == mapped.calls, "flush_prepare: the plan left no counts");
+  HQKV_CUDA(cudaEventRecord(lane.fork, st));
+  HQKV_CUDA(cudaStreamWaitEvent(lane.side, lane.fork, 0));
+  rc = launch_plan(A[0], st);
+  if (!rc)
+    rc = launch_range(f->v.residual, f->B, f->H, f->compress, f->v.residual_b_stride, f->v.residual_h_stride, f->norm_old, f->hist,
+                      f->norm_out, lane.side);
+  if (!rc)
+    rc = launch_rank(f->importance, f->times_range ? f->norm_out : nullptr, s.v_keys, f->block, static_cast<int>(total / f->block),
+                     s.v_sorted, lane.side);
+  if (!rc) rc = launch_plan(A[1], lane.side);
+  const int rec = check_cuda(cudaEventRecord(lane.join, lane.side), "flush_prepare: event");
+  if (!rc && !rec) rc = lane.counts(0, st, counts_host);
+  if (rc || rec) {
+    cudaStreamWaitEvent(st, lane.join, 0);
+    return rc ? rc : rec;
   }
-  for (int i = 0; i < 16; ++i) counts_host[i] = mapped.host[i];
   return HQKV_OK;
+}
+
+extern "C" int hqkv_flush_join(int32_t* counts_host, void* stream) {
+  FlushLane& lane = flush_lane;
+  HQKV_REQUIRE(lane.side && lane.calls, "flush_join: this thread has prepared no flush");
+  HQKV_CUDA(cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), lane.join, 0));
+  return counts_host ? lane.counts(1, lane.side, counts_host + 8) : HQKV_OK;
 }
 
 extern "C" int hqkv_flush_tiers(const hqkv_flush_t* f, int v_side, const void* workspace, const int32_t* counts_host,

@@ -437,10 +437,13 @@ int hqkv_flush_build(int v_side, const hqkv_flush_src_t* src_host, int B, int H,
 
 /*
  * A whole flush (KV_cache_hqe_2, quant/hqe_2.py:456-843) in three calls, for hosts that keep launches and allocations few:
- *   hqkv_flush_prepare   value ranges of the flushed tokens appended to norm_old (-> norm_out, hist + compress fp16),
- *                        V ranking from `importance` (as ranked for K, i.e. divided by the block size; not modified) and,
- *                        with times_range, those ranges; the plans of both sides; waits for the counts
- *                        (counts_host[0..8) K, [8..16) V as in hqkv_flush_plan)
+ *   hqkv_flush_prepare   K plan; beside it, on a stream of the library: value ranges of the flushed tokens appended to
+ *                        norm_old (-> norm_out, hist + compress fp16), V ranking from `importance` (as ranked for K,
+ *                        i.e. divided by the block size; not modified) and, with times_range, those ranges, V plan;
+ *                        waits for the K counts (counts_host[0..8) as in hqkv_flush_plan)
+ *   hqkv_flush_join      `stream` waits for the V side, the host for its counts (counts_host[8..16); null: not wanted).
+ *                        Follows every successful hqkv_flush_prepare, in the same thread, before any memory of that
+ *                        call is used for something else; the K tiers may be built before it
  *   hqkv_flush_tiers     hqkv_flush_build of one side from that plan
  *   hqkv_flush_evict     compacts norm_out to the V-side survivors (-> norm_kept) and moves the survivors' columns of an
  *                        importance ring (fp16 [rows][stride], null: none) to the front, in place
@@ -461,6 +464,7 @@ typedef struct {
 size_t hqkv_flush_workspace_bytes(int64_t total);
 int hqkv_flush_prepare(const hqkv_flush_t* flush_host, void* workspace, size_t workspace_bytes, int32_t* counts_host,
                        void* stream);
+int hqkv_flush_join(int32_t* counts_host, void* stream);
 int hqkv_flush_tiers(const hqkv_flush_t* flush_host, int v_side, const void* workspace, const int32_t* counts_host,
                      void* const* out_data_host, void* const* out_scale_host, void* const* out_zero_host,
                      int64_t* const* out_ids_host, void* rest_out, void* stream);
