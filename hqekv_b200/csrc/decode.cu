@@ -1976,22 +1976,24 @@ struct Layout {
   size_t acc_off, logits_off, kpart_off, total;
 };
 
-// How the CTAs of a plane share its units.  A CTA pays for its prologue, the softmax pairs and the output reduction
-// whatever it walks - about as much as two units - and the last wave of CTAs should be full: of one to four waves the
-// number of CTAs that finishes first (counted in units of 4 bits).  Where one or two units per CTA make a wave, a second tier
-// would double a CTA's latency: there a CTA keeps to one tier (two units at 8 bits).
+// How the CTAs of a plane share its units.  A CTA pays about a unit for its prologue, the softmax pairs and the output
+// reduction whatever it walks, and runs about as fast beside three others on its SM as beside one (its chain of loads
+// bounds it): up to one wave the number of CTAs that are on the GPU does not count, only how long each is.  Beyond, the time
+// lies between the load of the SMs and that of whole waves (the last wave starts as the first CTAs end).  13 x 16 planes of
+// 15 units: 53 us with two CTAs each (0.7 of a wave), 50 with four; 30 x 8 planes of 15 units: 50 with two (0.8), 55 with
+// three (1.2).
+// Where one or two units per CTA make a wave, a second tier would double a CTA's latency: there a CTA keeps to one tier
+// (two units at 8 bits).
 static void divide(DecodeParams& P, int64_t planes, int slots, bool v) {
   int total = 0;  // cost of a plane
   for (const TierDev& t : P.tier) total += static_cast<int>(ceil_div(v ? t.n_v : t.n_k, unit_tokens(t.bits))) * unit_cost(t.bits);
-  const int units = static_cast<int>(ceil_div(total, unit_cost(4)));
-  int ctas = 0;
-  int64_t best = -1;
-  for (int waves = 1; units > 0 && waves <= 4; ++waves) {
-    int64_t n = static_cast<int64_t>(slots) * waves / planes;
-    n = n < 1 ? 1 : n > units ? units : n;
-    const int64_t share = ceil_div(units, n), whole = ceil_div(units, share), cost = ceil_div(whole * planes, slots) * (share + 2);
-    // all of the wave's CTAs where each gets two units or more (the SMs' loads differ least), else those that whole shares fill
-    if (best < 0 || cost < best) best = cost, ctas = static_cast<int>(total / n >= 2 * unit_cost(4) ? n : whole);
+  constexpr int UNIT = unit_cost(4);
+  int ctas = total > 0 ? 1 : 0;
+  double best = 0.;
+  for (int n = 1; n == 1 || (total / n >= 2 * UNIT && (n - 1) * planes < 4 * slots); ++n) {
+    const double waves = static_cast<double>(n * planes) / slots;
+    const double cost = (static_cast<double>(total) / n + UNIT) * (waves <= 1. ? 1. : 0.5 * (waves + ceil(waves)));
+    if (n == 1 || cost < best) best = cost, ctas = total > 0 ? n : 0;
   }
   int per = ctas ? total / ctas : 0, more = ctas ? total % ctas : 0;
   // the cost that a CTA of one tier may have: the smallest with which the planes' CTAs fit one wave
