@@ -1316,6 +1316,9 @@ __device__ __noinline__ void v_prepare_any(const DecodeParams& P, const Where& w
   }
 }
 
+// A position that the bounds-check build has turned down (never in the regular build).
+__device__ __forceinline__ bool turned_down(uint32_t pos) { return HQKV_CHECKS_ENABLED && pos == 0xFFFFFFFFu; }
+
 // The same for a whole tile, four or two query heads and 128 >> GV channel groups known at compile time.  mh / inv: max *
 // log2(e) and 1 / sum of the lane's heads, wrow: their rows of probabilities (null: no such heads).
 template <int BITS, int GV>
@@ -1355,6 +1358,9 @@ __device__ __forceinline__ void v_prepare(uint32_t tile, const float (&x)[4][VTi
   for (int h = 0; h < HPL; ++h) {
     __half *a = wrow[h] + pos[0], *b = wrow[h] + pos[2];
     if (wrow[h] == nullptr) {
+    } else if (turned_down(pos[0]) || turned_down(pos[1]) || turned_down(pos[2]) || turned_down(pos[3])) {
+      v_store_pair(wrow[h], pos[0], pos[1], n2[h][0], false);
+      v_store_pair(wrow[h], pos[2], pos[3], n2[h][1], false);
     } else if (adjacent && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 3) == 0) {
       *reinterpret_cast<uint32_t*>(a) = n2[h][0];
       *reinterpret_cast<uint32_t*>(b) = n2[h][1];
@@ -1388,11 +1394,18 @@ __device__ __forceinline__ void v_prepare(uint32_t tile, const float (&x)[4][VTi
   }
 }
 
-// Four or two query heads: logits of the lane's tokens without conditions (position 0 stands in beyond the tier).
+// Four or two query heads: logits of the lane's tokens without conditions (position 0 stands in beyond the tier).  The
+// bounds-check build leaves out positions that are not below `limit`: no logit, and no probability is stored for them.
 template <int HPL>
-__device__ __forceinline__ void v_gather4(float (&x)[4][HPL], const uint32_t (&pos)[4], const float* base, uint32_t heads) {
+__device__ __forceinline__ void v_gather4(float (&x)[4][HPL], uint32_t (&pos)[4], const float* base, uint32_t heads, int limit) {
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
+    if (!HQKV_INDEX_OK(pos[j], limit)) {
+      pos[j] = 0xFFFFFFFFu;
+#pragma unroll
+      for (int h = 0; h < HPL; ++h) x[j][h] = -INFINITY;
+      continue;
+    }
     const float* p = base + static_cast<uint64_t>(pos[j]) * heads;
     if constexpr (HPL == 2) {
       const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
@@ -1557,7 +1570,7 @@ __device__ __forceinline__ void v_run(const DecodeParams& P, const TierDev& T, V
   // With two query heads the lanes of the other two take the first two's logits to a probability of 0 and write none.
   const float* lrow = P.logits + static_cast<int64_t>(w.bvh) * P.L * P.r4 + (L.h0 & (P.r4 - 1));
   auto gather = [&]() {
-    if constexpr (FAST) v_gather4<TL::HPL>(x, pos, lrow, static_cast<uint32_t>(P.r4));
+    if constexpr (FAST) v_gather4<TL::HPL>(x, pos, lrow, static_cast<uint32_t>(P.r4), P.L);
     else v_gather<TL::HPL>(P, w, x, pos, L.h0);
   };
   gather();
@@ -2284,7 +2297,7 @@ static int hqkv::decode_launch(const hqkv_cache_desc_t* cache_host, const void* 
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const bool fast = P.r4 >= 2 && !P.probs_in && !HQKV_CHECKS_ENABLED;
+    const bool fast = P.r4 >= 2 && !P.probs_in;
     HQKV_CUDA(cudaLaunchKernelEx(&cfg, v_kernels[P.v_more < 0][fast ? P.gv_shift - 4 : 0], P));
   }
   return HQKV_OK;
