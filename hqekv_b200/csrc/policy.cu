@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(RANGE_THREADS) token_range128_kernel(const __h
                                                                        int64_t b_stride, int64_t h_stride, int tshift,
                                                                        const __half* __restrict__ old, int64_t n_old, int ctas,
                                                                        __half* __restrict__ out) {
-  extern __shared__ uint32_t row_at[];  // [row = h * B + b] first element / 8, then the ranges [token][row]
+  extern __shared__ int64_t row_at[];  // [row = h * B + b] first element, then the ranges [token][row]
   __half* range_s = reinterpret_cast<__half*>(row_at + n);
   const int tid = threadIdx.x;
   if (static_cast<int>(blockIdx.x) >= ctas) {
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(RANGE_THREADS) token_range128_kernel(const __h
       if (base + j * RANGE_THREADS < n_old) out[base + j * RANGE_THREADS] = old[base + j * RANGE_THREADS];
     return;
   }
-  for (int r = tid; r < n; r += RANGE_THREADS) row_at[r] = static_cast<uint32_t>(((r % B) * b_stride + (r / B) * h_stride) >> 3);
+  for (int r = tid; r < n; r += RANGE_THREADS) row_at[r] = (r % B) * b_stride + (r / B) * h_stride;
   __syncthreads();
   const int hw = tid >> 4, l16 = tid & 15, tpc = 1 << tshift;
   const int64_t t0 = static_cast<int64_t>(blockIdx.x) << tshift;
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(RANGE_THREADS) token_range128_kernel(const __h
     for (int u = 0; u < 4; ++u) {
       const int it = min(base + u * (RANGE_THREADS / 16), items - 1);
       const int64_t t = min(t0 + (it & (tpc - 1)), T - 1);
-      w[u] = reinterpret_cast<const uint4*>(v)[row_at[it >> tshift] + t * 16 + l16];
+      w[u] = *reinterpret_cast<const uint4*>(v + row_at[it >> tshift] + t * D + 8 * l16);
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -564,12 +564,13 @@ extern "C" int hqkv_token_importance(const void* ring, int rows, int64_t ring_st
 // Ranges of T tokens behind the n_old that are copied.
 static int launch_range(const void* v, int B, int H, int64_t T, int64_t b_stride, int64_t h_stride, const void* old, int64_t n_old,
                         void* out, void* stream) {
-  // tokens per CTA: one until every SM has four CTAs, then up to sixteen (32 KB of ranges at most)
+  // tokens per CTA: one until every SM has four CTAs, then up to sixteen, of 4096 rows between
+  // them (with RANGE_MAX_ROWS rows to a token: 32 KB of row offsets and 8 KB of ranges)
   const int n = B * H;
   int tshift = 0;
-  while (tshift < 4 && T >> (tshift + 1) >= 4 * 148 && (static_cast<int64_t>(n) << (tshift + 2)) <= 2 * RANGE_MAX_ROWS) ++tshift;
+  while (tshift < 4 && T >> (tshift + 1) >= 4 * 148 && (static_cast<int64_t>(n) << (tshift + 1)) <= RANGE_MAX_ROWS) ++tshift;
   const int64_t ctas = ceil_div(T, 1 << tshift), copies = ceil_div(n_old, 8 * RANGE_THREADS);
-  token_range128_kernel<<<static_cast<unsigned>(ctas + copies), RANGE_THREADS, n * sizeof(uint32_t) + (static_cast<size_t>(n) << tshift) * sizeof(__half),
+  token_range128_kernel<<<static_cast<unsigned>(ctas + copies), RANGE_THREADS, n * sizeof(int64_t) + (static_cast<size_t>(n) << tshift) * sizeof(__half),
                           static_cast<cudaStream_t>(stream)>>>(static_cast<const __half*>(v), B, n, T, b_stride, h_stride, tshift,
                                                                static_cast<const __half*>(old), n_old, static_cast<int>(ctas),
                                                                static_cast<__half*>(out));
