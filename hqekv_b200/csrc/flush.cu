@@ -5,6 +5,8 @@
 // HBM-bound copying and quantising: what matters is that loads are wide, coalesced and many at a time.
 #include <string.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace hqkv {
@@ -29,7 +31,8 @@ struct BuildArgs {
   int32_t n[HQKV_NUM_TIERS];
   const __half* residual;
   int64_t res_b_stride, res_h_stride;
-  int wide;             // the residual's rows may be read 16 bytes at a time
+  int wide;             // the residual's rows may be read, and what stays of it stored, 16 bytes at a time
+  int tiers_wide;       // picks WIDE, see below (read by the host)
   int H, gshift;
   int normal_low;       // the 1-bit destination is written in the Gaussian-codebook codec
   BuildDst dst[HQKV_NUM_TIERS];
@@ -38,6 +41,14 @@ struct BuildArgs {
   __half* rest_out;
   int64_t rest_n;       // halfs per (batch, head)
 };
+
+// WIDE: sources and outputs lie where the widest accesses want them - codes on 16-byte boundaries, scales and zeros on 8-byte
+// ones - and K tiers hold whole runs of 32 tokens.  Else everything goes by the tensors' own types (views into larger
+// buffers may start anywhere): the same kernels, with words and halfs in the place of the wide pieces.
+template <bool WIDE>
+__device__ __forceinline__ uint2 load_words(const uint32_t* p) {
+  return WIDE ? *reinterpret_cast<const uint2*>(p) : make_uint2(p[0], p[1]);
+}
 
 __device__ __forceinline__ __half2 as_h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
 __device__ __forceinline__ uint32_t as_u32(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
@@ -95,6 +106,7 @@ struct KBuildShared {
 };
 
 // 32 values of channels ch, ch + 1 from source tier `src` at pos: v[t] = (ch, ch + 1) of token pos + t
+template <bool WIDE>
 __device__ __forceinline__ void k_load32(const BuildArgs& A, int src, int64_t pos, int bh, int ch, __half2 (&v)[32]) {
   if (src < 0) {
     const int b = bh / A.H, h = bh - b * A.H;
@@ -118,11 +130,11 @@ __device__ __forceinline__ void k_load32(const BuildArgs& A, int src, int64_t po
   const int64_t G = n >> A.gshift, gi = row * G + (pos >> A.gshift);
   const __half2 sc = __halves2half2(A.scale[src][gi], A.scale[src][gi + G]), ze = __halves2half2(A.zero[src][gi], A.zero[src][gi + G]);
   if (src == 1) {
-    const uint2 *p = reinterpret_cast<const uint2*>(reinterpret_cast<const unsigned char*>(A.data[1]) + row * n + pos);
-    const uint2 *q = reinterpret_cast<const uint2*>(reinterpret_cast<const unsigned char*>(p) + n);
+    const uint32_t *p = reinterpret_cast<const uint32_t*>(reinterpret_cast<const unsigned char*>(A.data[1]) + row * n + pos);
+    const uint32_t *q = reinterpret_cast<const uint32_t*>(reinterpret_cast<const unsigned char*>(p) + n);
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
-      const uint2 a = p[w], b = q[w];
+      const uint2 a = load_words<WIDE>(p + 2 * w), b = load_words<WIDE>(q + 2 * w);
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         const uint32_t x = k ? a.y : a.x, y = k ? b.y : b.x;
@@ -131,11 +143,11 @@ __device__ __forceinline__ void k_load32(const BuildArgs& A, int src, int64_t po
       }
     }
   } else if (src == 2) {
-    const uint2 *p = reinterpret_cast<const uint2*>(reinterpret_cast<const unsigned char*>(A.data[2]) + row * (n / 2) + pos / 2);
-    const uint2 *q = reinterpret_cast<const uint2*>(reinterpret_cast<const unsigned char*>(p) + n / 2);
+    const uint32_t *p = reinterpret_cast<const uint32_t*>(reinterpret_cast<const unsigned char*>(A.data[2]) + row * (n / 2) + pos / 2);
+    const uint32_t *q = reinterpret_cast<const uint32_t*>(reinterpret_cast<const unsigned char*>(p) + n / 2);
 #pragma unroll
     for (int w = 0; w < 2; ++w) {
-      const uint2 a = p[w], b = q[w];
+      const uint2 a = load_words<WIDE>(p + 2 * w), b = load_words<WIDE>(q + 2 * w);
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         const uint32_t x = k ? a.y : a.x, y = k ? b.y : b.x;
@@ -177,13 +189,14 @@ __device__ __forceinline__ void k_min_max(const __half2 (&v)[32], __half2& lo, _
 }
 
 // fp64 statistics of a group of the codebook tier in token order, channels ch and ch + 1: mean, std
+template <bool WIDE>
 __device__ __noinline__ void k_normal_stats(const BuildArgs& A, int src, int64_t pos, int bh, int ch, __half2& mean, __half2& sd) {
   const int group = 1 << A.gshift;
   const double share = static_cast<double>(1.f / static_cast<float>(group));  // (exact: a power of two)
   double s0 = 0.0, s1 = 0.0, q0 = 0.0, q1 = 0.0;
   __half2 v[32];
   for (int i = 0; i < group; i += 32) {
-    k_load32(A, src, pos + i, bh, ch, v);
+    k_load32<WIDE>(A, src, pos + i, bh, ch, v);
 #pragma unroll
     for (int t = 0; t < 32; ++t) {
       s0 += static_cast<double>(__low2float(v[t]));
@@ -192,7 +205,7 @@ __device__ __noinline__ void k_normal_stats(const BuildArgs& A, int src, int64_t
   }
   const double m0 = s0 * share, m1 = s1 * share;
   for (int i = 0; i < group; i += 32) {
-    if (group > 32) k_load32(A, src, pos + i, bh, ch, v);
+    if (group > 32) k_load32<WIDE>(A, src, pos + i, bh, ch, v);
 #pragma unroll
     for (int t = 0; t < 32; ++t) {
       const double a = static_cast<double>(__low2float(v[t])) - m0, b = static_cast<double>(__high2float(v[t])) - m1;
@@ -205,13 +218,14 @@ __device__ __noinline__ void k_normal_stats(const BuildArgs& A, int src, int64_t
 }
 
 // One arrival group of the codebook tier, channels ch and ch + 1.
+template <bool WIDE>
 __device__ __noinline__ void k_normal_group(const BuildArgs& A, KBuildShared& sh, int bh, int g, int ch) {
   const int per = 1 << (A.gshift - 5), s0 = g * per, group = 1 << A.gshift, src = sh.src[s0];
   const int64_t pos = sh.pos[s0];
   __half2 v[32];
   float s[2][2] = {}, c[2][2] = {}, ss[2][4] = {};
   for (int i = 0; i < per; ++i) {
-    k_load32(A, src, pos + 32 * i, bh, ch, v);
+    k_load32<WIDE>(A, src, pos + 32 * i, bh, ch, v);
 #pragma unroll
     for (int t = 0; t < 32; ++t) {
       add_compensated(s[0][t & 1], c[0][t & 1], __low2float(v[t]));
@@ -226,7 +240,7 @@ __device__ __noinline__ void k_normal_group(const BuildArgs& A, KBuildShared& sh
     m[k] = (s[k][0] + c[k][0]) * (1.f / static_cast<float>(group));
   }
   for (int i = 0; i < per; ++i) {
-    if (per > 1) k_load32(A, src, pos + 32 * i, bh, ch, v);
+    if (per > 1) k_load32<WIDE>(A, src, pos + 32 * i, bh, ch, v);
 #pragma unroll
     for (int t = 0; t < 32; ++t) {
       const float a = __low2float(v[t]) - m[0], b = __high2float(v[t]) - m[1];
@@ -240,10 +254,10 @@ __device__ __noinline__ void k_normal_group(const BuildArgs& A, KBuildShared& sh
   for (int k = 0; k < 2; ++k)
     sure &= normal1_fast(s[k][0], c[k][0], (ss[k][0] + ss[k][1]) + (ss[k][2] + ss[k][3]), group, mean[k], sd[k]);
   __half2 mean2 = __halves2half2(mean[0], mean[1]), sd2 = __halves2half2(sd[0], sd[1]);
-  if (!sure) k_normal_stats(A, src, pos, bh, ch, mean2, sd2);
+  if (!sure) k_normal_stats<WIDE>(A, src, pos, bh, ch, mean2, sd2);
   const __half2 bound = __halves2half2(normal1_bound(__low2half(sd2)), normal1_bound(__high2half(sd2)));
   for (int i = 0; i < per; ++i) {
-    if (per > 1) k_load32(A, src, pos + 32 * i, bh, ch, v);
+    if (per > 1) k_load32<WIDE>(A, src, pos + 32 * i, bh, ch, v);
     uint32_t a = 0, b = 0;
 #pragma unroll
     for (int t = 0; t < 32; ++t) {
@@ -275,7 +289,43 @@ struct PieceType<4> {
   using type = uint32_t;
 };
 
-template <int BITS>
+// a piece of a row of codes (fp16 values at 16 bits)
+template <int BITS, bool WIDE, typename Piece>
+__device__ __forceinline__ Piece load_piece(const unsigned char* p) {
+  if constexpr (WIDE) return *reinterpret_cast<const Piece*>(p);
+  Piece v;
+  uint32_t* u = reinterpret_cast<uint32_t*>(&v);
+#pragma unroll
+  for (int i = 0; i < static_cast<int>(sizeof(Piece) / 4); ++i) {
+    if constexpr (BITS == 16) {
+      const __half* h = reinterpret_cast<const __half*>(p) + 2 * i;
+      u[i] = as_u32(__halves2half2(h[0], h[1]));
+    } else {
+      u[i] = reinterpret_cast<const uint32_t*>(p)[i];
+    }
+  }
+  return v;
+}
+template <int BITS, bool WIDE, typename Piece>
+__device__ __forceinline__ void store_piece(unsigned char* p, const Piece& v) {
+  if constexpr (WIDE) {
+    *reinterpret_cast<Piece*>(p) = v;
+    return;
+  }
+  const uint32_t* u = reinterpret_cast<const uint32_t*>(&v);
+#pragma unroll
+  for (int i = 0; i < static_cast<int>(sizeof(Piece) / 4); ++i) {
+    if constexpr (BITS == 16) {
+      __half* h = reinterpret_cast<__half*>(p) + 2 * i;
+      h[0] = __low2half(as_h2(u[i]));
+      h[1] = __high2half(as_h2(u[i]));
+    } else {
+      reinterpret_cast<uint32_t*>(p)[i] = u[i];
+    }
+  }
+}
+
+template <int BITS, bool WIDE>
 __device__ __forceinline__ void k_build_tile(const BuildArgs& A, KBuildShared& sh, int t, int tile, int bh) {
   using KB = KBuild<BITS>;
   using Piece = typename PieceType<KB::PIECE>::type;
@@ -319,9 +369,9 @@ __device__ __forceinline__ void k_build_tile(const BuildArgs& A, KBuildShared& s
     in += r0 * in_row;
     Piece v[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const Piece*>(in + 32 * i * in_row);
+    for (int i = 0; i < 4; ++i) v[i] = load_piece<BITS, WIDE, Piece>(in + 32 * i * in_row);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) *reinterpret_cast<Piece*>(out + 32 * i * out_row) = v[i];
+    for (int i = 0; i < 4; ++i) store_piece<BITS, WIDE>(out + 32 * i * out_row, v[i]);
   }
   bool arrivals = false;
 #pragma unroll
@@ -333,7 +383,7 @@ __device__ __forceinline__ void k_build_tile(const BuildArgs& A, KBuildShared& s
       for (int i = set; i < nsub; i += 4) {
         if (sh.src[i] == t) continue;
         __half2 v[32];
-        k_load32(A, sh.src[i], sh.pos[i], bh, ch, v);
+        k_load32<WIDE>(A, sh.src[i], sh.pos[i], bh, ch, v);
 #pragma unroll
         for (int k = 0; k < 16; ++k) {
           w0[16 * i + k] = lo16(as_u32(v[2 * k]), as_u32(v[2 * k + 1]));
@@ -342,7 +392,7 @@ __device__ __forceinline__ void k_build_tile(const BuildArgs& A, KBuildShared& s
       }
     } else if (BITS == 1 && A.normal_low) {
       for (int g = set; g < (nsub << 5) >> A.gshift; g += 4)
-        if (sh.src[g << (A.gshift - 5)] != t) k_normal_group(A, sh, bh, g, ch);
+        if (sh.src[g << (A.gshift - 5)] != t) k_normal_group<WIDE>(A, sh, bh, g, ch);
     } else {
       constexpr float levels = static_cast<float>((1 << BITS) - 1);
       auto finish = [&](const __half2(&v)[32], __half2 lo, __half2 hi, int i, int g) {
@@ -363,7 +413,7 @@ __device__ __forceinline__ void k_build_tile(const BuildArgs& A, KBuildShared& s
         for (int i = set; i < nsub; i += 4) {
           if (sh.src[i] == t) continue;
           __half2 v[32], lo, hi;
-          k_load32(A, sh.src[i], sh.pos[i], bh, ch, v);
+          k_load32<WIDE>(A, sh.src[i], sh.pos[i], bh, ch, v);
           k_min_max(v, lo, hi);
           finish(v, lo, hi, i, i);
         }
@@ -371,7 +421,7 @@ __device__ __forceinline__ void k_build_tile(const BuildArgs& A, KBuildShared& s
         for (int i = set; i < nsub; i += 4) {
           if (sh.src[i] == t) continue;
           __half2 v[32], lo, hi;
-          k_load32(A, sh.src[i], sh.pos[i], bh, ch, v);
+          k_load32<WIDE>(A, sh.src[i], sh.pos[i], bh, ch, v);
           k_min_max(v, lo, hi);
           sh.lo[ch * KB_MAX_SUBS + i] = __low2half(lo);
           sh.lo[(ch + 1) * KB_MAX_SUBS + i] = __high2half(lo);
@@ -394,7 +444,7 @@ __device__ __forceinline__ void k_build_tile(const BuildArgs& A, KBuildShared& s
             }
           }
           __half2 v[32];
-          k_load32(A, sh.src[i], sh.pos[i], bh, ch, v);
+          k_load32<WIDE>(A, sh.src[i], sh.pos[i], bh, ch, v);
           finish(v, __halves2half2(l[0], l[1]), __halves2half2(h[0], h[1]), i, i >> (A.gshift - 5));
         }
       }
@@ -409,7 +459,7 @@ __device__ __forceinline__ void k_build_tile(const BuildArgs& A, KBuildShared& s
         uint32_t* u = reinterpret_cast<uint32_t*>(&v);
 #pragma unroll
         for (int k = 0; k < W; ++k) u[k] = w[k];
-        *reinterpret_cast<Piece*>(out + 32 * i * out_row) = v;
+        store_piece<BITS, WIDE>(out + 32 * i * out_row, v);
       }
     }
   }
@@ -427,6 +477,7 @@ __device__ __forceinline__ void k_build_tile(const BuildArgs& A, KBuildShared& s
   }
 }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(BUILD_THREADS, 4) flush_build_k_kernel(const __grid_constant__ BuildArgs A) {
   __shared__ KBuildShared sh;
   // From the back: arrivals, which take longer than copies, are at the end of a tier's list, and the lowest tier's longest.
@@ -435,11 +486,11 @@ __global__ void __launch_bounds__(BUILD_THREADS, 4) flush_build_k_kernel(const _
     copy_rest(A, bh);
     return;
   }
-  if (x >= A.dst[4].tile0) k_build_tile<1>(A, sh, 4, x - A.dst[4].tile0, bh);
-  else if (x >= A.dst[3].tile0) k_build_tile<2>(A, sh, 3, x - A.dst[3].tile0, bh);
-  else if (x >= A.dst[2].tile0) k_build_tile<4>(A, sh, 2, x - A.dst[2].tile0, bh);
-  else if (x >= A.dst[1].tile0) k_build_tile<8>(A, sh, 1, x - A.dst[1].tile0, bh);
-  else k_build_tile<16>(A, sh, 0, x, bh);
+  if (x >= A.dst[4].tile0) k_build_tile<1, WIDE>(A, sh, 4, x - A.dst[4].tile0, bh);
+  else if (x >= A.dst[3].tile0) k_build_tile<2, WIDE>(A, sh, 3, x - A.dst[3].tile0, bh);
+  else if (x >= A.dst[2].tile0) k_build_tile<4, WIDE>(A, sh, 2, x - A.dst[2].tile0, bh);
+  else if (x >= A.dst[1].tile0) k_build_tile<8, WIDE>(A, sh, 1, x - A.dst[1].tile0, bh);
+  else k_build_tile<16, WIDE>(A, sh, 0, x, bh);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -553,11 +604,15 @@ __device__ __forceinline__ void v_quantise32(const __half2 (&v)[16], int gshift,
 }
 // Store a lane's quarter q of token `tok` (32 channels, 4 * BITS bytes) and, from the first lane of a group, its scale and
 // zero.  live: the lane has a token.
-template <int BITS>
+template <int BITS, bool WIDE>
 __device__ __forceinline__ void v_store32(const BuildArgs& A, const BuildDst& dst, int64_t tok, int q, const __half2 (&v)[16], bool live) {
   uint32_t* row = reinterpret_cast<uint32_t*>(dst.data) + tok * (4 * BITS) + q * BITS;
   if constexpr (BITS == 16) {
-    if (live) {
+    if (live && !WIDE) {
+      __half* out = static_cast<__half*>(dst.data) + tok * D + 32 * q;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) out[2 * i] = __low2half(v[i]), out[2 * i + 1] = __high2half(v[i]);
+    } else if (live) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         reinterpret_cast<uint4*>(row)[i] = make_uint4(as_u32(v[4 * i]), as_u32(v[4 * i + 1]), as_u32(v[4 * i + 2]), as_u32(v[4 * i + 3]));
@@ -567,7 +622,10 @@ __device__ __forceinline__ void v_store32(const BuildArgs& A, const BuildDst& ds
     uint32_t w[BITS];
     v_quantise32<BITS>(v, A.gshift, A.normal_low != 0, w, sc, lo);
     if (!live) return;
-    if constexpr (BITS == 8) {
+    if constexpr (!WIDE) {
+#pragma unroll
+      for (int i = 0; i < BITS; ++i) row[i] = w[i];
+    } else if constexpr (BITS == 8) {
       reinterpret_cast<uint4*>(row)[0] = make_uint4(w[0], w[1], w[2], w[3]);
       reinterpret_cast<uint4*>(row)[1] = make_uint4(w[4], w[5], w[6], w[7]);
     } else if constexpr (BITS == 4) {
@@ -637,12 +695,12 @@ __device__ __forceinline__ void v_arrive(const BuildArgs& A, const BuildDst& dst
     __half2 v[16];
     v_unit_values<SB>(u, v);
     if (s + 8 < 32) v_unit_load<SB>(A, u, rows + (s + 8 + row) * (16 * SB), src, tok + s + 8 + row, q);
-    v_store32<BITS>(A, dst, out_tok + s + row, q, v, true);
+    v_store32<BITS, true>(A, dst, out_tok + s + row, q, v, true);
   }
 }
 
 // One token from any source, by the first four lanes of the warp.
-template <int BITS>
+template <int BITS, bool WIDE>
 __device__ __noinline__ void v_one_token(const BuildArgs& A, int t, int32_t enc, int64_t j, int bh) {
   const BuildDst& dst = A.dst[t];
   const int lane = threadIdx.x & 31, q = lane & 3, ng = D >> A.gshift;
@@ -650,8 +708,9 @@ __device__ __noinline__ void v_one_token(const BuildArgs& A, int t, int32_t enc,
   const int64_t pos = enc & 0x0FFFFFFF, out_tok = static_cast<int64_t>(bh) * dst.n + j;
   if (src == t) {  // kept: copy the row verbatim
     const int64_t tok = static_cast<int64_t>(bh) * A.n[t] + pos;
-    for (int w = lane; w < 4 * BITS; w += 32)
-      reinterpret_cast<uint32_t*>(dst.data)[out_tok * (4 * BITS) + w] = reinterpret_cast<const uint32_t*>(A.data[t])[tok * (4 * BITS) + w];
+    using Item = typename std::conditional<BITS == 16 && !WIDE, __half, uint32_t>::type;
+    constexpr int N = 16 * BITS / sizeof(Item);  // per row
+    for (int w = lane; w < N; w += 32) static_cast<Item*>(dst.data)[out_tok * N + w] = static_cast<const Item*>(A.data[t])[tok * N + w];
     if (BITS < 16 && lane < ng) {
       dst.scale[out_tok * ng + lane] = A.scale[t][tok * ng + lane];
       dst.zero[out_tok * ng + lane] = A.zero[t][tok * ng + lane];
@@ -674,10 +733,10 @@ __device__ __noinline__ void v_one_token(const BuildArgs& A, int t, int32_t enc,
     for (int i = 0; i < 16; ++i)
       v[i] = __halves2half2(h_add(h_mul(v_get(w, sb, 32 * q + 2 * i), sc), ze), h_add(h_mul(v_get(w, sb, 32 * q + 2 * i + 1), sc), ze));
   }
-  v_store32<BITS>(A, dst, out_tok, q, v, lane < 4);
+  v_store32<BITS, WIDE>(A, dst, out_tok, q, v, lane < 4);
 }
 
-template <int BITS>
+template <int BITS, bool WIDE>
 __device__ __forceinline__ void v_build_run(const BuildArgs& A, int t, int64_t run, int bh) {
   const BuildDst& dst = A.dst[t];
   const int lane = threadIdx.x & 31;
@@ -689,8 +748,8 @@ __device__ __forceinline__ void v_build_run(const BuildArgs& A, int t, int64_t r
     if (bh == 0 && dst.ids_out) dst.ids_out[j0 + lane] = dst.ids[j0 + lane];
   }
   const int32_t enc0 = __shfl_sync(0xffffffffu, enc, 0);
-  if (ntok < 32 || !__all_sync(0xffffffffu, enc == enc0 + lane) || !A.wide) {
-    for (int i = 0; i < ntok; ++i) v_one_token<BITS>(A, t, __shfl_sync(0xffffffffu, enc, i), j0 + i, bh);
+  if (!WIDE || ntok < 32 || !__all_sync(0xffffffffu, enc == enc0 + lane) || !A.wide) {
+    for (int i = 0; i < ntok; ++i) v_one_token<BITS, WIDE>(A, t, __shfl_sync(0xffffffffu, enc, i), j0 + i, bh);
     return;
   }
   const int src = (enc0 >> 28) - 1;
@@ -739,10 +798,11 @@ __device__ __forceinline__ void v_build_run(const BuildArgs& A, int t, int64_t r
   else if (BITS < 4 && sb == 4) v_arrive<BITS, 4>(A, dst, rows, src, tok, out_tok);
   else if (BITS < 2 && sb == 2) v_arrive<BITS, 2>(A, dst, rows, src, tok, out_tok);
   else
-    for (int i = 0; i < 32; ++i) v_one_token<BITS>(A, t, enc0 + i, j0 + i, bh);  // (not to wider tiers; all the same)
+    for (int i = 0; i < 32; ++i) v_one_token<BITS, WIDE>(A, t, enc0 + i, j0 + i, bh);  // (not to wider tiers; all the same)
 }
 
 constexpr int VB_WARPS = BUILD_THREADS / 32;
+template <bool WIDE>
 __global__ void __launch_bounds__(BUILD_THREADS, 4) flush_build_v_kernel(const __grid_constant__ BuildArgs A) {
   const int x = A.tiles - 1 - static_cast<int>(blockIdx.x), bh = blockIdx.y;  // from the back, as above
   if (x < 0) {
@@ -752,17 +812,17 @@ __global__ void __launch_bounds__(BUILD_THREADS, 4) flush_build_v_kernel(const _
   const int t = x >= A.dst[4].tile0 ? 4 : x >= A.dst[3].tile0 ? 3 : x >= A.dst[2].tile0 ? 2 : x >= A.dst[1].tile0 ? 1 : 0;
   const int64_t run = static_cast<int64_t>(x - A.dst[t].tile0) * VB_WARPS + (threadIdx.x >> 5);
   if (run * 32 >= A.dst[t].n) return;
-  if (t == 4) v_build_run<1>(A, 4, run, bh);
-  else if (t == 3) v_build_run<2>(A, 3, run, bh);
-  else if (t == 2) v_build_run<4>(A, 2, run, bh);
-  else if (t == 1) v_build_run<8>(A, 1, run, bh);
-  else v_build_run<16>(A, 0, run, bh);
+  if (t == 4) v_build_run<1, WIDE>(A, 4, run, bh);
+  else if (t == 3) v_build_run<2, WIDE>(A, 3, run, bh);
+  else if (t == 2) v_build_run<4, WIDE>(A, 2, run, bh);
+  else if (t == 1) v_build_run<8, WIDE>(A, 1, run, bh);
+  else v_build_run<16, WIDE>(A, 0, run, bh);
 }
 
 // ------------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------------
-static int fill_build_args(BuildArgs& A, const hqkv_flush_src_t* src, int B, int H, int Dd, int group, const char* who) {
+static int fill_build_args(BuildArgs& A, bool v_side, const hqkv_flush_src_t* src, int B, int H, int Dd, int group, const char* who) {
   HQKV_REQUIRE(src != nullptr, "%s: null source descriptor", who);
   HQKV_REQUIRE(Dd == D, "%s: head dim must be 128", who);
   HQKV_REQUIRE(B > 0 && H > 0 && static_cast<int64_t>(B) * H <= 65535, "%s: bad B/H", who);
@@ -770,14 +830,18 @@ static int fill_build_args(BuildArgs& A, const hqkv_flush_src_t* src, int B, int
   HQKV_REQUIRE(src->low_codec == HQKV_CODEC_UNIFORM || src->low_codec == HQKV_CODEC_NORMAL, "%s: unknown low_codec %d",
                who, src->low_codec);
   memset(&A, 0, sizeof(A));
+  A.tiers_wide = 1;
   A.wide = aligned(src->residual, 16) && src->residual_b_stride % 8 == 0 && src->residual_h_stride % 8 == 0;
   for (int t = 0; t < HQKV_NUM_TIERS; ++t) {
     A.data[t] = src->data[t];
     A.scale[t] = static_cast<const __half*>(src->scale[t]);
     A.zero[t] = static_cast<const __half*>(src->zero[t]);
     A.n[t] = src->n[t];
-    HQKV_REQUIRE(src->n[t] <= 0 || (aligned(src->data[t], 16) && aligned(src->scale[t], 8) && aligned(src->zero[t], 8)),
-                 "%s: tier %d is not 16-byte aligned", who, t);
+    if (src->n[t] <= 0) continue;
+    // (a K tier's scales are those of whole groups; the fp16 tier has none, and may hold any number of tokens)
+    HQKV_REQUIRE(v_side || t == 0 || src->n[t] % group == 0, "%s: tier %d holds %d tokens, not a multiple of the group %d", who, t,
+                 src->n[t], group);
+    A.tiers_wide &= aligned(src->data[t], 16) && aligned(src->scale[t], 8) && aligned(src->zero[t], 8) && (v_side || src->n[t] % 32 == 0);
   }
   A.residual = static_cast<const __half*>(src->residual);
   A.res_b_stride = src->residual_b_stride;
@@ -794,9 +858,9 @@ static int add_dst(BuildArgs& A, bool v_side, int t, int group, const int32_t* p
   if (n > 0) {
     HQKV_REQUIRE(plan && data, "%s: null pointer", who);
     HQKV_REQUIRE(t == 0 || (scale && zero), "%s: null scale/zero output", who);
-    HQKV_REQUIRE(aligned(data, 16) && aligned(scale, 8) && aligned(zero, 8), "%s: misaligned output", who);
     HQKV_REQUIRE(v_side || n % group == 0, "%s: n_dst (%lld) is not a multiple of the group %d", who, (long long)n, group);
   }
+  A.tiers_wide &= n == 0 || (aligned(data, 16) && aligned(scale, 8) && aligned(zero, 8));
   BuildDst& d = A.dst[t];
   d.plan = plan;
   d.n = n;
@@ -815,8 +879,9 @@ static int launch_build(BuildArgs& A, bool v_side, int B, int H, const char* who
   A.tiles = static_cast<int>(tiles);
   const dim3 grid(static_cast<unsigned>(tiles + (A.rest_n > 0 ? 1 : 0)), B * H);
   if (grid.x == 0) return HQKV_OK;
-  if (v_side) flush_build_v_kernel<<<grid, BUILD_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(A);
-  else flush_build_k_kernel<<<grid, BUILD_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(A);
+  const auto kernel = v_side ? (A.tiers_wide ? flush_build_v_kernel<true> : flush_build_v_kernel<false>)
+                             : (A.tiers_wide ? flush_build_k_kernel<true> : flush_build_k_kernel<false>);
+  kernel<<<grid, BUILD_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(A);
   HQKV_LAUNCH_CHECK(who);
   return HQKV_OK;
 }
@@ -824,7 +889,7 @@ static int build_one(bool v_side, const hqkv_flush_src_t* src_host, int B, int H
                      const int32_t* plan_src_row, int64_t n_dst, void* out_data, void* out_scale, void* out_zero, const char* who,
                      void* stream) {
   BuildArgs A;
-  int rc = fill_build_args(A, src_host, B, H, Dd, group, who);
+  int rc = fill_build_args(A, v_side, src_host, B, H, Dd, group, who);
   if (rc) return rc;
   HQKV_REQUIRE(dst_tier >= 0 && dst_tier < HQKV_NUM_TIERS, "%s: dst_tier out of range", who);
   rc = add_dst(A, v_side, dst_tier, group, plan_src_row, n_dst, out_data, out_scale, out_zero, who);
@@ -852,9 +917,9 @@ extern "C" int hqkv_flush_build(int v_side, const hqkv_flush_src_t* src_host, in
                                 int64_t* const* out_ids_host, int64_t compress, int64_t rest, void* rest_out, void* stream) {
   HQKV_REQUIRE(plan_src && plan_ids && counts_host && out_data_host && out_scale_host && out_zero_host && out_ids_host,
                "flush_build: null pointer");
-  HQKV_REQUIRE(rest >= 0 && (rest == 0 || (rest_out && aligned(rest_out, 16))), "flush_build: bad residual output");
+  HQKV_REQUIRE(rest >= 0 && (rest == 0 || rest_out), "flush_build: bad residual output");
   BuildArgs A;
-  int rc = fill_build_args(A, src_host, B, H, Dd, group, "flush_build");
+  int rc = fill_build_args(A, v_side != 0, src_host, B, H, Dd, group, "flush_build");
   if (rc) return rc;
   for (int t = 0; t < HQKV_NUM_TIERS; ++t) {
     HQKV_REQUIRE(counts_host[t] >= 0 && counts_host[t] <= total, "flush_build: bad count of tier %d", t);
@@ -868,5 +933,6 @@ extern "C" int hqkv_flush_build(int v_side, const hqkv_flush_src_t* src_host, in
   A.rest = A.residual + compress * D;
   A.rest_out = static_cast<__half*>(rest_out);
   A.rest_n = rest * D;
+  A.wide &= aligned(rest_out, 16);
   return launch_build(A, v_side != 0, B, H, "flush_build", stream);
 }
