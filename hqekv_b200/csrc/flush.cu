@@ -123,8 +123,12 @@ __device__ __forceinline__ void k_load32(const BuildArgs& A, int src, int64_t po
   const int64_t row = static_cast<int64_t>(bh) * D + ch, n = A.n[src];
   if (src == 0) {
     const __half *p = reinterpret_cast<const __half*>(A.data[0]) + row * n + pos, *q = p + n;
+    const int last = WIDE ? 31 : static_cast<int>(min(n - 1 - pos, static_cast<int64_t>(31)));
 #pragma unroll
-    for (int t = 0; t < 32; ++t) v[t] = __halves2half2(p[t], q[t]);
+    for (int t = 0; t < 32; ++t) {
+      const int i = WIDE ? t : min(t, last);
+      v[t] = __halves2half2(p[i], q[i]);
+    }
     return;
   }
   const int64_t G = n >> A.gshift, gi = row * G + (pos >> A.gshift);
@@ -190,13 +194,13 @@ __device__ __forceinline__ void k_min_max(const __half2 (&v)[32], __half2& lo, _
 
 // fp64 statistics of a group of the codebook tier in token order, channels ch and ch + 1: mean, std
 template <bool WIDE>
-__device__ __noinline__ void k_normal_stats(const BuildArgs& A, int src, int64_t pos, int bh, int ch, __half2& mean, __half2& sd) {
+__device__ __noinline__ void k_normal_stats(const BuildArgs& A, const KBuildShared& sh, int run0, int bh, int ch, __half2& mean, __half2& sd) {
   const int group = 1 << A.gshift;
   const double share = static_cast<double>(1.f / static_cast<float>(group));  // (exact: a power of two)
   double s0 = 0.0, s1 = 0.0, q0 = 0.0, q1 = 0.0;
   __half2 v[32];
   for (int i = 0; i < group; i += 32) {
-    k_load32<WIDE>(A, src, pos + i, bh, ch, v);
+    k_load32<WIDE>(A, sh.src[run0 + i / 32], sh.pos[run0 + i / 32], bh, ch, v);
 #pragma unroll
     for (int t = 0; t < 32; ++t) {
       s0 += static_cast<double>(__low2float(v[t]));
@@ -205,7 +209,7 @@ __device__ __noinline__ void k_normal_stats(const BuildArgs& A, int src, int64_t
   }
   const double m0 = s0 * share, m1 = s1 * share;
   for (int i = 0; i < group; i += 32) {
-    if (group > 32) k_load32<WIDE>(A, src, pos + i, bh, ch, v);
+    if (group > 32) k_load32<WIDE>(A, sh.src[run0 + i / 32], sh.pos[run0 + i / 32], bh, ch, v);
 #pragma unroll
     for (int t = 0; t < 32; ++t) {
       const double a = static_cast<double>(__low2float(v[t])) - m0, b = static_cast<double>(__high2float(v[t])) - m1;
@@ -220,12 +224,11 @@ __device__ __noinline__ void k_normal_stats(const BuildArgs& A, int src, int64_t
 // One arrival group of the codebook tier, channels ch and ch + 1.
 template <bool WIDE>
 __device__ __noinline__ void k_normal_group(const BuildArgs& A, KBuildShared& sh, int bh, int g, int ch) {
-  const int per = 1 << (A.gshift - 5), s0 = g * per, group = 1 << A.gshift, src = sh.src[s0];
-  const int64_t pos = sh.pos[s0];
+  const int per = 1 << (A.gshift - 5), s0 = g * per, group = 1 << A.gshift;
   __half2 v[32];
   float s[2][2] = {}, c[2][2] = {}, ss[2][4] = {};
   for (int i = 0; i < per; ++i) {
-    k_load32<WIDE>(A, src, pos + 32 * i, bh, ch, v);
+    k_load32<WIDE>(A, sh.src[s0 + i], sh.pos[s0 + i], bh, ch, v);
 #pragma unroll
     for (int t = 0; t < 32; ++t) {
       add_compensated(s[0][t & 1], c[0][t & 1], __low2float(v[t]));
@@ -240,7 +243,7 @@ __device__ __noinline__ void k_normal_group(const BuildArgs& A, KBuildShared& sh
     m[k] = (s[k][0] + c[k][0]) * (1.f / static_cast<float>(group));
   }
   for (int i = 0; i < per; ++i) {
-    if (per > 1) k_load32<WIDE>(A, src, pos + 32 * i, bh, ch, v);
+    if (per > 1) k_load32<WIDE>(A, sh.src[s0 + i], sh.pos[s0 + i], bh, ch, v);
 #pragma unroll
     for (int t = 0; t < 32; ++t) {
       const float a = __low2float(v[t]) - m[0], b = __high2float(v[t]) - m[1];
@@ -254,10 +257,10 @@ __device__ __noinline__ void k_normal_group(const BuildArgs& A, KBuildShared& sh
   for (int k = 0; k < 2; ++k)
     sure &= normal1_fast(s[k][0], c[k][0], (ss[k][0] + ss[k][1]) + (ss[k][2] + ss[k][3]), group, mean[k], sd[k]);
   __half2 mean2 = __halves2half2(mean[0], mean[1]), sd2 = __halves2half2(sd[0], sd[1]);
-  if (!sure) k_normal_stats<WIDE>(A, src, pos, bh, ch, mean2, sd2);
+  if (!sure) k_normal_stats<WIDE>(A, sh, s0, bh, ch, mean2, sd2);
   const __half2 bound = __halves2half2(normal1_bound(__low2half(sd2)), normal1_bound(__high2half(sd2)));
   for (int i = 0; i < per; ++i) {
-    if (per > 1) k_load32<WIDE>(A, src, pos + 32 * i, bh, ch, v);
+    if (per > 1) k_load32<WIDE>(A, sh.src[s0 + i], sh.pos[s0 + i], bh, ch, v);
     uint32_t a = 0, b = 0;
 #pragma unroll
     for (int t = 0; t < 32; ++t) {
@@ -289,17 +292,17 @@ struct PieceType<4> {
   using type = uint32_t;
 };
 
-// a piece of a row of codes (fp16 values at 16 bits)
+// a piece of a row of codes (fp16 values at 16 bits, of which the tier has `left` from here on)
 template <int BITS, bool WIDE, typename Piece>
-__device__ __forceinline__ Piece load_piece(const unsigned char* p) {
+__device__ __forceinline__ Piece load_piece(const unsigned char* p, int64_t left) {
   if constexpr (WIDE) return *reinterpret_cast<const Piece*>(p);
   Piece v;
   uint32_t* u = reinterpret_cast<uint32_t*>(&v);
 #pragma unroll
   for (int i = 0; i < static_cast<int>(sizeof(Piece) / 4); ++i) {
     if constexpr (BITS == 16) {
-      const __half* h = reinterpret_cast<const __half*>(p) + 2 * i;
-      u[i] = as_u32(__halves2half2(h[0], h[1]));
+      const __half* h = reinterpret_cast<const __half*>(p);
+      u[i] = as_u32(__halves2half2(h[min(static_cast<int64_t>(2 * i), left - 1)], h[min(static_cast<int64_t>(2 * i + 1), left - 1)]));
     } else {
       u[i] = reinterpret_cast<const uint32_t*>(p)[i];
     }
@@ -335,8 +338,12 @@ __device__ __forceinline__ void k_build_tile(const BuildArgs& A, KBuildShared& s
   const int nsub = static_cast<int>((dst.n - j0) / 32 < KB::SUBS ? (dst.n - j0) / 32 : KB::SUBS);
   if (tid < nsub) {
     const int32_t enc = dst.plan[j0 + 32 * tid];
-    sh.src[tid] = (enc >> 28) - 1;
-    sh.pos[tid] = enc & 0x0FFFFFFF;
+    const int src = (enc >> 28) - 1;
+    sh.src[tid] = src;
+    // Runs of 32 start on multiples of 32.  The positions of ids that split blocks do not; there is no right result for them,
+    // but no access may leave its boundary or its tier for them either (an fp16 tier that does not hold whole runs: see the
+    // loads without WIDE).
+    sh.pos[tid] = enc & (WIDE || src > 0 ? 0x0FFFFFE0 : 0x0FFFFFFF);
   }
   if (bh == 0 && dst.ids_out)
     for (int i = tid; i < 32 * nsub; i += BUILD_THREADS) dst.ids_out[j0 + i] = dst.ids[j0 + i];
@@ -369,7 +376,7 @@ __device__ __forceinline__ void k_build_tile(const BuildArgs& A, KBuildShared& s
     in += r0 * in_row;
     Piece v[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = load_piece<BITS, WIDE, Piece>(in + 32 * i * in_row);
+    for (int i = 0; i < 4; ++i) v[i] = load_piece<BITS, WIDE, Piece>(in + 32 * i * in_row, A.n[t] - sh.pos[sub] - (piece * KB::PIECE / 2 - sub * 32));
 #pragma unroll
     for (int i = 0; i < 4; ++i) store_piece<BITS, WIDE>(out + 32 * i * out_row, v[i]);
   }

@@ -1,5 +1,5 @@
 """Where the tensors of a flush may lie: tiers, residual windows and (C ABI) outputs that start on no more than their type's
-own boundary; bit for bit against the oracle and against the flush of aligned tensors."""
+own boundary, bit for bit against the oracle and against the flush of aligned tensors; and ranked ids that split blocks."""
 import ctypes as C
 
 import numpy as np
@@ -115,3 +115,26 @@ def test_outputs_on_their_types_boundaries(cuda_device, case):
                 assert torch.equal(plan_ids[t, :n[t]], after[s + 1])
             del keep
         cache, hist = after[:39] + (None, None, total), total - counts[5]
+
+
+@pytest.mark.parametrize("g,strategy,low,idx", [(32, UNIFORM, 3, 21), (64, NORMAL, 4, 29)])
+def test_ranked_ids_that_split_blocks(cuda_device, g, strategy, low, idx):
+    """Not a call that makes sense - K is quantised in blocks - but its positions are the caller's and must not send a wide
+    access off its boundary or out of a tier.  The id lists are those of the plan all the same."""
+    from hqekv_b200.quant.hqe_2 import KV_cache_hqe_2
+    rng = np.random.default_rng(5)
+    new = [torch.from_numpy(window(rng, 1, 1, 5 * g)).to(cuda_device) for _ in range(2)]
+    imp = torch.ones(5 * g, dtype=torch.float16, device=cuda_device)
+    counts = [0, 2 * g, 2 * g, 0, 0, 0]
+    cache = (None,) * 39 + tuple(x[:, :, :4 * g].contiguous() for x in new) + (4 * g,)
+    cache = KV_cache_hqe_2(cache, 4 * g, 0, torch.arange(4 * g, device=cuda_device), counts, list(counts), imp[:4 * g].clone(),
+                           strategy, None, g, g)
+    cache = cache[:39] + tuple(x[:, :, 4 * g:].contiguous() for x in new) + (5 * g,)
+    keep = np.sort(rng.permutation(2 * g)[:g])            # half of the 8-bit tier, any tokens; the rest goes to the low tier
+    rest = np.setdiff1d(np.arange(5 * g), keep)
+    ids = torch.from_numpy(np.concatenate((keep, rest))).to(cuda_device)
+    k_counts, v_counts = [0, g, 0, 0, 0, 0], [0, 2 * g, 0, 0, 0, 0]
+    k_counts[low], v_counts[low] = 4 * g, 3 * g
+    got = KV_cache_hqe_2(cache, g, 4 * g, ids, k_counts, v_counts, imp, strategy, None, g, g)
+    assert got[5].tolist() == keep.tolist() and sorted(got[idx].tolist()) == rest.tolist()
+    assert got[4].shape == (1, 1, 128, g // 4) and float(torch.ones(8, device=cuda_device).sum()) == 8.0
