@@ -631,9 +631,10 @@ extern "C" int hqkv_block_rank(void* importance, const void* range_or_null, int 
 extern "C" size_t hqkv_flush_plan_workspace_bytes(int64_t total) {
   if (total < 0) return 0;
   const size_t t = static_cast<size_t>(total);
-  // tgt (1 B) + fin (1 B) + rank (4 B) per token, each region rounded to 256 bytes; per-warp counts
+  // tgt (1 B) + fin (1 B) + rank (4 B) per token, each region rounded to 256 bytes; per-warp counts; and what it takes to
+  // start on a 16-byte boundary
   auto up = [](size_t v) { return (v + 255) & ~static_cast<size_t>(255); };
-  return up(t) + up(t) + up(4 * t) + up(sizeof(int32_t) * PLAN_CATS * PLAN_GWARPS);
+  return up(t) + up(t) + up(4 * t) + up(sizeof(int32_t) * PLAN_CATS * PLAN_GWARPS) + 15;
 }
 
 static int fill_plan_side(PlanSide& S, const int64_t* const* tier_idx_host, const int32_t* tier_n_host, int64_t hist, int64_t total,
@@ -657,6 +658,7 @@ static int fill_plan_side(PlanSide& S, const int64_t* const* tier_idx_host, cons
     prev = cum_counts_host[k];
   }
   auto up = [](size_t v) { return (v + 255) & ~static_cast<size_t>(255); };
+  ws += -reinterpret_cast<uintptr_t>(ws) & 15;
   S.tgt = reinterpret_cast<int8_t*>(ws);
   S.fin = reinterpret_cast<int8_t*>(ws + up(total));
   S.rank = reinterpret_cast<int32_t*>(ws + 2 * up(total));
@@ -684,7 +686,6 @@ extern "C" int hqkv_flush_plan(const int64_t* const* tier_idx_host, const int32_
   const int64_t total = hist + compress;
   HQKV_REQUIRE(total > 0 && total < (1ll << 28), "flush_plan: total length out of range");
   HQKV_REQUIRE(sorted_ids && plan_src && plan_ids && survivors && counts && workspace, "flush_plan: null pointer");
-  HQKV_REQUIRE(aligned(workspace, 16), "flush_plan: workspace must be 16-byte aligned");
   PlanArgs A;
   memset(&A, 0, sizeof(A));
   A.hist = hist;

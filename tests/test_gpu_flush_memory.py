@@ -72,7 +72,7 @@ def test_tiers_and_window_on_their_types_boundaries(cuda_device, case):
 
 @pytest.mark.parametrize("case", CASES)
 def test_outputs_on_their_types_boundaries(cuda_device, case):
-    """Plan and build of one tier at a time through the C ABI, with outputs on their types' boundaries."""
+    """Plan and build of one tier at a time through the C ABI, with outputs and plan scratch on their types' boundaries."""
     from hqekv_b200._lib import CODEC_NORMAL, CODEC_UNIFORM, check, lib, ptr, stream_ptr
     from hqekv_b200.model.public_func import get_block_token_idx
     from hqekv_b200.quant._cache import build_flush_src, void_p_array
@@ -97,7 +97,7 @@ def test_outputs_on_their_types_boundaries(cuda_device, case):
             plan_ids = torch.empty(5, total, dtype=torch.int64, device=cuda_device)
             surv = torch.empty(total, dtype=torch.int64, device=cuda_device)
             n = torch.zeros(8, dtype=torch.int32, device=cuda_device)
-            ws = torch.empty(lib.hqkv_flush_plan_workspace_bytes(total), dtype=torch.uint8, device=cuda_device)
+            ws = torch.empty(lib.hqkv_flush_plan_workspace_bytes(total) + 4, dtype=torch.uint8, device=cuda_device)[4:]
             check(lib.hqkv_flush_plan(void_p_array(idx), (C.c_int32 * 5)(*[0 if i is None else i.numel() for i in idx]), hist,
                                       flushed, ptr(ids), (C.c_int64 * 6)(*np.cumsum(counts)), ptr(plan_src), ptr(plan_ids),
                                       ptr(surv), ptr(n), ptr(ws), ws.numel(), st))
