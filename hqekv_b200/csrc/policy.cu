@@ -776,7 +776,7 @@ struct FlushLane {
       memset(p, 0, 64);
       host = static_cast<volatile int32_t*>(p);
     }
-    if (side && now == dev) return HQKV_OK;
+    if (now == dev) return HQKV_OK;
     close();
     int least = 0, greatest = 0;  // ahead of the K build's CTAs: the V side's clusters need room on eight SMs at once
     HQKV_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
@@ -787,10 +787,12 @@ struct FlushLane {
     return HQKV_OK;
   }
   void close() {
-    if (side) cudaStreamDestroy(side);
+    // a plan that nobody waited for (a call that ended early) may still write its counts: not into memory that is given back,
+    // nor after those of the next plan
+    if (side) cudaStreamSynchronize(side), cudaStreamDestroy(side);
     if (fork) cudaEventDestroy(fork);
     if (join) cudaEventDestroy(join);
-    side = nullptr, fork = join = nullptr;
+    side = nullptr, fork = join = nullptr, dev = -1;
   }
   // waits for the counts of a side whose plan is in stream st
   int counts(int v_side, cudaStream_t st, int32_t* out) {
