@@ -184,12 +184,13 @@ __global__ void __launch_bounds__(RANGE_THREADS) token_range128_kernel(const __h
 // Each CTA of the cluster forms the keys of its share of the blocks (elementwise pass, then one thread per block adds in
 // order) and stores them into the shared memory of all CTAs.  The keys - fp16 key, then block id - are all different, so a
 // block's place is the number of smaller keys: every warp counts for its own blocks, with no exchange between the
-// steps of a sort.  16.7 -> 6 us for 508 blocks and 25 -> 7 us for 1 020 against a bitonic sort by one CTA; the comparisons
-// grow with the square of the blocks, and beyond RANK_COUNT_MAX the sort is kept.
+// steps of a sort.  The comparisons grow with the square of the blocks, so beyond RANK_COUNT_MAX a bitonic sort (by every
+// CTA for itself) is kept.  us, blocks of 32 tokens, counting / sort: 512: 7.2 / 12.3, 1024: 10.2 / 14.4, 2048: 19.0 / 22.5,
+// 3072: 32.8 / 34.8, 4096: 51.2 / 36.9, 8192: 172 / 69.
 constexpr int RANK_THREADS = 1024;
 constexpr int RANK_CLUSTER = 8;
 constexpr int RANK_MAX_BLOCKS = 8192;
-constexpr int RANK_COUNT_MAX = 4096;
+constexpr int RANK_COUNT_MAX = 3072;
 
 __global__ void __launch_bounds__(RANK_THREADS) block_rank_kernel(const __half* importance, const __half* __restrict__ range,
                                                                   __half* divided, int block, int nblocks, int npow2,
