@@ -55,9 +55,6 @@ static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 __device__ __forceinline__ __half h_sub(__half a, __half b) {
   return __float2half_rn(__fsub_rn(__half2float(a), __half2float(b)));
 }
-__device__ __forceinline__ __half h_div(__half a, __half b) {
-  return __float2half_rn(__fdiv_rn(__half2float(a), __half2float(b)));
-}
 __device__ __forceinline__ __half h_divf(__half a, float b) {
   return __float2half_rn(__fdiv_rn(__half2float(a), b));
 }
@@ -184,11 +181,6 @@ __device__ __forceinline__ __half quant_scale(__half mn, __half mx, float levels
   return h_divf(h_sub(mx, mn), levels);
 }
 
-// Two-rounding dequantisation: half(half(code * scale) + mn).
-__device__ __forceinline__ __half dequant_2r(uint32_t code, __half scale, __half mn) {
-  return h_add(h_mul(__uint2half_rn(code), scale), mn);
-}
-
 // Gaussian-codebook codec at 1 bit.  std and mean of a group are torch.std_mean (unbiased) of its fp16
 // values: computed in fp64 (the sum of up to 128 fp16 values is exact there) and rounded once to fp16.
 __device__ __forceinline__ __half normal1_sd(double sum_sq_dev, int group) {
@@ -208,7 +200,7 @@ __device__ __forceinline__ bool normal1_fast(float s, float c, float ss, int gro
          __half_as_ushort(sd) == __half_as_ushort(__float2half_rn(d + off)) && fabsf(m) >= d * 0x1p-13f && d > 1e-6f &&
          d < 6e4f && fabsf(m) < 6e4f;
 }
-// x added to s + c, the rounding error of the addition kept in c
+// x added to s + c, the rounding error of the addition kept in c (Knuth's TwoSum)
 __device__ __forceinline__ void add_compensated(float& s, float& c, float x) {
   const float t = __fadd_rn(s, x), back = __fsub_rn(t, s);
   c += __fadd_rn(__fsub_rn(s, __fsub_rn(t, back)), __fsub_rn(x, back));

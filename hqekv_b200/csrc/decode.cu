@@ -84,10 +84,11 @@ struct DecodeParams {
 };
 
 // The tokens of a (batch, virtual kv head) plane are a list of UNITS - 256 tokens of one tier (128 at 8 bits, 64 of the
-// fp16 tier and of the residual window), tiers in order - and its CTAs take consecutive shares of it of equal COST: a unit
-// of 8 bits takes both passes 0.6 of the time of one of 4 or 2 bits (2.2 against 3.4 us in the K pass, 2.3 against 3.9
-// in the V pass with four CTAs on every SM), and the CTA with the longest share decides (20/40/40 at 24 x 8 x 15360 tokens
-// in shares of equal count: the V pass took 94 us, the time of the CTAs with 4 and 2 bits only).
+// fp16 tier and of the residual window), tiers in order - and its CTAs take consecutive shares of it of equal COST, for the
+// CTA with the longest share decides (20/40/40 at 24 x 8 x 15360 tokens in shares of equal count: the V pass took 94 us,
+// the time of the CTAs with 4 and 2 bits only).  us a unit with four CTAs on every SM, K / V pass: 8 bits 1.9 / 2.4,
+// 4 bits 3.2 / 3.2, 2 bits 2.9 / 2.9, 1 bit 3.3 / 3.2, fp16 tier 4.3 / 2.5, residual window 3.2 / 2.4.  One cost serves
+// both passes and the two kinds of fp16 unit, of which a plane has few.
 __host__ __device__ constexpr int unit_tokens(int bits) { return bits == 16 ? 64 : bits == 8 ? 128 : 256; }
 __host__ __device__ constexpr int unit_cost(int bits) { return bits == 8 ? 5 : 8; }
 // This CTA's tokens [t0, t1) of tier ti; false: none.
@@ -1058,10 +1059,7 @@ __global__ void __launch_bounds__(KTHREADS, K_MIN_CTAS) k_pass_kernel(const __gr
 // and MMAs.
 // Codes are streamed through ONE tile buffer: the copy of a 16-token step of the next tile is issued when this tile's
 // step has been consumed, so a whole tile's work lies between a request and its use.
-#ifndef HQKV_VM
-#define HQKV_VM 4
-#endif
-constexpr int V_MIN_CTAS = HQKV_VM;  // CTAs per SM the V pass is compiled for (102 registers; shared memory allows five)
+constexpr int V_MIN_CTAS = 4;  // CTAs per SM the V pass is compiled for (128 registers; PASS_SMEM is a quarter of an SM)
 constexpr int VWARPS = 4;
 constexpr int VTHREADS = VWARPS * 32;
 constexpr int V_ST = 72 * 4;                       // bytes per 16-token step of a B plane (64 words + 8: no bank conflicts)
