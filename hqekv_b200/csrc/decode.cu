@@ -1817,6 +1817,8 @@ __device__ __noinline__ void head_sum_chunk(const DecodeParams& P, const TierDev
 
 // GV: log2 of the channel group, with four or two query heads per CTA and the softmax of the scratch logits; 0: everything else.
 // ONE_TIER: no CTA has units of two tiers.
+// At 128 registers the one-tier kernels spill 24 - 40 bytes a thread and the others 136 - 160 (-Xptxas -v), around the loops
+// over tiles: local loads and stores are 0.1 % of a launch's instructions at batch 1 of 32 k tokens, 0.05 % at batch 8 of 16 k.
 template <int GV, bool ONE_TIER>
 __global__ void __launch_bounds__(VTHREADS, V_MIN_CTAS) v_pass_kernel(const __grid_constant__ DecodeParams P) {
   extern __shared__ __align__(128) unsigned char smem_raw[];

@@ -87,8 +87,12 @@ __device__ __forceinline__ void copy_rest(const BuildArgs& A, int bh) {
 // flight per thread, where a thread per channel copied a word at a time, a row apart from its neighbour's.  An arrival is a
 // thread per pair of channels and 32 tokens, all 32 in registers; its words and scales meet in shared memory and are
 // stored in the same runs.  32 tokens into 24 k: 36 us (126 with a launch per tier and a thread per channel), into 8 x 16 k:
-// 51 us (302; what it copies takes 28 at the copy rate); a prefill of 32 k tokens: 30 us (174).  What bounds it is latency:
-// the chain plan - source - store of a tile, and the few tiles with arrivals, which are started first for that reason.
+// 51 us (302; what it copies takes 28 at the copy rate); a prefill of 32 k tokens: 30 us (174).  What bounds a small flush is
+// latency: the chain plan - source - store of a tile, and the few tiles with arrivals, which are started first for that
+// reason (issue slots 23 % used, warps wait for memory).  A prefill, all arrivals: instructions (41 %) and their fetch.
+// 64 registers a thread, for four CTAs per SM, are less than an arrival wants: the kernel spills 666 bytes and reads 626 back
+// (-Xptxas -v), a codebook group 732 and 388.  Local loads and stores are 2 % of the instructions of that prefill, and
+// 8 % of the 32 tokens into 24 k, where groups arrive in the codebook tier.
 template <int BITS>
 struct KBuild {
   static constexpr int TOKENS = BITS == 16 ? 64 : BITS == 8 ? 128 : 256;
@@ -507,6 +511,9 @@ __global__ void __launch_bounds__(BUILD_THREADS, 4) flush_build_k_kernel(const _
 // consecutive in one source (one vote): kept ones are then a contiguous copy, 16 bytes per lane, and arrivals are eight
 // tokens per step, 32 channels per lane: a group's scale and reciprocal are one lane's.  (With eight channels per lane four
 // lanes repeated them, and those instructions were most of the kernel.)  Any other run of tokens goes one by one.
+// A prefill of 32 k tokens takes 20 us and is bound by instructions (63 % of the issue slots), 32 tokens into 24 k take 18 us and
+// are bound by latency.  64 registers a thread: 1160 bytes spilled, 2324 read back (-Xptxas -v), most of it on ways that few
+// warps take: 0.6 and 1.4 % of the instructions of the two are local loads and stores.
 __device__ __forceinline__ __half v_get(const void* p, int bits, int c) {  // code c of a packed row
   const uint32_t w = reinterpret_cast<const uint32_t*>(p)[c * bits / 32];
   return __uint2half_rn((w >> ((c * bits) & 31)) & ((1u << bits) - 1u));

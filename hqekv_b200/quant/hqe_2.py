@@ -4,8 +4,10 @@ Same names, arguments, results and errors as KV_cache_hqe_2 / KV_cache_reconstru
 reference's quant/hqe_2.py (:456-843, :967-1084).  The reference walks a ladder of up to 30
 isin / boolean-mask / torch.cat steps with a host synchronisation in most of them and an
 n_tier x n_all equality matrix for the re-ranking; here each side (K, V) is one planning kernel
-plus one build kernel per destination tier (hqekv_b200/csrc/policy.cu), with a single device-to-host
-copy of ten integers in between to size the new tensors.
+(hqekv_b200/csrc/policy.cu) and one kernel that builds all of its tiers (csrc/flush.cu), issued from native code
+(csrc/host.cpp).  The tier sizes come to the host through mapped memory while the plan still writes its lists, and
+the V side is ranked and planned on a second stream beside the K side's build.  Arguments that the native path does
+not take as they are go the way below: a kernel per destination tier, and one copy of the sizes to the host.
 """
 import torch
 

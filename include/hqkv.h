@@ -392,6 +392,7 @@ int hqkv_block_rank(void* importance, const void* range_or_null, int block, int 
  *   counts     int32 [8]          final size of the five tiers, number of survivors, 1 if any token was
  *                                 evicted else 0, 0
  * The caller reads `counts` back (one small copy) to size the new tier tensors.
+ * workspace: hqkv_flush_plan_workspace_bytes(hist + compress) bytes of any alignment.
  */
 int hqkv_flush_plan(const int64_t* const* tier_idx_host, const int32_t* tier_n_host, int64_t hist, int64_t compress,
                     const int64_t* sorted_ids, const int64_t* cum_counts_host, int32_t* plan_src, int64_t* plan_ids,
@@ -416,6 +417,10 @@ typedef struct {
  * destination width in groups of `group` tokens per channel (K_high_2_low / quant_new_K,
  * quant/hqe_2.py:16-42, 88-130).  n_dst = counts[dst_tier] from phase 1; outputs dense
  * [B,H,D,n_dst*bits/32] / [B,H,D,n_dst/group] (fp16 [B,H,D,n_dst] for the 16-bit tier).
+ * Sources, residual and outputs may start on any boundary of their element type (packed words 4 bytes, fp16 2); where all of
+ * them lie on 16-byte boundaries (V scales and zeros: 8) and the residual's strides are multiples of 8, the accesses are
+ * 16 bytes wide, else by element.  The tokens of a destination group come from one source and follow one another there;
+ * quantised K sources hold whole groups (n a multiple of `group`, refused otherwise).
  */
 int hqkv_flush_build_k(const hqkv_flush_src_t* src_host, int B, int H, int D, int group, int dst_tier,
                        const int32_t* plan_src_row, int64_t n_dst, void* out_data, void* out_scale, void* out_zero,
@@ -448,6 +453,8 @@ int hqkv_flush_build(int v_side, const hqkv_flush_src_t* src_host, int B, int H,
  *   hqkv_flush_evict     compacts norm_out to the V-side survivors (-> norm_kept) and moves the survivors' columns of an
  *                        importance ring (fp16 [rows][stride], null: none) to the front, in place
  * `workspace`: hqkv_flush_workspace_bytes(hist + compress) bytes, 256-byte aligned, kept between the calls.
+ * hqkv_flush_prepare takes D = 128, B*H <= 4096, at most 8192 blocks, and a V window that starts on a 16-byte boundary
+ * with strides that are multiples of 8; hqkv_flush_plan and hqkv_flush_build_k/v have none of these limits but D.
  */
 typedef struct {
   int32_t B, H, D, block, group, times_range;  /* block: K group = ranking block; group: V group */
