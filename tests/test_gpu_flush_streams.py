@@ -141,3 +141,17 @@ def test_threads_that_come_and_go(cuda_device):
         # the threads have ended before their results are looked at, one of them behind a flush that ended early
         in_threads([lambda: outs.append(work.run()), lambda: fails_early(cuda_device)])
         work.check(outs[0])
+
+
+def test_refused_under_capture(cuda_device):
+    """A flush asks the device for the tier sizes, so it cannot be captured: an error, and the next flush is as good as any."""
+    work = Work(30, cuda_device)
+    out = work.run()
+    torch.cuda.synchronize()
+    work.check(out)
+    with pytest.raises(RuntimeError):
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            work.run()
+    torch.cuda.synchronize()
+    for _ in range(2):
+        work.check(work.run())
