@@ -694,7 +694,7 @@ extern "C" int hqkv_flush_plan(const int64_t* const* tier_idx_host, const int32_
   int rc = fill_plan_side(A.side, tier_idx_host, tier_n_host, hist, total, sorted_ids, cum_counts_host, plan_src, plan_ids,
                           survivors, counts, static_cast<unsigned char*>(workspace));
   if (rc) return rc;
-  const size_t need = hqkv_flush_plan_workspace_bytes(total);
+  const size_t need = hqkv_flush_plan_workspace_bytes(total) - 15 + (-reinterpret_cast<uintptr_t>(workspace) & 15);
   if (workspace_bytes < need)
     return fail(HQKV_E_WORKSPACE, "flush_plan: workspace holds %zu bytes, %zu needed", workspace_bytes, need);
   return launch_plan(A, stream);
