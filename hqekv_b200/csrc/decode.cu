@@ -46,8 +46,12 @@ struct TierDev {
   int n_k, n_v;
   int bits;
   int normal;  // 1-bit tier in the Gaussian-codebook codec: value = std * (+-C) + mean, scale slots = std, zero = mean
-  int k_cost0, v_cost0;      // cost of the plane's units before the tier's (K pass, V pass)
-  int k_cta0, v_cta0;        // ... and its CTAs in the list of the plane's, where no CTA has units of two tiers
+  struct Units {
+    int tokens, cost;        // of a unit
+    unsigned per_cost;       // 2^32 / cost, rounded up
+    int cost0;               // cost of the plane's units before the tier's
+    int cta0;                // ... and its CTAs in the list of the plane's, where no CTA has units of two tiers
+  } unit[2];                 // K pass, V pass
 };
 
 struct DecodeParams {
@@ -60,6 +64,8 @@ struct DecodeParams {
   // Units per CTA.  more >= 0: equal shares, the first `more` CTAs take one more; -1: no CTA has units of two tiers (in
   // the K pass 8-bit units, which are half as long, count half).
   int k_per, k_more, v_per, v_more;
+  int v_pairs;             // 32 tokens a warp of the V pass takes at a time: 1, 2
+  int direct;              // the outputs are finished by whoever adds the last share (see v_finish), not by a CTA that reads them back
   float scale;
   const __half* q;
   const __half* mask;      // additive mask on the logits (null: none); element (b, head, pos) at b*bstride + head*hstride + pos
@@ -69,9 +75,9 @@ struct DecodeParams {
   unsigned* hs_count;      // [nv_ctas] arrival counters of that sum
   __half* weights;
   __half* out;
-  float* logits;   // [B][virtual kv head][L][r4]
+  float* logits;   // [B][virtual kv head], see logit_at
   float2* k_part;  // [B][virtual kv head][r4][nk_ctas]
-  double* v_acc;   // [B][nh_q][D] output accumulators: cleared by the K pass, summed into by the V pass
+  double* v_acc;   // [B][nh_q][D] output accumulators (or words, see v_finish): cleared by the K pass, summed into by the V pass
   __half* peer_out[HQKV_MAX_PEERS];  // copies of `out` in other GPUs' memory (kv-head sharding), n_peers used
   int n_peers;
   int peer_flagged;  // 1: peer_out are flagged 8-byte entries {two fp16 values, call number}, see peer_unpack_kernel
@@ -83,23 +89,30 @@ struct DecodeParams {
   unsigned* counters;  // [B][virtual kv head]
 };
 
-// The tokens of a (batch, virtual kv head) plane are a list of UNITS - 256 tokens of one tier (128 at 8 bits, 64 of the
-// fp16 tier and of the residual window), tiers in order - and its CTAs take consecutive shares of it of equal COST, for the
-// CTA with the longest share decides (20/40/40 at 24 x 8 x 15360 tokens in shares of equal count: the V pass took 94 us,
-// the time of the CTAs with 4 and 2 bits only).  us a unit with four CTAs on every SM, K / V pass: 8 bits 1.9 / 2.4,
-// 4 bits 3.2 / 3.2, 2 bits 2.9 / 2.9, 1 bit 3.3 / 3.2, fp16 tier 4.3 / 2.5, residual window 3.2 / 2.4.  One cost serves
-// both passes and the two kinds of fp16 unit, of which a plane has few.
+// The tokens of a (batch, virtual kv head) plane are a list of UNITS, tiers in order, and its CTAs take consecutive shares of
+// it of equal COST, for the CTA with the longest share decides (20/40/40 at 24 x 8 x 15360 tokens in shares of equal count:
+// the V pass took 94 us, the time of the CTAs with 4 and 2 bits only).  K pass: 256 tokens of a tier (128 at 8 bits, 64 of the
+// fp16 tier and of the residual window).  V pass: 256 (64 in fp16), or 128 where that many CTAs find a place at once.
+// us a unit with four CTAs on every SM, K pass: 8 bits 1.9, 4 bits 3.2, 2 bits 2.9, 1 bit 3.3, fp16 tier 4.3, residual window
+// 3.2; V pass: 8 bits 4.0, 4 bits 2.7, 2 bits 2.5, fp16 2.4.
 __host__ __device__ constexpr int unit_tokens(int bits) { return bits == 16 ? 64 : bits == 8 ? 128 : 256; }
 __host__ __device__ constexpr int unit_cost(int bits) { return bits == 8 ? 5 : 8; }
 // This CTA's tokens [t0, t1) of tier ti; false: none.
 template <bool V>
-__device__ __forceinline__ bool share_of(const DecodeParams& P, int ti, int bits, int& t0, int& t1) {
+__device__ __forceinline__ bool share_of(const DecodeParams& P, int ti, int& t0, int& t1) {
   const TierDev& T = P.tier[ti];
-  const int i = blockIdx.y, per = V ? P.v_per : P.k_per, more = V ? P.v_more : P.k_more;
-  const int c0 = i * per + min(i, more) - (V ? T.v_cost0 : T.k_cost0), c1 = c0 + per + (i < more ? 1 : 0);
-  const int c = unit_cost(bits);  // a unit belongs to the share that its cost starts in
-  t0 = (max(c0, 0) + c - 1) / c * unit_tokens(bits);
-  t1 = min((max(c1, 0) + c - 1) / c * unit_tokens(bits), V ? T.n_v : T.n_k);
+  const TierDev::Units& U = T.unit[V];
+  const int i = blockIdx.y, per = V ? P.v_per : P.k_per, more = V ? P.v_more : P.k_more, n = V ? T.n_v : T.n_k;
+  if (more < 0) {  // no CTA has units of two tiers
+    const int own = max(static_cast<int>(__umulhi(per, U.per_cost)), 1) * U.tokens;
+    t0 = (i - U.cta0) * own;
+    t1 = min(t0 + own, n);
+    return t0 >= 0 && t0 < t1;
+  }
+  const int c0 = i * per + min(i, more) - U.cost0, c1 = c0 + per + (i < more ? 1 : 0);
+  // a unit belongs to the share that its cost starts in
+  t0 = __umulhi(max(c0, 0) + U.cost - 1, U.per_cost) * U.tokens;
+  t1 = min(static_cast<int>(__umulhi(max(c1, 0) + U.cost - 1, U.per_cost)) * U.tokens, n);
   return t0 < t1;
 }
 // The same where no CTA has units of two tiers: the tier, too.
@@ -109,12 +122,16 @@ __device__ __forceinline__ int only_share(const DecodeParams& P, int& t0, int& t
   int ti = 0;
 #pragma unroll
   for (int t = 1; t <= HQKV_NUM_TIERS; ++t)
-    if (i >= (V ? P.tier[t].v_cta0 : P.tier[t].k_cta0)) ti = t;
-  const TierDev& T = P.tier[ti];
-  const int c = unit_cost(T.bits), n = max(V ? P.v_per : P.k_per, c) / c * unit_tokens(T.bits);
-  t0 = (i - (V ? T.v_cta0 : T.k_cta0)) * n;
-  t1 = min(t0 + n, V ? T.n_v : T.n_k);
+    if (i >= P.tier[t].unit[V].cta0) ti = t;
+  share_of<V>(P, ti, t0, t1);
   return ti;
+}
+
+// Scratch logits of a (batch, virtual kv head) plane: [pos / 4][head][4 positions], the last quad with as many positions as it
+// has.  A lane of the K pass has four or eight consecutive tokens of one head, a lane of the V pass takes four.
+__device__ __forceinline__ int64_t logit_at(int64_t pos, int head, int heads, int L) {
+  const int64_t quad = pos & ~static_cast<int64_t>(3);
+  return quad * heads + head * (L - quad < 4 ? static_cast<int>(L - quad) : 4) + (pos & 3);
 }
 
 // Grid: x = virtual kv head, y = share of the plane's units, z = batch.
@@ -158,6 +175,7 @@ __device__ __forceinline__ uint32_t h2_rem(uint32_t a, uint32_t b, uint32_t c) {
 // 16-bit halves of two words -> one half2 register: low halves, high halves
 __device__ __forceinline__ uint32_t pack_lo16(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x5410); }
 __device__ __forceinline__ uint32_t pack_hi16(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); }
+__device__ __forceinline__ uint32_t pack_hi_lo(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x5432); }  // high half of a, low half of b
 __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) { return h2_as_u32(__floats2half2_rn(lo, hi)); }
 
 // Streaming loads: the cache is read once per call, keep it out of L1.
@@ -203,6 +221,9 @@ __device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st
 __device__ __forceinline__ void sts64(uint32_t a, uint32_t x, uint32_t y) {
   asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(a), "r"(x), "r"(y) : "memory");
 }
+__device__ __forceinline__ void sts128(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
 
 // global -> shared copies without a register round trip; completion = wait_group + barrier
 __device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src) {
@@ -210,6 +231,10 @@ __device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src) {
 }
 __device__ __forceinline__ void cp_async_8(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+// the first `valid` bytes are read, the rest is set to 0
+__device__ __forceinline__ void cp_async_8_fill(uint32_t dst, const void* src, int valid) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(valid) : "memory");
 }
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -226,6 +251,10 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t row
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(row_addr) : "memory");
+}
+// two of them, at the row addresses of lanes 0-15
+__device__ __forceinline__ void ldmatrix_x2_trans(uint32_t (&r)[2], uint32_t row_addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(row_addr) : "memory");
 }
 
 // the same without the transposition: lane (g, tig) gets elements 2*tig, 2*tig+1 of row g
@@ -671,7 +700,7 @@ __device__ __forceinline__ void k_store_any(const DecodeParams& P, const TierDev
   using TL = KTile<BITS>;
   constexpr int NX = TL::NX, HALVES = TL::HALVES;
   const int tig = threadIdx.x & 3, lb = k_lane_base<BITS>();
-  float* out = P.logits + static_cast<int64_t>(w.bvh) * P.L * P.r4 + tig;
+  float* out = P.logits + static_cast<int64_t>(w.bvh) * P.L * P.r4;
   bool valid[HALVES];
 #pragma unroll
   for (int u = 0; u < HALVES; ++u) valid[u] = wt0 + 32 * u < T.n_k;
@@ -692,7 +721,7 @@ __device__ __forceinline__ void k_store_any(const DecodeParams& P, const TierDev
         ok = ok && HQKV_INDEX_OK(pos, P.L);
         if (ok) {
           if (mrow) x[j] += __half2float(mrow[pos]);
-          out[static_cast<int64_t>(pos) * P.r4] = x[j];
+          out[logit_at(pos, tig, P.r4, P.L)] = x[j];
         } else {
           x[j] = -INFINITY;
         }
@@ -708,7 +737,7 @@ __device__ __forceinline__ void k_emit(const DecodeParams& P, const TierDev& T, 
   constexpr int NX = TL::NX, HALVES = TL::HALVES;
   const int lane = threadIdx.x & 31, tig = lane & 3;
   const int lb = k_lane_base<BITS>();
-  float* out = P.logits + static_cast<int64_t>(w.bvh) * P.L * P.r4 + tig;
+  float* out = P.logits + static_cast<int64_t>(w.bvh) * P.L * P.r4 + 4 * tig;
   // whole 32-token units are valid or not (a tier holds a multiple of 32 tokens)
   bool valid[HALVES], dense = P.r4 >= 2 && P.mask == nullptr;
   uint32_t base[HALVES];
@@ -716,32 +745,53 @@ __device__ __forceinline__ void k_emit(const DecodeParams& P, const TierDev& T, 
   for (int u = 0; u < HALVES; ++u) {
     valid[u] = wt0 + 32 * u < T.n_k;
     base[u] = __shfl_sync(0xffffffffu, pu[u], 0);
-    dense = dense && (!valid[u] || (pu[u] == base[u] + lane && HQKV_INDEX_OK(pu[u], P.L)));
+    dense = dense && (!valid[u] || (pu[u] == base[u] + lane && (base[u] & 3) == 0 && HQKV_INDEX_OK(pu[u], P.L)));
   }
   if (__all_sync(0xffffffffu, dense)) {
     const bool on = tig < P.r4;
-    auto store = [&](auto heads) {  // a constant distance between a lane's tokens
+    auto store = [&](auto heads) {
       constexpr int R = decltype(heads)::value;
-      if constexpr (BITS == 4 || BITS == 8) {
+      // N logits at consecutive positions from `token` of unit u on, x[j], x[j + 2], ...; two heads start on 8-byte boundaries
+      auto run = [&](auto count, uint32_t unit, int token, int j, bool ok) {
+        constexpr int N = decltype(count)::value;
+        float* o = out + static_cast<int64_t>(unit + (token & ~3)) * R + (token & 3);
+        if (!ok) {
+#pragma unroll
+          for (int i = 0; i < N; ++i) x[j + 2 * i] = -INFINITY;
+        } else if constexpr (R == MAX_R4 && N == 4) {
+          *reinterpret_cast<float4*>(o) = make_float4(x[j], x[j + 2], x[j + 4], x[j + 6]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < N; i += 2) *reinterpret_cast<float2*>(o + i) = make_float2(x[j + 2 * i], x[j + 2 * i + 2]);
+        }
+      };
+      using Two = std::integral_constant<int, 2>;
+      using Four = std::integral_constant<int, 4>;
+      if constexpr (BITS == 8) {
+        const bool ok = valid[0] && (R == MAX_R4 || on);
+        run(Two(), base[0], lb, 0, ok);
+        run(Two(), base[0], lb + 16, 1, ok);
+      } else if constexpr (BITS == 4) {  // x[4u ...]: tokens 0, 2, 1, 3 of the lane's quad
 #pragma unroll
         for (int u = 0; u < HALVES; ++u) {
-          float* o = out + static_cast<int64_t>(base[u] + lb) * R;
           const bool ok = valid[u] && (R == MAX_R4 || on);
+          float* o = out + static_cast<int64_t>(base[u] + lb) * R;
+          if (!ok) {
 #pragma unroll
-          for (int j = 4 * u; j < 4 * u + 4; ++j) {
-            if (ok) o[k_step<BITS>(j) * R] = x[j];
-            else x[j] = -INFINITY;
+            for (int j = 4 * u; j < 4 * u + 4; ++j) x[j] = -INFINITY;
+          } else if constexpr (R == MAX_R4) {
+            *reinterpret_cast<float4*>(o) = make_float4(x[4 * u], x[4 * u + 2], x[4 * u + 1], x[4 * u + 3]);
+          } else {
+            reinterpret_cast<float2*>(o)[0] = make_float2(x[4 * u], x[4 * u + 2]);
+            reinterpret_cast<float2*>(o)[1] = make_float2(x[4 * u + 1], x[4 * u + 3]);
           }
         }
       } else {
         const bool second = k_lane_unit<BITS>() == 1;
         const bool ok = (second ? valid[HALVES - 1] : valid[0]) && (R == MAX_R4 || on);
-        float* o = out + static_cast<int64_t>((second ? base[HALVES - 1] : base[0]) + lb) * R;
-#pragma unroll
-        for (int j = 0; j < NX; ++j) {
-          if (ok) o[k_step<BITS>(j) * R] = x[j];
-          else x[j] = -INFINITY;
-        }
+        const uint32_t unit = second ? base[HALVES - 1] : base[0];
+        run(Four(), unit, lb, 0, ok);
+        run(Four(), unit, lb + (BITS == 2 ? 4 : 8), 1, ok);
       }
     };
     if (P.r4 == MAX_R4) store(std::integral_constant<int, MAX_R4>());
@@ -841,7 +891,7 @@ __device__ __forceinline__ void k_write_tile(const DecodeParams& P, const Where&
   const int lane = threadIdx.x & 31;
   const int rep = P.r4, rshift = P.r4_shift;
   const int h = lane & (rep - 1);
-  float* out = P.logits + static_cast<int64_t>(w.bvh) * P.L * rep + h;
+  float* out = P.logits + static_cast<int64_t>(w.bvh) * P.L * rep;
   const __half* mrow = P.mask ? P.mask + w.b * P.mask_bstride + static_cast<int64_t>(w.h0 + h) * P.mask_hstride : nullptr;
   const int tpr = 32 >> rshift;  // tokens per round
   float m = -INFINITY, l = 0.f;
@@ -852,7 +902,7 @@ __device__ __forceinline__ void k_write_tile(const DecodeParams& P, const Where&
     if (HQKV_INDEX_OK(pos, P.L)) {
       x[0] = tile[t * K_TROW + h];
       if (mrow) x[0] += __half2float(mrow[pos]);
-      out[pos * rep] = x[0];
+      out[logit_at(pos, h, rep, P.L)] = x[0];
     }
     softmax_push<1>(m, l, x);
   }
@@ -1001,12 +1051,12 @@ __global__ void __launch_bounds__(KTHREADS, K_MIN_CTAS) k_pass_kernel(const __gr
     else if (ti == 4) k_run<1>(P, P.tier[4], sh, w, t0, t1, m, l, first);
     else plain(ti, t0, t1);
   } else {
-    if (share_of<false>(P, 1, 8, t0, t1)) k_run<8>(P, P.tier[1], sh, w, t0, t1, m, l, first);
-    if (share_of<false>(P, 2, 4, t0, t1)) k_run<4>(P, P.tier[2], sh, w, t0, t1, m, l, first);
-    if (share_of<false>(P, 3, 2, t0, t1)) k_run<2>(P, P.tier[3], sh, w, t0, t1, m, l, first);
-    if (share_of<false>(P, 4, 1, t0, t1)) k_run<1>(P, P.tier[4], sh, w, t0, t1, m, l, first);
+    if (share_of<false>(P, 1, t0, t1)) k_run<8>(P, P.tier[1], sh, w, t0, t1, m, l, first);
+    if (share_of<false>(P, 2, t0, t1)) k_run<4>(P, P.tier[2], sh, w, t0, t1, m, l, first);
+    if (share_of<false>(P, 3, t0, t1)) k_run<2>(P, P.tier[3], sh, w, t0, t1, m, l, first);
+    if (share_of<false>(P, 4, t0, t1)) k_run<1>(P, P.tier[4], sh, w, t0, t1, m, l, first);
     for (int ti = 0; ti <= HQKV_NUM_TIERS; ti += HQKV_NUM_TIERS)
-      if (share_of<false>(P, ti, 16, t0, t1)) plain(ti, t0, t1);
+      if (share_of<false>(P, ti, t0, t1)) plain(ti, t0, t1);
   }
   // the warp's (max, sum-exp) per head: the eight lanes with the same tig
   {
@@ -1042,630 +1092,353 @@ __global__ void __launch_bounds__(KTHREADS, K_MIN_CTAS) k_pass_kernel(const __gr
 // ------------------------------------------------------------------------------------------------
 // v_pass
 // ------------------------------------------------------------------------------------------------
-// V tier, token-major rows of 128 channels.  Every warp of a CTA walks TILES of consecutive tokens of one tier on its own
-// (4 KB of codes at 8 / 4 bits = 32 / 64 tokens, 64 tokens at 2 / 1 bits) and keeps the output of all 128 channels x
-// four heads in its accumulators from tile to tile, so nothing but the end of the kernel needs the other warps.
-// The contraction runs over tokens, 16 per step.  ldmatrix.trans over 8 token rows x 16 bytes hands
-// lane (g, tig) the 16-bit block g (2 / 4 / 8 channels) of tokens 2*tig and 2*tig+1 in one register:
-// the two K-neighbours of an m16n8k16 A fragment.  As in the K pass the codes enter the tensor pipe
-// as fp16 subnormals (one AND per pair of codes) and the scale - here per token and channel
-// group - is folded into the B operand: out[h][c] = sum_t (p_t * scale_t,G) * code_t,c + sum_t p_t *
-// zero_t,G, with p*scale carried exactly as hi + lo in neighbouring columns (2-bit pieces of 64 channels: columns are
-// two channel groups, hi and lo are two MMAs).
-// A tile has two phases.  In the first a lane computes exp(logit - max) of four tokens for two heads (one at 8 bits),
-// writes the probabilities out, and leaves the finished B operand - p*scale, hi and lo, of every head, token pair and
-// channel group - in shared memory in the order the MMAs want it: computed once, where forming it per step in every
-// lane that holds a column cost twice the arithmetic plus the packing of scales.  The second phase is ldmatrix, masks
-// and MMAs.
-// Codes are streamed through ONE tile buffer: the copy of a 16-token step of the next tile is issued when this tile's
-// step has been consumed, so a whole tile's work lies between a request and its use.
+// V tier, token-major rows of 128 channels.  Every warp of a CTA walks TILES of 64 consecutive tokens of one tier on its own
+// and keeps the output of all 128 channels x four heads in its accumulators from tile to tile, so nothing but the end of the
+// kernel needs the other warps.  (Tiles of 32 where the work is small.)  The contraction runs over tokens, 16 per step.  ldmatrix.trans over 8 token rows x 16 bytes
+// hands lane (g, tig) the 16-bit block g (2 / 4 / 8 channels) of two K-neighbours in one register: an m16n8k16 A fragment.
+// As in the K pass the codes enter the tensor pipe as fp16 subnormals (one AND per pair of codes) and the scale - here per
+// token and channel group - is folded into the B operand: out[h][c] = sum_t (p_t * scale_t,G) * code_t,c + sum_t p_t * zero_t,G,
+// with p*scale carried exactly as hi + lo in neighbouring columns (below 4 bits, where 16 bytes are 64 channels, the columns
+// are two groups of 32 and hi and lo are two MMAs).
+//
+// What bounds the kernel is the number of instructions and of shared-memory wavefronts per token, so:
+//  * A lane takes four consecutive tokens (a QUAD) of one head through the softmax: one 16-byte load of their logits, one
+//    8-byte store of their probabilities, one position fetched per lane and compared with its neighbours'.
+//  * The k-order of a step's tokens is that of its quads (k = 2i, 2i+1, 2i+8, 2i+9 are the tokens of quad i), so that a
+//    lane's own probabilities are a column of the B operand, and those of the other step one exchange away: the operand is
+//    formed in registers.  (Formed once and left in shared memory it took as many bytes there, both ways, as the codes.)
+//  * The scales and zeros of a quad are transposed to [group][token] once per tile: pairs as the B operand (and the A
+//    operand of the zero term) wants them.
+//  * One loop serves all widths, with a copy of the MMA part per width: the kernel's code (129 KB with a copy of
+//    everything) has to come from L2 into every SM that has not run it lately, 1 us per 64-byte line of a cold chain.
+// Codes are streamed through ONE tile buffer: the copy of 32 tokens of the next tile is issued when this tile's have been
+// consumed, so a whole tile's work lies between a request and its use.
 constexpr int V_MIN_CTAS = 4;  // CTAs per SM the V pass is compiled for (128 registers; PASS_SMEM is a quarter of an SM)
 constexpr int VWARPS = 4;
 constexpr int VTHREADS = VWARPS * 32;
-constexpr int V_ST = 72 * 4;                       // bytes per 16-token step of a B plane (64 words + 8: no bank conflicts)
-constexpr int V_PLANE = 4 * V_ST + 32;             // B plane of one channel group: 4 steps (+ 8 words, likewise)
+constexpr int V_TILE = 64;                 // tokens per tile of a warp at most
 
-template <int BITS>
-struct VTile {
-  static constexpr int PITCH = 16 * BITS;                  // bytes per token row: 128, 64, 32, 16
-  static constexpr int TOKENS = BITS == 8 ? 32 : 64;
-  static constexpr int STEPS = TOKENS / 16;
-  static constexpr int NPIECE = PITCH / 16;                // 16-byte pieces per row: 8, 4, 2, 1
-  static constexpr int HPL = BITS == 8 ? 1 : 2;            // heads per lane in the first phase
-  static constexpr int STEP_BYTES = 16 * PITCH;
-  static __device__ __forceinline__ uint32_t offset(uint32_t row, uint32_t c) {
-    if constexpr (PITCH == 128) {
-      return row * 128u + ((c ^ (row & 7u)) << 4);
-    } else if constexpr (PITCH == 64) {
-      return row * 64u + ((c ^ ((row >> 1) & 3u)) << 4);
-    } else if constexpr (PITCH == 32) {
-      return row * 32u + ((c ^ ((row >> 2) & 1u)) << 4);
-    } else {
-      return row * 16u;  // 1 bit: read with 2-byte loads
-    }
-  }
-};
-static_assert(VWARPS * VTile<8>::TOKENS == unit_tokens(8) && VWARPS * VTile<4>::TOKENS == unit_tokens(4), "a unit is a tile per warp");
-
-struct VTileShared {
-  unsigned char codes[4096];
-  unsigned char s[512];            // scales as in memory: [token][group]
-  unsigned char z[512];
-  unsigned char b[4 * V_PLANE];    // [group][step][2 * head + (hi, lo)][tig]{tokens 2tig, +1 | +8, +9}
-  unsigned char p[4 * 128];        // [step][head][tig]{the same token pairs}: B operand of the zero term
-  unsigned char zt[4 * 128];       // zeros, [group][step pair][tig]{even step, odd step, even step +8, odd step +8}
-};
-static_assert(sizeof(VTileShared) % 128 == 0, "tile buffers stay aligned");
-constexpr int V_STD = 2048;        // Gaussian-codebook tier (1 bit: 1 KB of codes): std in the same order, behind the codes
-struct VWarpShared {
-  VTileShared t;
-  float red[MAX_R4][D];            // partial output of the tiers that are done
-};
-
-// importance row emitted by the V pass: staging limits (positions + per-head halfs live in the warps' tile buffers)
+// importance row emitted by the V pass: staging limits (positions + per-head halfs live in the warps' buffers)
 constexpr int HS_TOKENS = 512;   // tokens per round
 constexpr int HS_HEADS = 32;     // query heads it is built for (beyond that a separate launch sums the heads)
-struct VShared {
-  float gm[MAX_R4], ginv[MAX_R4];          // max * log2(e) and 1 / sum of the query heads
-  unsigned is_last;
-  unsigned pad_[3 + 4];
-  alignas(128) VWarpShared w[VWARPS];  // (lane addresses are formed by XOR within 128 bytes)
+struct VWarpShared {
+  alignas(128) unsigned char codes[V_TILE * D];   // rows in k-order
+  unsigned char raw[2][V_TILE * 8];               // scales, zeros as in memory: [token][group]
+  unsigned char t[2][V_TILE * 8];                 // scales, zeros as [quad][group][token]; four groups: see v_swizzle
+  float red[MAX_R4][D];                           // output of the tiers that are done
 };
+struct VShared {
+  VWarpShared w[VWARPS];
+  float gm[MAX_R4], ginv[MAX_R4];                 // max * log2(e) and 1 / sum of the query heads
+  unsigned is_last;
+  unsigned pad_[3];
+};
+// Four groups: a quad is two 16-byte pieces; those of every second step lie the other way round (bank conflicts).
+__device__ __forceinline__ uint32_t v_swizzle(uint32_t byte) { return byte ^ ((byte >> 3) & 16u); }
+
+// Where the probabilities come from: the softmax of the scratch logits of four query heads, of two or one, or the caller.
+enum VMode { V_FOUR, V_FEWER, V_GIVEN };
+constexpr uint32_t V_NONE = 0xFFFFFFFFu;
+
+// A value that the compiler cannot work out again from thread and block indices: what a loop uses of them is computed once.
+__device__ __forceinline__ uint32_t keep(uint32_t v) { return __shfl_sync(0xffffffffu, v, threadIdx.x & 31); }
+
+// Logits (or given weights) of the lane's NP quads, whose positions are idx[0 .. 3] and idx[32 .. 35] below `left`; -inf (0) beyond.
+// dense (the same for the warp): they are quad[j] and the next three, quads of the scratch.  Two query heads: the lanes of the
+// other two read the first two's.
+template <int MODE, int NP>
+__device__ __forceinline__ void v_gather(const DecodeParams& P, const Where& w, int head, bool dense, const uint32_t (&quad)[NP], const int64_t* idx,
+                                         int left, float (&x)[NP][4]) {
+  const float* logits = P.logits + static_cast<int64_t>(w.bvh) * P.L * P.r4;
+  if (dense) {
+#pragma unroll
+    for (int j = 0; j < NP; ++j) {
+      if constexpr (MODE == V_FOUR) {
+        const float4 v = __ldcg(reinterpret_cast<const float4*>(logits) + (quad[j] + static_cast<uint32_t>(head)));
+        x[j][0] = v.x, x[j][1] = v.y, x[j][2] = v.z, x[j][3] = v.w;
+      } else {  // (rows of two heads start on 8-byte boundaries)
+        const float2* q = reinterpret_cast<const float2*>(logits) + (quad[j] + 2u * static_cast<uint32_t>(head & 1));
+        const float2 a = __ldcg(q), b = __ldcg(q + 1);
+        x[j][0] = a.x, x[j][1] = a.y, x[j][2] = b.x, x[j][3] = b.y;
+      }
+    }
+    return;
+  }
+#pragma unroll 1
+  for (int i = 0; i < 4 * NP; ++i) {
+    const int t = (i & 3) + 8 * (i & 4);
+    float v = MODE == V_GIVEN ? 0.f : -INFINITY;
+    const uint32_t pos = t < left ? __ldg(reinterpret_cast<const uint32_t*>(idx + t)) : V_NONE;
+    if (pos != V_NONE && HQKV_INDEX_OK(pos, P.L)) {
+      if constexpr (MODE == V_GIVEN) {
+        const int64_t row = (static_cast<int64_t>(w.b) * P.nh_q + w.h0 + head) * P.L;
+        if (head < P.r4) v = __half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(P.probs_in) + row + pos)));
+      } else {
+        v = __ldcg(logits + logit_at(pos, head & (P.r4 - 1), P.r4, P.L));
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4 * NP - 1; ++k) x[k >> 2][k & 3] = x[(k + 1) >> 2][(k + 1) & 3];
+    x[NP - 1][3] = v;
+  }
+}
+
+// The probabilities n of the lane's quads (see v_gather; tokens 0 1, 2 3 of each) to their positions of the row that starts
+// at `at` elements of rows.  whole: all rows' quads start on 8-byte boundaries.
+template <int NP>
+__device__ __forceinline__ void v_store_probs(__half* rows, uint32_t at, bool whole, bool dense, const uint32_t (&quad)[NP], const int64_t* idx,
+                                              int left, int L, uint32_t (&n)[NP][2]) {
+  if (dense) {
+#pragma unroll
+    for (int j = 0; j < NP; ++j) {
+      __half* a = rows + (at + quad[j]);
+      if (whole) {
+        *reinterpret_cast<uint2*>(a) = make_uint2(n[j][0], n[j][1]);
+      } else if ((reinterpret_cast<uintptr_t>(a) & 2u) == 0u) {
+        reinterpret_cast<uint32_t*>(a)[0] = n[j][0];
+        reinterpret_cast<uint32_t*>(a)[1] = n[j][1];
+      } else {
+        a[0] = __ushort_as_half(static_cast<unsigned short>(n[j][0]));
+        *reinterpret_cast<uint32_t*>(a + 1) = pack_hi_lo(n[j][0], n[j][1]);
+        a[3] = __ushort_as_half(static_cast<unsigned short>(n[j][1] >> 16));
+      }
+    }
+    return;
+  }
+#pragma unroll 1
+  for (int i = 0; i < 4 * NP; ++i) {
+    const int t = (i & 3) + 8 * (i & 4);
+    if (t < left) {
+      const uint32_t pos = __ldg(reinterpret_cast<const uint32_t*>(idx + t));
+      if (!HQKV_CHECKS_ENABLED || pos < static_cast<uint32_t>(L)) rows[at + pos] = __ushort_as_half(static_cast<unsigned short>(n[0][0]));
+    }
+#pragma unroll
+    for (int k = 0; k < 2 * NP - 1; ++k) n[k >> 1][k & 1] = pack_hi_lo(n[k >> 1][k & 1], n[(k + 1) >> 1][(k + 1) & 1]);
+    n[NP - 1][1] >>= 16;
+  }
+}
+
+// -C * std, to 22 bits, as two halfs
+__device__ __forceinline__ void v_normal_offset(uint32_t sd, uint32_t& hi, uint32_t& lo) {
+  const float2 t = __half22float2(u32_as_h2(sd));
+  const float x = -HQKV_NORMAL1_CENTER * t.x, y = -HQKV_NORMAL1_CENTER * t.y;
+  const __half2 h = __floats2half2_rn(x, y);
+  const float2 r = __half22float2(h);
+  hi = h2_as_u32(h), lo = pack_f16x2(x - r.x, y - r.y);
+}
 
 // field f of a 16-bit block as the fp16 subnormal code * 2^(k-24), k = v_shift(f)
 template <int BITS>
 __host__ __device__ constexpr int v_shift(int f) { return BITS == 8 ? 0 : BITS * f; }
 
-// The tiles of one warp: tokens t0 + warp * TOKENS, then every fourth tile up to t1.
-template <int BITS>
+// A CTA's way through the tiles of a tier, and a lane's places in them.
 struct VRun {
-  const unsigned char *codes, *s, *z;   // this lane's first 16 (8) bytes of the next tile to request
-  const int64_t* idx;                   // the lane's first token of the next tile whose positions are wanted
-  int left;                             // tokens from the next tile to request on (may be <= 0)
+  const unsigned char *codes, *s, *z;   // the CTA's next tiles to request
+  uint32_t src, dst;                    // the lane's first piece of a step's codes: offset from there, place in shared memory
+  uint32_t lm;                          // its ldmatrix row of the first step (1 bit: its first 2-byte block)
 };
-
-// Copy step st of the next tile; dst = where this lane's first piece goes in step 0 of the buffer.
-template <int BITS>
-__device__ __forceinline__ void v_request_step(const VRun<BITS>& r, uint32_t dst, int st, bool whole) {
-  using TL = VTile<BITS>;
-  const int lane = threadIdx.x & 31;
-  constexpr int N = (TL::STEP_BYTES + 511) / 512, RPI = 32 / TL::NPIECE;  // copies per lane: 4, 2, 1, 1; rows per copy
-  const unsigned char* src = r.codes + st * TL::STEP_BYTES;
-  dst += st * TL::STEP_BYTES;
-  if (TL::STEP_BYTES < 512 && lane >= TL::STEP_BYTES / 16) return;
+// Copy tokens [32 j, 32 j + 32) of the next tile.  WHOLE: all of them; otherwise those of which the tier has `left`.
+template <int BITS, bool WHOLE>
+__device__ __forceinline__ void v_request_pair(const VRun& r, int j, int left) {
+  constexpr int STEP = 256 * BITS, LP = BITS == 8 ? 3 : BITS == 4 ? 2 : BITS == 2 ? 1 : 0;   // bytes; log2 of the pieces of a row
+  constexpr int N = BITS >= 4 ? STEP / 512 : 1;                                             // copies per lane and step
+  const int k = (threadIdx.x & 31) >> LP;
+  const int first = (k & 16) + ((k & 6) << 1) + ((k >> 2) & 2) + (k & 1);   // the token in place k
+  // (one bit: a step is 16 pieces, so the two halves of the warp take a step each)
 #pragma unroll
-  for (int i = 0; i < N; ++i)
-    // (four rows on, bit 2 of the row changes: the other half of the swizzle at 8 bits)
-    if (whole || 16 * st + i * RPI + lane / TL::NPIECE < r.left)
-      cp_async_16((BITS == 8 ? dst ^ ((i & 1) * 64u) : dst) + i * 512, src + i * 512);
-}
-// scale / zero rows of a tile: ng halfs per token, contiguous, 8-byte pieces
-template <int BITS>
-__device__ __forceinline__ void v_request_scales(const VRun<BITS>& r, uint32_t s, uint32_t z, int ng2) {
-  const int lane = threadIdx.x & 31;
-  const int bytes = min(VTile<BITS>::TOKENS, r.left) * ng2;
+  for (int st = 0; st < (BITS == 1 ? 1 : 2); ++st)
 #pragma unroll
-  for (int o = 0; o < VTile<BITS>::TOKENS * 8; o += 256)
-    if (o + 8 * lane < bytes) {
-      cp_async_8(s + o + 8 * lane, r.s + o);
-      cp_async_8(z + o + 8 * lane, r.z + o);
+    for (int i = 0; i < N; ++i) {
+      // rows 4 i (8 bits) or 8 i (4 bits) on in k-order: tokens 0, 8, 2, 10 or 0, 2 on
+      constexpr int T8[4] = {0, 8, 2, 10};
+      const int tok = 32 * j + 16 * st + (BITS == 8 ? T8[i] : 2 * i);
+      const uint32_t at = (BITS == 8 ? r.dst ^ ((i & 1) * 64u) : r.dst) + (2 * j + st) * STEP + i * 512;
+      if (WHOLE || tok + first < left) cp_async_16(at, r.codes + r.src + tok * 16 * BITS);
     }
 }
-
-// First phase, lane map: 16-token step st, token pairs 2tq, 2tq+1 and +8, +9 of it, heads h0 .. h0 + HPL - 1.
-template <int BITS>
-struct VLane {
-  int st, tq, h0, tok;
-  __device__ __forceinline__ VLane() {
-    const int lane = threadIdx.x & 31;
-    constexpr int QUADS = VTile<BITS>::TOKENS / 4;
-    const int quad = lane & (QUADS - 1);
-    st = quad >> 2;
-    tq = quad & 3;
-    tok = 16 * st + 2 * tq;
-    h0 = (lane / QUADS) * VTile<BITS>::HPL;
-  }
-};
-__device__ __forceinline__ constexpr int v_tok(int j) { return (j & 1) + 8 * (j >> 1); }
-
-// positions (low words) of the lane's four tokens, `none` beyond the tier
-__device__ __forceinline__ void v_positions(uint32_t (&pos)[4], const int64_t* idx, int ntok, int tok, uint32_t none) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    pos[j] = none;
-    if (tok + v_tok(j) < ntok) pos[j] = __ldg(reinterpret_cast<const uint32_t*>(idx + v_tok(j)));
-  }
-}
-// logits (or given weights) of the lane's tokens and heads
-template <int HPL>
-__device__ __forceinline__ void v_gather(const DecodeParams& P, const Where& w, float (&x)[4][HPL], uint32_t (&pos)[4], int h0) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-    if (pos[j] != 0xFFFFFFFFu && !HQKV_INDEX_OK(pos[j], P.L)) pos[j] = 0xFFFFFFFFu;
-  if (P.probs_in) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int h = 0; h < HPL; ++h) {
-        const unsigned short* row = reinterpret_cast<const unsigned short*>(P.probs_in) +
-                                    (static_cast<int64_t>(w.b) * P.nh_q + w.h0 + h0 + h) * P.L;
-        x[j][h] = pos[j] != 0xFFFFFFFFu && h0 + h < P.r4 ? __half2float(__ushort_as_half(__ldcg(row + pos[j]))) : 0.f;
-      }
-    return;
-  }
-  const float* base = P.logits + static_cast<int64_t>(w.bvh) * P.L * P.r4 + h0;
-  if (P.r4 == MAX_R4) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float* p = base + static_cast<int64_t>(pos[j]) * MAX_R4;
-      if constexpr (HPL == 2) {
-        const float2 v = pos[j] != 0xFFFFFFFFu ? __ldcg(reinterpret_cast<const float2*>(p)) : make_float2(-INFINITY, -INFINITY);
-        x[j][0] = v.x;
-        x[j][1] = v.y;
-      } else {
-        x[j][0] = pos[j] != 0xFFFFFFFFu ? __ldcg(p) : -INFINITY;
-      }
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int h = 0; h < HPL; ++h)
-        x[j][h] = pos[j] != 0xFFFFFFFFu && h0 + h < P.r4 ? __ldcg(base + static_cast<int64_t>(pos[j]) * P.r4 + h) : -INFINITY;
+template <bool WHOLE, int NP>
+__device__ __forceinline__ void v_request_tile(int bits, const VRun& r, int left) {
+#pragma unroll 1
+  for (int j = 0; j < NP; ++j) {
+    if (bits == 4) v_request_pair<4, WHOLE>(r, j, left);
+    else if (bits == 2) v_request_pair<2, WHOLE>(r, j, left);
+    else if (bits == 8) v_request_pair<8, WHOLE>(r, j, left);
+    else if (bits == 1) v_request_pair<1, WHOLE>(r, j, left);
+    cp_async_commit();
   }
 }
 
-// Two neighbouring tokens' probabilities of one head (packed) to their positions.
-__device__ __forceinline__ void v_store_pair(__half* row, uint32_t p0, uint32_t p1, uint32_t packed, bool even) {
-  if (even) {  // consecutive positions that start on a 4-byte boundary
-    *reinterpret_cast<uint32_t*>(row + p0) = packed;
-    return;
-  }
-  if (p0 != 0xFFFFFFFFu) row[p0] = __ushort_as_half(static_cast<unsigned short>(packed));
-  if (p1 != 0xFFFFFFFFu) row[p1] = __ushort_as_half(static_cast<unsigned short>(packed >> 16));
-}
-
-// First phase of a tile (see above), any number of heads, tokens, groups; given weights.  x: logits of the lane's tokens.
-// Not inlined: partial tiles and unusual calls, whose code would only be in the way of the other tiles'.
-template <int BITS>
-__device__ __noinline__ void v_prepare_any(const DecodeParams& P, const Where& w, const VShared& sh, uint32_t tile,
-                                           const float (&x)[4][VTile<BITS>::HPL], const uint32_t (&pos)[4], int ntok, bool normal) {
-  const VLane<BITS> L;
-  using TL = VTile<BITS>;
-  constexpr int HPL = TL::HPL;
-  using S = VTileShared;
-  const uint32_t s_a = tile + offsetof(S, s), z_a = tile + offsetof(S, z), b_a = tile + offsetof(S, b), p_a = tile + offsetof(S, p),
-                 zt_a = tile + offsetof(S, zt), nt_a = tile + V_STD;
-  uint32_t p2[HPL][2];  // [head][token pair]
-#pragma unroll
-  for (int h = 0; h < HPL; ++h) {
-    const int head = L.h0 + h;
-    const bool on = head < P.r4;
-    if (P.probs_in) {
-      p2[h][0] = pack_f16x2(x[0][h], x[1][h]);
-      p2[h][1] = pack_f16x2(x[2][h], x[3][h]);
-    } else {
-      const float mh = sh.gm[on ? head : 0], inv = sh.ginv[on ? head : 0];
-      float e[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) e[j] = on ? fast_exp2(fmaf(x[j][h], LOG2E, -mh)) : 0.f;  // exp2(-inf) = 0 beyond the tile
-      p2[h][0] = pack_f16x2(e[0], e[1]);
-      p2[h][1] = pack_f16x2(e[2], e[3]);
-      if (on) {
-        const int64_t at = (static_cast<int64_t>(w.b) * P.nh_q + w.h0 + head) * P.L;
-        __half* row = P.weights + at;
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          const uint32_t a = pos[2 * k], b = pos[2 * k + 1];
-          const bool even = b == a + 1 && b != 0 && ((reinterpret_cast<uintptr_t>(row + a) & 3) == 0);
-          v_store_pair(row, a, b, pack_f16x2(e[2 * k] * inv, e[2 * k + 1] * inv), even);
-        }
-      }
-    }
-    sts64(p_a + L.st * 128 + (L.h0 + h) * 32 + L.tq * 8, p2[h][0], p2[h][1]);
-  }
-  // scales and zeros of the two token pairs, one word per channel group
-  const int ng = D >> P.gv_shift;
-  uint32_t s2[2][4], z2[2][4];
+// Tokens [32 j, 32 j + 32) of a tile into acc[M-tile] (channels x columns, see v_store_output): p[step][tokens 0 1, 2 3 of quad
+// tig] of the lane's head; st: the lane's quad in the scales of the tile's first step; rem: all ones in the lanes of the lo columns.
+template <int BITS, int GV>
+__device__ __forceinline__ void v_pair_mma(float (&acc)[8][4], const uint32_t (&p)[2][2], uint32_t lm, uint32_t st, uint32_t rem) {
+  constexpr int NG = D >> GV;
+  constexpr bool PAIR = BITS <= 2 && GV == 5;   // neighbouring columns are two groups
+  const int g = (threadIdx.x & 31) >> 2;
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
-    const int t = L.tok + 8 * k;
-    if (ng == 4) {
-      const uint4 sv = lds128(s_a + t * 8), zv = lds128(z_a + t * 8);
-      s2[k][0] = pack_lo16(sv.x, sv.z), s2[k][1] = pack_hi16(sv.x, sv.z), s2[k][2] = pack_lo16(sv.y, sv.w), s2[k][3] = pack_hi16(sv.y, sv.w);
-      z2[k][0] = pack_lo16(zv.x, zv.z), z2[k][1] = pack_hi16(zv.x, zv.z), z2[k][2] = pack_lo16(zv.y, zv.w), z2[k][3] = pack_hi16(zv.y, zv.w);
-    } else if (ng == 2) {
-      const uint2 sv = lds64(s_a + t * 4), zv = lds64(z_a + t * 4);
-      s2[k][0] = pack_lo16(sv.x, sv.y), s2[k][1] = pack_hi16(sv.x, sv.y);
-      z2[k][0] = pack_lo16(zv.x, zv.y), z2[k][1] = pack_hi16(zv.x, zv.y);
+    const uint32_t row = lm + k * 256 * BITS, sq = st + k * (32 * NG);
+    if constexpr (PAIR) {
+      uint32_t R[4];
+      if constexpr (BITS == 2) ldmatrix_x4_trans(R, row);   // (octet, piece): (0, 0), (1, 0), (0, 1), (1, 1)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {      // 64 channels
+        // (the lane's group of the two: 8 bytes on)
+        const uint2 s = lds64((k ? sq + ((c * 16) ^ 16) : sq + c * 16) + (rem & 8u));
+        const uint32_t h0 = h2_mul(p[k][0], s.x), h1 = h2_mul(p[k][1], s.y), l0 = h2_rem(p[k][0], s.x, h0), l1 = h2_rem(p[k][1], s.y, h1);
+        uint32_t lo0, lo1;
+        if constexpr (BITS == 2) {
+          lo0 = R[2 * c], lo1 = R[2 * c + 1];
+        } else {
+          const uint32_t tb = row + 8 * c;
+          lo0 = pack_lo16(lds16(tb), lds16(tb + 16)) >> (4 * (g >> 2));
+          lo1 = pack_lo16(lds16(tb + 128), lds16(tb + 144)) >> (4 * (g >> 2));
+        }
+        const uint32_t hi0 = lo0 >> 8, hi1 = lo1 >> 8;
+        uint32_t a[4][4];
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+          const uint32_t m = (BITS == 2 ? 0x00030003u : 0x00010001u) << v_shift<BITS>(f);
+          a[f][0] = lo0 & m, a[f][1] = hi0 & m, a[f][2] = lo1 & m, a[f][3] = hi1 & m;
+        }
+#pragma unroll
+        for (int f = 0; f < 4; ++f) mma16816(acc[4 * c + f], a[f][0], a[f][1], a[f][2], a[f][3], h0, h1);
+#pragma unroll
+        for (int f = 0; f < 4; ++f) mma16816(acc[4 * c + f], a[f][0], a[f][1], a[f][2], a[f][3], l0, l1);
+      }
     } else {
-      s2[k][0] = lds32(s_a + t * 2), z2[k][0] = lds32(z_a + t * 2);
-    }
-    if (ntok < TL::TOKENS) {  // the scales of tokens beyond the tile are not there
-      const uint32_t keep = (t < ntok ? 0xFFFFu : 0u) | (t + 1 < ntok ? 0xFFFF0000u : 0u);
+      uint32_t s[NG][2], b[NG][2];
+      if constexpr (NG == 1) {
+        const uint2 u = lds64(sq);
+        s[0][0] = u.x, s[0][1] = u.y;
+      } else {
 #pragma unroll
-      for (int G = 0; G < 4; ++G) {
-        s2[k][G] &= keep;
-        z2[k][G] &= keep;
-      }
-    }
-  }
-#pragma unroll
-  for (int G = 0; G < 4; ++G) {
-    if (G < ng) {
-      const uint32_t bp = b_a + G * V_PLANE + L.st * V_ST + L.h0 * 64 + L.tq * 8;
-#pragma unroll
-      for (int h = 0; h < HPL; ++h) {
-        const uint32_t h0 = h2_mul(p2[h][0], s2[0][G]), h1 = h2_mul(p2[h][1], s2[1][G]);
-        sts64(bp + h * 64, h0, h1);
-        sts64(bp + h * 64 + 32, h2_rem(p2[h][0], s2[0][G], h0), h2_rem(p2[h][1], s2[1][G], h1));
-      }
-      // A operand of the zero term: one of the lanes that share these tokens writes it
-      if (BITS == 8 ? L.h0 == G : L.h0 == 2 * (G & 1)) {
-        const uint32_t zp = G * 128 + (L.st >> 1) * 64 + L.tq * 16 + (L.st & 1) * 4;
-        sts32(zt_a + zp, z2[0][G]);
-        sts32(zt_a + zp + 8, z2[1][G]);
-        if (BITS == 1 && normal) {
-          sts32(nt_a + zp, s2[0][G]);
-          sts32(nt_a + zp + 8, s2[1][G]);
+        for (int i = 0; i < NG / 2; ++i) {
+          const uint4 u = lds128(NG == 4 && k ? sq + ((i * 16) ^ 16) : sq + i * 16);
+          s[2 * i][0] = u.x, s[2 * i][1] = u.y, s[2 * i + 1][0] = u.z, s[2 * i + 1][1] = u.w;
         }
       }
-    }
-  }
-}
-
-// A position that the bounds-check build has turned down (never in the regular build).
-__device__ __forceinline__ bool turned_down(uint32_t pos) { return HQKV_CHECKS_ENABLED && pos == 0xFFFFFFFFu; }
-
-// The same for a whole tile, four or two query heads and 128 >> GV channel groups known at compile time.  mh / inv: max *
-// log2(e) and 1 / sum of the lane's heads, wrow: their rows of probabilities (null: no such heads).
-template <int BITS, int GV>
-__device__ __forceinline__ void v_prepare(uint32_t tile, const float (&x)[4][VTile<BITS>::HPL], const uint32_t (&pos)[4],
-                                          const VLane<BITS>& L, const float (&mh)[VTile<BITS>::HPL],
-                                          const float (&inv)[VTile<BITS>::HPL], __half* const (&wrow)[VTile<BITS>::HPL], bool normal) {
-  using TL = VTile<BITS>;
-  using S = VTileShared;
-  constexpr int HPL = TL::HPL, NG = D >> GV;
-  uint32_t s2[2][NG], z2[2][NG];
+      // even columns: hi = fp16(p*s); odd columns (m = -p): the exact remainder p*s - hi
+      const uint32_t m0 = (p[k][0] ^ 0x80008000u) & rem, m1 = (p[k][1] ^ 0x80008000u) & rem;
 #pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const uint32_t at = tile + offsetof(S, s) + (L.tok + 8 * k) * NG * 2, to_z = offsetof(S, z) - offsetof(S, s);
-    if constexpr (NG == 4) {
-      const uint4 sv = lds128(at), zv = lds128(at + to_z);
-      s2[k][0] = pack_lo16(sv.x, sv.z), s2[k][1] = pack_hi16(sv.x, sv.z), s2[k][2] = pack_lo16(sv.y, sv.w), s2[k][3] = pack_hi16(sv.y, sv.w);
-      z2[k][0] = pack_lo16(zv.x, zv.z), z2[k][1] = pack_hi16(zv.x, zv.z), z2[k][2] = pack_lo16(zv.y, zv.w), z2[k][3] = pack_hi16(zv.y, zv.w);
-    } else if constexpr (NG == 2) {
-      const uint2 sv = lds64(at), zv = lds64(at + to_z);
-      s2[k][0] = pack_lo16(sv.x, sv.y), s2[k][1] = pack_hi16(sv.x, sv.y);
-      z2[k][0] = pack_lo16(zv.x, zv.y), z2[k][1] = pack_hi16(zv.x, zv.y);
-    } else {
-      s2[k][0] = lds32(at), z2[k][0] = lds32(at + to_z);
-    }
-  }
-  uint32_t p2[HPL][2], n2[HPL][2];  // [head][token pair]: exp(logit - max), probability
+      for (int G = 0; G < NG; ++G) b[G][0] = h2_fma(p[k][0], s[G][0], h2_mul(m0, s[G][0])), b[G][1] = h2_fma(p[k][1], s[G][1], h2_mul(m1, s[G][1]));
+      if constexpr (BITS >= 4) {
+        uint32_t R[4];
 #pragma unroll
-  for (int h = 0; h < HPL; ++h)
+        for (int cb = 0; cb < 4; ++cb) {   // 32 channels: two M-tiles
+          const int G = cb >> (GV - 5);
+          uint32_t a[2][4];
+          if constexpr (BITS == 8) {       // (octet, piece): (0, 2cb), (0, 2cb + 1), (1, 2cb), (1, 2cb + 1)
+            ldmatrix_x4_trans(R, row ^ (cb * 32u));
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const float e0 = fast_exp2(fmaf(x[2 * k][h], LOG2E, -mh[h])), e1 = fast_exp2(fmaf(x[2 * k + 1][h], LOG2E, -mh[h]));
-      p2[h][k] = pack_f16x2(e0, e1);
-      n2[h][k] = pack_f16x2(e0 * inv[h], e1 * inv[h]);
-    }
-  const bool adjacent = pos[1] == pos[0] + 1 && pos[3] == pos[2] + 1;
+            for (int i = 0; i < 4; ++i) {
+              a[0][i] = R[i] & 0x00FF00FFu;
+              a[1][i] = __byte_perm(R[i], 0u, 0x4341);
+            }
+          } else {                         // (octet, piece): (0, cb), (1, cb), (0, cb + 1), (1, cb + 1)
+            if ((cb & 1) == 0) ldmatrix_x4_trans(R, row ^ (cb * 16u));
 #pragma unroll
-  for (int h = 0; h < HPL; ++h) {
-    __half *a = wrow[h] + pos[0], *b = wrow[h] + pos[2];
-    if (wrow[h] == nullptr) {
-    } else if (turned_down(pos[0]) || turned_down(pos[1]) || turned_down(pos[2]) || turned_down(pos[3])) {
-      v_store_pair(wrow[h], pos[0], pos[1], n2[h][0], false);
-      v_store_pair(wrow[h], pos[2], pos[3], n2[h][1], false);
-    } else if (adjacent && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 3) == 0) {
-      *reinterpret_cast<uint32_t*>(a) = n2[h][0];
-      *reinterpret_cast<uint32_t*>(b) = n2[h][1];
-    } else {
-      a[0] = __ushort_as_half(static_cast<unsigned short>(n2[h][0]));
-      wrow[h][pos[1]] = __ushort_as_half(static_cast<unsigned short>(n2[h][0] >> 16));
-      b[0] = __ushort_as_half(static_cast<unsigned short>(n2[h][1]));
-      wrow[h][pos[3]] = __ushort_as_half(static_cast<unsigned short>(n2[h][1] >> 16));
-    }
-    sts64(tile + offsetof(S, p) + L.st * 128 + (L.h0 + h) * 32 + L.tq * 8, p2[h][0], p2[h][1]);
-  }
-  const uint32_t bp = tile + offsetof(S, b) + L.st * V_ST + L.h0 * 64 + L.tq * 8;
-  const uint32_t zp = tile + offsetof(S, zt) + (L.st >> 1) * 64 + L.tq * 16 + (L.st & 1) * 4;
+            for (int i = 0; i < 2; ++i) {
+              const uint32_t r = R[2 * (cb & 1) + i], rs = r >> 8;
+              a[0][2 * i] = r & 0x000F000Fu, a[1][2 * i] = r & 0x00F000F0u;
+              a[0][2 * i + 1] = rs & 0x000F000Fu, a[1][2 * i + 1] = rs & 0x00F000F0u;
+            }
+          }
 #pragma unroll
-  for (int G = 0; G < NG; ++G) {
-#pragma unroll
-    for (int h = 0; h < HPL; ++h) {
-      const uint32_t h0 = h2_mul(p2[h][0], s2[0][G]), h1 = h2_mul(p2[h][1], s2[1][G]);
-      sts64(bp + G * V_PLANE + h * 64, h0, h1);
-      sts64(bp + G * V_PLANE + h * 64 + 32, h2_rem(p2[h][0], s2[0][G], h0), h2_rem(p2[h][1], s2[1][G], h1));
-    }
-    // A operand of the zero term: one of the lanes that share these tokens writes it
-    if (BITS == 8 ? L.h0 == G : L.h0 == 2 * (G & 1)) {
-      sts32(zp + G * 128, z2[0][G]);
-      sts32(zp + G * 128 + 8, z2[1][G]);
-      if (BITS == 1 && normal) {
-        sts32(zp + G * 128 + V_STD - offsetof(S, zt), s2[0][G]);
-        sts32(zp + G * 128 + V_STD - offsetof(S, zt) + 8, s2[1][G]);
-      }
-    }
-  }
-}
-
-// Four or two query heads: logits of the lane's tokens without conditions (position 0 stands in beyond the tier).  The
-// bounds-check build leaves out positions that are not below `limit`: no logit, and no probability is stored for them.
-template <int HPL>
-__device__ __forceinline__ void v_gather4(float (&x)[4][HPL], uint32_t (&pos)[4], const float* base, uint32_t heads, int limit) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    if (!HQKV_INDEX_OK(pos[j], limit)) {
-      pos[j] = 0xFFFFFFFFu;
-#pragma unroll
-      for (int h = 0; h < HPL; ++h) x[j][h] = -INFINITY;
-      continue;
-    }
-    const float* p = base + static_cast<uint64_t>(pos[j]) * heads;
-    if constexpr (HPL == 2) {
-      const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
-      x[j][0] = v.x;
-      x[j][1] = v.y;
-    } else {
-      x[j][0] = __ldcg(p);
-    }
-  }
-}
-
-// Second phase: one 16-token step of a tile into acc[M-tile] (channels x columns, see v_store_output).  lm = this lane's
-// ldmatrix row of the step, piece 0 or 1 (1 bit: its first 2-byte block); bl = the step in B plane 0 at this lane's column.
-template <int BITS, int GV>
-__device__ __forceinline__ void v_step(float (&acc)[8][4], uint32_t lm, uint32_t bl, int gv_runtime) {
-  const int gv_shift = GV ? GV : gv_runtime;
-  if constexpr (BITS >= 4) {
-    uint32_t R[4];
-#pragma unroll
-    for (int cb = 0; cb < 4; ++cb) {   // 32 channels: one channel group, two M-tiles
-      uint32_t a[2][4];
-      if constexpr (BITS == 8) {
-        ldmatrix_x4_trans(R, lm ^ (cb * 32u));
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          a[0][k] = R[k] & 0x00FF00FFu;
-          a[1][k] = __byte_perm(R[k], 0u, 0x4341);
+          for (int i = 0; i < 2; ++i) mma16816(acc[2 * cb + i], a[i][0], a[i][1], a[i][2], a[i][3], b[G][0], b[G][1]);
         }
       } else {
-        if ((cb & 1) == 0) ldmatrix_x4_trans(R, lm ^ (cb * 16u));
+        uint32_t R[4];
+        if constexpr (BITS == 2) ldmatrix_x4_trans(R, row);
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          const uint32_t r = R[2 * k + (cb & 1)], rs = r >> 8;
+        for (int c = 0; c < 2; ++c) {      // 64 channels of one group
+          const int G = NG == 2 ? c : 0;
+          uint32_t lo0, lo1;
+          if constexpr (BITS == 2) {
+            lo0 = R[2 * c], lo1 = R[2 * c + 1];
+          } else {
+            const uint32_t tb = row + 8 * c;
+            lo0 = pack_lo16(lds16(tb), lds16(tb + 16)) >> (4 * (g >> 2));
+            lo1 = pack_lo16(lds16(tb + 128), lds16(tb + 144)) >> (4 * (g >> 2));
+          }
+          const uint32_t hi0 = lo0 >> 8, hi1 = lo1 >> 8;
 #pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            a[i][2 * k] = r & (0x000F000Fu << (4 * i));
-            a[i][2 * k + 1] = rs & (0x000F000Fu << (4 * i));
+          for (int f = 0; f < 4; ++f) {
+            const uint32_t m = (BITS == 2 ? 0x00030003u : 0x00010001u) << v_shift<BITS>(f);
+            mma16816(acc[4 * c + f], lo0 & m, hi0 & m, lo1 & m, hi1 & m, b[G][0], b[G][1]);
           }
         }
       }
-      const uint2 b = lds64(bl + (cb >> (gv_shift - 5)) * V_PLANE);
-#pragma unroll
-      for (int i = 0; i < 2; ++i) mma16816(acc[2 * cb + i], a[i][0], a[i][1], a[i][2], a[i][3], b.x, b.y);
-    }
-  } else {
-    const int g = (threadIdx.x & 31) >> 2;
-    uint32_t R[4];
-    if constexpr (BITS == 2) ldmatrix_x4_trans(R, lm);
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {      // 64 channels: two channel groups of 32 in neighbouring columns
-      uint32_t lo0, lo1;
-      if constexpr (BITS == 2) {
-        lo0 = R[c], lo1 = R[2 + c];
-      } else {  // block 4c + (g & 3) of tokens 2tig, 2tig+1 (+8, +9) with 2-byte loads
-        const uint32_t tb = lm + 8 * c;
-        lo0 = pack_lo16(lds16(tb), lds16(tb + 16)) >> (4 * (g >> 2));
-        lo1 = pack_lo16(lds16(tb + 128), lds16(tb + 144)) >> (4 * (g >> 2));
-      }
-      const uint32_t hi0 = lo0 >> 8, hi1 = lo1 >> 8;
-      // column n = g: head n >> 1, channel group of channels 64c + 32*(n & 1)
-      const uint32_t bp = bl + ((2 * c + (g & 1)) >> (gv_shift - 5)) * V_PLANE;
-      const uint2 bh = lds64(bp), bl2 = lds64(bp + 32);
-      uint32_t a[4][4];
-#pragma unroll
-      for (int f = 0; f < 4; ++f) {
-        const uint32_t m = BITS == 2 ? 0x00030003u << (2 * f) : 0x00010001u << f;
-        a[f][0] = lo0 & m, a[f][1] = hi0 & m, a[f][2] = lo1 & m, a[f][3] = hi1 & m;
-      }
-#pragma unroll
-      for (int f = 0; f < 4; ++f) mma16816(acc[4 * c + f], a[f][0], a[f][1], a[f][2], a[f][3], bh.x, bh.y);
-#pragma unroll
-      for (int f = 0; f < 4; ++f) mma16816(acc[4 * c + f], a[f][0], a[f][1], a[f][2], a[f][3], bl2.x, bl2.y);
     }
   }
 }
 
-// Accumulators and zero term (lane: channel group g, head tig) added to red[head tig][channel] (`fresh`: nothing is in there yet).
+// The MMA part of a tile: pairs of steps, each refilled with the next tile's tokens when it is done.
+template <int BITS, int GV, int NP>
+__device__ __forceinline__ void v_tile(float (&acc)[8][4], const uint32_t (&p)[NP][2], const VRun& r, uint32_t t_s, uint32_t rem, bool refill) {
+  const bool odd = threadIdx.x & 4;
+  uint32_t p0 = p[0][0], p1 = p[0][1];
+#pragma unroll 1
+  for (int j = 0; j < NP; ++j) {
+    // own probabilities are those of step lane bit 2 (of the pair) of the lane's head; the other step's are four lanes away
+    const uint32_t a = __shfl_xor_sync(0xffffffffu, p0, 4), b = __shfl_xor_sync(0xffffffffu, p1, 4);
+    const uint32_t ps[2][2] = {{odd ? a : p0, odd ? b : p1}, {odd ? p0 : a, odd ? p1 : b}};
+    cp_async_wait<NP>();
+    __syncwarp();
+    v_pair_mma<BITS, GV>(acc, ps, r.lm + j * 512 * BITS, t_s + j * (64 * (D >> GV)), rem);
+    // (the MMAs have used the codes, and keep the warp together: no lane still reads them)
+    if (refill) v_request_pair<BITS, true>(r, j, 0);
+    cp_async_commit();
+    p0 = p[NP - 1][0], p1 = p[NP - 1][1];
+  }
+}
+
+// Accumulators and zero term (lane: channel rows g, head tig) added to red[head tig][channel].
 //   8 / 4 bits: M-tile 2*cb + i: rows g / g+8 = channels 32cb + 2g + i / + 16 (8 bits), 32cb + 4g + i / + 2 (4 bits);
 //               a head's neighbouring columns are hi and lo
-//   2 bits:     M-tile 4c + f: 64c + 8g + f / + 4;   1 bit: 64c + 16(g&3) + 4(g>>2) + f / + 8;   the columns are two
-//               channel groups, a row keeps its own
-template <int BITS>
-__device__ __forceinline__ void v_store_output(float (*red)[D], const float (&acc)[8][4], float gain, float zt, int gv_shift, bool fresh) {
+//   2 bits:     M-tile 4c + f: 64c + 8g + f / + 4;   1 bit: 64c + 16(g&3) + 4(g>>2) + f / + 8; in groups of 32 the columns
+//               are two groups, a row keeps its own
+// zt: zero term of channel group g % groups, head tig.
+template <int GV>
+__device__ __forceinline__ void v_store_output(float (*red)[D], const float (&acc)[8][4], int bits, float gain, float zt) {
   const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
+  const bool wide = bits >= 4, pair = GV == 5 && !wide;
+  const int second = bits == 2 ? g >> 2 : (g & 3) >> 1;                   // which group of the 64 channels the lane's rows are in
+  const int other = bits == 8 ? 16 : bits == 4 ? 2 : bits == 2 ? 4 : 8;   // from rows g to rows g + 8
+  float* out = red[tig] + (bits == 8 ? 2 * g : bits == 4 ? 4 * g : bits == 2 ? 8 * g : 16 * (g & 3) + 4 * (g >> 2));
+  const float base = static_cast<float>(1 << 24) * gain, step = bits == 8 ? 1.f : bits == 4 ? 0x1p-4f : bits == 2 ? 0x1p-2f : 0x1p-1f;
 #pragma unroll
   for (int mt = 0; mt < 8; ++mt) {
-    const int f = BITS >= 4 ? mt & 1 : mt & 3;
-    const float unscale = static_cast<float>(1 << 24) / static_cast<float>(1 << v_shift<BITS>(f)) * gain;
-    // the zero term of the M-tile's channels: 32-channel block mt >> 1 (8 / 4 bits), or the one this lane's rows are in
-    const int block = BITS >= 4 ? mt >> 1 : 2 * (mt >> 2) + (BITS == 2 ? g >> 2 : (g & 3) >> 1);
-    const float z = __shfl_sync(0xffffffffu, zt, 4 * (block >> (gv_shift - 5)) + tig);
+    const int f = wide ? mt & 1 : mt & 3;
+    const float unscale = base * (f == 0 ? 1.f : f == 1 ? step : f == 2 ? step * step : step * step * step);   // 2^24 / 2^v_shift(f)
+    const int block = wide ? mt >> 1 : 2 * (mt >> 2) + second;   // 32 channels
+    const float z = __shfl_sync(0xffffffffu, zt, 4 * (block >> (GV - 5)) + tig);
+    float* o = out + (wide ? 32 * (mt >> 1) : 64 * (mt >> 2)) + f;
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       const float* a = &acc[mt][2 * r];
-      int ch;
-      float v;
-      if constexpr (BITS >= 4) {
-        ch = 32 * (mt >> 1) + (BITS == 8 ? 2 * g + 16 * r : 4 * g + 2 * r) + f;
-        v = a[0] + a[1];
-      } else {
-        ch = 64 * (mt >> 2) + (BITS == 2 ? 8 * g + 4 * r : 16 * (g & 3) + 4 * (g >> 2) + 8 * r) + f;
-        v = (BITS == 2 ? g >> 2 : (g & 3) >> 1) ? a[1] : a[0];
-      }
-      const float y = fmaf(v, unscale, z);
-      red[tig][ch] = fresh ? y : red[tig][ch] + y;
+      o[r ? other : 0] += fmaf(pair ? (second ? a[1] : a[0]) : a[0] + a[1], unscale, z);
     }
   }
-}
-
-// Everything a warp does for its tiles of tokens [t0, t1) of a quantised V tier.  UNROLL: steps of the inner loop (one where
-// a CTA's code is that of several tiers: they run side by side on an SM and the instruction cache does not hold more).  `fold` folds the
-// K pass's softmax pairs (once per CTA; all its warps take part).
-template <int BITS, int GV, int UNROLL, typename Fold>
-__device__ __forceinline__ void v_run(const DecodeParams& P, const TierDev& T, VShared& sh, const Where& w, int t0, int t1,
-                                      Fold fold, bool& fresh) {
-  using TL = VTile<BITS>;
-  using S = VTileShared;
-  constexpr int STRIDE = VWARPS * TL::TOKENS;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tig = lane & 3;
-  VWarpShared& ws = sh.w[warp];
-  const uint32_t tile = smem_u32(&ws.t);
-  const uint32_t codes = tile + offsetof(S, codes), b_a = tile + offsetof(S, b), s_a = tile + offsetof(S, s), z_a = tile + offsetof(S, z);
-  constexpr bool FAST = GV != 0;
-  constexpr uint32_t NONE = FAST ? 0u : 0xFFFFFFFFu;
-  const int gv_shift = GV ? GV : P.gv_shift;
-  const int ng2 = (D >> gv_shift) * 2;
-  const bool normal = BITS == 1 && T.normal != 0;
-  const VLane<BITS> L;
-  const int first = t0 + warp * TL::TOKENS;
-  const int64_t tok0 = static_cast<int64_t>(w.bh) * T.n_v + first;
-  VRun<BITS> r;
-  r.codes = reinterpret_cast<const unsigned char*>(T.v_data) + tok0 * TL::PITCH + lane * 16;
-  r.s = reinterpret_cast<const unsigned char*>(T.v_scale) + tok0 * ng2 + lane * 8;
-  r.z = reinterpret_cast<const unsigned char*>(T.v_zero) + tok0 * ng2 + lane * 8;
-  r.idx = T.v_idx + first + L.tok;
-  r.left = t1 - first;
-  // lane addresses: first piece of a step's copy; ldmatrix row - matrices (token octet, piece) (0, c), (0, c'), (1, c),
-  // (1, c') - or 2-byte block; column of the B planes
-  const uint32_t dst = codes + TL::offset(lane / TL::NPIECE, lane % TL::NPIECE);
-  const uint32_t lm = BITS == 1 ? codes + 2 * tig * 16 + 2 * (g & 3) : codes + TL::offset(8 * (lane >> 4) + (lane & 7), (lane >> 3) & 1);
-  const uint32_t bl = b_a + (BITS >= 4 ? lane * 8 : (g >> 1) * 64 + tig * 8);
-  auto advance = [&]() {
-    r.codes += STRIDE * TL::PITCH;
-    r.s += STRIDE * ng2;
-    r.z += STRIDE * ng2;
-    r.left -= STRIDE;
-  };
-  __syncwarp();  // (the buffers may have served another tier)
-  // requests that read only the cache go out before the K pass is known to be complete
-  v_request_scales<BITS>(r, s_a, z_a, ng2);
-  cp_async_commit();
-#pragma unroll
-  for (int st = 0; st < TL::STEPS; ++st) {
-    v_request_step<BITS>(r, dst, st, false);
-    cp_async_commit();
-  }
-  uint32_t pos[4];
-  v_positions(pos, r.idx, r.left, L.tok, NONE);
-  advance();
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  float x[4][TL::HPL];
-  // With two query heads the lanes of the other two take the first two's logits to a probability of 0 and write none.
-  const float* lrow = P.logits + static_cast<int64_t>(w.bvh) * P.L * P.r4 + (L.h0 & (P.r4 - 1));
-  auto gather = [&]() {
-    if constexpr (FAST) v_gather4<TL::HPL>(x, pos, lrow, static_cast<uint32_t>(P.r4), P.L);
-    else v_gather<TL::HPL>(P, w, x, pos, L.h0);
-  };
-  gather();
-  fold();
-  float mh[TL::HPL], inv[TL::HPL];
-  __half* wrow[TL::HPL];
-  if constexpr (FAST) {
-#pragma unroll
-    for (int h = 0; h < TL::HPL; ++h) {
-      const bool on = L.h0 < P.r4;
-      mh[h] = on ? sh.gm[L.h0 + h] : INFINITY;
-      inv[h] = on ? sh.ginv[L.h0 + h] : 0.f;
-      wrow[h] = !on ? nullptr : P.weights + (static_cast<int64_t>(w.b) * P.nh_q + w.h0 + L.h0 + h) * P.L;
-    }
-  }
-  float acc[8][4], za[4] = {0.f, 0.f, 0.f, 0.f}, zb[4] = {0.f, 0.f, 0.f, 0.f};
-  float na[4] = {0.f, 0.f, 0.f, 0.f}, nb[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-  for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-  const int zg = g & ((D >> gv_shift) - 1);  // zero-term row g = group g (rows beyond the groups repeat)
-#pragma unroll 1
-  for (int left = t1 - first; left > 0; left -= STRIDE) {
-    const int ntok = min(TL::TOKENS, left);
-    uint32_t next[4];
-    r.idx += STRIDE;
-    v_positions(next, r.idx, r.left, L.tok, NONE);
-    cp_async_wait<TL::STEPS>();  // scales and zeros (the codes of the tile may still be on their way)
-    __syncwarp();
-    if (FAST && ntok == TL::TOKENS) {
-      if constexpr (FAST) v_prepare<BITS, GV>(tile, x, pos, L, mh, inv, wrow, normal);
-    } else {
-      float xa[4][TL::HPL];
-      uint32_t pa[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const bool in = L.tok + v_tok(j) < ntok;
-        pa[j] = in ? pos[j] : 0xFFFFFFFFu;
-#pragma unroll
-        for (int h = 0; h < TL::HPL; ++h) xa[j][h] = in ? x[j][h] : P.probs_in ? 0.f : -INFINITY;
-      }
-      v_prepare_any<BITS>(P, w, sh, tile, xa, pa, ntok, normal);
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) pos[j] = next[j];
-    gather();
-    __syncwarp();  // the B operand is complete, the scale buffers are free
-    v_request_scales<BITS>(r, s_a, z_a, ng2);
-    cp_async_commit();
-#pragma unroll
-    for (int sp = 0; sp < TL::STEPS / 2; ++sp) {
-      const uint4 z4 = lds128(tile + offsetof(S, zt) + zg * 128 + sp * 64 + tig * 16);
-      const uint2 pe = lds64(tile + offsetof(S, p) + (2 * sp) * 128 + (g >> 1) * 32 + tig * 8);
-      const uint2 po = lds64(tile + offsetof(S, p) + (2 * sp + 1) * 128 + (g >> 1) * 32 + tig * 8);
-      mma16816(za, z4.x, z4.y, z4.z, z4.w, pe.x, pe.y);   // rows 0-7: the even step's tokens
-      mma16816(zb, z4.x, z4.y, z4.z, z4.w, po.x, po.y);   // rows 8-15: the odd step's
-      if (BITS == 1 && normal) {
-        const uint4 n4 = lds128(tile + V_STD + zg * 128 + sp * 64 + tig * 16);
-        mma16816(na, n4.x, n4.y, n4.z, n4.w, pe.x, pe.y);
-        mma16816(nb, n4.x, n4.y, n4.z, n4.w, po.x, po.y);
-      }
-    }
-    const bool whole = r.left >= TL::TOKENS;
-  #pragma unroll UNROLL
-    for (int st = 0; st < TL::STEPS; ++st) {
-      cp_async_wait<TL::STEPS>();
-      __syncwarp();
-      v_step<BITS, GV>(acc, lm + st * TL::STEP_BYTES, bl + st * V_ST, gv_shift);
-      // (the MMAs have used the step's codes, and keep the warp together: no lane still reads them)
-      v_request_step<BITS>(r, dst, st, whole);
-      cp_async_commit();
-    }
-    advance();
-    __syncwarp();
-  }
-  cp_async_wait<0>();
-  __syncwarp();
-  // value = std * C * (2 code - 1) + mean: the code-free term is sum_t p (mean - C std)
-  const float zt = za[0] + zb[2] + (normal ? -HQKV_NORMAL1_CENTER * (na[0] + nb[2]) : 0.f);  // channel group g, head tig
-  v_store_output<BITS>(ws.red, acc, normal ? 2.f * HQKV_NORMAL1_CENTER : 1.f, zt, gv_shift, fresh);
-  fresh = false;
 }
 
 // fp16 tier and residual window, token-major rows [n][D] halfs: one 16-token step per warp straight
-// from global memory; B = p, column n = head n.
-__device__ __forceinline__ void v_plain_tile(const DecodeParams& P, const TierDev& T, VShared& sh, VWarpShared& ws, const Where& w,
+// from global memory; B = p, column n = head n.  The result is added to red.  ps: 128 bytes of shared memory.
+template <int MODE>
+__device__ __forceinline__ void v_plain_tile(const DecodeParams& P, const TierDev& T, const VShared& sh, __half* ps, float (*red)[D], const Where& w,
                                              int t0, int ntok, bool is_res) {
   const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-  const uint4* base = reinterpret_cast<const uint4*>(T.v_data) + static_cast<int64_t>(w.bh) * T.n_v * 16;
-  uint4 v[4][2];
+  const uint2* base = reinterpret_cast<const uint2*>(T.v_data) + (static_cast<int64_t>(w.bh) * T.n_v + t0) * 32;
+  uint2 v[4][2];   // tokens 2tig, +1, +8, +9 x four channels of two rows of pieces
+  auto load = [&](int half) {
 #pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    const int tl = 2 * tig + (p & 1) + (p >> 1) * 8;
-    const int64_t tok = t0 + min(tl, ntok - 1);
+    for (int p = 0; p < 4; ++p) {
+      const int tl = min(2 * tig + (p & 1) + (p >> 1) * 8, ntok - 1);
 #pragma unroll
-    for (int s = 0; s < 2; ++s) v[p][s] = ld_stream(base + tok * 16 + s * 8 + g);
-  }
-  __half* ps = reinterpret_cast<__half*>(ws.t.p);  // [head][16 tokens]
+      for (int s = 0; s < 2; ++s) v[p][s] = ld_stream(base + tl * 32 + (2 * half + s) * 8 + g);
+    }
+  };
+  load(0);
   {
     const int t = lane & 15;
     uint32_t pos = 0xFFFFFFFFu;
@@ -1678,10 +1451,10 @@ __device__ __forceinline__ void v_plain_tile(const DecodeParams& P, const TierDe
       const int64_t at = (static_cast<int64_t>(w.b) * P.nh_q + w.h0 + h) * P.L + pos;
       __half e = __float2half_rn(0.f);
       if (on) {
-        if (P.probs_in) {
+        if constexpr (MODE == V_GIVEN) {
           e = __ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(P.probs_in) + at));
         } else {
-          const float x = __ldcg(P.logits + (static_cast<int64_t>(w.bvh) * P.L + pos) * P.r4 + h);
+          const float x = __ldcg(P.logits + static_cast<int64_t>(w.bvh) * P.L * P.r4 + logit_at(pos, h, P.r4, P.L));
           const float f = fast_exp2(fmaf(x, LOG2E, -sh.gm[h]));
           e = __float2half_rn(f);
           P.weights[at] = __float2half_rn(f * sh.ginv[h]);
@@ -1691,37 +1464,34 @@ __device__ __forceinline__ void v_plain_tile(const DecodeParams& P, const TierDe
     }
   }
   __syncwarp();
-  float acc[8][4];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
   uint32_t b0 = 0u, b1 = 0u;
   if (g < MAX_R4) {
     b0 = *reinterpret_cast<const uint32_t*>(ps + g * 16 + 2 * tig);
     b1 = *reinterpret_cast<const uint32_t*>(ps + g * 16 + 2 * tig + 8);
   }
-  auto word = [](const uint4& u, int s) { return s == 0 ? u.x : s == 1 ? u.y : s == 2 ? u.z : u.w; };
 #pragma unroll
-  for (int s = 0; s < 4; ++s)
+  for (int half = 0; half < 2; ++half) {
+    if (half) load(1);
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {  // M-tile 2s + k: half k of word s of the lane's eight channels
+    for (int k = 0; k < 4; ++k) {  // M-tile: half k of the lane's four channels
       uint32_t a[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {  // fragment register: row slot q & 1, token pair q >> 1
-        const uint32_t x0 = word(v[2 * (q >> 1)][q & 1], s), x1 = word(v[2 * (q >> 1) + 1][q & 1], s);
-        a[q] = k ? pack_hi16(x0, x1) : pack_lo16(x0, x1);
+        const uint2 x0 = v[2 * (q >> 1)][q & 1], x1 = v[2 * (q >> 1) + 1][q & 1];
+        const uint32_t u0 = k < 2 ? x0.x : x0.y, u1 = k < 2 ? x1.x : x1.y;
+        a[q] = k & 1 ? pack_hi16(u0, u1) : pack_lo16(u0, u1);
       }
-      mma16816(acc[2 * s + k], a[0], a[1], a[2], a[3], b0, b1);
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+      mma16816(acc, a[0], a[1], a[2], a[3], b0, b1);
+      if (tig < 2) {  // rows g, g + 8: channels of the two rows of pieces; columns 2tig, 2tig+1 = heads (4-7: none)
+#pragma unroll
+        for (int s = 0; s < 2; ++s)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) red[2 * tig + e][4 * ((2 * half + s) * 8 + g) + k] += acc[s * 2 + e];
+      }
     }
-  __syncwarp();
-  // M-tile mt, slot s: channel 8*(8s + g) + mt; columns 2tig, 2tig+1 = heads (4-7: none)
-  if (tig < 2) {
-#pragma unroll
-    for (int mt = 0; mt < 8; ++mt)
-#pragma unroll
-      for (int s = 0; s < 2; ++s)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) ws.red[2 * tig + e][8 * (s * 8 + g) + mt] += acc[mt][s * 2 + e];
   }
+  __syncwarp();
 }
 
 // Cross-GPU barrier of one call, run by up to `world` threads of one CTA: thread r tells peer r "my stores
@@ -1755,33 +1525,34 @@ __device__ __forceinline__ void peer_barrier_device(unsigned* const* pad, int ra
   if (r == 0) *call_no = n;
 }
 
-static_assert(sizeof(VWarpShared) * VWARPS >= HS_TOKENS * 4 + HS_TOKENS * HS_HEADS * 2, "importance-row staging fits the tile buffers");
+static_assert(offsetof(VShared, gm) >= HS_TOKENS * 4 + HS_TOKENS * HS_HEADS * 2, "importance-row staging fits the tile buffers");
 // Importance row of n tokens from token c0 of a tier on, run by the last CTA to finish their grid row (not inlined: its registers are its own).
 __device__ __noinline__ void head_sum_chunk(const DecodeParams& P, const TierDev& T, VShared& sh, int c0, int n, bool is_res) {
   const int tid = threadIdx.x;
   __threadfence();
   __syncthreads();  // the round before is done with the staging buffers
-  // The warps' tile buffers are free by now: they stage the chunk's positions and, per token and head, the sum
+  // The warps' buffers are free by now: they stage the chunk's positions and, per token and head, the sum
   // over the batch rounded to fp16.  Loads first, all of them independent: an item is (token, eight heads),
   // four items - 32 gathers per batch entry - are in flight per thread; then one thread per token adds the
   // heads in head order.
-  uint32_t* pos_s = reinterpret_cast<uint32_t*>(sh.w);                       // [HS_TOKENS]
+  uint32_t* pos_s = reinterpret_cast<uint32_t*>(&sh);                        // [HS_TOKENS]
   __half* stage = reinterpret_cast<__half*>(pos_s + HS_TOKENS);              // [HS_TOKENS][HS_HEADS]
   for (int t = tid; t < n; t += VTHREADS)
     pos_s[t] = is_res ? static_cast<uint32_t>(P.L - T.n_v + c0 + t) : static_cast<uint32_t>(T.v_idx[c0 + t]);
   __syncthreads();
+  constexpr int ITEMS = 4;
   const int nhq = P.nh_q, ngr = (nhq + 7) >> 3, items = n * ngr;
   const unsigned short* w = reinterpret_cast<const unsigned short*>(P.weights);
-  for (int base = tid; base < items; base += 4 * VTHREADS) {
-    float ob[4][8];
+  for (int base = tid; base < items; base += ITEMS * VTHREADS) {
+    float ob[ITEMS][8];
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
+    for (int q = 0; q < ITEMS; ++q)
 #pragma unroll
       for (int j = 0; j < 8; ++j) ob[q][j] = 0.f;
     for (int bb = 0; bb < P.B; ++bb) {
-      unsigned short v[4][8];
+      unsigned short v[ITEMS][8];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
+      for (int q = 0; q < ITEMS; ++q) {
         const int item = base + q * VTHREADS;
         const int gq = item / n, t = item - gq * n;  // token fastest: neighbouring threads read neighbouring positions
         const bool live = item < items && HQKV_INDEX_OK(pos_s[t], P.L);
@@ -1793,12 +1564,12 @@ __device__ __noinline__ void head_sum_chunk(const DecodeParams& P, const TierDev
         }
       }
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
+      for (int q = 0; q < ITEMS; ++q)
 #pragma unroll
         for (int j = 0; j < 8; ++j) ob[q][j] = __fadd_rn(ob[q][j], __half2float(__ushort_as_half(v[q][j])));
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < ITEMS; ++q) {
       const int item = base + q * VTHREADS;
       if (item >= items) continue;
       const int gq = item / n, t = item - gq * n;
@@ -1815,107 +1586,309 @@ __device__ __noinline__ void head_sum_chunk(const DecodeParams& P, const TierDev
   }
 }
 
-// GV: log2 of the channel group, with four or two query heads per CTA and the softmax of the scratch logits; 0: everything else.
-// ONE_TIER: no CTA has units of two tiers.
-// At 128 registers the one-tier kernels spill 24 - 40 bytes a thread and the others 136 - 160 (-Xptxas -v), around the loops
-// over tiles: local loads and stores are 0.1 % of a launch's instructions at batch 1 of 32 k tokens, 0.05 % at batch 8 of 16 k.
-template <int GV, bool ONE_TIER>
+// A plane's outputs without anybody reading them back: every share's normalised output is added to a 64-bit word as a
+// multiple of 2^-33, together with a count in the bits above; the thread that finds the count complete in what its addition
+// returns has the whole sum and writes it.  (Reductions, a fence, a counter and a last CTA that reads the sums are three round
+// trips to L2 in a row, 2 us; this is one.)  A share is a weighted mean of a part of V, so it and every partial sum stay below
+// 2^17, the largest difference of two halfs, and the sum of up to V_MAX_SHARES roundings below 2^-25, half the smallest half;
+// sums of integers do not depend on their order.  What is not a finite number sets a bit of its own above the count.
+// (Not direct - more shares, or peers that get the outputs too: the same words, read by the last CTA.)
+constexpr int V_MAX_SHARES = 256;
+__device__ __forceinline__ float v_output(unsigned long long sum) {
+  const unsigned odd = static_cast<unsigned>(sum >> 61);   // +inf, -inf, NaN
+  if (odd) return odd == 1u ? INFINITY : odd == 2u ? -INFINITY : __int_as_float(0x7FC00000);
+  return static_cast<float>(static_cast<double>(static_cast<long long>(sum << 12) >> 12) * 0x1p-33);
+}
+__device__ __forceinline__ void v_finish(const DecodeParams& P, const VShared& sh, int64_t out0) {
+  unsigned long long* words = reinterpret_cast<unsigned long long*>(P.v_acc) + out0 + threadIdx.x;
+  unsigned long long sum[MAX_R4];
+#pragma unroll
+  for (int h = 0; h < MAX_R4; ++h) {
+    if (h >= P.r4) break;
+    float v = 0.f;
+#pragma unroll
+    for (int i = 0; i < VWARPS; ++i) v += sh.w[i].red[h][threadIdx.x];
+    v *= sh.ginv[h];
+    unsigned long long add = P.direct || blockIdx.y == 0 ? 1ull << 52 : 0ull;   // (not direct: one count, for a negative sum to borrow from)
+    if (fabsf(v) < 0x1p17f) add += static_cast<unsigned long long>(__float2ll_rn(v * 0x1p33f));
+    else atomicOr(words + h * D, v > 0.f ? 1ull << 61 : v < 0.f ? 1ull << 62 : 1ull << 63);   // (before the thread's own addition to the word)
+    sum[h] = atomicAdd(words + h * D, add) + add;
+  }
+  if (!P.direct) return;
+#pragma unroll
+  for (int h = 0; h < MAX_R4; ++h) {
+    if (h >= P.r4) break;
+    // (a negative sum borrows from the count)
+    if (((sum[h] + (1ull << 51)) >> 52 & 0x1FFu) == static_cast<unsigned>(P.nv_ctas)) P.out[out0 + h * D + threadIdx.x] = __float2half_rn(v_output(sum[h]));
+  }
+}
+
+// GV: log2 of the channel group.  NP: pairs of 16-token steps in a tile.
+template <int GV, int MODE, int NP>
 __global__ void __launch_bounds__(VTHREADS, V_MIN_CTAS) v_pass_kernel(const __grid_constant__ DecodeParams P) {
+  constexpr int NG = D >> GV;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   VShared& sh = *reinterpret_cast<VShared*>(smem_raw);
   const Where w = where(P);
-  const int row = blockIdx.y;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // (the warp's number in a form that the compiler knows to be the same in all lanes: what depends on it is uniform)
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), g = lane >> 2, tig = lane & 3;
 
   // The next kernel of the stream - the K pass of the next decode call, if it was launched with
   // programmatic stream serialisation - may start its cache-only prologue while this grid drains.
   asm volatile("griddepcontrol.launch_dependents;");
   VWarpShared& ws = sh.w[warp];
-  bool fresh = true;  // the warp's partial output is still to be set
-  // ---- global (max, sum) of the heads from the K pass's pairs: warp = head, up to four pairs per lane in
-  //      flight (weights given by the caller: nothing to fold, nothing to normalise by)
-  bool folded = false;
-  auto fold = [&]() {
-    if (folded) return;
-    folded = true;
-    if (!P.probs_in && warp < P.r4) {
-      const float2* part = P.k_part + (static_cast<int64_t>(w.bvh) * P.r4 + warp) * P.nk_ctas;
-      float m = -INFINITY, l = 0.f;
-      for (int c0 = lane; c0 < P.nk_ctas; c0 += 4 * 32) {
-        float2 v[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = c0 + 32 * j < P.nk_ctas ? __ldcg(part + c0 + 32 * j) : make_float2(-INFINITY, 0.f);
+  for (int i = 0; i < MAX_R4; ++i) reinterpret_cast<float4*>(ws.red[i])[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+  // The lane in the softmax: head lane / 8, quad lane % 8 of the eight of a pair of steps.
+  constexpr int tile = 32 * NP, stride = VWARPS * tile;   // tokens of a warp, of the CTA at a time
+  const int head = lane >> 3, wtok = warp * tile + 4 * (lane & 7), mine = keep(wtok + head);   // first token of its first quad; whose position it fetches
+  __half* rows = P.weights + (static_cast<int64_t>(w.b) * P.nh_q + w.h0) * P.L;
+  const uint32_t row = MODE != V_GIVEN && head < P.r4 ? static_cast<uint32_t>(head) * static_cast<uint32_t>(P.L) : V_NONE;
+  float mh = INFINITY, inv = 0.f;   // max * log2(e), 1 / sum; of a head that is not there: probability 0
+  const bool whole = ((reinterpret_cast<uintptr_t>(rows) | (static_cast<uintptr_t>(P.L) << 1)) & 7u) == 0u;
+  const uint32_t rem = keep((g & 1) ? 0xFFFFFFFFu : 0u);
+  // Its places in shared memory: 8 bytes of scales as they come; the quad it transposes (lanes 16 - 31: of the zeros), from and
+  // to; quad tig in the scales, and with channel group g % NG in the zeros, of the first step.
+  const uint32_t raw = smem_u32(ws.raw);
+  const uint32_t sdst = keep(raw + (NG == 4 ? v_swizzle(lane * 8) : lane * 8));
+  const uint32_t from = keep(raw + (lane >> 4) * (V_TILE * 8) + (NG == 4 ? v_swizzle((lane & 15) * 32) : (lane & 15) * (8 * NG)));
+  const uint32_t t_s = keep(smem_u32(ws.t) + tig * (8 * NG));
+  const uint32_t t_z = keep(smem_u32(ws.t[1]) + tig * (8 * NG) + (g & (NG - 1)) * 8);
+  constexpr uint32_t TO = sizeof(VWarpShared::raw);   // from raw to t
+
+  // One round per quantised tier, and an empty one where a CTA has none.
+  bool begun = false;
+#pragma unroll 1
+  for (int ti = 1; ti <= HQKV_NUM_TIERS; ++ti) {
+    int t0 = 0, t1 = 0;
+    if (ti < HQKV_NUM_TIERS ? !share_of<true>(P, ti, t0, t1) : begun) continue;
+    const TierDev& T = P.tier[ti];
+    const int bits = T.bits;
+    const bool normal = T.normal != 0;
+    int left = t1 - t0;   // tokens from the CTA's next tiles on; those of the warp start tile * warp further
+    const int64_t tok0 = static_cast<int64_t>(w.bh) * T.n_v + t0;
+    VRun r;
+    {
+      const int lp = bits == 8 ? 3 : bits == 4 ? 2 : bits == 2 ? 1 : 0;   // log2 of the pieces of a row
+      // codes: the 16-byte pieces of a step are shared out in the order they lie in shared memory, rows in k-order, the piece
+      // index XORed with row bits so that the eight rows of an ldmatrix spread over all banks
+      const int k = lane >> lp, piece = lane & ((1 << lp) - 1);
+      const int token = (k & 16) + ((k & 6) << 1) + ((k >> 2) & 2) + (k & 1);
+      const uint32_t codes = smem_u32(ws.codes);
+      r.src = keep(((warp * tile + token) << (lp + 4)) + piece * 16);
+      r.dst = keep(codes + (k << (lp + 4)) + ((piece ^ ((k >> (3 - lp)) & ((1 << lp) - 1))) << 4));
+      // ldmatrix: matrices (octet, piece) (0, 0), (0, 1), (1, 0), (1, 1) at 8 bits, else (0, 0), (1, 0), (0, 1), (1, 1)
+      const int octet = bits == 8 ? lane >> 4 : (lane >> 3) & 1, c = bits == 8 ? (lane >> 3) & 1 : lane >> 4, kk = 8 * octet + (lane & 7);
+      r.lm = keep(bits == 1 ? codes + 2 * tig * 16 + 2 * (g & 3)
+                            : codes + (kk << (lp + 4)) + ((c ^ ((kk >> (3 - lp)) & ((1 << lp) - 1))) << 4));
+      r.codes = static_cast<const unsigned char*>(T.v_data) + (tok0 << (lp + 4));
+      r.s = reinterpret_cast<const unsigned char*>(T.v_scale) + tok0 * (NG * 2);
+      r.z = reinterpret_cast<const unsigned char*>(T.v_zero) + tok0 * (NG * 2);
+    }
+    const int64_t* idx = T.v_idx + t0;   // positions of the tiles
+    // (what lies beyond the tier is filled with zeros)
+    auto request_scales = [&](int left) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) softmax_merge(m, l, v[j].x, v[j].y);
+      for (int o = 0; o < V_TILE * NG * 2; o += 256) {
+        const int mine = o + lane * 8;
+        if (mine < tile * (NG * 2)) {
+          const int at = warp * (tile * (NG * 2)) + mine, valid = max(0, min(8, left * (NG * 2) - at));
+          const uint32_t from = valid ? at : 0;
+          cp_async_8_fill(sdst + o, r.s + from, valid);
+          cp_async_8_fill(sdst + V_TILE * 8 + o, r.z + from, valid);
+        }
       }
-      float mx = m;
+    };
+    // position of token `head` of the lane's quads (low word), of the tile after the next
+    uint32_t at[NP], quad[NP];
+    bool dense = false;
+    auto positions = [&](const int64_t* idx, int left) {
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      float sum = l * fast_exp2((m - (mx == -INFINITY ? 0.f : mx)) * LOG2E);
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      if (lane == 0) {
-        sh.gm[warp] = mx * LOG2E;
-        sh.ginv[warp] = 1.f / sum;
+      for (int j = 0; j < NP; ++j) {
+        const int t = mine + 32 * j;
+        at[j] = t < left ? __ldg(reinterpret_cast<const uint32_t*>(idx + t)) : V_NONE;
       }
+    };
+    float x[NP][4];
+    // Requested for the tiles that have `left` tokens from the first on: the logits (positions in at), the positions of the ones after them.
+    auto gather = [&](int left) {
+      bool ok = MODE == V_FOUR || (MODE == V_FEWER && P.r4 == 2);
+#pragma unroll
+      for (int j = 0; j < NP; ++j) {
+          quad[j] = __shfl_sync(0xffffffffu, at[j], lane & 7);
+        ok = ok && at[j] == quad[j] + head && (quad[j] & 3u) == 0u && quad[j] < (static_cast<uint32_t>(P.L) & ~3u);
+      }
+      dense = __all_sync(0xffffffffu, ok);
+      v_gather<MODE, NP>(P, w, head, dense, quad, idx + wtok, min(left - wtok, tile), x);
+      positions(idx + stride, left - stride);
+    };
+    __syncwarp();   // (the buffers may have served another tier)
+    if (left > 0) {
+      request_scales(left);
+      cp_async_commit();
+      if (left >= stride) v_request_tile<true, NP>(bits, r, 0);
+      else v_request_tile<false, NP>(bits, r, left - warp * tile);
+      positions(idx, left);
+    }
+    const bool waited = begun;
+    begun = true;
+    // (what reads only the cache has been requested before the K pass is known to be complete)
+    if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (left > 0) gather(left);
+    if (!waited && MODE != V_GIVEN) {
+      // global (max, sum) of the heads from the K pass's pairs: warp = head, up to four pairs per lane in flight
+      if (warp < P.r4) {
+        const float2* pairs = P.k_part + (static_cast<int64_t>(w.bvh) * P.r4 + warp) * P.nk_ctas;
+        float m = -INFINITY, l = 0.f;
+#pragma unroll 1
+        for (int c0 = lane; c0 < P.nk_ctas; c0 += 4 * 32) {
+          float2 v[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[j] = c0 + 32 * j < P.nk_ctas ? __ldcg(pairs + c0 + 32 * j) : make_float2(-INFINITY, 0.f);
+          const float mx = fmaxf(fmaxf(fmaxf(v[0].x, v[1].x), fmaxf(v[2].x, v[3].x)), m);
+          const float ref = mx == -INFINITY ? 0.f : mx;   // every position masked out: 0, not NaN
+          l *= fast_exp2((m - ref) * LOG2E);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) l += v[j].y * fast_exp2((v[j].x - ref) * LOG2E);
+          m = mx;
+        }
+        float mx = m;
+#pragma unroll
+        for (int k = 1; k < 32; k <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, k));
+        float sum = l * fast_exp2((m - (mx == -INFINITY ? 0.f : mx)) * LOG2E);
+#pragma unroll
+        for (int k = 1; k < 32; k <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, k);
+        if (lane == 0) {
+          sh.gm[warp] = mx * LOG2E;
+          sh.ginv[warp] = 1.f / sum;
+        }
+      }
+      __syncthreads();
+      if (head < P.r4) mh = sh.gm[head], inv = sh.ginv[head];
+    }
+    if (left <= 0) continue;
+    float acc[8][4], za[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+#pragma unroll 1
+    for (; left > 0; left -= stride) {
+      const int next = left - stride;
+      r.codes += stride * 16 * bits;
+      r.s += stride * NG * 2;
+      r.z += stride * NG * 2;
+      cp_async_wait<NP>();   // scales and zeros (the codes of the tile may still be on their way)
+      __syncwarp();
+      // [token][group] -> [group][token] of a quad
+      if constexpr (NG == 4) {
+        const uint4 u = lds128(from), v = lds128(from ^ 16u);
+        sts128(from + TO, pack_lo16(u.x, u.z), pack_lo16(v.x, v.z), pack_hi16(u.x, u.z), pack_hi16(v.x, v.z));
+        sts128((from ^ 16u) + TO, pack_lo16(u.y, u.w), pack_lo16(v.y, v.w), pack_hi16(u.y, u.w), pack_hi16(v.y, v.w));
+      } else if constexpr (NG == 2) {
+        const uint4 u = lds128(from);
+        sts128(from + TO, pack_lo16(u.x, u.y), pack_lo16(u.z, u.w), pack_hi16(u.x, u.y), pack_hi16(u.z, u.w));
+      } else {
+        const uint2 u = lds64(from);
+        sts64(from + TO, u.x, u.y);
+      }
+      __syncwarp();
+      if (next > 0) request_scales(next);
+      cp_async_commit();
+      uint32_t p[NP][2], n[NP][2];
+#pragma unroll
+      for (int j = 0; j < NP; ++j) {
+          if constexpr (MODE == V_GIVEN) {
+          p[j][0] = pack_f16x2(x[j][0], x[j][1]), p[j][1] = pack_f16x2(x[j][2], x[j][3]);
+        } else {
+          float e[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) e[i] = fast_exp2(fmaf(x[j][i], LOG2E, -mh));  // exp2(-inf) = 0 beyond the tier
+          p[j][0] = pack_f16x2(e[0], e[1]), p[j][1] = pack_f16x2(e[2], e[3]);
+          n[j][0] = pack_f16x2(e[0] * inv, e[1] * inv), n[j][1] = pack_f16x2(e[2] * inv, e[3] * inv);
+        }
+        // Zero term.  Rows g of A are the channel groups of the even step's quads, rows g + 8 of the odd one's; B is the lane's own
+        // probabilities: of the columns, head * 2 + (lane's step & 1), a lane keeps head tig of the step that the row is of:
+        // acc[0] and acc[3].
+        const uint32_t zq = t_z + j * (64 * NG);
+        const uint32_t zo = (NG == 4 ? zq ^ 16u : zq) + 32 * NG;
+        const uint2 ze = lds64(zq), zp = lds64(zo);
+        mma16816(za, ze.x, zp.x, ze.y, zp.y, p[j][0], p[j][1]);
+        if (normal) {  // value = std * C * (2 code - 1) + mean: the code-free term is sum_t p (mean - C std)
+          const uint2 se = lds64(zq - V_TILE * 8), so = lds64(zo - V_TILE * 8);
+          const uint32_t sd[4] = {se.x, so.x, se.y, so.y};
+          uint32_t hi[4], lo[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) v_normal_offset(sd[i], hi[i], lo[i]);
+          mma16816(za, hi[0], hi[1], hi[2], hi[3], p[j][0], p[j][1]);
+          mma16816(za, lo[0], lo[1], lo[2], lo[3], p[j][0], p[j][1]);
+        }
+      }
+      if (MODE == V_FOUR || (MODE == V_FEWER && row != V_NONE)) v_store_probs<NP>(rows, row, whole, dense, quad, idx + wtok, min(left - wtok, tile), P.L, n);
+      idx += stride;
+      if (next > 0) gather(next);
+      const bool refill = next >= stride;
+      if (bits == 4) v_tile<4, GV, NP>(acc, p, r, t_s, rem, refill);
+      else if (bits == 2) v_tile<2, GV, NP>(acc, p, r, t_s, rem, refill);
+      else if (bits == 8) v_tile<8, GV, NP>(acc, p, r, t_s, rem, refill);
+      else v_tile<1, GV, NP>(acc, p, r, t_s, rem, refill);
+      if (next > 0 && !refill) {   // the tier ends within the next tiles
+        __syncwarp();
+        v_request_tile<false, NP>(bits, r, next - warp * tile);
+      }
+    }
+    cp_async_wait<0>();
+    __syncwarp();
+    v_store_output<GV>(ws.red, acc, bits, normal ? 2.f * HQKV_NORMAL1_CENTER : 1.f, za[0] + za[3]);
+  }
+  __syncwarp();
+  // ---- fp16 tier, residual window
+#pragma unroll 1
+  for (int ti = 0; ti <= HQKV_NUM_TIERS; ti += HQKV_NUM_TIERS) {
+    int t0, t1;
+    if (!share_of<true>(P, ti, t0, t1)) continue;
+    for (int t = t0 + 16 * warp; t < t1; t += 16 * VWARPS)
+      v_plain_tile<MODE>(P, P.tier[ti], sh, reinterpret_cast<__half*>(ws.raw), ws.red, w, t, min(16, t1 - t), ti != 0);
+  }
+  __syncthreads();
+  // ---- the output of this CTA (warps added in index order) joins those of its plane
+  const int64_t out0 = (static_cast<int64_t>(w.b) * P.nh_q + w.h0) * D;
+  // Weights given by the caller may add up to anything: fp64 reductions, whose sum depends on the order of the fp32 partials
+  // only below 2^-53.
+  double* accum = P.v_acc + out0;
+  if constexpr (MODE == V_GIVEN) {
+    for (int h = 0; h < P.r4; ++h) {
+      float v = 0.f;
+#pragma unroll
+      for (int i = 0; i < VWARPS; ++i) v += sh.w[i].red[h][tid];
+      atomicAdd(accum + h * D + tid, static_cast<double>(v));
+    }
+  } else {
+    v_finish(P, sh, out0);
+  }
+  // ---- not direct: the last CTA of this (batch, virtual kv head) writes the output
+  if (tid == 0) sh.is_last = 0u;
+  if (!P.direct) {
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();  // the CTA's adds, which the barrier has ordered before this thread's fence
+      const unsigned prev = atomicAdd(&P.counters[w.bvh], 1u);
+      sh.is_last = (prev == static_cast<unsigned>(P.nv_ctas) - 1u) ? 1u : 0u;
+      if (sh.is_last) P.counters[w.bvh] = 0u;  // ready for the next call
     }
     __syncthreads();
-  };
-  // ---- the warp's tiles: probabilities of its tokens, then sum_t p_t * V_t
-  auto plain = [&](int ti, int t0, int t1) {  // fp16 tier, residual window
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    fold();
-    if (fresh) {
-#pragma unroll
-      for (int i = 0; i < MAX_R4; ++i) reinterpret_cast<float4*>(ws.red[i])[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-      fresh = false;
-    }
-    for (int t = t0 + 16 * warp; t < t1; t += 16 * VWARPS) v_plain_tile(P, P.tier[ti], sh, ws, w, t, min(16, t1 - t), ti != 0);
-  };
-  int t0, t1;
-  if constexpr (ONE_TIER) {
-    const int ti = only_share<true>(P, t0, t1);
-    if (ti == 1) v_run<8, GV, 2>(P, P.tier[1], sh, w, t0, t1, fold, fresh);
-    else if (ti == 2) v_run<4, GV, 2>(P, P.tier[2], sh, w, t0, t1, fold, fresh);
-    else if (ti == 3) v_run<2, GV, 2>(P, P.tier[3], sh, w, t0, t1, fold, fresh);
-    else if (ti == 4) v_run<1, GV, 2>(P, P.tier[4], sh, w, t0, t1, fold, fresh);
-    else plain(ti, t0, t1);
-  } else {
-    if (share_of<true>(P, 1, 8, t0, t1)) v_run<8, GV, 1>(P, P.tier[1], sh, w, t0, t1, fold, fresh);
-    if (share_of<true>(P, 2, 4, t0, t1)) v_run<4, GV, 1>(P, P.tier[2], sh, w, t0, t1, fold, fresh);
-    if (share_of<true>(P, 3, 2, t0, t1)) v_run<2, GV, 1>(P, P.tier[3], sh, w, t0, t1, fold, fresh);
-    if (share_of<true>(P, 4, 1, t0, t1)) v_run<1, GV, 1>(P, P.tier[4], sh, w, t0, t1, fold, fresh);
-    for (int ti = 0; ti <= HQKV_NUM_TIERS; ti += HQKV_NUM_TIERS)
-      if (share_of<true>(P, ti, 16, t0, t1)) plain(ti, t0, t1);
+  } else if (!P.head_sum) {
+    return;
   }
-  __syncthreads();
-  // ---- partial output of this CTA (warps added in index order) joins the accumulators of its heads.  The adds are
-  //      fire-and-forget fp64 reductions: the sum of the fp32 partials
-  //      depends on their order only below 2^-53, far below the fp16 rounding of the output, and no
-  //      CTA has to read other CTAs' partials back (a chain of dependent L2 round trips that used to
-  //      be a quarter of the kernel at batch 1).
-  double* accum = P.v_acc + (static_cast<int64_t>(w.b) * P.nh_q + w.h0) * D;
-  for (int h = 0; h < P.r4; ++h) {
-    float v = 0.f;
-#pragma unroll
-    for (int i = 0; i < VWARPS; ++i) v += sh.w[i].red[h][tid];
-    atomicAdd(accum + h * D + tid, static_cast<double>(v));
-  }
-  // ---- the last CTA of this (batch, virtual kv head) normalises and writes the output
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();  // the CTA's adds, which the barrier has ordered before this thread's fence
-    const unsigned prev = atomicAdd(&P.counters[w.bvh], 1u);
-    sh.is_last = (prev == static_cast<unsigned>(P.nv_ctas) - 1u) ? 1u : 0u;
-    if (sh.is_last) P.counters[w.bvh] = 0u;  // ready for the next call
-  }
-  __syncthreads();
-  if (sh.is_last) {
+  if (!P.direct && sh.is_last) {
     __threadfence();
     for (int i = tid * 2; i < P.r4 * D; i += VTHREADS * 2) {
-      const double2 v = __ldcg(reinterpret_cast<const double2*>(accum + i));
-      const float inv = P.probs_in ? 1.f : sh.ginv[i >> 7];
-      const __half2 o = __floats2half2_rn(static_cast<float>(v.x) * inv, static_cast<float>(v.y) * inv);
+      __half2 o;
+      if constexpr (MODE == V_GIVEN) {
+        const double2 v = __ldcg(reinterpret_cast<const double2*>(accum + i));
+        o = __floats2half2_rn(static_cast<float>(v.x), static_cast<float>(v.y));
+      } else {
+        const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2*>(accum + i));
+        o = __floats2half2_rn(v_output(v.x), v_output(v.y));
+      }
       const int64_t at = (static_cast<int64_t>(w.b) * P.nh_q + w.h0) * D + i;
       *reinterpret_cast<__half2*>(P.out + at) = o;
       // kv-head sharding: the same rows go straight into every peer's copy of the gathered output
@@ -1956,15 +1929,15 @@ __global__ void __launch_bounds__(VTHREADS, V_MIN_CTAS) v_pass_kernel(const __gr
     __threadfence();  // this CTA's probabilities
     __syncthreads();
     if (tid == 0) {
-      const unsigned prev = atomicAdd(&P.hs_count[row], 1u);
+      const unsigned prev = atomicAdd(&P.hs_count[blockIdx.y], 1u);
       sh.is_last = (prev == gridDim.x * gridDim.z - 1u) ? 1u : 0u;
-      if (sh.is_last) P.hs_count[row] = 0u;  // ready for the next call
+      if (sh.is_last) P.hs_count[blockIdx.y] = 0u;  // ready for the next call
     }
     __syncthreads();
     if (sh.is_last) {
-      const int only = ONE_TIER ? only_share<true>(P, t0, t1) : -1;
+      int t0, t1;
       for (int ti = 0; ti <= HQKV_NUM_TIERS; ++ti)
-        if (ONE_TIER ? ti == only : share_of<true>(P, ti, P.tier[ti].bits, t0, t1))
+        if (share_of<true>(P, ti, t0, t1))
           for (int c0 = t0; c0 < t1; c0 += HS_TOKENS) head_sum_chunk(P, P.tier[ti], sh, c0, min(HS_TOKENS, t1 - c0), ti == HQKV_NUM_TIERS);
     }
   }
@@ -1998,35 +1971,54 @@ struct Layout {
 // Where one or two units per CTA make a wave, a second tier would double a CTA's latency: there a CTA keeps to one tier
 // (two units at 8 bits).
 static void divide(DecodeParams& P, int64_t planes, int slots, bool v) {
-  int total = 0;  // cost of a plane
-  for (const TierDev& t : P.tier) total += static_cast<int>(ceil_div(v ? t.n_v : t.n_k, unit_tokens(t.bits))) * unit_cost(t.bits);
-  constexpr int UNIT = unit_cost(4);
-  int ctas = total > 0 ? 1 : 0;
-  double best = 0.;
-  for (int n = 1; n == 1 || (total / n >= 2 * UNIT && (n - 1) * planes < 4 * slots); ++n) {
-    const double waves = static_cast<double>(n * planes) / slots;
-    const double cost = (static_cast<double>(total) / n + UNIT) * (waves <= 1. ? 1. : 0.5 * (waves + ceil(waves)));
-    if (n == 1 || cost < best) best = cost, ctas = total > 0 ? n : 0;
-  }
-  int per = ctas ? total / ctas : 0, more = ctas ? total % ctas : 0;
-  // the cost that a CTA of one tier may have: the smallest with which the planes' CTAs fit one wave
+  int total = 0, unit = 0;  // cost of a plane; of a unit of most widths
+  auto tokens = [&](const TierDev& t) { return v ? t.n_v : t.n_k; };
+  auto set_units = [&](int pairs) {
+    total = 0;
+    for (TierDev& t : P.tier) {
+      TierDev::Units& u = t.unit[v];
+      u.tokens = !v || t.bits == 16 ? unit_tokens(t.bits) : 128 * pairs;
+      u.cost = !v || t.bits == 16 ? unit_cost(t.bits) : t.bits == 8 ? 6 * pairs : 4 * pairs;
+      u.per_cost = 0xFFFFFFFFu / u.cost + 1u;
+      u.cost0 = total;
+      total += static_cast<int>(ceil_div(tokens(t), u.tokens)) * u.cost;
+    }
+    unit = P.tier[2].unit[v].cost;
+  };
+  // CTAs of one tier each, of at most this cost (at least a unit each)
   auto one_tier = [&](int budget, bool set) {
     int n = 0;
     for (TierDev& t : P.tier) {
-      const int u = budget < unit_cost(t.bits) ? 1 : budget / unit_cost(t.bits);
-      if (set) (v ? t.v_cta0 : t.k_cta0) = n;
-      n += static_cast<int>(ceil_div(v ? t.n_v : t.n_k, unit_tokens(t.bits) * u));
+      TierDev::Units& u = t.unit[v];
+      if (set) u.cta0 = n;
+      n += static_cast<int>(ceil_div(tokens(t), u.tokens * (budget < u.cost ? 1 : budget / u.cost)));
     }
     return n;
   };
-  int budget = 2 * unit_cost(8);
-  while (budget <= 2 * unit_cost(4) && static_cast<int64_t>(one_tier(budget, false)) * planes > slots) ++budget;
-  if (total > 0 && budget <= 2 * unit_cost(4)) {
-    ctas = one_tier(budget, true), per = budget, more = -1;
+  auto take = [&](int ctas, int per, int more) {
+    (v ? P.nv_ctas : P.nk_ctas) = ctas;
+    (v ? P.v_per : P.k_per) = per;
+    (v ? P.v_more : P.k_more) = more;
+  };
+  if (v) {
+    set_units(P.v_pairs = 1);
+    if (total > 0 && one_tier(unit, false) * planes <= slots) return take(one_tier(unit, true), unit, -1);
+    P.v_pairs = 2;
   }
-  (v ? P.nv_ctas : P.nk_ctas) = ctas;
-  (v ? P.v_per : P.k_per) = per;
-  (v ? P.v_more : P.k_more) = more;
+  set_units(2);
+  if (total == 0) return take(0, 0, 0);
+  // the smallest cost with which the planes' CTAs of one tier fit one wave
+  int budget = v ? unit : 2 * unit_cost(8);
+  while (budget <= 2 * unit && one_tier(budget, false) * planes > slots) ++budget;
+  if (budget <= 2 * unit) return take(one_tier(budget, true), budget, -1);
+  int ctas = 1;
+  double best = 0.;
+  for (int n = 1; n == 1 || (total / n >= 2 * unit && (n - 1) * planes < 4 * slots); ++n) {
+    const double waves = static_cast<double>(n * planes) / slots;
+    const double cost = (static_cast<double>(total) / n + unit) * (waves <= 1. ? 1. : 0.5 * (waves + ceil(waves)));
+    if (n == 1 || cost < best) best = cost, ctas = n;
+  }
+  take(ctas, total / ctas, total % ctas);
 }
 
 // sides: 1 = only the K side of the descriptor is looked at, 2 = only the V side, 3 = both
@@ -2054,7 +2046,6 @@ static int build_params(const hqkv_cache_desc_t* c, DecodeParams& P, Layout& lay
   P.scale = c->softmax_scale;
   static const int expect_bits[HQKV_NUM_TIERS] = {16, 8, 4, 2, 1};
   int64_t nk_total = 0, nv_total = 0;
-  int kc = 0, vc = 0;
   for (int t = 0; t < HQKV_NUM_TIERS; ++t) {
     const hqkv_tier_t& s = c->tier[t];
     TierDev& d = P.tier[t];
@@ -2098,10 +2089,6 @@ static int build_params(const hqkv_cache_desc_t* c, DecodeParams& P, Layout& lay
     d.v_zero = static_cast<const __half*>(s.v_zero);
     d.v_idx = s.v_idx;
     HQKV_REQUIRE(static_cast<int64_t>(s.n_k) * D * d.bits / 8 < (1ll << 31), "decode: tier %d K plane of one head exceeds 2 GiB", t);
-    d.k_cost0 = kc;
-    d.v_cost0 = vc;
-    kc += static_cast<int>(ceil_div(d.n_k, unit_tokens(d.bits))) * unit_cost(d.bits);
-    vc += static_cast<int>(ceil_div(d.n_v, unit_tokens(d.bits))) * unit_cost(d.bits);
     nk_total += d.n_k;
     nv_total += d.n_v;
   }
@@ -2117,8 +2104,6 @@ static int build_params(const hqkv_cache_desc_t* c, DecodeParams& P, Layout& lay
   }
   r.k_data = c->new_k;
   r.v_data = c->new_v;
-  r.k_cost0 = kc;
-  r.v_cost0 = vc;
   const int64_t L = ((sides & 1) ? nk_total : nv_total) + c->n_new;
   HQKV_REQUIRE(L > 0, "decode: the cache is empty");
   HQKV_REQUIRE(L < (1ll << 30), "decode: cache too long");
@@ -2206,9 +2191,12 @@ extern "C" int hqkv_decode_attention_gather(const hqkv_cache_desc_t* cache_host,
 
 using PassKernel = void (*)(const DecodeParams);
 static constexpr PassKernel k_kernels[2] = {k_pass_kernel<false>, k_pass_kernel<true>};  // [one tier per CTA]
-static constexpr PassKernel v_kernels[2][4] = {
-    {v_pass_kernel<0, false>, v_pass_kernel<5, false>, v_pass_kernel<6, false>, v_pass_kernel<7, false>},
-    {v_pass_kernel<0, true>, v_pass_kernel<5, true>, v_pass_kernel<6, true>, v_pass_kernel<7, true>}};
+template <int MODE, int NP>
+static constexpr PassKernel v_kernels_of[3] = {v_pass_kernel<5, MODE, NP>, v_pass_kernel<6, MODE, NP>, v_pass_kernel<7, MODE, NP>};
+static constexpr const PassKernel* v_kernels[3][2] = {  // [VMode][pairs of steps - 1][log2 of the channel group - 5]
+    {v_kernels_of<V_FOUR, 1>, v_kernels_of<V_FOUR, 2>},
+    {v_kernels_of<V_FEWER, 1>, v_kernels_of<V_FEWER, 2>},
+    {v_kernels_of<V_GIVEN, 1>, v_kernels_of<V_GIVEN, 2>}};
 
 static int hqkv::decode_launch(const hqkv_cache_desc_t* cache_host, const void* q, void* attn_weights, void* attn_output,
                                void* workspace, size_t workspace_bytes, int phases, const PeerArgs& peers, void* stream,
@@ -2254,6 +2242,7 @@ static int hqkv::decode_launch(const hqkv_cache_desc_t* cache_host, const void* 
   P.logits = reinterpret_cast<float*>(ws + lay.logits_off);
   P.k_part = reinterpret_cast<float2*>(ws + lay.kpart_off);
   P.v_acc = reinterpret_cast<double*>(ws + lay.acc_off);
+  P.direct = !probs_in && peers.n_peers == 0 && !peers.pads && P.nv_ctas <= V_MAX_SHARES;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const unsigned VH = static_cast<unsigned>(P.H * P.halves);
   HQKV_REQUIRE(P.nk_ctas <= 65535 && P.nv_ctas <= 65535, "decode: too many chunks");
@@ -2265,11 +2254,15 @@ static int hqkv::decode_launch(const hqkv_cache_desc_t* cache_host, const void* 
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
       // all of them with the same (largest) share of the L1 for shared memory: CTAs of kernels that ask for different
       // shares cannot be on an SM together
-      for (int one = 0; one < 2; ++one)
-        for (PassKernel f : {k_kernels[one], v_kernels[one][0], v_kernels[one][1], v_kernels[one][2], v_kernels[one][3]}) {
-          HQKV_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(PASS_SMEM)));
-          HQKV_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-        }
+      auto opt_in = [](PassKernel f) {
+        HQKV_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(PASS_SMEM)));
+        HQKV_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        return 0;
+      };
+      for (PassKernel f : k_kernels)
+        if (int rc = opt_in(f)) return rc;
+      for (int i = 0; i < 18; ++i)
+        if (int rc = opt_in(v_kernels[i / 6][i / 3 % 2][i % 3])) return rc;
       if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
   }
@@ -2297,8 +2290,7 @@ static int hqkv::decode_launch(const hqkv_cache_desc_t* cache_host, const void* 
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const bool fast = P.r4 >= 2 && !P.probs_in;
-    HQKV_CUDA(cudaLaunchKernelEx(&cfg, v_kernels[P.v_more < 0][fast ? P.gv_shift - 4 : 0], P));
+    HQKV_CUDA(cudaLaunchKernelEx(&cfg, v_kernels[P.probs_in ? V_GIVEN : P.r4 == MAX_R4 ? V_FOUR : V_FEWER][P.v_pairs - 1][P.gv_shift - 5], P));
   }
   return HQKV_OK;
 }
@@ -2336,12 +2328,13 @@ extern "C" int hqkv_decode_attention_headsum(const hqkv_cache_desc_t* cache_host
 // The two passes as operators of their own: raw logits of every tier, and the product of given weights with V
 // ------------------------------------------------------------------------------------------------
 namespace hqkv {
-// fp32 logits of the scratch [plane][L][heads] -> fp16 rows [plane][head][L]
+// fp32 logits of the scratch -> fp16 rows [plane][head][L]
 __global__ void __launch_bounds__(256) logits_out_kernel(const float* logits, __half* out, int64_t planes, int64_t L, int heads) {
   const int64_t n = planes * L, stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
     const int64_t plane = i / L, pos = i - plane * L;
-    for (int h = 0; h < heads; ++h) out[(plane * heads + h) * L + pos] = __float2half_rn(__ldcg(logits + i * heads + h));
+    for (int h = 0; h < heads; ++h)
+      out[(plane * heads + h) * L + pos] = __float2half_rn(__ldcg(logits + plane * L * heads + logit_at(pos, h, heads, static_cast<int>(L))));
   }
 }
 }  // namespace hqkv
