@@ -64,7 +64,7 @@ struct DecodeParams {
   // Units per CTA.  more >= 0: equal shares, the first `more` CTAs take one more; -1: no CTA has units of two tiers (in
   // the K pass 8-bit units, which are half as long, count half).
   int k_per, k_more, v_per, v_more;
-  int v_pairs;             // 32 tokens a warp of the V pass takes at a time: 1, 2
+  int v_pairs, v_warps;    // 32 tokens a warp of the V pass takes at a time: 1, 2; warps per CTA: 8, 4
   int direct;              // the outputs are finished by whoever adds the last share (see v_finish), not by a CTA that reads them back
   float scale;
   const __half* q;
@@ -1113,9 +1113,8 @@ __global__ void __launch_bounds__(KTHREADS, K_MIN_CTAS) k_pass_kernel(const __gr
 //    everything) has to come from L2 into every SM that has not run it lately, 1 us per 64-byte line of a cold chain.
 // Codes are streamed through ONE tile buffer: the copy of 32 tokens of the next tile is issued when this tile's have been
 // consumed, so a whole tile's work lies between a request and its use.
-constexpr int V_MIN_CTAS = 4;  // CTAs per SM the V pass is compiled for (128 registers; PASS_SMEM is a quarter of an SM)
-constexpr int VWARPS = 4;
-constexpr int VTHREADS = VWARPS * 32;
+// CTAs of eight warps (half as many outputs to add up, half as many softmax pairs to fold), or of four where those fill the SMs better.
+constexpr int V_SM_WARPS = 16;             // warps per SM the V pass is compiled for (128 registers)
 constexpr int V_TILE = 64;                 // tokens per tile of a warp at most
 
 // importance row emitted by the V pass: staging limits (positions + per-head halfs live in the warps' buffers)
@@ -1127,8 +1126,9 @@ struct VWarpShared {
   unsigned char t[2][V_TILE * 8];                 // scales, zeros as [quad][group][token]; four groups: see v_swizzle
   float red[MAX_R4][D];                           // output of the tiers that are done
 };
+template <int NW>
 struct VShared {
-  VWarpShared w[VWARPS];
+  VWarpShared w[NW];
   float gm[MAX_R4], ginv[MAX_R4];                 // max * log2(e) and 1 / sum of the query heads
   unsigned is_last;
   unsigned pad_[3];
@@ -1424,8 +1424,8 @@ __device__ __forceinline__ void v_store_output(float (*red)[D], const float (&ac
 
 // fp16 tier and residual window, token-major rows [n][D] halfs: one 16-token step per warp straight
 // from global memory; B = p, column n = head n.  The result is added to red.  ps: 128 bytes of shared memory.
-template <int MODE>
-__device__ __forceinline__ void v_plain_tile(const DecodeParams& P, const TierDev& T, const VShared& sh, __half* ps, float (*red)[D], const Where& w,
+template <int MODE, int NW>
+__device__ __forceinline__ void v_plain_tile(const DecodeParams& P, const TierDev& T, const VShared<NW>& sh, __half* ps, float (*red)[D], const Where& w,
                                              int t0, int ntok, bool is_res) {
   const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
   const uint2* base = reinterpret_cast<const uint2*>(T.v_data) + (static_cast<int64_t>(w.bh) * T.n_v + t0) * 32;
@@ -1525,9 +1525,11 @@ __device__ __forceinline__ void peer_barrier_device(unsigned* const* pad, int ra
   if (r == 0) *call_no = n;
 }
 
-static_assert(offsetof(VShared, gm) >= HS_TOKENS * 4 + HS_TOKENS * HS_HEADS * 2, "importance-row staging fits the tile buffers");
+static_assert(sizeof(VShared<4>::w) >= HS_TOKENS * 4 + HS_TOKENS * HS_HEADS * 2, "importance-row staging fits the tile buffers");
 // Importance row of n tokens from token c0 of a tier on, run by the last CTA to finish their grid row (not inlined: its registers are its own).
-__device__ __noinline__ void head_sum_chunk(const DecodeParams& P, const TierDev& T, VShared& sh, int c0, int n, bool is_res) {
+template <int NW>
+__device__ __noinline__ void head_sum_chunk(const DecodeParams& P, const TierDev& T, VShared<NW>& sh, int c0, int n, bool is_res) {
+  constexpr int VTHREADS = NW * 32;
   const int tid = threadIdx.x;
   __threadfence();
   __syncthreads();  // the round before is done with the staging buffers
@@ -1599,36 +1601,41 @@ __device__ __forceinline__ float v_output(unsigned long long sum) {
   if (odd) return odd == 1u ? INFINITY : odd == 2u ? -INFINITY : __int_as_float(0x7FC00000);
   return static_cast<float>(static_cast<double>(static_cast<long long>(sum << 12) >> 12) * 0x1p-33);
 }
-__device__ __forceinline__ void v_finish(const DecodeParams& P, const VShared& sh, int64_t out0) {
-  unsigned long long* words = reinterpret_cast<unsigned long long*>(P.v_acc) + out0 + threadIdx.x;
-  unsigned long long sum[MAX_R4];
+template <int NW>
+__device__ __forceinline__ void v_finish(const DecodeParams& P, const VShared<NW>& sh, int64_t out0) {
+  constexpr int EACH = MAX_R4 * D / (NW * 32), STEP = MAX_R4 / EACH;   // outputs of a thread: heads h0, h0 + STEP, ...
+  const int c = threadIdx.x & (D - 1), h0 = threadIdx.x / D;
+  unsigned long long* words = reinterpret_cast<unsigned long long*>(P.v_acc) + out0 + c;
+  unsigned long long sum[EACH];
 #pragma unroll
-  for (int h = 0; h < MAX_R4; ++h) {
+  for (int k = 0; k < EACH; ++k) {
+    const int h = h0 + STEP * k;
     if (h >= P.r4) break;
     float v = 0.f;
 #pragma unroll
-    for (int i = 0; i < VWARPS; ++i) v += sh.w[i].red[h][threadIdx.x];
+    for (int i = 0; i < NW; ++i) v += sh.w[i].red[h][c];
     v *= sh.ginv[h];
     unsigned long long add = P.direct || blockIdx.y == 0 ? 1ull << 52 : 0ull;   // (not direct: one count, for a negative sum to borrow from)
     if (fabsf(v) < 0x1p17f) add += static_cast<unsigned long long>(__float2ll_rn(v * 0x1p33f));
     else atomicOr(words + h * D, v > 0.f ? 1ull << 61 : v < 0.f ? 1ull << 62 : 1ull << 63);   // (before the thread's own addition to the word)
-    sum[h] = atomicAdd(words + h * D, add) + add;
+    sum[k] = atomicAdd(words + h * D, add) + add;
   }
   if (!P.direct) return;
 #pragma unroll
-  for (int h = 0; h < MAX_R4; ++h) {
+  for (int k = 0; k < EACH; ++k) {
+    const int h = h0 + STEP * k;
     if (h >= P.r4) break;
     // (a negative sum borrows from the count)
-    if (((sum[h] + (1ull << 51)) >> 52 & 0x1FFu) == static_cast<unsigned>(P.nv_ctas)) P.out[out0 + h * D + threadIdx.x] = __float2half_rn(v_output(sum[h]));
+    if (((sum[k] + (1ull << 51)) >> 52 & 0x1FFu) == static_cast<unsigned>(P.nv_ctas)) P.out[out0 + h * D + c] = __float2half_rn(v_output(sum[k]));
   }
 }
 
-// GV: log2 of the channel group.  NP: pairs of 16-token steps in a tile.
-template <int GV, int MODE, int NP>
-__global__ void __launch_bounds__(VTHREADS, V_MIN_CTAS) v_pass_kernel(const __grid_constant__ DecodeParams P) {
-  constexpr int NG = D >> GV;
+// GV: log2 of the channel group.  NP: pairs of 16-token steps in a tile.  NW: warps.
+template <int GV, int MODE, int NP, int NW>
+__global__ void __launch_bounds__(NW * 32, V_SM_WARPS / NW) v_pass_kernel(const __grid_constant__ DecodeParams P) {
+  constexpr int NG = D >> GV, VTHREADS = NW * 32;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  VShared& sh = *reinterpret_cast<VShared*>(smem_raw);
+  VShared<NW>& sh = *reinterpret_cast<VShared<NW>*>(smem_raw);
   const Where w = where(P);
   // (the warp's number in a form that the compiler knows to be the same in all lanes: what depends on it is uniform)
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), g = lane >> 2, tig = lane & 3;
@@ -1640,7 +1647,7 @@ __global__ void __launch_bounds__(VTHREADS, V_MIN_CTAS) v_pass_kernel(const __gr
 #pragma unroll
   for (int i = 0; i < MAX_R4; ++i) reinterpret_cast<float4*>(ws.red[i])[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
   // The lane in the softmax: head lane / 8, quad lane % 8 of the eight of a pair of steps.
-  constexpr int tile = 32 * NP, stride = VWARPS * tile;   // tokens of a warp, of the CTA at a time
+  constexpr int tile = 32 * NP, stride = NW * tile;   // tokens of a warp, of the CTA at a time
   const int head = lane >> 3, wtok = warp * tile + 4 * (lane & 7), mine = keep(wtok + head);   // first token of its first quad; whose position it fetches
   __half* rows = P.weights + (static_cast<int64_t>(w.b) * P.nh_q + w.h0) * P.L;
   const uint32_t row = MODE != V_GIVEN && head < P.r4 ? static_cast<uint32_t>(head) * static_cast<uint32_t>(P.L) : V_NONE;
@@ -1845,7 +1852,7 @@ __global__ void __launch_bounds__(VTHREADS, V_MIN_CTAS) v_pass_kernel(const __gr
   for (int ti = 0; ti <= HQKV_NUM_TIERS; ti += HQKV_NUM_TIERS) {
     int t0, t1;
     if (!share_of<true>(P, ti, t0, t1)) continue;
-    for (int t = t0 + 16 * warp; t < t1; t += 16 * VWARPS)
+    for (int t = t0 + 16 * warp; t < t1; t += 16 * NW)
       v_plain_tile<MODE>(P, P.tier[ti], sh, reinterpret_cast<__half*>(ws.raw), ws.red, w, t, min(16, t1 - t), ti != 0);
   }
   __syncthreads();
@@ -1855,11 +1862,11 @@ __global__ void __launch_bounds__(VTHREADS, V_MIN_CTAS) v_pass_kernel(const __gr
   // only below 2^-53.
   double* accum = P.v_acc + out0;
   if constexpr (MODE == V_GIVEN) {
-    for (int h = 0; h < P.r4; ++h) {
+    for (int k = tid; k < P.r4 * D; k += VTHREADS) {
       float v = 0.f;
 #pragma unroll
-      for (int i = 0; i < VWARPS; ++i) v += sh.w[i].red[h][tid];
-      atomicAdd(accum + h * D + tid, static_cast<double>(v));
+      for (int i = 0; i < NW; ++i) v += sh.w[i].red[k >> 7][k & (D - 1)];
+      atomicAdd(accum + k, static_cast<double>(v));
     }
   } else {
     v_finish(P, sh, out0);
@@ -1949,8 +1956,10 @@ __global__ void __launch_bounds__(VTHREADS, V_MIN_CTAS) v_pass_kernel(const __gr
 // Both passes ask for the same amount of shared memory: their CTAs follow each other on an SM, and with two sizes the
 // gaps that one kind leaves do not fit the other (four of one kind, then only three of the other, half the SMs a wave
 // behind: 77 against 60 us per layer at batch 8).
-constexpr size_t PASS_SMEM = sizeof(KShared) > sizeof(VShared) ? sizeof(KShared) : sizeof(VShared);
+constexpr size_t PASS_SMEM = sizeof(KShared) > sizeof(VShared<4>) ? sizeof(KShared) : sizeof(VShared<4>);
 static_assert(4 * (PASS_SMEM + 1024) <= 228 * 1024, "four CTAs per SM");
+constexpr size_t PASS_SMEM_8 = 2 * PASS_SMEM + 1024;   // a CTA of eight warps takes the place of two
+static_assert(sizeof(VShared<8>) <= PASS_SMEM_8, "two CTAs of eight warps per SM");
 
 static int ilog2(int v) {
   int s = 0;
@@ -1970,14 +1979,17 @@ struct Layout {
 // three (1.2).
 // Where one or two units per CTA make a wave, a second tier would double a CTA's latency: there a CTA keeps to one tier
 // (two units at 8 bits).
-static void divide(DecodeParams& P, int64_t planes, int slots, bool v) {
+//
+// warps: 4 (K pass), 4 or 8 (V pass).  Returns what the longest of the waves takes in units of cost, 0 for CTAs of one tier.
+static double divide(DecodeParams& P, int64_t planes, bool v, int warps) {
+  const int slots = 148 * 16 / warps;
   int total = 0, unit = 0;  // cost of a plane; of a unit of most widths
   auto tokens = [&](const TierDev& t) { return v ? t.n_v : t.n_k; };
   auto set_units = [&](int pairs) {
     total = 0;
     for (TierDev& t : P.tier) {
       TierDev::Units& u = t.unit[v];
-      u.tokens = !v || t.bits == 16 ? unit_tokens(t.bits) : 128 * pairs;
+      u.tokens = !v || t.bits == 16 ? unit_tokens(t.bits) : 32 * warps * pairs;
       u.cost = !v || t.bits == 16 ? unit_cost(t.bits) : t.bits == 8 ? 6 * pairs : 4 * pairs;
       u.per_cost = 0xFFFFFFFFu / u.cost + 1u;
       u.cost0 = total;
@@ -2001,16 +2013,26 @@ static void divide(DecodeParams& P, int64_t planes, int slots, bool v) {
     (v ? P.v_more : P.k_more) = more;
   };
   if (v) {
+    P.v_warps = warps;
     set_units(P.v_pairs = 1);
-    if (total > 0 && one_tier(unit, false) * planes <= slots) return take(one_tier(unit, true), unit, -1);
+    if (warps == 8 && total > 0 && one_tier(unit, false) * planes <= slots) {
+      take(one_tier(unit, true), unit, -1);
+      return 0.;
+    }
     P.v_pairs = 2;
   }
   set_units(2);
-  if (total == 0) return take(0, 0, 0);
+  if (total == 0) {
+    take(0, 0, 0);
+    return 0.;
+  }
   // the smallest cost with which the planes' CTAs of one tier fit one wave
   int budget = v ? unit : 2 * unit_cost(8);
   while (budget <= 2 * unit && one_tier(budget, false) * planes > slots) ++budget;
-  if (budget <= 2 * unit) return take(one_tier(budget, true), budget, -1);
+  if (budget <= 2 * unit) {
+    take(one_tier(budget, true), budget, -1);
+    return 0.;
+  }
   int ctas = 1;
   double best = 0.;
   for (int n = 1; n == 1 || (total / n >= 2 * unit && (n - 1) * planes < 4 * slots); ++n) {
@@ -2019,6 +2041,7 @@ static void divide(DecodeParams& P, int64_t planes, int slots, bool v) {
     if (n == 1 || cost < best) best = cost, ctas = n;
   }
   take(ctas, total / ctas, total % ctas);
+  return best;
 }
 
 // sides: 1 = only the K side of the descriptor is looked at, 2 = only the V side, 3 = both
@@ -2109,8 +2132,11 @@ static int build_params(const hqkv_cache_desc_t* c, DecodeParams& P, Layout& lay
   HQKV_REQUIRE(L < (1ll << 30), "decode: cache too long");
   P.L = static_cast<int>(L);
   const int64_t planes = static_cast<int64_t>(c->B) * c->H * P.halves;
-  divide(P, planes, 148 * K_MIN_CTAS, false);
-  divide(P, planes, 148 * V_MIN_CTAS, true);
+  divide(P, planes, false, KWARPS);
+  // V pass: eight warps where one wave or as good a last wave comes of it.  (Batch 4 of 128 k tokens: 123 us a layer with eight
+  // and 127 with four; batch 8 of 16 k, where four CTAs of eight warps per plane fill 86 % of the places: 57 and 55.)
+  if (const double eight = divide(P, planes, true, 8))
+    if (1.04 * divide(P, planes, true, 4) >= eight) divide(P, planes, true, 8);
   lay.acc_off = HQKV_WS_HEADER_BYTES;
   lay.logits_off = (lay.acc_off + static_cast<size_t>(c->B) * c->nh_q * D * sizeof(double) + 255) & ~static_cast<size_t>(255);
   size_t off = lay.logits_off + static_cast<size_t>(c->B) * c->nh_q * L * sizeof(float);
@@ -2191,12 +2217,12 @@ extern "C" int hqkv_decode_attention_gather(const hqkv_cache_desc_t* cache_host,
 
 using PassKernel = void (*)(const DecodeParams);
 static constexpr PassKernel k_kernels[2] = {k_pass_kernel<false>, k_pass_kernel<true>};  // [one tier per CTA]
-template <int MODE, int NP>
-static constexpr PassKernel v_kernels_of[3] = {v_pass_kernel<5, MODE, NP>, v_pass_kernel<6, MODE, NP>, v_pass_kernel<7, MODE, NP>};
-static constexpr const PassKernel* v_kernels[3][2] = {  // [VMode][pairs of steps - 1][log2 of the channel group - 5]
-    {v_kernels_of<V_FOUR, 1>, v_kernels_of<V_FOUR, 2>},
-    {v_kernels_of<V_FEWER, 1>, v_kernels_of<V_FEWER, 2>},
-    {v_kernels_of<V_GIVEN, 1>, v_kernels_of<V_GIVEN, 2>}};
+template <int MODE, int NP, int NW>
+static constexpr PassKernel v_kernels_of[3] = {v_pass_kernel<5, MODE, NP, NW>, v_pass_kernel<6, MODE, NP, NW>, v_pass_kernel<7, MODE, NP, NW>};
+static constexpr const PassKernel* v_kernels[3][2][2] = {  // [VMode][8, 4 warps][pairs of steps - 1][log2 of the channel group - 5]
+    {{v_kernels_of<V_FOUR, 1, 8>, v_kernels_of<V_FOUR, 2, 8>}, {nullptr, v_kernels_of<V_FOUR, 2, 4>}},
+    {{v_kernels_of<V_FEWER, 1, 8>, v_kernels_of<V_FEWER, 2, 8>}, {nullptr, v_kernels_of<V_FEWER, 2, 4>}},
+    {{v_kernels_of<V_GIVEN, 1, 8>, v_kernels_of<V_GIVEN, 2, 8>}, {nullptr, v_kernels_of<V_GIVEN, 2, 4>}}};
 
 static int hqkv::decode_launch(const hqkv_cache_desc_t* cache_host, const void* q, void* attn_weights, void* attn_output,
                                void* workspace, size_t workspace_bytes, int phases, const PeerArgs& peers, void* stream,
@@ -2254,15 +2280,18 @@ static int hqkv::decode_launch(const hqkv_cache_desc_t* cache_host, const void* 
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
       // all of them with the same (largest) share of the L1 for shared memory: CTAs of kernels that ask for different
       // shares cannot be on an SM together
-      auto opt_in = [](PassKernel f) {
-        HQKV_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(PASS_SMEM)));
+      auto opt_in = [](PassKernel f, size_t bytes) {
+        HQKV_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
         HQKV_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         return 0;
       };
       for (PassKernel f : k_kernels)
-        if (int rc = opt_in(f)) return rc;
-      for (int i = 0; i < 18; ++i)
-        if (int rc = opt_in(v_kernels[i / 6][i / 3 % 2][i % 3])) return rc;
+        if (int rc = opt_in(f, PASS_SMEM)) return rc;
+      for (const auto& mode : v_kernels)
+        for (int four = 0; four < 2; ++four)
+          for (const PassKernel* groups : mode[four])
+            for (int g = 0; groups && g < 3; ++g)
+              if (int rc = opt_in(groups[g], four ? PASS_SMEM : PASS_SMEM_8)) return rc;
       if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
   }
@@ -2285,12 +2314,12 @@ static int hqkv::decode_launch(const hqkv_cache_desc_t* cache_host, const void* 
   if ((phases & 2) && P.nv_ctas > 0) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(VH, P.nv_ctas, P.B);
-    cfg.blockDim = dim3(VTHREADS);
-    cfg.dynamicSmemBytes = PASS_SMEM;
+    cfg.blockDim = dim3(32 * P.v_warps);
+    cfg.dynamicSmemBytes = P.v_warps == 4 ? PASS_SMEM : PASS_SMEM_8;
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    HQKV_CUDA(cudaLaunchKernelEx(&cfg, v_kernels[P.probs_in ? V_GIVEN : P.r4 == MAX_R4 ? V_FOUR : V_FEWER][P.v_pairs - 1][P.gv_shift - 5], P));
+    HQKV_CUDA(cudaLaunchKernelEx(&cfg, v_kernels[P.probs_in ? V_GIVEN : P.r4 == MAX_R4 ? V_FOUR : V_FEWER][P.v_warps == 4][P.v_pairs - 1][P.gv_shift - 5], P));
   }
   return HQKV_OK;
 }
