@@ -548,19 +548,21 @@ __device__ __forceinline__ void softmax_push(float& m, float& l, const float (&x
 // The lane's logits of one chunk: x[j], j = NX logits of head tig.  zq = zero terms of the chunk's first group on, scale =
 // softmax scale (pscale: that of the code term).  codes = address of the chunk's
 // codes, srow0 = scale row of the chunk's first group, qrow = this lane's B fragments of q.
-template <int BITS>
+// WG: groups of 64 or 128, whose scales serve all of the warp's 64 tokens.
+template <int BITS, bool WG>
 __device__ __forceinline__ void k_chunk_logits(float (&x)[KTile<BITS>::NX], uint32_t codes, uint32_t srow0, uint32_t qrow,
                                                const float (*zq)[MAX_R4][KWARPS], float scale, float pscale, int gk_shift) {
   using TL = KTile<BITS>;
-  constexpr bool ONE_GROUP = TL::ONE_GROUP;
+  constexpr bool ONE_GROUP = TL::ONE_GROUP || WG;   // the columns are hi and lo of a head
   constexpr int UNITS = BITS == 4 ? 2 : 1;          // accumulator sets
-  constexpr int NM = ONE_GROUP ? 2 : 4;             // M-tiles per set
+  constexpr int NM = BITS >= 4 ? 2 : 4;             // M-tiles per set
+  constexpr int SETS = WG ? 1 : UNITS;              // of scales
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tig = lane & 3;
   const uint32_t remainder = (g & 1) ? 0xFFFFFFFFu : 0u;
   // scale rows of this lane's B column
-  uint32_t srow[UNITS];
+  uint32_t srow[SETS];
 #pragma unroll
-  for (int u = 0; u < UNITS; ++u) srow[u] = srow0 + ((warp * TL::WTOK + 32 * (ONE_GROUP ? u : (g & 1))) >> gk_shift) * K_SROW + tig * 16;
+  for (int u = 0; u < SETS; ++u) srow[u] = srow0 + ((warp * TL::WTOK + 32 * (ONE_GROUP ? u : (g & 1))) >> gk_shift) * K_SROW + tig * 16;
   // ldmatrix row address of this lane for step 0
   uint32_t kb = codes, kb1 = 0;
   if constexpr (BITS == 8) {
@@ -582,7 +584,7 @@ __device__ __forceinline__ void k_chunk_logits(float (&x)[KTile<BITS>::NX], uint
   // Two 16-channel steps per iteration.  The operands of the next iteration are requested before this one's are used:
   // with four warps per scheduler the round trip to shared memory is not covered by other warps.
   uint32_t Rb[2][2][4];
-  uint4 qb[2], sb4[2][UNITS];
+  uint4 qb[2], sb4[2][SETS];
   auto fetch = [&](int p) {
     uint32_t(&R)[2][4] = Rb[p & 1];
     if constexpr (BITS == 8) {
@@ -600,7 +602,7 @@ __device__ __forceinline__ void k_chunk_logits(float (&x)[KTile<BITS>::NX], uint
     }
     qb[p & 1] = lds128(qrow + p * sizeof(KShared::q[0]));
 #pragma unroll
-    for (int u = 0; u < UNITS; ++u) sb4[p & 1][u] = lds128(srow[u] + p * 64);
+    for (int u = 0; u < SETS; ++u) sb4[p & 1][u] = lds128(srow[u] + p * 64);
   };
   fetch(0);
 #pragma unroll
@@ -616,25 +618,29 @@ __device__ __forceinline__ void k_chunk_logits(float (&x)[KTile<BITS>::NX], uint
 #pragma unroll
         for (int h = 0; h < 2; ++h) qm[k][h] = (q[k][h] ^ 0x80008000u) & remainder;
 #pragma unroll
-      for (int u = 0; u < UNITS; ++u) {
-        const uint4 s4 = sb4[p & 1][u];
-        const uint32_t s[2][2] = {{s4.x, s4.y}, {s4.z, s4.w}};
+      for (int k = 0; k < 2; ++k) {
+        // even columns (qm = 0): hi = fp16(q*s); odd columns (qm = -q): the exact remainder q*s - hi
+        uint32_t b[SETS][2];
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          // even columns (qm = 0): hi = fp16(q*s); odd columns (qm = -q): the exact remainder q*s - hi
-          const uint32_t b0 = h2_fma(q[k][0], s[k][0], h2_mul(qm[k][0], s[k][0]));
-          const uint32_t b1 = h2_fma(q[k][1], s[k][1], h2_mul(qm[k][1], s[k][1]));
-          if constexpr (BITS == 8) {
-            const uint32_t* r = R[k];
-            mma16816(acc[u][0], r[0] & 0x00FF00FFu, r[1] & 0x00FF00FFu, r[2] & 0x00FF00FFu, r[3] & 0x00FF00FFu, b0, b1);
-            mma16816(acc[u][1], __byte_perm(r[0], 0u, 0x4341), __byte_perm(r[1], 0u, 0x4341), __byte_perm(r[2], 0u, 0x4341),
-                     __byte_perm(r[3], 0u, 0x4341), b0, b1);
-          } else {
-            const uint32_t ra = R[u][2 * k], rb = R[u][2 * k + 1], sa = ra >> 8, sb = rb >> 8;
+        for (int u = 0; u < SETS; ++u) {
+          const uint4 s4 = sb4[p & 1][u];
+          const uint32_t s0 = k ? s4.z : s4.x, s1 = k ? s4.w : s4.y;
+          b[u][0] = h2_fma(q[k][0], s0, h2_mul(qm[k][0], s0));
+          b[u][1] = h2_fma(q[k][1], s1, h2_mul(qm[k][1], s1));
+        }
+        if constexpr (BITS == 8) {
+          const uint32_t* r = R[k];
+          mma16816(acc[0][0], r[0] & 0x00FF00FFu, r[1] & 0x00FF00FFu, r[2] & 0x00FF00FFu, r[3] & 0x00FF00FFu, b[0][0], b[0][1]);
+          mma16816(acc[0][1], __byte_perm(r[0], 0u, 0x4341), __byte_perm(r[1], 0u, 0x4341), __byte_perm(r[2], 0u, 0x4341),
+                   __byte_perm(r[3], 0u, 0x4341), b[0][0], b[0][1]);
+        } else {
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-              const uint32_t m = 0x000F000Fu << (4 * i);
-              mma16816(acc[u][i], ra & m, sa & m, rb & m, sb & m, b0, b1);
+          for (int u = 0; u < UNITS; ++u) {
+            const uint32_t shift = BITS == 1 ? 4 * (g >> 2) : 0, ra = R[u][2 * k] >> shift, rb = R[u][2 * k + 1] >> shift, sa = ra >> 8, sb = rb >> 8;
+#pragma unroll
+            for (int i = 0; i < NM; ++i) {
+              const uint32_t m = (BITS == 4 ? 0x000F000Fu : BITS == 2 ? 0x00030003u : 0x00010001u) << (BITS * i);
+              mma16816(acc[u][i], ra & m, sa & m, rb & m, sb & m, b[u < SETS ? u : 0][0], b[u < SETS ? u : 0][1]);
             }
           }
         }
@@ -804,7 +810,7 @@ __device__ __forceinline__ void k_emit(const DecodeParams& P, const TierDev& T, 
 
 // Tokens [t0, t1) of a quantised tier; m, l: the lane's running softmax pair (head tig).  `first`: nothing has run before
 // in this CTA.
-template <int BITS>
+template <int BITS, bool WG>
 __device__ __forceinline__ void k_run(const DecodeParams& P, const TierDev& T, KShared& sh, const Where& w, int t0, int t1,
                                       float& m, float& l, bool& first) {
   using TL = KTile<BITS>;
@@ -876,7 +882,7 @@ __device__ __forceinline__ void k_run(const DecodeParams& P, const TierDev& T, K
       const int in_block = (c % PER_BLOCK) * TL::TOKENS;
       float x[TL::NX];
       const int g0 = in_block >> P.gk_shift;  // first group of the chunk within the block
-      k_chunk_logits<BITS>(x, codes + (c & 1) * K_CODES, srows + g0 * K_SROW, qrow, sh.zq + g0, P.scale, pscale, P.gk_shift);
+      k_chunk_logits<BITS, WG>(x, codes + (c & 1) * K_CODES, srows + g0 * K_SROW, qrow, sh.zq + g0, P.scale, pscale, P.gk_shift);
       k_emit<BITS>(P, T, w, x, at, wt0, m, l);
     }
   }
@@ -1015,8 +1021,8 @@ __device__ __forceinline__ void k_residual_tile(const DecodeParams& P, const Tie
   k_write_tile(P, w, tile, min(16, n - tile_t0), nullptr, static_cast<int64_t>(P.L) - n + tile_t0, m, l);
 }
 
-// ONE_TIER: no CTA has units of two tiers.
-template <bool ONE_TIER>
+// ONE_TIER: no CTA has units of two tiers.  WG: K groups of 64 or 128.
+template <bool ONE_TIER, bool WG>
 __global__ void __launch_bounds__(KTHREADS, K_MIN_CTAS) k_pass_kernel(const __grid_constant__ DecodeParams P) {
   extern __shared__ __align__(128) unsigned char k_smem[];
   KShared& sh = *reinterpret_cast<KShared*>(k_smem);
@@ -1045,16 +1051,16 @@ __global__ void __launch_bounds__(KTHREADS, K_MIN_CTAS) k_pass_kernel(const __gr
   int t0, t1;
   if constexpr (ONE_TIER) {
     const int ti = only_share<false>(P, t0, t1);
-    if (ti == 1) k_run<8>(P, P.tier[1], sh, w, t0, t1, m, l, first);
-    else if (ti == 2) k_run<4>(P, P.tier[2], sh, w, t0, t1, m, l, first);
-    else if (ti == 3) k_run<2>(P, P.tier[3], sh, w, t0, t1, m, l, first);
-    else if (ti == 4) k_run<1>(P, P.tier[4], sh, w, t0, t1, m, l, first);
+    if (ti == 1) k_run<8, WG>(P, P.tier[1], sh, w, t0, t1, m, l, first);
+    else if (ti == 2) k_run<4, WG>(P, P.tier[2], sh, w, t0, t1, m, l, first);
+    else if (ti == 3) k_run<2, WG>(P, P.tier[3], sh, w, t0, t1, m, l, first);
+    else if (ti == 4) k_run<1, WG>(P, P.tier[4], sh, w, t0, t1, m, l, first);
     else plain(ti, t0, t1);
   } else {
-    if (share_of<false>(P, 1, t0, t1)) k_run<8>(P, P.tier[1], sh, w, t0, t1, m, l, first);
-    if (share_of<false>(P, 2, t0, t1)) k_run<4>(P, P.tier[2], sh, w, t0, t1, m, l, first);
-    if (share_of<false>(P, 3, t0, t1)) k_run<2>(P, P.tier[3], sh, w, t0, t1, m, l, first);
-    if (share_of<false>(P, 4, t0, t1)) k_run<1>(P, P.tier[4], sh, w, t0, t1, m, l, first);
+    if (share_of<false>(P, 1, t0, t1)) k_run<8, WG>(P, P.tier[1], sh, w, t0, t1, m, l, first);
+    if (share_of<false>(P, 2, t0, t1)) k_run<4, WG>(P, P.tier[2], sh, w, t0, t1, m, l, first);
+    if (share_of<false>(P, 3, t0, t1)) k_run<2, WG>(P, P.tier[3], sh, w, t0, t1, m, l, first);
+    if (share_of<false>(P, 4, t0, t1)) k_run<1, WG>(P, P.tier[4], sh, w, t0, t1, m, l, first);
     for (int ti = 0; ti <= HQKV_NUM_TIERS; ti += HQKV_NUM_TIERS)
       if (share_of<false>(P, ti, t0, t1)) plain(ti, t0, t1);
   }
@@ -1663,6 +1669,8 @@ __global__ void __launch_bounds__(NW * 32, V_SM_WARPS / NW) v_pass_kernel(const 
   const uint32_t t_z = keep(smem_u32(ws.t[1]) + tig * (8 * NG) + (g & (NG - 1)) * 8);
   constexpr uint32_t TO = sizeof(VWarpShared::raw);   // from raw to t
 
+  int f16_0, f16_1, res_0, res_1;   // (looked up here, where there is time)
+  const bool f16 = share_of<true>(P, 0, f16_0, f16_1), res = share_of<true>(P, HQKV_NUM_TIERS, res_0, res_1);
   // One round per quantised tier, and an empty one where a CTA has none.
   bool begun = false;
 #pragma unroll 1
@@ -1712,8 +1720,11 @@ __global__ void __launch_bounds__(NW * 32, V_SM_WARPS / NW) v_pass_kernel(const 
     auto positions = [&](const int64_t* idx, int left) {
 #pragma unroll
       for (int j = 0; j < NP; ++j) {
-        const int t = mine + 32 * j;
-        at[j] = t < left ? __ldg(reinterpret_cast<const uint32_t*>(idx + t)) : V_NONE;
+        // (Beyond the tier, whose last 32 tokens are all there wherever it holds a multiple of 32: those once more.  Their
+        // probabilities are stored once more, too, and count with scales and zeros of 0.)
+        int t = mine + 32 * j;
+        if (t >= left) t = left - 32 + (t & 31);
+        at[j] = left >= 32 ? __ldg(reinterpret_cast<const uint32_t*>(idx + t)) : V_NONE;
       }
     };
     float x[NP][4];
@@ -1850,8 +1861,8 @@ __global__ void __launch_bounds__(NW * 32, V_SM_WARPS / NW) v_pass_kernel(const 
   // ---- fp16 tier, residual window
 #pragma unroll 1
   for (int ti = 0; ti <= HQKV_NUM_TIERS; ti += HQKV_NUM_TIERS) {
-    int t0, t1;
-    if (!share_of<true>(P, ti, t0, t1)) continue;
+    if (!(ti ? res : f16)) continue;
+    const int t0 = ti ? res_0 : f16_0, t1 = ti ? res_1 : f16_1;
     for (int t = t0 + 16 * warp; t < t1; t += 16 * NW)
       v_plain_tile<MODE>(P, P.tier[ti], sh, reinterpret_cast<__half*>(ws.raw), ws.red, w, t, min(16, t1 - t), ti != 0);
   }
@@ -2216,7 +2227,8 @@ extern "C" int hqkv_decode_attention_gather(const hqkv_cache_desc_t* cache_host,
 }
 
 using PassKernel = void (*)(const DecodeParams);
-static constexpr PassKernel k_kernels[2] = {k_pass_kernel<false>, k_pass_kernel<true>};  // [one tier per CTA]
+static constexpr PassKernel k_kernels[4] = {k_pass_kernel<false, false>, k_pass_kernel<true, false>, k_pass_kernel<false, true>,
+                                            k_pass_kernel<true, true>};  // [groups of more than 32][one tier per CTA]
 template <int MODE, int NP, int NW>
 static constexpr PassKernel v_kernels_of[3] = {v_pass_kernel<5, MODE, NP, NW>, v_pass_kernel<6, MODE, NP, NW>, v_pass_kernel<7, MODE, NP, NW>};
 static constexpr const PassKernel* v_kernels[3][2][2] = {  // [VMode][8, 4 warps][pairs of steps - 1][log2 of the channel group - 5]
@@ -2309,7 +2321,7 @@ static int hqkv::decode_launch(const hqkv_cache_desc_t* cache_host, const void* 
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    HQKV_CUDA(cudaLaunchKernelEx(&cfg, k_kernels[P.k_more < 0], P));
+    HQKV_CUDA(cudaLaunchKernelEx(&cfg, k_kernels[2 * (P.gk_shift > 5) + (P.k_more < 0)], P));
   }
   if ((phases & 2) && P.nv_ctas > 0) {
     cudaLaunchConfig_t cfg = {};
