@@ -106,6 +106,9 @@ _SIGNATURES = {
     "hqkv_flush_join": (C.c_int, [C.POINTER(C.c_int32), C.c_void_p]),
     "hqkv_flush_tiers": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.POINTER(C.c_int32), C.POINTER(C.c_void_p),
                                    C.POINTER(C.c_void_p), C.POINTER(C.c_void_p), C.POINTER(C.c_void_p), C.c_void_p, C.c_void_p]),
+    "hqkv_flush_tiers_beside": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.POINTER(C.c_int32), C.POINTER(C.c_void_p),
+                                   C.POINTER(C.c_void_p), C.POINTER(C.c_void_p), C.POINTER(C.c_void_p), C.c_void_p, C.c_void_p]),
+    "hqkv_flush_finish": (C.c_int, [C.c_void_p]),
     "hqkv_flush_evict": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_int64, C.c_int, C.c_void_p]),
     "hqkv_gather_columns_f16": (C.c_int, [C.c_void_p, C.c_int64, C.c_int, C.c_void_p, C.c_int64, C.c_void_p,
                                           C.c_int64, C.c_void_p]),
@@ -142,8 +145,8 @@ def _load_host():
     module.bind(*[C.cast(getattr(lib, name), C.c_void_p).value for name in
                   ("hqkv_decode_workspace_bytes", "hqkv_decode_attention", "hqkv_decode_attention_headsum",
                    "hqkv_quantize_pack", "hqkv_dequantize_unpack", "hqkv_head_sum", "hqkv_token_importance", "hqkv_block_rank",
-                   "hqkv_flush_workspace_bytes", "hqkv_flush_prepare", "hqkv_flush_join", "hqkv_flush_tiers",
-                   "hqkv_flush_evict")],
+                   "hqkv_flush_workspace_bytes", "hqkv_flush_prepare", "hqkv_flush_join", "hqkv_flush_tiers_beside",
+                   "hqkv_flush_finish", "hqkv_flush_evict")],
                 decode_workspace)
     return module
 

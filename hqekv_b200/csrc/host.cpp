@@ -39,7 +39,8 @@ struct Lib {
   decltype(&hqkv_flush_workspace_bytes) flush_workspace_bytes;
   decltype(&hqkv_flush_prepare) flush_prepare;
   decltype(&hqkv_flush_join) flush_join;
-  decltype(&hqkv_flush_tiers) flush_tiers;
+  decltype(&hqkv_flush_tiers_beside) flush_tiers_beside;
+  decltype(&hqkv_flush_finish) flush_finish;
   decltype(&hqkv_flush_evict) flush_evict;
 } L;
 PyObject* g_workspace_fn = nullptr;  // _lib.decode_workspace(device, bytes, stream): owns the scratch buffers
@@ -66,10 +67,10 @@ inline void* ptr(const at::Tensor* t) { return t ? t->data_ptr() : nullptr; }
 PyObject* none() { Py_RETURN_NONE; }
 
 PyObject* bind(PyObject*, PyObject* args) {
-  unsigned long long a[13];
+  unsigned long long a[14];
   PyObject* fn;
-  if (!PyArg_ParseTuple(args, "KKKKKKKKKKKKKO", &a[0], &a[1], &a[2], &a[3], &a[4], &a[5], &a[6], &a[7], &a[8], &a[9], &a[10],
-                        &a[11], &a[12], &fn))
+  if (!PyArg_ParseTuple(args, "KKKKKKKKKKKKKKO", &a[0], &a[1], &a[2], &a[3], &a[4], &a[5], &a[6], &a[7], &a[8], &a[9], &a[10],
+                        &a[11], &a[12], &a[13], &fn))
     return nullptr;
   int i = 0;
   auto take = [&](auto& f) { f = reinterpret_cast<std::decay_t<decltype(f)>>(a[i++]); };
@@ -84,7 +85,8 @@ PyObject* bind(PyObject*, PyObject* args) {
   take(L.flush_workspace_bytes);
   take(L.flush_prepare);
   take(L.flush_join);
-  take(L.flush_tiers);
+  take(L.flush_tiers_beside);
+  take(L.flush_finish);
   take(L.flush_evict);
   Py_INCREF(fn);
   Py_XDECREF(g_workspace_fn);
@@ -487,7 +489,7 @@ PyObject* flush(PyObject*, PyObject* const* a, Py_ssize_t na) {
   rc = L.flush_prepare(&f, ws.data_ptr(), static_cast<size_t>(ws.numel()), counts, st);
   Py_END_ALLOW_THREADS
   if (rc) return none();
-  struct Join {  // the V side runs on another stream: this one waits for it before the call's memory is let go
+  struct Join {  // the V side and the builds run on other streams: this one waits for them before the call's memory is let go
     cudaStream_t st;
     int32_t* counts;
     bool done = false;
@@ -497,6 +499,7 @@ PyObject* flush(PyObject*, PyObject* const* a, Py_ssize_t na) {
     }
     ~Join() {
       if (!done) L.flush_join(nullptr, st);
+      L.flush_finish(st);
     }
   } join{st, counts};
   for (int t = 0; t < HQKV_NUM_TIERS; ++t)
@@ -538,16 +541,17 @@ PyObject* flush(PyObject*, PyObject* const* a, Py_ssize_t na) {
     }
     at::Tensor& rest = out[side ? kSlotNewV : kSlotNewK];
     if (f.rest) rest = at::empty({B, H, f.rest, D}, half);
-    rc = L.flush_tiers(&f, side, ws.data_ptr(), counts, data, scale, zero, ids, f.rest ? rest.data_ptr() : nullptr, st);
+    rc = L.flush_tiers_beside(&f, side, ws.data_ptr(), counts, data, scale, zero, ids, f.rest ? rest.data_ptr() : nullptr, st);
     if (rc) return none();
   }
   out[kSlotNorm] = norm_out;
-  if (counts[14]) {  // something was evicted on the V side: compact the range vector and the ring
+  if (counts[14]) {  // something was evicted on the V side: compact the range vector and the ring (beside the builds)
     out[kSlotNorm] = at::empty({counts[13]}, half);
     rc = L.flush_evict(&f, ws.data_ptr(), counts[13], out[kSlotNorm].data_ptr(), ptr(ring), ring ? ring->size(1) : 0,
                        ring ? static_cast<int>(ring->size(0)) : 0, st);
     if (rc) return none();
   }
+  if (L.flush_finish(st)) return none();
   PyObject* res = PyTuple_New(kSlots);
   if (!res) return nullptr;
   for (int i = 0; i < kSlots; ++i) {

@@ -759,13 +759,15 @@ __global__ void __launch_bounds__(EVICT_THREADS) evict_kernel(__half* ring, int6
 }  // namespace hqkv
 
 namespace hqkv {
-// What a thread keeps between its flushes: a second stream, two events, and 64 bytes of host memory that the plans write
+// What a thread keeps between its flushes: two streams, six events, and 64 bytes of host memory that the plans write
 // the counts to - they are there as soon as the tokens are counted, while the plan still writes its lists, and no copy has
 // to be launched.  Made on first use, for one device at a time; given back when the thread ends.
 struct FlushLane {
   int dev = -1;
-  cudaStream_t side = nullptr;
+  cudaStream_t side = nullptr, build = nullptr;   // V side; K build
   cudaEvent_t fork = nullptr, join = nullptr;
+  cudaEvent_t ready[2] = {}, built[2] = {};       // a side's outputs may be written; are written
+  bool building[2] = {};                          // ... and the caller's stream does not wait for that yet
   volatile int32_t* host = nullptr;
   int32_t calls = 0;
   int open() {
@@ -784,6 +786,11 @@ struct FlushLane {
     HQKV_CUDA(cudaStreamCreateWithPriority(&side, cudaStreamNonBlocking, greatest));
     HQKV_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
     HQKV_CUDA(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+    HQKV_CUDA(cudaStreamCreateWithPriority(&build, cudaStreamNonBlocking, least));
+    for (int i = 0; i < 2; ++i) {
+      HQKV_CUDA(cudaEventCreateWithFlags(&ready[i], cudaEventDisableTiming));
+      HQKV_CUDA(cudaEventCreateWithFlags(&built[i], cudaEventDisableTiming));
+    }
     dev = now;
     return HQKV_OK;
   }
@@ -791,9 +798,12 @@ struct FlushLane {
     // a plan that nobody waited for (a call that ended early) may still write its counts: not into memory that is given back,
     // nor after those of the next plan
     if (side) cudaStreamSynchronize(side), cudaStreamDestroy(side);
-    if (fork) cudaEventDestroy(fork);
-    if (join) cudaEventDestroy(join);
-    side = nullptr, fork = join = nullptr, dev = -1;
+    if (build) cudaStreamSynchronize(build), cudaStreamDestroy(build);
+    for (cudaEvent_t* e : {&fork, &join, &ready[0], &ready[1], &built[0], &built[1]}) {
+      if (*e) cudaEventDestroy(*e);
+      *e = nullptr;
+    }
+    side = build = nullptr, building[0] = building[1] = false, dev = -1;
   }
   // waits for the counts of a side whose plan is in stream st
   int counts(int v_side, cudaStream_t st, int32_t* out) {
@@ -892,6 +902,34 @@ extern "C" int hqkv_flush_tiers(const hqkv_flush_t* f, int v_side, const void* w
   return hqkv_flush_build(side, side ? &f->v : &f->k, f->B, f->H, f->D, side ? f->group : f->block, s.plan_src[side], s.plan_ids[side],
                           total, counts_host + 8 * side, out_data_host, out_scale_host, out_zero_host, out_ids_host, f->compress,
                           f->rest, rest_out, stream);
+}
+
+// The builds of the two sides beside each other: each waits for little else than its plan and memory, and neither fills the
+// GPU (small flush: 33 and 18 us one after the other).  Neither is put into the caller's stream: what is written to was
+// allocated for that stream, so each waits for what the stream holds by then, and that must not be the other.
+extern "C" int hqkv_flush_tiers_beside(const hqkv_flush_t* f, int v_side, const void* workspace, const int32_t* counts_host,
+                                       void* const* out_data_host, void* const* out_scale_host, void* const* out_zero_host,
+                                       int64_t* const* out_ids_host, void* rest_out, void* stream) {
+  FlushLane& lane = flush_lane;
+  HQKV_REQUIRE(lane.side && lane.calls, "flush_tiers_beside: this thread has prepared no flush");
+  const int side = v_side ? 1 : 0;
+  const cudaStream_t own = side ? lane.side : lane.build;
+  HQKV_CUDA(cudaEventRecord(lane.ready[side], static_cast<cudaStream_t>(stream)));
+  HQKV_CUDA(cudaStreamWaitEvent(own, lane.ready[side], 0));
+  const int rc = hqkv_flush_tiers(f, v_side, workspace, counts_host, out_data_host, out_scale_host, out_zero_host, out_ids_host, rest_out, own);
+  HQKV_CUDA(cudaEventRecord(lane.built[side], own));
+  lane.building[side] = true;
+  return rc;
+}
+
+extern "C" int hqkv_flush_finish(void* stream) {
+  FlushLane& lane = flush_lane;
+  for (int side = 0; side < 2; ++side)
+    if (lane.building[side]) {
+      lane.building[side] = false;
+      HQKV_CUDA(cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), lane.built[side], 0));
+    }
+  return HQKV_OK;
 }
 
 extern "C" int hqkv_flush_evict(const hqkv_flush_t* f, const void* workspace, int64_t survivors, void* norm_kept, void* ring,

@@ -450,6 +450,10 @@ int hqkv_flush_build(int v_side, const hqkv_flush_src_t* src_host, int B, int H,
  *                        Follows every successful hqkv_flush_prepare, in the same thread, before any memory of that
  *                        call is used for something else; the K tiers may be built before it
  *   hqkv_flush_tiers     hqkv_flush_build of one side from that plan
+ *   hqkv_flush_tiers_beside  the same on a stream of the library, after what `stream` holds by now; the plan of the V side
+ *                        must have been joined
+ *   hqkv_flush_finish    `stream` waits for those (nothing to wait for: no effect).  Follows them in the same thread, before
+ *                        any memory of the call is used for something else
  *   hqkv_flush_evict     compacts norm_out to the V-side survivors (-> norm_kept) and moves the survivors' columns of an
  *                        importance ring (fp16 [rows][stride], null: none) to the front, in place
  * `workspace`: hqkv_flush_workspace_bytes(hist + compress) bytes, 256-byte aligned, kept between the calls.
@@ -475,6 +479,10 @@ int hqkv_flush_join(int32_t* counts_host, void* stream);
 int hqkv_flush_tiers(const hqkv_flush_t* flush_host, int v_side, const void* workspace, const int32_t* counts_host,
                      void* const* out_data_host, void* const* out_scale_host, void* const* out_zero_host,
                      int64_t* const* out_ids_host, void* rest_out, void* stream);
+int hqkv_flush_tiers_beside(const hqkv_flush_t* flush_host, int v_side, const void* workspace, const int32_t* counts_host,
+                            void* const* out_data_host, void* const* out_scale_host, void* const* out_zero_host,
+                            int64_t* const* out_ids_host, void* rest_out, void* stream);
+int hqkv_flush_finish(void* stream);
 int hqkv_flush_evict(const hqkv_flush_t* flush_host, const void* workspace, int64_t survivors, void* norm_kept, void* ring,
                      int64_t ring_stride, int ring_rows, void* stream);
 
