@@ -155,25 +155,27 @@ __global__ void __launch_bounds__(128) quantize_cols_kernel(const __half* __rest
 // The usual case of an even, 4-byte aligned channel count: a tile of 128 tokens x 128 channels per CTA, 32 tokens of two
 // adjacent channels per thread, kept in registers (one pass over the source, 128 contiguous bytes per token and warp).
 // Groups of 64 and 128 tokens exchange their minima and maxima through shared memory.  The words and the scale / zero
-// halfs of the tile meet in shared memory too, and each channel's run (16 x BITS bytes of codes) is stored by
-// consecutive threads.  Four small CTAs per SM rather than fewer large ones: a CTA loads, computes and stores in turn, and
-// only other CTAs fill the gaps.  131072 x 8 heads at 4 bits: 77 us (84 with 256-token tiles, two runs per thread one after
-// the other); 2 x 3136 tokens, 2 bits, groups of 64: 8.2 us (16.7 with a thread per channel pair that stored single words).
-// 64 registers a thread: 18 - 26 bytes spilled (-Xptxas -v), 2 % of the instructions of a launch at 8 bits; DRAM 58 % and
-// issue slots 63 % used there.
+// halfs of the tile meet in shared memory too, and each channel's run (16 x BITS bytes of codes, up to 8 of scales or minima)
+// is stored by consecutive threads, at addresses that advance by constants.  Four small CTAs per SM rather than fewer large
+// ones: a CTA loads, computes and stores in turn, and only other CTAs fill the gaps.  Issue slots are what it runs short of
+// (68 % used with 833 instructions per warp and tile), so rows of TS = 128 elements, a cache's, have their token offsets in
+// the load instructions (TS = 0: computed for any distance), the output loops carry no divisions and 64-bit products, and a
+// quotient is one multiplication.  131072 x 8 heads at 8 / 4 / 2 / 1 bits: 66 / 60 / 58 / 60 us (80 / 74 / 74 / 74 before;
+// HBM allows 64 / 53 / 48 / 46); 32768 x 8 at 4 bits 18.7 (23.4).  Loads of the next tile by cp.async in a persistent CTA
+// took 89 us at 4 bits: the loads were not what it waited for.  64 registers a thread, nothing spilled.
 constexpr int QT_SUBS = 4;       // runs of 32 tokens per tile
 constexpr int QT_CH = 128;       // channels per tile
-template <int BITS>
+template <int BITS, int TS>
 __global__ void __launch_bounds__(256, 4) quantize_cols_tile_kernel(const __half* __restrict__ x, int64_t inner, int64_t T,
                                                                     int64_t outer_stride, int64_t t_stride, int gshift,
-                                                                    bool vec_out, uint32_t* __restrict__ code,
+                                                                    int vec_out, uint32_t* __restrict__ code,
                                                                     __half* __restrict__ scale, __half* __restrict__ mn_out) {
   // words of a staged channel row: 16-byte steps, and the rows of neighbouring lanes (every other channel: even channels
   // are staged before odd ones) start in different banks
   constexpr int ROW = QT_SUBS * BITS + 4;
   __shared__ __align__(16) uint32_t s_words[QT_CH * ROW];
   __shared__ __half2 s_lo[256], s_hi[256];
-  __shared__ __half s_scale[QT_CH * QT_SUBS], s_min[QT_CH * QT_SUBS];
+  __shared__ __align__(4) __half s_group[2][QT_SUBS][QT_CH];  // scales and minima: [group of the tile][channel]
   const float levels = static_cast<float>((1 << BITS) - 1);
   const int tid = threadIdx.x, cp = tid & 63, sub = tid >> 6, gs = gshift - 5;  // 2^gs runs per group
   const int64_t subs = T / 32, first = static_cast<int64_t>(blockIdx.x) * QT_SUBS;
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(256, 4) quantize_cols_tile_kernel(const __half
   if (live) {
     const __half* src = x + o * outer_stride + d0 + ch + (first + sub) * 32 * t_stride;
 #pragma unroll
-    for (int t = 0; t < 32; ++t) v[t] = *reinterpret_cast<const __half2*>(src + t * t_stride);
+    for (int t = 0; t < 32; ++t) v[t] = *reinterpret_cast<const __half2*>(src + t * (TS ? TS : t_stride));
     lo = hi = v[0];
 #pragma unroll
     for (int t = 1; t < 32; ++t) {
@@ -228,34 +230,53 @@ __global__ void __launch_bounds__(256, 4) quantize_cols_tile_kernel(const __half
       }
     }
     if ((sub & ((1 << gs) - 1)) == 0) {
-      const int at = ch * QT_SUBS + (sub >> gs);
-      s_scale[at] = sc0;
-      s_min[at] = __low2half(lo);
-      s_scale[at + QT_SUBS] = sc1;
-      s_min[at + QT_SUBS] = __high2half(lo);
+      *reinterpret_cast<__half2*>(&s_group[0][sub >> gs][ch]) = __halves2half2(sc0, sc1);
+      *reinterpret_cast<__half2*>(&s_group[1][sub >> gs][ch]) = lo;
     }
   }
   __syncthreads();
   const int64_t row0 = o * inner + d0, W = subs * BITS, G = subs >> gs, g_first = first >> gs;
   auto staged = [&](int r) { return s_words + ((r & 1) * 64 + (r >> 1)) * ROW; };
-  if (vec_out && nsub == QT_SUBS) {
-    for (int i = tid; i < nch * BITS; i += 256) {
-      const int r = i / BITS, w = i % BITS;
-      reinterpret_cast<uint4*>(code + (row0 + r) * W + first * BITS)[w] = reinterpret_cast<const uint4*>(staged(r))[w];
-    }
+  const int per = 2 - gs;  // log2(groups per tile)
+  if ((vec_out & 1) && nsub == QT_SUBS) {
+    // BITS lanes store a channel's codes, and a step takes 256 / BITS channels: addresses by constant steps
+    const int r = tid / BITS, w = tid % BITS;
+    uint4* dst = reinterpret_cast<uint4*>(code + (row0 + r) * W + first * BITS) + w;
+    const uint4* src = reinterpret_cast<const uint4*>(staged(r)) + w;
+#pragma unroll
+    for (int k = 0; k < (BITS + 1) / 2; ++k)
+      if (r + k * (256 / BITS) < nch) dst[k * (64 / BITS) * W] = src[k * (128 / BITS) * (ROW / 4)];
   } else {
     for (int i = tid; i < nch * QT_SUBS * BITS; i += 256) {
       const int r = i / (QT_SUBS * BITS), w = i % (QT_SUBS * BITS);
       if (w < nsub * BITS) code[(row0 + r) * W + first * BITS + w] = staged(r)[w];
     }
   }
-  const int per = 2 - gs;  // log2(groups per tile)
-  for (int i = tid; i < nch << per; i += 256) {
-    const int r = i >> per, g = i & ((1 << per) - 1);
-    if (g << gs >= nsub) continue;
-    scale[(row0 + r) * G + g_first + g] = s_scale[r * QT_SUBS + g];
-    mn_out[(row0 + r) * G + g_first + g] = s_min[r * QT_SUBS + g];
+  if ((vec_out & 2) && nsub == QT_SUBS) {
+    // a thread stores a channel's scales or its minima
+    const int c = tid & (QT_CH - 1), which = tid >> 7;
+    if (c < nch) {
+      __half* to = (which ? mn_out : scale) + (row0 + c) * G + g_first;
+      const unsigned short* from = reinterpret_cast<const unsigned short*>(&s_group[which][0][c]);
+      if (per == 2) *reinterpret_cast<uint2*>(to) = make_uint2(from[0] | from[QT_CH] << 16, from[2 * QT_CH] | from[3 * QT_CH] << 16);
+      else if (per == 1) *reinterpret_cast<uint32_t*>(to) = from[0] | from[QT_CH] << 16;
+      else *reinterpret_cast<unsigned short*>(to) = from[0];
+    }
+  } else {
+    for (int i = tid; i < nch << per; i += 256) {
+      const int r = i >> per, g = i & ((1 << per) - 1);
+      if (g << gs >= nsub) continue;
+      scale[(row0 + r) * G + g_first + g] = s_group[0][g][r];
+      mn_out[(row0 + r) * G + g_first + g] = s_group[1][g][r];
+    }
   }
+}
+
+template <int BITS>
+static void launch_quant_cols(dim3 tiles, const __half* x, int64_t inner, int64_t T, int64_t outer_stride, int64_t t_stride, int gshift,
+                              int vec_out, uint32_t* code, __half* scale, __half* mn, cudaStream_t st) {
+  auto* f = t_stride == QT_CH ? quantize_cols_tile_kernel<BITS, QT_CH> : quantize_cols_tile_kernel<BITS, 0>;
+  f<<<tiles, 256, 0, st>>>(x, inner, T, outer_stride, t_stride, gshift, vec_out, code, scale, mn);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -476,13 +497,15 @@ extern "C" int hqkv_quantize_pack(const void* x, int64_t rows, int64_t T, int64_
               static_cast<unsigned>(outer));
     if (inner % 2 == 0 && aligned(x, 4) && outer_stride % 2 == 0 && t_stride % 2 == 0) {
       const dim3 tiles(static_cast<unsigned>(ceil_div(T, 32 * QT_SUBS)), grid.y, grid.z);
-      const bool vec_out = aligned(code, 16) && T / 32 * bits % 4 == 0;
+      // codes in pieces of 16 bytes; a tile's scales or minima of a channel (up to 8 bytes) in one
+      const int vec_out = (aligned(code, 16) && T / 32 * bits % 4 == 0 ? 1 : 0) |
+                          (T % (32 * QT_SUBS) == 0 && aligned(s, 8) && aligned(m, 8) ? 2 : 0);
       const int gshift = log2_group(group);
       switch (bits) {
-        case 8: quantize_cols_tile_kernel<8><<<tiles, 256, 0, st>>>(xs, inner, T, outer_stride, t_stride, gshift, vec_out, c, s, m); break;
-        case 4: quantize_cols_tile_kernel<4><<<tiles, 256, 0, st>>>(xs, inner, T, outer_stride, t_stride, gshift, vec_out, c, s, m); break;
-        case 2: quantize_cols_tile_kernel<2><<<tiles, 256, 0, st>>>(xs, inner, T, outer_stride, t_stride, gshift, vec_out, c, s, m); break;
-        default: quantize_cols_tile_kernel<1><<<tiles, 256, 0, st>>>(xs, inner, T, outer_stride, t_stride, gshift, vec_out, c, s, m); break;
+        case 8: launch_quant_cols<8>(tiles, xs, inner, T, outer_stride, t_stride, gshift, vec_out, c, s, m, st); break;
+        case 4: launch_quant_cols<4>(tiles, xs, inner, T, outer_stride, t_stride, gshift, vec_out, c, s, m, st); break;
+        case 2: launch_quant_cols<2>(tiles, xs, inner, T, outer_stride, t_stride, gshift, vec_out, c, s, m, st); break;
+        default: launch_quant_cols<1>(tiles, xs, inner, T, outer_stride, t_stride, gshift, vec_out, c, s, m, st); break;
       }
     } else
     switch (bits) {

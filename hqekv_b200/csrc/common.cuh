@@ -96,15 +96,15 @@ __device__ __forceinline__ uint32_t quant_code_fast(__half x, const QuantGroup& 
   u = fminf(fmaxf(u, 0.f), g.levels);  // fmaxf(NaN, 0) == 0
   return static_cast<uint32_t>(__float2int_rn(u));
 }
-// Codes of 32 values at a time.  The quotient is the correctly rounded fp32 one, as above, from 1/scale in two floats: d * lo is
-// far below half an ulp, so RN(d * hi + d * lo) is RN(d / scale) wherever d / scale keeps more than 2^-46 of it from a rounding
-// boundary, and the quotient of two 11-bit significands keeps 2^-36.  Two instructions for a pair of elements (f32x2)
-// instead of six; a group whose scale is 0, inf or NaN has all codes 0, by one mask for its words instead of a test per
-// element.  Pairs are gathered into bytes and the bytes into words, four elements at a time.  NAN_IN: a NaN element may be in a
+// Codes of 32 values at a time.  Only half(d / scale) is wanted, and half(RN(d * RN(1 / scale))) is that for every pair of
+// 11-bit significands and every exponent between a quotient of 1/8 and one of 256, ties included (all 12 million of them:
+// tests/test_quantise_quotient.py); smaller ones have code 0 and larger ones the largest code either way.  One instruction
+// for a pair of elements (f32x2); a group whose scale is 0, inf or NaN has all codes 0, by one mask for its words instead of a
+// test per element.  Pairs are gathered into bytes and the bytes into words, four elements at a time.  NAN_IN: a NaN element may be in a
 // group whose scale is a number (where minimum and maximum are taken element by element); its code is 0.
 struct QuantPair {  // low half of a pair in one group, high half in another or the same
   __half2 mn;
-  float2 rcp, lo;
+  float2 rcp;
   uint32_t keep0, keep1;  // 0 where all codes of the group are 0
 };
 __device__ __forceinline__ QuantPair quant_pair(__half mn0, __half sc0, __half mn1, __half sc1) {
@@ -112,7 +112,6 @@ __device__ __forceinline__ QuantPair quant_pair(__half mn0, __half sc0, __half m
   g.mn = __halves2half2(mn0, mn1);
   const float s0 = __half2float(sc0), s1 = __half2float(sc1);
   g.rcp = make_float2(__frcp_rn(s0), __frcp_rn(s1));
-  g.lo = make_float2(__fmaf_rn(-g.rcp.x, s0, 1.f) * g.rcp.x, __fmaf_rn(-g.rcp.y, s1, 1.f) * g.rcp.y);
   g.keep0 = s0 > 0.f && s0 < __int_as_float(0x7F800000) ? 0xFFFFFFFFu : 0u;
   g.keep1 = s1 > 0.f && s1 < __int_as_float(0x7F800000) ? 0xFFFFFFFFu : 0u;
   return g;
@@ -123,10 +122,9 @@ template <int BITS, bool NAN_IN>
 __device__ __forceinline__ uint32_t quant_pair_bytes(__half2 x, const QuantPair& g) {
   const float2 d = __half22float2(__hsub2(x, g.mn));
   float2 q;
-  asm("{\n.reg .b64 d, r, l, q;\nmov.b64 d, {%2, %3};\nmov.b64 r, {%4, %5};\nmov.b64 l, {%6, %7};\nmul.rn.f32x2 q, d, l;\n"
-      "fma.rn.f32x2 q, d, r, q;\nmov.b64 {%0, %1}, q;\n}"
+  asm("{\n.reg .b64 d, r, q;\nmov.b64 d, {%2, %3};\nmov.b64 r, {%4, %5};\nmul.rn.f32x2 q, d, r;\nmov.b64 {%0, %1}, q;\n}"
       : "=f"(q.x), "=f"(q.y)
-      : "f"(d.x), "f"(d.y), "f"(g.rcp.x), "f"(g.rcp.y), "f"(g.lo.x), "f"(g.lo.y));
+      : "f"(d.x), "f"(d.y), "f"(g.rcp.x), "f"(g.rcp.y));
   __half2 u = __floats2half2_rn(q.x, q.y);
   if (NAN_IN) u = __hmax2(u, __float2half2_rn(0.f));  // max(NaN, 0) == 0
   u = __hmin2(u, __float2half2_rn(static_cast<float>((1 << BITS) - 1)));
