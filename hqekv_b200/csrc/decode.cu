@@ -1982,8 +1982,9 @@ struct Layout {
   size_t acc_off, logits_off, kpart_off, total;
 };
 
-// How the CTAs of a plane share its units.  A CTA pays about a unit for its prologue, the softmax pairs and the output
-// reduction whatever it walks, and runs about as fast beside three others on its SM as beside one (its chain of loads
+// How the CTAs of a plane share its units.  Whatever it walks, a CTA pays about a unit for its prologue and the softmax pairs,
+// and one more in the V pass for the output (16 x 8 planes of 33 units: V 30 us with four CTAs each, 0.9 of a wave, 33 with nine,
+// 1.95; 20 x 8 planes: 33.8 with three, 34.8 with seven), and runs about as fast beside three others on its SM as beside one (its chain of loads
 // bounds it): up to one wave the number of CTAs that are on the GPU does not count, only how long each is.  Beyond, the time
 // lies between the load of the SMs and that of whole waves (the last wave starts as the first CTAs end).  13 x 16 planes of
 // 15 units: 53 us with two CTAs each (0.7 of a wave), 50 with four; 30 x 8 planes of 15 units: 50 with two (0.8), 55 with
@@ -2048,7 +2049,7 @@ static double divide(DecodeParams& P, int64_t planes, bool v, int warps) {
   double best = 0.;
   for (int n = 1; n == 1 || (total / n >= 2 * unit && (n - 1) * planes < 4 * slots); ++n) {
     const double waves = static_cast<double>(n * planes) / slots;
-    const double cost = (static_cast<double>(total) / n + unit) * (waves <= 1. ? 1. : 0.5 * (waves + ceil(waves)));
+    const double cost = (static_cast<double>(total) / n + (v ? 2 * unit : unit)) * (waves <= 1. ? 1. : 0.5 * (waves + ceil(waves)));
     if (n == 1 || cost < best) best = cost, ctas = n;
   }
   take(ctas, total / ctas, total % ctas);
