@@ -65,6 +65,7 @@ struct DecodeParams {
   // the K pass 8-bit units, which are half as long, count half).
   int k_per, k_more, v_per, v_more;
   int v_pairs, v_warps;    // 32 tokens a warp of the V pass takes at a time: 1, 2; warps per CTA: 8, 4
+  int v_count_at, v_frac;  // an output's word: first bit of the count, bits of its fraction (see v_finish)
   int direct;              // the outputs are finished by whoever adds the last share (see v_finish), not by a CTA that reads them back
   float scale;
   const __half* q;
@@ -1595,17 +1596,21 @@ __device__ __noinline__ void head_sum_chunk(const DecodeParams& P, const TierDev
 }
 
 // A plane's outputs without anybody reading them back: every share's normalised output is added to a 64-bit word as a
-// multiple of 2^-33, together with a count in the bits above; the thread that finds the count complete in what its addition
+// multiple of 2^-frac, together with a count in the bits above; the thread that finds the count complete in what its addition
 // returns has the whole sum and writes it.  (Reductions, a fence, a counter and a last CTA that reads the sums are three round
-// trips to L2 in a row, 2 us; this is one.)  A share is a weighted mean of a part of V, so it and every partial sum stay below
-// 2^17, the largest difference of two halfs, and the sum of up to V_MAX_SHARES roundings below 2^-25, half the smallest half;
-// sums of integers do not depend on their order.  What is not a finite number sets a bit of its own above the count.
+// trips to L2 in a row, 2 us; this is one.)  Sums of integers do not depend on their order.  What is not a finite number below
+// 2^17, the largest difference of two halfs, sets one of the two highest bits, or both.
+//   up to 64 shares: 55 bits of 2^-31 and 7 of count; the roundings add up to 2^-26 at most, and no sum of the shares leaves
+//     the 55 bits;
+//   up to 1023: 52 bits of 2^-33 and 10 of count.  A share is a weighted mean of a part of V, so all partial sums stay below
+//     2^17 as long as the values of V do.  V_MAX_SHARES of them round by 2^-25 at most, half the smallest half.
 // (Not direct - more shares, or peers that get the outputs too: the same words, read by the last CTA.)
-constexpr int V_MAX_SHARES = 256;
-__device__ __forceinline__ float v_output(unsigned long long sum) {
-  const unsigned odd = static_cast<unsigned>(sum >> 61);   // +inf, -inf, NaN
+constexpr int V_MAX_SHARES = 512;
+__device__ __forceinline__ float v_output(unsigned long long sum, int count_at, int frac) {
+  const unsigned odd = static_cast<unsigned>(sum >> 62);   // +inf, -inf, NaN
   if (odd) return odd == 1u ? INFINITY : odd == 2u ? -INFINITY : __int_as_float(0x7FC00000);
-  return static_cast<float>(static_cast<double>(static_cast<long long>(sum << 12) >> 12) * 0x1p-33);
+  const int up = 64 - count_at;
+  return static_cast<float>(static_cast<double>(static_cast<long long>(sum << up) >> up) * (frac == 31 ? 0x1p-31 : 0x1p-33));
 }
 template <int NW>
 __device__ __forceinline__ void v_finish(const DecodeParams& P, const VShared<NW>& sh, int64_t out0) {
@@ -1621,9 +1626,9 @@ __device__ __forceinline__ void v_finish(const DecodeParams& P, const VShared<NW
 #pragma unroll
     for (int i = 0; i < NW; ++i) v += sh.w[i].red[h][c];
     v *= sh.ginv[h];
-    unsigned long long add = P.direct || blockIdx.y == 0 ? 1ull << 52 : 0ull;   // (not direct: one count, for a negative sum to borrow from)
-    if (fabsf(v) < 0x1p17f) add += static_cast<unsigned long long>(__float2ll_rn(v * 0x1p33f));
-    else atomicOr(words + h * D, v > 0.f ? 1ull << 61 : v < 0.f ? 1ull << 62 : 1ull << 63);   // (before the thread's own addition to the word)
+    unsigned long long add = 1ull << P.v_count_at;
+    if (fabsf(v) < 0x1p17f) add += static_cast<unsigned long long>(__float2ll_rn(v * (P.v_frac == 31 ? 0x1p31f : 0x1p33f)));
+    else atomicOr(words + h * D, v > 0.f ? 1ull << 62 : v < 0.f ? 1ull << 63 : 3ull << 62);   // (before the thread's own addition to the word)
     sum[k] = atomicAdd(words + h * D, add) + add;
   }
   if (!P.direct) return;
@@ -1632,7 +1637,8 @@ __device__ __forceinline__ void v_finish(const DecodeParams& P, const VShared<NW
     const int h = h0 + STEP * k;
     if (h >= P.r4) break;
     // (a negative sum borrows from the count)
-    if (((sum[k] + (1ull << 51)) >> 52 & 0x1FFu) == static_cast<unsigned>(P.nv_ctas)) P.out[out0 + h * D + c] = __float2half_rn(v_output(sum[k]));
+    const unsigned count = static_cast<unsigned>((sum[k] + (1ull << (P.v_count_at - 1)) & ~(3ull << 62)) >> P.v_count_at);
+    if (count == static_cast<unsigned>(P.nv_ctas)) P.out[out0 + h * D + c] = __float2half_rn(v_output(sum[k], P.v_count_at, P.v_frac));
   }
 }
 
@@ -1905,7 +1911,7 @@ __global__ void __launch_bounds__(NW * 32, V_SM_WARPS / NW) v_pass_kernel(const 
         o = __floats2half2_rn(static_cast<float>(v.x), static_cast<float>(v.y));
       } else {
         const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2*>(accum + i));
-        o = __floats2half2_rn(v_output(v.x), v_output(v.y));
+        o = __floats2half2_rn(v_output(v.x, P.v_count_at, P.v_frac), v_output(v.y, P.v_count_at, P.v_frac));
       }
       const int64_t at = (static_cast<int64_t>(w.b) * P.nh_q + w.h0) * D + i;
       *reinterpret_cast<__half2*>(P.out + at) = o;
@@ -2047,7 +2053,7 @@ static double divide(DecodeParams& P, int64_t planes, bool v, int warps) {
   }
   int ctas = 1;
   double best = 0.;
-  for (int n = 1; n == 1 || (total / n >= 2 * unit && (n - 1) * planes < 4 * slots); ++n) {
+  for (int n = 1; n == 1 || (n < 1024 && total / n >= 2 * unit && (n - 1) * planes < 4 * slots); ++n) {  // (v_finish counts to 1023)
     const double waves = static_cast<double>(n * planes) / slots;
     const double cost = (static_cast<double>(total) / n + (v ? 2 * unit : unit)) * (waves <= 1. ? 1. : 0.5 * (waves + ceil(waves)));
     if (n == 1 || cost < best) best = cost, ctas = n;
@@ -2282,6 +2288,8 @@ static int hqkv::decode_launch(const hqkv_cache_desc_t* cache_host, const void* 
   P.k_part = reinterpret_cast<float2*>(ws + lay.kpart_off);
   P.v_acc = reinterpret_cast<double*>(ws + lay.acc_off);
   P.direct = !probs_in && peers.n_peers == 0 && !peers.pads && P.nv_ctas <= V_MAX_SHARES;
+  P.v_frac = P.nv_ctas <= 64 ? 31 : 33;
+  P.v_count_at = P.nv_ctas <= 64 ? 55 : 52;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const unsigned VH = static_cast<unsigned>(P.H * P.halves);
   HQKV_REQUIRE(P.nk_ctas <= 65535 && P.nv_ctas <= 65535, "decode: too many chunks");
