@@ -907,12 +907,19 @@ extern "C" int hqkv_flush_tiers(const hqkv_flush_t* f, int v_side, const void* w
 // The builds of the two sides beside each other: each waits for little else than its plan and memory, and neither fills the
 // GPU (small flush: 33 and 18 us one after the other).  Neither is put into the caller's stream: what is written to was
 // allocated for that stream, so each waits for what the stream holds by then, and that must not be the other.
+// Below a line of work (rows that are copied, new ones four times) the six calls for streams and events cost the host more
+// than the overlap gives: there both go into the caller's stream.  us, one after the other / beside: 8 planes, 32 tokens into
+// 12 k 76 / 82, 24 k 87 / 80; 32 planes, 32 into 3 k 73.8 / 74.6, 5 k 78.6 / 74.8; 64 planes, 32 into 4 k 92 / 76; 8 planes,
+// first flush of 4 k 77.7 / 77.4, 8 k 85 / 78, 16 k 114 / 96.
+constexpr int64_t FLUSH_BESIDE_WORK = 160 << 10;
 extern "C" int hqkv_flush_tiers_beside(const hqkv_flush_t* f, int v_side, const void* workspace, const int32_t* counts_host,
                                        void* const* out_data_host, void* const* out_scale_host, void* const* out_zero_host,
                                        int64_t* const* out_ids_host, void* rest_out, void* stream) {
   FlushLane& lane = flush_lane;
   HQKV_REQUIRE(lane.side && lane.calls, "flush_tiers_beside: this thread has prepared no flush");
   const int side = v_side ? 1 : 0;
+  if (static_cast<int64_t>(f->B) * f->H * (f->hist + 4 * f->compress) < FLUSH_BESIDE_WORK)
+    return hqkv_flush_tiers(f, v_side, workspace, counts_host, out_data_host, out_scale_host, out_zero_host, out_ids_host, rest_out, stream);
   const cudaStream_t own = side ? lane.side : lane.build;
   HQKV_CUDA(cudaEventRecord(lane.ready[side], static_cast<cudaStream_t>(stream)));
   HQKV_CUDA(cudaStreamWaitEvent(own, lane.ready[side], 0));
