@@ -6,8 +6,9 @@
 //            plus one (max, sum-exp) pair per CTA and head.
 //   v_pass : every CTA first folds the k_pass pairs into the global (max, sum) of its heads; each
 //            warp then writes the normalised probabilities of its own tokens and accumulates
-//            sum_t exp(logit_t - max) * V^_t over them; the CTA's partial output joins fp64
-//            accumulators, and the last CTA of each (batch, kv head) normalises and writes fp16.
+//            sum_t exp(logit_t - max) * V^_t over them; the CTA's normalised part of the output joins
+//            64-bit words, and whoever completes a word writes fp16 (weights given by the caller, and
+//            outputs that peers get too: the last CTA of each (batch, kv head) writes).
 //
 // The roofline is HBM: every packed word, scale and zero is read exactly once per call and is
 // shared by the query heads of its kv head (GQA).  At 2-4 bits there are 1.6-2.7 codes per byte;
@@ -1022,7 +1023,8 @@ __device__ __forceinline__ void k_residual_tile(const DecodeParams& P, const Tie
   k_write_tile(P, w, tile, min(16, n - tile_t0), nullptr, static_cast<int64_t>(P.L) - n + tile_t0, m, l);
 }
 
-// ONE_TIER: no CTA has units of two tiers.  WG: K groups of 64 or 128.
+// ONE_TIER: no CTA has units of two tiers.  WG: K groups of 64 or 128, which hold all 64 tokens of a warp: one set of scales
+// and B operands instead of two, and at 2 and 1 bits one MMA for hi and lo (8 x 16 k g 64 28.3 -> 27.5 us, 32 x 4 k g 128 28.5 -> 27.5).
 template <bool ONE_TIER, bool WG>
 __global__ void __launch_bounds__(KTHREADS, K_MIN_CTAS) k_pass_kernel(const __grid_constant__ DecodeParams P) {
   extern __shared__ __align__(128) unsigned char k_smem[];
@@ -1101,8 +1103,8 @@ __global__ void __launch_bounds__(KTHREADS, K_MIN_CTAS) k_pass_kernel(const __gr
 // ------------------------------------------------------------------------------------------------
 // V tier, token-major rows of 128 channels.  Every warp of a CTA walks TILES of 64 consecutive tokens of one tier on its own
 // and keeps the output of all 128 channels x four heads in its accumulators from tile to tile, so nothing but the end of the
-// kernel needs the other warps.  (Tiles of 32 where the work is small.)  The contraction runs over tokens, 16 per step.  ldmatrix.trans over 8 token rows x 16 bytes
-// hands lane (g, tig) the 16-bit block g (2 / 4 / 8 channels) of two K-neighbours in one register: an m16n8k16 A fragment.
+// kernel needs the other warps.  (Tiles of 32 where the work is small.)  The contraction runs over tokens, 16 per step.
+// ldmatrix.trans over 8 token rows x 16 bytes hands lane (g, tig) the 16-bit block g (2 / 4 / 8 channels) of two K-neighbours in one register: an m16n8k16 A fragment.
 // As in the K pass the codes enter the tensor pipe as fp16 subnormals (one AND per pair of codes) and the scale - here per
 // token and channel group - is folded into the B operand: out[h][c] = sum_t (p_t * scale_t,G) * code_t,c + sum_t p_t * zero_t,G,
 // with p*scale carried exactly as hi + lo in neighbouring columns (below 4 bits, where 16 bytes are 64 channels, the columns
@@ -1116,8 +1118,11 @@ __global__ void __launch_bounds__(KTHREADS, K_MIN_CTAS) k_pass_kernel(const __gr
 //    formed in registers.  (Formed once and left in shared memory it took as many bytes there, both ways, as the codes.)
 //  * The scales and zeros of a quad are transposed to [group][token] once per tile: pairs as the B operand (and the A
 //    operand of the zero term) wants them.
-//  * One loop serves all widths, with a copy of the MMA part per width: the kernel's code (129 KB with a copy of
-//    everything) has to come from L2 into every SM that has not run it lately, 1 us per 64-byte line of a cold chain.
+//  * One loop serves all widths, with a copy of the MMA part per width: what a kernel executes has to come from L2 into every SM
+//    that has not run it lately, and a CTA of one or two tiles runs little of it twice.
+// us a launch, before (operand through shared memory, a copy of the loop per width, a last CTA that writes) and now: batch 1 of
+// 32 k tokens 12.6 / 10.1, 8 x 16 k g 64 30.7 / 26.0, 4 x 128 k 69 / 57.6, 32 x 4 k g 128 31.8 / 28.2, 57 x 8 planes of 1.6 k in
+// five tiers 71 / 55.  At 8 x 16 k a launch executes 11.1 M warp instructions (12.3 M before); issue slots 44 %, HBM 43 % used.
 // Codes are streamed through ONE tile buffer: the copy of 32 tokens of the next tile is issued when this tile's have been
 // consumed, so a whole tile's work lies between a request and its use.
 // CTAs of eight warps (half as many outputs to add up, half as many softmax pairs to fold), or of four where those fill the SMs better.

@@ -160,8 +160,7 @@ size_t hqkv_decode_workspace_zero_bytes(const hqkv_cache_desc_t* cache_host);
  * packed codes dequantised in registers, softmax in fp32, p.V for every tier, plus the fp16
  * residual window and the fp16 tier.  Two launches chained by programmatic dependent launch: the K pass
  * (logits of every cached token at its logical position, one softmax pair per CTA) and the V pass (folds the
- * pairs, writes the probabilities, accumulates p.V; the last CTA of a (batch, kv head) normalises and
- * writes).  Stands in for qkv_matmul_hqe_2
+ * pairs, writes the probabilities, accumulates p.V; whoever adds the last part of an output writes it).  Stands in for qkv_matmul_hqe_2
  * (quant/hqe_matmul.py:354-451) and everything below it: the layout glue of
  * cuda_bmm_fA_qB_uniform_group (quant/matmul.py:263-299), gemv_forward_cuda_uniform_group and
  * bgemv_kernel_uniform_group_{8,4,2} (quant/csrc/gemv_cuda_uniform.cu:1533-1599, 411-733), the
@@ -450,8 +449,8 @@ int hqkv_flush_build(int v_side, const hqkv_flush_src_t* src_host, int B, int H,
  *                        Follows every successful hqkv_flush_prepare, in the same thread, before any memory of that
  *                        call is used for something else; the K tiers may be built before it
  *   hqkv_flush_tiers     hqkv_flush_build of one side from that plan
- *   hqkv_flush_tiers_beside  the same on a stream of the library, after what `stream` holds by now; the plan of the V side
- *                        must have been joined
+ *   hqkv_flush_tiers_beside  the same on a stream of the library, after what `stream` holds by now (a small flush: in `stream`
+ *                        itself); the plan of the V side must have been joined
  *   hqkv_flush_finish    `stream` waits for those (nothing to wait for: no effect).  Follows them in the same thread, before
  *                        any memory of the call is used for something else
  *   hqkv_flush_evict     compacts norm_out to the V-side survivors (-> norm_kept) and moves the survivors' columns of an
