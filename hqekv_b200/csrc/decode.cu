@@ -6,9 +6,9 @@
 //            plus one (max, sum-exp) pair per CTA and head.
 //   v_pass : every CTA first folds the k_pass pairs into the global (max, sum) of its heads; each
 //            warp then writes the normalised probabilities of its own tokens and accumulates
-//            sum_t exp(logit_t - max) * V^_t over them; the CTA's normalised part of the output joins
-//            64-bit words, and whoever completes a word writes fp16 (weights given by the caller, and
-//            outputs that peers get too: the last CTA of each (batch, kv head) writes).
+//            sum_t exp(logit_t - max) * V^_t over them; the CTA's part of the output joins pairs of
+//            64-bit words, and whoever completes a pair normalises and writes fp16 (weights given by the caller, and
+//            outputs that peers get too: fp64 sums, written by the last CTA of each (batch, kv head)).
 //
 // The roofline is HBM: every packed word, scale and zero is read exactly once per call and is
 // shared by the query heads of its kv head (GQA).  At 2-4 bits there are 1.6-2.7 codes per byte;
@@ -66,7 +66,7 @@ struct DecodeParams {
   // the K pass 8-bit units, which are half as long, count half).
   int k_per, k_more, v_per, v_more;
   int v_pairs, v_warps;    // 32 tokens a warp of the V pass takes at a time: 1, 2; warps per CTA: 8, 4
-  int v_count_at, v_frac;  // an output's word: first bit of the count, bits of its fraction (see v_finish)
+  float v_limit, v_units, v_unit;  // an output's two words (see v_finish): bound of a share; the high word's units per 1, and back
   int direct;              // the outputs are finished by whoever adds the last share (see v_finish), not by a CTA that reads them back
   float scale;
   const __half* q;
@@ -79,7 +79,8 @@ struct DecodeParams {
   __half* out;
   float* logits;   // [B][virtual kv head], see logit_at
   float2* k_part;  // [B][virtual kv head][r4][nk_ctas]
-  double* v_acc;   // [B][nh_q][D] output accumulators (or words, see v_finish): cleared by the K pass, summed into by the V pass
+  double* v_acc;   // [B][nh_q][D] output accumulators (or high words, see v_finish): cleared by the K pass, summed into by the V pass
+  unsigned long long* v_lows;  // ... and the low words (null: the scratch has no room for them)
   __half* peer_out[HQKV_MAX_PEERS];  // copies of `out` in other GPUs' memory (kv-head sharding), n_peers used
   int n_peers;
   int peer_flagged;  // 1: peer_out are flagged 8-byte entries {two fp16 values, call number}, see peer_unpack_kernel
@@ -1085,8 +1086,11 @@ __global__ void __launch_bounds__(KTHREADS, K_MIN_CTAS) k_pass_kernel(const __gr
   // adds into them, starts after this grid has finished); everything above has passed its
   // griddepcontrol.wait, so the previous call is done with them
   if (blockIdx.y == 0) {
-    double* accum = P.v_acc + (static_cast<int64_t>(w.b) * P.nh_q + w.h0) * D;
-    for (int i = tid; i < P.r4 * D; i += KTHREADS) accum[i] = 0.0;
+    const int64_t out0 = (static_cast<int64_t>(w.b) * P.nh_q + w.h0) * D;
+    for (int i = 2 * tid; i < P.r4 * D; i += 2 * KTHREADS) {
+      *reinterpret_cast<double2*>(P.v_acc + out0 + i) = make_double2(0., 0.);
+      if (P.v_lows) *reinterpret_cast<ulonglong2*>(P.v_lows + out0 + i) = make_ulonglong2(0ull, 0ull);
+    }
   }
   // (max, sum) of this CTA per head from the warps' pairs
   __syncthreads();
@@ -1600,50 +1604,88 @@ __device__ __noinline__ void head_sum_chunk(const DecodeParams& P, const TierDev
   }
 }
 
-// A plane's outputs without anybody reading them back: every share's normalised output is added to a 64-bit word as a
-// multiple of 2^-frac, together with a count in the bits above; the thread that finds the count complete in what its addition
-// returns has the whole sum and writes it.  (Reductions, a fence, a counter and a last CTA that reads the sums are three round
-// trips to L2 in a row, 2 us; this is one.)  Sums of integers do not depend on their order.  What is not a finite number below
-// 2^17, the largest difference of two halfs, sets one of the two highest bits, or both.
-//   up to 64 shares: 55 bits of 2^-31 and 7 of count; the roundings add up to 2^-26 at most, and no sum of the shares leaves
-//     the 55 bits;
-//   up to 1023: 52 bits of 2^-33 and 10 of count.  A share is a weighted mean of a part of V, so all partial sums stay below
-//     2^17 as long as the values of V do.  V_MAX_SHARES of them round by 2^-25 at most, half the smallest half.
-// (Not direct - more shares, or peers that get the outputs too: the same words, read by the last CTA.)
-constexpr int V_MAX_SHARES = 512;
-__device__ __forceinline__ float v_output(unsigned long long sum, int count_at, int frac) {
-  const unsigned odd = static_cast<unsigned>(sum >> 62);   // +inf, -inf, NaN
-  if (odd) return odd == 1u ? INFINITY : odd == 2u ? -INFINITY : __int_as_float(0x7FC00000);
-  const int up = 64 - count_at;
-  return static_cast<float>(static_cast<double>(static_cast<long long>(sum << up) >> up) * (frac == 31 ? 0x1p-31 : 0x1p-33));
+// A plane's outputs without anybody reading them back.  An output has two 64-bit words, and every share adds its (not yet
+// normalised) part to them as whole numbers: to the high word multiples of 2^-f, to the low word what that rounds off, in
+// multiples of 2^-(f + 42), and a count to the bits above both.  The thread that finds both counts complete in what its own
+// additions return has the whole sum; it normalises and writes it.  (Reductions, a fence, a counter and a last CTA that reads
+// the sums are three round trips to L2 in a row, 2 us; this is one.)
+//   Bits 0-51 the sum, 52-61 the count (up to V_MAX_SHARES = 512 shares), and of the high word 62 / 63 +inf / -inf, both NaN.
+//   A value of V is below 2^25 (255 x 65504 + 65504) and a probability at most 1, so a plane of up to 2^b tokens sums up to
+//   less than 2^(25 + b) in whatever order and combination of shares: with f = 25 - b that is 2^50 units.  The low word's shares
+//   are at most 2^41 units each.
+//   What the words round off is 2^-(68 - b) a share at most, 2^-42 of an output for 512 shares of 128 k tokens (the smallest
+//   half is 2^-24, and its parts come as fp32 sums): the sum of fp32 parts, like the fp64 sum of the other form below, but the same
+//   whatever the order.  One word with the fraction that is left beside the largest V (27 bits) rounded small outputs visibly.
+// Whether high and low word become complete in the same thread's additions is for the memory system to say; mostly they do.
+// Otherwise the thread with the high word marks the low one: either it finds it complete by then, or whoever completes it
+// finds the mark and takes the high word.
+// (Not direct - more shares, more than 4 M tokens, or peers that get the outputs too: fp64 sums, read by the last CTA.)
+constexpr int V_MAX_SHARES = 512, V_MAX_BITS = 22, V_COUNT_AT = 52, V_LOW_BITS = 42;
+constexpr unsigned long long V_MARK = 1ull << 63;
+__device__ __forceinline__ int v_count(unsigned long long word) { return static_cast<int>((word + (1ull << (V_COUNT_AT - 1)) & ~(3ull << 62)) >> V_COUNT_AT); }  // (a negative sum borrows from the count)
+__device__ __forceinline__ double v_part(unsigned long long word) {
+  return static_cast<double>(static_cast<long long>(word << (64 - V_COUNT_AT)) >> (64 - V_COUNT_AT));
 }
-template <int NW>
+template <int NW, bool FOUR>
 __device__ __forceinline__ void v_finish(const DecodeParams& P, const VShared<NW>& sh, int64_t out0) {
   constexpr int EACH = MAX_R4 * D / (NW * 32), STEP = MAX_R4 / EACH;   // outputs of a thread: heads h0, h0 + STEP, ...
   const int c = threadIdx.x & (D - 1), h0 = threadIdx.x / D;
-  unsigned long long* words = reinterpret_cast<unsigned long long*>(P.v_acc) + out0 + c;
-  unsigned long long sum[EACH];
+  unsigned long long* high = reinterpret_cast<unsigned long long*>(P.v_acc) + out0 + c;
+  unsigned long long* low = P.v_lows + out0 + c;
+  unsigned long long a[EACH], b[EACH];
 #pragma unroll
   for (int k = 0; k < EACH; ++k) {
     const int h = h0 + STEP * k;
-    if (h >= P.r4) break;
+    if (!FOUR && h >= P.r4) break;
     float v = 0.f;
 #pragma unroll
     for (int i = 0; i < NW; ++i) v += sh.w[i].red[h][c];
-    v *= sh.ginv[h];
-    unsigned long long add = 1ull << P.v_count_at;
-    if (fabsf(v) < 0x1p17f) add += static_cast<unsigned long long>(__float2ll_rn(v * (P.v_frac == 31 ? 0x1p31f : 0x1p33f)));
-    else atomicOr(words + h * D, v > 0.f ? 1ull << 62 : v < 0.f ? 1ull << 63 : 3ull << 62);   // (before the thread's own addition to the word)
-    sum[k] = atomicAdd(words + h * D, add) + add;
+    a[k] = b[k] = 1ull << V_COUNT_AT;
+    if (fabsf(v) < P.v_limit) {
+      const float units = rintf(v * P.v_units);
+      a[k] += static_cast<unsigned long long>(__float2ll_rn(units));
+      b[k] += static_cast<unsigned long long>(__float2ll_rn(fmaf(v, P.v_units, -units) * static_cast<float>(1ull << V_LOW_BITS)));  // (the difference is exact)
+    } else {
+      atomicOr(high + h * D, v > 0.f ? 1ull << 62 : v < 0.f ? 1ull << 63 : 3ull << 62);   // (before the thread's own addition to the word)
+    }
   }
-  if (!P.direct) return;
 #pragma unroll
   for (int k = 0; k < EACH; ++k) {
     const int h = h0 + STEP * k;
-    if (h >= P.r4) break;
-    // (a negative sum borrows from the count)
-    const unsigned count = static_cast<unsigned>((sum[k] + (1ull << (P.v_count_at - 1)) & ~(3ull << 62)) >> P.v_count_at);
-    if (count == static_cast<unsigned>(P.nv_ctas)) P.out[out0 + h * D + c] = __float2half_rn(v_output(sum[k], P.v_count_at, P.v_frac));
+    if (!FOUR && h >= P.r4) break;
+    b[k] += atomicAdd(low + h * D, b[k]);
+    a[k] += atomicAdd(high + h * D, a[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < EACH; ++k) {
+    const int h = h0 + STEP * k;
+    if (!FOUR && h >= P.r4) break;
+    const bool high_done = v_count(a[k]) == P.nv_ctas;
+    bool low_done = v_count(b[k]) == P.nv_ctas;
+    if (high_done && !low_done) {
+      // (the missing additions were issued before those that the high word has: mostly another look is enough)
+#pragma unroll 1
+      for (int looks = 0; looks < 4 && !low_done; ++looks) {
+        b[k] = *const_cast<volatile unsigned long long*>(low + h * D);
+        low_done = v_count(b[k]) == P.nv_ctas;
+      }
+      if (!low_done) {
+        __threadfence();   // (whoever finds the mark finds the high word complete)
+        b[k] = atomicOr(low + h * D, V_MARK);
+        low_done = v_count(b[k]) == P.nv_ctas;
+      }
+    } else if (!high_done && low_done) {
+      low_done = (b[k] & V_MARK) != 0;
+      if (low_done) {
+        __threadfence();
+        a[k] = atomicAdd(high + h * D, 0ull);
+      }
+    }
+    if (!low_done) continue;
+    const unsigned odd = static_cast<unsigned>(a[k] >> 62);
+    double sum = (v_part(a[k]) + v_part(b[k]) * (1. / (1ull << V_LOW_BITS))) * P.v_unit;
+    if (odd) sum = odd == 1u ? INFINITY : odd == 2u ? -INFINITY : __int_as_float(0x7FC00000);
+    P.out[out0 + h * D + c] = __float2half_rn(static_cast<float>(sum) * sh.ginv[h]);
   }
 }
 
@@ -1880,20 +1922,20 @@ __global__ void __launch_bounds__(NW * 32, V_SM_WARPS / NW) v_pass_kernel(const 
   __syncthreads();
   // ---- the output of this CTA (warps added in index order) joins those of its plane
   const int64_t out0 = (static_cast<int64_t>(w.b) * P.nh_q + w.h0) * D;
-  // Weights given by the caller may add up to anything: fp64 reductions, whose sum depends on the order of the fp32 partials
-  // only below 2^-53.
+  // (Weights given by the caller may add up to anything.)  fp64 reductions: their sum depends on the order of the fp32
+  // partials only below 2^-53.
   double* accum = P.v_acc + out0;
-  if constexpr (MODE == V_GIVEN) {
+  if (MODE != V_GIVEN && P.direct) {
+    v_finish<NW, MODE == V_FOUR>(P, sh, out0);
+  } else {
     for (int k = tid; k < P.r4 * D; k += VTHREADS) {
       float v = 0.f;
 #pragma unroll
       for (int i = 0; i < NW; ++i) v += sh.w[i].red[k >> 7][k & (D - 1)];
       atomicAdd(accum + k, static_cast<double>(v));
     }
-  } else {
-    v_finish(P, sh, out0);
   }
-  // ---- not direct: the last CTA of this (batch, virtual kv head) writes the output
+  // ---- not direct: the last CTA of this (batch, virtual kv head) normalises and writes the output
   if (tid == 0) sh.is_last = 0u;
   if (!P.direct) {
     __syncthreads();
@@ -1910,14 +1952,9 @@ __global__ void __launch_bounds__(NW * 32, V_SM_WARPS / NW) v_pass_kernel(const 
   if (!P.direct && sh.is_last) {
     __threadfence();
     for (int i = tid * 2; i < P.r4 * D; i += VTHREADS * 2) {
-      __half2 o;
-      if constexpr (MODE == V_GIVEN) {
-        const double2 v = __ldcg(reinterpret_cast<const double2*>(accum + i));
-        o = __floats2half2_rn(static_cast<float>(v.x), static_cast<float>(v.y));
-      } else {
-        const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2*>(accum + i));
-        o = __floats2half2_rn(v_output(v.x, P.v_count_at, P.v_frac), v_output(v.y, P.v_count_at, P.v_frac));
-      }
+      const double2 v = __ldcg(reinterpret_cast<const double2*>(accum + i));
+      const float inv = MODE == V_GIVEN ? 1.f : sh.ginv[i >> 7];
+      const __half2 o = __floats2half2_rn(static_cast<float>(v.x) * inv, static_cast<float>(v.y) * inv);
       const int64_t at = (static_cast<int64_t>(w.b) * P.nh_q + w.h0) * D + i;
       *reinterpret_cast<__half2*>(P.out + at) = o;
       // kv-head sharding: the same rows go straight into every peer's copy of the gathered output
@@ -1990,7 +2027,7 @@ static int ilog2(int v) {
 }
 
 struct Layout {
-  size_t acc_off, logits_off, kpart_off, total;
+  size_t acc_off, logits_off, kpart_off, lows_off, total;   // (scratch that ends before the low words is taken, too)
 };
 
 // How the CTAs of a plane share its units.  Whatever it walks, a CTA pays about a unit for its prologue and the softmax pairs,
@@ -2166,7 +2203,8 @@ static int build_params(const hqkv_cache_desc_t* c, DecodeParams& P, Layout& lay
   off = (off + 255) & ~static_cast<size_t>(255);
   lay.kpart_off = off;
   off += static_cast<size_t>(c->B) * c->nh_q * P.nk_ctas * sizeof(float2);
-  lay.total = (off + 255) & ~static_cast<size_t>(255);
+  lay.lows_off = (off + 255) & ~static_cast<size_t>(255);
+  lay.total = lay.lows_off + ((static_cast<size_t>(c->B) * c->nh_q * D * sizeof(unsigned long long) + 255) & ~static_cast<size_t>(255));
   return HQKV_OK;
 }
 
@@ -2280,8 +2318,8 @@ static int hqkv::decode_launch(const hqkv_cache_desc_t* cache_host, const void* 
   P.mask_bstride = mask_bstride;
   P.mask_hstride = mask_hstride;
   HQKV_REQUIRE(aligned(workspace, 256), "decode: workspace must be 256-byte aligned");
-  if (workspace_bytes < lay.total)
-    return fail(HQKV_E_WORKSPACE, "decode: workspace holds %zu bytes, %zu needed", workspace_bytes, lay.total);
+  if (workspace_bytes < lay.lows_off)
+    return fail(HQKV_E_WORKSPACE, "decode: workspace holds %zu bytes, %zu needed", workspace_bytes, lay.lows_off);
   unsigned char* ws = static_cast<unsigned char*>(workspace);
   P.q = static_cast<const __half*>(q);
   P.weights = static_cast<__half*>(attn_weights);
@@ -2292,9 +2330,12 @@ static int hqkv::decode_launch(const hqkv_cache_desc_t* cache_host, const void* 
   P.logits = reinterpret_cast<float*>(ws + lay.logits_off);
   P.k_part = reinterpret_cast<float2*>(ws + lay.kpart_off);
   P.v_acc = reinterpret_cast<double*>(ws + lay.acc_off);
-  P.direct = !probs_in && peers.n_peers == 0 && !peers.pads && P.nv_ctas <= V_MAX_SHARES;
-  P.v_frac = P.nv_ctas <= 64 ? 31 : 33;
-  P.v_count_at = P.nv_ctas <= 64 ? 55 : 52;
+  if (workspace_bytes >= lay.total) P.v_lows = reinterpret_cast<unsigned long long*>(ws + lay.lows_off);
+  const int bits = ilog2(P.L);
+  P.direct = !probs_in && peers.n_peers == 0 && !peers.pads && P.v_lows && P.nv_ctas <= V_MAX_SHARES && bits <= V_MAX_BITS;
+  P.v_limit = ldexpf(1.f, 25 + bits);
+  P.v_units = ldexpf(1.f, 25 - bits);
+  P.v_unit = ldexpf(1.f, bits - 25);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const unsigned VH = static_cast<unsigned>(P.H * P.halves);
   HQKV_REQUIRE(P.nk_ctas <= 65535 && P.nv_ctas <= 65535, "decode: too many chunks");
@@ -2421,7 +2462,7 @@ extern "C" int hqkv_decode_weighted_sum(const hqkv_cache_desc_t* cache_host, con
     Layout lay;
     int rc = build_params(cache_host, P, lay, 2);
     if (rc) return rc;
-    HQKV_REQUIRE(workspace && workspace_bytes >= lay.total, "decode_weighted_sum: workspace too small");
+    HQKV_REQUIRE(workspace && workspace_bytes >= lay.lows_off, "decode_weighted_sum: workspace too small");
     HQKV_CUDA(cudaMemsetAsync(static_cast<unsigned char*>(workspace) + lay.acc_off, 0, lay.logits_off - lay.acc_off,
                               static_cast<cudaStream_t>(stream)));
   }
@@ -2487,7 +2528,9 @@ extern "C" size_t hqkv_decode_static_scratch_bytes(void) { return HQKV_STATIC_SC
 
 extern "C" int hqkv_decode_attention_static(const hqkv_cache_desc_t* cache_host, const void* q, void* attn_weights,
                                             void* attn_output, void* stream) {
-  const size_t need = hqkv_decode_workspace_bytes(cache_host);
+  DecodeParams P;
+  Layout lay;
+  const size_t need = build_params(cache_host, P, lay) == HQKV_OK ? lay.lows_off : 0;
   if (need == 0)  // invalid descriptor: let the regular path produce the precise message
     return hqkv_decode_attention(cache_host, q, attn_weights, attn_output, nullptr, 0, stream);
   if (need > HQKV_STATIC_SCRATCH_BYTES)

@@ -149,7 +149,8 @@ typedef struct {
   hqkv_tier_t tier[HQKV_NUM_TIERS];
 } hqkv_cache_desc_t;
 
-/* Bytes of scratch hqkv_decode_attention needs for this cache on the current device (0 on invalid input). */
+/* Bytes of scratch hqkv_decode_attention wants for this cache on the current device (0 on invalid input).  The last
+ * 8 * B * nh_q * D of them, in whole 256 bytes, only save a round trip at the end of the call: without them it still runs. */
 size_t hqkv_decode_workspace_bytes(const hqkv_cache_desc_t* cache_host);
 /* Leading part of that scratch (arrival counters) that must be zero before a call:
  * HQKV_WS_HEADER_BYTES whatever the cache; 0 on invalid input. */
@@ -295,8 +296,8 @@ int hqkv_peer_unpack(const void* recv, void* gathered, int rank, int world, int 
  * decode kernel comes from a fixed array of HQKV_STATIC_SCRATCH_BYTES inside the library, resident on
  * every GPU that loads it for the life of the process.  The call allocates and frees nothing.
  *
- *  - Limit: caches whose hqkv_decode_workspace_bytes() exceeds HQKV_STATIC_SCRATCH_BYTES are refused
- *    with HQKV_E_WORKSPACE (16 MiB covers batch 1 up to ~100k cached tokens with 32 query heads; the
+ *  - Limit: caches whose hqkv_decode_workspace_bytes(), less 8 * B * nh_q * D (see there), exceeds
+ *    HQKV_STATIC_SCRATCH_BYTES are refused with HQKV_E_WORKSPACE (16 MiB covers batch 1 up to ~100k cached tokens with 32 query heads; the
  *    need grows with B * nh_q * L * 4 bytes).
  *  - The first call on each device looks up the array's device address (cudaGetSymbolAddress with
  *    that device current).  Make that first call outside any stream capture, and make it at start-up,
