@@ -1686,6 +1686,7 @@ __device__ __forceinline__ void v_finish(const DecodeParams& P, const VShared<NW
     double sum = (v_part(a[k]) + v_part(b[k]) * (1. / (1ull << V_LOW_BITS))) * P.v_unit;
     if (odd) sum = odd == 1u ? INFINITY : odd == 2u ? -INFINITY : __int_as_float(0x7FC00000);
     P.out[out0 + h * D + c] = __float2half_rn(static_cast<float>(sum) * sh.ginv[h]);
+    high[h * D] = low[h * D] = 0ull;   // (nobody else comes: a V pass without a K pass before it starts from zero, too)
   }
 }
 
@@ -1953,6 +1954,7 @@ __global__ void __launch_bounds__(NW * 32, V_SM_WARPS / NW) v_pass_kernel(const 
     __threadfence();
     for (int i = tid * 2; i < P.r4 * D; i += VTHREADS * 2) {
       const double2 v = __ldcg(reinterpret_cast<const double2*>(accum + i));
+      *reinterpret_cast<double2*>(accum + i) = make_double2(0., 0.);   // (as in v_finish)
       const float inv = MODE == V_GIVEN ? 1.f : sh.ginv[i >> 7];
       const __half2 o = __floats2half2_rn(static_cast<float>(v.x) * inv, static_cast<float>(v.y) * inv);
       const int64_t at = (static_cast<int64_t>(w.b) * P.nh_q + w.h0) * D + i;

@@ -217,7 +217,7 @@ int hqkv_decode_attention_headsum(const hqkv_cache_desc_t* cache_host, const voi
 /*
  * The same call restricted to one of its launches: phases = 1 runs the K pass only (logits and
  * per-CTA softmax statistics into the workspace), 2 the V pass only (needs the workspace a K-only
- * call of the same cache left), 3 both.  Serves
+ * call of the same cache left; any number of V-only calls may follow it), 3 both.  Serves
  * cuda_bmm_forward_qk_group_hq / cuda_bmm_forward_wv_group_hq style callers and the timing of the two
  * halves; the split itself has no counterpart in the reference.
  */
