@@ -915,6 +915,7 @@ constexpr int64_t FLUSH_BESIDE_WORK = 160 << 10;
 extern "C" int hqkv_flush_tiers_beside(const hqkv_flush_t* f, int v_side, const void* workspace, const int32_t* counts_host,
                                        void* const* out_data_host, void* const* out_scale_host, void* const* out_zero_host,
                                        int64_t* const* out_ids_host, void* rest_out, void* stream) {
+  HQKV_REQUIRE(f && workspace && counts_host, "flush_tiers_beside: null pointer");
   FlushLane& lane = flush_lane;
   HQKV_REQUIRE(lane.side && lane.calls, "flush_tiers_beside: this thread has prepared no flush");
   const int side = v_side ? 1 : 0;
@@ -924,19 +925,26 @@ extern "C" int hqkv_flush_tiers_beside(const hqkv_flush_t* f, int v_side, const 
   HQKV_CUDA(cudaEventRecord(lane.ready[side], static_cast<cudaStream_t>(stream)));
   HQKV_CUDA(cudaStreamWaitEvent(own, lane.ready[side], 0));
   const int rc = hqkv_flush_tiers(f, v_side, workspace, counts_host, out_data_host, out_scale_host, out_zero_host, out_ids_host, rest_out, own);
-  HQKV_CUDA(cudaEventRecord(lane.built[side], own));
+  if (const int failed = check_cuda(cudaEventRecord(lane.built[side], own), "cudaEventRecord")) {
+    cudaStreamSynchronize(own);   // (there is no event to wait for, and the caller may let the memory go)
+    return failed;
+  }
   lane.building[side] = true;
   return rc;
 }
 
 extern "C" int hqkv_flush_finish(void* stream) {
   FlushLane& lane = flush_lane;
+  int rc = HQKV_OK;
   for (int side = 0; side < 2; ++side)
     if (lane.building[side]) {
       lane.building[side] = false;
-      HQKV_CUDA(cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), lane.built[side], 0));
+      if (const int failed = check_cuda(cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), lane.built[side], 0), "cudaStreamWaitEvent")) {
+        cudaEventSynchronize(lane.built[side]);
+        rc = failed;
+      }
     }
-  return HQKV_OK;
+  return rc;
 }
 
 extern "C" int hqkv_flush_evict(const hqkv_flush_t* f, const void* workspace, int64_t survivors, void* norm_kept, void* ring,

@@ -287,3 +287,12 @@ def test_tier_schedule_matches_reference_layer(name):
             assert f"c{call}_bit_num" not in z.files
         assert [sch.current_length, sch.history_reserve_length] == [int(v) for v in z[f"c{call}_state"][:2]], f"{name} call {call}"
     assert flushes >= 2
+
+
+def test_flush_tiers_beside_refuses_null_pointers(lib):
+    """Like hqkv_flush_tiers, and before it looks at anything else."""
+    L = lib.lib
+    for call in (L.hqkv_flush_tiers, L.hqkv_flush_tiers_beside):
+        assert call(None, 0, None, None, None, None, None, None, None, None) == -1
+        assert b"null pointer" in L.hqkv_last_error()
+    assert L.hqkv_flush_finish(None) == 0   # nothing to wait for
