@@ -556,7 +556,7 @@ template <int BITS, bool WG>
 __device__ __forceinline__ void k_chunk_logits(float (&x)[KTile<BITS>::NX], uint32_t codes, uint32_t srow0, uint32_t qrow,
                                                const float (*zq)[MAX_R4][KWARPS], float scale, float pscale, int gk_shift) {
   using TL = KTile<BITS>;
-  constexpr bool ONE_GROUP = TL::ONE_GROUP || WG;   // the columns are hi and lo of a head
+  constexpr bool ONE_GROUP = TL::ONE_GROUP;         // the columns are hi and lo of a head
   constexpr int UNITS = BITS == 4 ? 2 : 1;          // accumulator sets
   constexpr int NM = BITS >= 4 ? 2 : 4;             // M-tiles per set
   constexpr int SETS = WG ? 1 : UNITS;              // of scales
@@ -639,10 +639,10 @@ __device__ __forceinline__ void k_chunk_logits(float (&x)[KTile<BITS>::NX], uint
         } else {
 #pragma unroll
           for (int u = 0; u < UNITS; ++u) {
-            const uint32_t shift = BITS == 1 ? 4 * (g >> 2) : 0, ra = R[u][2 * k] >> shift, rb = R[u][2 * k + 1] >> shift, sa = ra >> 8, sb = rb >> 8;
+            const uint32_t ra = R[u][2 * k], rb = R[u][2 * k + 1], sa = ra >> 8, sb = rb >> 8;
 #pragma unroll
             for (int i = 0; i < NM; ++i) {
-              const uint32_t m = (BITS == 4 ? 0x000F000Fu : BITS == 2 ? 0x00030003u : 0x00010001u) << (BITS * i);
+              const uint32_t m = 0x000F000Fu << (4 * i);
               mma16816(acc[u][i], ra & m, sa & m, rb & m, sb & m, b[u < SETS ? u : 0][0], b[u < SETS ? u : 0][1]);
             }
           }
@@ -1024,8 +1024,9 @@ __device__ __forceinline__ void k_residual_tile(const DecodeParams& P, const Tie
   k_write_tile(P, w, tile, min(16, n - tile_t0), nullptr, static_cast<int64_t>(P.L) - n + tile_t0, m, l);
 }
 
-// ONE_TIER: no CTA has units of two tiers.  WG: K groups of 64 or 128, which hold all 64 tokens of a warp: one set of scales
-// and B operands instead of two, and at 2 and 1 bits one MMA for hi and lo (8 x 16 k g 64 28.3 -> 27.5 us, 32 x 4 k g 128 28.5 -> 27.5).
+// ONE_TIER: no CTA has units of two tiers.  WG: K groups of 64 or 128, which hold all 64 tokens of a warp: at 4 bits one set of
+// scales and B operands instead of two.  (At 2 and 1 bits one MMA with hi and lo in neighbouring columns would do, too: 8 x 16 k g 64
+// 27.5 us instead of 28.3.  But then the logits of the same codes and scales depend on the size of the group, in their last bits.)
 template <bool ONE_TIER, bool WG>
 __global__ void __launch_bounds__(KTHREADS, K_MIN_CTAS) k_pass_kernel(const __grid_constant__ DecodeParams P) {
   extern __shared__ __align__(128) unsigned char k_smem[];
