@@ -1403,7 +1403,9 @@ __device__ __forceinline__ void v_tile(float (&acc)[8][4], const uint32_t (&p)[N
     cp_async_wait<NP>();
     __syncwarp();
     v_pair_mma<BITS, GV>(acc, ps, r.lm + j * 512 * BITS, t_s + j * (64 * (D >> GV)), rem);
-    // (the MMAs have used the codes, and keep the warp together: no lane still reads them)
+    // The codes make room for the next tile's.  At 8, 4 and 2 bits ldmatrix has read them for the whole warp; at 1 bit every lane
+    // reads for itself, and the MMAs between need not stay before the copies.
+    if constexpr (BITS == 1) __syncwarp();
     if (refill) v_request_pair<BITS, true>(r, j, 0);
     cp_async_commit();
     p0 = p[NP - 1][0], p1 = p[NP - 1][1];
