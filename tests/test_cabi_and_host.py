@@ -296,3 +296,50 @@ def test_flush_tiers_beside_refuses_null_pointers(lib):
         assert call(None, 0, None, None, None, None, None, None, None, None) == -1
         assert b"null pointer" in L.hqkv_last_error()
     assert L.hqkv_flush_finish(None) == 0   # nothing to wait for
+
+
+def test_decode_division_is_the_best_of_all(lib):
+    """The K pass's CTAs per plane (the softmax pairs in the workspace tell their number): CTAs of one tier where those fit one
+    wave of 592, else the number of shares that takes the least time by the model that the library states, the first of equals."""
+    import math
+    import random
+    rng = random.Random(1)
+    tokens_of, cost_of = {16: 64, 8: 128, 4: 256, 2: 256, 1: 256}, {16: 8, 8: 5, 4: 8, 2: 8, 1: 8}
+
+    def expected(planes, tiers):
+        units = [(-(-n // tokens_of[b]), n, b) for b, n in tiers]
+        for budget in range(10, 17):
+            ctas = sum(-(-n // (tokens_of[b] * max(1, budget // cost_of[b]))) for _, n, b in units)
+            if ctas * planes <= 592:
+                return ctas
+        total = sum(u * cost_of[b] for u, _, b in units)
+        best, ctas, n = 0.0, 0, 1
+        while n == 1 or (n < 1024 and total // n >= 16 and (n - 1) * planes < 4 * 592):
+            waves = n * planes / 592
+            cost = (total / n + 8) * (1.0 if waves <= 1 else 0.5 * (waves + math.ceil(waves)))
+            if n == 1 or cost < best:
+                best, ctas = cost, n
+            n += 1
+        return ctas
+
+    up = lambda n: (n + 255) // 256 * 256  # noqa: E731
+    for _ in range(400):
+        batch, kv = round(math.exp(rng.uniform(0, math.log(128)))), rng.choice((1, 2, 4, 8))
+        length = round(math.exp(rng.uniform(math.log(64), math.log(140000))))
+        shares = [rng.random() * (rng.random() < 0.7) for _ in range(5)]
+        desc = lib.CacheDesc()
+        desc.B, desc.H, desc.nh_q, desc.D, desc.group_k, desc.group_v = batch, kv, 4 * kv, 128, 32, 32
+        desc.new_k = desc.new_v = 4096
+        desc.n_new = rng.randint(1, 200)
+        tiers = [(16, desc.n_new)]
+        for t, bits in enumerate((16, 8, 4, 2, 1)):
+            n = int(length * shares[t] / (sum(shares) or 1)) // 32 * 32
+            tier = desc.tier[t]
+            tier.bits, tier.n_k, tier.n_v = bits, n, n
+            for name in ("k_data", "k_idx", "k_scale", "k_zero", "v_data", "v_idx", "v_scale", "v_zero"):
+                setattr(tier, name, 4096)   # (nothing reads them)
+            tiers.append((bits, n))
+        rows, tokens = batch * 4 * kv, sum(n for _, n in tiers)
+        fixed = up(up(12288 + rows * 128 * 8) + rows * tokens * 4)
+        pairs = lib.lib.hqkv_decode_workspace_bytes(desc) - fixed - up(rows * 128 * 8)
+        assert pairs == up(rows * expected(batch * kv, tiers) * 8), (batch, kv, tiers)
