@@ -187,13 +187,6 @@ __device__ __forceinline__ uint2 ld_stream(const uint2* p) {
   asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
   return v;
 }
-__device__ __forceinline__ uint4 ld_stream(const uint4* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p));
-  return v;
-}
 
 // shared memory by 32-bit address: loads with compile-time offsets, no generic-address arithmetic
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -207,11 +200,6 @@ __device__ __forceinline__ uint4 lds128(uint32_t a) {
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
   return v;
 }
-__device__ __forceinline__ uint32_t lds32(uint32_t a) {
-  uint32_t v;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
-  return v;
-}
 __device__ __forceinline__ uint32_t lds16(uint32_t a) {
   unsigned short v;
   asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
@@ -220,7 +208,6 @@ __device__ __forceinline__ uint32_t lds16(uint32_t a) {
 __device__ __forceinline__ void sts16(uint32_t a, uint32_t v) {
   asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"(static_cast<unsigned short>(v)) : "memory");
 }
-__device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
 __device__ __forceinline__ void sts64(uint32_t a, uint32_t x, uint32_t y) {
   asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(a), "r"(x), "r"(y) : "memory");
 }
@@ -255,11 +242,6 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t row
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(row_addr) : "memory");
 }
-// two of them, at the row addresses of lanes 0-15
-__device__ __forceinline__ void ldmatrix_x2_trans(uint32_t (&r)[2], uint32_t row_addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(row_addr) : "memory");
-}
-
 // the same without the transposition: lane (g, tig) gets elements 2*tig, 2*tig+1 of row g
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t row_addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -713,28 +695,28 @@ __device__ __forceinline__ void k_store_any(const DecodeParams& P, const TierDev
   bool valid[HALVES];
 #pragma unroll
   for (int u = 0; u < HALVES; ++u) valid[u] = wt0 + 32 * u < T.n_k;
-      const bool on = tig < P.r4;
-      const __half* mrow = P.mask ? P.mask + w.b * P.mask_bstride + (w.h0 + (on ? tig : 0)) * P.mask_hstride : nullptr;
-  #pragma unroll
-      for (int j = 0; j < NX; ++j) {
-        const int src = lb + k_step<BITS>(j);
-        uint32_t pos = __shfl_sync(0xffffffffu, pu[BITS == 4 ? j >> 2 : 0], src);
-        bool ok = on && valid[BITS == 4 ? j >> 2 : 0];
-        if constexpr (BITS <= 2) {
-          const uint32_t pos1 = __shfl_sync(0xffffffffu, pu[HALVES - 1], src);
-          if (k_lane_unit<BITS>() == 1) {
-            pos = pos1;
-            ok = on && valid[HALVES - 1];
-          }
-        }
-        ok = ok && HQKV_INDEX_OK(pos, P.L);
-        if (ok) {
-          if (mrow) x[j] += __half2float(mrow[pos]);
-          out[logit_at(pos, tig, P.r4, P.L)] = x[j];
-        } else {
-          x[j] = -INFINITY;
-        }
+  const bool on = tig < P.r4;
+  const __half* mrow = P.mask ? P.mask + w.b * P.mask_bstride + (w.h0 + (on ? tig : 0)) * P.mask_hstride : nullptr;
+#pragma unroll
+  for (int j = 0; j < NX; ++j) {
+    const int src = lb + k_step<BITS>(j);
+    uint32_t pos = __shfl_sync(0xffffffffu, pu[BITS == 4 ? j >> 2 : 0], src);
+    bool ok = on && valid[BITS == 4 ? j >> 2 : 0];
+    if constexpr (BITS <= 2) {
+      const uint32_t pos1 = __shfl_sync(0xffffffffu, pu[HALVES - 1], src);
+      if (k_lane_unit<BITS>() == 1) {
+        pos = pos1;
+        ok = on && valid[HALVES - 1];
       }
+    }
+    ok = ok && HQKV_INDEX_OK(pos, P.L);
+    if (ok) {
+      if (mrow) x[j] += __half2float(mrow[pos]);
+      out[logit_at(pos, tig, P.r4, P.L)] = x[j];
+    } else {
+      x[j] = -INFINITY;
+    }
+  }
 }
 
 // Store the lane's logits at their positions and add them to its running softmax statistics.  wt0 = the warp's first
@@ -1790,7 +1772,7 @@ __global__ void __launch_bounds__(NW * 32, V_SM_WARPS / NW) v_pass_kernel(const 
       bool ok = MODE == V_FOUR || (MODE == V_FEWER && P.r4 == 2);
 #pragma unroll
       for (int j = 0; j < NP; ++j) {
-          quad[j] = __shfl_sync(0xffffffffu, at[j], lane & 7);
+        quad[j] = __shfl_sync(0xffffffffu, at[j], lane & 7);
         ok = ok && at[j] == quad[j] + head && (quad[j] & 3u) == 0u && quad[j] < (static_cast<uint32_t>(P.L) & ~3u);
       }
       dense = __all_sync(0xffffffffu, ok);
@@ -1871,7 +1853,7 @@ __global__ void __launch_bounds__(NW * 32, V_SM_WARPS / NW) v_pass_kernel(const 
       uint32_t p[NP][2], n[NP][2];
 #pragma unroll
       for (int j = 0; j < NP; ++j) {
-          if constexpr (MODE == V_GIVEN) {
+        if constexpr (MODE == V_GIVEN) {
           p[j][0] = pack_f16x2(x[j][0], x[j][1]), p[j][1] = pack_f16x2(x[j][2], x[j][3]);
         } else {
           float e[4];
