@@ -1,5 +1,7 @@
 """The variants of the V pass (pairs of 16-token steps and warps per CTA, channel groups, heads that are there) and of the K pass
 (groups of 64 and 128) at the edges of their tiles, and outputs that are not numbers; against the fp32 oracle."""
+import re
+
 import numpy as np
 import pytest
 import torch
@@ -8,6 +10,7 @@ from oracle import hqkv_oracle as O
 
 pytestmark = pytest.mark.gpu
 CODEBOOK = "high_uniform_group_low_normal_group"
+tilings = []
 
 
 def _build(dev, B, nh_q, nh_kv, ctx, res, shares, f16, group, strategy, shuffled, seed=3):
@@ -25,16 +28,17 @@ def _oracle(cache, q, group, strategy):
     return O.decode_attention(q.cpu().numpy(), host, None, group, group, quant_strategy=strategy)
 
 
-# (batch, query heads, kv heads, context, residual, shares, fp16 tokens, group, strategy, shuffled), GV, mode, pairs, warps
+# The shapes were taken so that every tiling runs (how a shape is divided is the library's affair: test_every_tiling_ran).
+# (batch, query heads, kv heads, context, residual, shares, fp16 tokens, group, strategy, shuffled), GV, mode
 @pytest.mark.parametrize("case,kernel", [
-    ((1, 32, 8, 3 * 256 + 32 + 33, 33, (0.3, 0.4, 0.3), 0, 32, "uniform_group", False), (5, 0, 1, 8)),     # last tile of 32, L odd
-    ((1, 16, 8, 1024 + 2, 2, (0.25, 0.25, 0.25, 0.25), 64, 32, CODEBOOK, True), (5, 1, 1, 8)),             # two heads, any positions
-    ((1, 8, 8, 2 * 256 + 7, 7, (0.5, 0.25, 0.25), 0, 64, "uniform_group", False), (6, 1, 1, 8)),           # one head
-    ((1, 32, 8, 32640 + 45, 45, (0.0, 0.34, 0.33, 0.33), 64, 32, CODEBOOK, False), (5, 0, 2, 8)),
-    ((1, 32, 8, 32640 + 2, 2, (0.2, 0.4, 0.4), 0, 128, "uniform_group", True), (7, 0, 2, 8)),
-    ((40, 32, 8, 1376 + 32 + 13, 13, (0.3, 0.4, 0.3), 0, 64, "uniform_group", False), (6, 0, 2, 4)),
-    ((40, 16, 8, 1152 + 4, 4, (0.25, 0.25, 0.25, 0.25), 128, 128, "uniform_group", False), (7, 1, 2, 4)),       # 2 and 1 bits, groups of 128
-    ((40, 32, 8, 1088 + 6, 6, (0.2, 0.2, 0.3, 0.3), 32, 64, CODEBOOK, True), (6, 0, 2, 4))])
+    ((1, 32, 8, 3 * 256 + 32 + 33, 33, (0.3, 0.4, 0.3), 0, 32, "uniform_group", False), (5, 0)),     # last tile of 32, L odd
+    ((1, 16, 8, 1024 + 2, 2, (0.25, 0.25, 0.25, 0.25), 64, 32, CODEBOOK, True), (5, 1)),             # two heads, any positions
+    ((1, 8, 8, 2 * 256 + 7, 7, (0.5, 0.25, 0.25), 0, 64, "uniform_group", False), (6, 1)),           # one head
+    ((1, 32, 8, 32640 + 45, 45, (0.0, 0.34, 0.33, 0.33), 64, 32, CODEBOOK, False), (5, 0)),
+    ((1, 32, 8, 32640 + 2, 2, (0.2, 0.4, 0.4), 0, 128, "uniform_group", True), (7, 0)),
+    ((40, 32, 8, 1376 + 32 + 13, 13, (0.3, 0.4, 0.3), 0, 64, "uniform_group", False), (6, 0)),
+    ((40, 16, 8, 1152 + 4, 4, (0.25, 0.25, 0.25, 0.25), 128, 128, "uniform_group", False), (7, 1)),       # 2 and 1 bits, groups of 128
+    ((40, 32, 8, 1088 + 6, 6, (0.2, 0.2, 0.3, 0.3), 32, 64, CODEBOOK, True), (6, 0))])
 def test_variants(cuda_device, case, kernel):
     from torch.profiler import ProfilerActivity, profile
 
@@ -46,12 +50,21 @@ def test_variants(cuda_device, case, kernel):
     with profile(activities=[ProfilerActivity.CUDA]) as prof:
         w, out = qkv_matmul_hqe_2(q, cache, None, 128, strategy, group, group)
         torch.cuda.synchronize()
-    names = [e.key for e in prof.key_averages()]
-    assert any("v_pass_kernel<%d, %d, %d, %d>" % kernel in n for n in names), names
+    ran = [tuple(map(int, m.groups())) for e in prof.key_averages()
+           for m in [re.search(r"v_pass_kernel<(\d+), (?:\(.*?\))?(\d+), (\d+), (\d+)>", e.key)] if m]
+    assert len(ran) == 1 and ran[0][:2] == kernel, [e.key for e in prof.key_averages()]
+    tilings.append(ran[0][2:])
     ow, oo = _oracle(cache, q, group, strategy)
     out, w = out.float().cpu().numpy(), w.float().cpu().numpy()
     assert float((np.abs(out - oo).max(-1) / np.abs(oo).max(-1)).max()) <= 2e-3
     assert np.all(np.abs(w - ow) <= 2.0 ** -24 + 2.0 ** -9 * ow)
+
+
+def test_every_tiling_ran():
+    """(pairs of steps, warps) of the calls above: if this fails, the division of work has changed and other shapes are due there."""
+    if len(tilings) < 8:
+        pytest.skip("follows the whole of test_variants")
+    assert set(tilings) == {(1, 8), (2, 8), (2, 4)}
 
 
 # shares of a plane: up to 64, more, more than 256
