@@ -1142,51 +1142,62 @@ constexpr uint32_t V_NONE = 0xFFFFFFFFu;
 // A value that the compiler cannot work out again from thread and block indices: what a loop uses of them is computed once.
 __device__ __forceinline__ uint32_t keep(uint32_t v) { return __shfl_sync(0xffffffffu, v, threadIdx.x & 31); }
 
-// Logits (or given weights) of the lane's NP quads, whose positions are idx[0 .. 3] and idx[32 .. 35] below `left`; -inf (0) beyond.
-// dense (the same for the warp): they are quad[j] and the next three, quads of the scratch.  Two query heads: the lanes of the
-// other two read the first two's.
+// Logits (or given weights) of the lane's NP quads, tokens 0 .. 3 and 32 .. 35 below `left`; -inf (0) beyond.  at: positions as the
+// warp has them, of token `head` of the lane's quads.  dense (the same for the warp): they are quad[j] and the next three, quads of the
+// scratch.  Fewer query heads: the lanes of the others read the first ones'.  Given weights are those of `rows`, the head's from
+// `row` on (V_NONE: no such head); whole: its quads start on 8-byte boundaries.
 template <int MODE, int NP>
-__device__ __forceinline__ void v_gather(const DecodeParams& P, const Where& w, int head, bool dense, const uint32_t (&quad)[NP], const int64_t* idx,
-                                         int left, float (&x)[NP][4]) {
+__device__ __forceinline__ void v_gather(const DecodeParams& P, const Where& w, int head, const __half* rows, uint32_t row, bool whole, bool dense,
+                                         const uint32_t (&quad)[NP], const uint32_t (&at)[NP], int left, float (&x)[NP][4]) {
   const float* logits = P.logits + static_cast<int64_t>(w.bvh) * P.L * P.r4;
+  const unsigned short* given = reinterpret_cast<const unsigned short*>(rows) + (row != V_NONE ? row : 0u);
   if (dense) {
 #pragma unroll
     for (int j = 0; j < NP; ++j) {
       if constexpr (MODE == V_FOUR) {
         const float4 v = __ldcg(reinterpret_cast<const float4*>(logits) + (quad[j] + static_cast<uint32_t>(head)));
         x[j][0] = v.x, x[j][1] = v.y, x[j][2] = v.z, x[j][3] = v.w;
-      } else {  // (rows of two heads start on 8-byte boundaries)
+      } else if (MODE == V_GIVEN) {
+        uint2 v = make_uint2(0u, 0u);
+        if (row != V_NONE) {
+          const unsigned short* p = given + quad[j];
+          if (whole) v = __ldcg(reinterpret_cast<const uint2*>(p));
+          else v = make_uint2(pack_lo16(__ldcg(p), __ldcg(p + 1)), pack_lo16(__ldcg(p + 2), __ldcg(p + 3)));
+        }
+        const float2 a = __half22float2(u32_as_h2(v.x)), b = __half22float2(u32_as_h2(v.y));
+        x[j][0] = a.x, x[j][1] = a.y, x[j][2] = b.x, x[j][3] = b.y;
+      } else if (P.r4 == 2) {  // (rows of two heads start on 8-byte boundaries)
         const float2* q = reinterpret_cast<const float2*>(logits) + (quad[j] + 2u * static_cast<uint32_t>(head & 1));
         const float2 a = __ldcg(q), b = __ldcg(q + 1);
         x[j][0] = a.x, x[j][1] = a.y, x[j][2] = b.x, x[j][3] = b.y;
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[j][i] = __ldcg(logits + (quad[j] + i));
       }
     }
     return;
   }
-#pragma unroll 1
-  for (int i = 0; i < 4 * NP; ++i) {
-    const int t = (i & 3) + 8 * (i & 4);
-    float v = MODE == V_GIVEN ? 0.f : -INFINITY;
-    const uint32_t pos = t < left ? __ldg(reinterpret_cast<const uint32_t*>(idx + t)) : V_NONE;
-    if (pos != V_NONE && HQKV_INDEX_OK(pos, P.L)) {
-      if constexpr (MODE == V_GIVEN) {
-        const int64_t row = (static_cast<int64_t>(w.b) * P.nh_q + w.h0 + head) * P.L;
-        if (head < P.r4) v = __half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(P.probs_in) + row + pos)));
-      } else {
-        v = __ldcg(logits + logit_at(pos, head & (P.r4 - 1), P.r4, P.L));
+#pragma unroll
+  for (int j = 0; j < NP; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      x[j][i] = MODE == V_GIVEN ? 0.f : -INFINITY;
+      const uint32_t pos = __shfl_sync(0xffffffffu, at[j], 8 * i + (threadIdx.x & 7));
+      if (32 * j + i < left && pos != V_NONE && HQKV_INDEX_OK(pos, P.L)) {
+        if constexpr (MODE == V_GIVEN) {
+          if (row != V_NONE) x[j][i] = __half2float(__ushort_as_half(__ldcg(given + pos)));
+        } else {
+          x[j][i] = __ldcg(logits + logit_at(pos, head & (P.r4 - 1), P.r4, P.L));
+        }
       }
     }
-#pragma unroll
-    for (int k = 0; k < 4 * NP - 1; ++k) x[k >> 2][k & 3] = x[(k + 1) >> 2][(k + 1) & 3];
-    x[NP - 1][3] = v;
-  }
 }
 
-// The probabilities n of the lane's quads (see v_gather; tokens 0 1, 2 3 of each) to their positions of the row that starts
+// The probabilities n of the lane's quads (tokens 0 1, 2 3 of each), whose positions are idx[0 .. 3] and idx[32 .. 35], to the row that starts
 // at `at` elements of rows.  whole: all rows' quads start on 8-byte boundaries.
 template <int NP>
 __device__ __forceinline__ void v_store_probs(__half* rows, uint32_t at, bool whole, bool dense, const uint32_t (&quad)[NP], const int64_t* idx,
-                                              int left, int L, uint32_t (&n)[NP][2]) {
+                                              int left, int L, const uint32_t (&n)[NP][2]) {
   if (dense) {
 #pragma unroll
     for (int j = 0; j < NP; ++j) {
@@ -1204,17 +1215,16 @@ __device__ __forceinline__ void v_store_probs(__half* rows, uint32_t at, bool wh
     }
     return;
   }
-#pragma unroll 1
+  uint32_t pos[4 * NP];
+#pragma unroll
   for (int i = 0; i < 4 * NP; ++i) {
     const int t = (i & 3) + 8 * (i & 4);
-    if (t < left) {
-      const uint32_t pos = __ldg(reinterpret_cast<const uint32_t*>(idx + t));
-      if (!HQKV_CHECKS_ENABLED || pos < static_cast<uint32_t>(L)) rows[at + pos] = __ushort_as_half(static_cast<unsigned short>(n[0][0]));
-    }
-#pragma unroll
-    for (int k = 0; k < 2 * NP - 1; ++k) n[k >> 1][k & 1] = pack_hi_lo(n[k >> 1][k & 1], n[(k + 1) >> 1][(k + 1) & 1]);
-    n[NP - 1][1] >>= 16;
+    pos[i] = t < left ? __ldg(reinterpret_cast<const uint32_t*>(idx + t)) : V_NONE;
   }
+#pragma unroll
+  for (int i = 0; i < 4 * NP; ++i)
+    if (pos[i] != V_NONE && (!HQKV_CHECKS_ENABLED || pos[i] < static_cast<uint32_t>(L)))
+      rows[at + pos[i]] = __ushort_as_half(static_cast<unsigned short>(i & 1 ? n[i >> 2][(i >> 1) & 1] >> 16 : n[i >> 2][(i >> 1) & 1]));
 }
 
 // -C * std, to 22 bits, as two halfs
@@ -1694,8 +1704,8 @@ __global__ void __launch_bounds__(NW * 32, V_SM_WARPS / NW) v_pass_kernel(const 
   // The lane in the softmax: head lane / 8, quad lane % 8 of the eight of a pair of steps.
   constexpr int tile = 32 * NP, stride = NW * tile;   // tokens of a warp, of the CTA at a time
   const int head = lane >> 3, wtok = warp * tile + 4 * (lane & 7), mine = keep(wtok + head);   // first token of its first quad; whose position it fetches
-  __half* rows = P.weights + (static_cast<int64_t>(w.b) * P.nh_q + w.h0) * P.L;
-  const uint32_t row = MODE != V_GIVEN && head < P.r4 ? static_cast<uint32_t>(head) * static_cast<uint32_t>(P.L) : V_NONE;
+  __half* rows = (MODE == V_GIVEN ? const_cast<__half*>(P.probs_in) : P.weights) + (static_cast<int64_t>(w.b) * P.nh_q + w.h0) * P.L;   // (given ones are read)
+  const uint32_t row = head < P.r4 ? static_cast<uint32_t>(head) * static_cast<uint32_t>(P.L) : V_NONE;
   float mh = INFINITY, inv = 0.f;   // max * log2(e), 1 / sum; of a head that is not there: probability 0
   const bool whole = ((reinterpret_cast<uintptr_t>(rows) | (static_cast<uintptr_t>(P.L) << 1)) & 7u) == 0u;
   const uint32_t rem = keep((g & 1) ? 0xFFFFFFFFu : 0u);
@@ -1762,21 +1772,21 @@ __global__ void __launch_bounds__(NW * 32, V_SM_WARPS / NW) v_pass_kernel(const 
         // (Beyond the tier, whose last 32 tokens are all there wherever it holds a multiple of 32: those once more.  Their
         // probabilities are stored once more, too, and count with scales and zeros of 0.)
         int t = mine + 32 * j;
-        if (t >= left) t = left - 32 + (t & 31);
-        at[j] = left >= 32 ? __ldg(reinterpret_cast<const uint32_t*>(idx + t)) : V_NONE;
+        if (t >= left && left >= 32) t = left - 32 + (t & 31);
+        at[j] = t < left ? __ldg(reinterpret_cast<const uint32_t*>(idx + t)) : V_NONE;
       }
     };
     float x[NP][4];
     // Requested for the tiles that have `left` tokens from the first on: the logits (positions in at), the positions of the ones after them.
     auto gather = [&](int left) {
-      bool ok = MODE == V_FOUR || (MODE == V_FEWER && P.r4 == 2);
+      bool ok = true;
 #pragma unroll
       for (int j = 0; j < NP; ++j) {
         quad[j] = __shfl_sync(0xffffffffu, at[j], lane & 7);
         ok = ok && at[j] == quad[j] + head && (quad[j] & 3u) == 0u && quad[j] < (static_cast<uint32_t>(P.L) & ~3u);
       }
       dense = __all_sync(0xffffffffu, ok);
-      v_gather<MODE, NP>(P, w, head, dense, quad, idx + wtok, min(left - wtok, tile), x);
+      v_gather<MODE, NP>(P, w, head, rows, row, whole, dense, quad, at, min(left - wtok, tile), x);
       positions(idx + stride, left - stride);
     };
     __syncwarp();   // (the buffers may have served another tier)
