@@ -95,9 +95,10 @@ struct DecodeParams {
 // The tokens of a (batch, virtual kv head) plane are a list of UNITS, tiers in order, and its CTAs take consecutive shares of
 // it of equal COST, for the CTA with the longest share decides (20/40/40 at 24 x 8 x 15360 tokens in shares of equal count:
 // the V pass took 94 us, the time of the CTAs with 4 and 2 bits only).  K pass: 256 tokens of a tier (128 at 8 bits, 64 of the
-// fp16 tier and of the residual window).  V pass: 256 (64 in fp16), or 128 where that many CTAs find a place at once.
-// us a unit with four CTAs on every SM, K pass: 8 bits 1.9, 4 bits 3.2, 2 bits 2.9, 1 bit 3.3, fp16 tier 4.3, residual window
-// 3.2; V pass: 8 bits 4.0, 4 bits 2.7, 2 bits 2.5, fp16 2.4.
+// fp16 tier and of the residual window).  V pass: a tile per warp, so 256 or 512 (64 in fp16).
+// us a unit, K pass with four CTAs on every SM: 8 bits 1.9, 4 bits 3.2, 2 bits 2.9, 1 bit 3.3, fp16 tier 4.3, residual window
+// 3.2; V pass with two CTAs of eight warps and 512 tokens: 8 bits 6.5, 4 bits 4.1, 2 bits 4.2, 1 bit 4.8 (16 x 8 planes of 16 k: 89,
+// 57, 58 and 66 us a launch).
 __host__ __device__ constexpr int unit_tokens(int bits) { return bits == 16 ? 64 : bits == 8 ? 128 : 256; }
 __host__ __device__ constexpr int unit_cost(int bits) { return bits == 8 ? 5 : 8; }
 // This CTA's tokens [t0, t1) of tier ti; false: none.
@@ -1146,6 +1147,10 @@ __device__ __forceinline__ uint32_t keep(uint32_t v) { return __shfl_sync(0xffff
 // warp has them, of token `head` of the lane's quads.  dense (the same for the warp): they are quad[j] and the next three, quads of the
 // scratch.  Fewer query heads: the lanes of the others read the first ones'.  Given weights are those of `rows`, the head's from
 // `row` on (V_NONE: no such head); whole: its quads start on 8-byte boundaries.
+// What is not a quad goes four tokens at a time: eight at a time cost the usual path 7 of 311 us (16 layers of 32 k tokens) in registers.
+// us a call at 8 x 16 k, before quads (four tokens' loads together) / quads, the rest one by one / now: one head 74 / 81 / 59, any
+// positions 91 / 111 / 96, given weights 38 / 41 / 28, and 55 / 50 / 44 at any positions.  Consecutive positions that start between quads
+// take 57 / 86 / 72: the K pass writes their logits four bytes at a time.
 template <int MODE, int NP>
 __device__ __forceinline__ void v_gather(const DecodeParams& P, const Where& w, int head, const __half* rows, uint32_t row, bool whole, bool dense,
                                          const uint32_t (&quad)[NP], const uint32_t (&at)[NP], int left, float (&x)[NP][4]) {
@@ -1177,20 +1182,26 @@ __device__ __forceinline__ void v_gather(const DecodeParams& P, const Where& w, 
     }
     return;
   }
-#pragma unroll
-  for (int j = 0; j < NP; ++j)
+  uint32_t mine = at[0];
+#pragma unroll 1
+  for (int j = 0; j < NP; ++j) {
+    float y[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      x[j][i] = MODE == V_GIVEN ? 0.f : -INFINITY;
-      const uint32_t pos = __shfl_sync(0xffffffffu, at[j], 8 * i + (threadIdx.x & 7));
+      y[i] = MODE == V_GIVEN ? 0.f : -INFINITY;
+      const uint32_t pos = __shfl_sync(0xffffffffu, mine, 8 * i + (threadIdx.x & 7));
       if (32 * j + i < left && pos != V_NONE && HQKV_INDEX_OK(pos, P.L)) {
         if constexpr (MODE == V_GIVEN) {
-          if (row != V_NONE) x[j][i] = __half2float(__ushort_as_half(__ldcg(given + pos)));
+          if (row != V_NONE) y[i] = __half2float(__ushort_as_half(__ldcg(given + pos)));
         } else {
-          x[j][i] = __ldcg(logits + logit_at(pos, head & (P.r4 - 1), P.r4, P.L));
+          y[i] = __ldcg(logits + logit_at(pos, head & (P.r4 - 1), P.r4, P.L));
         }
       }
     }
+    mine = at[NP - 1];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[0][i] = x[NP - 1][i], x[NP - 1][i] = y[i];
+  }
 }
 
 // The probabilities n of the lane's quads (tokens 0 1, 2 3 of each), whose positions are idx[0 .. 3] and idx[32 .. 35], to the row that starts
@@ -1215,16 +1226,18 @@ __device__ __forceinline__ void v_store_probs(__half* rows, uint32_t at, bool wh
     }
     return;
   }
-  uint32_t pos[4 * NP];
+  uint32_t a = n[0][0], b = n[0][1];
+#pragma unroll 1
+  for (int j = 0; j < NP; ++j) {
+    uint32_t pos[4];
 #pragma unroll
-  for (int i = 0; i < 4 * NP; ++i) {
-    const int t = (i & 3) + 8 * (i & 4);
-    pos[i] = t < left ? __ldg(reinterpret_cast<const uint32_t*>(idx + t)) : V_NONE;
+    for (int i = 0; i < 4; ++i) pos[i] = 32 * j + i < left ? __ldg(reinterpret_cast<const uint32_t*>(idx + 32 * j + i)) : V_NONE;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (pos[i] != V_NONE && (!HQKV_CHECKS_ENABLED || pos[i] < static_cast<uint32_t>(L)))
+        rows[at + pos[i]] = __ushort_as_half(static_cast<unsigned short>((i < 2 ? a : b) >> 16 * (i & 1)));
+    a = n[NP - 1][0], b = n[NP - 1][1];
   }
-#pragma unroll
-  for (int i = 0; i < 4 * NP; ++i)
-    if (pos[i] != V_NONE && (!HQKV_CHECKS_ENABLED || pos[i] < static_cast<uint32_t>(L)))
-      rows[at + pos[i]] = __ushort_as_half(static_cast<unsigned short>(i & 1 ? n[i >> 2][(i >> 1) & 1] >> 16 : n[i >> 2][(i >> 1) & 1]));
 }
 
 // -C * std, to 22 bits, as two halfs
